@@ -12,7 +12,8 @@
 //   dK/dV kernel per 128-key tile:  S^T = K Q^T, dP^T = V dO^T, P^T and dS^T to shared memory, dV += P^T dO, dK += dS^T Q.
 //   dQ kernel per 128-query tile:   S = Q K^T, dP = dO V^T, dS to shared memory, dQ += dS K.
 // RoPE's backward rotation of dQ/dK can be applied in the epilogue (each thread holds a full head row).
-// Head sizes other than 64/128 (or unaligned strides) use a plain SIMT implementation further down.
+// Bidirectional attention and the other head sizes that are multiples of 16: attn_split.cuh.  What is left (odd head sizes,
+// unaligned pointers) uses a plain SIMT implementation further down.
 #include "../tc.cuh"
 #include <algorithm>
 #include <mutex>
@@ -2101,6 +2102,8 @@ int set_smem(K kern, int bytes) {
   return (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
+#include "attn_split.cuh"
+
 bool tc_ok(const void* qkv, const void* other, int H, int hd) {
   const int C = H * hd;
   return !g_attn_force_simt && (hd == 64 || hd == 128) && ((uintptr_t)qkv % 16 == 0) && ((uintptr_t)other % 16 == 0) && (C % 8 == 0);
@@ -2229,23 +2232,32 @@ MLB_API int mlb_attn_fwd(void* out, float* lse, const void* qkv, int B, int T, i
     return (int)cudaGetLastError();
   }
   if (hd > 256) return -4;
+  if (split_ok(qkv, out, out, T, hd, 1)) return split_fwd(out, lse, qkv, B, T, H, hd, 1, st);
   attn_fwd_simt_k<<<dim3(T, H, B), 128, (T + 32) * sizeof(float), st>>>((bf16*)out, lse, (const bf16*)qkv, B, T, H, hd, scale);
   return (int)cudaGetLastError();
 }
 
-// Bidirectional (no causal mask) attention for short sequences such as a vision encoder's patch tokens: the scalar
-// kernels, any T and head size <= 256.  Same layouts as mlb_attn_fwd / mlb_attn_bwd; delta is scratch of B*H*T floats.
+// Bidirectional (no causal mask) attention for short sequences such as a vision encoder's patch tokens: head sizes that are
+// multiples of 16 up to 128 on the tensor cores (attn_split.cuh), any other up to 256 in the scalar kernels.  Same layouts as mlb_attn_fwd / mlb_attn_bwd; delta is scratch of B*H*T floats.
 MLB_API int mlb_attn_bidir_fwd(void* out, float* lse, const void* qkv, int B, int T, int H, int hd, cudaStream_t st) {
   if (hd > 256 || (size_t)(T + 32) * sizeof(float) > 48 * 1024) return -4;
+  if (split_ok(qkv, out, out, T, hd, 1)) return split_fwd(out, lse, qkv, B, T, H, hd, 0, st);
   attn_fwd_simt_k<<<dim3(T, H, B), 128, (T + 32) * sizeof(float), st>>>((bf16*)out, lse, (const bf16*)qkv, B, T, H, hd, 1.0f / sqrtf((float)hd), 0);
   return (int)cudaGetLastError();
+}
+static void attn_delta_launch(float* delta, const void* dout, const void* out, int B, int T, int H, int hd, cudaStream_t st) {
+  const long heads = (long)B * T * H;
+  const int gsz = hd / 8;
+  const bool vec = (hd % 8 == 0) && heads * gsz < (1L << 31) && gsz <= 32 && (gsz & (gsz - 1)) == 0 && ((uintptr_t)dout % 16 == 0) && ((uintptr_t)out % 16 == 0);
+  if (vec) mlb_launch(attn_delta_k, dim3((unsigned)((heads * gsz + 255) / 256)), dim3(256), 0, st, delta, (const bf16*)dout, (const bf16*)out, B, T, H, hd);
+  else attn_delta_scalar_k<<<(unsigned)((heads * 32 + 255) / 256), 256, 0, st>>>(delta, (const bf16*)dout, (const bf16*)out, B, T, H, hd);
 }
 MLB_API int mlb_attn_bidir_bwd(void* dqkv, const void* dout, const void* qkv, const void* out, const float* lse, float* delta, int B, int T,
                                int H, int hd, cudaStream_t st) {
   if (hd > 256 || (size_t)2 * T * sizeof(float) > 48 * 1024) return -4;
   const float scale = 1.0f / sqrtf((float)hd);
-  const long heads = (long)B * T * H;
-  attn_delta_scalar_k<<<(unsigned)((heads * 32 + 255) / 256), 256, 0, st>>>(delta, (const bf16*)dout, (const bf16*)out, B, T, H, hd);
+  attn_delta_launch(delta, dout, out, B, T, H, hd, st);
+  if (split_ok(qkv, dqkv, dout, T, hd, 1)) return split_bwd(dqkv, dout, qkv, lse, delta, B, T, H, hd, 0, st);
   attn_bwd_q_simt_k<<<dim3(T, H, B), 128, T * sizeof(float), st>>>((bf16*)dqkv, (const bf16*)dout, (const bf16*)qkv, lse, delta, B, T, H, hd, scale, 0);
   attn_bwd_kv_simt_k<<<dim3(T, H, B), 128, 2 * T * sizeof(float), st>>>((bf16*)dqkv, (const bf16*)dout, (const bf16*)qkv, lse, delta, B, T, H, hd, scale, 0);
   return (int)cudaGetLastError();
@@ -2279,13 +2291,7 @@ static int attn_bwd_impl(void* dqkv, const void* dout, const void* qkv, const vo
                          int B, int T, int H, int hd, const float* cosT, const float* sinT, int have_delta, cudaStream_t st) {
   const int C = H * hd;
   const float scale = 1.0f / sqrtf((float)hd);
-  if (!have_delta) {
-    const long heads = (long)B * T * H;
-    const int gsz = hd / 8;
-    const bool vec = (hd % 8 == 0) && heads * gsz < (1L << 31) && gsz <= 32 && (gsz & (gsz - 1)) == 0 && ((uintptr_t)dout % 16 == 0) && ((uintptr_t)out % 16 == 0);
-    if (vec) mlb_launch(attn_delta_k, dim3((unsigned)((heads * gsz + 255) / 256)), dim3(256), 0, st, delta, (const bf16*)dout, (const bf16*)out, B, T, H, hd);
-    else attn_delta_scalar_k<<<(unsigned)((heads * 32 + 255) / 256), 256, 0, st>>>(delta, (const bf16*)dout, (const bf16*)out, B, T, H, hd);
-  }
+  if (!have_delta) attn_delta_launch(delta, dout, out, B, T, H, hd, st);
   if (tc_ok(qkv, dout, H, hd) && ((uintptr_t)dqkv % 16 == 0)) {
     const CUtensorMap* tq = mlb_tmap_cached(qkv, (uint64_t)B * T, 3 * C, 3 * C, 128, 64);
     const CUtensorMap* td = mlb_tmap_cached(dout, (uint64_t)B * T, C, C, 128, 64);
@@ -2335,6 +2341,10 @@ static int attn_bwd_impl(void* dqkv, const void* dout, const void* qkv, const vo
     return cosT ? 1 : 0;
   }
   if (hd > 256) return -4;
+  if (split_ok(qkv, dqkv, dout, T, hd, 2)) {
+    const int rc = split_bwd(dqkv, dout, qkv, lse, delta, B, T, H, hd, 1, st);
+    return rc > 0 ? rc + 1000 : rc;
+  }
   attn_bwd_q_simt_k<<<dim3(T, H, B), 128, T * sizeof(float), st>>>((bf16*)dqkv, (const bf16*)dout, (const bf16*)qkv, lse, delta, B, T, H,
                                                                   hd, scale);
   attn_bwd_kv_simt_k<<<dim3(T, H, B), 128, 2 * T * sizeof(float), st>>>((bf16*)dqkv, (const bf16*)dout, (const bf16*)qkv, lse, delta, B,

@@ -1,0 +1,456 @@
+// Attention with full-precision probabilities on the tensor cores: bidirectional attention (the image encoder's) and causal
+// attention at the head sizes the kernels of attn.cu are not built for (any multiple of 16 up to 128 but 64 and 128).
+// Included by attn.cu (shares its error word and helpers).
+//
+// The scalar kernels these replace keep P and dS in fp32, so a bf16 operand alone would lose precision.  Each value goes
+// to the tensor core as two bf16 terms, x = hi + lo with hi = bf16(x), lo = bf16(x - hi): 16 significant bits, and Q, K, V, dO are
+// bf16 to begin with, so a product costs one more MMA pass and its error (2^-17) disappears under the bf16 rounding of the result.
+//
+// One CTA of 128 threads (thread = one row of the 128-row tile) per tile, (head, sample); the other operand streams in
+// 64-row blocks, double buffered by TMA.  The hi / lo terms are written over the TMEM columns of the scores they came from
+// (32 fp32 scores -> 16 columns hi + 16 columns lo) and feed the next product as its A operand from there, so no shared
+// memory is spent on them and two (backward) to four (forward) CTAs share an SM: their MMAs, exponentials and loads
+// overlap across CTAs, which is why a CTA by itself is a plain sequence.  What bounds it is that sequence's latency, not a
+// unit.  64-row blocks because the encoder's sequences are short (197 tokens = 3.1 blocks of 64, 1.5 of 128).
+// Sequences are the third dimension of the tensor maps: rows past a sample's end arrive as zeros, never as the next
+// sample's values (0 * inf would be NaN).
+struct SplitArgs {
+  int B, T, H, hd, causal;
+  float scale;
+  bf16* out;            // forward: out[B*T, C]; backward: dqkv[B*T, 3C]
+  float* lse;           // [B,H,T]
+  const float* delta;   // [B,H,T]
+};
+
+constexpr int SPLIT_THREADS = 128;
+constexpr int BOX_BYTES = 64 * 64 * 2;      // one TMA box: 64 rows x 64 columns, 128-byte swizzled rows
+
+// [64 x (64 * chunks)] block, chunks BOX_BYTES apart: K-major k-step of 16 columns / MN-major k-step of 16 rows.
+__device__ __forceinline__ uint64_t desc64_k(uint32_t base, int ks) {
+  return tc::smem_desc_sw128(base + (ks >> 2) * BOX_BYTES + (ks & 3) * 32, 16, 1024);
+}
+__device__ __forceinline__ uint64_t desc64_mn(uint32_t base, int ks) { return tc::smem_desc_sw128(base + ks * 2048, BOX_BYTES, 1024); }
+// TMEM column of the hi term of k-step ks (16 rows of the 64-row block); the lo term is 16 columns further
+__device__ __forceinline__ uint32_t split_col(int ks) { return (uint32_t)((ks >> 1) * 32 + (ks & 1) * 8); }
+
+__device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo) {
+  hi = pack_bf16(a, b);
+  lo = pack_bf16(a - __uint_as_float(hi << 16), b - __uint_as_float(hi & 0xffff0000u));
+}
+
+// An earlier CTA of this library gave up on a wait: leave at once instead of queueing more waits behind it (CTA-uniform).
+__device__ __forceinline__ bool attn_given_up() {
+  __shared__ int s_skip;
+  if (threadIdx.x == 0) s_skip = *(volatile int*)&g_mlb_error;
+  __syncthreads();
+  return s_skip != 0;
+}
+
+// rows [r0, r0 + 64 * boxes) of `CH` 64-column chunks starting at column x0 of sample z
+template <int CH>
+__device__ __forceinline__ void split_load(uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, int x0, int r0, int z, int boxes) {
+  for (int c = 0; c < CH; c++)
+    for (int i = 0; i < boxes; i++) tc::tma_load_3d(dst + (c * boxes + i) * BOX_BYTES, tm, bar, x0 + c * 64, r0 + i * 64, z);
+}
+
+// hd columns of this thread's TMEM row, times f, as bf16 to dst (16-byte aligned, hd a multiple of 16)
+template <int HDT>
+__device__ __forceinline__ void split_store_row(bf16* dst, uint32_t taddr, int hd, float f, bool live) {
+#pragma unroll
+  for (int c = 0; c < HDT; c += 32) {
+    uint32_t r[32];
+    tc::tmem_ld32(taddr + c, r);      // (warp-collective: every lane takes part, live or not)
+    tc::tmem_ld_wait();
+#pragma unroll
+    for (int v = 0; v < 4; v++) {
+      if (live && c + v * 8 < hd) {
+        uint4 w;
+        w.x = pack_bf16(__uint_as_float(r[v * 8]) * f, __uint_as_float(r[v * 8 + 1]) * f);
+        w.y = pack_bf16(__uint_as_float(r[v * 8 + 2]) * f, __uint_as_float(r[v * 8 + 3]) * f);
+        w.z = pack_bf16(__uint_as_float(r[v * 8 + 4]) * f, __uint_as_float(r[v * 8 + 5]) * f);
+        w.w = pack_bf16(__uint_as_float(r[v * 8 + 6]) * f, __uint_as_float(r[v * 8 + 7]) * f);
+        *reinterpret_cast<uint4*>(dst + c + v * 8) = w;
+      }
+    }
+  }
+}
+
+template <int HDT>
+struct SplitFwdSmem {
+  static constexpr int CH = HDT == 128 ? 2 : 1;
+  static constexpr int Q = 0;
+  static constexpr int K = Q + 2 * CH * BOX_BYTES;      // 2 buffers
+  static constexpr int V = K + 2 * CH * BOX_BYTES;      // 2 buffers
+  static constexpr int BAR = V + 2 * CH * BOX_BYTES;
+  static constexpr int TOTAL = BAR + 128 + 1024;
+};
+
+template <int HDT>
+__global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_constant__ CUtensorMap tm, const SplitArgs a) {
+  using S = SplitFwdSmem<HDT>;
+  constexpr int CH = S::CH;
+  constexpr uint32_t TMEM_COLS = HDT == 128 ? 256 : 128;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint64_t* bars = (uint64_t*)(smem + S::BAR);
+  uint64_t *bar_q = bars, *bar_k = bars + 1 /*[2]*/, *bar_v = bars + 3 /*[2]*/, *bar_s = bars + 5, *bar_o = bars + 6;
+  uint32_t* tmem_slot = (uint32_t*)(bars + 7);
+  volatile int* s_abort = (volatile int*)(bars + 8);
+  if (attn_given_up()) return;
+
+  const int ntile = (a.T + 127) / 128;
+  const int qt = ntile - 1 - (int)blockIdx.x, h = blockIdx.y, b = blockIdx.z;     // (causal: longest rows first)
+  const int q0 = qt * 128, C = a.H * a.hd;
+  const int tid = threadIdx.x, warp = tid >> 5;
+  if (tid == 0) {
+    for (int i = 0; i < 7; i++) tc::mbar_init(&bars[i], 1);
+    *s_abort = 0;
+    tc::mbar_fence_init();
+    tc::tma_prefetch_desc(&tm);
+  }
+  if (warp == 0) tc::tmem_alloc(tmem_slot, TMEM_COLS);
+  tc::tc_fence_before();
+  __syncthreads();
+  tc::tc_fence_after();
+  mlb_pdl_sync();
+  const uint32_t t_s = *tmem_slot, t_o = t_s + 64, lane_addr = (uint32_t)(warp * 32) << 16;
+  // Bounded, sticky: after one expiry every later wait of the CTA returns at once and all threads keep the same sequence of barriers
+  auto wait = [&](uint64_t* bar, uint32_t phase, int where) {
+    if (*s_abort) return;
+    if (!tc::mbar_wait(bar, phase, where)) *s_abort = 1;
+  };
+  const int nblk = (a.T + 63) / 64;
+  const int nkb = a.causal ? min(nblk, q0 / 64 + 2) : nblk;
+  const uint32_t idesc_s = tc::idesc_bf16(128, 64, 0, 0), idesc_o = tc::idesc_bf16(128, a.hd, 0, 1);
+  const int nks = a.hd >> 4;
+  const uint32_t sQ = tc::smem_u32(smem + S::Q);
+  auto load_kv = [&](int j) {
+    const int sl = j & 1;
+    tc::mbar_expect_tx(&bar_k[sl], CH * BOX_BYTES);
+    split_load<CH>(smem + S::K + sl * CH * BOX_BYTES, &tm, &bar_k[sl], C + h * a.hd, j * 64, b, 1);
+    tc::mbar_expect_tx(&bar_v[sl], CH * BOX_BYTES);
+    split_load<CH>(smem + S::V + sl * CH * BOX_BYTES, &tm, &bar_v[sl], 2 * C + h * a.hd, j * 64, b, 1);
+  };
+  auto issue_s = [&](int j) {
+    wait(&bar_k[j & 1], (j >> 1) & 1, 41);
+    tc::tc_fence_after();
+    const uint32_t sK = tc::smem_u32(smem + S::K + (j & 1) * CH * BOX_BYTES);
+    if (!*s_abort)
+      for (int ks = 0; ks < nks; ks++) tc::mma_bf16_ss(t_s, desc_k(sQ, ks), desc64_k(sK, ks), idesc_s, ks > 0);
+    tc::mma_commit(bar_s);
+  };
+  if (tid == 0) {
+    tc::mbar_expect_tx(bar_q, 2 * CH * BOX_BYTES);
+    split_load<CH>(smem + S::Q, &tm, bar_q, h * a.hd, q0, b, 2);
+    load_kv(0);
+    wait(bar_q, 0, 40);
+    issue_s(0);
+  }
+  const float sl2 = a.scale * LOG2E;
+  const int qrow = q0 + tid;
+  float m = -INFINITY, l = 0.f;
+  float o[HDT];
+#pragma unroll
+  for (int i = 0; i < HDT; i++) o[i] = 0.f;
+  for (int j = 0; j < nkb; j++) {
+    if (tid == 0 && j + 1 < nkb) load_kv(j + 1);     // (block j - 1, the buffers' last reader, is complete: bar_o of it was waited for)
+    wait(bar_s, j & 1, 42);
+    __syncwarp();
+    tc::tc_fence_after();
+    uint32_t r[2][32];
+    tc::tmem_ld32(t_s + lane_addr, r[0]);
+    tc::tmem_ld32(t_s + 32 + lane_addr, r[1]);
+    tc::tmem_ld_wait();
+    const int k0 = j * 64;
+    const int last = a.causal ? min(qrow, a.T - 1) : a.T - 1;      // last key this row sees
+    if (k0 + 63 > last) {
+#pragma unroll
+      for (int i = 0; i < 64; i++)
+        if (k0 + i > last) r[i >> 5][i & 31] = 0xff800000u;
+    }
+    float mx = m;
+#pragma unroll
+    for (int i = 0; i < 32; i++) mx = max3(mx, __uint_as_float(r[0][i]) * sl2, __uint_as_float(r[1][i]) * sl2);
+    const float mu = mx == -INFINITY ? 0.f : mx;      // nothing finite seen yet: exp2(-inf - 0) = 0
+    const float alpha = ex2_approx(m - mu);
+    m = mx;
+    float rs = 0.f;
+#pragma unroll
+    for (int half = 0; half < 2; half++) {
+      uint32_t hi[16], lo[16];
+#pragma unroll
+      for (int i = 0; i < 16; i++) {
+        const float p0 = ex2_approx(fmaf(__uint_as_float(r[half][2 * i]), sl2, -mu));
+        const float p1 = ex2_approx(fmaf(__uint_as_float(r[half][2 * i + 1]), sl2, -mu));
+        rs += p0 + p1;
+        split2(p0, p1, hi[i], lo[i]);
+      }
+      tc::tmem_st16(t_s + half * 32 + lane_addr, hi);
+      tc::tmem_st16(t_s + half * 32 + 16 + lane_addr, lo);
+    }
+    l = l * alpha + rs;
+    tc::tmem_st_wait();
+    tc::tc_fence_before();
+    __syncthreads();
+    if (tid == 0) {
+      wait(&bar_v[j & 1], (j >> 1) & 1, 43);
+      tc::tc_fence_after();
+      const uint32_t sV = tc::smem_u32(smem + S::V + (j & 1) * CH * BOX_BYTES);
+      if (!*s_abort) {
+#pragma unroll
+        for (int ks = 0; ks < 4; ks++) {
+          tc::mma_bf16_ts(t_o, t_s + split_col(ks), desc64_mn(sV, ks), idesc_o, ks > 0);
+          tc::mma_bf16_ts(t_o, t_s + split_col(ks) + 16, desc64_mn(sV, ks), idesc_o, 1);
+        }
+      }
+      tc::mma_commit(bar_o);
+      if (j + 1 < nkb) issue_s(j + 1);      // MMAs of one thread run in order: these scores replace P after it has been read
+    }
+    wait(bar_o, j & 1, 44);
+    __syncwarp();
+    tc::tc_fence_after();
+#pragma unroll
+    for (int c = 0; c < HDT; c += 32) {
+      uint32_t ro[32];
+      tc::tmem_ld32(t_o + c + lane_addr, ro);
+      tc::tmem_ld_wait();
+#pragma unroll
+      for (int i = 0; i < 32; i++) o[c + i] = fmaf(o[c + i], alpha, __uint_as_float(ro[i]));
+    }
+    tc::tc_fence_before();
+  }
+  if (qrow < a.T && !*s_abort) {
+    const float inv = 1.f / l;
+    bf16* dst = a.out + ((size_t)b * a.T + qrow) * C + h * a.hd;
+#pragma unroll
+    for (int c = 0; c < HDT; c += 8) {
+      if (c < a.hd) {
+        uint4 w;
+        w.x = pack_bf16(o[c] * inv, o[c + 1] * inv); w.y = pack_bf16(o[c + 2] * inv, o[c + 3] * inv);
+        w.z = pack_bf16(o[c + 4] * inv, o[c + 5] * inv); w.w = pack_bf16(o[c + 6] * inv, o[c + 7] * inv);
+        *reinterpret_cast<uint4*>(dst + c) = w;
+      }
+    }
+    a.lse[((size_t)b * a.H + h) * a.T + qrow] = (m + log2f(l)) * LN2;
+  }
+  tc::tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tc::tmem_dealloc(t_s, TMEM_COLS);
+}
+
+// Backward, KV = true: dK and dV of a 128-key tile, streaming Q / dO;  KV = false: dQ of a 128-query tile, streaming K / V.
+// X, Y are the resident tiles (K, V or Q, dO), x, y the streamed ones (Q, dO or K, V); per block
+//   s = X x^T,  d = Y y^T  (scores, and the gradient of the probabilities; transposed in the KV form)
+//   p = exp2(s c - lse),  g = p (d - delta);    KV: dV += p dO, dK += g Q      else: dQ += g K
+template <int HDT, bool KV>
+struct SplitBwdSmem {
+  static constexpr int CH = HDT == 128 ? 2 : 1;
+  static constexpr int RX = 0;
+  static constexpr int RY = RX + 2 * CH * BOX_BYTES;
+  static constexpr int SX = RY + 2 * CH * BOX_BYTES;      // 2 buffers
+  static constexpr int SY = SX + 2 * CH * BOX_BYTES;      // 2 buffers
+  static constexpr int STAT = SY + 2 * CH * BOX_BYTES;    // 2 buffers x (lse [64], delta [64])
+  static constexpr int BAR = STAT + 1024;
+  static constexpr int TOTAL = BAR + 128 + 1024;
+};
+
+template <int HDT, bool KV>
+__global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUtensorMap tm_do,
+                                                                  const SplitArgs a) {
+  using S = SplitBwdSmem<HDT, KV>;
+  constexpr int CH = S::CH;
+  constexpr uint32_t TMEM_COLS = (KV && HDT == 128) ? 512 : 256;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint64_t* bars = (uint64_t*)(smem + S::BAR);
+  uint64_t *bar_r = bars, *bar_x = bars + 1 /*[2]*/, *bar_s = bars + 3;
+  uint32_t* tmem_slot = (uint32_t*)(bars + 4);
+  volatile int* s_abort = (volatile int*)(bars + 5);
+  float* stat = (float*)(smem + S::STAT);
+  if (attn_given_up()) return;
+
+  const int tid = threadIdx.x, warp = tid >> 5;
+  const int ntile = (a.T + 127) / 128;
+  const int tile = KV ? (int)blockIdx.x : ntile - 1 - (int)blockIdx.x, h = blockIdx.y, b = blockIdx.z;   // (causal: longest first)
+  const int r0 = tile * 128, C = a.H * a.hd, xh = h * a.hd;
+  if (tid == 0) {
+    for (int i = 0; i < 4; i++) tc::mbar_init(&bars[i], 1);
+    *s_abort = 0;
+    tc::mbar_fence_init();
+    tc::tma_prefetch_desc(&tm);
+    tc::tma_prefetch_desc(&tm_do);
+  }
+  if (warp == 0) tc::tmem_alloc(tmem_slot, TMEM_COLS);
+  tc::tc_fence_before();
+  __syncthreads();
+  tc::tc_fence_after();
+  mlb_pdl_sync();
+  const uint32_t t_s = *tmem_slot, t_d = t_s + 64, t_a0 = t_s + 128, t_a1 = t_a0 + HDT;      // a0: dV or dQ, a1: dK
+  const uint32_t lane_addr = (uint32_t)(warp * 32) << 16;
+  auto wait = [&](uint64_t* bar, uint32_t phase, int where) {
+    if (*s_abort) return;
+    if (!tc::mbar_wait(bar, phase, where)) *s_abort = 1;
+  };
+  const int nblk = (a.T + 63) / 64;
+  const int i0 = (KV && a.causal) ? r0 / 64 : 0;
+  const int n = (!KV && a.causal) ? min(nblk, r0 / 64 + 2) : nblk - i0;
+  const uint32_t idesc_s = tc::idesc_bf16(128, 64, 0, 0), idesc_g = tc::idesc_bf16(128, a.hd, 0, 1);
+  const int nks = a.hd >> 4;
+  const size_t si = ((size_t)b * a.H + h) * a.T;
+  auto load_x = [&](int it) {
+    const int sl = it & 1, y = (i0 + it) * 64;
+    tc::mbar_expect_tx(&bar_x[sl], 2 * CH * BOX_BYTES);
+    split_load<CH>(smem + S::SX + sl * CH * BOX_BYTES, &tm, &bar_x[sl], KV ? xh : C + xh, y, b, 1);
+    split_load<CH>(smem + S::SY + sl * CH * BOX_BYTES, KV ? &tm_do : &tm, &bar_x[sl], KV ? xh : 2 * C + xh, y, b, 1);
+  };
+  auto issue_scores = [&](int it) {
+    const int sl = it & 1;
+    wait(&bar_x[sl], (it >> 1) & 1, 46);
+    tc::tc_fence_after();
+    const uint32_t rx = tc::smem_u32(smem + S::RX), ry = tc::smem_u32(smem + S::RY);
+    const uint32_t sx = tc::smem_u32(smem + S::SX + sl * CH * BOX_BYTES), sy = tc::smem_u32(smem + S::SY + sl * CH * BOX_BYTES);
+    if (!*s_abort) {
+      for (int ks = 0; ks < nks; ks++) tc::mma_bf16_ss(t_s, desc_k(rx, ks), desc64_k(sx, ks), idesc_s, ks > 0);
+      for (int ks = 0; ks < nks; ks++) tc::mma_bf16_ss(t_d, desc_k(ry, ks), desc64_k(sy, ks), idesc_s, ks > 0);
+    }
+  };
+  // statistics of the 64 streamed queries (KV form); a query past the end has lse = +inf: p = 0
+  auto load_stat = [&](int it) {
+    const int q = (i0 + it) * 64 + (tid & 63);
+    float* st = stat + (it & 1) * 128;
+    if (tid < 64) st[tid] = q < a.T ? a.lse[si + q] * LOG2E : INFINITY;
+    else st[tid] = q < a.T ? a.delta[si + q] : 0.f;
+  };
+  if (tid == 0) {
+    tc::mbar_expect_tx(bar_r, 4 * CH * BOX_BYTES);
+    split_load<CH>(smem + S::RX, &tm, bar_r, KV ? C + xh : xh, r0, b, 2);
+    split_load<CH>(smem + S::RY, KV ? &tm : &tm_do, bar_r, KV ? 2 * C + xh : xh, r0, b, 2);
+    load_x(0);
+    wait(bar_r, 0, 45);
+    issue_scores(0);
+    tc::mma_commit(bar_s);
+  }
+  const float sl2 = a.scale * LOG2E;
+  const int row = r0 + tid;
+  float lse_r = INFINITY, delta_r = 0.f;      // dQ form: this thread's query
+  if (KV) {
+    load_stat(0);
+  } else if (row < a.T) {
+    lse_r = a.lse[si + row] * LOG2E;
+    delta_r = a.delta[si + row];
+  }
+  __syncthreads();
+  for (int it = 0; it < n; it++) {
+    wait(bar_s, it & 1, 47);
+    __syncwarp();
+    tc::tc_fence_after();
+    if (tid == 0 && it + 1 < n) load_x(it + 1);      // every MMA issued so far is complete: the other buffer is free
+    const int c0 = (i0 + it) * 64;
+    const float* st = stat + (it & 1) * 128;
+#pragma unroll
+    for (int half = 0; half < 2; half++) {
+      uint32_t rs[32], rd[32];
+      tc::tmem_ld32(t_s + half * 32 + lane_addr, rs);
+      tc::tmem_ld32(t_d + half * 32 + lane_addr, rd);
+      tc::tmem_ld_wait();
+      uint32_t hi[16], lo[16], gh[16], gl[16];
+#pragma unroll
+      for (int i = 0; i < 16; i++) {
+        float p[2], g[2];
+#pragma unroll
+        for (int x = 0; x < 2; x++) {
+          const int e = 2 * i + x, col = half * 32 + e;
+          const float L = KV ? st[col] : lse_r, D = KV ? st[64 + col] : delta_r;
+          float pv = ex2_approx(fmaf(__uint_as_float(rs[e]), sl2, -L));
+          // causal: the key may not lie behind the query; dQ form: keys past the end are not there (KV form: lse = +inf)
+          if (KV ? (a.causal && c0 + col < row) : ((a.causal && c0 + col > row) || c0 + col >= a.T)) pv = 0.f;
+          p[x] = pv;
+          g[x] = pv * (__uint_as_float(rd[e]) - D);
+        }
+        if (KV) split2(p[0], p[1], hi[i], lo[i]);
+        split2(g[0], g[1], gh[i], gl[i]);
+      }
+      if (KV) {
+        tc::tmem_st16(t_s + half * 32 + lane_addr, hi);
+        tc::tmem_st16(t_s + half * 32 + 16 + lane_addr, lo);
+      }
+      tc::tmem_st16(t_d + half * 32 + lane_addr, gh);
+      tc::tmem_st16(t_d + half * 32 + 16 + lane_addr, gl);
+    }
+    tc::tmem_st_wait();
+    if (KV && it + 1 < n) load_stat(it + 1);
+    tc::tc_fence_before();
+    __syncthreads();
+    if (tid == 0) {
+      tc::tc_fence_after();
+      const uint32_t sx = tc::smem_u32(smem + S::SX + (it & 1) * CH * BOX_BYTES), sy = tc::smem_u32(smem + S::SY + (it & 1) * CH * BOX_BYTES);
+      if (!*s_abort) {
+#pragma unroll
+        for (int ks = 0; ks < 4; ks++) {
+          if (KV) {
+            tc::mma_bf16_ts(t_a0, t_s + split_col(ks), desc64_mn(sy, ks), idesc_g, (it > 0 || ks > 0));
+            tc::mma_bf16_ts(t_a0, t_s + split_col(ks) + 16, desc64_mn(sy, ks), idesc_g, 1);
+          }
+          tc::mma_bf16_ts(KV ? t_a1 : t_a0, t_d + split_col(ks), desc64_mn(sx, ks), idesc_g, (it > 0 || ks > 0));
+          tc::mma_bf16_ts(KV ? t_a1 : t_a0, t_d + split_col(ks) + 16, desc64_mn(sx, ks), idesc_g, 1);
+        }
+      }
+      if (it + 1 < n) issue_scores(it + 1);      // in order behind the products that read p and g out of these columns
+      tc::mma_commit(bar_s);
+    }
+  }
+  wait(bar_s, n & 1, 48);
+  __syncwarp();
+  tc::tc_fence_after();
+  const bool live = row < a.T && !*s_abort;
+  bf16* dst = a.out + ((size_t)b * a.T + (row < a.T ? row : 0)) * 3 * C + xh;
+  if (KV) {
+    split_store_row<HDT>(dst + C, t_a1 + lane_addr, a.hd, a.scale, live);
+    split_store_row<HDT>(dst + 2 * C, t_a0 + lane_addr, a.hd, 1.f, live);
+  } else {
+    split_store_row<HDT>(dst, t_a0 + lane_addr, a.hd, a.scale, live);
+  }
+  tc::tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tc::tmem_dealloc(t_s, TMEM_COLS);
+}
+
+template <int HDT>
+static int split_fwd_launch(const CUtensorMap* tm, const SplitArgs& a, cudaStream_t st) {
+  static int once = (int)cudaFuncSetAttribute(attn_split_fwd_k<HDT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitFwdSmem<HDT>::TOTAL);
+  if (once) return once;
+  mlb_launch_tmem(attn_split_fwd_k<HDT>, dim3((a.T + 127) / 128, a.H, a.B), dim3(SPLIT_THREADS), SplitFwdSmem<HDT>::TOTAL, st, *tm, a);
+  return (int)cudaGetLastError();
+}
+template <int HDT>
+static int split_bwd_launch(const CUtensorMap* tm, const CUtensorMap* td, const SplitArgs& a, cudaStream_t st) {
+  static int once = (int)cudaFuncSetAttribute(attn_split_bwd_k<HDT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitBwdSmem<HDT, true>::TOTAL) |
+                    (int)cudaFuncSetAttribute(attn_split_bwd_k<HDT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitBwdSmem<HDT, false>::TOTAL);
+  if (once) return once;
+  const dim3 grid((a.T + 127) / 128, a.H, a.B);
+  mlb_launch_tmem(attn_split_bwd_k<HDT, true>, grid, dim3(SPLIT_THREADS), SplitBwdSmem<HDT, true>::TOTAL, st, *tm, *td, a);
+  mlb_launch_tmem(attn_split_bwd_k<HDT, false>, grid, dim3(SPLIT_THREADS), SplitBwdSmem<HDT, false>::TOTAL, st, *tm, *td, a);
+  return (int)cudaGetLastError();
+}
+
+// The shapes the kernels above take: head sizes that are multiples of the MMA's k-step, 16-byte aligned rows and heads.
+// T up to what the scalar kernels' score row in shared memory allows, so that a call is taken or refused as there.
+static bool split_ok(const void* qkv, const void* a, const void* b, int T, int hd, size_t floats_per_key) {
+  return !g_attn_force_simt && hd % 16 == 0 && hd >= 16 && hd <= 128 && (((uintptr_t)qkv | (uintptr_t)a | (uintptr_t)b) & 15) == 0 &&
+         (floats_per_key * T + 32) * sizeof(float) <= 48 * 1024;
+}
+static int split_fwd(void* out, float* lse, const void* qkv, int B, int T, int H, int hd, int causal, cudaStream_t st) {
+  const CUtensorMap* tm = mlb_tmap_seq3d_cached(qkv, B, T, 3L * H * hd);
+  if (!tm) return -2;
+  SplitArgs a{B, T, H, hd, causal, 1.0f / sqrtf((float)hd), (bf16*)out, lse, nullptr};
+  return hd <= 32 ? split_fwd_launch<32>(tm, a, st) : hd <= 64 ? split_fwd_launch<64>(tm, a, st) : split_fwd_launch<128>(tm, a, st);
+}
+// `delta` = rowsum(dO * O) is already there
+static int split_bwd(void* dqkv, const void* dout, const void* qkv, const float* lse, const float* delta, int B, int T, int H, int hd, int causal,
+                     cudaStream_t st) {
+  const CUtensorMap* tm = mlb_tmap_seq3d_cached(qkv, B, T, 3L * H * hd);
+  const CUtensorMap* td = mlb_tmap_seq3d_cached(dout, B, T, (long)H * hd);
+  if (!tm || !td) return -2;
+  SplitArgs a{B, T, H, hd, causal, 1.0f / sqrtf((float)hd), (bf16*)dqkv, const_cast<float*>(lse), delta};
+  return hd <= 32 ? split_bwd_launch<32>(tm, td, a, st) : hd <= 64 ? split_bwd_launch<64>(tm, td, a, st) : split_bwd_launch<128>(tm, td, a, st);
+}

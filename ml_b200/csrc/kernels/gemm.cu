@@ -846,6 +846,27 @@ const CUtensorMap* mlb_tmap_mn3d_cached(const void* base, uint64_t k_rows, uint6
   return m;
 }
 
+const CUtensorMap* mlb_tmap_seq3d_cached(const void* base, uint64_t seqs, uint64_t rows, uint64_t cols) {
+  EncodeTiledFn enc = get_encode();
+  if (!enc || ((uintptr_t)base & 15) || ((cols * 2) & 15)) return nullptr;
+  std::lock_guard<std::mutex> lk(g_tmap_mu);
+  TmapKey key(base, seqs, rows, cols, 64, 0xfffffffeu, -4);
+  auto it = g_tmaps.find(key);
+  if (it != g_tmaps.end()) return it->second;
+  tmap_cache_trim_locked();
+  CUtensorMap* m = new CUtensorMap;
+  cuuint64_t dims[3] = {cols, rows, seqs};
+  cuuint64_t strides[2] = {cols * 2, rows * cols * 2};
+  cuuint32_t box[3] = {64, 64, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) { delete m; return nullptr; }
+  g_tmaps[key] = m;
+  return m;
+}
+
 namespace {
 
 int g_use_3d = 1;            // tuning hook: 0 = always use 64-wide 2-D boxes for MN-major operands

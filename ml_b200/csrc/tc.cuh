@@ -335,3 +335,6 @@ const CUtensorMap* mlb_tmap_mn3d_cached(const void* base, uint64_t k_rows, uint6
 // Cached lookup (key = all arguments); the returned pointer stays valid for the life of the process.
 const CUtensorMap* mlb_tmap_cached(const void* base, uint64_t rows, uint64_t cols, uint64_t pitch_elems,
                                    uint32_t box_rows, uint32_t box_cols = 64, int elem_bytes = 2);
+// [seqs][rows][cols] bf16, contiguous, box {64 columns, 64 rows, 1 sequence}, 128-byte swizzle: rows past a sequence's end read as
+// zeros instead of the next sequence's.  Needs a 16-byte aligned base and cols a multiple of 8.
+const CUtensorMap* mlb_tmap_seq3d_cached(const void* base, uint64_t seqs, uint64_t rows, uint64_t cols);

@@ -818,3 +818,48 @@ def test_linear_dx_delta_epilogue(B, T, H, N):
     nat().attn_bwd(a, dx, qkv, out, lse, B, T, H, hd, have_delta=True)
     nat().attn_bwd(b, dx, qkv, out, lse, B, T, H, hd)
     close(a, b.float(), name="attention backward with the epilogue's delta", fro=6e-3)
+
+
+def _attn64(qkv, dout, B, T, H, hd, causal):
+    """out, lse, dqkv of plain attention in 64 bits."""
+    x = qkv.double().view(B, T, 3, H, hd).permute(2, 0, 3, 1, 4).contiguous().requires_grad_(True)
+    s = x[0] @ x[1].transpose(-1, -2) / hd ** 0.5
+    if causal:
+        s = s.masked_fill(torch.ones(T, T, dtype=torch.bool, device=s.device).triu(1), float("-inf"))
+    out = (torch.softmax(s, -1) @ x[2]).transpose(1, 2).reshape(B * T, H * hd)
+    (g,) = torch.autograd.grad(out, x, dout.double())
+    return out.detach(), torch.logsumexp(s, -1).detach(), g.permute(1, 3, 0, 2, 4).reshape(B * T, 3 * H * hd)
+
+
+def _rel(a, e):
+    return ((a.double() - e).norm() / e.norm()).item()
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("T,hd", [(1, 16), (17, 32), (63, 64), (64, 48), (65, 64), (127, 128), (128, 16), (129, 80), (197, 64), (257, 32), (321, 112)])
+def test_attention_with_split_probabilities(T, hd, causal):
+    """Edges of the 128-row tiles and 64-row blocks and every padded head size.  Results are rounded to bf16 once (at most 2^-9
+    per element), P and dS carry 2^-17; delta comes from the bf16 output, whose rounding adds up to 2^-9 of the delta term."""
+    if causal and hd in (64, 128):
+        pytest.skip("those head sizes have their own causal kernels")
+    torch.manual_seed(T * 131 + hd)
+    B, H = 2, 3
+    qkv, dout = rnd(B * T, 3 * H * hd), rnd(B * T, H * hd)
+    out, lse, dqkv = rnd(B * T, H * hd), torch.empty(B, H, T, device=dev()), torch.zeros(B * T, 3 * H * hd, device=dev(), dtype=torch.bfloat16)
+    n = nat()
+    if causal:
+        n.attn_fwd(out, lse, qkv, B, T, H, hd)
+        assert n.attn_bwd(dqkv, dout, qkv, out, lse, B, T, H, hd) is False
+    else:
+        n.attn_bidir_fwd(out, lse, qkv, B, T, H, hd)
+        n.attn_bidir_bwd(dqkv, dout, qkv, out, lse, B, T, H, hd)
+    eo, el, ed = _attn64(qkv, dout, B, T, H, hd, causal)
+    assert _rel(out, eo) < 2 ** -9 and _rel(lse, el) < 1e-6
+    if T > 1:
+        assert _rel(dqkv, ed) < 2 ** -8
+    # a sample full of infinities leaves its neighbour alone (its rows lie right behind the other's last, partial block)
+    qkv2 = qkv.clone()
+    qkv2[T:] = float("inf")
+    out2 = torch.empty_like(out)
+    (n.attn_fwd if causal else n.attn_bidir_fwd)(out2, lse, qkv2, B, T, H, hd)
+    assert torch.equal(out2[:T], out[:T])
