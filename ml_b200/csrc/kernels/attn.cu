@@ -1165,14 +1165,19 @@ __device__ __forceinline__ void store_pairs_rope(bf16* dst_row, uint32_t taddr, 
   float x0[32], x1[32];
 #pragma unroll
   for (int i = 0; i < 32; i++) { x0[i] = __uint_as_float(ra[i]) * out_scale; x1[i] = __uint_as_float(rb[i]) * out_scale; }
-  if (cosT) {
-    const float* c = cosT + (size_t)t * (HD / 2) + c0;
-    const float* s = sinT + (size_t)t * (HD / 2) + c0;
+  if (cosT) {      // 16-byte loads: every lane reads its own row of the tables, an instruction costs the L1 a line per lane whatever its width
+    const float4* c4 = reinterpret_cast<const float4*>(cosT + (size_t)t * (HD / 2) + c0);
+    const float4* s4 = reinterpret_cast<const float4*>(sinT + (size_t)t * (HD / 2) + c0);
 #pragma unroll
-    for (int i = 0; i < 32; i++) {
-      const float d0 = x0[i], d1 = x1[i], cc = c[i], ss = s[i];
-      x0[i] = d0 * cc + d1 * ss;
-      x1[i] = d1 * cc - d0 * ss;
+    for (int q = 0; q < 8; q++) {
+      const float4 cv = __ldg(c4 + q), sv = __ldg(s4 + q);
+      const float cc[4] = {cv.x, cv.y, cv.z, cv.w}, ss[4] = {sv.x, sv.y, sv.z, sv.w};
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        const float d0 = x0[q * 4 + e], d1 = x1[q * 4 + e];
+        x0[q * 4 + e] = d0 * cc[e] + d1 * ss[e];
+        x1[q * 4 + e] = d1 * cc[e] - d0 * ss[e];
+      }
     }
   }
 #pragma unroll
@@ -2103,6 +2108,7 @@ int set_smem(K kern, int bytes) {
 }
 
 #include "attn_split.cuh"
+#include "attn_hd128.cuh"
 
 bool tc_ok(const void* qkv, const void* other, int H, int hd) {
   const int C = H * hd;
@@ -2225,9 +2231,17 @@ MLB_API int mlb_attn_fwd(void* out, float* lse, const void* qkv, int B, int T, i
       (void)once;
       attn_fwd_tc_kernel<64><<<grid, ATT_THREADS, FwdSmem<64>::TOTAL, st>>>(*tm, a);
     } else {
-      static int once = set_smem(attn_fwd_tc_kernel<128>, FwdSmem<128>::TOTAL);
+      const CUtensorMap* t3 = mlb_tmap_seq3d_cached(qkv, B, T, 3L * C);
+      const CUtensorMap* to = (T % 128 == 0) ? mlb_tmap_cached(out, (uint64_t)B * T, C, C, 32, 64, 2) : nullptr;
+      if (!t3) return -2;
+      a.out_tma = to != nullptr;
+      if (!to) to = tm;      // unused by the kernel then
+      const long pairs = (long)(((T + 127) / 128 + 1) / 2) * H * B;
+      const dim3 grid2((unsigned)(pairs < sms ? pairs : sms));
+      a.sched = pairs > sms ? attn_schedule(0, B, H, T, (int)grid2.x, &a.sched_stride, st) : nullptr;
+      static int once = set_smem(attn_fwd128_k, Fwd128Smem::TOTAL);
       (void)once;
-      attn_fwd_tc_kernel<128><<<grid, ATT_THREADS, FwdSmem<128>::TOTAL, st>>>(*tm, a);
+      mlb_launch_tmem(attn_fwd128_k, grid2, dim3(FWD128_THREADS), Fwd128Smem::TOTAL, st, *t3, *to, a);
     }
     return (int)cudaGetLastError();
   }
@@ -2292,6 +2306,7 @@ static int attn_bwd_impl(void* dqkv, const void* dout, const void* qkv, const vo
   const int C = H * hd;
   const float scale = 1.0f / sqrtf((float)hd);
   if (!have_delta) attn_delta_launch(delta, dout, out, B, T, H, hd, st);
+  if (((uintptr_t)cosT | (uintptr_t)sinT) & 15) cosT = sinT = nullptr;      // the epilogues read the tables in 16-byte units; the caller rotates
   if (tc_ok(qkv, dout, H, hd) && ((uintptr_t)dqkv % 16 == 0)) {
     const CUtensorMap* tq = mlb_tmap_cached(qkv, (uint64_t)B * T, 3 * C, 3 * C, 128, 64);
     const CUtensorMap* td = mlb_tmap_cached(dout, (uint64_t)B * T, C, C, 128, 64);
@@ -2330,11 +2345,22 @@ static int attn_bwd_impl(void* dqkv, const void* dout, const void* qkv, const vo
       attn_bwd_kv_tc_kernel<64><<<grid, BWD_THREADS, BwdKVSmem<64>::TOTAL, st>>>(*tq, *td, a);
       attn_bwd_q_tc_kernel<64><<<grid, BWD_THREADS, BwdQSmem<64>::TOTAL, st>>>(*tq, *td, a);
     } else {
-      static int o1 = set_smem(attn_bwd_kv_tc_kernel<128>, BwdKVSmem<128>::TOTAL);
-      static int o2 = set_smem(attn_bwd_q_tc_kernel<128>, BwdQSmem<128>::TOTAL);
+      const CUtensorMap* t3 = mlb_tmap_seq3d_cached(qkv, B, T, 3L * C);
+      const CUtensorMap* d3 = mlb_tmap_seq3d_cached(dout, B, T, C);
+      if (!t3 || !d3) return -2;
+      static int o1 = set_smem(attn_bwd_kv128_k, BwdKV128Smem::TOTAL);
+      static int o2 = set_smem(attn_bwd_q128_k, BwdQ128Smem::TOTAL);
       (void)o1; (void)o2;
-      attn_bwd_kv_tc_kernel<128><<<grid, BWD_THREADS, BwdKVSmem<128>::TOTAL, st>>>(*tq, *td, a);
-      attn_bwd_q_tc_kernel<128><<<grid, BWD_THREADS, BwdQSmem<128>::TOTAL, st>>>(*tq, *td, a);
+      int sms = 0, devid = 0;
+      cudaGetDevice(&devid);
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, devid);
+      if (sms <= 0) sms = 148;
+      const long n_items = (long)((T + 127) / 128) * H * B;
+      const dim3 grid_p((unsigned)(n_items < sms ? n_items : sms));
+      // one table for both: item w of either kernel has the same number of blocks
+      a.sched = n_items > sms ? attn_schedule(1, B, H, T, (int)grid_p.x, &a.sched_stride, st) : nullptr;
+      mlb_launch_tmem(attn_bwd_kv128_k, grid_p, dim3(BWD128_THREADS), BwdKV128Smem::TOTAL, st, *t3, *d3, a);
+      mlb_launch_tmem(attn_bwd_q128_k, grid_p, dim3(BWD128_THREADS), BwdQ128Smem::TOTAL, st, *t3, *d3, a);
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return (int)e + 1000;

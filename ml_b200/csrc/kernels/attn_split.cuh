@@ -12,6 +12,8 @@
 // memory is spent on them and two (backward) to four (forward) CTAs share an SM: their MMAs, exponentials and loads
 // overlap across CTAs, which is why a CTA by itself is a plain sequence.  What bounds it is that sequence's latency, not a
 // unit.  64-row blocks because the encoder's sequences are short (197 tokens = 3.1 blocks of 64, 1.5 of 128).
+// The next block's scores overwrite those columns: one thread's MMAs run in order only as long as they have the same shape (head
+// size 64: all are 128 x 64 x 16); at the other sizes the products that read the columns are waited for first.
 // Sequences are the third dimension of the tensor maps: rows past a sample's end arrive as zeros, never as the next
 // sample's values (0 * inf would be NaN).
 struct SplitArgs {
@@ -25,11 +27,12 @@ struct SplitArgs {
 constexpr int SPLIT_THREADS = 128;
 constexpr int BOX_BYTES = 64 * 64 * 2;      // one TMA box: 64 rows x 64 columns, 128-byte swizzled rows
 
-// [64 x (64 * chunks)] block, chunks BOX_BYTES apart: K-major k-step of 16 columns / MN-major k-step of 16 rows.
-__device__ __forceinline__ uint64_t desc64_k(uint32_t base, int ks) {
-  return tc::smem_desc_sw128(base + (ks >> 2) * BOX_BYTES + (ks & 3) * 32, 16, 1024);
-}
-__device__ __forceinline__ uint64_t desc64_mn(uint32_t base, int ks) { return tc::smem_desc_sw128(base + ks * 2048, BOX_BYTES, 1024); }
+// Offsets to a tile's first descriptor, in its address units of 16 bytes, all known at compile time: a thread that puts descriptors
+// together from scratch issues an MMA every ~200 cycles, one that adds a constant keeps up with the tensor core (64).
+// k-step ks of 16 elements of a K-major tile whose 64-column chunks are `chunk` bytes apart; of 16 rows of an MN-major tile.
+__host__ __device__ constexpr uint64_t off_k(int ks, int chunk) { return (uint64_t)((ks >> 2) * (chunk >> 4) + (ks & 3) * 2); }
+__host__ __device__ constexpr uint64_t off_mn(int ks) { return (uint64_t)(ks * 128); }
+__device__ __forceinline__ uint64_t desc64_base_mn(uint32_t base) { return tc::smem_desc_sw128(base, BOX_BYTES, 1024); }
 // TMEM column of the hi term of k-step ks (16 rows of the 64-row block); the lo term is 16 columns further
 __device__ __forceinline__ uint32_t split_col(int ks) { return (uint32_t)((ks >> 1) * 32 + (ks & 1) * 8); }
 
@@ -123,7 +126,8 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
   const int nkb = a.causal ? min(nblk, q0 / 64 + 2) : nblk;
   const uint32_t idesc_s = tc::idesc_bf16(128, 64, 0, 0), idesc_o = tc::idesc_bf16(128, a.hd, 0, 1);
   const int nks = a.hd >> 4;
-  const uint32_t sQ = tc::smem_u32(smem + S::Q);
+  const uint64_t dQ = desc_base_k(tc::smem_u32(smem + S::Q)), dK0 = desc_base_k(tc::smem_u32(smem + S::K)),
+                 dV0 = desc64_base_mn(tc::smem_u32(smem + S::V));
   auto load_kv = [&](int j) {
     const int sl = j & 1;
     tc::mbar_expect_tx(&bar_k[sl], CH * BOX_BYTES);
@@ -134,9 +138,12 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
   auto issue_s = [&](int j) {
     wait(&bar_k[j & 1], (j >> 1) & 1, 41);
     tc::tc_fence_after();
-    const uint32_t sK = tc::smem_u32(smem + S::K + (j & 1) * CH * BOX_BYTES);
-    if (!*s_abort)
-      for (int ks = 0; ks < nks; ks++) tc::mma_bf16_ss(t_s, desc_k(sQ, ks), desc64_k(sK, ks), idesc_s, ks > 0);
+    const uint64_t dK = dK0 + (uint64_t)((j & 1) * (CH * BOX_BYTES >> 4));
+    if (!*s_abort) {
+#pragma unroll
+      for (int ks = 0; ks < HDT / 16; ks++)
+        if (ks < nks) tc::mma_bf16_ss(t_s, dQ + off_k(ks, TILE_BYTES), dK + off_k(ks, BOX_BYTES), idesc_s, ks > 0);
+    }
     tc::mma_commit(bar_s);
   };
   if (tid == 0) {
@@ -157,31 +164,39 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
     wait(bar_s, j & 1, 42);
     __syncwarp();
     tc::tc_fence_after();
-    uint32_t r[2][32];
-    tc::tmem_ld32(t_s + lane_addr, r[0]);
-    tc::tmem_ld32(t_s + 32 + lane_addr, r[1]);
-    tc::tmem_ld_wait();
     const int k0 = j * 64;
     const int last = a.causal ? min(qrow, a.T - 1) : a.T - 1;      // last key this row sees
-    if (k0 + 63 > last) {
+    // the scores are read twice, 32 at a time (once for the maximum): a row's 64 in registers on top of its HDT output columns
+    // would cost a resident CTA
+    auto load_scores = [&](int half, uint32_t (&r)[32]) {
+      tc::tmem_ld32(t_s + half * 32 + lane_addr, r);
+      tc::tmem_ld_wait();
+      if (k0 + half * 32 + 31 > last) {
 #pragma unroll
-      for (int i = 0; i < 64; i++)
-        if (k0 + i > last) r[i >> 5][i & 31] = 0xff800000u;
-    }
+        for (int i = 0; i < 32; i++)
+          if (k0 + half * 32 + i > last) r[i] = 0xff800000u;
+      }
+    };
     float mx = m;
 #pragma unroll
-    for (int i = 0; i < 32; i++) mx = max3(mx, __uint_as_float(r[0][i]) * sl2, __uint_as_float(r[1][i]) * sl2);
+    for (int half = 0; half < 2; half++) {
+      uint32_t r[32];
+      load_scores(half, r);
+#pragma unroll
+      for (int i = 0; i < 32; i += 2) mx = max3(mx, __uint_as_float(r[i]) * sl2, __uint_as_float(r[i + 1]) * sl2);
+    }
     const float mu = mx == -INFINITY ? 0.f : mx;      // nothing finite seen yet: exp2(-inf - 0) = 0
     const float alpha = ex2_approx(m - mu);
     m = mx;
     float rs = 0.f;
 #pragma unroll
     for (int half = 0; half < 2; half++) {
-      uint32_t hi[16], lo[16];
+      uint32_t r[32], hi[16], lo[16];
+      load_scores(half, r);
 #pragma unroll
       for (int i = 0; i < 16; i++) {
-        const float p0 = ex2_approx(fmaf(__uint_as_float(r[half][2 * i]), sl2, -mu));
-        const float p1 = ex2_approx(fmaf(__uint_as_float(r[half][2 * i + 1]), sl2, -mu));
+        const float p0 = ex2_approx(fmaf(__uint_as_float(r[2 * i]), sl2, -mu));
+        const float p1 = ex2_approx(fmaf(__uint_as_float(r[2 * i + 1]), sl2, -mu));
         rs += p0 + p1;
         split2(p0, p1, hi[i], lo[i]);
       }
@@ -195,16 +210,19 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
     if (tid == 0) {
       wait(&bar_v[j & 1], (j >> 1) & 1, 43);
       tc::tc_fence_after();
-      const uint32_t sV = tc::smem_u32(smem + S::V + (j & 1) * CH * BOX_BYTES);
+      const uint64_t dV = dV0 + (uint64_t)((j & 1) * (CH * BOX_BYTES >> 4));
       if (!*s_abort) {
 #pragma unroll
         for (int ks = 0; ks < 4; ks++) {
-          tc::mma_bf16_ts(t_o, t_s + split_col(ks), desc64_mn(sV, ks), idesc_o, ks > 0);
-          tc::mma_bf16_ts(t_o, t_s + split_col(ks) + 16, desc64_mn(sV, ks), idesc_o, 1);
+          tc::mma_bf16_ts(t_o, t_s + split_col(ks), dV + off_mn(ks), idesc_o, ks > 0);
+          tc::mma_bf16_ts(t_o, t_s + split_col(ks) + 16, dV + off_mn(ks), idesc_o, 1);
         }
       }
       tc::mma_commit(bar_o);
-      if (j + 1 < nkb) issue_s(j + 1);      // MMAs of one thread run in order: these scores replace P after it has been read
+      if (j + 1 < nkb) {      // these scores replace P, which the product above reads
+        if (a.hd != 64) wait(bar_o, j & 1, 44);
+        issue_s(j + 1);
+      }
     }
     wait(bar_o, j & 1, 44);
     __syncwarp();
@@ -263,9 +281,9 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = (uint64_t*)(smem + S::BAR);
-  uint64_t *bar_r = bars, *bar_x = bars + 1 /*[2]*/, *bar_s = bars + 3;
-  uint32_t* tmem_slot = (uint32_t*)(bars + 4);
-  volatile int* s_abort = (volatile int*)(bars + 5);
+  uint64_t *bar_r = bars, *bar_x = bars + 1 /*[2]*/, *bar_s = bars + 3, *bar_g = bars + 4;
+  uint32_t* tmem_slot = (uint32_t*)(bars + 5);
+  volatile int* s_abort = (volatile int*)(bars + 6);
   float* stat = (float*)(smem + S::STAT);
   if (attn_given_up()) return;
 
@@ -274,7 +292,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
   const int tile = KV ? (int)blockIdx.x : ntile - 1 - (int)blockIdx.x, h = blockIdx.y, b = blockIdx.z;   // (causal: longest first)
   const int r0 = tile * 128, C = a.H * a.hd, xh = h * a.hd;
   if (tid == 0) {
-    for (int i = 0; i < 4; i++) tc::mbar_init(&bars[i], 1);
+    for (int i = 0; i < 5; i++) tc::mbar_init(&bars[i], 1);
     *s_abort = 0;
     tc::mbar_fence_init();
     tc::tma_prefetch_desc(&tm);
@@ -297,6 +315,9 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
   const uint32_t idesc_s = tc::idesc_bf16(128, 64, 0, 0), idesc_g = tc::idesc_bf16(128, a.hd, 0, 1);
   const int nks = a.hd >> 4;
   const size_t si = ((size_t)b * a.H + h) * a.T;
+  const uint64_t drx = desc_base_k(tc::smem_u32(smem + S::RX)), dry = desc_base_k(tc::smem_u32(smem + S::RY));
+  const uint64_t dsx = desc_base_k(tc::smem_u32(smem + S::SX)), dsy = desc_base_k(tc::smem_u32(smem + S::SY));      // as B of the scores
+  const uint64_t gsx = desc64_base_mn(tc::smem_u32(smem + S::SX)), gsy = desc64_base_mn(tc::smem_u32(smem + S::SY));   // as B of the gradients
   auto load_x = [&](int it) {
     const int sl = it & 1, y = (i0 + it) * 64;
     tc::mbar_expect_tx(&bar_x[sl], 2 * CH * BOX_BYTES);
@@ -307,11 +328,14 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
     const int sl = it & 1;
     wait(&bar_x[sl], (it >> 1) & 1, 46);
     tc::tc_fence_after();
-    const uint32_t rx = tc::smem_u32(smem + S::RX), ry = tc::smem_u32(smem + S::RY);
-    const uint32_t sx = tc::smem_u32(smem + S::SX + sl * CH * BOX_BYTES), sy = tc::smem_u32(smem + S::SY + sl * CH * BOX_BYTES);
+    const uint64_t slot = (uint64_t)(sl * (CH * BOX_BYTES >> 4)), sx = dsx + slot, sy = dsy + slot;
     if (!*s_abort) {
-      for (int ks = 0; ks < nks; ks++) tc::mma_bf16_ss(t_s, desc_k(rx, ks), desc64_k(sx, ks), idesc_s, ks > 0);
-      for (int ks = 0; ks < nks; ks++) tc::mma_bf16_ss(t_d, desc_k(ry, ks), desc64_k(sy, ks), idesc_s, ks > 0);
+#pragma unroll
+      for (int ks = 0; ks < HDT / 16; ks++)
+        if (ks < nks) tc::mma_bf16_ss(t_s, drx + off_k(ks, TILE_BYTES), sx + off_k(ks, BOX_BYTES), idesc_s, ks > 0);
+#pragma unroll
+      for (int ks = 0; ks < HDT / 16; ks++)
+        if (ks < nks) tc::mma_bf16_ss(t_d, dry + off_k(ks, TILE_BYTES), sy + off_k(ks, BOX_BYTES), idesc_s, ks > 0);
     }
   };
   // statistics of the 64 streamed queries (KV form); a query past the end has lse = +inf: p = 0
@@ -383,19 +407,25 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
     __syncthreads();
     if (tid == 0) {
       tc::tc_fence_after();
-      const uint32_t sx = tc::smem_u32(smem + S::SX + (it & 1) * CH * BOX_BYTES), sy = tc::smem_u32(smem + S::SY + (it & 1) * CH * BOX_BYTES);
+      const uint64_t slot = (uint64_t)((it & 1) * (CH * BOX_BYTES >> 4)), sx = gsx + slot, sy = gsy + slot;
       if (!*s_abort) {
 #pragma unroll
         for (int ks = 0; ks < 4; ks++) {
           if (KV) {
-            tc::mma_bf16_ts(t_a0, t_s + split_col(ks), desc64_mn(sy, ks), idesc_g, (it > 0 || ks > 0));
-            tc::mma_bf16_ts(t_a0, t_s + split_col(ks) + 16, desc64_mn(sy, ks), idesc_g, 1);
+            tc::mma_bf16_ts(t_a0, t_s + split_col(ks), sy + off_mn(ks), idesc_g, (it > 0 || ks > 0));
+            tc::mma_bf16_ts(t_a0, t_s + split_col(ks) + 16, sy + off_mn(ks), idesc_g, 1);
           }
-          tc::mma_bf16_ts(KV ? t_a1 : t_a0, t_d + split_col(ks), desc64_mn(sx, ks), idesc_g, (it > 0 || ks > 0));
-          tc::mma_bf16_ts(KV ? t_a1 : t_a0, t_d + split_col(ks) + 16, desc64_mn(sx, ks), idesc_g, 1);
+          tc::mma_bf16_ts(KV ? t_a1 : t_a0, t_d + split_col(ks), sx + off_mn(ks), idesc_g, (it > 0 || ks > 0));
+          tc::mma_bf16_ts(KV ? t_a1 : t_a0, t_d + split_col(ks) + 16, sx + off_mn(ks), idesc_g, 1);
         }
       }
-      if (it + 1 < n) issue_scores(it + 1);      // in order behind the products that read p and g out of these columns
+      if (it + 1 < n) {      // these scores replace p and g, which the products above read
+        if (a.hd != 64) {
+          tc::mma_commit(bar_g);
+          wait(bar_g, it & 1, 49);
+        }
+        issue_scores(it + 1);
+      }
       tc::mma_commit(bar_s);
     }
   }

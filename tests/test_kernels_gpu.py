@@ -863,3 +863,27 @@ def test_attention_with_split_probabilities(T, hd, causal):
     out2 = torch.empty_like(out)
     (n.attn_fwd if causal else n.attn_bidir_fwd)(out2, lse, qkv2, B, T, H, hd)
     assert torch.equal(out2[:T], out[:T])
+
+
+@pytest.mark.parametrize("B,T,H", [(2, 1, 3), (2, 64, 1), (1, 128, 2), (2, 130, 3), (1, 257, 2), (2, 384, 2), (1, 640, 3), (12, 384, 16), (1, 2048, 2)])
+def test_causal_attention_head_size_128(B, T, H):
+    """One and two query tiles per pair, partial tiles, few items and more items than SMs.  P and the result are bf16 (at most 2^-9 per
+    element each): below 2^-8.  In backward dS is, and it carries the rounding of O through delta besides: twice that."""
+    torch.manual_seed(T + 7 * B)
+    hd = 128
+    qkv, dout = rnd(B * T, 3 * H * hd), rnd(B * T, H * hd)
+    out, lse, dqkv = rnd(B * T, H * hd), torch.empty(B, H, T, device=dev()), torch.zeros(B * T, 3 * H * hd, device=dev(), dtype=torch.bfloat16)
+    n = nat()
+    n.attn_fwd(out, lse, qkv, B, T, H, hd)
+    n.attn_bwd(dqkv, dout, qkv, out, lse, B, T, H, hd)
+    eo, el, ed = _attn64(qkv, dout, B, T, H, hd, True)
+    assert _rel(out, eo) < 2 ** -8 and _rel(lse, el) < 1e-6
+    assert _rel(dqkv, ed) < 2 ** -7
+    again = torch.empty_like(dqkv)
+    n.attn_bwd(again, dout, qkv, out, lse, B, T, H, hd)
+    assert torch.equal(again, dqkv)
+    # scores that grow along the keys: the running maximum is passed again and again
+    qkv.view(B, T, 3, H, hd)[:, :, 1] *= torch.linspace(0.1, 8, T, device=dev()).bfloat16().view(1, T, 1, 1)
+    n.attn_fwd(out, lse, qkv, B, T, H, hd)
+    eo, el, _ = _attn64(qkv, dout, B, T, H, hd, True)
+    assert _rel(out, eo) < 2 ** -8 and _rel(lse, el) < 1e-6
