@@ -66,7 +66,8 @@ struct GemmArgs {
   int a3d, b3d;      // MN-major operand fetched through a 3-D tensor map (one TMA per stage) instead of 64-wide 2-D boxes
   int streamk;       // pair kernel, fp32 add epilogue: every cluster (group) takes an equal contiguous share of all (tile, k-block) units
   int sk_group, sk_group_m;   // stream-K group size (tiles along the short dimension) and whether that dimension is M
-  int nt_fast;       // static schedule: consecutive work items walk N first (tiles in flight share rows of A) instead of M
+  int nt_fast;       // pair kernel: consecutive work items walk N first (tiles in flight share rows of A) instead of M
+  int sk_dp;         // stream-K: this many tiles go out whole first, one per cluster and wave; only the rest is cut up
   // optional rotary embedding in the bf16 epilogue (pair kernel): output columns [0, rope_cols) are heads of 64 columns
   // whose halves (i, i + 32) are rotated by the angle table row (output row % rope_T)
   const float* cosT;
@@ -96,14 +97,25 @@ struct GemmArgs {
 // gets at most a tail piece of one tile, whole tiles, and a head piece of another; every piece is add-reduced into the
 // fp32 output, which is what the split-K epilogue does anyway.
 struct WorkItem { int mt, nt, kb0, kb1; };
+// SPLIT: forms that may cut up the reduction (the fp32 add-reduce products); the others know nothing but whole tiles, walked
+// without a division (the issuing thread computes its next tile between two tiles' MMAs, and a tile of a short reduction is
+// only ~3000 cycles long).
+template <bool SPLIT>
 struct WorkIter {
   int t, step, total, tiles_m, tiles_n, kb_per_split, kb_total;
-  int member, G, grouped_m;     // stream-K: this cluster's tile index along the grouped dimension
+  int fast, slow, dfast, dslow, nfast;   // tile t's coordinates along the dimension walked first and the other, their steps, extent of the first
+  int member, G, grouped_m, dp;          // stream-K: this cluster's tile index along the grouped dimension; tiles handed out whole
   long u, u1;
   bool sk, nt_fast;
   __device__ WorkIter(const GemmArgs& g, int cid, int ncl)
-      : t(cid), step(ncl), total(g.tiles_m * g.tiles_n * g.splits), tiles_m(g.tiles_m), tiles_n(g.tiles_n),
-        kb_per_split(g.kb_per_split), kb_total(g.kb_total), sk(g.streamk != 0), nt_fast(g.nt_fast != 0) {
+      : t(cid), step(ncl), total(g.tiles_m * g.tiles_n), tiles_m(g.tiles_m), tiles_n(g.tiles_n), kb_total(g.kb_total), nt_fast(g.nt_fast != 0) {
+    nfast = nt_fast ? tiles_n : tiles_m;
+    slow = cid / nfast; fast = cid - slow * nfast;
+    dslow = ncl / nfast; dfast = ncl - dslow * nfast;
+    if (!SPLIT) return;
+    kb_per_split = g.kb_per_split;
+    dp = g.sk_dp;
+    sk = g.streamk != 0;
     // Stream-K in groups: the G tiles that share the wide operand (same index along the long dimension) are given to G
     // neighbouring clusters with IDENTICAL (long-dimension tile, k-block) ranges, so that operand is fetched from DRAM
     // once and found in L2 by the other members; the narrow operand is small enough to live in L2.
@@ -111,7 +123,7 @@ struct WorkIter {
     grouped_m = g.sk_group_m;
     const int ngroups = ncl / G, grp = cid / G;
     member = cid % G;
-    const int long_tiles = G == 1 ? g.tiles_m * g.tiles_n : (grouped_m ? g.tiles_n : g.tiles_m);   // G == 1: every tile on its own
+    const int long_tiles = G == 1 ? tiles_m * tiles_n - dp : (grouped_m ? g.tiles_n : g.tiles_m);   // G == 1: every tile on its own
     const long units = (long)long_tiles * g.kb_total;
     if (sk && grp < ngroups) {
       u = units * grp / ngroups;
@@ -119,25 +131,38 @@ struct WorkIter {
     } else {
       u = u1 = 0;
     }
+    total = sk ? dp : total * g.splits;      // (whole tiles first)
+  }
+  __device__ void place(WorkItem& w, int f, int s) const {
+    w.mt = nt_fast ? s : f;
+    w.nt = nt_fast ? f : s;
   }
   __device__ bool next(WorkItem& w) {
-    if (sk) {
-      if (u >= u1) return false;
-      const int lt = (int)(u / kb_total);
-      w.kb0 = (int)(u % kb_total);
-      w.kb1 = (int)min((long)kb_total, w.kb0 + (u1 - u));
-      if (G == 1) { w.mt = lt % tiles_m; w.nt = lt / tiles_m; }
-      else if (grouped_m) { w.mt = member; w.nt = lt; }
-      else { w.mt = lt; w.nt = member; }
-      u += w.kb1 - w.kb0;
+    if (t < total) {
+      w.kb0 = 0;
+      w.kb1 = kb_total;
+      if (SPLIT && !sk) {
+        const int tiles = tiles_m * tiles_n, sp = t / tiles, i = t - sp * tiles;
+        place(w, i % nfast, i / nfast);
+        w.kb0 = sp * kb_per_split;
+        w.kb1 = min(w.kb0 + kb_per_split, kb_total);
+      } else {
+        place(w, fast, slow);
+        fast += dfast;
+        slow += dslow;
+        if (fast >= nfast) { fast -= nfast; slow++; }
+      }
+      t += step;
       return true;
     }
-    if (t >= total) return false;
-    const int sp = t / (tiles_m * tiles_n);
-    if (nt_fast) { w.nt = t % tiles_n; w.mt = (t / tiles_n) % tiles_m; }
-    else { w.mt = t % tiles_m; w.nt = (t / tiles_m) % tiles_n; }
-    w.kb0 = sp * kb_per_split; w.kb1 = min(w.kb0 + kb_per_split, kb_total);
-    t += step;
+    if (!SPLIT || u >= u1) return false;
+    const int lt = (int)(u / kb_total);
+    w.kb0 = (int)(u % kb_total);
+    w.kb1 = (int)min((long)kb_total, w.kb0 + (u1 - u));
+    if (G == 1) place(w, (dp + lt) % nfast, (dp + lt) / nfast);
+    else if (grouped_m) { w.mt = member; w.nt = lt; }
+    else { w.mt = lt; w.nt = member; }
+    u += w.kb1 - w.kb0;
     return true;
   }
 };
@@ -470,7 +495,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     if (tc::elect_one()) {
       int stage = 0, phase = 0;
       bool ok = true;
-      WorkIter iter(g, cid, ncl);
+      WorkIter<EPI == EPI_F32_ADD> iter(g, cid, ncl);
       WorkItem w;
       while (ok && iter.next(w)) {
         const int m0 = w.mt * PM + (int)rank * 128;
@@ -506,7 +531,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       constexpr uint32_t idesc = F8 ? tc::idesc_e4m3(PM, BN) : tc::idesc_bf16(PM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
       int stage = 0, phase = 0, it = 0;
       bool ok = true;
-      WorkIter iter(g, cid, ncl);
+      WorkIter<EPI == EPI_F32_ADD> iter(g, cid, ncl);
       WorkItem w;
       for (; ok && iter.next(w); it++) {
         const int kb0 = w.kb0, kb1 = w.kb1;
@@ -541,7 +566,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     constexpr int ELEM = (EPI == EPI_BF16) ? 2 : 4;
     int it = 0, slab = 0;
     bool ok = true;
-    WorkIter iter(g, cid, ncl);
+    WorkIter<EPI == EPI_F32_ADD> iter(g, cid, ncl);
     WorkItem w;
     for (; ok && iter.next(w); it++) {
       const int m0 = w.mt * PM + (int)rank * 128 + lg * 32, n0 = w.nt * BN + half * 128;
@@ -869,6 +894,7 @@ const CUtensorMap* mlb_tmap_seq3d_cached(const void* base, uint64_t seqs, uint64
 
 namespace {
 
+int g_sk_whole = 1;          // tuning hook: 0 = stream-K cuts up all tiles, not only those of the last, partial wave
 int g_use_3d = 1;            // tuning hook: 0 = always use 64-wide 2-D boxes for MN-major operands
 int g_num_sms = 0;
 int num_sms() {
@@ -1041,12 +1067,22 @@ int gemm_dispatch_impl(void* out, int ldo, const bf16* A, int lda, const bf16* B
   g.a3d = g.b3d = 0;
   g.streamk = (pairs && EPI == EPI_F32_ADD && g_streamk && g_force_splits == 0) ? 1 : 0;
   // Tiles in flight should share the operand that does not fit in L2: walk N first when A is the larger one.
-  g.nt_fast = (g_tile_order == 2) ? 1 : (g_tile_order == 1 ? 0 : ((long)M > (long)N ? 1 : 0));
+  g.nt_fast = (g_tile_order == 2 || (g_tile_order != 1 && M > N)) ? 1 : 0;
+  g.sk_dp = 0;
   g.sk_group = 1; g.sk_group_m = 0;
   if (g.streamk) {
     // group along the dimension with fewer tiles (its operand is the narrow one); at most 4 members, else plain stream-K
     const int short_tiles = g.tiles_m < g.tiles_n ? g.tiles_m : g.tiles_n;
     if (g_sk_groups && short_tiles <= 4 && short_tiles >= 1 && pair_clusters() >= 4 * short_tiles) { g.sk_group = short_tiles; g.sk_group_m = g.tiles_m < g.tiles_n ? 1 : 0; }
+  }
+  if (g.streamk) {
+    // Whole waves of tiles first, only the tiles of the last, partial wave cut up: with every tile cut, the clusters sit at 74 different
+    // depths of the reduction and no two of them want the same slice of the operands at the same time (dW of 11008 x 2048 over
+    // 16384 rows: 554 us cut up throughout, 459 us this way; 2048 x 5504: 366 and 284 us).  Short reductions (less than 32
+    // k-blocks) have no time to drift apart, and their tail pieces would be mostly epilogue.
+    const int tiles = g.tiles_m * g.tiles_n, pc = pair_clusters();
+    if (g_sk_whole && g.sk_group == 1 && tiles >= pc && g.kb_total >= 32) g.sk_dp = tiles / pc * pc;
+    else g.nt_fast = 0;
   }
   const CUtensorMap* tmA = nullptr;
   const CUtensorMap* tmB = nullptr;
@@ -1167,7 +1203,8 @@ int gemm_fp8_dispatch(void* out, int ldo, const uint8_t* A, int lda, const uint8
   g.tiles_n = swi ? swi->I / 128 : ceil_div_i(N, 256);
   g.kb_total = ceil_div_i(K, 128);
   g.splits = 1; g.kb_per_split = g.kb_total; g.a3d = g.b3d = 0; g.streamk = 0; g.sk_group = 1; g.sk_group_m = 0;
-  g.nt_fast = (g_tile_order == 2) ? 1 : (g_tile_order == 1 ? 0 : ((long)M > (long)N ? 1 : 0));
+  g.nt_fast = (g_tile_order == 2 || (g_tile_order != 1 && M > N)) ? 1 : 0;
+  g.sk_dp = 0;
   const CUtensorMap* tmA = mlb_tmap_cached(A, M, K, lda, 128, 128, 1);
   const CUtensorMap* tmB = mlb_tmap_cached(B, N, K, ldb, 128, 128, 1);
   const CUtensorMap* tmD = mlb_tmap_cached(out, M, N, ldo, 32, 64, 2);
@@ -1298,7 +1335,8 @@ MLB_API int mlb_linear_fwd_gather(void* out, const void* x, int M, int N, int K,
   GemmArgs g;
   g.out = out; g.M = M; g.N = N; g.K = K; g.ldo = ldo;
   g.tiles_m = ceil_div_i(M, BM); g.tiles_n = ceil_div_i(N, BN); g.kb_total = ceil_div_i(K, BK);
-  g.splits = 1; g.kb_per_split = g.kb_total; g.a3d = g.b3d = 0; g.streamk = 0; g.sk_group = 1; g.sk_group_m = 0; g.nt_fast = 0;
+  g.nt_fast = 0; g.sk_dp = 0;
+  g.splits = 1; g.kb_per_split = g.kb_total; g.a3d = g.b3d = 0; g.streamk = 0; g.sk_group = 1; g.sk_group_m = 0;
   g.cosT = g.sinT = nullptr; g.rope_T = 1; g.rope_cols = 0; g.sw_out = nullptr; g.sw_I = 0; g.out_scale = 1.f; g.pos = nullptr; g.pos_period = 1; g.dl_o = nullptr; g.dl_out = nullptr; g.dl_T = 1; g.dl_H = 1;
   GatherArgs ga;
   ga.src = (const uint4* const*)src_ptrs; ga.dst = (uint4*)unit_dst; ga.shard_vec = shard_elems / 8;
@@ -1397,3 +1435,4 @@ MLB_API void mlb_gemm_tile_order(int mode) { g_tile_order = mode; }
 MLB_API void mlb_gemm_streamk_groups(int on) { g_sk_groups = on; }
 
 MLB_DEFINE_ERROR_WORD(gemm)
+MLB_API void mlb_gemm_streamk_whole(int on) { g_sk_whole = on; }
