@@ -566,21 +566,24 @@ __device__ __forceinline__ float exp2f_fast(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__global__ void __launch_bounds__(512, 4) ce_fwd_bwd_k(float* __restrict__ losses, bf16* __restrict__ logits,
-                                                    const int* __restrict__ tgt, int V, long ld, float dscale) {
+__global__ void __launch_bounds__(512, 4) ce_fwd_bwd_k(float* __restrict__ losses, bf16* dlogits, const bf16* logits,
+                                                    const int* __restrict__ tgt, int V, long ld, float dscale,
+                                                    const float* __restrict__ dscale_dev) {
   mlb_pdl_sync();
   __shared__ float red[32];
   const long row = blockIdx.x;
-  bf16* z = logits + row * ld;
+  const bf16* z = logits + row * ld;
+  bf16* dz = dlogits + row * ld;
+  const bool grad = dlogits != nullptr;
   const int t = tgt[row];
   const bool vec = ((V & 7) == 0) && ((ld & 7) == 0);
   if (t >= V && threadIdx.x == 0) mlb_set_error(MLB_ERR_BOUNDS, 0xCE);      // treated like an ignored row
   if (t < 0 || t >= V) {
     if (threadIdx.x == 0) losses[row] = 0.f;
-    if (vec) {
-      for (int i = threadIdx.x * 8; i < V; i += blockDim.x * 8) *reinterpret_cast<uint4*>(z + i) = make_uint4(0, 0, 0, 0);
-    } else {
-      for (int i = threadIdx.x; i < V; i += blockDim.x) z[i] = __float2bfloat16(0.f);
+    if (grad && vec) {
+      for (int i = threadIdx.x * 8; i < V; i += blockDim.x * 8) *reinterpret_cast<uint4*>(dz + i) = make_uint4(0, 0, 0, 0);
+    } else if (grad) {
+      for (int i = threadIdx.x; i < V; i += blockDim.x) dz[i] = __float2bfloat16(0.f);
     }
     return;
   }
@@ -618,6 +621,8 @@ __global__ void __launch_bounds__(512, 4) ce_fwd_bwd_k(float* __restrict__ losse
   const float zt = __bfloat162float(z[t]);
   __syncthreads();  // everyone has read z[t] before anyone overwrites it
   if (threadIdx.x == 0) losses[row] = __logf(S) + M - zt;
+  if (!grad) return;
+  if (dscale_dev) dscale = *dscale_dev;
   const float inv = dscale / S;
   if (vec) {
     const int step = blockDim.x * 8;
@@ -632,17 +637,17 @@ __global__ void __launch_bounds__(512, 4) ce_fwd_bwd_k(float* __restrict__ losse
       unpack8(rb, xb);
 #pragma unroll
       for (int j = 0; j < 8; j++) xa[j] = exp2f_fast(fmaf(xa[j], L2E, nM)) * inv - ((i + j == t) ? dscale : 0.f);
-      store8(z + i, xa);
+      store8(dz + i, xa);
       if (two) {
 #pragma unroll
         for (int j = 0; j < 8; j++) xb[j] = exp2f_fast(fmaf(xb[j], L2E, nM)) * inv - ((i + step + j == t) ? dscale : 0.f);
-        store8(z + i + step, xb);
+        store8(dz + i + step, xb);
       }
     }
   } else {
     for (int i = threadIdx.x; i < V; i += blockDim.x) {
       float x = __bfloat162float(z[i]);
-      z[i] = __float2bfloat16(__expf(x - M) * inv - ((i == t) ? dscale : 0.f));
+      dz[i] = __float2bfloat16(__expf(x - M) * inv - ((i == t) ? dscale : 0.f));
     }
   }
 }
@@ -907,6 +912,55 @@ __global__ void __launch_bounds__(1024) sum_scale_k(float* __restrict__ out, con
   s = block_sum(s, red);
   if (threadIdx.x == 0) out[0] = s * scale;
 }
+// stats[0] = 1 / max(n, 1) with n = targets >= 0, stats[1] = max(n, 1) (as an integer): one block, the targets are a few 10 KB
+__global__ void __launch_bounds__(1024) ce_count_k(float* __restrict__ stats, const int* __restrict__ tgt, long rows) {
+  __shared__ int red[32];
+  int c = 0;
+  for (long i = threadIdx.x; i < rows; i += 1024) c += tgt[i] >= 0;
+  c = __reduce_add_sync(0xffffffffu, c);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = c;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    c = max(__reduce_add_sync(0xffffffffu, red[threadIdx.x]), 1);
+    if (threadIdx.x == 0) { stats[0] = (float)(1.0 / (double)c); stats[1] = __int_as_float(c); }
+  }
+}
+// out[0] = sum(x) / n, summed in double in a fixed order
+__global__ void __launch_bounds__(1024) sum_mean_k(float* __restrict__ out, const float* __restrict__ x, const float* __restrict__ stats, long rows) {
+  __shared__ double red[32];
+  double s = 0.0;
+  for (long i = threadIdx.x; i < rows; i += 1024) s += (double)x[i];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    s = red[threadIdx.x];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (threadIdx.x == 0) out[0] = (float)(s / (double)__float_as_int(stats[1]));
+  }
+}
+// out = x * s[0] in bf16 (fp32 product, one rounding), s in device memory: the gradient of the logits times the gradient of the
+// loss.  Two 16-byte loads in flight per thread; bound by the read and the write (1.65 GB each way at 16384 x 50304).
+__global__ void __launch_bounds__(256) scale_dev_k(bf16* __restrict__ out, const bf16* __restrict__ x, const float* __restrict__ s, long n) {
+  mlb_pdl_sync();
+  const float f = *s;
+  const long i = ((long)blockIdx.x * 512 + threadIdx.x) * 8, i2 = i + 256 * 8;
+  if (i2 + 7 < n) {
+    const uint4 ra = __ldcs(reinterpret_cast<const uint4*>(x + i)), rb = __ldcs(reinterpret_cast<const uint4*>(x + i2));
+    float a[8], b[8];
+    unpack8(ra, a);
+    unpack8(rb, b);
+#pragma unroll
+    for (int j = 0; j < 8; j++) { a[j] *= f; b[j] *= f; }
+    store8(out + i, a);
+    store8(out + i2, b);
+    return;
+  }
+  for (int h = 0; h < 2; h++)
+    for (long e = h ? i2 : i, end = e + 8; e < end && e < n; e++) out[e] = __float2bfloat16(__bfloat162float(x[e]) * f);
+}
 __global__ void cast_b2f_k(float* __restrict__ out, const bf16* __restrict__ in, long n, float scale) {
   long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) out[i] = __bfloat162float(in[i]) * scale;
@@ -1138,7 +1192,24 @@ MLB_API int mlb_ce_fwd_bwd(float* losses, void* logits, const int* tgt, long row
     mlb_launch(ce_fwd_bwd_smem_k, dim3((unsigned)rows), dim3(512), sh, st, losses, (bf16*)logits, tgt, V, ld, dscale);
     LAUNCH_RET;
   }
-  mlb_launch(ce_fwd_bwd_k, dim3((unsigned)rows), dim3(threads), 0, st, losses, (bf16*)logits, tgt, V, ld, dscale);
+  mlb_launch(ce_fwd_bwd_k, dim3((unsigned)rows), dim3(threads), 0, st, losses, (bf16*)logits, (const bf16*)logits, tgt, V, ld, dscale, (const float*)nullptr);
+  LAUNCH_RET;
+}
+// Mean cross-entropy over the rows with a target, out of place and without a word of it on the host: stats[0] = 1 / rows with a
+// target (at least 1), losses per row, dlogits (may be null: losses only) = d loss / d logits, loss[0] = the mean.
+MLB_API int mlb_ce_mean(float* loss, float* losses, float* stats, void* dlogits, const void* logits, const int* tgt, long rows, int V, cudaStream_t st) {
+  // (without this check a vector access could be misaligned: the in-place entry's callers own their buffers, this one's may pass views)
+  if ((((uintptr_t)dlogits | (uintptr_t)logits) & 15) && V % 8 == 0) return -7;
+  if (rows > 0) {
+    ce_count_k<<<1, 1024, 0, st>>>(stats, tgt, rows);
+    mlb_launch(ce_fwd_bwd_k, dim3((unsigned)rows), dim3(512), 0, st, losses, (bf16*)dlogits, (const bf16*)logits, tgt, V, (long)V, 0.f, (const float*)stats);
+    sum_mean_k<<<1, 1024, 0, st>>>(loss, losses, stats, rows);
+  }
+  LAUNCH_RET;
+}
+MLB_API int mlb_scale_dev(void* out, const void* x, const float* s, long n, cudaStream_t st) {
+  if (((uintptr_t)out | (uintptr_t)x) & 15) return -7;
+  if (n > 0) mlb_launch(scale_dev_k, dim3((unsigned)((n + 4095) / 4096)), dim3(256), 0, st, (bf16*)out, (const bf16*)x, s, n);
   LAUNCH_RET;
 }
 MLB_API int mlb_ce_chunk_stats(float* rowmax, float* rowsum, float* tgt_logit, const void* chunk, const int* tgt, long rows, int n,

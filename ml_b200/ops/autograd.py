@@ -146,21 +146,25 @@ class LayerNorm(torch.autograd.Function):
 
 
 class CrossEntropy(torch.autograd.Function):
-    """Mean loss over rows with tgt >= 0; the logits buffer is consumed (overwritten by its gradient)."""
+    """Mean loss over rows with tgt >= 0.  The gradient is computed here, in the same kernel, when it will be asked for."""
 
     @staticmethod
     def forward(ctx, logits, tgt):
-        valid = int((tgt >= 0).sum().item())
+        logits = logits.contiguous()
         losses = _like(logits, logits.shape[0], dtype=torch.float32)
-        work = logits.contiguous().clone()
-        ops.ce_fwd_bwd(losses, work, tgt, 1.0 / max(valid, 1))
-        ctx.save_for_backward(work)
-        return losses.sum() / max(valid, 1)
+        loss = _like(logits, (), dtype=torch.float32)
+        grad = _like(logits, *logits.shape) if ctx.needs_input_grad[0] else None
+        ops.ce_mean(loss, losses, grad, logits, tgt)
+        if grad is not None:
+            ctx.save_for_backward(grad)
+        return loss
 
     @staticmethod
     def backward(ctx, g):
         (dlogits,) = ctx.saved_tensors
-        return dlogits * g.to(dlogits.dtype), None
+        out = _like(dlogits, *dlogits.shape)
+        ops.scale_dev(out, dlogits, g.float().contiguous())
+        return out, None
 
 
 class Embedding(torch.autograd.Function):

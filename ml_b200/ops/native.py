@@ -59,6 +59,8 @@ def lib():
         "mlb_swiglu_fwd": [_vp, _vp, _i64, _i32, _vp],
         "mlb_swiglu_bwd": [_vp, _vp, _vp, _i64, _i32, _vp],
         "mlb_ce_fwd_bwd": [_vp, _vp, _vp, _i64, _i32, _i64, _f32, _i32, _vp],
+        "mlb_ce_mean": [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i32, _vp],
+        "mlb_scale_dev": [_vp, _vp, _vp, _i64, _vp],
         "mlb_fp8_qdq": [_vp, _vp, _i64, _f32, _vp],
         "mlb_ce_chunk_stats": [_vp, _vp, _vp, _vp, _vp, _i64, _i32, _i64, _i32, _vp],
         "mlb_ce_chunk_grad": [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i32, _i64, _i32, _f32, _vp],
@@ -454,6 +456,23 @@ def ce_fwd_bwd(losses, logits, tgt, dscale, V_valid=None, threads=512):
     rows, V = logits.shape
     _chk(lib().mlb_ce_fwd_bwd(_f(losses), _b(logits), _i(tgt), rows, V if V_valid is None else V_valid, logits.stride(0),
                               dscale, threads, _st()), "ce_fwd_bwd")
+
+
+def ce_mean(loss, losses, dlogits, logits, tgt):
+    rows, V = logits.shape
+    if rows == 0:
+        return loss.zero_()
+    stats = torch.empty(2, dtype=torch.float32, device=logits.device)
+    d = _b(dlogits) if dlogits is not None else None
+    rc = lib().mlb_ce_mean(_f(loss), _f(losses), _f(stats), d, _b(logits), _i(tgt), rows, V, _st())
+    if rc == -7:      # misaligned rows: through an aligned copy
+        work = logits.clone() if dlogits is None else dlogits.copy_(logits)
+        rc = lib().mlb_ce_mean(_f(loss), _f(losses), _f(stats), work.data_ptr() if d else None, work.data_ptr(), _i(tgt), rows, V, _st())
+    _chk(rc, "ce_mean")
+
+
+def scale_dev(out, x, s):
+    _chk(lib().mlb_scale_dev(_b(out), _b(x), _f(s), out.numel(), _st()), "scale_dev")
 
 
 def ce_chunk_stats(rowmax, rowsum, tgt_logit, chunk, tgt, off):

@@ -255,6 +255,22 @@ def ce_fwd_bwd(losses, logits, tgt, dscale, V_valid=None):
     logits.copy_(p)
 
 
+def ce_mean(loss, losses, dlogits, logits, tgt):
+    """Mean cross-entropy over the rows with tgt >= 0 (at least one is counted): loss (0-d) and losses[rows]; dlogits, if not
+    None, receives the gradient of the mean.  The logits are left alone."""
+    valid = max(int((tgt >= 0).sum().item()), 1)
+    work = logits.clone() if dlogits is None else dlogits
+    if dlogits is not None:
+        work.copy_(logits)
+    ce_fwd_bwd(losses, work, tgt, 1.0 / valid)
+    loss.copy_(losses.sum() / valid)
+
+
+def scale_dev(out, x, s):
+    """out = x * s with s a one-element fp32 tensor."""
+    out.copy_(_f(x) * s)
+
+
 def ce_chunk_stats(rowmax, rowsum, tgt_logit, chunk, tgt, off):
     """Folds columns off .. off+n of the vocabulary (chunk[rows, n]) into the running per-row maximum, sum of
     exp(z - max) and target logit (train/gpt_kernels.cuh:1244-1277).  Rows with tgt < 0 are left alone."""

@@ -887,3 +887,30 @@ def test_causal_attention_head_size_128(B, T, H):
     n.attn_fwd(out, lse, qkv, B, T, H, hd)
     eo, el, _ = _attn64(qkv, dout, B, T, H, hd, True)
     assert _rel(out, eo) < 2 ** -8 and _rel(lse, el) < 1e-6
+
+
+@pytest.mark.parametrize("rows,V", [(1, 8), (5, 1001), (300, 512), (33, 50304)])
+def test_ce_mean_and_scale(rows, V):
+    torch.manual_seed(rows)
+    logits = rnd(rows, V, scale=2.0)
+    keep = logits.clone()
+    tgt = torch.randint(0, V, (rows,), device=dev(), dtype=torch.int32)
+    if rows > 2:
+        tgt[1] = -1
+    loss, losses, d = torch.empty((), device=dev()), torch.empty(rows, device=dev()), torch.empty_like(logits)
+    nat().ce_mean(loss, losses, d, logits, tgt)
+    assert torch.equal(logits, keep)
+    z = logits.double().requires_grad_(True)
+    e = torch.nn.functional.cross_entropy(z, tgt.long(), ignore_index=-1)
+    (g,) = torch.autograd.grad(e, z)
+    assert abs(loss.item() - e.item()) < 1e-5 * max(1.0, e.item())
+    assert _rel(d, g) < 2 ** -8
+    l2 = torch.empty_like(loss)
+    nat().ce_mean(l2, losses, None, logits, tgt)
+    assert torch.equal(l2, loss)
+    s = torch.tensor(0.37, device=dev())
+    nat().scale_dev(logits, d, s)
+    assert torch.equal(logits, (d.float() * s).bfloat16())
+    view = rnd(rows * V + 1, 1)[1:].view(rows, V)      # rows that start two bytes off a 16-byte boundary
+    nat().ce_mean(loss, losses, d, view, tgt)
+    assert abs(loss.item() - torch.nn.functional.cross_entropy(view.double(), tgt.long(), ignore_index=-1).item()) < 1e-4
