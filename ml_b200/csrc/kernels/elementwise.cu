@@ -468,6 +468,65 @@ __global__ void rope_k(bf16* __restrict__ qkv, const float* __restrict__ cosT, c
   store8(p0, o0);
   store8(p1, o1);
 }
+// Out of place, and from grouped heads: src rows are [H query | Hkv key | Hkv value] heads, dst rows [H | H | H] with Q and K rotated
+// and every key / value head repeated for its H / Hkv query heads (Hkv = H: a plain copy of V).  One read and one write of the
+// tensors, which is what bounds it (qkv[16384, 6144]: 402 MB); copying first and rotating in place moves 670 MB, expanding the heads
+// with copies more.  32-bit index arithmetic (the host checks the range); a thread takes 8 rotation pairs of one
+// dst head, or the same two 16-byte units of V.
+__global__ void __launch_bounds__(256) rope_copy_k(bf16* __restrict__ dst, const bf16* __restrict__ src, const float* __restrict__ cosT,
+                                                   const float* __restrict__ sinT, unsigned total, int T, int H, int Hkv, int hd) {
+  mlb_pdl_sync();
+  const unsigned idx = blockIdx.x * 256u + threadIdx.x;
+  if (idx >= total) return;
+  const unsigned h2 = (unsigned)hd >> 1, vph = h2 >> 3, per_row = 3u * H * vph, rep = (unsigned)(H / Hkv);
+  const unsigned row = idx / per_row, r = idx % per_row, head = r / vph, v = r % vph;      // head of [Q | K | V]
+  const unsigned sh = head < (unsigned)H ? head : head < 2u * H ? H + (head - H) / rep : H + Hkv + (head - 2u * H) / rep;
+  const bf16* s0 = src + (size_t)row * ((unsigned)(H + 2 * Hkv) * hd) + sh * hd + v * 8;
+  bf16* d0 = dst + (size_t)row * (3u * H * hd) + head * hd + v * 8;
+  const uint4 ra = __ldg(reinterpret_cast<const uint4*>(s0)), rb = __ldg(reinterpret_cast<const uint4*>(s0 + h2));
+  if (head >= 2u * H) {
+    *reinterpret_cast<uint4*>(d0) = ra;
+    *reinterpret_cast<uint4*>(d0 + h2) = rb;
+    return;
+  }
+  float a[8], b[8], c[8], s[8], o0[8], o1[8];
+  unpack8(ra, a);
+  unpack8(rb, b);
+  const size_t te = (size_t)(row % (unsigned)T) * h2 + v * 8;
+  *reinterpret_cast<float4*>(c) = *reinterpret_cast<const float4*>(cosT + te); *reinterpret_cast<float4*>(c + 4) = *reinterpret_cast<const float4*>(cosT + te + 4);
+  *reinterpret_cast<float4*>(s) = *reinterpret_cast<const float4*>(sinT + te); *reinterpret_cast<float4*>(s + 4) = *reinterpret_cast<const float4*>(sinT + te + 4);
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    o0[j] = a[j] * c[j] - b[j] * s[j];
+    o1[j] = b[j] * c[j] + a[j] * s[j];
+  }
+  store8(d0, o0);
+  store8(d0 + h2, o1);
+}
+// Its backward for grouped heads (behind the attention backward, which has undone the rotation): Q copied, the gradients of the
+// H / Hkv copies of a key / value head added in fp32 and rounded once.
+__global__ void __launch_bounds__(256) kv_group_sum_k(bf16* __restrict__ dst, const bf16* __restrict__ src, unsigned total, int H, int Hkv, int hd) {
+  mlb_pdl_sync();
+  const unsigned idx = blockIdx.x * 256u + threadIdx.x;
+  if (idx >= total) return;
+  const unsigned vph = (unsigned)hd >> 3, heads = (unsigned)(H + 2 * Hkv), rep = (unsigned)(H / Hkv);
+  const unsigned row = idx / (heads * vph), r = idx % (heads * vph), head = r / vph, v = r % vph;
+  const bf16* s0 = src + (size_t)row * (3u * H * hd) + v * 8;
+  bf16* d0 = dst + (size_t)row * (heads * hd) + head * hd + v * 8;
+  if (head < (unsigned)H) {
+    *reinterpret_cast<uint4*>(d0) = *reinterpret_cast<const uint4*>(s0 + head * hd);
+    return;
+  }
+  const unsigned first = head < (unsigned)(H + Hkv) ? H + (head - H) * rep : 2u * H + (head - H - Hkv) * rep;
+  float acc[8] = {};
+  for (unsigned i = 0; i < rep; i++) {
+    float x[8];
+    load8(s0 + (size_t)(first + i) * hd, x);
+#pragma unroll
+    for (int j = 0; j < 8; j++) acc[j] += x[j];
+  }
+  store8(d0, acc);
+}
 __global__ void rope_scalar_k(bf16* __restrict__ qkv, const float* __restrict__ cosT, const float* __restrict__ sinT, long rows,
                               int T, int H, int hd, float sign) {
   const int h2 = hd >> 1;
@@ -1167,6 +1226,20 @@ MLB_API int mlb_rope(void* qkv, const float* cosT, const float* sinT, long rows,
     long n = rows * 2L * H * h2;
     rope_scalar_k<<<gs(n, 256), 256, 0, st>>>((bf16*)qkv, cosT, sinT, rows, T, H, hd, sign);
   }
+  LAUNCH_RET;
+}
+// -7: the shape or alignment does not take these kernels (nothing was launched)
+MLB_API int mlb_rope_copy(void* dst, const void* src, const float* cosT, const float* sinT, long rows, int T, int H, int Hkv, int hd,
+                          cudaStream_t st) {
+  const long n = rows * 3L * H * (hd / 16);
+  if (hd % 16 != 0 || n <= 0 || n >= (1L << 31) || (((uintptr_t)dst | (uintptr_t)src | (uintptr_t)cosT | (uintptr_t)sinT) & 15)) return -7;
+  mlb_launch(rope_copy_k, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, (bf16*)dst, (const bf16*)src, cosT, sinT, (unsigned)n, T, H, Hkv, hd);
+  LAUNCH_RET;
+}
+MLB_API int mlb_kv_group_sum(void* dst, const void* src, long rows, int H, int Hkv, int hd, cudaStream_t st) {
+  const long n = rows * (H + 2L * Hkv) * (hd / 8);
+  if (hd % 8 != 0 || n <= 0 || n >= (1L << 31) || (((uintptr_t)dst | (uintptr_t)src) & 15)) return -7;
+  mlb_launch(kv_group_sum_k, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, (bf16*)dst, (const bf16*)src, (unsigned)n, H, Hkv, hd);
   LAUNCH_RET;
 }
 MLB_API int mlb_swiglu_fwd(void* out, const void* gu, long rows, int I, cudaStream_t st) {

@@ -6,7 +6,7 @@ inside ordinary PyTorch code (custom losses, torch optimizers); use `Trainer` / 
 
 Two options of the reference's prototype model configuration (csrc/include/model.h:17-60: grouped-query attention and
 QKV biases, Qwen2.5 style) exist only here: `Decoder(cfg, n_kv_heads=..., qkv_bias=True)`.  K / V heads are repeated up
-to the H query heads in front of the attention op, so the attention kernels see the usual [B*T, 3C] layout; such a
+to the H query heads by the kernel that rotates Q and K, so the attention kernels see the usual [B*T, 3C] layout; such a
 module has no flat-buffer counterpart (`from_flat` / `load_flat` are for the default architecture).
 """
 from __future__ import annotations
@@ -34,23 +34,13 @@ class Block(nn.Module):
         self.ln2, self.gate_up, self.down = mk(C), mk(2 * I, C), mk(C, I)
         self.cfg = cfg
 
-    def _full_qkv(self, qkv):
-        """[N, (H + 2 Hkv) hd] -> [N, 3 H hd]: every K / V head serves H / Hkv consecutive query heads."""
-        c = self.cfg
-        if self.Hkv == c.H:
-            return qkv
-        N, H, hd, rep = qkv.shape[0], c.H, c.hd, c.H // self.Hkv
-        q, k, v = qkv.split([H * hd, self.Hkv * hd, self.Hkv * hd], dim=1)
-        grow = lambda t: t.view(N, self.Hkv, 1, hd).expand(N, self.Hkv, rep, hd).reshape(N, H * hd)
-        return torch.cat([q, grow(k), grow(v)], dim=1)
-
     def forward(self, x, cos, sin, B):
         c = self.cfg
         h = F.rmsnorm(x, self.ln1, c.eps)
         qkv = F.linear(h, self.qkv)
         if self.qkv_bias is not None:
             qkv = qkv + self.qkv_bias
-        a = F.rope_causal_attention(self._full_qkv(qkv).contiguous(), cos, sin, B, c.T, c.H, c.hd)
+        a = F.rope_causal_attention(qkv, cos, sin, B, c.T, c.H, c.hd, self.Hkv)
         x = x + F.linear(a, self.o)
         h = F.rmsnorm(x, self.ln2, c.eps)
         return x + F.linear(F.swiglu(F.linear(h, self.gate_up)), self.down)

@@ -75,17 +75,20 @@ class SwiGLU(torch.autograd.Function):
 
 
 class RopeCausalAttention(torch.autograd.Function):
-    """qkv[B*T, 3C] -> out[B*T, C]: rotate-half RoPE on Q and K, then causal attention (scale 1/sqrt(hd))."""
+    """qkv[B*T, (H + 2 Hkv) hd] -> out[B*T, H hd]: rotate-half RoPE on Q and K, then causal attention (scale 1/sqrt(hd)); every key /
+    value head serves H / Hkv consecutive query heads (Hkv None: one each)."""
 
     @staticmethod
-    def forward(ctx, qkv, cos, sin, B, T, H, hd):
-        q = qkv.contiguous().clone()
-        ops.rope_fwd(q, cos, sin, B, T, H, hd)
+    def forward(ctx, qkv, cos, sin, B, T, H, hd, Hkv=None):
+        qkv = qkv.contiguous()
+        q = _like(qkv, B * T, 3 * H * hd)
+        ops.rope_copy(q, qkv, cos, sin, B, T, H, hd, Hkv)
         out = _like(qkv, B * T, H * hd)
         lse = _like(qkv, B, H, T, dtype=torch.float32)
         ops.attn_fwd(out, lse, q, B, T, H, hd)
         ctx.save_for_backward(q, out, lse, cos, sin)
         ctx.dims = (B, T, H, hd)
+        ctx.Hkv, ctx.shape = Hkv, qkv.shape
         return out
 
     @staticmethod
@@ -96,7 +99,10 @@ class RopeCausalAttention(torch.autograd.Function):
         fused = ops.attn_bwd(dqkv, dout.contiguous(), q, out, lse, B, T, H, hd, rope=(cos, sin))
         if not fused:
             ops.rope_bwd(dqkv, cos, sin, B, T, H, hd)
-        return dqkv, None, None, None, None, None, None
+        if ctx.Hkv not in (None, H):
+            full, dqkv = dqkv, _like(q, B * T, (H + 2 * ctx.Hkv) * hd)
+            ops.kv_group_sum(dqkv, full, B, T, H, hd, ctx.Hkv)
+        return dqkv.view(ctx.shape), None, None, None, None, None, None, None
 
 
 class BidirAttention(torch.autograd.Function):

@@ -56,6 +56,8 @@ def lib():
         "mlb_rmsnorm_bwd_blocks": [_i64],
         "mlb_rmsnorm_bwd": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i32, _vp, _vp, _vp],
         "mlb_rope": [_vp, _vp, _vp, _i64, _i32, _i32, _i32, _f32, _vp],
+        "mlb_rope_copy": [_vp, _vp, _vp, _vp, _i64, _i32, _i32, _i32, _i32, _vp],
+        "mlb_kv_group_sum": [_vp, _vp, _i64, _i32, _i32, _i32, _vp],
         "mlb_swiglu_fwd": [_vp, _vp, _i64, _i32, _vp],
         "mlb_swiglu_bwd": [_vp, _vp, _vp, _i64, _i32, _vp],
         "mlb_ce_fwd_bwd": [_vp, _vp, _vp, _i64, _i32, _i64, _f32, _i32, _vp],
@@ -436,6 +438,27 @@ def rmsnorm_bwd(dx, dw, dy, x, w, rstd, add=None):
 # ------------------------------------------------------------------ rope / swiglu / CE / AdamW
 def rope_fwd(qkv, cos, sin, B, T, H, hd):
     _chk(lib().mlb_rope(_b(qkv), _f(cos), _f(sin), B * T, T, H, hd, 1.0, _st()), "rope_fwd")
+
+
+def rope_copy(out, qkv, cos, sin, B, T, H, hd, Hkv=None):
+    rc = lib().mlb_rope_copy(_b(out), _b(qkv), _f(cos), _f(sin), B * T, T, H, H if Hkv is None else Hkv, hd, _st())
+    if rc == -7:      # a head size or alignment that kernel does not take: heads laid out first, then rotated in place
+        N, rep = B * T, 1 if Hkv is None else H // Hkv
+        o, x = out.view(N, 3 * H, hd), qkv.view(N, -1, hd)
+        o[:, :H] = x[:, :H]
+        o[:, H:] = x[:, H:].repeat_interleave(rep, 1)
+        return rope_fwd(out, cos, sin, B, T, H, hd)
+    _chk(rc, "rope_copy")
+
+
+def kv_group_sum(out, dqkv, B, T, H, hd, Hkv):
+    rc = lib().mlb_kv_group_sum(_b(out), _b(dqkv), B * T, H, Hkv, hd, _st())
+    if rc == -7:
+        o, x = out.view(B * T, -1, hd), dqkv.view(B * T, 3 * H, hd)
+        o[:, :H] = x[:, :H]
+        o[:, H:] = x[:, H:].reshape(B * T, 2 * Hkv, H // Hkv, hd).sum(2)
+        return
+    _chk(rc, "kv_group_sum")
 
 
 def rope_bwd(dqkv, cos, sin, B, T, H, hd):

@@ -97,6 +97,26 @@ def rope_fwd(qkv, cos, sin, B, T, H, hd):
     _rope(qkv, cos, sin, B, T, H, hd, 1.0)
 
 
+def rope_copy(out, qkv, cos, sin, B, T, H, hd, Hkv=None):
+    """out[B*T, 3 H hd] = qkv[B*T, (H + 2 Hkv) hd] with rotate-half RoPE on Q and K, every key / value head repeated for its H / Hkv
+    query heads (Hkv None: H)."""
+    Hkv = H if Hkv is None else Hkv
+    N, rep = B * T, H // Hkv
+    qkv = qkv.view(N, -1)
+    q, k, v = qkv.split([H * hd, Hkv * hd, Hkv * hd], dim=1)
+    grow = lambda t: t.view(N, Hkv, 1, hd).expand(N, Hkv, rep, hd).reshape(N, H * hd)
+    out.copy_(qkv if rep == 1 else torch.cat([q, grow(k.contiguous()), grow(v.contiguous())], dim=1))
+    rope_fwd(out, cos, sin, B, T, H, hd)
+
+
+def kv_group_sum(out, dqkv, B, T, H, hd, Hkv):
+    """Gradient of the repetition in rope_copy: out[B*T, (H + 2 Hkv) hd] from dqkv[B*T, 3 H hd]."""
+    N, C = B * T, H * hd
+    out[:, :C] = dqkv[:, :C]
+    for i in (1, 2):
+        out[:, C + (i - 1) * Hkv * hd:C + i * Hkv * hd] = _f(dqkv[:, i * C:(i + 1) * C]).view(N, Hkv, H // Hkv, hd).sum(2).reshape(N, Hkv * hd).to(out.dtype)
+
+
 def rope_bwd(dqkv, cos, sin, B, T, H, hd):
     _rope(dqkv, cos, sin, B, T, H, hd, -1.0)
 

@@ -914,3 +914,18 @@ def test_ce_mean_and_scale(rows, V):
     view = rnd(rows * V + 1, 1)[1:].view(rows, V)      # rows that start two bytes off a 16-byte boundary
     nat().ce_mean(loss, losses, d, view, tgt)
     assert abs(loss.item() - torch.nn.functional.cross_entropy(view.double(), tgt.long(), ignore_index=-1).item()) < 1e-4
+
+
+@pytest.mark.parametrize("B,T,H,Hkv,hd", [(2, 65, 4, 2, 64), (1, 33, 6, 1, 32), (2, 17, 3, 3, 128), (1, 9, 4, 2, 24)])
+def test_rope_copy_with_grouped_heads(B, T, H, Hkv, hd):
+    torch.manual_seed(hd)
+    x = rnd(B * T, (H + 2 * Hkv) * hd)
+    cos, sin = ref.rope_tables(T, hd, 10000.0, dev())
+    out, e = rnd(B * T, 3 * H * hd), torch.empty(B * T, 3 * H * hd, device=dev())
+    nat().rope_copy(out, x, cos, sin, B, T, H, hd, Hkv)
+    ref.rope_copy(e, x, cos, sin, B, T, H, hd, Hkv)
+    assert _rel(out, e.double()) < 2 ** -9
+    back, eb = torch.empty_like(x), torch.empty_like(x)
+    nat().kv_group_sum(back, out, B, T, H, hd, Hkv)
+    ref.kv_group_sum(eb, out, B, T, H, hd, Hkv)
+    assert _rel(back, eb.double()) < 2 ** -8      # (the two round the same sums, in another order)
