@@ -1435,4 +1435,14 @@ MLB_API void mlb_gemm_tile_order(int mode) { g_tile_order = mode; }
 MLB_API void mlb_gemm_streamk_groups(int on) { g_sk_groups = on; }
 
 MLB_DEFINE_ERROR_WORD(gemm)
+// 1: dW[N,K] = dout[M,N]^T . x[M,K] in bf16 is cheaper as one product than as add-reduced pieces plus zero-fill and cast (the estimates
+// of gemm_dispatch_impl, in cycles; the two extra launches ~2.5 us each, their 14 bytes per element at 3400 bytes per cycle).
+MLB_API int mlb_gemm_dw_direct(int N, int K, int M) {
+  if (N % 8 != 0 || K % 8 != 0) return 0;
+  const double kb = ceil_div_i(M, BK), pc = pair_clusters(), sm = g_max_ctas > 0 ? g_max_ctas : num_sms();
+  const double pt = (double)ceil_div_i(N, 256) * ceil_div_i(K, 256), ct = (double)ceil_div_i(N, 128) * ceil_div_i(K, 128);
+  const double direct = std::min(ceil(pt / pc) * (kb * 512.0 + 2000.0), ceil(ct / sm) * (kb * 320.0 + 2000.0));
+  const double split = std::max(pt * kb / pc, 8.0) * 512.0 + 4000.0 + 9000.0 + 14.0 * N * K / 3400.0;
+  return direct <= split ? 1 : 0;
+}
 MLB_API void mlb_gemm_streamk_whole(int on) { g_sk_whole = on; }

@@ -37,9 +37,7 @@ class Block(nn.Module):
     def forward(self, x, cos, sin, B):
         c = self.cfg
         h = F.rmsnorm(x, self.ln1, c.eps)
-        qkv = F.linear(h, self.qkv)
-        if self.qkv_bias is not None:
-            qkv = qkv + self.qkv_bias
+        qkv = F.linear(h, self.qkv, self.qkv_bias)
         a = F.rope_causal_attention(qkv, cos, sin, B, c.T, c.H, c.hd, self.Hkv)
         x = x + F.linear(a, self.o)
         h = F.rmsnorm(x, self.ln2, c.eps)

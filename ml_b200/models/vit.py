@@ -42,11 +42,11 @@ class ViTBlock(nn.Module):
 
     def forward(self, x, B, T):
         h = self._norm(x, self.n1_w, self.n1_b)
-        qkv = F.linear(h, self.qkv_w) + self.qkv_b
+        qkv = F.linear(h, self.qkv_w, self.qkv_b)
         a = F.bidir_attention(qkv, B, T, self.H, self.C // self.H)
-        x = x + F.linear(a, self.o_w) + self.o_b
+        x = x + F.linear(a, self.o_w, self.o_b)
         h = self._norm(x, self.n2_w, self.n2_b)
-        return x + F.linear(F.swiglu(F.linear(h, self.gu_w) + self.gu_b), self.down_w) + self.down_b
+        return x + F.linear(F.swiglu(F.linear(h, self.gu_w, self.gu_b)), self.down_w, self.down_b)
 
 
 class ViTEncoder(nn.Module):
@@ -96,7 +96,7 @@ class ViTEncoder(nn.Module):
         C, T, NP = self.C, self.T, self.n_patch
         rows = torch.empty(B * NP, self.channels * self.patch * self.patch, dtype=self.patch_w.dtype, device=pixels.device)
         ops.patchify(rows, pixels.contiguous().float(), self.patch)
-        x = self._norm(F.linear(rows, self.patch_w) + self.patch_b, self.pn_w, self.pn_b)
+        x = self._norm(F.linear(rows, self.patch_w, self.patch_b), self.pn_w, self.pn_b)
         x = torch.cat([self.cls.expand(B, 1, C), x.view(B, NP, C)], dim=1) + self.pos
         x = x.reshape(B * T, C)
         for blk in self.blocks:

@@ -18,13 +18,17 @@ def _like(x, *shape, dtype=None):
 
 
 class Linear(torch.autograd.Function):
-    """y[M,N] = x[M,K] @ W[N,K]^T; dW is produced in fp32 and cast to W's dtype."""
+    """y[M,N] = x[M,K] @ W[N,K]^T (+ b[N], added to the fp32 accumulators); dW is summed in fp32 and rounded once to W's dtype."""
 
     @staticmethod
-    def forward(ctx, x, W):
+    def forward(ctx, x, W, b=None):
         ctx.save_for_backward(x, W)
+        ctx.bias = None if b is None else b.dtype
         out = _like(x, x.shape[0], W.shape[0])
-        ops.linear_fwd(out, x.contiguous(), W.contiguous())
+        if b is None:
+            ops.linear_fwd(out, x.contiguous(), W.contiguous())
+        else:
+            ops.linear_bias_fwd(out, x.contiguous(), W.contiguous(), b.contiguous())
         return out
 
     @staticmethod
@@ -33,9 +37,9 @@ class Linear(torch.autograd.Function):
         dout = dout.contiguous()
         dx = _like(x, *x.shape)
         ops.linear_dx(dx, dout, W.contiguous())
-        dW = torch.zeros(W.shape, dtype=torch.float32, device=W.device)
-        ops.linear_dw(dW, dout, x.contiguous())
-        return dx, dW.to(W.dtype)
+        dW = _like(W, *W.shape)
+        ops.linear_dw_cast(dW, dout, x.contiguous())
+        return dx, dW, (None if ctx.bias is None else dout.sum(0).to(ctx.bias))
 
 
 class RMSNorm(torch.autograd.Function):

@@ -31,6 +31,7 @@ def lib():
         "mlb_linear_dx": [_vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _vp],
         "mlb_linear_dw": [_vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _vp],
         "mlb_gemm": [_vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _vp],
+        "mlb_gemm_dw_direct": [_i32, _i32, _i32],
         "mlb_gemm_force_simt": [_i32],
         "mlb_gemm_set_max_ctas": [_i32],
         "mlb_gemm_set_splits": [_i32],
@@ -287,6 +288,26 @@ def linear_dw(dW, dout, x):
     M, N = dout.shape
     K = x.shape[1]
     _chk(lib().mlb_linear_dw(_f(dW), _b(dout), _b(x), M, N, K, dW.stride(0), dout.stride(0), x.stride(0), _st()), "linear_dw")
+
+
+def linear_bias_fwd(out, x, W, b):
+    """out = x . W^T + b: the position-table epilogue with a period of one row; where the shape does not take it the bias is added
+    behind the product."""
+    if not linear_fwd_posembed(out, x, W, b.view(1, -1), 1):
+        linear_fwd(out, x, W)
+        out += b
+
+
+def linear_dw_cast(dW, dout, x):
+    """dW (bf16, overwritten) = dout^T . x with fp32 accumulation and one rounding.  Either one product that stores bf16, or the
+    add-reduce product into a zeroed fp32 buffer and a cast: the second cuts the reduction over the rows up to fill the machine,
+    the first saves two launches and 14 bytes per element of dW.  The library's estimate of both decides."""
+    if dW.dtype == torch.bfloat16 and (lib().mlb_gemm_dw_direct(dout.shape[1], x.shape[1], dout.shape[0]) or dW.numel() == 0):
+        return gemm(dW, dout, x, True, True, False)
+    acc = torch.empty(dW.shape, dtype=torch.float32, device=dW.device)
+    zero_(acc)
+    linear_dw(acc, dout, x)
+    cast(dW, acc)
 
 
 def gemm(out, A, B, a_mn=False, b_mn=False, accumulate=False):

@@ -147,6 +147,16 @@ def linear_dx(dx, dout, W):
     dx.copy_(_f(dout) @ _f(W))
 
 
+def linear_bias_fwd(out, x, W, b):
+    """out = x @ W^T + b, rounded once."""
+    out.copy_(_f(x) @ _f(W).T + _f(b))
+
+
+def linear_dw_cast(dW, dout, x):
+    """dW = dout^T @ x (overwritten), summed in fp32 and rounded once to dW's dtype."""
+    dW.copy_(_f(dout).T @ _f(x))
+
+
 def linear_dw(dW, dout, x):
     """dW[N,K] (fp32) += dout[M,N]^T @ x[M,K]"""
     dW.add_(_f(dout).t() @ _f(x))

@@ -929,3 +929,14 @@ def test_rope_copy_with_grouped_heads(B, T, H, Hkv, hd):
     nat().kv_group_sum(back, out, B, T, H, hd, Hkv)
     ref.kv_group_sum(eb, out, B, T, H, hd, Hkv)
     assert _rel(back, eb.double()) < 2 ** -8      # (the two round the same sums, in another order)
+
+
+@pytest.mark.parametrize("M,N,K", [(64, 96, 64), (200, 264, 136), (1003, 768, 768), (3000, 2304, 256), (50, 1024, 2048)])
+def test_linear_bias_dw_cast(M, N, K):
+    torch.manual_seed(M)
+    x, W, b, d = rnd(M, K), rnd(N, K, scale=0.1), rnd(N), rnd(M, N)
+    out, dW = rnd(M, N), rnd(N, K)
+    nat().linear_bias_fwd(out, x, W, b)
+    assert _rel(out, x.double() @ W.double().T + b.double()) < 2 ** -8      # twice rounded where the epilogue does not take the shape
+    nat().linear_dw_cast(dW, d, x)
+    assert _rel(dW, d.double().T @ x.double()) < 2 ** -9
