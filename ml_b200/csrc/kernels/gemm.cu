@@ -799,6 +799,22 @@ EncodeTiledFn get_encode() {
   return fn;
 }
 
+// Encoding a tensor map is a driver call and needs the device's context bound to the calling thread.  Launches and the other runtime
+// calls bind it themselves, but a thread whose first call is this one (an autograd worker that finds its memory in the
+// allocator's cache) may have none: bind it and try once more.
+int g_encode_error = 0;      // the driver's code of the last map it refused
+template <typename... A>
+CUresult encode_map(EncodeTiledFn enc, A... args) {
+  CUresult r = enc(args...);
+  if (r != CUDA_SUCCESS) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess && cudaFree(nullptr) == cudaSuccess) r = enc(args...);
+    else cudaGetLastError();
+    if (r != CUDA_SUCCESS) g_encode_error = (int)r;
+  }
+  return r;
+}
+
 std::mutex g_tmap_mu;
 typedef std::tuple<const void*, uint64_t, uint64_t, uint64_t, uint32_t, uint32_t, int> TmapKey;
 std::map<TmapKey, CUtensorMap*> g_tmaps;
@@ -831,7 +847,7 @@ bool mlb_make_tmap(CUtensorMap* out, const void* base, uint64_t rows, uint64_t c
   cuuint32_t estr[2] = {1, 1};
   const CUtensorMapDataType dt = elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
                                  : (elem_bytes == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32);
-  CUresult r = enc(out, dt, 2, const_cast<void*>(base), dims, strides, box, estr,
+  CUresult r = encode_map(enc, out, dt, 2, const_cast<void*>(base), dims, strides, box, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
@@ -863,7 +879,7 @@ const CUtensorMap* mlb_tmap_mn3d_cached(const void* base, uint64_t k_rows, uint6
   cuuint64_t strides[2] = {pitch_elems * 2, 128};
   cuuint32_t box[3] = {64, 64, chunks};
   cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+  CUresult r = encode_map(enc, m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) { delete m; g_tmaps[key] = nullptr; return nullptr; }
@@ -884,7 +900,7 @@ const CUtensorMap* mlb_tmap_seq3d_cached(const void* base, uint64_t seqs, uint64
   cuuint64_t strides[2] = {cols * 2, rows * cols * 2};
   cuuint32_t box[3] = {64, 64, 1};
   cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+  CUresult r = encode_map(enc, m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) { delete m; return nullptr; }
@@ -1445,4 +1461,6 @@ MLB_API int mlb_gemm_dw_direct(int N, int K, int M) {
   const double split = std::max(pt * kb / pc, 8.0) * 512.0 + 4000.0 + 9000.0 + 14.0 * N * K / 3400.0;
   return direct <= split ? 1 : 0;
 }
+// The driver's code of the last tensor map it refused (a -2 of the entry points), 0 if none
+MLB_API int mlb_tmap_error(void) { return g_encode_error; }
 MLB_API void mlb_gemm_streamk_whole(int on) { g_sk_whole = on; }

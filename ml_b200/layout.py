@@ -14,6 +14,7 @@ Vision tower order (train/gpt.cu:813-843):
 """
 from __future__ import annotations
 
+import math
 from dataclasses import dataclass
 from typing import List, Tuple
 
@@ -29,6 +30,21 @@ class LayerOff:
     gate: int
     up: int
     down: int
+
+
+class FlatViews:
+    """Shaped views of ranges of a flat buffer, each made once: two tensor operations per parameter and use are most of the
+    host time of a small step."""
+
+    def __init__(self):
+        self._views = {}
+
+    def get(self, base, off: int, shape):
+        key = (off, shape)
+        v = self._views.get(key)
+        if v is None or v[0] is not base:      # (the buffer behind the name may be replaced)
+            v = self._views[key] = (base, base[off:off + math.prod(shape)].view(*shape))
+        return v[1]
 
 
 class DecoderLayout:

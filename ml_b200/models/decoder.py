@@ -12,14 +12,13 @@ while the rest of backward runs.
 """
 from __future__ import annotations
 
-import math
 from typing import Callable, Optional
 
 import torch
 
 from .. import ops
 from ..config import Config
-from ..layout import DecoderLayout, flops_per_step
+from ..layout import DecoderLayout, FlatViews, flops_per_step
 from ..utils import rng as _rng
 
 import os as _os
@@ -73,6 +72,7 @@ class GPT:
         self.np = L.num_params
         dev = self.device
         self.sharded = sharded
+        self._pviews, self._gviews, self._p8views = FlatViews(), FlatViews(), FlatViews()
         self.res = None          # optional view resolver: res.param(off, shape) / res.grad(off, shape)
         self.pre_hook = None     # optional pre_hook(unit_name, phase) called before a unit's parameters are first used
         self.cp = None           # optional sequence-parallel attention (ml_b200.parallel.cp.SequenceParallel)
@@ -175,14 +175,16 @@ class GPT:
     def P(self, off, *shape):
         if self.res is not None:
             return self.res.param(off, shape)
-        n = math.prod(shape)
-        return self.params[off:off + n].view(*shape)
+        return self._pviews.get(self.params, off, shape)
 
     def G(self, off, *shape):
         if self.res is not None:
             return self.res.grad(off, shape)
-        n = math.prod(shape)
-        return self.grads[off:off + n].view(*shape)
+        return self._gviews.get(self.grads, off, shape)
+
+    def _rows(self, n):
+        """t -> its first n rows; the buffer itself when that is all of them (no view to make)."""
+        return (lambda t: t) if n == self.B * self.cfg.T else (lambda t: t[:n])
 
     def _pre(self, unit, phase):
         if self.pre_hook is not None:
@@ -205,7 +207,7 @@ class GPT:
         self.refresh_params8()
 
     def P8(self, off, *shape):
-        return self.params8[off:off + math.prod(shape)].view(*shape)
+        return self._p8views.get(self.params8, off, shape)
 
     def refresh_params8(self):
         """E4M3 copy of the bf16 parameters (x ENTROPY_FP8_W_SCALE) for the 8-bit forward.  AdamW writes it in the same pass
@@ -231,7 +233,7 @@ class GPT:
         if (self.fp8_native and x_in is None and has_head and self.cp is None and self.res is None and
                 not ({"norm", "swiglu"} & self.skip)):       # the reference drops to bf16 under those two ablations too
             return self._forward_fp8(ids, B, prefix, n_pre)
-        sl = lambda t: t[:BT]
+        sl = self._rows(BT)
         x0 = sl(self.x0)
         if x_in is not None:
             x0.copy_(x_in)
@@ -269,7 +271,7 @@ class GPT:
                 if self.cp is not None:     # sequence shards: attention runs head-sharded over the full sequences
                     self.cp.attn_fwd(self, l, sl(self.atty[l]), qkv, B)
                 else:
-                    ops.attn_fwd(sl(self.atty[l]), self.lse[l][:B], qkv, B, T, H, hd)
+                    ops.attn_fwd(sl(self.atty[l]), (self.lse[l] if B == self.B else self.lse[l][:B]), qkv, B, T, H, hd)
             self._mark("F_attn")
             proj = sl(self.proj)
             ops.linear_fwd(proj, sl(self.atty[l]), self.P(o.o, C, C))
@@ -321,7 +323,7 @@ class GPT:
         nat = ops.native_module()
         T, C, I, H, hd = c.T, c.C, c.I, c.H, c.hd
         BT = B * T
-        sl = lambda t: t[:BT]
+        sl = self._rows(BT)
         sa, deq = self.fp8_act_scale, 1.0 / (self.fp8_act_scale * self.fp8_w_scale)
         x0 = sl(self.x0)
         ops.embed_fwd(x0, self.P(Lo.off_wte, c.V, C), ids)
@@ -347,7 +349,7 @@ class GPT:
                     ops.rope_fwd(qkv, self.cos, self.sin, B, T, H, hd)
             self._mark("F_qkv+rope")
             if "attn" not in self.skip:
-                ops.attn_fwd(sl(self.atty[l]), self.lse[l][:B], qkv, B, T, H, hd)
+                ops.attn_fwd(sl(self.atty[l]), (self.lse[l] if B == self.B else self.lse[l][:B]), qkv, B, T, H, hd)
             self._mark("F_attn")
             proj = sl(self.proj)
             ops.linear_fwd(proj, sl(self.atty[l]), self.P(o.o, C, C))
@@ -383,7 +385,7 @@ class GPT:
         B = self.B if B is None else B
         T, C, I, H, hd, V = c.T, c.C, c.I, c.H, c.hd, c.V
         BT = B * T
-        sl = lambda t: t[:BT]
+        sl = self._rows(BT)
         if zero and self.grads is not None:
             ops.zero_(self.grads)
         valid = valid_tokens if valid_tokens is not None else BT - B * n_pre
@@ -434,7 +436,7 @@ class GPT:
                 self.cp.attn_bwd(self, l, dqkv, datty, B)
                 fused = False
             else:
-                fused = ops.attn_bwd(dqkv, datty, sl(self.qkv[l]), sl(self.atty[l]), self.lse[l][:B], B, T, H, hd,
+                fused = ops.attn_bwd(dqkv, datty, sl(self.qkv[l]), sl(self.atty[l]), (self.lse[l] if B == self.B else self.lse[l][:B]), B, T, H, hd,
                                      rope=(self.cos, self.sin) if want_rope else None, have_delta=bool(have_delta))
             if want_rope and not fused:
                 ops.rope_bwd(dqkv, self.cos, self.sin, B, T, H, hd)

@@ -8,14 +8,13 @@ sample.  Own flat master/params/grads/m/v buffers.  The reference takes already-
 """
 from __future__ import annotations
 
-import math
 from typing import Optional
 
 import torch
 
 from .. import ops
 from ..config import VisionConfig
-from ..layout import VisionLayout
+from ..layout import FlatViews, VisionLayout
 from ..utils import rng as _rng
 
 
@@ -35,6 +34,7 @@ class VisionTower:
         self.grads = mk(self.np, torch.float32).zero_()
         self.m = torch.zeros(self.np, dtype=torch.float32, device=dev)
         self.v = torch.zeros(self.np, dtype=torch.float32, device=dev)
+        self._pviews, self._gviews = FlatViews(), FlatViews()
         NP = B * vc.n_patch
         e = lambda *s: torch.empty(*s, dtype=dtype, device=dev)
         f = lambda *s: torch.empty(*s, dtype=torch.float32, device=dev)
@@ -51,10 +51,10 @@ class VisionTower:
         self.dgu, self.dsw, self.dfn, self.dimg = e(NP, 2 * vI), e(NP, vI), e(NP, vC), e(NP, C)
 
     def P(self, off, *shape):
-        return self.params[off:off + math.prod(shape)].view(*shape)
+        return self._pviews.get(self.params, off, shape)
 
     def G(self, off, *shape):
-        return self.grads[off:off + math.prod(shape)].view(*shape)
+        return self._gviews.get(self.grads, off, shape)
 
     def init_weights(self, seed: int = 777):
         self.master.copy_(_rng.init_vision(self.layout, seed).to(self.device))

@@ -3,6 +3,8 @@ in-tree shared library; a missing library on a GPU machine is an error, never a 
 CPU tensors go to the fp32 PyTorch oracle (`ops.ref`), which is also what the GPU tests compare against."""
 from __future__ import annotations
 
+import torch
+
 from . import ref
 
 _NAMES = [
@@ -29,9 +31,11 @@ def _make(name):
     rf = getattr(ref, name)
 
     def op(*args, **kw):
-        t = next(a for a in args if hasattr(a, "is_cuda"))
+        t = args[0]
+        if not isinstance(t, torch.Tensor):
+            t = next(a for a in args if hasattr(a, "is_cuda"))
         if t.is_cuda:
-            return getattr(_load_native(), name)(*args, **kw)
+            return getattr(_native_mod or _load_native(), name)(*args, **kw)
         return rf(*args, **kw)
 
     op.__name__ = name

@@ -75,11 +75,33 @@ def lib():
         "mlb_patchify": [_vp, _vp, _i32, _i32, _i32, _i32, _i32, _vp],
         "mlb_add_posembed": [_vp, _vp, _i64, _i32, _i32, _vp],
         "mlb_posembed_grad": [_vp, _vp, _i64, _i32, _i32, _vp],
+        "mlb_linear_fwd_rope": [_vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _vp, _vp, _i32, _i32, _vp],
+        "mlb_linear_fwd_swiglu": [_vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _vp],
+        "mlb_linear_fwd_posembed": [_vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _vp],
+        "mlb_linear_fwd_gather": [_vp, _vp, _i32, _i32, _i32, _i32, _i32, _vp, _i64, _vp, _i64, _i32, _vp, _vp, C.c_double, _vp],
+        "mlb_linear_dx_delta": [_vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _vp],
+        "mlb_attn_bidir_fwd": [_vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp],
+        "mlb_attn_bidir_bwd": [_vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp],
+        "mlb_layernorm_fwd": [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i32, _f32, _vp],
+        "mlb_layernorm_bwd": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i32, _vp],
+        "mlb_linear_fwd_fp8": [_vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _f32, _vp],
+        "mlb_linear_fwd_fp8_rope": [_vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _f32, _vp, _vp, _i32, _i32, _vp],
+        "mlb_linear_fwd_fp8_swiglu": [_vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _f32, _vp],
+        "mlb_rmsnorm_fwd_fp8": [_vp, _vp, _vp, _vp, _vp, _i64, _i32, _f32, _f32, _vp],
+        "mlb_add_rmsnorm_fwd_fp8": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i32, _f32, _f32, _vp],
+        "mlb_swiglu_fwd_fp8": [_vp, _vp, _vp, _i64, _i32, _f32, _vp],
+        "mlb_cast_bf16_fp8": [_vp, _vp, _i64, _f32, _vp],
+        "mlb_adamw_fp8": [_vp] * 6 + [_i64] + [_f32] * 9 + [_vp, _vp],
+        "mlb_sum_scale": [_vp, _vp, _i64, _f32, _vp],
+        "mlb_zero": [_vp, _i64, _vp],
     }
     for name, args in sig.items():
         fn = getattr(L, name)
         fn.argtypes = args
         fn.restype = _i32
+    L.mlb_attn_bwd_have_delta.argtypes = L.mlb_attn_bwd.argtypes
+    L.mlb_attn_bwd_have_delta.restype = _i32
+    L.mlb_attn_bwd_scratch_bytes.restype = _i64
     for tag in ("gemm", "attn", "elementwise", "comm"):
         for pre in ("mlb_get_error_", "mlb_clear_error_"):
             if hasattr(L, pre + tag):
@@ -131,7 +153,8 @@ LAUNCHES = 0  # number of kernel-launching calls made through this module (bench
 
 
 def _st():
-    return torch.cuda.current_stream().cuda_stream
+    # the current stream's handle without a Stream object around it (that costs more than the rest of a call's arguments)
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _chk(rc, name):
@@ -142,6 +165,8 @@ def _chk(rc, name):
 
 
 def _cuda_err(rc):
+    if rc == -2:
+        return f"tensor map refused, driver code {lib().mlb_tmap_error()}"
     try:
         return torch.cuda.cudart().cudaGetErrorString(rc) if rc > 0 else "library error"
     except Exception:
@@ -232,10 +257,7 @@ def linear_fwd_rope(out, x, W, cos, sin, T, rope_cols):
     columns, position = row % T).  Returns False when the shape does not take that path (nothing was launched)."""
     M, K = x.shape
     N = W.shape[0]
-    L = lib()
-    fn = L.mlb_linear_fwd_rope
-    fn.argtypes = [_vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _vp, _vp, _i32, _i32, _vp]
-    fn.restype = _i32
+    fn = lib().mlb_linear_fwd_rope
     rc = fn(_b(out), _b(x), _b(W), M, N, K, out.stride(0), x.stride(0), W.stride(0), _f(cos), _f(sin), T, rope_cols, _st())
     if rc == -7:
         return False
@@ -252,8 +274,6 @@ def linear_fwd_swiglu(gu, sw, x, W):
     if W.shape[0] != 2 * I or gu.shape[1] != 2 * I or sw.stride(0) != I:
         return False
     fn = lib().mlb_linear_fwd_swiglu
-    fn.argtypes = [_vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _vp]
-    fn.restype = _i32
     rc = fn(_b(gu), _b(sw), _b(x), _b(W), M, I, K, gu.stride(0), x.stride(0), W.stride(0), _st())
     if rc == -7:
         return False
@@ -269,8 +289,6 @@ def linear_fwd_posembed(out, x, W, pos, period):
     if pos.shape[-1] != N or not pos.is_contiguous():
         return False
     fn = lib().mlb_linear_fwd_posembed
-    fn.argtypes = [_vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _vp]
-    fn.restype = _i32
     rc = fn(_b(out), _b(x), _b(W), _b(pos), period, M, N, K, out.stride(0), x.stride(0), W.stride(0), _st())
     if rc == -7:
         return False
@@ -322,10 +340,7 @@ def gemm(out, A, B, a_mn=False, b_mn=False, accumulate=False):
 def linear_fwd_gather(out, x, N, K, unit_dst, w_off, src_table, shard_elems, world, flags, ctr, spin_limit_s=20.0):
     """out = x . W^T with W = unit_dst[w_off : w_off + N*K] viewed [N, K]; the same launch all-gathers the whole sharded
     unit into unit_dst from the ranks' shards (device pointer table `src_table`).  Cooperative launch."""
-    L = lib()
-    fn = L.mlb_linear_fwd_gather
-    fn.argtypes = [_vp, _vp, _i32, _i32, _i32, _i32, _i32, _vp, _i64, _vp, _i64, _i32, _vp, _vp, C.c_double, _vp]
-    fn.restype = _i32
+    fn = lib().mlb_linear_fwd_gather
     M = x.shape[0]
     _chk(fn(_b(out), _b(x), M, N, K, out.stride(0), x.stride(0), _b(unit_dst), w_off, src_table.data_ptr(), shard_elems, world,
             _i(flags), _i(ctr), spin_limit_s, _st()), "linear_fwd_gather")
@@ -350,8 +365,6 @@ def linear_dx_delta(dx, dout, W, o, B, T, H):
         return False
     delta = scratch("attn_delta", B * H * T, torch.float32, dout.device)
     fn = lib().mlb_linear_dx_delta
-    fn.argtypes = [_vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _vp]
-    fn.restype = _i32
     rc = fn(_b(dx), _b(dout), _b(W), _b(o), _f(delta), T, H, M, N, Cc, dx.stride(0), dout.stride(0), W.stride(0), _st())
     if rc == -7:
         return False
@@ -367,9 +380,7 @@ def attn_bwd(dqkv, dout, qkv, out, lse, B, T, H, hd, rope=None, have_delta=False
     acc = None
     if hd == 64 and FUSED_ATTN_BWD:
         # per-(query tile, key tile) bf16 partials of dQ; past FUSED_ATTN_BWD_MAX_SCRATCH the two-kernel backward runs
-        L = lib()
-        L.mlb_attn_bwd_scratch_bytes.restype = C.c_long
-        nbytes = L.mlb_attn_bwd_scratch_bytes(B, T, H, hd)
+        nbytes = lib().mlb_attn_bwd_scratch_bytes(B, T, H, hd)
         if 0 < nbytes <= FUSED_ATTN_BWD_MAX_SCRATCH:
             acc = scratch(("attn_dq_part", nbytes), nbytes // 2, torch.bfloat16, qkv.device).data_ptr()
     cp = _f(rope[0]) if rope is not None else None
@@ -377,8 +388,6 @@ def attn_bwd(dqkv, dout, qkv, out, lse, B, T, H, hd, rope=None, have_delta=False
     fn = lib().mlb_attn_bwd
     if have_delta:
         fn = lib().mlb_attn_bwd_have_delta
-        fn.argtypes = lib().mlb_attn_bwd.argtypes
-        fn.restype = _i32
     rc = fn(_b(dqkv), _b(dout), _b(qkv), _b(out), _f(lse), _f(delta), acc, B, T, H, hd, cp, sp, _st())
     global LAUNCHES
     LAUNCHES += 2 if have_delta else 3
@@ -389,16 +398,12 @@ def attn_bwd(dqkv, dout, qkv, out, lse, B, T, H, hd, rope=None, have_delta=False
 
 def attn_bidir_fwd(out, lse, qkv, B, T, H, hd):
     fn = lib().mlb_attn_bidir_fwd
-    fn.argtypes = [_vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp]
-    fn.restype = _i32
     _chk(fn(_b(out), _f(lse), _b(qkv), B, T, H, hd, _st()), "attn_bidir_fwd")
 
 
 def attn_bidir_bwd(dqkv, dout, qkv, out, lse, B, T, H, hd):
     delta = scratch("attn_delta", B * H * T, torch.float32, qkv.device)
     fn = lib().mlb_attn_bidir_bwd
-    fn.argtypes = [_vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp]
-    fn.restype = _i32
     _chk(fn(_b(dqkv), _b(dout), _b(qkv), _b(out), _f(lse), _f(delta), B, T, H, hd, _st()), "attn_bidir_bwd")
 
 
@@ -433,16 +438,12 @@ def add_rmsnorm_fwd(resid, out, rstd, a, b, w, eps):
 def layernorm_fwd(out, mean, rstd, x, w, b, eps):
     rows, Cc = x.shape
     fn = lib().mlb_layernorm_fwd
-    fn.argtypes = [_vp, _vp, _vp, _vp, _vp, _vp, C.c_long, _i32, C.c_float, _vp]
-    fn.restype = _i32
     _chk(fn(_b(out), _f(mean), _f(rstd), _b(x), _b(w), _b(b) if b is not None else None, rows, Cc, eps, _st()), "layernorm_fwd")
 
 
 def layernorm_bwd(dx, dw, db, dy, x, w, mean, rstd):
     rows, Cc = x.shape
     fn = lib().mlb_layernorm_bwd
-    fn.argtypes = [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, C.c_long, _i32, _vp]
-    fn.restype = _i32
     _chk(fn(_b(dx), _f(dw), _f(db) if db is not None else None, _b(dy), _b(x), _b(w), _f(mean), _f(rstd), rows, Cc, _st()), "layernorm_bwd")
 
 
@@ -582,8 +583,6 @@ def linear_fwd_fp8(out, x8, W8, out_scale):
     M, K = x8.shape
     N = W8.shape[0]
     fn = lib().mlb_linear_fwd_fp8
-    fn.argtypes = [_vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, C.c_float, _vp]
-    fn.restype = _i32
     rc = fn(_b(out), _u8(x8), _u8(W8), M, N, K, out.stride(0), x8.stride(0), W8.stride(0), out_scale, _st())
     if rc == -7:
         return False
@@ -595,8 +594,6 @@ def linear_fwd_fp8_rope(out, x8, W8, out_scale, cos, sin, T, rope_cols):
     M, K = x8.shape
     N = W8.shape[0]
     fn = lib().mlb_linear_fwd_fp8_rope
-    fn.argtypes = [_vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, C.c_float, _vp, _vp, _i32, _i32, _vp]
-    fn.restype = _i32
     rc = fn(_b(out), _u8(x8), _u8(W8), M, N, K, out.stride(0), x8.stride(0), W8.stride(0), out_scale, _f(cos), _f(sin), T, rope_cols, _st())
     if rc == -7:
         return False
@@ -610,8 +607,6 @@ def linear_fwd_fp8_swiglu(gu, sw, x8, W8, out_scale):
     if W8.shape[0] != 2 * I or gu.shape[1] != 2 * I or sw.stride(0) != I:
         return False
     fn = lib().mlb_linear_fwd_fp8_swiglu
-    fn.argtypes = [_vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, C.c_float, _vp]
-    fn.restype = _i32
     rc = fn(_b(gu), _b(sw), _u8(x8), _u8(W8), M, I, K, gu.stride(0), x8.stride(0), W8.stride(0), out_scale, _st())
     if rc == -7:
         return False
@@ -622,39 +617,29 @@ def linear_fwd_fp8_swiglu(gu, sw, x8, W8, out_scale):
 def rmsnorm_fwd_fp8(out, out8, rstd, x, w, eps, scale):
     rows, Cc = x.shape
     fn = lib().mlb_rmsnorm_fwd_fp8
-    fn.argtypes = [_vp, _vp, _vp, _vp, _vp, C.c_long, _i32, C.c_float, C.c_float, _vp]
-    fn.restype = _i32
     _chk(fn(_b(out), _u8(out8), _f(rstd), _b(x), _b(w), rows, Cc, eps, scale, _st()), "rmsnorm_fwd_fp8")
 
 
 def add_rmsnorm_fwd_fp8(resid, out, out8, rstd, a, b, w, eps, scale):
     rows, Cc = a.shape
     fn = lib().mlb_add_rmsnorm_fwd_fp8
-    fn.argtypes = [_vp, _vp, _vp, _vp, _vp, _vp, _vp, C.c_long, _i32, C.c_float, C.c_float, _vp]
-    fn.restype = _i32
     _chk(fn(_b(resid), _b(out), _u8(out8), _f(rstd), _b(a), _b(b), _b(w), rows, Cc, eps, scale, _st()), "add_rmsnorm_fwd_fp8")
 
 
 def swiglu_fwd_fp8(out, out8, gu, scale):
     rows, I2 = gu.shape
     fn = lib().mlb_swiglu_fwd_fp8
-    fn.argtypes = [_vp, _vp, _vp, C.c_long, _i32, C.c_float, _vp]
-    fn.restype = _i32
     _chk(fn(_b(out), _u8(out8), _b(gu), rows, I2 // 2, scale, _st()), "swiglu_fwd_fp8")
 
 
 def cast_bf16_fp8(out8, x, scale):
     fn = lib().mlb_cast_bf16_fp8
-    fn.argtypes = [_vp, _vp, C.c_long, C.c_float, _vp]
-    fn.restype = _i32
     _chk(fn(_u8(out8), _b(x), x.numel(), scale, _st()), "cast_bf16_fp8")
 
 
 def adamw_fp8(master, params, params8, grads, m, v, lr, b1, b2, eps, wd, bc1, bc2, grad_scale, w_scale, dev_hyper=None):
     """AdamW that also writes the E4M3 copy of the updated weights (x w_scale) the 8-bit forward reads."""
     fn = lib().mlb_adamw_fp8
-    fn.argtypes = [_vp] * 6 + [C.c_long] + [C.c_float] * 9 + [_vp, _vp]
-    fn.restype = _i32
     hp = _f(dev_hyper) if dev_hyper is not None else None
     _chk(fn(_f(master), _b(params), _u8(params8), _f(grads), _f(m), _f(v), master.numel(), lr, b1, b2, eps, wd, bc1, bc2, grad_scale,
             w_scale, hp, _st()), "adamw_fp8")
@@ -667,15 +652,11 @@ def fp8_qdq(out, x, scale=1.0):
 def sum_scale(out, x, scale):
     """out[0] = scale * sum(x) on the device (x fp32, contiguous)."""
     fn = lib().mlb_sum_scale
-    fn.argtypes = [_vp, _vp, C.c_long, C.c_float, _vp]
-    fn.restype = _i32
     _chk(fn(_f(out), _f(x), x.numel(), scale, _st()), "sum_scale")
 
 
 def zero_(x):
     fn = lib().mlb_zero
-    fn.argtypes = [_vp, C.c_long, _vp]
-    fn.restype = _i32
     assert x.is_cuda and x.is_contiguous()
     _chk(fn(x.data_ptr(), x.numel() * x.element_size(), _st()), "zero")
     global LAUNCHES

@@ -940,3 +940,22 @@ def test_linear_bias_dw_cast(M, N, K):
     assert _rel(out, x.double() @ W.double().T + b.double()) < 2 ** -8      # twice rounded where the epilogue does not take the shape
     nat().linear_dw_cast(dW, d, x)
     assert _rel(dW, d.double().T @ x.double()) < 2 ** -9
+
+
+def test_first_call_of_a_thread_may_be_a_product():
+    """A worker thread whose memory comes out of the allocator's cache has no context bound when it asks for a tensor map."""
+    import threading
+    x, W, out = rnd(136, 72), rnd(200, 72), rnd(136, 200)
+    torch.cuda.synchronize()
+    errs = []
+
+    def work():
+        try:
+            nat().linear_fwd(out, x, W)
+        except Exception as e:      # noqa: BLE001
+            errs.append(e)
+    t = threading.Thread(target=work)
+    t.start()
+    t.join()
+    assert not errs, errs
+    assert _rel(out, x.double() @ W.double().T) < 2 ** -9
