@@ -269,8 +269,8 @@ __global__ void __launch_bounds__(256) layernorm_bwd_k(bf16* __restrict__ dx, fl
 // by whichever blocks finish last (see the end of the kernel).  Scratch: `partial` = (gridDim.x + RMS_GROUPS) * C
 // floats, `ticket` = 1 + RMS_GROUPS ints that are 0 on entry and left 0 on exit.
 constexpr int RMS_GROUPS = 16;
-template <int VPL>  // VPL = C / 256 (vectors of 8 per lane); 0 = generic C (scalar path)
-__global__ void __launch_bounds__(256, (VPL <= 3) ? 2 : 1) rmsnorm_bwd_k(bf16* __restrict__ dx, float* __restrict__ dw, const bf16* __restrict__ dy,
+template <int VPL>  // VPL = C / 256 (vectors of 8 per lane) up to 3; 0 = generic C (scalar path)
+__global__ void __launch_bounds__(256, 2) rmsnorm_bwd_k(bf16* __restrict__ dx, float* __restrict__ dw, const bf16* __restrict__ dy,
                                                      const bf16* __restrict__ x, const bf16* __restrict__ w,
                                                      const float* __restrict__ rstd, const bf16* __restrict__ add, long rows,
                                                      int C, float* __restrict__ partial, int* __restrict__ ticket) {
@@ -283,9 +283,7 @@ __global__ void __launch_bounds__(256, (VPL <= 3) ? 2 : 1) rmsnorm_bwd_k(bf16* _
   const float invC = 1.f / (float)C;
   if (VPL > 0) {
     constexpr int NV = VPL > 0 ? VPL : 1;
-    constexpr bool CACHE = NV <= 4;    // x / dy of the row stay in registers between the two passes (wider rows re-read them from L1)
-    constexpr bool CACHE_W = NV <= 2;  // the weight vector too (two resident blocks per SM leave 128 registers per thread)
-    constexpr int NC = CACHE ? NV : 1;
+    constexpr bool CACHE_W = NV <= 2;  // the weight vector stays in registers (two resident blocks per SM leave 128 per thread)
     constexpr int NW = CACHE_W ? NV : 1;
     float acc[NV][8];
     float ww[NW][8];
@@ -300,19 +298,19 @@ __global__ void __launch_bounds__(256, (VPL <= 3) ? 2 : 1) rmsnorm_bwd_k(bf16* _
       // The row's x, dy and residual-stream gradient stay in registers PACKED (four registers per eight values) between
       // the two passes, and every load of the row is issued before the row's reduction: `add` does not depend on it, and
       // fetching it only afterwards cost a second DRAM round trip per row.
-      uint4 xr[NC], dr[NC], ar[NC];
+      uint4 xr[NV], dr[NV], ar[NV];
       float dot = 0.f;
 #pragma unroll
       for (int v = 0; v < NV; v++) {
         const long off = row * C + (v * 32 + lane) * 8;
-        const int cv = CACHE ? v : 0, cw = CACHE_W ? v : 0;
-        xr[cv] = *reinterpret_cast<const uint4*>(x + off);
-        dr[cv] = *reinterpret_cast<const uint4*>(dy + off);
-        if (CACHE) ar[cv] = add ? *reinterpret_cast<const uint4*>(add + off) : make_uint4(0, 0, 0, 0);
+        const int cw = CACHE_W ? v : 0;
+        xr[v] = *reinterpret_cast<const uint4*>(x + off);
+        dr[v] = *reinterpret_cast<const uint4*>(dy + off);
+        ar[v] = add ? *reinterpret_cast<const uint4*>(add + off) : make_uint4(0, 0, 0, 0);
         if (!CACHE_W) load8(w + (v * 32 + lane) * 8, ww[0]);
         float xf[8], df[8];
-        unpack8(xr[cv], xf);
-        unpack8(dr[cv], df);
+        unpack8(xr[v], xf);
+        unpack8(dr[v], df);
 #pragma unroll
         for (int j = 0; j < 8; j++) dot += df[j] * ww[cw][j] * xf[j];
       }
@@ -321,17 +319,12 @@ __global__ void __launch_bounds__(256, (VPL <= 3) ? 2 : 1) rmsnorm_bwd_k(bf16* _
 #pragma unroll
       for (int v = 0; v < NV; v++) {
         const long off = row * C + (v * 32 + lane) * 8;
-        const int cv = CACHE ? v : 0, cw = CACHE_W ? v : 0;
-        if (!CACHE) {
-          xr[0] = *reinterpret_cast<const uint4*>(x + off);
-          dr[0] = *reinterpret_cast<const uint4*>(dy + off);
-          ar[0] = add ? *reinterpret_cast<const uint4*>(add + off) : make_uint4(0, 0, 0, 0);
-        }
+        const int cw = CACHE_W ? v : 0;
         if (!CACHE_W) load8(w + (v * 32 + lane) * 8, ww[0]);
         float xf[8], df[8], o[8];
-        unpack8(xr[cv], xf);
-        unpack8(dr[cv], df);
-        unpack8(ar[cv], o);
+        unpack8(xr[v], xf);
+        unpack8(dr[v], df);
+        unpack8(ar[v], o);
 #pragma unroll
         for (int j = 0; j < 8; j++) {
           o[j] += df[j] * ww[cw][j] * r - xf[j] * k;
@@ -431,6 +424,164 @@ __global__ void __launch_bounds__(256, (VPL <= 3) ? 2 : 1) rmsnorm_bwd_k(bf16* _
     }
   }
   if (threadIdx.x == 0) ticket[0] = 0;
+}
+
+// ------------------------------------------------------------------ column sums in two launches, deterministic
+// Norm backward over whole rows per thread group: C / 8 threads share a row, each owning 8 columns for all of the group's rows, so the
+// column sums (dw, and db of LayerNorm) stay in 8 (16) registers and need no folding over a warp's rows.  Three rows at a time:
+// their 6-9 16-byte loads are in flight together and their dots cost one barrier.  One warp per row (rmsnorm_bwd_k)
+// needs C / 4 accumulators per lane, which at C = 2048 spill: 84 us for 16384 rows, 2.4 TB/s.
+// Partial sums: partial[block][C (RMS) | 2 C (LN: dw, db)], added up by fold_cols_k.
+// Shapes: C % 256 == 0 and C <= 2048 (whole warps, at most 256 threads a row).
+constexpr int NB_ROWS = 3;
+template <bool LN>
+__global__ void __launch_bounds__(256, 2) norm_bwd_rows_k(bf16* __restrict__ dx, const bf16* __restrict__ dy, const bf16* __restrict__ x,
+                                                          const bf16* __restrict__ w, const float* __restrict__ mean,
+                                                          const float* __restrict__ rstd, const bf16* __restrict__ add, long rows, int C,
+                                                          float* __restrict__ partial) {
+  mlb_pdl_sync();
+  __shared__ float red[2][NB_ROWS][2][8];
+  __shared__ float fold[2048];
+  const int gt = C >> 3, G = blockDim.x / gt, grp = threadIdx.x / gt, t = threadIdx.x % gt;      // group = the threads of one row
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, w0 = grp * (gt >> 5), nw = gt >> 5;
+  float aw[8], ab[8];
+  const uint4 wr = *reinterpret_cast<const uint4*>(w + t * 8);
+#pragma unroll
+  for (int j = 0; j < 8; j++) aw[j] = ab[j] = 0.f;
+  const float invC = 1.f / (float)C;
+  int buf = 0;
+  for (long base = ((long)blockIdx.x * G + grp) * NB_ROWS; base < rows; base += (long)gridDim.x * G * NB_ROWS, buf ^= 1) {
+    uint4 xr[NB_ROWS], dr[NB_ROWS], ar[NB_ROWS];
+    float mu[NB_ROWS], rs[NB_ROWS];
+#pragma unroll
+    for (int k = 0; k < NB_ROWS; k++) {
+      const bool live = base + k < rows;
+      const size_t off = (size_t)(live ? base + k : base) * C + t * 8;
+      xr[k] = *reinterpret_cast<const uint4*>(x + off);
+      dr[k] = live ? *reinterpret_cast<const uint4*>(dy + off) : make_uint4(0, 0, 0, 0);      // a row past the end adds nothing
+      if (!LN) ar[k] = add ? *reinterpret_cast<const uint4*>(add + off) : make_uint4(0, 0, 0, 0);
+      rs[k] = rstd[live ? base + k : base];
+      if (LN) mu[k] = mean[live ? base + k : base];
+    }
+#pragma unroll
+    for (int k = 0; k < NB_ROWS; k++) {
+      float xf[8], df[8], ww[8], s = 0.f, sx = 0.f;
+      unpack8(wr, ww);
+      unpack8(xr[k], xf);
+      unpack8(dr[k], df);
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        const float g = df[j] * ww[j];
+        if (LN) { s += g; sx += g * ((xf[j] - mu[k]) * rs[k]); }
+        else sx += g * xf[j];
+      }
+      sx = warp_sum(sx);
+      if (LN) s = warp_sum(s);
+      if (lane == 0) {
+        red[buf][k][0][warp] = sx;
+        if (LN) red[buf][k][1][warp] = s;
+      }
+    }
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "r"(gt) : "memory");      // (two buffers: one barrier per round is enough)
+#pragma unroll
+    for (int k = 0; k < NB_ROWS; k++) {
+      if (base + k >= rows) break;
+      float s = 0.f, sx = 0.f;
+      for (int i = 0; i < nw; i++) {
+        sx += red[buf][k][0][w0 + i];
+        if (LN) s += red[buf][k][1][w0 + i];
+      }
+      float xf[8], df[8], ww[8], o[8];
+      unpack8(wr, ww);
+      unpack8(xr[k], xf);
+      unpack8(dr[k], df);
+      const float r = rs[k];
+      if (LN) {
+        s *= invC;
+        sx *= invC;
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          const float xh = (xf[j] - mu[k]) * r;
+          o[j] = r * (df[j] * ww[j] - s - xh * sx);
+          aw[j] += df[j] * xh;
+          ab[j] += df[j];
+        }
+      } else {
+        const float kk = r * r * r * invC * sx;
+        unpack8(ar[k], o);
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          o[j] += df[j] * ww[j] * r - xf[j] * kk;
+          aw[j] += df[j] * xf[j] * r;
+        }
+      }
+      store8(dx + (size_t)(base + k) * C + t * 8, o);
+    }
+  }
+  // the block's groups in order
+  float* out = partial + (size_t)blockIdx.x * (LN ? 2 * C : C);
+#pragma unroll
+  for (int half = 0; half < (LN ? 2 : 1); half++) {
+    const float* acc = half ? ab : aw;
+    for (int g = 0; g < G; g++) {
+      if (grp == g) {
+#pragma unroll
+        for (int j = 0; j < 8; j++) fold[t * 8 + j] = acc[j] + (g ? fold[t * 8 + j] : 0.f);
+      }
+      __syncthreads();
+    }
+    for (int i = threadIdx.x; i < C; i += blockDim.x) out[half * C + i] = fold[i];
+    __syncthreads();
+  }
+}
+// partial[split][N]: column sums of x[M, N] over the split's rows; a warp takes 256 columns of every 8th row
+__global__ void __launch_bounds__(256) colsum_k(float* __restrict__ partial, const bf16* __restrict__ x, long M, int N) {
+  mlb_pdl_sync();
+  __shared__ float red[8][256];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = (blockIdx.x * 32 + lane) * 8;
+  const long per = (M + gridDim.y - 1) / gridDim.y, r0 = per * blockIdx.y, r1 = min(M, r0 + per);
+  float a[8] = {};
+  if (c < N) {
+#pragma unroll 4
+    for (long r = r0 + warp; r < r1; r += 8) {
+      float f[8];
+      load8(x + (size_t)r * N + c, f);
+#pragma unroll
+      for (int j = 0; j < 8; j++) a[j] += f[j];
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 8; j++) red[warp][lane * 8 + j] = a[j];
+  __syncthreads();
+  const int col = blockIdx.x * 256 + threadIdx.x;
+  if (col >= N) return;
+  float s = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; i++) s += red[i][threadIdx.x];
+  partial[(size_t)blockIdx.y * N + col] = s;
+}
+// The partial rows added up in a fixed order: columns [0, C) to dw, [C, W) to db (either may be null).  bf16: rounded and stored;
+// fp32: added to what is there.  A block takes 32 columns, 8 row slices.
+template <bool BF>
+__global__ void __launch_bounds__(256) fold_cols_k(void* __restrict__ dw, void* __restrict__ db, const float* __restrict__ partial, int nrows, int C, int W) {
+  mlb_pdl_sync();
+  __shared__ float red[8][32];
+  const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
+  float s = 0.f;
+  if (c < W) {
+#pragma unroll 8
+    for (int r = sl; r < nrows; r += 8) s += partial[(size_t)r * W + c];
+  }
+  red[sl][lane] = s;
+  __syncthreads();
+  if (sl != 0 || c >= W) return;
+#pragma unroll
+  for (int i = 1; i < 8; i++) s += red[i][lane];
+  void* dst = c < C ? dw : db;
+  if (dst == nullptr) return;
+  const int i = c < C ? c : c - C;
+  if (BF) ((bf16*)dst)[i] = __float2bfloat16(s);
+  else ((float*)dst)[i] += s;
 }
 
 // ------------------------------------------------------------------ RoPE (in place on the Q and K slices of qkv[B*T, 3C])
@@ -1197,6 +1348,46 @@ MLB_API int mlb_rmsnorm_bwd_blocks(long rows) {
   long b = (rows + 7) / 8;
   return (int)(b < 296 ? b : 296);
 }
+// Norm backward with the column sums in `partial` (mlb_rmsnorm_bwd_blocks(rows) rows of C floats, 2 C for LayerNorm, contents do not
+// matter) and then dw (and db): bf16 and overwritten, or fp32 and added to.  -7: not a shape of these kernels.
+static bool norm_rows_ok(const void* dx, const void* dy, const void* x, const void* w, const void* add, long rows, int C) {
+  return rows > 0 && C % 256 == 0 && C <= 2048 &&
+         (((uintptr_t)dx | (uintptr_t)dy | (uintptr_t)x | (uintptr_t)w | (uintptr_t)add) & 15) == 0;
+}
+template <bool LN>
+static void norm_rows_launch(void* dx, void* dw, void* db, bool bf, const void* dy, const void* x, const void* w, const float* mean, const float* rstd,
+                             const void* add, long rows, int C, float* partial, cudaStream_t st) {
+  const int blocks = mlb_rmsnorm_bwd_blocks(rows), gt = C / 8, W = LN ? 2 * C : C;
+  mlb_launch(norm_bwd_rows_k<LN>, dim3(blocks), dim3(256 / gt * gt), 0, st, (bf16*)dx, (const bf16*)dy, (const bf16*)x, (const bf16*)w, mean, rstd,
+             (const bf16*)add, rows, C, partial);
+  if (bf) mlb_launch(fold_cols_k<true>, dim3((W + 31) / 32), dim3(256), 0, st, dw, db, (const float*)partial, blocks, C, W);
+  else mlb_launch(fold_cols_k<false>, dim3((W + 31) / 32), dim3(256), 0, st, dw, db, (const float*)partial, blocks, C, W);
+}
+MLB_API int mlb_rmsnorm_bwd_cast(void* dx, void* dw, const void* dy, const void* x, const void* w, const float* rstd, const void* add, long rows, int C,
+                                 float* partial, cudaStream_t st) {
+  if (!norm_rows_ok(dx, dy, x, w, add, rows, C)) return -7;
+  norm_rows_launch<false>(dx, dw, nullptr, true, dy, x, w, nullptr, rstd, add, rows, C, partial, st);
+  LAUNCH_RET;
+}
+MLB_API int mlb_layernorm_bwd2(void* dx, void* dw, void* db, int bf, const void* dy, const void* x, const void* w, const float* mean, const float* rstd,
+                               long rows, int C, float* partial, cudaStream_t st) {
+  if (!norm_rows_ok(dx, dy, x, w, nullptr, rows, C)) return -7;
+  norm_rows_launch<true>(dx, dw, db, bf != 0, dy, x, w, mean, rstd, nullptr, rows, C, partial, st);
+  LAUNCH_RET;
+}
+// Splits of the rows colsum_k works with: enough blocks to fill the machine twice, at least 32 rows each
+MLB_API int mlb_colsum_splits(long M, int N) {
+  const long cols = (N + 255) / 256, want = (296 + cols - 1) / cols, most = (M + 31) / 32;
+  return (int)(want < most ? want : (most < 1 ? 1 : most));
+}
+// out[N] (bf16) = column sums of x[M, N], fp32 inside; partial: mlb_colsum_splits(M, N) * N floats
+MLB_API int mlb_colsum(void* out, const void* x, long M, int N, float* partial, cudaStream_t st) {
+  if (M <= 0 || N <= 0 || N % 8 != 0 || ((uintptr_t)x & 15)) return -7;
+  const int S = mlb_colsum_splits(M, N);
+  mlb_launch(colsum_k, dim3((N + 255) / 256, S), dim3(256), 0, st, partial, (const bf16*)x, M, N);
+  mlb_launch(fold_cols_k<true>, dim3((N + 31) / 32), dim3(256), 0, st, out, (void*)nullptr, (const float*)partial, S, N, N);
+  LAUNCH_RET;
+}
 MLB_API int mlb_rmsnorm_bwd(void* dx, float* dw, const void* dy, const void* x, const void* w, const float* rstd, const void* add,
                             long rows, int C, float* partial, int* ticket, cudaStream_t st) {
   const int blocks = mlb_rmsnorm_bwd_blocks(rows);
@@ -1205,13 +1396,14 @@ MLB_API int mlb_rmsnorm_bwd(void* dx, float* dw, const void* dy, const void* x, 
   mlb_launch(rmsnorm_bwd_k<V>, dim3(blocks), dim3(256), sh, st, (bf16*)dx, dw, (const bf16*)dy, (const bf16*)x, (const bf16*)w, rstd,   \
                                             (const bf16*)add, rows, C, partial, ticket)
   if (sh > 48 * 1024) return -3;
+  if (C >= 1024 && norm_rows_ok(dx, dy, x, w, add, rows, C)) {      // (narrower rows fit a warp's registers, and one launch)
+    norm_rows_launch<false>(dx, dw, nullptr, false, dy, x, w, nullptr, rstd, add, rows, C, partial, st);
+    LAUNCH_RET;
+  }
   switch ((C % 256 == 0) ? C / 256 : 0) {
     case 1: RB(1); break;
     case 2: RB(2); break;
     case 3: RB(3); break;
-    case 4: RB(4); break;
-    case 6: RB(6); break;
-    case 8: RB(8); break;
     default: RB(0); break;
   }
 #undef RB

@@ -9,10 +9,10 @@ from . import ref
 
 _NAMES = [
     "embed_fwd", "embed_bwd", "set_prefix", "gather_prefix_grad",
-    "rmsnorm_fwd", "add_rmsnorm_fwd", "rmsnorm_bwd",
+    "rmsnorm_fwd", "add_rmsnorm_fwd", "rmsnorm_bwd", "rmsnorm_bwd_cast", "colsum",
     "rope_fwd", "rope_copy", "kv_group_sum", "rope_bwd", "swiglu_fwd", "swiglu_bwd",
     "linear_fwd", "linear_bias_fwd", "linear_dx", "linear_dw", "linear_dw_cast", "gemm", "attn_fwd", "attn_bwd",
-    "attn_bidir_fwd", "attn_bidir_bwd", "layernorm_fwd", "layernorm_bwd",
+    "attn_bidir_fwd", "attn_bidir_bwd", "layernorm_fwd", "layernorm_bwd", "layernorm_bwd_cast",
     "ce_fwd_bwd", "ce_mean", "scale_dev", "ce_chunk_stats", "ce_chunk_grad", "adamw", "patchify", "add_posembed", "posembed_grad", "residual_add", "cast", "fp8_qdq", "sum_scale", "zero_",
 ]
 

@@ -14,7 +14,7 @@ from .. import ops
 
 
 def _like(x, *shape, dtype=None):
-    return torch.empty(*shape, dtype=dtype or x.dtype, device=x.device)
+    return x.new_empty(*shape) if dtype is None else x.new_empty(*shape, dtype=dtype)
 
 
 class Linear(torch.autograd.Function):
@@ -39,7 +39,11 @@ class Linear(torch.autograd.Function):
         ops.linear_dx(dx, dout, W.contiguous())
         dW = _like(W, *W.shape)
         ops.linear_dw_cast(dW, dout, x.contiguous())
-        return dx, dW, (None if ctx.bias is None else dout.sum(0).to(ctx.bias))
+        db = None
+        if ctx.bias is not None:
+            db = _like(dout, dout.shape[1], dtype=ctx.bias)
+            ops.colsum(db, dout)
+        return dx, dW, db
 
 
 class RMSNorm(torch.autograd.Function):
@@ -54,10 +58,9 @@ class RMSNorm(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x, w, rstd = ctx.saved_tensors
-        dx = _like(x, *x.shape)
-        dw = torch.zeros(w.shape, dtype=torch.float32, device=w.device)
-        ops.rmsnorm_bwd(dx, dw, dy.contiguous(), x.contiguous(), w, rstd, None)
-        return dx, dw.to(w.dtype), None
+        dx, dw = _like(x, *x.shape), _like(w, *w.shape)
+        ops.rmsnorm_bwd_cast(dx, dw, dy.contiguous(), x.contiguous(), w, rstd)
+        return dx, dw, None
 
 
 class SwiGLU(torch.autograd.Function):
@@ -148,11 +151,10 @@ class LayerNorm(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x, w, mean, rstd = ctx.saved_tensors
-        dx = _like(x, *x.shape)
-        dw = torch.zeros(w.shape, dtype=torch.float32, device=w.device)
-        db = torch.zeros(w.shape, dtype=torch.float32, device=w.device) if ctx.has_b else None
-        ops.layernorm_bwd(dx, dw, db, dy.contiguous(), x, w, mean, rstd)
-        return dx, dw.to(w.dtype), (db.to(w.dtype) if db is not None else None), None
+        dx, dw = _like(x, *x.shape), _like(w, *w.shape)
+        db = _like(w, *w.shape) if ctx.has_b else None
+        ops.layernorm_bwd_cast(dx, dw, db, dy.contiguous(), x, w, mean, rstd)
+        return dx, dw, db, None
 
 
 class CrossEntropy(torch.autograd.Function):

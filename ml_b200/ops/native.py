@@ -57,6 +57,10 @@ def lib():
         "mlb_rmsnorm_bwd_blocks": [_i64],
         "mlb_rmsnorm_bwd": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i32, _vp, _vp, _vp],
         "mlb_rope": [_vp, _vp, _vp, _i64, _i32, _i32, _i32, _f32, _vp],
+        "mlb_rmsnorm_bwd_cast": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i32, _vp, _vp],
+        "mlb_layernorm_bwd2": [_vp, _vp, _vp, _i32, _vp, _vp, _vp, _vp, _vp, _i64, _i32, _vp, _vp],
+        "mlb_colsum_splits": [_i64, _i32],
+        "mlb_colsum": [_vp, _vp, _i64, _i32, _vp, _vp],
         "mlb_rope_copy": [_vp, _vp, _vp, _vp, _i64, _i32, _i32, _i32, _i32, _vp],
         "mlb_kv_group_sum": [_vp, _vp, _i64, _i32, _i32, _i32, _vp],
         "mlb_swiglu_fwd": [_vp, _vp, _i64, _i32, _vp],
@@ -441,10 +445,63 @@ def layernorm_fwd(out, mean, rstd, x, w, b, eps):
     _chk(fn(_b(out), _f(mean), _f(rstd), _b(x), _b(w), _b(b) if b is not None else None, rows, Cc, eps, _st()), "layernorm_fwd")
 
 
+def _partial(numel, device):
+    # of the caching allocator, per call: calls on different streams do not share it
+    return torch.empty(numel, dtype=torch.float32, device=device)
+
+
 def layernorm_bwd(dx, dw, db, dy, x, w, mean, rstd):
     rows, Cc = x.shape
-    fn = lib().mlb_layernorm_bwd
-    _chk(fn(_b(dx), _f(dw), _f(db) if db is not None else None, _b(dy), _b(x), _b(w), _f(mean), _f(rstd), rows, Cc, _st()), "layernorm_bwd")
+    L = lib()
+    part = _partial(L.mlb_rmsnorm_bwd_blocks(rows) * 2 * Cc, x.device)
+    d = _f(db) if db is not None else None
+    rc = L.mlb_layernorm_bwd2(_b(dx), _f(dw), d, 0, _b(dy), _b(x), _b(w), _f(mean), _f(rstd), rows, Cc, part.data_ptr(), _st())
+    if rc == -7:      # a width those kernels do not take
+        rc = L.mlb_layernorm_bwd(_b(dx), _f(dw), d, _b(dy), _b(x), _b(w), _f(mean), _f(rstd), rows, Cc, _st())
+    _chk(rc, "layernorm_bwd")
+
+
+def layernorm_bwd_cast(dx, dw, db, dy, x, w, mean, rstd):
+    """layernorm_bwd with dw (and db) in bf16, overwritten."""
+    rows, Cc = x.shape
+    L = lib()
+    part = _partial(L.mlb_rmsnorm_bwd_blocks(rows) * 2 * Cc, x.device)
+    rc = L.mlb_layernorm_bwd2(_b(dx), _b(dw), _b(db) if db is not None else None, 1, _b(dy), _b(x), _b(w), _f(mean), _f(rstd), rows, Cc,
+                              part.data_ptr(), _st())
+    if rc == -7:
+        aw, ab = torch.zeros_like(dw, dtype=torch.float32), torch.zeros_like(dw, dtype=torch.float32)
+        layernorm_bwd(dx, aw, ab, dy, x, w, mean, rstd)
+        dw.copy_(aw)
+        if db is not None:
+            db.copy_(ab)
+        return
+    _chk(rc, "layernorm_bwd_cast")
+
+
+def rmsnorm_bwd_cast(dx, dw, dy, x, w, rstd, add=None):
+    """rmsnorm_bwd with dw in bf16, overwritten."""
+    rows, Cc = x.shape
+    L = lib()
+    part = _partial(L.mlb_rmsnorm_bwd_blocks(rows) * Cc, x.device)
+    rc = L.mlb_rmsnorm_bwd_cast(_b(dx), _b(dw), _b(dy), _b(x), _b(w), _f(rstd), _b(add) if add is not None else None, rows, Cc, part.data_ptr(), _st())
+    if rc == -7:
+        acc = torch.zeros_like(dw, dtype=torch.float32)
+        rmsnorm_bwd(dx, acc, dy, x, w, rstd, add)
+        dw.copy_(acc)
+        return
+    _chk(rc, "rmsnorm_bwd_cast")
+
+
+def colsum(out, x):
+    """out[N] (bf16) = sum of x[M, N] over its rows, in fp32."""
+    M, N = x.shape
+    L = lib()
+    part = _partial(L.mlb_colsum_splits(M, N) * N, x.device)
+    rc = L.mlb_colsum(_b(out), _b(x), M, N, part.data_ptr(), _st())
+    if rc == -7:
+        out.copy_(x.sum(0))
+        return
+    _chk(rc, "colsum")
 
 
 def rmsnorm_bwd(dx, dw, dy, x, w, rstd, add=None):

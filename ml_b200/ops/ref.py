@@ -265,6 +265,27 @@ def layernorm_bwd(dx, dw, db, dy, x, w, mean, rstd):
         db.add_(_f(dy).sum(0))
 
 
+def layernorm_bwd_cast(dx, dw, db, dy, x, w, mean, rstd):
+    """layernorm_bwd with dw (and db) overwritten, in their own dtype."""
+    aw, ab = torch.zeros_like(dw, dtype=torch.float32), torch.zeros_like(dw, dtype=torch.float32)
+    layernorm_bwd(dx, aw, ab, dy, x, w, mean, rstd)
+    dw.copy_(aw)
+    if db is not None:
+        db.copy_(ab)
+
+
+def rmsnorm_bwd_cast(dx, dw, dy, x, w, rstd, add=None):
+    """rmsnorm_bwd with dw overwritten, in its own dtype."""
+    acc = torch.zeros_like(dw, dtype=torch.float32)
+    rmsnorm_bwd(dx, acc, dy, x, w, rstd, add)
+    dw.copy_(acc)
+
+
+def colsum(out, x):
+    """out[N] = sum of x[M, N] over its rows, in fp32."""
+    out.copy_(_f(x).sum(0))
+
+
 # ------------------------------------------------------------------ cross entropy
 def ce_fwd_bwd(losses, logits, tgt, dscale, V_valid=None):
     """Fused CE: losses[row] = logsumexp(z) - z[tgt]; logits are overwritten IN PLACE with

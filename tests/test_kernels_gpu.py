@@ -959,3 +959,32 @@ def test_first_call_of_a_thread_may_be_a_product():
     t.join()
     assert not errs, errs
     assert _rel(out, x.double() @ W.double().T) < 2 ** -9
+
+
+@pytest.mark.parametrize("M,N", [(1, 8), (64, 96), (200, 264), (1003, 768), (3000, 2304), (50, 1024)])
+def test_colsum(M, N):
+    torch.manual_seed(M)
+    d, db = rnd(M, N), rnd(N)
+    nat().colsum(db, d)
+    assert _rel(db, d.double().sum(0)) < 2 ** -8
+
+
+@pytest.mark.parametrize("rows,C", [(1, 256), (7, 768), (100, 1024), (37, 1536), (1000, 2048), (9, 100)])
+def test_norm_backward_with_cast_column_sums(rows, C):
+    torch.manual_seed(rows)
+    x, dy, add, w, b = rnd(rows, C), rnd(rows, C), rnd(rows, C), 1 + rnd(C, scale=0.1), rnd(C)
+    o, mean, rstd, dx, dw, db = torch.empty_like(x), *(torch.empty(rows, device=dev()) for _ in range(2)), torch.empty_like(x), rnd(C), rnd(C)
+    xd, wd, bd = (t.double().requires_grad_(True) for t in (x, w, b))
+    nat().rmsnorm_fwd(o, rstd, x, w, 1e-5)
+    nat().rmsnorm_bwd_cast(dx, dw, dy, x, w, rstd, add)
+    y = xd * torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + 1e-5) * wd
+    gx, gw = torch.autograd.grad(y, [xd, wd], dy.double())
+    assert _rel(dx, gx + add.double()) < 2 ** -8 and _rel(dw, gw) < 2 ** -8
+    acc = torch.ones(C, device=dev())
+    nat().rmsnorm_bwd(dx, acc, dy, x, w, rstd, None)
+    assert _rel(dx, gx) < 2 ** -8 and _rel(acc - 1, gw) < 1e-4
+    nat().layernorm_fwd(o, mean, rstd, x, w, b, 1e-5)
+    nat().layernorm_bwd_cast(dx, dw, db, dy, x, w, mean, rstd)
+    y = torch.nn.functional.layer_norm(xd, (C,), wd, bd, 1e-5)
+    gx, gw, gb = torch.autograd.grad(y, [xd, wd, bd], dy.double())
+    assert _rel(dx, gx) < 2 ** -8 and _rel(dw, gw) < 2 ** -8 and _rel(db, gb) < 2 ** -8
