@@ -5,12 +5,8 @@
 // window), writes O into atty[B,T,C], saves the per-row log-sum-exp, and in backward writes dQ, dK, dV strided into
 // dqkv[B,T,3C].  Scale 1/sqrt(hd), causal over the whole sequence, no dropout.
 //
-// Forward, one CTA (128 threads) per 128-query tile: S = Q K^T by tcgen05.mma into TMEM, each thread owns one query
-// row (TMEM lane) for the online softmax, P is written bf16 into 128B-swizzled shared memory and fed back as the A
-// operand of O_blk = P V (V consumed MN-major, i.e. untransposed), O is rescaled in registers.
-// Backward, two kernels that each own their accumulators in TMEM (no atomics, deterministic):
-//   dK/dV kernel per 128-key tile:  S^T = K Q^T, dP^T = V dO^T, P^T and dS^T to shared memory, dV += P^T dO, dK += dS^T Q.
-//   dQ kernel per 128-query tile:   S = Q K^T, dP = dO V^T, dS to shared memory, dQ += dS K.
+// Head size 64 is in this file (thread-per-row forward, one fused backward kernel, and the older forms they replaced, which remain as
+// options), head size 128 in attn_hd128.cuh.  All accumulators live in TMEM (no atomics, deterministic).
 // RoPE's backward rotation of dQ/dK can be applied in the epilogue (each thread holds a full head row).
 // Bidirectional attention and the other head sizes that are multiples of 16: attn_split.cuh.  What is left (odd head sizes,
 // unaligned pointers) uses a plain SIMT implementation further down.
@@ -111,15 +107,11 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   return r;
 }
 
-template <int HD>
 struct FwdSmem {
-  static constexpr int CH = HD / 64;
-  static constexpr int VBUF = (HD == 64) ? 2 : 1;
-  static constexpr int QBUF = (HD == 64) ? 2 : 1;
-  static constexpr int Q = 0;                                   // QBUF buffers
-  static constexpr int K = Q + QBUF * CH * TILE_BYTES;          // 2 slots
-  static constexpr int V = K + 2 * CH * TILE_BYTES;             // VBUF slots
-  static constexpr int P = V + VBUF * CH * TILE_BYTES;          // 2 buffers x [128 x 128] bf16
+  static constexpr int Q = 0;                                   // 2 buffers
+  static constexpr int K = Q + 2 * TILE_BYTES;                  // 2 slots
+  static constexpr int V = K + 2 * TILE_BYTES;                  // 2 slots
+  static constexpr int P = V + 2 * TILE_BYTES;                  // 2 buffers x [128 x 128] bf16
   static constexpr int RED = P + 2 * 2 * TILE_BYTES;            // 3 x 4 x 128 floats: per-quarter row maxima (x2) / sums
   static constexpr int BAR = RED + 6144;
   static constexpr int TOTAL = BAR + 256 + 1024;
@@ -151,10 +143,9 @@ struct FwdCursor {   // position of one key block in the flattened (item, block)
   }
 };
 
-template <int HD>
 __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm, const AttnArgs a) {
-  using S = FwdSmem<HD>;
-  constexpr int CH = HD / 64, OC = HD / 4, VBUF = S::VBUF, QBUF = S::QBUF;
+  using S = FwdSmem;
+  constexpr int HD = 64, OC = HD / 4;
   constexpr uint32_t TMEM_COLS = 512;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -201,31 +192,28 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_tc_kernel(const __gri
   if (warp == ATT_SOFTMAX_WARPS) {
     // ---------------------------------------------------------------- control warp
     // Everything is indexed by g, the running number of the key block in this CTA's flattened sequence:
-    // K slot / score buffer / P buffer / O buffer = g & 1, V slot = g % VBUF, Q buffer = (local item number) % QBUF.
+    // K and V slot / score buffer / P buffer / O buffer = g & 1, Q buffer = (local item number) & 1.
     if (lane == 0) {
       constexpr uint32_t idesc_s = tc::idesc_bf16(128, 128, 0, 0);
       constexpr uint32_t idesc_o = tc::idesc_bf16(128, HD, 0, 1);
       auto load_q = [&](const FwdItem& it) {
-        const int qb = it.li % QBUF;
-        tc::mbar_expect_tx(&bar_q[qb], CH * TILE_BYTES);
-        for (int c = 0; c < CH; c++)
-          tc::tma_load_2d(smem + S::Q + (qb * CH + c) * TILE_BYTES, &tm, &bar_q[qb], it.h * HD + c * 64, it.b * a.T + it.qt * 128);
+        const int qb = it.li & 1;
+        tc::mbar_expect_tx(&bar_q[qb], TILE_BYTES);
+        tc::tma_load_2d(smem + S::Q + qb * TILE_BYTES, &tm, &bar_q[qb], it.h * HD, it.b * a.T + it.qt * 128);
       };
       auto load_k = [&](const FwdCursor& c, int g) {
         const int sl = g & 1;
-        tc::mbar_expect_tx(&bar_k[sl], CH * TILE_BYTES);
-        for (int x = 0; x < CH; x++)
-          tc::tma_load_2d(smem + S::K + (sl * CH + x) * TILE_BYTES, &tm, &bar_k[sl], C + c.it.h * HD + x * 64, c.it.b * a.T + c.j * 128);
+        tc::mbar_expect_tx(&bar_k[sl], TILE_BYTES);
+        tc::tma_load_2d(smem + S::K + sl * TILE_BYTES, &tm, &bar_k[sl], C + c.it.h * HD, c.it.b * a.T + c.j * 128);
       };
       auto load_v = [&](const FwdCursor& c, int g) {
-        const int sl = g % VBUF;
-        tc::mbar_expect_tx(&bar_v[sl], CH * TILE_BYTES);
-        for (int x = 0; x < CH; x++)
-          tc::tma_load_2d(smem + S::V + (sl * CH + x) * TILE_BYTES, &tm, &bar_v[sl], 2 * C + c.it.h * HD + x * 64, c.it.b * a.T + c.j * 128);
+        const int sl = g & 1;
+        tc::mbar_expect_tx(&bar_v[sl], TILE_BYTES);
+        tc::tma_load_2d(smem + S::V + sl * TILE_BYTES, &tm, &bar_v[sl], 2 * C + c.it.h * HD, c.it.b * a.T + c.j * 128);
       };
       auto issue_s = [&](const FwdCursor& c, int g) {   // S(g) = Q K^T into score buffer g & 1
-        const uint32_t sQ = tc::smem_u32(smem + S::Q + (c.it.li % QBUF) * CH * TILE_BYTES);
-        const uint32_t sK = tc::smem_u32(smem + S::K + (g & 1) * CH * TILE_BYTES);
+        const uint32_t sQ = tc::smem_u32(smem + S::Q + (c.it.li & 1) * TILE_BYTES);
+        const uint32_t sK = tc::smem_u32(smem + S::K + (g & 1) * TILE_BYTES);
 #pragma unroll
         for (int ks = 0; ks < HD / 16; ks++) tc::mma_bf16_ss(tmem + (g & 1) * 128, desc_k(sQ, ks), desc_k(sK, ks), idesc_s, ks > 0);
       };
@@ -240,25 +228,19 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_tc_kernel(const __gri
       load_v(c0, 0);
       if (c1.it.valid) {
         load_k(c1, 1);
-        if (VBUF == 2) load_v(c1, 1);
-        if (c1.it.li != c0.it.li && QBUF == 2) load_q(c1.it);
+        load_v(c1, 1);
+        if (c1.it.li != c0.it.li) load_q(c1.it);
       }
       if (wait(&bar_q[0], 0, 10) && wait(&bar_k[0], 0, 11)) { tc::tc_fence_after(); issue_s(c0, 0); }
       tc::mma_commit(&bar_s[0]);
       if (c1.it.valid) {
         bool okq = true;
-        if (c1.it.li != c0.it.li) {
-          if (QBUF == 1) {   // single Q buffer: S(0) must be done before the next item's Q may land
-            okq = wait(&bar_s[0], 0, 12);
-            if (okq) load_q(c1.it);
-          }
-          okq = okq && wait(&bar_q[c1.it.li % QBUF], (c1.it.li / QBUF) & 1, 10);
-        }
+        if (c1.it.li != c0.it.li) okq = wait(&bar_q[c1.it.li & 1], (c1.it.li >> 1) & 1, 10);
         if (okq && wait(&bar_k[1], 0, 11)) { tc::tc_fence_after(); issue_s(c1, 1); }
         tc::mma_commit(&bar_s[1]);
       }
       int q_loaded_li = c1.it.valid ? c1.it.li : c0.it.li;   // highest local item whose Q load has been issued
-      if (QBUF == 2) {   // the item after the last loaded one can be prefetched once its buffer is free
+      {   // the item after the last loaded one can be prefetched once its buffer is free
         FwdItem nx;
         nx.set(blockIdx.x + (q_loaded_li + 1) * stride, q_loaded_li + 1, total, nq, BH, a.H);
         if (nx.valid) { pending_q_w = nx.w; pending_q_li = nx.li; }
@@ -269,7 +251,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_tc_kernel(const __gri
         //     prefetch whose buffer was last read by an item that ended at or before g can go out
         const bool s_done = wait(&bar_s[sl], ph, 12);
         if (s_done && c2.it.valid) load_k(c2, g + 2);
-        if (s_done && QBUF == 2 && pending_q_w >= 0 && pending_q_li - 2 < c0.it.li + (c0.j == c0.it.nkb - 1 ? 1 : 0)) {
+        if (s_done && pending_q_w >= 0 && pending_q_li - 2 < c0.it.li + (c0.j == c0.it.nkb - 1 ? 1 : 0)) {
           // buffer (pending_q_li & 1) was used by local item pending_q_li - 2, all of whose blocks are <= g here
           FwdItem nx;
           nx.set(pending_q_w, pending_q_li, total, nq, BH, a.H);
@@ -278,10 +260,10 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_tc_kernel(const __gri
           pending_q_w = -1;
         }
         // (b) P(g) written (and S(g) fully read) -> O_blk(g) = P V
-        if (wait(&bar_p[sl], ph, 13) && wait(&bar_v[g % VBUF], (g / VBUF) & 1, 14)) {
+        if (wait(&bar_p[sl], ph, 13) && wait(&bar_v[sl], ph, 14)) {
           tc::tc_fence_after();
           const uint32_t sP = tc::smem_u32(smem + S::P + sl * 2 * TILE_BYTES);
-          const uint32_t sV = tc::smem_u32(smem + S::V + (g % VBUF) * CH * TILE_BYTES);
+          const uint32_t sV = tc::smem_u32(smem + S::V + sl * TILE_BYTES);
 #pragma unroll
           for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ss(t_o + sl * HD, desc_k(sP, ks), desc_mn(sV, ks), idesc_o, ks > 0);
         }
@@ -291,13 +273,13 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_tc_kernel(const __gri
           bool okq = true;
           if (c2.j == 0) {
             if (c2.it.li > q_loaded_li) {
-              // not prefetched (single Q buffer, or the prefetch condition never became true): the buffer's previous user
+              // not prefetched (the prefetch condition never became true): the buffer's previous user
               // ends at block g+1, whose S was issued in the previous iteration
               okq = wait(&bar_s[(g + 1) & 1], ((g + 1) >> 1) & 1, 12);
               if (okq) { load_q(c2.it); q_loaded_li = c2.it.li; if (pending_q_li == c2.it.li) pending_q_w = -1; }
             }
-            okq = okq && wait(&bar_q[c2.it.li % QBUF], (c2.it.li / QBUF) & 1, 10);
-            if (QBUF == 2 && pending_q_w < 0) {
+            okq = okq && wait(&bar_q[c2.it.li & 1], (c2.it.li >> 1) & 1, 10);
+            if (pending_q_w < 0) {
               FwdItem nx;
               nx.set(c2.it.w + stride, c2.it.li + 1, total, nq, BH, a.H);
               if (nx.valid && nx.li > q_loaded_li) { pending_q_w = nx.w; pending_q_li = nx.li; }
@@ -307,8 +289,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_tc_kernel(const __gri
           tc::mma_commit(&bar_s[sl]);
         }
         // (d) V slot free once P V of block g has completed
-        const FwdCursor& cv = (VBUF == 2) ? c2 : c1;
-        if (cv.it.valid && wait(&bar_o[sl], ph, 16)) load_v(cv, g + VBUF);
+        if (c2.it.valid && wait(&bar_o[sl], ph, 16)) load_v(c2, g + 2);
         c0 = c1; c1 = c2; c2.advance(total, nq, BH, a.H, stride);
       }
     }
@@ -330,19 +311,11 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_tc_kernel(const __gri
 #pragma unroll
       for (int i = 0; i < OC; i++) o[i] = 0.f;
       auto fold = [&](int gb, float alpha) {   // O = O * alpha + (P V) of block gb
-        if (OC == 16) {
-          uint32_t ro[16];
-          tc::tmem_ld16(t_o + (gb & 1) * HD + lane_addr + cq * 16, ro);
-          tc::tmem_ld_wait();
+        uint32_t ro[16];
+        tc::tmem_ld16(t_o + (gb & 1) * HD + lane_addr + cq * 16, ro);
+        tc::tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 16; i++) o[i] = o[i] * alpha + __uint_as_float(ro[i]);
-        } else {
-          uint32_t ro[32];
-          tc::tmem_ld32(t_o + (gb & 1) * HD + lane_addr + cq * 32, ro);
-          tc::tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 32; i++) o[i % OC] = o[i % OC] * alpha + __uint_as_float(ro[i]);
-        }
+        for (int i = 0; i < 16; i++) o[i] = o[i] * alpha + __uint_as_float(ro[i]);
         tc::tc_fence_before();
       };
       for (int j = 0; j < it.nkb; j++, g++) {
@@ -1151,21 +1124,49 @@ __global__ void attn_delta_scalar_k(float* __restrict__ delta, const bf16* __res
   if (lane == 0) delta[((long)b * H + h) * T + t] = s;
 }
 
-// Epilogue helper for the backward kernels: one warp moves 64 accumulator columns of its 32 rows from TMEM to
-// dst as bf16: columns [c0, c0+32) and [c0 + HD/2, c0 + HD/2 + 32), which are exactly RoPE's rotation pairs
-// (i, i + HD/2).  With tables given, RoPE's backward rotation (d0' = d0 c + d1 s, d1' = d1 c - d0 s) is applied.
+// Four lanes (a quad) exchange the 16-byte units of a 4 x 4 block: lane q's a[k] becomes lane k's a[q].  With one row per lane a
+// store instruction touches 32 rows, 16 bytes of each; after the exchange it touches 8 rows, 64 bytes of each.
+__device__ __forceinline__ void quad_transpose(uint4 (&a)[4], int lane) {
+#pragma unroll
+  for (int b = 1; b <= 2; b <<= 1) {
+    const bool up = lane & b;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      if (i & b) continue;
+      const int j = i | b;
+      uint4 x = up ? a[i] : a[j];
+      x.x = __shfl_xor_sync(0xffffffffu, x.x, b); x.y = __shfl_xor_sync(0xffffffffu, x.y, b);
+      x.z = __shfl_xor_sync(0xffffffffu, x.z, b); x.w = __shfl_xor_sync(0xffffffffu, x.w, b);
+      if (up) a[i] = x; else a[j] = x;
+    }
+  }
+}
+// 32 bf16 columns (four 16-byte units per lane) of 32 consecutive rows to memory: `dst` = this lane's row at the first column, rows
+// `pitch` elements apart, `nlive` of the warp's rows exist (whole warp, converged).
+__device__ __forceinline__ void store_rows32(bf16* dst, long pitch, uint4 (&a)[4], int lane, int nlive) {
+  quad_transpose(a, lane);
+  const int q = lane & 3;
+  bf16* base = dst - q * pitch + q * 8;      // row of the quad's first lane, this lane's unit
+#pragma unroll
+  for (int k = 0; k < 4; k++)
+    if ((lane & ~3) + k < nlive) *reinterpret_cast<uint4*>(base + k * pitch) = a[k];
+}
+
+// Epilogue helper for the backward kernels: one warp moves 64 accumulator columns of its 32 rows from TMEM to memory as bf16:
+// columns [c0, c0+32) and [c0 + HD/2, c0 + HD/2 + 32), which are exactly RoPE's rotation pairs (i, i + HD/2).  With tables given,
+// RoPE's backward rotation (d0' = d0 c + d1 s, d1' = d1 c - d0 s) is applied.  dst_row: the lane's row, rows `pitch` apart; t its
+// position; nlive rows of the warp exist (0: nothing is stored).  Whole warp.
 template <int HD>
-__device__ __forceinline__ void store_pairs_rope(bf16* dst_row, uint32_t taddr, int c0, bool live, const float* cosT,
+__device__ __forceinline__ void store_pairs_rope(bf16* dst_row, long pitch, uint32_t taddr, int c0, int lane, int nlive, const float* cosT,
                                                  const float* sinT, int t, float out_scale = 1.f) {
   uint32_t ra[32], rb[32];
   tc::tmem_ld32(taddr + c0, ra);
   tc::tmem_ld32(taddr + c0 + HD / 2, rb);
   tc::tmem_ld_wait();
-  if (!live) return;
   float x0[32], x1[32];
 #pragma unroll
   for (int i = 0; i < 32; i++) { x0[i] = __uint_as_float(ra[i]) * out_scale; x1[i] = __uint_as_float(rb[i]) * out_scale; }
-  if (cosT) {      // 16-byte loads: every lane reads its own row of the tables, an instruction costs the L1 a line per lane whatever its width
+  if (cosT && lane < nlive) {   // 16-byte loads: every lane reads its own row of the tables, an instruction costs the L1 a line per lane whatever its width
     const float4* c4 = reinterpret_cast<const float4*>(cosT + (size_t)t * (HD / 2) + c0);
     const float4* s4 = reinterpret_cast<const float4*>(sinT + (size_t)t * (HD / 2) + c0);
 #pragma unroll
@@ -1180,16 +1181,18 @@ __device__ __forceinline__ void store_pairs_rope(bf16* dst_row, uint32_t taddr, 
       }
     }
   }
+  __syncwarp();
+  uint4 u[4];
 #pragma unroll
-  for (int v8 = 0; v8 < 4; v8++) {
-    uint4 pa, pb;
-    pa.x = pack_bf16(x0[v8 * 8 + 0], x0[v8 * 8 + 1]); pa.y = pack_bf16(x0[v8 * 8 + 2], x0[v8 * 8 + 3]);
-    pa.z = pack_bf16(x0[v8 * 8 + 4], x0[v8 * 8 + 5]); pa.w = pack_bf16(x0[v8 * 8 + 6], x0[v8 * 8 + 7]);
-    pb.x = pack_bf16(x1[v8 * 8 + 0], x1[v8 * 8 + 1]); pb.y = pack_bf16(x1[v8 * 8 + 2], x1[v8 * 8 + 3]);
-    pb.z = pack_bf16(x1[v8 * 8 + 4], x1[v8 * 8 + 5]); pb.w = pack_bf16(x1[v8 * 8 + 6], x1[v8 * 8 + 7]);
-    *reinterpret_cast<uint4*>(dst_row + c0 + v8 * 8) = pa;
-    *reinterpret_cast<uint4*>(dst_row + c0 + HD / 2 + v8 * 8) = pb;
-  }
+  for (int v = 0; v < 4; v++)
+    u[v] = make_uint4(pack_bf16(x0[v * 8], x0[v * 8 + 1]), pack_bf16(x0[v * 8 + 2], x0[v * 8 + 3]), pack_bf16(x0[v * 8 + 4], x0[v * 8 + 5]),
+                      pack_bf16(x0[v * 8 + 6], x0[v * 8 + 7]));
+  store_rows32(dst_row + c0, pitch, u, lane, nlive);
+#pragma unroll
+  for (int v = 0; v < 4; v++)
+    u[v] = make_uint4(pack_bf16(x1[v * 8], x1[v * 8 + 1]), pack_bf16(x1[v * 8 + 2], x1[v * 8 + 3]), pack_bf16(x1[v * 8 + 4], x1[v * 8 + 5]),
+                      pack_bf16(x1[v * 8 + 6], x1[v * 8 + 7]));
+  store_rows32(dst_row + c0 + HD / 2, pitch, u, lane, nlive);
 }
 
 constexpr int BWD_THREADS = 512;
@@ -1197,33 +1200,29 @@ constexpr int BWD_THREADS = 512;
 // ================================================================== backward: dK, dV (one CTA per 128-key tile)
 // 512 threads; thread (row = key, quarter cq) handles 32 of the 128 query columns of S^T / dP^T.  The MMAs of the next
 // query block are queued right behind the dV/dK MMAs of the current one, so one commit covers both.
-template <int HD>
 struct BwdKVSmem {
-  static constexpr int CH = HD / 64;
-  static constexpr int NBUF = (HD == 64) ? 2 : 1;
   static constexpr int K = 0;
-  static constexpr int V = K + CH * TILE_BYTES;
-  static constexpr int Q = V + CH * TILE_BYTES;                 // NBUF buffers
-  static constexpr int DO = Q + NBUF * CH * TILE_BYTES;         // NBUF buffers
-  static constexpr int PT = DO + NBUF * CH * TILE_BYTES;
+  static constexpr int V = K + TILE_BYTES;
+  static constexpr int Q = V + TILE_BYTES;                      // 2 buffers
+  static constexpr int DO = Q + 2 * TILE_BYTES;                 // 2 buffers
+  static constexpr int PT = DO + 2 * TILE_BYTES;
   static constexpr int DST = PT + 2 * TILE_BYTES;
   static constexpr int STAT = DST + 2 * TILE_BYTES;             // lse[128], delta[128] floats
   static constexpr int BAR = STAT + 1024;
   static constexpr int TOTAL = BAR + 128 + 1024;
 };
 
-template <int HD>
 __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kv_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv,
                                                                         const __grid_constant__ CUtensorMap tm_do,
                                                                         const AttnArgs a) {
-  using S = BwdKVSmem<HD>;
-  constexpr int CH = HD / 64, NBUF = S::NBUF;
+  using S = BwdKVSmem;
+  constexpr int HD = 64;
   constexpr uint32_t TMEM_COLS = 512;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = (uint64_t*)(smem + S::BAR);
-  uint64_t *bar_kv = bars, *bar_q = bars + 1 /*[2]*/, *bar_s = bars + 3, *bar_d = bars + 4;
-  uint32_t* tmem_slot = (uint32_t*)(bars + 5);
+  uint64_t *bar_kv = bars, *bar_q = bars + 1 /*[2]*/, *bar_s = bars + 3;
+  uint32_t* tmem_slot = (uint32_t*)(bars + 4);
   float* s_lse = (float*)(smem + S::STAT);
   float* s_delta = s_lse + 128;
 
@@ -1237,7 +1236,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kv_tc_kernel(const __
 
   if (tid == 0) {
     tc::mbar_init(bar_kv, 1); tc::mbar_init(&bar_q[0], 1); tc::mbar_init(&bar_q[1], 1);
-    tc::mbar_init(bar_s, 1); tc::mbar_init(bar_d, 1);
+    tc::mbar_init(bar_s, 1);
     tc::mbar_fence_init();
     tc::tma_prefetch_desc(&tm_qkv);
     tc::tma_prefetch_desc(&tm_do);
@@ -1255,14 +1254,12 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kv_tc_kernel(const __
   const uint32_t sPT = tc::smem_u32(smem + S::PT), sDST = tc::smem_u32(smem + S::DST);
 
   auto load_q_do = [&](int i, int buf) {
-    tc::mbar_expect_tx(&bar_q[buf], 2 * CH * TILE_BYTES);
-    for (int c = 0; c < CH; c++) {
-      tc::tma_load_2d(smem + S::Q + (buf * CH + c) * TILE_BYTES, &tm_qkv, &bar_q[buf], h * HD + c * 64, row0 + i * 128);
-      tc::tma_load_2d(smem + S::DO + (buf * CH + c) * TILE_BYTES, &tm_do, &bar_q[buf], h * HD + c * 64, row0 + i * 128);
-    }
+    tc::mbar_expect_tx(&bar_q[buf], 2 * TILE_BYTES);
+    tc::tma_load_2d(smem + S::Q + buf * TILE_BYTES, &tm_qkv, &bar_q[buf], h * HD, row0 + i * 128);
+    tc::tma_load_2d(smem + S::DO + buf * TILE_BYTES, &tm_do, &bar_q[buf], h * HD, row0 + i * 128);
   };
   auto issue_scores = [&](int buf) {   // S^T = K Q^T and dP^T = V dO^T for the block in `buf`
-    const uint32_t sQ = tc::smem_u32(smem + S::Q + buf * CH * TILE_BYTES), sDO = tc::smem_u32(smem + S::DO + buf * CH * TILE_BYTES);
+    const uint32_t sQ = tc::smem_u32(smem + S::Q + buf * TILE_BYTES), sDO = tc::smem_u32(smem + S::DO + buf * TILE_BYTES);
 #pragma unroll
     for (int ks = 0; ks < HD / 16; ks++) tc::mma_bf16_ss(t_st, desc_k(sK, ks), desc_k(sQ, ks), idesc_s, ks > 0);
 #pragma unroll
@@ -1270,11 +1267,9 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kv_tc_kernel(const __
   };
   const int n_it = nq - kt;
   if (tid == 0) {
-    tc::mbar_expect_tx(bar_kv, 2 * CH * TILE_BYTES);
-    for (int c = 0; c < CH; c++) {
-      tc::tma_load_2d(smem + S::K + c * TILE_BYTES, &tm_qkv, bar_kv, C + h * HD + c * 64, row0 + k0);
-      tc::tma_load_2d(smem + S::V + c * TILE_BYTES, &tm_qkv, bar_kv, 2 * C + h * HD + c * 64, row0 + k0);
-    }
+    tc::mbar_expect_tx(bar_kv, 2 * TILE_BYTES);
+    tc::tma_load_2d(smem + S::K, &tm_qkv, bar_kv, C + h * HD, row0 + k0);
+    tc::tma_load_2d(smem + S::V, &tm_qkv, bar_kv, 2 * C + h * HD, row0 + k0);
     load_q_do(kt, 0);
     if (tc::mbar_wait(bar_kv, 0, 20) && tc::mbar_wait(&bar_q[0], 0, 21)) {
       tc::tc_fence_after();
@@ -1287,7 +1282,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kv_tc_kernel(const __
   bool ok = true;
   for (int it = 0; it < n_it; it++) {
     const int i = kt + it, q0 = i * 128;
-    const int buf = (NBUF == 2) ? (it & 1) : 0;
+    const int buf = it & 1;
     if (tid < 256) {   // per-query statistics of this block (queries past the sequence end contribute nothing)
       const int q = q0 + (tid & 127);
       const size_t si = ((size_t)b * a.H + h) * a.T + q;
@@ -1298,7 +1293,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kv_tc_kernel(const __
     if (!tc::mbar_wait(bar_s, it & 1, 22)) { ok = false; break; }
     tc::tc_fence_after();
     // every MMA issued so far has completed: the other Q/dO buffer (read by the previous dV/dK) can be refilled
-    if (NBUF == 2 && tid == 0 && it + 1 < n_it) load_q_do(i + 1, buf ^ 1);
+    if (tid == 0 && it + 1 < n_it) load_q_do(i + 1, buf ^ 1);
     const bool diag = (it == 0);
     {
       uint32_t rs[32], rd[32];
@@ -1329,23 +1324,15 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kv_tc_kernel(const __
     __syncthreads();
     if (tid == 0) {
       tc::tc_fence_after();
-      const uint32_t sQ = tc::smem_u32(smem + S::Q + buf * CH * TILE_BYTES), sDO = tc::smem_u32(smem + S::DO + buf * CH * TILE_BYTES);
+      const uint32_t sQ = tc::smem_u32(smem + S::Q + buf * TILE_BYTES), sDO = tc::smem_u32(smem + S::DO + buf * TILE_BYTES);
 #pragma unroll
       for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ss(t_dv, desc_k(sPT, ks), desc_mn(sDO, ks), idesc_d, (it > 0 || ks > 0));
 #pragma unroll
       for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ss(t_dk, desc_k(sDST, ks), desc_mn(sQ, ks), idesc_d, (it > 0 || ks > 0));
       if (it + 1 < n_it) {
-        bool ready = true;
-        if (NBUF == 1) {   // single buffer: dV/dK must finish reading Q/dO before the next block is loaded over them
-          tc::mma_commit(bar_d);
-          ready = tc::mbar_wait(bar_d, it & 1, 23);
-          if (ready) load_q_do(i + 1, 0);
-        }
-        const int nb = (NBUF == 2) ? (buf ^ 1) : 0;
-        const int nphase = (NBUF == 2) ? (((it + 1) >> 1) & 1) : ((it + 1) & 1);
-        if (ready && tc::mbar_wait(&bar_q[nb], nphase, 24)) {
+        if (tc::mbar_wait(&bar_q[buf ^ 1], ((it + 1) >> 1) & 1, 24)) {
           tc::tc_fence_after();
-          issue_scores(nb);
+          issue_scores(buf ^ 1);
         }
       }
       tc::mma_commit(bar_s);
@@ -1353,14 +1340,12 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kv_tc_kernel(const __
   }
   if (ok) ok = tc::mbar_wait(bar_s, n_it & 1, 25);   // dV / dK of the last block are complete
   tc::tc_fence_after();
-  if (ok) {
-    // jobs: HD/64 column-pair slabs for dK (with RoPE) then HD/64 for dV; one job per quarter-group of warps
-    constexpr int JOBS = HD / 64;
-    if (cq < 2 * JOBS) {
-      const bool is_k = cq < JOBS;
-      const int pass = is_k ? cq : cq - JOBS;
+  if (__all_sync(0xffffffffu, ok)) {
+    // dK (with RoPE) by the first quarter-group of warps, dV by the second
+    if (cq < 2) {
+      const bool is_k = cq == 0;
       bf16* dst = a.out + ((size_t)(row0 + krow)) * 3 * C + (is_k ? C : 2 * C) + h * HD;
-      store_pairs_rope<HD>(dst, (is_k ? t_dk : t_dv) + lane_addr, pass * 32, krow < a.T, is_k ? a.cosT : nullptr,
+      store_pairs_rope<HD>(dst, 3L * C, (is_k ? t_dk : t_dv) + lane_addr, 0, lane, a.T - (krow - lane), is_k ? a.cosT : nullptr,
                            is_k ? a.sinT : nullptr, krow);
     }
   }
@@ -1775,8 +1760,9 @@ __global__ void __maxnreg__(120) attn_bwd_fused_tc_kernel(const __grid_constant_
       // the wait above covered the last block: dV and dK of this key tile are final
       {
         bf16* dk = a.out + ((size_t)(row0 + krow)) * 3 * C + C + h * HD;
-        store_pairs_rope<HD>(dk, t_dk + lane_addr, 0, !*s_abort && krow < a.T, a.cosT, a.sinT, krow, a.scale);
-        store_pairs_rope<HD>(dk + C, t_dv + lane_addr, 0, !*s_abort && krow < a.T, nullptr, nullptr, krow, 1.f);
+        const int nlive = *s_abort ? 0 : a.T - (krow - lane);
+        store_pairs_rope<HD>(dk, 3L * C, t_dk + lane_addr, 0, lane, nlive, a.cosT, a.sinT, krow, a.scale);
+        store_pairs_rope<HD>(dk + C, 3L * C, t_dv + lane_addr, 0, lane, nlive, nullptr, nullptr, krow, 1.f);
       }
       tc::tc_fence_before();
       __syncwarp();
@@ -1854,31 +1840,27 @@ __global__ void __launch_bounds__(256) attn_dq_finish_k(bf16* __restrict__ dqkv,
 }
 
 // ================================================================== backward: dQ (one CTA per 128-query tile)
-template <int HD>
 struct BwdQSmem {
-  static constexpr int CH = HD / 64;
-  static constexpr int NBUF = (HD == 64) ? 2 : 1;
   static constexpr int Q = 0;
-  static constexpr int DO = Q + CH * TILE_BYTES;
-  static constexpr int K = DO + CH * TILE_BYTES;               // NBUF
-  static constexpr int V = K + NBUF * CH * TILE_BYTES;         // NBUF
-  static constexpr int DS = V + NBUF * CH * TILE_BYTES;
+  static constexpr int DO = Q + TILE_BYTES;
+  static constexpr int K = DO + TILE_BYTES;                    // 2 buffers
+  static constexpr int V = K + 2 * TILE_BYTES;                 // 2 buffers
+  static constexpr int DS = V + 2 * TILE_BYTES;
   static constexpr int BAR = DS + 2 * TILE_BYTES;
   static constexpr int TOTAL = BAR + 128 + 1024;
 };
 
-template <int HD>
 __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_q_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv,
                                                                        const __grid_constant__ CUtensorMap tm_do,
                                                                        const AttnArgs a) {
-  using S = BwdQSmem<HD>;
-  constexpr int CH = HD / 64, NBUF = S::NBUF;
+  using S = BwdQSmem;
+  constexpr int HD = 64;
   constexpr uint32_t TMEM_COLS = 512;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = (uint64_t*)(smem + S::BAR);
-  uint64_t *bar_q = bars, *bar_kv = bars + 1 /*[2]*/, *bar_s = bars + 3, *bar_d = bars + 4;
-  uint32_t* tmem_slot = (uint32_t*)(bars + 5);
+  uint64_t *bar_q = bars, *bar_kv = bars + 1 /*[2]*/, *bar_s = bars + 3;
+  uint32_t* tmem_slot = (uint32_t*)(bars + 4);
 
   const int nq = (a.T + 127) / 128;
   const int qt = nq - 1 - blockIdx.x, h = blockIdx.y, b = blockIdx.z;
@@ -1890,7 +1872,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_q_tc_kernel(const __g
 
   if (tid == 0) {
     tc::mbar_init(bar_q, 1); tc::mbar_init(&bar_kv[0], 1); tc::mbar_init(&bar_kv[1], 1);
-    tc::mbar_init(bar_s, 1); tc::mbar_init(bar_d, 1);
+    tc::mbar_init(bar_s, 1);
     tc::mbar_fence_init();
     tc::tma_prefetch_desc(&tm_qkv);
     tc::tma_prefetch_desc(&tm_do);
@@ -1907,14 +1889,12 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_q_tc_kernel(const __g
   const uint32_t sQ = tc::smem_u32(smem + S::Q), sDO = tc::smem_u32(smem + S::DO), sDS = tc::smem_u32(smem + S::DS);
 
   auto load_kv = [&](int j, int buf) {
-    tc::mbar_expect_tx(&bar_kv[buf], 2 * CH * TILE_BYTES);
-    for (int c = 0; c < CH; c++) {
-      tc::tma_load_2d(smem + S::K + (buf * CH + c) * TILE_BYTES, &tm_qkv, &bar_kv[buf], C + h * HD + c * 64, row0 + j * 128);
-      tc::tma_load_2d(smem + S::V + (buf * CH + c) * TILE_BYTES, &tm_qkv, &bar_kv[buf], 2 * C + h * HD + c * 64, row0 + j * 128);
-    }
+    tc::mbar_expect_tx(&bar_kv[buf], 2 * TILE_BYTES);
+    tc::tma_load_2d(smem + S::K + buf * TILE_BYTES, &tm_qkv, &bar_kv[buf], C + h * HD, row0 + j * 128);
+    tc::tma_load_2d(smem + S::V + buf * TILE_BYTES, &tm_qkv, &bar_kv[buf], 2 * C + h * HD, row0 + j * 128);
   };
   auto issue_scores = [&](int buf) {   // S = Q K^T and dP = dO V^T for the key block in `buf`
-    const uint32_t sK = tc::smem_u32(smem + S::K + buf * CH * TILE_BYTES), sV = tc::smem_u32(smem + S::V + buf * CH * TILE_BYTES);
+    const uint32_t sK = tc::smem_u32(smem + S::K + buf * TILE_BYTES), sV = tc::smem_u32(smem + S::V + buf * TILE_BYTES);
 #pragma unroll
     for (int ks = 0; ks < HD / 16; ks++) tc::mma_bf16_ss(t_s, desc_k(sQ, ks), desc_k(sK, ks), idesc_s, ks > 0);
 #pragma unroll
@@ -1922,11 +1902,9 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_q_tc_kernel(const __g
   };
   const int nkb = qt + 1;
   if (tid == 0) {
-    tc::mbar_expect_tx(bar_q, 2 * CH * TILE_BYTES);
-    for (int c = 0; c < CH; c++) {
-      tc::tma_load_2d(smem + S::Q + c * TILE_BYTES, &tm_qkv, bar_q, h * HD + c * 64, row0 + q0);
-      tc::tma_load_2d(smem + S::DO + c * TILE_BYTES, &tm_do, bar_q, h * HD + c * 64, row0 + q0);
-    }
+    tc::mbar_expect_tx(bar_q, 2 * TILE_BYTES);
+    tc::tma_load_2d(smem + S::Q, &tm_qkv, bar_q, h * HD, row0 + q0);
+    tc::tma_load_2d(smem + S::DO, &tm_do, bar_q, h * HD, row0 + q0);
     load_kv(0, 0);
     if (tc::mbar_wait(bar_q, 0, 30) && tc::mbar_wait(&bar_kv[0], 0, 31)) {
       tc::tc_fence_after();
@@ -1941,11 +1919,11 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_q_tc_kernel(const __g
   const float delta = (qrow < a.T) ? a.delta[si] : 0.f;
   bool ok = true;
   for (int j = 0; j < nkb; j++) {
-    const int buf = (NBUF == 2) ? (j & 1) : 0;
+    const int buf = j & 1;
     const int k0 = j * 128;
     if (!tc::mbar_wait(bar_s, j & 1, 32)) { ok = false; break; }
     tc::tc_fence_after();
-    if (NBUF == 2 && tid == 0 && j + 1 < nkb) load_kv(j + 1, buf ^ 1);
+    if (tid == 0 && j + 1 < nkb) load_kv(j + 1, buf ^ 1);
     const bool diag = (j == qt);
     {
       uint32_t rs[32], rd[32];
@@ -1972,21 +1950,13 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_q_tc_kernel(const __g
     __syncthreads();
     if (tid == 0) {
       tc::tc_fence_after();
-      const uint32_t sK = tc::smem_u32(smem + S::K + buf * CH * TILE_BYTES);
+      const uint32_t sK = tc::smem_u32(smem + S::K + buf * TILE_BYTES);
 #pragma unroll
       for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ss(t_dq, desc_k(sDS, ks), desc_mn(sK, ks), idesc_d, (j > 0 || ks > 0));
       if (j + 1 < nkb) {
-        bool ready = true;
-        if (NBUF == 1) {
-          tc::mma_commit(bar_d);
-          ready = tc::mbar_wait(bar_d, j & 1, 33);
-          if (ready) load_kv(j + 1, 0);
-        }
-        const int nb = (NBUF == 2) ? (buf ^ 1) : 0;
-        const int nphase = (NBUF == 2) ? (((j + 1) >> 1) & 1) : ((j + 1) & 1);
-        if (ready && tc::mbar_wait(&bar_kv[nb], nphase, 34)) {
+        if (tc::mbar_wait(&bar_kv[buf ^ 1], ((j + 1) >> 1) & 1, 34)) {
           tc::tc_fence_after();
-          issue_scores(nb);
+          issue_scores(buf ^ 1);
         }
       }
       tc::mma_commit(bar_s);
@@ -1994,9 +1964,9 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_q_tc_kernel(const __g
   }
   if (ok) ok = tc::mbar_wait(bar_s, nkb & 1, 35);
   tc::tc_fence_after();
-  if (ok && cq < HD / 64) {
+  if (__all_sync(0xffffffffu, ok) && cq == 0) {
     bf16* dst = a.out + ((size_t)(row0 + qrow)) * 3 * C + h * HD;
-    store_pairs_rope<HD>(dst, t_dq + lane_addr, cq * 32, qrow < a.T, a.cosT, a.sinT, qrow);
+    store_pairs_rope<HD>(dst, 3L * C, t_dq + lane_addr, 0, lane, a.T - (qrow - lane), a.cosT, a.sinT, qrow);
   }
   tc::tc_fence_before();
   __syncthreads();
@@ -2227,9 +2197,9 @@ MLB_API int mlb_attn_fwd(void* out, float* lse, const void* qkv, int B, int T, i
       }
 #undef MLB_FWD2
     } else if (hd == 64) {
-      static int once = set_smem(attn_fwd_tc_kernel<64>, FwdSmem<64>::TOTAL);
+      static int once = set_smem(attn_fwd_tc_kernel, FwdSmem::TOTAL);
       (void)once;
-      attn_fwd_tc_kernel<64><<<grid, ATT_THREADS, FwdSmem<64>::TOTAL, st>>>(*tm, a);
+      attn_fwd_tc_kernel<<<grid, ATT_THREADS, FwdSmem::TOTAL, st>>>(*tm, a);
     } else {
       const CUtensorMap* t3 = mlb_tmap_seq3d_cached(qkv, B, T, 3L * C);
       const CUtensorMap* to = (T % 128 == 0) ? mlb_tmap_cached(out, (uint64_t)B * T, C, C, 32, 64, 2) : nullptr;
@@ -2339,11 +2309,11 @@ static int attn_bwd_impl(void* dqkv, const void* dout, const void* qkv, const vo
       return cosT ? 1 : 0;
     }
     if (hd == 64) {
-      static int o1 = set_smem(attn_bwd_kv_tc_kernel<64>, BwdKVSmem<64>::TOTAL);
-      static int o2 = set_smem(attn_bwd_q_tc_kernel<64>, BwdQSmem<64>::TOTAL);
+      static int o1 = set_smem(attn_bwd_kv_tc_kernel, BwdKVSmem::TOTAL);
+      static int o2 = set_smem(attn_bwd_q_tc_kernel, BwdQSmem::TOTAL);
       (void)o1; (void)o2;
-      attn_bwd_kv_tc_kernel<64><<<grid, BWD_THREADS, BwdKVSmem<64>::TOTAL, st>>>(*tq, *td, a);
-      attn_bwd_q_tc_kernel<64><<<grid, BWD_THREADS, BwdQSmem<64>::TOTAL, st>>>(*tq, *td, a);
+      attn_bwd_kv_tc_kernel<<<grid, BWD_THREADS, BwdKVSmem::TOTAL, st>>>(*tq, *td, a);
+      attn_bwd_q_tc_kernel<<<grid, BWD_THREADS, BwdQSmem::TOTAL, st>>>(*tq, *td, a);
     } else {
       const CUtensorMap* t3 = mlb_tmap_seq3d_cached(qkv, B, T, 3L * C);
       const CUtensorMap* d3 = mlb_tmap_seq3d_cached(dout, B, T, C);

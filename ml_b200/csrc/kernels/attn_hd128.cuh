@@ -38,10 +38,12 @@ struct ItemList {
 
 // Forward over pairs of query tiles (256 queries) of one (sample, head).  TMEM: S0 S1 O0 O1.  Per tile and key block
 //   S = Q K^T -> one thread per row: m, p = exp2(s c - m) -> P over S -> O += P V -> next S
-// is a chain; the two tiles run it out of phase, one on the tensor core while the other takes exponentials.  P V starts
-// when the first half of P is there.  m is the maximum of an earlier block as long as no row of the warp has grown past it
+// is a chain; the two tiles run it out of phase, one on the tensor core while the other takes exponentials: they take turns.  Left
+// alone they fall into step, and a step of both tiles takes 5400 cycles instead of 3700 (8 x 2048 tokens, 16 heads: 192 -> 161 us, 853
+// TFLOP/s over the causal half).  P V starts when the first half of P is there.  160 registers leave a sub-partition with three of
+// these warps room for one 32-register warp of a communication kernel.  m is the maximum of an earlier block as long as no row of the warp has grown past it
 // by more than 2^8; only then O (in place) and l are rescaled.
-__global__ void __launch_bounds__(FWD128_THREADS, 1) attn_fwd128_k(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUtensorMap tm_out,
+__global__ void __maxnreg__(160) attn_fwd128_k(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUtensorMap tm_out,
                                                                    const AttnArgs a) {
   mlb_pdl_sync();
   using S = Fwd128Smem;
@@ -50,8 +52,9 @@ __global__ void __launch_bounds__(FWD128_THREADS, 1) attn_fwd128_k(const __grid_
   uint64_t* bars = (uint64_t*)(smem + S::BAR);
   uint64_t *bar_q = bars, *bar_qf = bars + 2, *bar_k = bars + 4, *bar_kf = bars + 6, *bar_v = bars + 8, *bar_vf = bars + 10, *bar_s = bars + 12,
            *bar_pa = bars + 14, *bar_pb = bars + 16, *bar_o = bars + 18;      // [2] each: per tile (q, s, p, o) or slot (k, v)
-  uint32_t* tmem_slot = (uint32_t*)(bars + 20);
-  volatile int* s_abort = (volatile int*)(bars + 21);
+  volatile int* s_turn = (volatile int*)(bars + 20);      // [2][4]: blocks whose exponentials tile t's warp on sub-partition lg has taken
+  uint32_t* tmem_slot = (uint32_t*)(bars + 24);
+  volatile int* s_abort = (volatile int*)(bars + 25);
   if (attn_given_up()) return;
   const int nq = (a.T + 127) / 128, npair = (nq + 1) / 2, BH = a.B * a.H, C = a.H * H128;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -65,6 +68,7 @@ __global__ void __launch_bounds__(FWD128_THREADS, 1) attn_fwd128_k(const __grid_
       tc::mbar_init(&bar_v[i], 1); tc::mbar_init(&bar_vf[i], 2); tc::mbar_init(&bar_s[i], 1); tc::mbar_init(&bar_pa[i], 4);
       tc::mbar_init(&bar_pb[i], 4); tc::mbar_init(&bar_o[i], 1);
     }
+    for (int i = 0; i < 8; i++) s_turn[i] = 0;
     *s_abort = 0;
     tc::mbar_fence_init();
     tc::tma_prefetch_desc(&tm);
@@ -171,11 +175,11 @@ __global__ void __launch_bounds__(FWD128_THREADS, 1) attn_fwd128_k(const __grid_
     const float sl2 = a.scale * LOG2E;
     const uint64_t sl2x2 = pk2(sl2, sl2);
     uint8_t* stage = smem + S::OST + warp * 4096;
-    int gt = 0;
+    int gt = 0, other = 0;      // blocks taken by this tile, and by the other tile in earlier items
     for (int li = 0, w; (w = items.at(li)) >= 0; li++) {
       const Item it = item_of(w);
-      const int n = blocks_of(it, t);
-      if (n == 0) continue;
+      const int n = blocks_of(it, t), n_other = blocks_of(it, t ^ 1);
+      if (n == 0) { other += n_other; continue; }
       const int qt = 2 * it.pair + t, qrow = qt * 128 + row;
       float m = 0.f, l = 0.f;
       for (int j = 0; j < n; j++, gt++) {
@@ -191,12 +195,12 @@ __global__ void __launch_bounds__(FWD128_THREADS, 1) attn_fwd128_k(const __grid_
           for (int i = 0; i < 128; i++)
             if (i > row) r[i >> 5][i & 31] = 0xff800000u;
         }
-        float mx = -INFINITY;
+        float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};      // four chains: one of 64 dependent maxima takes ~500 cycles
 #pragma unroll
-        for (int c = 0; c < 4; c++)
+        for (int i = 0; i < 32; i += 2)
 #pragma unroll
-          for (int i = 0; i < 32; i += 2) mx = max3(mx, __uint_as_float(r[c][i]), __uint_as_float(r[c][i + 1]));
-        const float z = mx * sl2;
+          for (int c = 0; c < 4; c++) m4[c] = max3(m4[c], __uint_as_float(r[c][i]), __uint_as_float(r[c][i + 1]));
+        const float z = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * sl2;
         if (j == 0) {
           m = z == -INFINITY ? 0.f : z;
         } else if (__any_sync(0xffffffffu, z > m + 8.f)) {
@@ -217,8 +221,15 @@ __global__ void __launch_bounds__(FWD128_THREADS, 1) attn_fwd128_k(const __grid_
           }
           tc::tmem_st_wait();
         }
+        // Turns: the two warps of a sub-partition take their exponentials one after the other (tile 0's block j, tile 1's block j, ...).
+        // Left alone they fall into step, both on the special-function unit and then both waiting for the tensor core.
+        // A counter and not an mbarrier, since one tile may be many blocks behind (a pair without a second tile); only the order hangs on
+        // it, so a warp that has polled for long goes on.
+        const int turn = other + min(j + t, n_other);      // blocks the other tile's warp is to have taken before
+        for (int spin = 0; s_turn[(t ^ 1) * 4 + lg] < turn && spin < (1 << 16) && !*s_abort; spin++) { }
+        __syncwarp();
         const uint64_t nm2 = pk2(-m, -m);
-        uint64_t rs2 = pk2(0.f, 0.f);
+        uint64_t rs2 = pk2(0.f, 0.f), rs3 = rs2;
 #pragma unroll
         for (int c = 0; c < 4; c++) {
           uint32_t pw[16];
@@ -227,21 +238,30 @@ __global__ void __launch_bounds__(FWD128_THREADS, 1) attn_fwd128_k(const __grid_
             float z0, z1;
             upk2(fma2(pk2(__uint_as_float(r[c][2 * i]), __uint_as_float(r[c][2 * i + 1])), sl2x2, nm2), z0, z1);
             const float p0 = ex2_approx(z0), p1 = ex2_approx(z1);
-            rs2 = add2(rs2, pk2(p0, p1));
+            if (i & 1) rs3 = add2(rs3, pk2(p0, p1));
+            else rs2 = add2(rs2, pk2(p0, p1));
             pw[i] = pack_bf16(p0, p1);
           }
-          tc::tmem_st16(t_s + c * 16, pw);
-          if (c == 1 || c == 3) {
+          // the first half of P is handed over a quarter late, when its stores have long landed: waiting for them at once stalls the warp
+          if (c == 2) {
             tc::tmem_st_wait();
             tc::tc_fence_before();
             __syncwarp();
-            if (lane == 0) tc::mbar_arrive(c == 1 ? &bar_pa[t] : &bar_pb[t]);
+            if (lane == 0) tc::mbar_arrive(&bar_pa[t]);
           }
+          tc::tmem_st16(t_s + c * 16, pw);
         }
+        if (lane == 0) s_turn[t * 4 + lg] = gt + 1;
+        tc::tmem_st_wait();
+        tc::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&bar_pb[t]);
+        rs2 = add2(rs2, rs3);
         float lo, hi;
         upk2(rs2, lo, hi);
         l += lo + hi;
       }
+      other += n_other;
       // ---- epilogue: O / l as bf16
       wait(&bar_o[t], (gt - 1) & 1, 60);
       __syncwarp();
@@ -293,15 +313,17 @@ __global__ void __launch_bounds__(FWD128_THREADS, 1) attn_fwd128_k(const __grid_
 // ------------------------------------------------------------------ backward
 // dK / dV of a 128-key tile, streaming query blocks.  TMEM: S^T, dP^T, dV, dK.  The tensor core's sequence is
 //   dV(i)  S^T(i+1)  dK(i)  dP^T(i+1)  dV(i+1) ...
-// so the exponentials of block i+1 run under dK(i) and dP^T(i+1), and dS(i+1) under dV(i+1) and S^T(i+2).  256 element-wise threads: a
-// thread has one key and 64 of the block's 128 queries; its P^T / dS^T go over its own score columns.
+// so the exponentials of block i+1 run under dK(i) and dP^T(i+1), and dS(i+1) under dV(i+1) and S^T(i+2).  512 element-wise threads: a
+// thread has one key and 32 of the block's 128 queries; its P^T / dS^T go over its own score columns.  Four warps per sub-partition
+// hide each other's TMEM and barrier latencies: with two (64 queries a thread) a block took them 3000 cycles, of which 1024 are the
+// special-function unit's.
 struct BwdKV128Smem {
   static constexpr int K = 0;
   static constexpr int V = K + T128_BYTES;
   static constexpr int Q = V + T128_BYTES;               // 2 slots
   static constexpr int DO = Q + 2 * T128_BYTES;          // 2 slots
-  static constexpr int STAT = DO + 2 * T128_BYTES;       // 8 warps x 2 buffers x (lse * log2 e [64], delta [64])
-  static constexpr int BAR = STAT + 8 * 1024;
+  static constexpr int STAT = DO + 2 * T128_BYTES;       // 16 warps x 2 buffers x (lse * log2 e [32], delta [32])
+  static constexpr int BAR = STAT + 16 * 512;
   static constexpr int SCHED = BAR + 256;
   static constexpr int TOTAL = SCHED + 256 + 1024;
 };
@@ -317,9 +339,10 @@ struct BwdQ128Smem {
   static constexpr int SCHED = BAR + 256;
   static constexpr int TOTAL = SCHED + 256 + 1024;
 };
-constexpr int BWD128_THREADS = 10 * 32;      // 8 element-wise warps (lane group w & 3, column half w >> 2), MMA warp, loader
-// A-operand columns of k-step ks of a bf16 tile whose two 64-column halves sit over their own fp32 columns
-__device__ __forceinline__ uint32_t half_col(int ks) { return (uint32_t)((ks >> 2) * 64 + (ks & 3) * 8); }
+constexpr int BWD128_E_WARPS = 16;      // element-wise warps: lane group w & 3, quarter of the 128 columns w >> 2
+constexpr int BWD128_MMA_WARP = BWD128_E_WARPS, BWD128_LOAD_WARP = BWD128_E_WARPS + 1;
+constexpr int BWD128_THREADS = (BWD128_E_WARPS + 2) * 32;
+// (split_col(ks): A-operand column of k-step ks of a bf16 tile whose 32-column quarters sit over their own fp32 columns)
 
 __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUtensorMap tm_do,
                                                                       const AttnArgs a) {
@@ -340,13 +363,13 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
   if (srow && tid < 64) s_sched[tid] = tid < a.sched_stride ? __ldg(srow + tid) : -1;
   const ItemList items{srow, s_sched, (int)blockIdx.x, (int)gridDim.x, nq * BH};
   if (tid == 0) {
-    for (int i = 0; i < 15; i++) tc::mbar_init(&bars[i], (i == 12 || i == 13) ? 8 : 1);
+    for (int i = 0; i < 15; i++) tc::mbar_init(&bars[i], (i == 12 || i == 13) ? BWD128_E_WARPS : 1);
     *s_abort = 0;
     tc::mbar_fence_init();
     tc::tma_prefetch_desc(&tm);
     tc::tma_prefetch_desc(&tm_do);
   }
-  if (warp == 8) tc::tmem_alloc(tmem_slot, 512);
+  if (warp == BWD128_MMA_WARP) tc::tmem_alloc(tmem_slot, 512);
   tc::tc_fence_before();
   __syncthreads();
   tc::tc_fence_after();
@@ -357,7 +380,7 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
     if (!tc::mbar_wait(bar, phase, where)) *s_abort = 1;
   };
   // item w = key tile (heaviest, the first, first) of (sample, head)
-  if (warp == 9) {
+  if (warp == BWD128_LOAD_WARP) {
     if (lane == 0) {
       int g = 0;
       for (int li = 0, w; (w = items.at(li)) >= 0; li++) {
@@ -377,7 +400,7 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
         }
       }
     }
-  } else if (warp == 8) {
+  } else if (warp == BWD128_MMA_WARP) {
     if (lane == 0) {
       constexpr uint32_t idesc_s = tc::idesc_bf16(128, 128, 0, 0), idesc_g = tc::idesc_bf16(128, H128, 0, 1);
       const uint64_t dK = desc_base_k(tc::smem_u32(smem + S::K)), dV = desc_base_k(tc::smem_u32(smem + S::V));
@@ -412,13 +435,13 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
           wait(bar_p, g & 1, 67);      // (of an item's first block: also the accumulators of the previous item have been read out)
           tc::tc_fence_after();
 #pragma unroll
-          for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ts(t_dv, t_s + half_col(ks), gO + off_mn(ks), idesc_g, (i > 0 || ks > 0));
+          for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ts(t_dv, t_s + split_col(ks), gO + off_mn(ks), idesc_g, (i > 0 || ks > 0));
           tc::mma_commit(&bar_dof[sl]);
           if (i + 1 < n) scores(g + 1);
           wait(bar_ds, g & 1, 68);
           tc::tc_fence_after();
 #pragma unroll
-          for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ts(t_dk, t_dp + half_col(ks), gQ + off_mn(ks), idesc_g, (i > 0 || ks > 0));
+          for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ts(t_dk, t_dp + split_col(ks), gQ + off_mn(ks), idesc_g, (i > 0 || ks > 0));
           tc::mma_commit(&bar_qf[sl]);
           if (i + 1 < n) dprobs(g + 1, i + 2 == n);
           else tc::mma_commit(bar_done);
@@ -426,66 +449,61 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
       }
     }
   } else {
-    const int lg = warp & 3, hf = warp >> 2, row = lg * 32 + lane;
+    const int lg = warp & 3, qd = warp >> 2, row = lg * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(lg * 32) << 16;
-    const uint32_t ts = t_s + hf * 64 + lane_addr, tdp = t_dp + hf * 64 + lane_addr;
+    const uint32_t ts = t_s + qd * 32 + lane_addr, tdp = t_dp + qd * 32 + lane_addr;
     const float sl2 = a.scale * LOG2E;
-    float* stat = (float*)(smem + S::STAT + warp * 1024);
+    float* stat = (float*)(smem + S::STAT + warp * 512);
     int g = 0;
-    for (int li = 0, w; (w = items.at(li)) >= 0; li++) {
+    // statistics of the warp's 32 queries, one per lane, fetched a block ahead (an item's first ones under the epilogue before it); a
+    // query past the end has lse = +inf: p = 0
+    float nl = 0.f, nd = 0.f;
+    auto fetch = [&](int w, int i) {
+      const int q = i * 128 + qd * 32 + lane;
+      const size_t e = (size_t)(w % BH) * a.T + q;
+      nl = q < a.T ? a.lse[e] * LOG2E : INFINITY;
+      nd = q < a.T ? a.delta[e] : 0.f;
+    };
+    int w = items.at(0);
+    if (w >= 0) fetch(w, w / BH);
+    for (int li = 0; w >= 0; li++) {
       const int kt = w / BH, bh = w % BH, b = bh / a.H, h = bh % a.H;
-      const size_t si = ((size_t)b * a.H + h) * a.T;
       const int krow = kt * 128 + row;
-      // statistics of the warp's 64 queries; a query past the end has lse = +inf: p = 0
-      float sv[4];
-      auto fetch = [&](int i) {
-#pragma unroll
-        for (int x = 0; x < 2; x++) {
-          const int q = i * 128 + hf * 64 + x * 32 + lane;
-          sv[x] = q < a.T ? a.lse[si + q] * LOG2E : INFINITY;
-          sv[2 + x] = q < a.T ? a.delta[si + q] : 0.f;
-        }
-      };
       auto publish = [&](int gb) {
-#pragma unroll
-        for (int x = 0; x < 4; x++) stat[(gb & 1) * 128 + x * 32 + lane] = sv[x];
+        stat[(gb & 1) * 64 + lane] = nl;
+        stat[(gb & 1) * 64 + 32 + lane] = nd;
         __syncwarp();
       };
-      fetch(kt);
       publish(g);
       for (int i = kt; i < nq; i++, g++) {
-        const float* st = stat + (g & 1) * 128;
-        if (i + 1 < nq) fetch(i + 1);
+        const float* st = stat + (g & 1) * 64;
+        if (i + 1 < nq) fetch(w, i + 1);
         wait(bar_s, g & 1, 69);
         __syncwarp();
         tc::tc_fence_after();
-        float p[64];
+        float p[32];
         {
-          uint32_t r[2][32];
-          tc::tmem_ld32(ts, r[0]);
-          tc::tmem_ld32(ts + 32, r[1]);
+          uint32_t r[32];
+          tc::tmem_ld32(ts, r);
           tc::tmem_ld_wait();
 #pragma unroll
-          for (int e = 0; e < 64; e += 4) {
+          for (int e = 0; e < 32; e += 4) {
             const float4 L = *reinterpret_cast<const float4*>(st + e);
-            p[e] = ex2_approx(fmaf(__uint_as_float(r[e >> 5][e & 31]), sl2, -L.x));
-            p[e + 1] = ex2_approx(fmaf(__uint_as_float(r[e >> 5][(e & 31) + 1]), sl2, -L.y));
-            p[e + 2] = ex2_approx(fmaf(__uint_as_float(r[e >> 5][(e & 31) + 2]), sl2, -L.z));
-            p[e + 3] = ex2_approx(fmaf(__uint_as_float(r[e >> 5][(e & 31) + 3]), sl2, -L.w));
+            p[e] = ex2_approx(fmaf(__uint_as_float(r[e]), sl2, -L.x));
+            p[e + 1] = ex2_approx(fmaf(__uint_as_float(r[e + 1]), sl2, -L.y));
+            p[e + 2] = ex2_approx(fmaf(__uint_as_float(r[e + 2]), sl2, -L.z));
+            p[e + 3] = ex2_approx(fmaf(__uint_as_float(r[e + 3]), sl2, -L.w));
           }
         }
         if (i == kt) {      // the diagonal block: query before key
 #pragma unroll
-          for (int e = 0; e < 64; e++)
-            if (hf * 64 + e < row) p[e] = 0.f;
+          for (int e = 0; e < 32; e++)
+            if (qd * 32 + e < row) p[e] = 0.f;
         }
+        uint32_t pw[16];
 #pragma unroll
-        for (int c = 0; c < 2; c++) {
-          uint32_t pw[16];
-#pragma unroll
-          for (int x = 0; x < 16; x++) pw[x] = pack_bf16(p[c * 32 + 2 * x], p[c * 32 + 2 * x + 1]);
-          tc::tmem_st16(ts + c * 16, pw);
-        }
+        for (int x = 0; x < 16; x++) pw[x] = pack_bf16(p[2 * x], p[2 * x + 1]);
+        tc::tmem_st16(ts, pw);
         tc::tmem_st_wait();
         tc::tc_fence_before();
         __syncwarp();
@@ -493,42 +511,40 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
         wait(bar_dp, g & 1, 70);
         __syncwarp();
         tc::tc_fence_after();
-#pragma unroll
-        for (int c = 0; c < 2; c++) {
-          uint32_t d[32], dw[16];
-          tc::tmem_ld32(tdp + c * 32, d);
+        {
+          uint32_t d[32];
+          tc::tmem_ld32(tdp, d);
           tc::tmem_ld_wait();
 #pragma unroll
-          for (int x = 0; x < 32; x += 4) {
-            const int e = c * 32 + x;
-            const float4 D = *reinterpret_cast<const float4*>(st + 64 + e);
-            dw[x / 2] = pack_bf16(p[e] * (__uint_as_float(d[x]) - D.x), p[e + 1] * (__uint_as_float(d[x + 1]) - D.y));
-            dw[x / 2 + 1] = pack_bf16(p[e + 2] * (__uint_as_float(d[x + 2]) - D.z), p[e + 3] * (__uint_as_float(d[x + 3]) - D.w));
+          for (int e = 0; e < 32; e += 4) {
+            const float4 D = *reinterpret_cast<const float4*>(st + 32 + e);
+            pw[e / 2] = pack_bf16(p[e] * (__uint_as_float(d[e]) - D.x), p[e + 1] * (__uint_as_float(d[e + 1]) - D.y));
+            pw[e / 2 + 1] = pack_bf16(p[e + 2] * (__uint_as_float(d[e + 2]) - D.z), p[e + 3] * (__uint_as_float(d[e + 3]) - D.w));
           }
-          tc::tmem_st16(tdp + c * 16, dw);
         }
+        tc::tmem_st16(tdp, pw);
         tc::tmem_st_wait();
         tc::tc_fence_before();
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(bar_ds);
         if (i + 1 < nq) publish(g + 1);
       }
-      // ---- epilogue: warps 0-3 store dK (softmax scale and RoPE's backward rotation applied), warps 4-7 dV
+      // ---- epilogue: a warp stores 64 columns of dK (quarters 0, 1; softmax scale and RoPE's backward rotation applied) or dV (2, 3)
+      w = items.at(li + 1);
+      if (w >= 0) fetch(w, w / BH);
       wait(bar_done, li & 1, 71);
       __syncwarp();
       tc::tc_fence_after();
-      const bool live = krow < a.T && !*s_abort;
-      bf16* dst = a.out + ((size_t)(b * a.T + (live ? krow : 0))) * 3 * C + (hf == 0 ? C : 2 * C) + h * H128;
-#pragma unroll 1
-      for (int c0 = 0; c0 < 64; c0 += 32)
-        store_pairs_rope<H128>(dst, (hf == 0 ? t_dk : t_dv) + lane_addr, c0, live, hf == 0 ? a.cosT : nullptr, hf == 0 ? a.sinT : nullptr, krow,
-                               hf == 0 ? a.scale : 1.f);
+      const bool is_k = qd < 2;
+      bf16* dst = a.out + ((size_t)(b * a.T + krow)) * 3 * C + (is_k ? C : 2 * C) + h * H128;
+      store_pairs_rope<H128>(dst, 3L * C, (is_k ? t_dk : t_dv) + lane_addr, (qd & 1) * 32, lane, *s_abort ? 0 : a.T - (krow - lane),
+                             is_k ? a.cosT : nullptr, is_k ? a.sinT : nullptr, krow, is_k ? a.scale : 1.f);
       tc::tc_fence_before();
     }
   }
   tc::tc_fence_before();
   __syncthreads();
-  if (warp == 8) tc::tmem_dealloc(tmem, 512);
+  if (warp == BWD128_MMA_WARP) tc::tmem_dealloc(tmem, 512);
 }
 
 __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUtensorMap tm_do,
@@ -550,13 +566,13 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
   if (srow && tid < 64) s_sched[tid] = tid < a.sched_stride ? __ldg(srow + tid) : -1;
   const ItemList items{srow, s_sched, (int)blockIdx.x, (int)gridDim.x, nq * BH};
   if (tid == 0) {
-    for (int i = 0; i < 17; i++) tc::mbar_init(&bars[i], i == 16 ? 8 : 1);
+    for (int i = 0; i < 17; i++) tc::mbar_init(&bars[i], i == 16 ? BWD128_E_WARPS : 1);
     *s_abort = 0;
     tc::mbar_fence_init();
     tc::tma_prefetch_desc(&tm);
     tc::tma_prefetch_desc(&tm_do);
   }
-  if (warp == 8) tc::tmem_alloc(tmem_slot, 512);
+  if (warp == BWD128_MMA_WARP) tc::tmem_alloc(tmem_slot, 512);
   tc::tc_fence_before();
   __syncthreads();
   tc::tc_fence_after();
@@ -567,7 +583,7 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
     if (!tc::mbar_wait(bar, phase, where)) *s_abort = 1;
   };
   // item w = query tile (heaviest, the last, first) of (sample, head), with qt + 1 key blocks
-  if (warp == 9) {
+  if (warp == BWD128_LOAD_WARP) {
     if (lane == 0) {
       int g = 0;
       for (int li = 0, w; (w = items.at(li)) >= 0; li++) {
@@ -587,7 +603,7 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
         }
       }
     }
-  } else if (warp == 8) {
+  } else if (warp == BWD128_MMA_WARP) {
     if (lane == 0) {
       constexpr uint32_t idesc_s = tc::idesc_bf16(128, 128, 0, 0), idesc_g = tc::idesc_bf16(128, H128, 0, 1);
       const uint64_t dQ = desc_base_k(tc::smem_u32(smem + S::Q)), dO = desc_base_k(tc::smem_u32(smem + S::DO));
@@ -627,7 +643,7 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
           const uint64_t gK = gK0 + kr * T128_UNITS;
           const uint32_t t_ds = tmem + (g & 1) * 128;
 #pragma unroll
-          for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ts(t_dq, t_ds + half_col(ks), gK + off_mn(ks), idesc_g, (j > 0 || ks > 0));
+          for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ts(t_dq, t_ds + split_col(ks), gK + off_mn(ks), idesc_g, (j > 0 || ks > 0));
           tc::mma_commit(&bar_kf[kr]);
           kr = kr == 2 ? 0 : kr + 1;
           if (j + 2 < n) scores(g + 2);      // over dS(j), behind dQ(j)
@@ -636,67 +652,70 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
       }
     }
   } else {
-    const int lg = warp & 3, hf = warp >> 2, row = lg * 32 + lane;
+    const int lg = warp & 3, qd = warp >> 2, row = lg * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(lg * 32) << 16;
     const float sl2 = a.scale * LOG2E;
     int g = 0;
-    for (int li = 0, w; (w = items.at(li)) >= 0; li++) {
+    float next_nl = 0.f, next_delta = 0.f;      // this thread's query of the next item (fetched under the epilogue before it)
+    auto fetch = [&](int w) {
+      const int q = (nq - 1 - w / BH) * 128 + row;
+      const size_t e = (size_t)(w % BH) * a.T + q;
+      next_nl = q < a.T ? -a.lse[e] * LOG2E : -INFINITY;
+      next_delta = q < a.T ? a.delta[e] : 0.f;
+    };
+    int w = items.at(0);
+    if (w >= 0) fetch(w);
+    for (int li = 0; w >= 0; li++) {
       const int qt = nq - 1 - w / BH, bh = w % BH, b = bh / a.H, h = bh % a.H;
       const int qrow = qt * 128 + row;
-      const size_t si = ((size_t)b * a.H + h) * a.T + qrow;
-      const float nl = qrow < a.T ? -a.lse[si] * LOG2E : -INFINITY;
-      const float delta = qrow < a.T ? a.delta[si] : 0.f;
+      const float nl = next_nl, delta = next_delta;
       for (int j = 0; j <= qt; j++, g++) {
-        const uint32_t ts = tmem + (g & 1) * 128 + hf * 64 + lane_addr, tdp = t_dp + hf * 64 + lane_addr;
+        const uint32_t ts = tmem + (g & 1) * 128 + qd * 32 + lane_addr, tdp = t_dp + qd * 32 + lane_addr;
         wait(&bar_s[g & 1], (g >> 1) & 1, 79);
         __syncwarp();
         tc::tc_fence_after();
-        float p[64];
+        float p[32];
         {
-          uint32_t r[2][32];
-          tc::tmem_ld32(ts, r[0]);
-          tc::tmem_ld32(ts + 32, r[1]);
+          uint32_t r[32];
+          tc::tmem_ld32(ts, r);
           tc::tmem_ld_wait();
 #pragma unroll
-          for (int e = 0; e < 64; e++) p[e] = ex2_approx(fmaf(__uint_as_float(r[e >> 5][e & 31]), sl2, nl));
+          for (int e = 0; e < 32; e++) p[e] = ex2_approx(fmaf(__uint_as_float(r[e]), sl2, nl));
         }
         if (j == qt) {      // the diagonal block
 #pragma unroll
-          for (int e = 0; e < 64; e++)
-            if (hf * 64 + e > row) p[e] = 0.f;
+          for (int e = 0; e < 32; e++)
+            if (qd * 32 + e > row) p[e] = 0.f;
         }
         wait(bar_dp, g & 1, 80);
         __syncwarp();
         tc::tc_fence_after();
-        uint32_t d[2][32];
-        tc::tmem_ld32(tdp, d[0]);
-        tc::tmem_ld32(tdp + 32, d[1]);
+        uint32_t d[32], dw[16];
+        tc::tmem_ld32(tdp, d);
         tc::tmem_ld_wait();
 #pragma unroll
-        for (int c = 0; c < 2; c++) {
-          uint32_t dw[16];
-#pragma unroll
-          for (int x = 0; x < 16; x++) {
-            const int e = c * 32 + 2 * x;
-            dw[x] = pack_bf16(p[e] * (__uint_as_float(d[c][2 * x]) - delta), p[e + 1] * (__uint_as_float(d[c][2 * x + 1]) - delta));
-          }
-          tc::tmem_st16(ts + c * 16, dw);
-        }
+        for (int x = 0; x < 16; x++)
+          dw[x] = pack_bf16(p[2 * x] * (__uint_as_float(d[2 * x]) - delta), p[2 * x + 1] * (__uint_as_float(d[2 * x + 1]) - delta));
+        tc::tmem_st16(ts, dw);
         tc::tmem_st_wait();
         tc::tc_fence_before();
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(bar_ds);
       }
+      // ---- epilogue: 64 columns by each warp of quarters 0 and 1
+      w = items.at(li + 1);
+      if (w >= 0) fetch(w);
       wait(bar_done, li & 1, 81);
       __syncwarp();
       tc::tc_fence_after();
-      const bool live = qrow < a.T && !*s_abort;
-      bf16* dst = a.out + ((size_t)(b * a.T + (live ? qrow : 0))) * 3 * C + h * H128;
-      store_pairs_rope<H128>(dst, t_dq + lane_addr, hf * 32, live, a.cosT, a.sinT, qrow, a.scale);
+      if (qd < 2) {
+        bf16* dst = a.out + ((size_t)(b * a.T + qrow)) * 3 * C + h * H128;
+        store_pairs_rope<H128>(dst, 3L * C, t_dq + lane_addr, qd * 32, lane, *s_abort ? 0 : a.T - (qrow - lane), a.cosT, a.sinT, qrow, a.scale);
+      }
       tc::tc_fence_before();
     }
   }
   tc::tc_fence_before();
   __syncthreads();
-  if (warp == 8) tc::tmem_dealloc(tmem, 512);
+  if (warp == BWD128_MMA_WARP) tc::tmem_dealloc(tmem, 512);
 }

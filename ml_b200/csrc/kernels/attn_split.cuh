@@ -56,25 +56,27 @@ __device__ __forceinline__ void split_load(uint8_t* dst, const CUtensorMap* tm, 
     for (int i = 0; i < boxes; i++) tc::tma_load_3d(dst + (c * boxes + i) * BOX_BYTES, tm, bar, x0 + c * 64, r0 + i * 64, z);
 }
 
-// hd columns of this thread's TMEM row, times f, as bf16 to dst (16-byte aligned, hd a multiple of 16)
+// hd columns of the warp's 32 TMEM rows, times f, as bf16 to memory (16-byte aligned, hd a multiple of 16): dst = the lane's row,
+// rows `pitch` apart, nlive of them exist.  Whole warp.
 template <int HDT>
-__device__ __forceinline__ void split_store_row(bf16* dst, uint32_t taddr, int hd, float f, bool live) {
+__device__ __forceinline__ void split_store_rows(bf16* dst, long pitch, uint32_t taddr, int hd, float f, int lane, int nlive) {
 #pragma unroll
   for (int c = 0; c < HDT; c += 32) {
     uint32_t r[32];
-    tc::tmem_ld32(taddr + c, r);      // (warp-collective: every lane takes part, live or not)
+    tc::tmem_ld32(taddr + c, r);
     tc::tmem_ld_wait();
+    uint4 u[4];
 #pragma unroll
     for (int v = 0; v < 4; v++) {
-      if (live && c + v * 8 < hd) {
-        uint4 w;
-        w.x = pack_bf16(__uint_as_float(r[v * 8]) * f, __uint_as_float(r[v * 8 + 1]) * f);
-        w.y = pack_bf16(__uint_as_float(r[v * 8 + 2]) * f, __uint_as_float(r[v * 8 + 3]) * f);
-        w.z = pack_bf16(__uint_as_float(r[v * 8 + 4]) * f, __uint_as_float(r[v * 8 + 5]) * f);
-        w.w = pack_bf16(__uint_as_float(r[v * 8 + 6]) * f, __uint_as_float(r[v * 8 + 7]) * f);
-        *reinterpret_cast<uint4*>(dst + c + v * 8) = w;
-      }
+      const float* x = reinterpret_cast<const float*>(r) + v * 8;
+      u[v] = make_uint4(pack_bf16(x[0] * f, x[1] * f), pack_bf16(x[2] * f, x[3] * f), pack_bf16(x[4] * f, x[5] * f), pack_bf16(x[6] * f, x[7] * f));
     }
+    quad_transpose(u, lane);
+    const int q = lane & 3;
+    bf16* base = dst - q * pitch + c + q * 8;
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if ((lane & ~3) + k < nlive && c + q * 8 < hd) *reinterpret_cast<uint4*>(base + k * pitch) = u[k];
   }
 }
 
@@ -237,20 +239,27 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
     }
     tc::tc_fence_before();
   }
-  if (qrow < a.T && !*s_abort) {
-    const float inv = 1.f / l;
-    bf16* dst = a.out + ((size_t)b * a.T + qrow) * C + h * a.hd;
+  const float inv = 1.f / l;
+  const int lane = tid & 31, nlive = *s_abort ? 0 : a.T - (qrow - lane);
+  bf16* dst = a.out + ((size_t)b * a.T + qrow) * C + h * a.hd;
+  __syncwarp();
 #pragma unroll
-    for (int c = 0; c < HDT; c += 8) {
-      if (c < a.hd) {
-        uint4 w;
-        w.x = pack_bf16(o[c] * inv, o[c + 1] * inv); w.y = pack_bf16(o[c + 2] * inv, o[c + 3] * inv);
-        w.z = pack_bf16(o[c + 4] * inv, o[c + 5] * inv); w.w = pack_bf16(o[c + 6] * inv, o[c + 7] * inv);
-        *reinterpret_cast<uint4*>(dst + c) = w;
-      }
+  for (int c = 0; c < HDT; c += 32) {
+    uint4 u[4];
+#pragma unroll
+    for (int v = 0; v < 4; v++) {
+      const float* x = o + c + v * 8;
+      u[v] = make_uint4(pack_bf16(x[0] * inv, x[1] * inv), pack_bf16(x[2] * inv, x[3] * inv), pack_bf16(x[4] * inv, x[5] * inv),
+                        pack_bf16(x[6] * inv, x[7] * inv));
     }
-    a.lse[((size_t)b * a.H + h) * a.T + qrow] = (m + log2f(l)) * LN2;
+    quad_transpose(u, lane);
+    const int q = lane & 3;
+    bf16* base = dst - q * (long)C + c + q * 8;
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if ((lane & ~3) + k < nlive && c + q * 8 < a.hd) *reinterpret_cast<uint4*>(base + k * (long)C) = u[k];
   }
+  if (lane < nlive) a.lse[((size_t)b * a.H + h) * a.T + qrow] = (m + log2f(l)) * LN2;
   tc::tc_fence_before();
   __syncthreads();
   if (warp == 0) tc::tmem_dealloc(t_s, TMEM_COLS);
@@ -432,13 +441,14 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
   wait(bar_s, n & 1, 48);
   __syncwarp();
   tc::tc_fence_after();
-  const bool live = row < a.T && !*s_abort;
-  bf16* dst = a.out + ((size_t)b * a.T + (row < a.T ? row : 0)) * 3 * C + xh;
+  const int lane = tid & 31, nlive = *s_abort ? 0 : a.T - (row - lane);
+  bf16* dst = a.out + ((size_t)b * a.T + row) * 3 * C + xh;
+  __syncwarp();
   if (KV) {
-    split_store_row<HDT>(dst + C, t_a1 + lane_addr, a.hd, a.scale, live);
-    split_store_row<HDT>(dst + 2 * C, t_a0 + lane_addr, a.hd, 1.f, live);
+    split_store_rows<HDT>(dst + C, 3L * C, t_a1 + lane_addr, a.hd, a.scale, lane, nlive);
+    split_store_rows<HDT>(dst + 2 * C, 3L * C, t_a0 + lane_addr, a.hd, 1.f, lane, nlive);
   } else {
-    split_store_row<HDT>(dst, t_a0 + lane_addr, a.hd, a.scale, live);
+    split_store_rows<HDT>(dst, 3L * C, t_a0 + lane_addr, a.hd, a.scale, lane, nlive);
   }
   tc::tc_fence_before();
   __syncthreads();
