@@ -179,9 +179,12 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
           if (k0 + half * 32 + i > last) r[i] = 0xff800000u;
       }
     };
+    // (an encoder's sequence is a square and the class token: its last block has few keys, and the second half of it none)
+    const bool both = k0 + 32 < a.T;
     float mx = m;
 #pragma unroll
     for (int half = 0; half < 2; half++) {
+      if (half && !both) break;
       uint32_t r[32];
       load_scores(half, r);
 #pragma unroll
@@ -193,6 +196,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
     float rs = 0.f;
 #pragma unroll
     for (int half = 0; half < 2; half++) {
+      if (half && !both) break;
       uint32_t r[32], hi[16], lo[16];
       load_scores(half, r);
 #pragma unroll
@@ -216,6 +220,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
       if (!*s_abort) {
 #pragma unroll
         for (int ks = 0; ks < 4; ks++) {
+          if (ks >= 2 && !both) break;
           tc::mma_bf16_ts(t_o, t_s + split_col(ks), dV + off_mn(ks), idesc_o, ks > 0);
           tc::mma_bf16_ts(t_o, t_s + split_col(ks) + 16, dV + off_mn(ks), idesc_o, 1);
         }
@@ -380,8 +385,10 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
     if (tid == 0 && it + 1 < n) load_x(it + 1);      // every MMA issued so far is complete: the other buffer is free
     const int c0 = (i0 + it) * 64;
     const float* st = stat + (it & 1) * 128;
+    const bool both = c0 + 32 < a.T;      // (as in forward)
 #pragma unroll
     for (int half = 0; half < 2; half++) {
+      if (half && !both) break;
       uint32_t rs[32], rd[32];
       tc::tmem_ld32(t_s + half * 32 + lane_addr, rs);
       tc::tmem_ld32(t_d + half * 32 + lane_addr, rd);
@@ -420,6 +427,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
       if (!*s_abort) {
 #pragma unroll
         for (int ks = 0; ks < 4; ks++) {
+          if (ks >= 2 && !both) break;
           if (KV) {
             tc::mma_bf16_ts(t_a0, t_s + split_col(ks), sy + off_mn(ks), idesc_g, (it > 0 || ks > 0));
             tc::mma_bf16_ts(t_a0, t_s + split_col(ks) + 16, sy + off_mn(ks), idesc_g, 1);
