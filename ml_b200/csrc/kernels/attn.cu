@@ -12,6 +12,8 @@
 // unaligned pointers) uses a plain SIMT implementation further down.
 #include "../tc.cuh"
 #include <algorithm>
+#include <array>
+#include <map>
 #include <mutex>
 #include <queue>
 #include <vector>
@@ -2104,24 +2106,64 @@ MLB_API void mlb_attn_set_timeline(void* buf) { g_timeline = (long long*)buf; }
 // so far.  Forward, B=16 H=12 T=1024, 148 CTAs: round robin leaves the slowest CTA with 30 key-block steps where the
 // average is 26, this assignment gets 26.  Backward: 768 equal CTAs of 9 blocks each ran as 5.2 waves (54 blocks on the
 // slowest SM); 1536 single-tile items scheduled this way give 47.  The table lives in device memory, one row of `stride`
-// entries per CTA, -1 terminated (with room for a look-ahead of two items), cached per shape; it is built with a
-// blocking copy, so while the stream is being captured into a graph and the shape is new, nullptr is returned and the
-// kernels fall back to round robin.
-struct AttnSchedule { int kind, dev, B, H, T, grid, stride; int* table; };
+// entries per CTA, -1 terminated (with room for a look-ahead of two items), cached per shape.  It is copied on the stream
+// that will read it and waited for before anyone else can find it: a plain cudaMemcpy from pageable memory may return while
+// the copy is still on its way, and nothing orders a non-blocking stream behind it.  While the stream is being captured
+// into a graph and the shape is new there is no table and the kernels fall back to round robin.
+// At most SCHED_MAX tables (some 10 KB each) are kept; a further shape takes the place of the one unused for longest, which is
+// freed when the device has finished with it.  A graph holds the address of the table it was captured with, so those stay.
+struct AttnSchedule { int stride; int* table; bool captured; unsigned long long used; };
 static std::mutex g_sched_mu;
-static std::vector<AttnSchedule> g_sched;
+static std::map<std::array<int, 6>, AttnSchedule> g_sched;      // (kind, device, B, H, T, grid)
+static unsigned long long g_sched_clock = 0;
+constexpr size_t SCHED_MAX = 256;
 static int g_fwd_balance = 1;
 MLB_API void mlb_attn_fwd_balance(int on) { g_fwd_balance = on; }   // (both directions)
-static const int* attn_schedule(int kind /*0 forward pairs, 1 backward key tiles*/, int B, int H, int T, int grid, int* stride_out,
-                                cudaStream_t st) {
-  if (!g_fwd_balance) return nullptr;
+MLB_API int mlb_attn_schedule_count() {
+  std::lock_guard<std::mutex> lk(g_sched_mu);
+  return (int)g_sched.size();
+}
+// Keeps the cache as it is from the look-up to the launch that reads the table (until it goes out of scope)
+struct SchedUse {
+  std::unique_lock<std::mutex> lk;
+  const int* table = nullptr;
+  int stride = 0;
+};
+// Room for one more table; false if there is none to be had.  Called with the lock held.
+static bool attn_schedule_room() {
+  if (g_sched.size() < SCHED_MAX) return true;
+  auto oldest = g_sched.end();
+  for (auto it = g_sched.begin(); it != g_sched.end(); ++it)
+    if (!it->second.captured && (oldest == g_sched.end() || it->second.used < oldest->second.used)) oldest = it;
+  if (oldest == g_sched.end()) return false;
+  int cur = 0;
+  if (cudaGetDevice(&cur) != cudaSuccess || oldest->first[1] != cur) return false;      // (another device's: not worth switching for)
+  if (cudaDeviceSynchronize() != cudaSuccess) { cudaGetLastError(); return false; }
+  cudaFree(oldest->second.table);
+  g_sched.erase(oldest);
+  return true;
+}
+static SchedUse attn_schedule(int kind /*0 forward pairs, 1 backward key tiles*/, int B, int H, int T, int grid, cudaStream_t st) {
+  SchedUse use;
+  if (!g_fwd_balance) return use;
   int dev = 0;
   cudaGetDevice(&dev);
-  std::lock_guard<std::mutex> lk(g_sched_mu);
-  for (const AttnSchedule& e : g_sched)
-    if (e.kind == kind && e.dev == dev && e.B == B && e.H == H && e.T == T && e.grid == grid) { *stride_out = e.stride; return e.table; }
+  use.lk = std::unique_lock<std::mutex>(g_sched_mu);
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return nullptr;
+  const bool capturing = cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
+  const std::array<int, 6> key = {kind, dev, B, H, T, grid};
+  auto found = g_sched.find(key);
+  if (found != g_sched.end()) {
+    found->second.used = ++g_sched_clock;
+    found->second.captured |= capturing;
+    use.table = found->second.table;
+    use.stride = found->second.stride;
+    return use;
+  }
+  if (capturing) return use;
+  // allocating and waiting here must not break a capture that another thread has under way
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
   const int nq = (T + 127) / 128, npair = (nq + 1) / 2, BH = B * H;
   const int total = (kind == 0 ? npair : nq) * BH;
   std::vector<std::vector<int>> rows(grid);
@@ -2143,15 +2185,19 @@ static const int* attn_schedule(int kind /*0 forward pairs, 1 backward key tiles
   std::vector<int> host((size_t)grid * stride, -1);
   for (int c = 0; c < grid; c++) std::copy(rows[c].begin(), rows[c].end(), host.begin() + (size_t)c * stride);
   int* table = nullptr;
-  if (cudaMalloc(&table, host.size() * sizeof(int)) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-  if (cudaMemcpy(table, host.data(), host.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess) {
-    cudaGetLastError();
-    cudaFree(table);
-    return nullptr;
+  if (attn_schedule_room() && cudaMalloc(&table, host.size() * sizeof(int)) == cudaSuccess) {
+    if (cudaMemcpyAsync(table, host.data(), host.size() * sizeof(int), cudaMemcpyHostToDevice, st) == cudaSuccess &&
+        cudaStreamSynchronize(st) == cudaSuccess) {
+      g_sched[key] = {stride, table, false, ++g_sched_clock};
+      use.table = table;
+      use.stride = stride;
+    } else {
+      cudaFree(table);
+    }
   }
-  g_sched.push_back({kind, dev, B, H, T, grid, stride, table});
-  *stride_out = stride;
-  return table;
+  if (!use.table) cudaGetLastError();
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  return use;
 }
 
 // out[B,T,C], lse[B,H,T] from qkv[B,T,3C].
@@ -2174,7 +2220,9 @@ MLB_API int mlb_attn_fwd(void* out, float* lse, const void* qkv, int B, int T, i
       const long pairs = (long)(((T + 127) / 128 + 1) / 2) * H * B;
       const dim3 grid2((unsigned)(pairs < sms ? pairs : sms));
       a.dynamic = (g_attn_dynamic && g_fwd_rows != 1 && g_fwd_rows != 2) ? 1 : 0;      // (the default variant only)
-      a.sched = (pairs > sms && !a.dynamic) ? attn_schedule(0, B, H, T, (int)grid2.x, &a.sched_stride, st) : nullptr;
+      const SchedUse sched = (pairs > sms && !a.dynamic) ? attn_schedule(0, B, H, T, (int)grid2.x, st) : SchedUse{};
+      a.sched = sched.table;
+      a.sched_stride = sched.stride;
       const CUtensorMap* to = (T % 128 == 0 && g_fwd_rows >= 2) ? mlb_tmap_cached(out, (uint64_t)B * T, C, C, 32, 64, 2) : nullptr;
       a.out_tma = to != nullptr;
       if (!to) to = tm;      // unused by the kernel then
@@ -2208,7 +2256,9 @@ MLB_API int mlb_attn_fwd(void* out, float* lse, const void* qkv, int B, int T, i
       if (!to) to = tm;      // unused by the kernel then
       const long pairs = (long)(((T + 127) / 128 + 1) / 2) * H * B;
       const dim3 grid2((unsigned)(pairs < sms ? pairs : sms));
-      a.sched = pairs > sms ? attn_schedule(0, B, H, T, (int)grid2.x, &a.sched_stride, st) : nullptr;
+      const SchedUse sched = pairs > sms ? attn_schedule(0, B, H, T, (int)grid2.x, st) : SchedUse{};
+      a.sched = sched.table;
+      a.sched_stride = sched.stride;
       static int once = set_smem(attn_fwd128_k, Fwd128Smem::TOTAL);
       (void)once;
       mlb_launch_tmem(attn_fwd128_k, grid2, dim3(FWD128_THREADS), Fwd128Smem::TOTAL, st, *t3, *to, a);
@@ -2299,7 +2349,9 @@ static int attn_bwd_impl(void* dqkv, const void* dout, const void* qkv, const vo
       const long n_items = nqh * H * B;
       dim3 grid_f((unsigned)(n_items < sms ? n_items : sms));
       a.dynamic = g_attn_dynamic;
-      a.sched = (n_items > sms && !a.dynamic) ? attn_schedule(1, B, H, T, (int)grid_f.x, &a.sched_stride, st) : nullptr;
+      const SchedUse sched = (n_items > sms && !a.dynamic) ? attn_schedule(1, B, H, T, (int)grid_f.x, st) : SchedUse{};
+      a.sched = sched.table;
+      a.sched_stride = sched.stride;
       if (a.dynamic) mlb_launch_tmem(attn_bwd_fused_tc_kernel<true>, grid_f, dim3(BWDF_THREADS), BwdFusedSmem::TOTAL, st, *tq, *td, *tpart, a);
       else mlb_launch_tmem(attn_bwd_fused_tc_kernel<false>, grid_f, dim3(BWDF_THREADS), BwdFusedSmem::TOTAL, st, *tq, *td, *tpart, a);
       const long groups = (long)B * T * H * (hd / 32);
@@ -2328,7 +2380,9 @@ static int attn_bwd_impl(void* dqkv, const void* dout, const void* qkv, const vo
       const long n_items = (long)((T + 127) / 128) * H * B;
       const dim3 grid_p((unsigned)(n_items < sms ? n_items : sms));
       // one table for both: item w of either kernel has the same number of blocks
-      a.sched = n_items > sms ? attn_schedule(1, B, H, T, (int)grid_p.x, &a.sched_stride, st) : nullptr;
+      const SchedUse sched = n_items > sms ? attn_schedule(1, B, H, T, (int)grid_p.x, st) : SchedUse{};
+      a.sched = sched.table;
+      a.sched_stride = sched.stride;
       mlb_launch_tmem(attn_bwd_kv128_k, grid_p, dim3(BWD128_THREADS), BwdKV128Smem::TOTAL, st, *t3, *d3, a);
       mlb_launch_tmem(attn_bwd_q128_k, grid_p, dim3(BWD128_THREADS), BwdQ128Smem::TOTAL, st, *t3, *d3, a);
     }

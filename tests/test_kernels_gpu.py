@@ -988,3 +988,31 @@ def test_norm_backward_with_cast_column_sums(rows, C):
     y = torch.nn.functional.layer_norm(xd, (C,), wd, bd, 1e-5)
     gx, gw, gb = torch.autograd.grad(y, [xd, wd, bd], dy.double())
     assert _rel(dx, gx) < 2 ** -8 and _rel(dw, gw) < 2 ** -8 and _rel(db, gb) < 2 ** -8
+
+
+def test_attention_work_tables_are_bounded():
+    """More shapes than tables are kept: results of a shape whose table was given back, and of a graph that holds one, stay the same.
+    The first calls run on a stream of their own (its copy of the table is waited for)."""
+    n, B, hd = nat(), 160, 64
+    qkv = rnd(B * 300, 3 * hd)
+
+    def run(T):
+        out, lse = torch.empty(B * T, hd, device=dev(), dtype=torch.bfloat16), torch.empty(B, 1, T, device=dev())
+        n.attn_fwd(out, lse, qkv[:B * T], B, T, 1, hd)
+        return out, lse
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        first, _ = run(131)
+    side.synchronize()
+    assert _rel(first, _attn64(qkv[:B * 131], qkv[:B * 131, :hd], B, 131, 1, hd, True)[0]) < 2 ** -8
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        held, _ = run(131)
+    run(132)
+    for T in range(1, 300):
+        run(T)
+    assert 200 < n.lib().mlb_attn_schedule_count() <= 256
+    graph.replay()
+    assert torch.equal(held, first) and torch.equal(run(131)[0], first)
+    assert torch.equal(run(132)[0], run(132)[0])
