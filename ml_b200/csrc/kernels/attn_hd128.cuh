@@ -4,8 +4,9 @@
 // exponentials take the special-function units (2048 cycles each), and in backward the products lead (2048 / 1536 cycles against
 // 1024), so the kernels are built around never letting one wait for the other; tensor memory is the constraint (a 128 x 128
 // fp32 tile is 128 of its 512 columns).  P and dS are written as bf16 pairs over the score columns they came from and are read
-// from there as the A operand of the next product: no shared memory, and no columns of their own.  MMAs issued by one
-// thread run in order, so a product that overwrites such columns is simply issued behind the one that reads them.
+// from there as the A operand of the next product: no shared memory, and no columns of their own.  MMAs are promised to run in
+// the order of their issue only where accumulator and shape are the same, so a product that overwrites such columns is issued when
+// the one that reads them has completed (its commit is waited for).
 // All three kernels are persistent, one CTA per SM over a balanced table of items (attn_schedule); every wait is bounded and
 // sticky (after one expiry the CTA's later waits return at once and its roles still walk the same sequence of barriers).
 // Loads go through per-sequence tensor maps: rows past a sample's end are zeros.
@@ -126,9 +127,10 @@ __global__ void __maxnreg__(160) attn_fwd128_k(const __grid_constant__ CUtensorM
       for (int li = 0, w; (w = items.at(li)) >= 0; li++) {
         const Item it = item_of(w);
         const int n = blocks_of(it, t);
-        auto scores = [&](int j) {
+        auto scores = [&](int j, int pv) {      // over the columns that the tile's latest P V (number pv - 1) reads P from
           const int sl = (g + j) & 1;
           wait(&bar_k[sl], ((g + j) >> 1) & 1, 53);
+          if (pv > 0) wait(&bar_o[t], (pv - 1) & 1, 82);
           tc::tc_fence_after();
           const uint64_t dK = dK0 + sl * T128_UNITS;
 #pragma unroll
@@ -140,7 +142,7 @@ __global__ void __maxnreg__(160) attn_fwd128_k(const __grid_constant__ CUtensorM
         if (n > 0) {
           wait(&bar_q[t], cq & 1, 54);
           cq++;
-          scores(0);
+          scores(0, gt);
         }
         for (int j = 0; j < n; j++, gt++) {
           const int sl = (g + j) & 1;
@@ -156,7 +158,7 @@ __global__ void __maxnreg__(160) attn_fwd128_k(const __grid_constant__ CUtensorM
           for (int ks = 4; ks < 8; ks++) tc::mma_bf16_ts(t_o, t_s + ks * 8, dV + off_mn(ks), idesc_o, 1);
           tc::mma_commit(&bar_o[t]);
           tc::mma_commit(&bar_vf[sl]);
-          if (j + 1 < n) scores(j + 1);      // behind P V, which reads P out of these columns
+          if (j + 1 < n) scores(j + 1, gt + 1);
         }
         for (int j = n; j < it.nkb; j++) {      // blocks only the other tile sees: released once they have landed
           const int sl = (g + j) & 1, ph = ((g + j) >> 1) & 1;
@@ -409,16 +411,18 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
       int g = 0;
       for (int li = 0, w; (w = items.at(li)) >= 0; li++) {
         const int n = nq - w / BH;
-        auto scores = [&](int gb) {
+        auto scores = [&](int gb) {      // over P^T, which the block before's dV reads
           wait(&bar_q[gb & 1], (gb >> 1) & 1, 64);
+          if (gb > 0) wait(&bar_dof[(gb - 1) & 1], ((gb - 1) >> 1) & 1, 83);
           tc::tc_fence_after();
           const uint64_t dQ = dQ0 + (gb & 1) * T128_UNITS;
 #pragma unroll
           for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ss(t_s, dK + off_k(ks, TILE_BYTES), dQ + off_k(ks, TILE_BYTES), idesc_s, ks > 0);
           tc::mma_commit(bar_s);
         };
-        auto dprobs = [&](int gb, bool last) {
+        auto dprobs = [&](int gb, bool last) {      // over dS^T, which the block before's dK reads
           wait(&bar_do[gb & 1], (gb >> 1) & 1, 65);
+          if (gb > 0) wait(&bar_qf[(gb - 1) & 1], ((gb - 1) >> 1) & 1, 84);
           tc::tc_fence_after();
           const uint64_t dO = dO0 + (gb & 1) * T128_UNITS;
 #pragma unroll
@@ -612,9 +616,10 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
       int g = 0, kr = 0;      // kr = g % 3
       for (int li = 0, w; (w = items.at(li)) >= 0; li++) {
         const int n = nq - w / BH;
-        auto scores = [&](int gb) {
+        auto scores = [&](int gb) {      // over dS of block gb - 2, which its dQ reads
           const int sl = gb % 3;
           wait(&bar_k[sl], (gb / 3) & 1, 75);
+          if (gb > 1) wait(&bar_kf[(gb - 2) % 3], ((gb - 2) / 3) & 1, 85);
           tc::tc_fence_after();
           const uint64_t dK = dK0 + sl * T128_UNITS;
           const uint32_t t_s = tmem + (gb & 1) * 128;
@@ -646,7 +651,7 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
           for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ts(t_dq, t_ds + split_col(ks), gK + off_mn(ks), idesc_g, (j > 0 || ks > 0));
           tc::mma_commit(&bar_kf[kr]);
           kr = kr == 2 ? 0 : kr + 1;
-          if (j + 2 < n) scores(g + 2);      // over dS(j), behind dQ(j)
+          if (j + 2 < n) scores(g + 2);
           if (j + 1 == n) tc::mma_commit(bar_done);
         }
       }

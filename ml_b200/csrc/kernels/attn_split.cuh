@@ -12,8 +12,8 @@
 // memory is spent on them and two (backward) to four (forward) CTAs share an SM: their MMAs, exponentials and loads
 // overlap across CTAs, which is why a CTA by itself is a plain sequence.  What bounds it is that sequence's latency, not a
 // unit.  64-row blocks because the encoder's sequences are short (197 tokens = 3.1 blocks of 64, 1.5 of 128).
-// The next block's scores overwrite those columns: one thread's MMAs run in order only as long as they have the same shape (head
-// size 64: all are 128 x 64 x 16); at the other sizes the products that read the columns are waited for first.
+// The next block's scores overwrite those columns.  MMAs are promised to run in the order of their issue only where accumulator and
+// shape are the same, so the products that read the columns are waited for first.
 // Sequences are the third dimension of the tensor maps: rows past a sample's end arrive as zeros, never as the next
 // sample's values (0 * inf would be NaN).
 struct SplitArgs {
@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
       }
       tc::mma_commit(bar_o);
       if (j + 1 < nkb) {      // these scores replace P, which the product above reads
-        if (a.hd != 64) wait(bar_o, j & 1, 44);
+        wait(bar_o, j & 1, 44);
         issue_s(j + 1);
       }
     }
@@ -437,10 +437,8 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
         }
       }
       if (it + 1 < n) {      // these scores replace p and g, which the products above read
-        if (a.hd != 64) {
-          tc::mma_commit(bar_g);
-          wait(bar_g, it & 1, 49);
-        }
+        tc::mma_commit(bar_g);
+        wait(bar_g, it & 1, 49);
         issue_scores(it + 1);
       }
       tc::mma_commit(bar_s);
