@@ -314,8 +314,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_tc_kernel(const __gri
       for (int i = 0; i < OC; i++) o[i] = 0.f;
       auto fold = [&](int gb, float alpha) {   // O = O * alpha + (P V) of block gb
         uint32_t ro[16];
-        tc::tmem_ld16(t_o + (gb & 1) * HD + lane_addr + cq * 16, ro);
-        tc::tmem_ld_wait();
+        tc::tmem_ld16_wait(t_o + (gb & 1) * HD + lane_addr + cq * 16, ro);
 #pragma unroll
         for (int i = 0; i < 16; i++) o[i] = o[i] * alpha + __uint_as_float(ro[i]);
         tc::tc_fence_before();
@@ -326,8 +325,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_tc_kernel(const __gri
         if (!have_scores) {   // first block of this CTA: nothing was prefetched
           wait(&bar_s[sl], (g >> 1) & 1, 17);
           tc::tc_fence_after();
-          tc::tmem_ld32(tmem + sl * 128 + lane_addr + cq * 32, r);
-          tc::tmem_ld_wait();
+          tc::tmem_ld32_wait(tmem + sl * 128 + lane_addr + cq * 32, r);
           have_scores = true;
         }
         float mx = -INFINITY;
@@ -383,8 +381,9 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_tc_kernel(const __gri
           wait(&bar_o[(g - 1) & 1], ((g - 1) >> 1) & 1, 18);
           tc::tc_fence_after();
           fold(g - 1, alpha_prev);     // its tcgen05.wait::ld also covers the score prefetch
+          tc::tmem_ld_tie(r);
         } else if (more) {
-          tc::tmem_ld_wait();
+          tc::tmem_ld_wait(r);
         }
         alpha_prev = alpha;
       }
@@ -752,9 +751,7 @@ __global__ void __maxnreg__(160) attn_fwd_rows_tc_kernel(const __grid_constant__
       auto fold = [&](float alpha) {   // O = O * alpha + (P V) of the previous block
         if constexpr (!LAZY) {
           uint32_t r0[32], r1[32];
-          tc::tmem_ld32(t_o, r0);
-          tc::tmem_ld32(t_o + 32, r1);
-          tc::tmem_ld_wait();
+          tc::tmem_ld32x2_wait(t_o, r0, t_o + 32, r1);
           tc::tc_fence_before();
           __syncwarp();
           if (lane == 0) tc::mbar_arrive(&bar_of[t]);
@@ -769,8 +766,7 @@ __global__ void __maxnreg__(160) attn_fwd_rows_tc_kernel(const __grid_constant__
 #pragma unroll
         for (int c = 0; c < 2; c++) {
           uint32_t r[32], w0[16], w1[16];
-          tc::tmem_ld32(t_o + c * 32, r);
-          tc::tmem_ld_wait();
+          tc::tmem_ld32_wait(t_o + c * 32, r);
 #pragma unroll
           for (int i = 0; i < 16; i++) {
             w0[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
@@ -833,8 +829,7 @@ __global__ void __maxnreg__(160) attn_fwd_rows_tc_kernel(const __grid_constant__
 #pragma unroll
                 for (int c = 0; c < 4; c++) {
                   uint32_t r[32];
-                  tc::tmem_ld32(t_s + c * 32, r);
-                  tc::tmem_ld_wait();
+                  tc::tmem_ld32_wait(t_s + c * 32, r);
                   mask(c, r);
 #pragma unroll
                   for (int i = 0; i < 32; i += 2) mx = max3(mx, __uint_as_float(r[i]), __uint_as_float(r[i + 1]));
@@ -867,13 +862,12 @@ __global__ void __maxnreg__(160) attn_fwd_rows_tc_kernel(const __grid_constant__
               // done, and S is handed back to the MMA thread there - the next block's Q K^T runs under the second half
               // of this block's exponentials instead of after them.
               uint32_t ra[32], rb[32], pw0[16], pw1[16];
-              tc::tmem_ld32(t_s, ra);
-              tc::tmem_ld_wait();
+              tc::tmem_ld32_wait(t_s, ra);
               mask(0, ra);
               tc::tmem_ld32(t_s + 32, rb);
               exps(ra, pw0, std::true_type{});
               if (tl && g < 16) tl[g * 8 + 2] = clock64();     // mode 3: stamps 2..5 = chunks done
-              tc::tmem_ld_wait();
+              tc::tmem_ld_wait(rb);
               mask(1, rb);
               tc::tmem_ld32(t_s + 64, ra);
               free_p();
@@ -881,8 +875,8 @@ __global__ void __maxnreg__(160) attn_fwd_rows_tc_kernel(const __grid_constant__
               exps(rb, pw1, std::true_type{});
               tc::tmem_st16(t_p + 16, pw1);
               if (tl && g < 16) tl[g * 8 + 3] = clock64();
-              tc::tmem_ld32(t_s + 96, rb);
-              tc::tmem_ld_wait();
+              tc::tmem_ld32_wait(t_s + 96, rb);
+              tc::tmem_ld_tie(ra);
               mask(2, ra);
               mask(3, rb);
               if (!exact) {
@@ -933,8 +927,7 @@ __global__ void __maxnreg__(160) attn_fwd_rows_tc_kernel(const __grid_constant__
 #pragma unroll
           for (int c = 0; c < 4; c++) {
             uint32_t r[32];
-            tc::tmem_ld32(t_s + c * 32, r);
-            tc::tmem_ld_wait();
+            tc::tmem_ld32_wait(t_s + c * 32, r);
             if (diag) {
 #pragma unroll
               for (int i = 0; i < 32; i++)
@@ -987,8 +980,7 @@ __global__ void __maxnreg__(160) attn_fwd_rows_tc_kernel(const __grid_constant__
 #pragma unroll
           for (int c = 0; c < 4; c++) {
             uint32_t r[32], pw[16];
-            tc::tmem_ld32(t_s + c * 32, r);
-            tc::tmem_ld_wait();
+            tc::tmem_ld32_wait(t_s + c * 32, r);
 #pragma unroll
             for (int x = 0; x < 16; x++) {
               float z0, z1;
@@ -1037,8 +1029,7 @@ __global__ void __maxnreg__(160) attn_fwd_rows_tc_kernel(const __grid_constant__
   #pragma unroll
         for (int c = 0; c < 2; c++) {
           uint32_t r[32];
-          tc::tmem_ld32(t_o + c * 32, r);
-          tc::tmem_ld_wait();
+          tc::tmem_ld32_wait(t_o + c * 32, r);
 #pragma unroll
           for (int v8 = 0; v8 < 4; v8++) {
             uint4 pk;
@@ -1162,9 +1153,7 @@ template <int HD>
 __device__ __forceinline__ void store_pairs_rope(bf16* dst_row, long pitch, uint32_t taddr, int c0, int lane, int nlive, const float* cosT,
                                                  const float* sinT, int t, float out_scale = 1.f) {
   uint32_t ra[32], rb[32];
-  tc::tmem_ld32(taddr + c0, ra);
-  tc::tmem_ld32(taddr + c0 + HD / 2, rb);
-  tc::tmem_ld_wait();
+  tc::tmem_ld32x2_wait(taddr + c0, ra, taddr + c0 + HD / 2, rb);
   float x0[32], x1[32];
 #pragma unroll
   for (int i = 0; i < 32; i++) { x0[i] = __uint_as_float(ra[i]) * out_scale; x1[i] = __uint_as_float(rb[i]) * out_scale; }
@@ -1299,9 +1288,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kv_tc_kernel(const __
     const bool diag = (it == 0);
     {
       uint32_t rs[32], rd[32];
-      tc::tmem_ld32(t_st + lane_addr + cq * 32, rs);
-      tc::tmem_ld32(t_dpt + lane_addr + cq * 32, rd);
-      tc::tmem_ld_wait();
+      tc::tmem_ld32x2_wait(t_st + lane_addr + cq * 32, rs, t_dpt + lane_addr + cq * 32, rd);
 #pragma unroll
       for (int v8 = 0; v8 < 4; v8++) {
         float p[8], ds[8];
@@ -1654,9 +1641,7 @@ __global__ void __maxnreg__(120) attn_bwd_fused_tc_kernel(const __grid_constant_
         for (int hf = 0; hf < 2; hf++) {
           uint32_t rs[32], rd[32];
           const int c0 = ch * 64 + hf * 32;      // first query column of this pass
-          tc::tmem_ld32(t_st + lane_addr + c0, rs);
-          tc::tmem_ld32(t_dpt + lane_addr + c0, rd);
-          tc::tmem_ld_wait();
+          tc::tmem_ld32x2_wait(t_st + lane_addr + c0, rs, t_dpt + lane_addr + c0, rd);
           if (hf == 1) {
             tc::tc_fence_before();
             __syncwarp();
@@ -1730,9 +1715,7 @@ __global__ void __maxnreg__(120) attn_bwd_fused_tc_kernel(const __grid_constant_
         wait(&bar_d[blk & 1], (blk >> 1) & 1, 50);          // dV, dK, dQ MMAs of this block are complete
         tc::tc_fence_after();
         uint32_t r0[32], r1[32];
-        tc::tmem_ld32(t_dq + lane_addr, r0);
-        tc::tmem_ld32(t_dq + lane_addr + 32, r1);
-        tc::tmem_ld_wait();
+        tc::tmem_ld32x2_wait(t_dq + lane_addr, r0, t_dq + lane_addr + 32, r1);
         tc::tc_fence_before();
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(bar_dqf);
@@ -1929,9 +1912,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_q_tc_kernel(const __g
     const bool diag = (j == qt);
     {
       uint32_t rs[32], rd[32];
-      tc::tmem_ld32(t_s + lane_addr + cq * 32, rs);
-      tc::tmem_ld32(t_dp + lane_addr + cq * 32, rd);
-      tc::tmem_ld_wait();
+      tc::tmem_ld32x2_wait(t_s + lane_addr + cq * 32, rs, t_dp + lane_addr + cq * 32, rd);
 #pragma unroll
       for (int v8 = 0; v8 < 4; v8++) {
         float ds[8];

@@ -189,9 +189,7 @@ __global__ void __maxnreg__(160) attn_fwd128_k(const __grid_constant__ CUtensorM
         __syncwarp();
         tc::tc_fence_after();
         uint32_t r[4][32];
-#pragma unroll
-        for (int c = 0; c < 4; c++) tc::tmem_ld32(t_s + c * 32, r[c]);
-        tc::tmem_ld_wait();
+        tc::tmem_ld32x4_wait(t_s, r);
         if (j == n - 1) {      // the diagonal block
 #pragma unroll
           for (int i = 0; i < 128; i++)
@@ -215,8 +213,7 @@ __global__ void __maxnreg__(160) attn_fwd128_k(const __grid_constant__ CUtensorM
 #pragma unroll
           for (int c = 0; c < 8; c++) {
             uint32_t o[16];
-            tc::tmem_ld16(t_o + c * 16, o);
-            tc::tmem_ld_wait();
+            tc::tmem_ld16_wait(t_o + c * 16, o);
 #pragma unroll
             for (int i = 0; i < 16; i++) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
             tc::tmem_st16(t_o + c * 16, o);
@@ -280,8 +277,7 @@ __global__ void __maxnreg__(160) attn_fwd128_k(const __grid_constant__ CUtensorM
 #pragma unroll
         for (int c = 0; c < 2; c++) {
           uint32_t o[32];
-          tc::tmem_ld32(t_o + half * 64 + c * 32, o);
-          tc::tmem_ld_wait();
+          tc::tmem_ld32_wait(t_o + half * 64 + c * 32, o);
 #pragma unroll
           for (int v = 0; v < 4; v++) {
             uint4 x;
@@ -488,8 +484,7 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
         float p[32];
         {
           uint32_t r[32];
-          tc::tmem_ld32(ts, r);
-          tc::tmem_ld_wait();
+          tc::tmem_ld32_wait(ts, r);
 #pragma unroll
           for (int e = 0; e < 32; e += 4) {
             const float4 L = *reinterpret_cast<const float4*>(st + e);
@@ -517,8 +512,7 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
         tc::tc_fence_after();
         {
           uint32_t d[32];
-          tc::tmem_ld32(tdp, d);
-          tc::tmem_ld_wait();
+          tc::tmem_ld32_wait(tdp, d);
 #pragma unroll
           for (int e = 0; e < 32; e += 4) {
             const float4 D = *reinterpret_cast<const float4*>(st + 32 + e);
@@ -682,8 +676,7 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
         float p[32];
         {
           uint32_t r[32];
-          tc::tmem_ld32(ts, r);
-          tc::tmem_ld_wait();
+          tc::tmem_ld32_wait(ts, r);
 #pragma unroll
           for (int e = 0; e < 32; e++) p[e] = ex2_approx(fmaf(__uint_as_float(r[e]), sl2, nl));
         }
@@ -696,8 +689,7 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
         __syncwarp();
         tc::tc_fence_after();
         uint32_t d[32], dw[16];
-        tc::tmem_ld32(tdp, d);
-        tc::tmem_ld_wait();
+        tc::tmem_ld32_wait(tdp, d);
 #pragma unroll
         for (int x = 0; x < 16; x++)
           dw[x] = pack_bf16(p[2 * x] * (__uint_as_float(d[2 * x]) - delta), p[2 * x + 1] * (__uint_as_float(d[2 * x + 1]) - delta));

@@ -63,8 +63,7 @@ __device__ __forceinline__ void split_store_rows(bf16* dst, long pitch, uint32_t
 #pragma unroll
   for (int c = 0; c < HDT; c += 32) {
     uint32_t r[32];
-    tc::tmem_ld32(taddr + c, r);
-    tc::tmem_ld_wait();
+    tc::tmem_ld32_wait(taddr + c, r);
     uint4 u[4];
 #pragma unroll
     for (int v = 0; v < 4; v++) {
@@ -171,8 +170,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
     // the scores are read twice, 32 at a time (once for the maximum): a row's 64 in registers on top of its HDT output columns
     // would cost a resident CTA
     auto load_scores = [&](int half, uint32_t (&r)[32]) {
-      tc::tmem_ld32(t_s + half * 32 + lane_addr, r);
-      tc::tmem_ld_wait();
+      tc::tmem_ld32_wait(t_s + half * 32 + lane_addr, r);
       if (k0 + half * 32 + 31 > last) {
 #pragma unroll
         for (int i = 0; i < 32; i++)
@@ -237,8 +235,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
 #pragma unroll
     for (int c = 0; c < HDT; c += 32) {
       uint32_t ro[32];
-      tc::tmem_ld32(t_o + c + lane_addr, ro);
-      tc::tmem_ld_wait();
+      tc::tmem_ld32_wait(t_o + c + lane_addr, ro);
 #pragma unroll
       for (int i = 0; i < 32; i++) o[c + i] = fmaf(o[c + i], alpha, __uint_as_float(ro[i]));
     }
@@ -390,9 +387,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
     for (int half = 0; half < 2; half++) {
       if (half && !both) break;
       uint32_t rs[32], rd[32];
-      tc::tmem_ld32(t_s + half * 32 + lane_addr, rs);
-      tc::tmem_ld32(t_d + half * 32 + lane_addr, rd);
-      tc::tmem_ld_wait();
+      tc::tmem_ld32x2_wait(t_s + half * 32 + lane_addr, rs, t_d + half * 32 + lane_addr, rd);
       uint32_t hi[16], lo[16], gh[16], gl[16];
 #pragma unroll
       for (int i = 0; i < 16; i++) {

@@ -163,7 +163,105 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
       : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// A tcgen05.ld's registers hold their values once wait::ld has returned, and the wait names no registers: with the two in separate
+// statements nothing keeps the compiler from moving arithmetic on the registers in front of the wait.  So load and wait are one
+// statement, whose outputs are defined when it is over (early clobber where a later load's address is still to be read).
+__device__ __forceinline__ void tmem_ld16_wait(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld32_wait(uint32_t taddr, uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
+        "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
+        "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld32x2_wait(uint32_t taddr_a, uint32_t (&a)[32], uint32_t taddr_b, uint32_t (&b)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%64];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, "
+      "%48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%65];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=&r"(a[0]), "=&r"(a[1]), "=&r"(a[2]), "=&r"(a[3]), "=&r"(a[4]), "=&r"(a[5]), "=&r"(a[6]), "=&r"(a[7]), "=&r"(a[8]),
+        "=&r"(a[9]),
+        "=&r"(a[10]), "=&r"(a[11]), "=&r"(a[12]), "=&r"(a[13]), "=&r"(a[14]), "=&r"(a[15]), "=&r"(a[16]), "=&r"(a[17]), "=&r"(a[18]),
+        "=&r"(a[19]), "=&r"(a[20]), "=&r"(a[21]), "=&r"(a[22]), "=&r"(a[23]), "=&r"(a[24]), "=&r"(a[25]), "=&r"(a[26]), "=&r"(a[27]),
+        "=&r"(a[28]), "=&r"(a[29]), "=&r"(a[30]), "=&r"(a[31]), "=&r"(b[0]), "=&r"(b[1]), "=&r"(b[2]), "=&r"(b[3]), "=&r"(b[4]),
+        "=&r"(b[5]), "=&r"(b[6]), "=&r"(b[7]), "=&r"(b[8]), "=&r"(b[9]), "=&r"(b[10]), "=&r"(b[11]), "=&r"(b[12]), "=&r"(b[13]),
+        "=&r"(b[14]), "=&r"(b[15]), "=&r"(b[16]), "=&r"(b[17]), "=&r"(b[18]), "=&r"(b[19]), "=&r"(b[20]), "=&r"(b[21]), "=&r"(b[22]),
+        "=&r"(b[23]), "=&r"(b[24]), "=&r"(b[25]), "=&r"(b[26]), "=&r"(b[27]), "=&r"(b[28]), "=&r"(b[29]), "=&r"(b[30]), "=&r"(b[31])
+      : "r"(taddr_a), "r"(taddr_b)
+      : "memory");
+}
+// 128 consecutive columns
+__device__ __forceinline__ void tmem_ld32x4_wait(uint32_t taddr, uint32_t (&r)[4][32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%128];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, "
+      "%48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%129];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%64, %65, %66, %67, %68, %69, %70, %71, %72, %73, %74, %75, %76, %77, %78, %79, "
+      "%80, %81, %82, %83, %84, %85, %86, %87, %88, %89, %90, %91, %92, %93, %94, %95}, [%130];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%96, %97, %98, %99, %100, %101, %102, %103, %104, %105, %106, %107, %108, %109, %110, %111, "
+      "%112, %113, %114, %115, %116, %117, %118, %119, %120, %121, %122, %123, %124, %125, %126, %127}, [%131];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=&r"(r[0][0]), "=&r"(r[0][1]), "=&r"(r[0][2]), "=&r"(r[0][3]), "=&r"(r[0][4]), "=&r"(r[0][5]), "=&r"(r[0][6]), "=&r"(r[0][7]),
+        "=&r"(r[0][8]), "=&r"(r[0][9]), "=&r"(r[0][10]), "=&r"(r[0][11]), "=&r"(r[0][12]), "=&r"(r[0][13]), "=&r"(r[0][14]),
+        "=&r"(r[0][15]), "=&r"(r[0][16]), "=&r"(r[0][17]), "=&r"(r[0][18]), "=&r"(r[0][19]), "=&r"(r[0][20]), "=&r"(r[0][21]),
+        "=&r"(r[0][22]), "=&r"(r[0][23]), "=&r"(r[0][24]), "=&r"(r[0][25]), "=&r"(r[0][26]), "=&r"(r[0][27]), "=&r"(r[0][28]),
+        "=&r"(r[0][29]), "=&r"(r[0][30]), "=&r"(r[0][31]), "=&r"(r[1][0]), "=&r"(r[1][1]), "=&r"(r[1][2]), "=&r"(r[1][3]),
+        "=&r"(r[1][4]), "=&r"(r[1][5]), "=&r"(r[1][6]), "=&r"(r[1][7]), "=&r"(r[1][8]), "=&r"(r[1][9]), "=&r"(r[1][10]),
+        "=&r"(r[1][11]), "=&r"(r[1][12]), "=&r"(r[1][13]), "=&r"(r[1][14]), "=&r"(r[1][15]), "=&r"(r[1][16]), "=&r"(r[1][17]),
+        "=&r"(r[1][18]), "=&r"(r[1][19]), "=&r"(r[1][20]), "=&r"(r[1][21]), "=&r"(r[1][22]), "=&r"(r[1][23]), "=&r"(r[1][24]),
+        "=&r"(r[1][25]), "=&r"(r[1][26]), "=&r"(r[1][27]), "=&r"(r[1][28]), "=&r"(r[1][29]), "=&r"(r[1][30]), "=&r"(r[1][31]),
+        "=&r"(r[2][0]), "=&r"(r[2][1]), "=&r"(r[2][2]), "=&r"(r[2][3]), "=&r"(r[2][4]), "=&r"(r[2][5]), "=&r"(r[2][6]), "=&r"(r[2][7]),
+        "=&r"(r[2][8]), "=&r"(r[2][9]), "=&r"(r[2][10]), "=&r"(r[2][11]), "=&r"(r[2][12]), "=&r"(r[2][13]), "=&r"(r[2][14]),
+        "=&r"(r[2][15]), "=&r"(r[2][16]), "=&r"(r[2][17]), "=&r"(r[2][18]), "=&r"(r[2][19]), "=&r"(r[2][20]), "=&r"(r[2][21]),
+        "=&r"(r[2][22]), "=&r"(r[2][23]), "=&r"(r[2][24]), "=&r"(r[2][25]), "=&r"(r[2][26]), "=&r"(r[2][27]), "=&r"(r[2][28]),
+        "=&r"(r[2][29]), "=&r"(r[2][30]), "=&r"(r[2][31]), "=&r"(r[3][0]), "=&r"(r[3][1]), "=&r"(r[3][2]), "=&r"(r[3][3]),
+        "=&r"(r[3][4]), "=&r"(r[3][5]), "=&r"(r[3][6]), "=&r"(r[3][7]), "=&r"(r[3][8]), "=&r"(r[3][9]), "=&r"(r[3][10]),
+        "=&r"(r[3][11]), "=&r"(r[3][12]), "=&r"(r[3][13]), "=&r"(r[3][14]), "=&r"(r[3][15]), "=&r"(r[3][16]), "=&r"(r[3][17]),
+        "=&r"(r[3][18]), "=&r"(r[3][19]), "=&r"(r[3][20]), "=&r"(r[3][21]), "=&r"(r[3][22]), "=&r"(r[3][23]), "=&r"(r[3][24]),
+        "=&r"(r[3][25]), "=&r"(r[3][26]), "=&r"(r[3][27]), "=&r"(r[3][28]), "=&r"(r[3][29]), "=&r"(r[3][30]), "=&r"(r[3][31])
+      : "r"(taddr), "r"(taddr + 32), "r"(taddr + 64), "r"(taddr + 96)
+      : "memory");
+}
+// The wait by itself, for a load that other work goes on under: the empty statements behind it take the loaded registers in and out
+// again, and all uses come after them (a copy of each register, so only where the overlap is worth more).
+template <int N>
+__device__ __forceinline__ void tmem_ld_tie(uint32_t (&r)[N]) {
+  static_assert(N % 8 == 0, "whole groups of eight");
+#pragma unroll
+  for (int i = 0; i < N; i += 8)
+    asm volatile("" : "+r"(r[i]), "+r"(r[i + 1]), "+r"(r[i + 2]), "+r"(r[i + 3]), "+r"(r[i + 4]), "+r"(r[i + 5]), "+r"(r[i + 6]), "+r"(r[i + 7]));
+}
+// r: every array loaded since the last wait
+template <typename... R>
+__device__ __forceinline__ void tmem_ld_wait(R&... r) {
+  static_assert(sizeof...(R) > 0, "name the loaded registers");
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+  (tmem_ld_tie(r), ...);
+}
 
 // ------------------------------------------------------------------ descriptors
 // Shared-memory matrix descriptor, 128-byte swizzle (the layout TMA writes with CU_TENSOR_MAP_SWIZZLE_128B;
