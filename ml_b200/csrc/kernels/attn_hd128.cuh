@@ -8,7 +8,9 @@
 // the order of their issue only where accumulator and shape are the same, so a product that overwrites such columns is issued when
 // the one that reads them has completed (its commit is waited for).
 // All three kernels are persistent, one CTA per SM over a balanced table of items (attn_schedule); every wait is bounded and
-// sticky (after one expiry the CTA's later waits return at once and its roles still walk the same sequence of barriers).
+// sticky: after one expiry the CTA's later waits return at once, its loader and MMA threads stop, and the element-wise warps walk on to
+// the common end.  Loader and MMA threads come there when what they have issued is complete (attn_settle), whatever happened.
+// (At the end itself, for all warps, that costs the dK / dV kernel registers: 353 us instead of 345.)
 // Loads go through per-sequence tensor maps: rows past a sample's end are zeros.
 constexpr int H128 = 128;
 constexpr int T128_BYTES = 2 * TILE_BYTES;      // one [128 x 128] bf16 tile: two 64-column chunks
@@ -54,8 +56,9 @@ __global__ void __maxnreg__(160) attn_fwd128_k(const __grid_constant__ CUtensorM
   uint64_t *bar_q = bars, *bar_qf = bars + 2, *bar_k = bars + 4, *bar_kf = bars + 6, *bar_v = bars + 8, *bar_vf = bars + 10, *bar_s = bars + 12,
            *bar_pa = bars + 14, *bar_pb = bars + 16, *bar_o = bars + 18;      // [2] each: per tile (q, s, p, o) or slot (k, v)
   volatile int* s_turn = (volatile int*)(bars + 20);      // [2][4]: blocks whose exponentials tile t's warp on sub-partition lg has taken
-  uint32_t* tmem_slot = (uint32_t*)(bars + 24);
-  volatile int* s_abort = (volatile int*)(bars + 25);
+  uint64_t* bar_end = bars + 24;      // [2]: the MMA threads' last commits
+  uint32_t* tmem_slot = (uint32_t*)(bars + 26);
+  volatile int* s_abort = (volatile int*)(bars + 27);
   if (attn_given_up()) return;
   const int nq = (a.T + 127) / 128, npair = (nq + 1) / 2, BH = a.B * a.H, C = a.H * H128;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -67,7 +70,7 @@ __global__ void __maxnreg__(160) attn_fwd128_k(const __grid_constant__ CUtensorM
     for (int i = 0; i < 2; i++) {
       tc::mbar_init(&bar_q[i], 1); tc::mbar_init(&bar_qf[i], 1); tc::mbar_init(&bar_k[i], 1); tc::mbar_init(&bar_kf[i], 2);
       tc::mbar_init(&bar_v[i], 1); tc::mbar_init(&bar_vf[i], 2); tc::mbar_init(&bar_s[i], 1); tc::mbar_init(&bar_pa[i], 4);
-      tc::mbar_init(&bar_pb[i], 4); tc::mbar_init(&bar_o[i], 1);
+      tc::mbar_init(&bar_pb[i], 4); tc::mbar_init(&bar_o[i], 1); tc::mbar_init(&bar_end[i], 1);
     }
     for (int i = 0; i < 8; i++) s_turn[i] = 0;
     *s_abort = 0;
@@ -80,9 +83,12 @@ __global__ void __maxnreg__(160) attn_fwd128_k(const __grid_constant__ CUtensorM
   __syncthreads();
   tc::tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  auto wait = [&](uint64_t* bar, uint32_t phase, int where) {
-    if (tc::mbar_try(bar, phase) || *s_abort) return;
-    if (!tc::mbar_wait(bar, phase, where)) *s_abort = 1;
+  auto wait = [&](uint64_t* bar, uint32_t phase, int where) -> bool {
+    if (tc::mbar_try(bar, phase)) return true;
+    if (*s_abort) return false;
+    if (tc::mbar_wait(bar, phase, where)) return true;
+    *s_abort = 1;
+    return false;
   };
   // item w = pair (heaviest first) of (sample, head); tile t of it has n(t) key blocks (none when the pair has no second tile)
   struct Item { int pair, b, h, nkb; };
@@ -94,26 +100,32 @@ __global__ void __maxnreg__(160) attn_fwd128_k(const __grid_constant__ CUtensorM
 
   if (warp == 9) {
     if (lane == 0) {
-      int g = 0, cq[2] = {0, 0};
-      for (int li = 0, w; (w = items.at(li)) >= 0; li++) {
+      int g = 0, cq[2] = {0, 0}, odd = 0;      // odd: a K without its V
+      bool ok = true;
+      for (int li = 0, w; ok && (w = items.at(li)) >= 0; li++) {
         const Item it = item_of(w);
         auto load_q = [&](int t) {
-          if (blocks_of(it, t) == 0) return;
-          if (cq[t] > 0) wait(&bar_qf[t], (cq[t] - 1) & 1, 50);
+          if (blocks_of(it, t) == 0 || !ok) return;
+          if (cq[t] > 0 && !wait(&bar_qf[t], (cq[t] - 1) & 1, 50)) { ok = false; return; }
           cq[t]++;
           tc::mbar_expect_tx(&bar_q[t], T128_BYTES);
           split_load<2>(smem + S::Q + t * T128_BYTES, &tm, &bar_q[t], it.h * H128, (2 * it.pair + t) * 128, it.b, 2);
         };
         for (int j = 0; j < it.nkb; j++, g++) {
           const int sl = g & 1, ph = ((g >> 1) + 1) & 1;
-          if (g >= 2) wait(&bar_kf[sl], ph, 51);
+          if (!ok || (g >= 2 && !wait(&bar_kf[sl], ph, 51))) { ok = false; break; }
           tc::mbar_expect_tx(&bar_k[sl], T128_BYTES);
           split_load<2>(smem + S::K + sl * T128_BYTES, &tm, &bar_k[sl], C + it.h * H128, j * 128, it.b, 2);
           if (j == 0) { load_q(0); load_q(1); }
-          if (g >= 2) wait(&bar_vf[sl], ph, 52);
+          if (!ok || (g >= 2 && !wait(&bar_vf[sl], ph, 52))) { ok = false; odd = 1; break; }
           tc::mbar_expect_tx(&bar_v[sl], T128_BYTES);
           split_load<2>(smem + S::V + sl * T128_BYTES, &tm, &bar_v[sl], 2 * C + it.h * H128, j * 128, it.b, 2);
         }
+      }
+      for (int i = 0; i < 2; i++) {
+        attn_settle(&bar_q[i], cq[i]);
+        attn_settle(&bar_k[i], (g + odd + 1 - i) / 2);
+        attn_settle(&bar_v[i], (g + 1 - i) / 2);
       }
     }
   } else if (warp == 8 || warp == 10) {
@@ -124,13 +136,13 @@ __global__ void __maxnreg__(160) attn_fwd128_k(const __grid_constant__ CUtensorM
       const uint64_t dQ = desc_base_k(tc::smem_u32(smem + S::Q + t * T128_BYTES)), dK0 = desc_base_k(tc::smem_u32(smem + S::K)),
                      dV0 = desc_base_mn(tc::smem_u32(smem + S::V));
       int g = 0, gt = 0, cq = 0;
-      for (int li = 0, w; (w = items.at(li)) >= 0; li++) {
+      bool ok = true;
+      for (int li = 0, w; ok && (w = items.at(li)) >= 0; li++) {
         const Item it = item_of(w);
         const int n = blocks_of(it, t);
         auto scores = [&](int j, int pv) {      // over the columns that the tile's latest P V (number pv - 1) reads P from
           const int sl = (g + j) & 1;
-          wait(&bar_k[sl], ((g + j) >> 1) & 1, 53);
-          if (pv > 0) wait(&bar_o[t], (pv - 1) & 1, 82);
+          if (!ok || !wait(&bar_k[sl], ((g + j) >> 1) & 1, 53) || (pv > 0 && !wait(&bar_o[t], (pv - 1) & 1, 82))) { ok = false; return; }
           tc::tc_fence_after();
           const uint64_t dK = dK0 + sl * T128_UNITS;
 #pragma unroll
@@ -140,19 +152,18 @@ __global__ void __maxnreg__(160) attn_fwd128_k(const __grid_constant__ CUtensorM
           if (j == n - 1) tc::mma_commit(&bar_qf[t]);
         };
         if (n > 0) {
-          wait(&bar_q[t], cq & 1, 54);
+          ok = wait(&bar_q[t], cq & 1, 54);
           cq++;
           scores(0, gt);
         }
         for (int j = 0; j < n; j++, gt++) {
           const int sl = (g + j) & 1;
           const uint64_t dV = dV0 + sl * T128_UNITS;
-          wait(&bar_v[sl], ((g + j) >> 1) & 1, 55);
-          wait(&bar_pa[t], gt & 1, 56);
+          if (!ok || !wait(&bar_v[sl], ((g + j) >> 1) & 1, 55) || !wait(&bar_pa[t], gt & 1, 56)) { ok = false; break; }
           tc::tc_fence_after();
 #pragma unroll
           for (int ks = 0; ks < 4; ks++) tc::mma_bf16_ts(t_o, t_s + ks * 8, dV + off_mn(ks), idesc_o, (j > 0 || ks > 0));
-          wait(&bar_pb[t], gt & 1, 57);
+          if (!wait(&bar_pb[t], gt & 1, 57)) { ok = false; break; }
           tc::tc_fence_after();
 #pragma unroll
           for (int ks = 4; ks < 8; ks++) tc::mma_bf16_ts(t_o, t_s + ks * 8, dV + off_mn(ks), idesc_o, 1);
@@ -160,15 +171,17 @@ __global__ void __maxnreg__(160) attn_fwd128_k(const __grid_constant__ CUtensorM
           tc::mma_commit(&bar_vf[sl]);
           if (j + 1 < n) scores(j + 1, gt + 1);
         }
-        for (int j = n; j < it.nkb; j++) {      // blocks only the other tile sees: released once they have landed
+        for (int j = n; ok && j < it.nkb; j++) {      // blocks only the other tile sees: released once they have landed
           const int sl = (g + j) & 1, ph = ((g + j) >> 1) & 1;
-          wait(&bar_k[sl], ph, 53);
+          if (!wait(&bar_k[sl], ph, 53)) { ok = false; break; }
           tc::mbar_arrive(&bar_kf[sl]);
-          wait(&bar_v[sl], ph, 55);
+          if (!wait(&bar_v[sl], ph, 55)) { ok = false; break; }
           tc::mbar_arrive(&bar_vf[sl]);
         }
         g += it.nkb;
       }
+      tc::mma_commit(&bar_end[t]);
+      attn_settle(&bar_end[t], 1);
     }
   } else {
     const int t = warp >> 2, lg = warp & 3, row = lg * 32 + lane;
@@ -351,8 +364,9 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
   uint64_t* bars = (uint64_t*)(smem + S::BAR);
   uint64_t *bar_kv = bars, *bar_kvf = bars + 1, *bar_q = bars + 2 /*[2]*/, *bar_qf = bars + 4 /*[2]*/, *bar_do = bars + 6 /*[2]*/, *bar_dof = bars + 8 /*[2]*/,
            *bar_s = bars + 10, *bar_dp = bars + 11, *bar_p = bars + 12, *bar_ds = bars + 13, *bar_done = bars + 14;
-  uint32_t* tmem_slot = (uint32_t*)(bars + 15);
-  volatile int* s_abort = (volatile int*)(bars + 16);
+  uint64_t* bar_end = bars + 15;      // the MMA thread's last commit
+  uint32_t* tmem_slot = (uint32_t*)(bars + 16);
+  volatile int* s_abort = (volatile int*)(bars + 17);
   if (attn_given_up()) return;
   const int nq = (a.T + 127) / 128, BH = a.B * a.H, C = a.H * H128;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -361,7 +375,7 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
   if (srow && tid < 64) s_sched[tid] = tid < a.sched_stride ? __ldg(srow + tid) : -1;
   const ItemList items{srow, s_sched, (int)blockIdx.x, (int)gridDim.x, nq * BH};
   if (tid == 0) {
-    for (int i = 0; i < 15; i++) tc::mbar_init(&bars[i], (i == 12 || i == 13) ? BWD128_E_WARPS : 1);
+    for (int i = 0; i < 16; i++) tc::mbar_init(&bars[i], (i == 12 || i == 13) ? BWD128_E_WARPS : 1);
     *s_abort = 0;
     tc::mbar_fence_init();
     tc::tma_prefetch_desc(&tm);
@@ -373,29 +387,39 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
   tc::tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const uint32_t t_s = tmem, t_dp = tmem + 128, t_dv = tmem + 256, t_dk = tmem + 384;
-  auto wait = [&](uint64_t* bar, uint32_t phase, int where) {
-    if (tc::mbar_try(bar, phase) || *s_abort) return;
-    if (!tc::mbar_wait(bar, phase, where)) *s_abort = 1;
+  auto wait = [&](uint64_t* bar, uint32_t phase, int where) -> bool {
+    if (tc::mbar_try(bar, phase)) return true;
+    if (*s_abort) return false;
+    if (tc::mbar_wait(bar, phase, where)) return true;
+    *s_abort = 1;
+    return false;
   };
   // item w = key tile (heaviest, the first, first) of (sample, head)
   if (warp == BWD128_LOAD_WARP) {
     if (lane == 0) {
-      int g = 0;
-      for (int li = 0, w; (w = items.at(li)) >= 0; li++) {
+      int g = 0, nkv = 0, odd = 0;      // odd: a Q without its dO
+      bool ok = true;
+      for (int li = 0, w; ok && (w = items.at(li)) >= 0; li++) {
         const int kt = w / BH, bh = w % BH, b = bh / a.H, xh = (bh % a.H) * H128;
-        if (li > 0) wait(bar_kvf, (li - 1) & 1, 61);
+        if (li > 0 && !wait(bar_kvf, (li - 1) & 1, 61)) break;
+        nkv++;
         tc::mbar_expect_tx(bar_kv, 2 * T128_BYTES);
         split_load<2>(smem + S::K, &tm, bar_kv, C + xh, kt * 128, b, 2);
         split_load<2>(smem + S::V, &tm, bar_kv, 2 * C + xh, kt * 128, b, 2);
         for (int i = kt; i < nq; i++, g++) {
           const int sl = g & 1, ph = ((g >> 1) + 1) & 1;
-          if (g >= 2) wait(&bar_qf[sl], ph, 62);
+          if (g >= 2 && !wait(&bar_qf[sl], ph, 62)) { ok = false; break; }
           tc::mbar_expect_tx(&bar_q[sl], T128_BYTES);
           split_load<2>(smem + S::Q + sl * T128_BYTES, &tm, &bar_q[sl], xh, i * 128, b, 2);
-          if (g >= 2) wait(&bar_dof[sl], ph, 63);
+          if (g >= 2 && !wait(&bar_dof[sl], ph, 63)) { ok = false; odd = 1; break; }
           tc::mbar_expect_tx(&bar_do[sl], T128_BYTES);
           split_load<2>(smem + S::DO + sl * T128_BYTES, &tm_do, &bar_do[sl], xh, i * 128, b, 2);
         }
+      }
+      attn_settle(bar_kv, nkv);
+      for (int i = 0; i < 2; i++) {
+        attn_settle(&bar_q[i], (g + odd + 1 - i) / 2);
+        attn_settle(&bar_do[i], (g + 1 - i) / 2);
       }
     }
   } else if (warp == BWD128_MMA_WARP) {
@@ -405,11 +429,11 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
       const uint64_t dQ0 = desc_base_k(tc::smem_u32(smem + S::Q)), dO0 = desc_base_k(tc::smem_u32(smem + S::DO));      // as B of the scores
       const uint64_t gQ0 = desc_base_mn(tc::smem_u32(smem + S::Q)), gO0 = desc_base_mn(tc::smem_u32(smem + S::DO));    // as B of the gradients
       int g = 0;
-      for (int li = 0, w; (w = items.at(li)) >= 0; li++) {
+      bool ok = true;
+      for (int li = 0, w; ok && (w = items.at(li)) >= 0; li++) {
         const int n = nq - w / BH;
         auto scores = [&](int gb) {      // over P^T, which the block before's dV reads
-          wait(&bar_q[gb & 1], (gb >> 1) & 1, 64);
-          if (gb > 0) wait(&bar_dof[(gb - 1) & 1], ((gb - 1) >> 1) & 1, 83);
+          if (!ok || !wait(&bar_q[gb & 1], (gb >> 1) & 1, 64) || (gb > 0 && !wait(&bar_dof[(gb - 1) & 1], ((gb - 1) >> 1) & 1, 83))) { ok = false; return; }
           tc::tc_fence_after();
           const uint64_t dQ = dQ0 + (gb & 1) * T128_UNITS;
 #pragma unroll
@@ -417,8 +441,7 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
           tc::mma_commit(bar_s);
         };
         auto dprobs = [&](int gb, bool last) {      // over dS^T, which the block before's dK reads
-          wait(&bar_do[gb & 1], (gb >> 1) & 1, 65);
-          if (gb > 0) wait(&bar_qf[(gb - 1) & 1], ((gb - 1) >> 1) & 1, 84);
+          if (!ok || !wait(&bar_do[gb & 1], (gb >> 1) & 1, 65) || (gb > 0 && !wait(&bar_qf[(gb - 1) & 1], ((gb - 1) >> 1) & 1, 84))) { ok = false; return; }
           tc::tc_fence_after();
           const uint64_t dO = dO0 + (gb & 1) * T128_UNITS;
 #pragma unroll
@@ -426,19 +449,19 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
           tc::mma_commit(bar_dp);
           if (last) tc::mma_commit(bar_kvf);
         };
-        wait(bar_kv, li & 1, 66);
+        ok = wait(bar_kv, li & 1, 66);
         scores(g);
         dprobs(g, n == 1);
         for (int i = 0; i < n; i++, g++) {
           const int sl = g & 1;
           const uint64_t gQ = gQ0 + sl * T128_UNITS, gO = gO0 + sl * T128_UNITS;
-          wait(bar_p, g & 1, 67);      // (of an item's first block: also the accumulators of the previous item have been read out)
+          if (!ok || !wait(bar_p, g & 1, 67)) { ok = false; break; }      // (of an item's first block: also the accumulators of the previous item have been read out)
           tc::tc_fence_after();
 #pragma unroll
           for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ts(t_dv, t_s + split_col(ks), gO + off_mn(ks), idesc_g, (i > 0 || ks > 0));
           tc::mma_commit(&bar_dof[sl]);
           if (i + 1 < n) scores(g + 1);
-          wait(bar_ds, g & 1, 68);
+          if (!ok || !wait(bar_ds, g & 1, 68)) { ok = false; break; }
           tc::tc_fence_after();
 #pragma unroll
           for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ts(t_dk, t_dp + split_col(ks), gQ + off_mn(ks), idesc_g, (i > 0 || ks > 0));
@@ -447,6 +470,8 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
           else tc::mma_commit(bar_done);
         }
       }
+      tc::mma_commit(bar_end);
+      attn_settle(bar_end, 1);
     }
   } else {
     const int lg = warp & 3, qd = warp >> 2, row = lg * 32 + lane;
@@ -554,8 +579,9 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
   uint64_t* bars = (uint64_t*)(smem + S::BAR);
   uint64_t *bar_x = bars, *bar_xf = bars + 1, *bar_k = bars + 2 /*[3]*/, *bar_kf = bars + 5 /*[3]*/, *bar_v = bars + 8 /*[2]*/, *bar_vf = bars + 10 /*[2]*/,
            *bar_s = bars + 12 /*[2]*/, *bar_dp = bars + 14, *bar_done = bars + 15, *bar_ds = bars + 16;
-  uint32_t* tmem_slot = (uint32_t*)(bars + 17);
-  volatile int* s_abort = (volatile int*)(bars + 18);
+  uint64_t* bar_end = bars + 17;      // the MMA thread's last commit
+  uint32_t* tmem_slot = (uint32_t*)(bars + 18);
+  volatile int* s_abort = (volatile int*)(bars + 19);
   if (attn_given_up()) return;
   const int nq = (a.T + 127) / 128, BH = a.B * a.H, C = a.H * H128;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -564,7 +590,7 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
   if (srow && tid < 64) s_sched[tid] = tid < a.sched_stride ? __ldg(srow + tid) : -1;
   const ItemList items{srow, s_sched, (int)blockIdx.x, (int)gridDim.x, nq * BH};
   if (tid == 0) {
-    for (int i = 0; i < 17; i++) tc::mbar_init(&bars[i], i == 16 ? BWD128_E_WARPS : 1);
+    for (int i = 0; i < 18; i++) tc::mbar_init(&bars[i], i == 16 ? BWD128_E_WARPS : 1);
     *s_abort = 0;
     tc::mbar_fence_init();
     tc::tma_prefetch_desc(&tm);
@@ -576,30 +602,38 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
   tc::tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const uint32_t t_dp = tmem + 256, t_dq = tmem + 384;      // S buffers at +0 and +128
-  auto wait = [&](uint64_t* bar, uint32_t phase, int where) {
-    if (tc::mbar_try(bar, phase) || *s_abort) return;
-    if (!tc::mbar_wait(bar, phase, where)) *s_abort = 1;
+  auto wait = [&](uint64_t* bar, uint32_t phase, int where) -> bool {
+    if (tc::mbar_try(bar, phase)) return true;
+    if (*s_abort) return false;
+    if (tc::mbar_wait(bar, phase, where)) return true;
+    *s_abort = 1;
+    return false;
   };
   // item w = query tile (heaviest, the last, first) of (sample, head), with qt + 1 key blocks
   if (warp == BWD128_LOAD_WARP) {
     if (lane == 0) {
-      int g = 0;
-      for (int li = 0, w; (w = items.at(li)) >= 0; li++) {
+      int g = 0, nx = 0, odd = 0;      // odd: a K without its V
+      bool ok = true;
+      for (int li = 0, w; ok && (w = items.at(li)) >= 0; li++) {
         const int qt = nq - 1 - w / BH, bh = w % BH, b = bh / a.H, xh = (bh % a.H) * H128;
-        if (li > 0) wait(bar_xf, (li - 1) & 1, 72);
+        if (li > 0 && !wait(bar_xf, (li - 1) & 1, 72)) break;
+        nx++;
         tc::mbar_expect_tx(bar_x, 2 * T128_BYTES);
         split_load<2>(smem + S::Q, &tm, bar_x, xh, qt * 128, b, 2);
         split_load<2>(smem + S::DO, &tm_do, bar_x, xh, qt * 128, b, 2);
         for (int j = 0; j <= qt; j++, g++) {
           const int ks = g % 3, vs = g & 1;
-          if (g >= 3) wait(&bar_kf[ks], (g / 3 + 1) & 1, 73);
+          if (g >= 3 && !wait(&bar_kf[ks], (g / 3 + 1) & 1, 73)) { ok = false; break; }
           tc::mbar_expect_tx(&bar_k[ks], T128_BYTES);
           split_load<2>(smem + S::K + ks * T128_BYTES, &tm, &bar_k[ks], C + xh, j * 128, b, 2);
-          if (g >= 2) wait(&bar_vf[vs], ((g >> 1) + 1) & 1, 74);
+          if (g >= 2 && !wait(&bar_vf[vs], ((g >> 1) + 1) & 1, 74)) { ok = false; odd = 1; break; }
           tc::mbar_expect_tx(&bar_v[vs], T128_BYTES);
           split_load<2>(smem + S::V + vs * T128_BYTES, &tm, &bar_v[vs], 2 * C + xh, j * 128, b, 2);
         }
       }
+      attn_settle(bar_x, nx);
+      for (int i = 0; i < 3; i++) attn_settle(&bar_k[i], (g + odd + 2 - i) / 3);
+      for (int i = 0; i < 2; i++) attn_settle(&bar_v[i], (g + 1 - i) / 2);
     }
   } else if (warp == BWD128_MMA_WARP) {
     if (lane == 0) {
@@ -608,12 +642,12 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
       const uint64_t dK0 = desc_base_k(tc::smem_u32(smem + S::K)), dV0 = desc_base_k(tc::smem_u32(smem + S::V));
       const uint64_t gK0 = desc_base_mn(tc::smem_u32(smem + S::K));      // as B of dQ
       int g = 0, kr = 0;      // kr = g % 3
-      for (int li = 0, w; (w = items.at(li)) >= 0; li++) {
+      bool ok = true;
+      for (int li = 0, w; ok && (w = items.at(li)) >= 0; li++) {
         const int n = nq - w / BH;
         auto scores = [&](int gb) {      // over dS of block gb - 2, which its dQ reads
           const int sl = gb % 3;
-          wait(&bar_k[sl], (gb / 3) & 1, 75);
-          if (gb > 1) wait(&bar_kf[(gb - 2) % 3], ((gb - 2) / 3) & 1, 85);
+          if (!ok || !wait(&bar_k[sl], (gb / 3) & 1, 75) || (gb > 1 && !wait(&bar_kf[(gb - 2) % 3], ((gb - 2) / 3) & 1, 85))) { ok = false; return; }
           tc::tc_fence_after();
           const uint64_t dK = dK0 + sl * T128_UNITS;
           const uint32_t t_s = tmem + (gb & 1) * 128;
@@ -622,7 +656,7 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
           tc::mma_commit(&bar_s[gb & 1]);
         };
         auto dprobs = [&](int gb, bool last) {
-          wait(&bar_v[gb & 1], (gb >> 1) & 1, 76);
+          if (!ok || !wait(&bar_v[gb & 1], (gb >> 1) & 1, 76)) { ok = false; return; }
           tc::tc_fence_after();
           const uint64_t dV = dV0 + (gb & 1) * T128_UNITS;
 #pragma unroll
@@ -631,12 +665,12 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
           tc::mma_commit(&bar_vf[gb & 1]);
           if (last) tc::mma_commit(bar_xf);      // (the last scores were issued before)
         };
-        wait(bar_x, li & 1, 77);
+        ok = wait(bar_x, li & 1, 77);
         scores(g);
         if (n > 1) scores(g + 1);
         dprobs(g, n == 1);
         for (int j = 0; j < n; j++, g++) {
-          wait(bar_ds, g & 1, 78);      // dP(j) read, dS(j) stored (of an item's first block: the previous dQ read out)
+          if (!ok || !wait(bar_ds, g & 1, 78)) { ok = false; break; }      // dP(j) read, dS(j) stored (of an item's first block: the previous dQ read out)
           tc::tc_fence_after();
           if (j + 1 < n) dprobs(g + 1, j + 2 == n);
           const uint64_t gK = gK0 + kr * T128_UNITS;
@@ -649,6 +683,8 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
           if (j + 1 == n) tc::mma_commit(bar_done);
         }
       }
+      tc::mma_commit(bar_end);
+      attn_settle(bar_end, 1);
     }
   } else {
     const int lg = warp & 3, qd = warp >> 2, row = lg * 32 + lane;

@@ -49,6 +49,15 @@ __device__ __forceinline__ bool attn_given_up() {
   return s_skip != 0;
 }
 
+// A CTA one of whose waits has run out loads and multiplies nothing more.  What its threads have already issued still uses its shared
+// and tensor memory, so before they are given back the issuing thread waits, 2 ms at most, for the last of it: `begun` phases of a
+// barrier that counts a load's bytes or a commit (each begun when the one before was complete).
+__device__ __forceinline__ void attn_settle(uint64_t* bar, int begun) {
+  if (begun <= 0) return;
+  const uint64_t t0 = tc::globaltimer_ns();
+  while (!tc::mbar_try(bar, (begun - 1) & 1) && tc::globaltimer_ns() - t0 < 2000000) { }
+}
+
 // rows [r0, r0 + 64 * boxes) of `CH` 64-column chunks starting at column x0 of sample z
 template <int CH>
 __device__ __forceinline__ void split_load(uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, int x0, int r0, int z, int boxes) {
@@ -97,9 +106,9 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = (uint64_t*)(smem + S::BAR);
-  uint64_t *bar_q = bars, *bar_k = bars + 1 /*[2]*/, *bar_v = bars + 3 /*[2]*/, *bar_s = bars + 5, *bar_o = bars + 6;
-  uint32_t* tmem_slot = (uint32_t*)(bars + 7);
-  volatile int* s_abort = (volatile int*)(bars + 8);
+  uint64_t *bar_q = bars, *bar_k = bars + 1 /*[2]*/, *bar_v = bars + 3 /*[2]*/, *bar_s = bars + 5, *bar_o = bars + 6, *bar_end = bars + 7;
+  uint32_t* tmem_slot = (uint32_t*)(bars + 8);
+  volatile int* s_abort = (volatile int*)(bars + 9);
   if (attn_given_up()) return;
 
   const int ntile = (a.T + 127) / 128;
@@ -107,7 +116,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
   const int q0 = qt * 128, C = a.H * a.hd;
   const int tid = threadIdx.x, warp = tid >> 5;
   if (tid == 0) {
-    for (int i = 0; i < 7; i++) tc::mbar_init(&bars[i], 1);
+    for (int i = 0; i < 8; i++) tc::mbar_init(&bars[i], 1);
     *s_abort = 0;
     tc::mbar_fence_init();
     tc::tma_prefetch_desc(&tm);
@@ -129,8 +138,10 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
   const int nks = a.hd >> 4;
   const uint64_t dQ = desc_base_k(tc::smem_u32(smem + S::Q)), dK0 = desc_base_k(tc::smem_u32(smem + S::K)),
                  dV0 = desc64_base_mn(tc::smem_u32(smem + S::V));
+  int loads = 0;      // blocks of K and V asked for (thread 0)
   auto load_kv = [&](int j) {
     const int sl = j & 1;
+    loads = j + 1;
     tc::mbar_expect_tx(&bar_k[sl], CH * BOX_BYTES);
     split_load<CH>(smem + S::K + sl * CH * BOX_BYTES, &tm, &bar_k[sl], C + h * a.hd, j * 64, b, 1);
     tc::mbar_expect_tx(&bar_v[sl], CH * BOX_BYTES);
@@ -161,7 +172,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
 #pragma unroll
   for (int i = 0; i < HDT; i++) o[i] = 0.f;
   for (int j = 0; j < nkb; j++) {
-    if (tid == 0 && j + 1 < nkb) load_kv(j + 1);     // (block j - 1, the buffers' last reader, is complete: bar_o of it was waited for)
+    if (tid == 0 && j + 1 < nkb && !*s_abort) load_kv(j + 1);     // (block j - 1, the buffers' last reader, is complete: bar_o of it was waited for)
     wait(bar_s, j & 1, 42);
     __syncwarp();
     tc::tc_fence_after();
@@ -264,6 +275,18 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
   if (lane < nlive) a.lse[((size_t)b * a.H + h) * a.T + qrow] = (m + log2f(l)) * LN2;
   tc::tc_fence_before();
   __syncthreads();
+  if (*s_abort) {
+    if (tid == 0) {
+      tc::mma_commit(bar_end);
+      attn_settle(bar_end, 1);
+      attn_settle(bar_q, 1);
+      for (int sl = 0; sl < 2; sl++) {
+        attn_settle(&bar_k[sl], (loads + 1 - sl) / 2);
+        attn_settle(&bar_v[sl], (loads + 1 - sl) / 2);
+      }
+    }
+    __syncthreads();
+  }
   if (warp == 0) tc::tmem_dealloc(t_s, TMEM_COLS);
 }
 
@@ -292,9 +315,9 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = (uint64_t*)(smem + S::BAR);
-  uint64_t *bar_r = bars, *bar_x = bars + 1 /*[2]*/, *bar_s = bars + 3, *bar_g = bars + 4;
-  uint32_t* tmem_slot = (uint32_t*)(bars + 5);
-  volatile int* s_abort = (volatile int*)(bars + 6);
+  uint64_t *bar_r = bars, *bar_x = bars + 1 /*[2]*/, *bar_s = bars + 3, *bar_g = bars + 4, *bar_end = bars + 5;
+  uint32_t* tmem_slot = (uint32_t*)(bars + 6);
+  volatile int* s_abort = (volatile int*)(bars + 7);
   float* stat = (float*)(smem + S::STAT);
   if (attn_given_up()) return;
 
@@ -303,7 +326,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
   const int tile = KV ? (int)blockIdx.x : ntile - 1 - (int)blockIdx.x, h = blockIdx.y, b = blockIdx.z;   // (causal: longest first)
   const int r0 = tile * 128, C = a.H * a.hd, xh = h * a.hd;
   if (tid == 0) {
-    for (int i = 0; i < 5; i++) tc::mbar_init(&bars[i], 1);
+    for (int i = 0; i < 6; i++) tc::mbar_init(&bars[i], 1);
     *s_abort = 0;
     tc::mbar_fence_init();
     tc::tma_prefetch_desc(&tm);
@@ -329,8 +352,10 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
   const uint64_t drx = desc_base_k(tc::smem_u32(smem + S::RX)), dry = desc_base_k(tc::smem_u32(smem + S::RY));
   const uint64_t dsx = desc_base_k(tc::smem_u32(smem + S::SX)), dsy = desc_base_k(tc::smem_u32(smem + S::SY));      // as B of the scores
   const uint64_t gsx = desc64_base_mn(tc::smem_u32(smem + S::SX)), gsy = desc64_base_mn(tc::smem_u32(smem + S::SY));   // as B of the gradients
+  int loads = 0;      // streamed blocks asked for (thread 0)
   auto load_x = [&](int it) {
     const int sl = it & 1, y = (i0 + it) * 64;
+    loads = it + 1;
     tc::mbar_expect_tx(&bar_x[sl], 2 * CH * BOX_BYTES);
     split_load<CH>(smem + S::SX + sl * CH * BOX_BYTES, &tm, &bar_x[sl], KV ? xh : C + xh, y, b, 1);
     split_load<CH>(smem + S::SY + sl * CH * BOX_BYTES, KV ? &tm_do : &tm, &bar_x[sl], KV ? xh : 2 * C + xh, y, b, 1);
@@ -379,7 +404,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
     wait(bar_s, it & 1, 47);
     __syncwarp();
     tc::tc_fence_after();
-    if (tid == 0 && it + 1 < n) load_x(it + 1);      // every MMA issued so far is complete: the other buffer is free
+    if (tid == 0 && it + 1 < n && !*s_abort) load_x(it + 1);      // every MMA issued so far is complete: the other buffer is free
     const int c0 = (i0 + it) * 64;
     const float* st = stat + (it & 1) * 128;
     const bool both = c0 + 32 < a.T;      // (as in forward)
@@ -453,6 +478,15 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
   }
   tc::tc_fence_before();
   __syncthreads();
+  if (*s_abort) {
+    if (tid == 0) {
+      tc::mma_commit(bar_end);
+      attn_settle(bar_end, 1);
+      attn_settle(bar_r, 1);
+      for (int sl = 0; sl < 2; sl++) attn_settle(&bar_x[sl], (loads + 1 - sl) / 2);
+    }
+    __syncthreads();
+  }
   if (warp == 0) tc::tmem_dealloc(t_s, TMEM_COLS);
 }
 
