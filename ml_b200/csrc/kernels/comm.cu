@@ -263,7 +263,7 @@ __device__ __forceinline__ void ddp_bucket_body(const BucketArgs& a) {
 template <int GM>
 __global__ void __maxnreg__(32) ddp_bucket_lean_kernel(const BucketArgs a) { ddp_bucket_body<GM>(a); }
 template <int GM>
-__global__ void __launch_bounds__(256) ddp_bucket_kernel(const BucketArgs a) { ddp_bucket_body<GM>(a); }
+__global__ void __launch_bounds__(256, 4) ddp_bucket_kernel(const BucketArgs a) { ddp_bucket_body<GM>(a); }
 
 // All-gather by peer loads: dst[w*chunk_bytes ...] = shard of rank w, for every w; 16-byte vectors, system-scope loads.
 // No barrier is needed here: the producer of the shards (the reduce-scatter + AdamW kernel of the previous step) ends
@@ -316,10 +316,31 @@ __global__ void flag_timeout_probe_kernel(const int* flag, int epoch, long limit
 
 MLB_API int mlb_comm_max_world() { return MAX_WORLD; }
 
+// Largest grid of a bucket kernel, 0 = any.  In the bf16 modes a CTA that has finished its part of the staging copy waits until the
+// LAST CTA of the grid has (that one opens the entry barrier), so the whole grid has to be resident; half of what the
+// machine holds, so that two engines' kernels (decoder and vision tower) are resident together: at 64 registers and 256 threads two
+// CTAs per SM.  In the fp32 modes CTA 0 opens it, which waits for nobody.
+template <typename K>
+static int half_resident(K kern, int threads) {
+  int per_sm = 0, dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, 0) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    cudaGetLastError();
+    return 1;
+  }
+  return per_sm * sms / 2 > 0 ? per_sm * sms / 2 : 1;
+}
+MLB_API int mlb_ddp_bucket_max_ctas(int gmode, int lean) {
+  if (gmode == GM_BF16_PEER) return lean ? half_resident(ddp_bucket_lean_kernel<GM_BF16_PEER>, 128) : half_resident(ddp_bucket_kernel<GM_BF16_PEER>, 256);
+  if (gmode == GM_BF16_MC) return lean ? half_resident(ddp_bucket_lean_kernel<GM_BF16_MC>, 128) : half_resident(ddp_bucket_kernel<GM_BF16_MC>, 256);
+  return 0;
+}
+
 // One bucket of the fused data-parallel gradient step.  Pointer arrays live in device memory (world entries each).
 //   gmode        GM_* above.  The multicast modes need the matching multicast address; the bf16 modes need the staging
 //                pointer table (and `done_counter` 2 * max_buckets ints long), off and n multiples of 8.
-//   ctas         grid size (256 threads each); lean != 0 selects the 32-register form (see above)
+//   ctas         grid size (256 threads each; at most mlb_ddp_bucket_max_ctas); lean != 0 selects the 32-register form, of 128 threads
 MLB_API int mlb_ddp_bucket2(const void* grads_ptrs, const void* params_ptrs, const void* flags_ptrs, float* master, float* m, float* v,
                             int* done_counter, int* epoch_ctr, long off, long n, int rank, int world, int bucket, int max_buckets,
                             int bcast, float lr, float b1, float b2, float eps, float wd, float bc1, float bc2, float scale,
@@ -342,6 +363,8 @@ MLB_API int mlb_ddp_bucket2(const void* grads_ptrs, const void* params_ptrs, con
   long want = (chunk / 4 + 127) / 128;
   if (want < 1) want = 1;
   if (ctas < 1) ctas = 64;
+  const int most = mlb_ddp_bucket_max_ctas(gmode, lean);
+  if (most > 0 && ctas > most) ctas = most;
   const int grid = (int)(want < ctas ? want : ctas);
   // An SM's split between L1 and shared memory is fixed while CTAs are resident on it.  The tensor-core kernels need the
   // largest shared-memory split; a bucket CTA that got onto an idle SM first with the default (L1-heavy) split would keep

@@ -518,3 +518,34 @@ def test_linear_fwd_gather_world1_and_two_shards_on_one_gpu():
         err = (out.float() - exp).abs().max().item()
         assert err <= 2e-2 + 2e-2 * exp.abs().max().item(), (call, err)
     assert int(ctr[0]) == 2 and int(ctr[1]) == 0
+
+
+@pytest.mark.parametrize("lean", [0, 1])
+def test_bf16_bucket_grid_is_resident(lean):
+    """In the bf16 modes every CTA waits for the grid's last one: whatever grid is asked for, at most half of what the machine holds
+    is launched, and the launch ends without the wait running out.  One rank, against AdamW on the rounded gradients."""
+    from ml_b200.ops import native
+    L, n, dev = native.lib(), 1 << 22, torch.device("cuda:0")
+    sms = torch.cuda.get_device_properties(dev).multi_processor_count
+    most = L.mlb_ddp_bucket_max_ctas(2, lean)
+    assert sms <= most <= sms * (16 if lean else 4) // 2 and L.mlb_ddp_bucket_max_ctas(0, lean) == 0
+    torch.manual_seed(0)
+    g, master = torch.randn(n, device=dev), torch.randn(n, device=dev)
+    p, stage = master.bfloat16(), torch.empty(n, dtype=torch.bfloat16, device=dev)
+    m, v = torch.zeros(n, device=dev), torch.zeros(n, device=dev)
+    flags, done, epoch = (torch.zeros(k, dtype=torch.int32, device=dev) for k in (2 * L.mlb_comm_max_world(), 2, 1))
+    tab = torch.tensor([t.data_ptr() for t in (g, p, flags, stage)], dtype=torch.int64, device=dev)
+    at = lambda i: tab.data_ptr() + 8 * i
+    e = master.double()
+    fn = L.mlb_ddp_bucket2
+    fn.argtypes = [C.c_void_p] * 8 + [C.c_long, C.c_long] + [C.c_int] * 5 + [C.c_float] * 8 + [C.c_void_p, C.c_int, C.c_double] + \
+        [C.c_void_p] * 4 + [C.c_int, C.c_int, C.c_void_p]
+    rc = fn(at(0), at(1), at(2), master.data_ptr(), m.data_ptr(), v.data_ptr(), done.data_ptr(), epoch.data_ptr(), 0, n, 0, 1, 0, 1, 1,
+            1e-3, 0.9, 0.95, 1e-8, 0.1, 0.1, 0.05, 1.0, None, 1 << 20, 1.0, None, None, at(3), None, 2, lean,
+            torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert rc == 0 and native.get_error() == 0 and int(epoch) == 1
+    gb = g.bfloat16().double()
+    e -= 1e-3 * (gb / (gb.abs() + 1e-8) + 0.1 * e)
+    assert (master - e).abs().max() < 1e-5      # (fp32 arithmetic on values of order 1 and a step of 1e-3)
+    assert torch.equal(p, master.bfloat16())
