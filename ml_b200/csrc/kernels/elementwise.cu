@@ -1344,6 +1344,13 @@ MLB_API int mlb_layernorm_bwd(void* dx, float* dw, float* db, const void* dy, co
 
 // Number of blocks rmsnorm_bwd uses for `rows`; the caller provides scratch of (blocks + 16) * C floats and
 // 17 zeroed ints.
+// Number of the graph capture `st` takes part in, 0 if none
+MLB_API unsigned long long mlb_capture_id(cudaStream_t st) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamGetCaptureInfo(st, &cs, &id) != cudaSuccess) { cudaGetLastError(); return 0; }
+  return cs == cudaStreamCaptureStatusActive ? id : 0;
+}
 MLB_API int mlb_rmsnorm_bwd_blocks(long rows) {
   long b = (rows + 7) / 8;
   return (int)(b < 296 ? b : 296);

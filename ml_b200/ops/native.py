@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import threading
 from functools import lru_cache
 
 import torch
@@ -106,6 +107,8 @@ def lib():
     L.mlb_attn_bwd_have_delta.argtypes = L.mlb_attn_bwd.argtypes
     L.mlb_attn_bwd_have_delta.restype = _i32
     L.mlb_attn_bwd_scratch_bytes.restype = _i64
+    L.mlb_capture_id.argtypes = [_vp]
+    L.mlb_capture_id.restype = C.c_ulonglong
     for tag in ("gemm", "attn", "elementwise", "comm"):
         for pre in ("mlb_get_error_", "mlb_clear_error_"):
             if hasattr(L, pre + tag):
@@ -237,15 +240,28 @@ def _i(t, name="tensor"):
     return t.data_ptr()
 
 
-_scratch = {}
+_scratch = threading.local()
+
+
+def _capture_id(st):
+    """Number of the graph capture the stream takes part in, 0 outside one."""
+    return lib().mlb_capture_id(st) if torch._C._cuda_isCurrentStreamCapturing() else 0
 
 
 def scratch(key, numel, dtype, device, zero=False):
-    k = (key, str(device), dtype)
-    t = _scratch.get(k)
+    """Workspace kept from call to call: of the calling thread, on its current stream (another thread or stream may be in the middle
+    of the same sequence of kernels), and inside a graph capture of that capture (its replays run when and where they like;
+    zero-filled ones are zeroed by every replay).  Grows; what it grew out of goes back to the allocator."""
+    st = _st()
+    cap = _capture_id(st)
+    tensors = getattr(_scratch, "tensors", None)
+    if tensors is None or (cap and cap != _scratch.capture):      # (an earlier capture is over: its graph owns its memory)
+        _scratch.capture = cap
+        tensors = _scratch.tensors = {k: t for k, t in (tensors or {}).items() if k[4] == 0}
+    k = (key, device, dtype, st, cap)
+    t = tensors.get(k)
     if t is None or t.numel() < numel:
-        t = (torch.zeros if zero else torch.empty)(numel, dtype=dtype, device=device)
-        _scratch[k] = t
+        t = tensors[k] = (torch.zeros if zero else torch.empty)(numel, dtype=dtype, device=device)
     return t
 
 
@@ -381,12 +397,13 @@ def attn_bwd(dqkv, dout, qkv, out, lse, B, T, H, hd, rope=None, have_delta=False
     have_delta: linear_dx_delta has just written this call's delta term, the pass over dO and O is left out.
     Returns True if it did (tensor-core path), False if the caller still has to call rope_bwd."""
     delta = scratch("attn_delta", B * H * T, torch.float32, qkv.device)
-    acc = None
+    acc = part = None
     if hd == 64 and FUSED_ATTN_BWD:
         # per-(query tile, key tile) bf16 partials of dQ; past FUSED_ATTN_BWD_MAX_SCRATCH the two-kernel backward runs
         nbytes = lib().mlb_attn_bwd_scratch_bytes(B, T, H, hd)
         if 0 < nbytes <= FUSED_ATTN_BWD_MAX_SCRATCH:
-            acc = scratch(("attn_dq_part", nbytes), nbytes // 2, torch.bfloat16, qkv.device).data_ptr()
+            part = torch.empty(nbytes // 2, dtype=torch.bfloat16, device=qkv.device)      # (too large to be kept per stream)
+            acc = part.data_ptr()
     cp = _f(rope[0]) if rope is not None else None
     sp = _f(rope[1]) if rope is not None else None
     fn = lib().mlb_attn_bwd
@@ -508,10 +525,10 @@ def rmsnorm_bwd(dx, dw, dy, x, w, rstd, add=None):
     rows, Cc = x.shape
     L = lib()
     blocks = L.mlb_rmsnorm_bwd_blocks(rows)
-    part = scratch("rms_partial", (blocks + 16) * Cc, torch.float32, x.device)
-    ticket = scratch("rms_ticket", 32, torch.int32, x.device, zero=True)
+    # 32 words of tickets, zero between calls, then the partial sums
+    ws = scratch("rms_bwd", 32 + (blocks + 16) * Cc, torch.float32, x.device, zero=True).data_ptr()
     _chk(L.mlb_rmsnorm_bwd(_b(dx), _f(dw), _b(dy), _b(x), _b(w), _f(rstd), _b(add) if add is not None else None,
-                           rows, Cc, part.data_ptr(), ticket.data_ptr(), _st()), "rmsnorm_bwd")
+                           rows, Cc, ws + 128, ws, _st()), "rmsnorm_bwd")
 
 
 # ------------------------------------------------------------------ rope / swiglu / CE / AdamW

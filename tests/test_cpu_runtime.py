@@ -557,3 +557,27 @@ def test_event_profiler_regions_cover_a_step():
         assert expect <= set(agg), expect - set(agg)
         assert all(v >= 0 for v in agg.values()) and lines[-1].split()[0] == "total"
         assert abs(sum(agg.values()) - float(lines[-1].split()[1])) < 1e-2
+
+
+def test_scratch_belongs_to_one_thread_stream_and_capture(monkeypatch):
+    """Workspace handed from call to call is found again only by the same thread on the same stream, inside the same graph capture."""
+    import threading
+    from ml_b200.ops import native
+    at = {"stream": 1, "capture": 0}
+    monkeypatch.setattr(native, "_st", lambda: at["stream"])
+    monkeypatch.setattr(native, "_capture_id", lambda st: at["capture"], raising=False)
+
+    def get(stream=1, capture=0, n=8):
+        at.update(stream=stream, capture=capture)
+        return native.scratch("test_scratch", n, torch.float32, torch.device("cpu"), zero=True)
+    mine = get()
+    assert get() is mine and get(n=4) is mine and get(stream=2) is not mine
+    in_graph = get(capture=7)
+    assert in_graph is not mine and get(capture=7) is in_graph and get(capture=8) is not in_graph
+    assert get() is mine
+    other = []
+    t = threading.Thread(target=lambda: other.append(get()))
+    t.start()
+    t.join()
+    assert other[0] is not mine and get() is mine
+    assert get(n=9).numel() == 9

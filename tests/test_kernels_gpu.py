@@ -1016,3 +1016,65 @@ def test_attention_work_tables_are_bounded():
     graph.replay()
     assert torch.equal(held, first) and torch.equal(run(131)[0], first)
     assert torch.equal(run(132)[0], run(132)[0])
+
+
+@pytest.mark.parametrize("T,H,hd", [(384, 6, 64), (384, 4, 128), (200, 6, 32)])
+def test_backwards_on_two_streams_keep_apart(T, H, hd):
+    """Attention and norm backward on two streams at once, from two threads: bit for bit what each gives alone."""
+    import threading
+    n, B, C = nat(), 4, H * hd
+    torch.manual_seed(hd)
+    W = rnd(C, C, scale=C ** -0.5)
+
+    def work(seed, rounds, results):
+        g = torch.Generator(device=dev()).manual_seed(seed)
+        r = lambda *s: torch.randn(*s, generator=g, device=dev()).bfloat16()
+        qkv, dy, x, w = r(B * T, 3 * C), r(B * T, C), r(B * T, 256), r(256)
+        out, lse, rstd = torch.empty(B * T, C, device=dev(), dtype=torch.bfloat16), torch.empty(B, H, T, device=dev()), torch.rand(B * T, device=dev(), generator=g)
+        n.attn_fwd(out, lse, qkv, B, T, H, hd)
+        for _ in range(rounds):
+            dqkv, dx, dw, d = torch.zeros_like(qkv), torch.empty_like(x), torch.zeros(256, device=dev()), torch.empty_like(out)
+            have = hd == 64 and n.linear_dx_delta(d, dy, W, out, B, T, H)
+            n.attn_bwd(dqkv, d if have else dy, qkv, out, lse, B, T, H, hd, have_delta=bool(have))
+            n.rmsnorm_bwd(dx, dw, x, x, w, rstd)
+            results.append((dqkv, dx, dw))
+    alone = [[], []]
+    for i in (0, 1):
+        work(i, 1, alone[i])
+    torch.cuda.synchronize()
+    got = [[], []]
+
+    def on_stream(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            work(i, 20, got[i])
+            torch.cuda.current_stream().synchronize()
+    threads = [threading.Thread(target=on_stream, args=(i,)) for i in (0, 1)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for i in (0, 1):
+        assert len(got[i]) == 20
+        for r in got[i]:
+            assert all(torch.equal(a, b) for a, b in zip(r, alone[i][0]))
+
+
+def test_norm_backward_in_graphs_whose_first_one_never_ran():
+    """The ticket of the one-launch norm backward is part of its graph: zero at every replay, whatever other graphs have done."""
+    n, rows, C = nat(), 300, 768
+    x, dy, w, rstd = rnd(rows, C), rnd(rows, C), rnd(C), torch.rand(rows, device=dev())
+    e, dx = torch.zeros(C, device=dev()), torch.empty_like(x)
+    n.rmsnorm_bwd(dx, e, dy, x, w, rstd)
+    graphs, dws = [], []
+    for _ in range(2):
+        dw = torch.zeros(C, device=dev())
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            n.rmsnorm_bwd(dx, dw, dy, x, w, rstd)
+        graphs.append(g)
+        dws.append(dw)
+    graphs[1].replay()
+    n.rmsnorm_bwd(dx, dws[0], dy, x, w, rstd)
+    assert torch.equal(dws[1], e) and torch.equal(dws[0], e)
+    graphs[1].replay()
+    assert torch.equal(dws[1], e + e)
