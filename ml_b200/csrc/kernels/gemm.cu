@@ -68,6 +68,7 @@ struct GemmArgs {
   int sk_group, sk_group_m;   // stream-K group size (tiles along the short dimension) and whether that dimension is M
   int nt_fast;       // pair kernel: consecutive work items walk N first (tiles in flight share rows of A) instead of M
   int sk_dp;         // stream-K: this many tiles go out whole first, one per cluster and wave; only the rest is cut up
+  int sk_q;          // ... so many tiles of the rest at a time shared by one cluster more than they are (0: all by all clusters)
   // optional rotary embedding in the bf16 epilogue (pair kernel): output columns [0, rope_cols) are heads of 64 columns
   // whose halves (i, i + 32) are rotated by the angle table row (output row % rope_T)
   const float* cosT;
@@ -124,12 +125,17 @@ struct WorkIter {
     const int ngroups = ncl / G, grp = cid / G;
     member = cid % G;
     const int long_tiles = G == 1 ? tiles_m * tiles_n - dp : (grouped_m ? g.tiles_n : g.tiles_m);   // G == 1: every tile on its own
-    const long units = (long)long_tiles * g.kb_total;
-    if (sk && grp < ngroups) {
+    u = u1 = 0;
+    if (sk && g.sk_q > 0) {
+      const int first = cid / (g.sk_q + 1) * g.sk_q, part = cid % (g.sk_q + 1), n = min(g.sk_q, long_tiles - first);
+      if (n > 0 && part <= n) {
+        u = (long)first * g.kb_total + (long)n * g.kb_total * part / (n + 1);
+        u1 = (long)first * g.kb_total + (long)n * g.kb_total * (part + 1) / (n + 1);
+      }
+    } else if (sk && grp < ngroups) {
+      const long units = (long)long_tiles * g.kb_total;
       u = units * grp / ngroups;
       u1 = units * (grp + 1) / ngroups;
-    } else {
-      u = u1 = 0;
     }
     total = sk ? dp : total * g.splits;      // (whole tiles first)
   }
@@ -954,7 +960,7 @@ int g_streamk = 1;           // tuning hook: weight-gradient products cut into e
 int g_epi_mode = 1;          // tuning hook: pair kernel's epilogue, 0 = TMA store / reduce, 1 = coalesced stores by the warps
 int g_small_tiles = 1;       // tuning hook: 0 = never trade the CTA-pair tile for 128 x 128 tiles on small problems
 template <bool A_MN, bool B_MN, int EPI, int EMODE, bool POS = false, bool DELTA = false>
-int launch_tc2(const CUtensorMap* tmA, const CUtensorMap* tmB, const CUtensorMap* tmD, const GemmArgs& g, cudaStream_t st) {
+int launch_tc2(const CUtensorMap* tmA, const CUtensorMap* tmB, const CUtensorMap* tmD, GemmArgs g, cudaStream_t st) {
   using Gemm2Smem = Gemm2Smem<EMODE>;
   auto kern = gemm_tc2_kernel<A_MN, B_MN, EPI, EMODE, false, POS, DELTA>;
   static int max_clusters = -1;
@@ -974,6 +980,23 @@ int launch_tc2(const CUtensorMap* tmA, const CUtensorMap* tmB, const CUtensorMap
   int cap = max_clusters;
   if (g_max_ctas > 0 && g_max_ctas / 2 < cap) cap = g_max_ctas / 2 > 0 ? g_max_ctas / 2 : 1;
   int clusters = total < cap ? total : cap;
+  if (g.streamk) {
+    // Whole waves of tiles first, only the tiles of the last, partial wave cut up: with every tile cut, the clusters sit at 74 different
+    // depths of the reduction and no two of them want the same slice of the operands at the same time (dW of 11008 x 2048 over
+    // 16384 rows: 554 us cut up throughout, 459 us this way; 2048 x 5504: 366 and 284 us).  Short reductions (less than 32
+    // k-blocks) have no time to drift apart, and their tail pieces would be mostly epilogue.  A wave is what is launched here.
+    // Two clusters at most add to a tile: q tiles are shared by q + 1 clusters, each of which takes q / (q + 1) of one.  A sum of two
+    // pieces and what was there before (zero, in a weight gradient of its own) does not depend on which comes first; shared evenly by all
+    // clusters a tile has three pieces and more, and the low bits changed from run to run.  Over 16384 rows: 11008 x 2048 451 us (459
+    // shared evenly), 2048 x 5504 227 (223), 6144 x 2048 246 (278), 4096 x 2048 169 (169); 2304 x 2304, 7 tiles left over, 135 (109).
+    const int tiles = g.tiles_m * g.tiles_n, rest = tiles % clusters;
+    if (g_sk_whole && g.sk_group == 1 && tiles >= clusters && g.kb_total >= 32) {
+      g.sk_dp = tiles - rest;
+      g.sk_q = rest > 0 ? ceil_div_i(rest, clusters - rest) : 1;
+    } else {
+      g.nt_fast = 0;
+    }
+  }
   return (int)mlb_launch_tmem(kern, dim3(2 * clusters), dim3(GEMM2_THREADS), Gemm2Smem::TOTAL, st, *tmA, *tmB, *tmD, g);
 }
 int pair_clusters() { return (g_max_ctas > 0 ? g_max_ctas : num_sms()) / 2; }
@@ -1085,21 +1108,12 @@ int gemm_dispatch_impl(void* out, int ldo, const bf16* A, int lda, const bf16* B
   g.streamk = (pairs && EPI == EPI_F32_ADD && g_streamk && g_force_splits == 0) ? 1 : 0;
   // Tiles in flight should share the operand that does not fit in L2: walk N first when A is the larger one.
   g.nt_fast = (g_tile_order == 2 || (g_tile_order != 1 && M > N)) ? 1 : 0;
-  g.sk_dp = 0;
+  g.sk_dp = g.sk_q = 0;
   g.sk_group = 1; g.sk_group_m = 0;
   if (g.streamk) {
     // group along the dimension with fewer tiles (its operand is the narrow one); at most 4 members, else plain stream-K
     const int short_tiles = g.tiles_m < g.tiles_n ? g.tiles_m : g.tiles_n;
     if (g_sk_groups && short_tiles <= 4 && short_tiles >= 1 && pair_clusters() >= 4 * short_tiles) { g.sk_group = short_tiles; g.sk_group_m = g.tiles_m < g.tiles_n ? 1 : 0; }
-  }
-  if (g.streamk) {
-    // Whole waves of tiles first, only the tiles of the last, partial wave cut up: with every tile cut, the clusters sit at 74 different
-    // depths of the reduction and no two of them want the same slice of the operands at the same time (dW of 11008 x 2048 over
-    // 16384 rows: 554 us cut up throughout, 459 us this way; 2048 x 5504: 366 and 284 us).  Short reductions (less than 32
-    // k-blocks) have no time to drift apart, and their tail pieces would be mostly epilogue.
-    const int tiles = g.tiles_m * g.tiles_n, pc = pair_clusters();
-    if (g_sk_whole && g.sk_group == 1 && tiles >= pc && g.kb_total >= 32) g.sk_dp = tiles / pc * pc;
-    else g.nt_fast = 0;
   }
   const CUtensorMap* tmA = nullptr;
   const CUtensorMap* tmB = nullptr;
@@ -1221,7 +1235,7 @@ int gemm_fp8_dispatch(void* out, int ldo, const uint8_t* A, int lda, const uint8
   g.kb_total = ceil_div_i(K, 128);
   g.splits = 1; g.kb_per_split = g.kb_total; g.a3d = g.b3d = 0; g.streamk = 0; g.sk_group = 1; g.sk_group_m = 0;
   g.nt_fast = (g_tile_order == 2 || (g_tile_order != 1 && M > N)) ? 1 : 0;
-  g.sk_dp = 0;
+  g.sk_dp = g.sk_q = 0;
   const CUtensorMap* tmA = mlb_tmap_cached(A, M, K, lda, 128, 128, 1);
   const CUtensorMap* tmB = mlb_tmap_cached(B, N, K, ldb, 128, 128, 1);
   const CUtensorMap* tmD = mlb_tmap_cached(out, M, N, ldo, 32, 64, 2);
@@ -1352,7 +1366,7 @@ MLB_API int mlb_linear_fwd_gather(void* out, const void* x, int M, int N, int K,
   GemmArgs g;
   g.out = out; g.M = M; g.N = N; g.K = K; g.ldo = ldo;
   g.tiles_m = ceil_div_i(M, BM); g.tiles_n = ceil_div_i(N, BN); g.kb_total = ceil_div_i(K, BK);
-  g.nt_fast = 0; g.sk_dp = 0;
+  g.nt_fast = 0; g.sk_dp = g.sk_q = 0;
   g.splits = 1; g.kb_per_split = g.kb_total; g.a3d = g.b3d = 0; g.streamk = 0; g.sk_group = 1; g.sk_group_m = 0;
   g.cosT = g.sinT = nullptr; g.rope_T = 1; g.rope_cols = 0; g.sw_out = nullptr; g.sw_I = 0; g.out_scale = 1.f; g.pos = nullptr; g.pos_period = 1; g.dl_o = nullptr; g.dl_out = nullptr; g.dl_T = 1; g.dl_H = 1;
   GatherArgs ga;

@@ -1078,3 +1078,31 @@ def test_norm_backward_in_graphs_whose_first_one_never_ran():
     assert torch.equal(dws[1], e) and torch.equal(dws[0], e)
     graphs[1].replay()
     assert torch.equal(dws[1], e + e)
+
+
+@pytest.mark.parametrize("order", [0, 1, 2])
+@pytest.mark.parametrize("M,N,K", [(2048, 2304, 2304), (2100, 2312, 2200), (2048, 1536, 9472), (2048, 2560, 5504), (4160, 2048, 2432)])
+def test_linear_dw_whole_waves_then_shared_tiles(M, N, K, order):
+    """Weight gradients of 76 to 222 tiles on 74 clusters: whole waves, then q tiles shared by q + 1 clusters (q = 1, 2), none
+    left over (222), ragged rows, columns and reductions, both tile orders, and every tile cut up (the hook off).  Added to what
+    is there, in fp32: products of bf16 are exact, sums of <= 4160 terms in any order are off by less than 4160 * 2^-24 of their
+    terms' norm (1e-5 of the result here).  From zero, two runs agree bit for bit."""
+    torch.manual_seed(N + K)
+    n = nat()
+    x, d = rnd(M, K), rnd(M, N)
+    e = d.double().T @ x.double() + 1
+    L = n.lib()
+    try:
+        L.mlb_gemm_tile_order(order)
+        for whole in (1, 0):
+            L.mlb_gemm_streamk_whole(whole)
+            dW = torch.ones(N, K, device=dev())
+            n.linear_dw(dW, d, x)
+            assert _rel(dW, e) < 1e-5
+            runs = [torch.zeros(N, K, device=dev()) for _ in range(3)]
+            for r in runs:
+                n.linear_dw(r, d, x)
+            assert torch.equal(runs[0], runs[1]) and torch.equal(runs[0], runs[2])
+    finally:
+        L.mlb_gemm_tile_order(0)
+        L.mlb_gemm_streamk_whole(1)
