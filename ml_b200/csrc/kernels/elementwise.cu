@@ -1427,15 +1427,17 @@ MLB_API int mlb_rope(void* qkv, const float* cosT, const float* sinT, long rows,
   }
   LAUNCH_RET;
 }
-// -7: the shape or alignment does not take these kernels (nothing was launched)
+// -7: the shape or alignment does not take these kernels (nothing was launched); -1: the key / value heads do not divide the query heads
 MLB_API int mlb_rope_copy(void* dst, const void* src, const float* cosT, const float* sinT, long rows, int T, int H, int Hkv, int hd,
                           cudaStream_t st) {
+  if (H <= 0 || Hkv <= 0 || H % Hkv != 0 || T <= 0) return -1;
   const long n = rows * 3L * H * (hd / 16);
   if (hd % 16 != 0 || n <= 0 || n >= (1L << 31) || (((uintptr_t)dst | (uintptr_t)src | (uintptr_t)cosT | (uintptr_t)sinT) & 15)) return -7;
   mlb_launch(rope_copy_k, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, (bf16*)dst, (const bf16*)src, cosT, sinT, (unsigned)n, T, H, Hkv, hd);
   LAUNCH_RET;
 }
 MLB_API int mlb_kv_group_sum(void* dst, const void* src, long rows, int H, int Hkv, int hd, cudaStream_t st) {
+  if (H <= 0 || Hkv <= 0 || H % Hkv != 0) return -1;
   const long n = rows * (H + 2L * Hkv) * (hd / 8);
   if (hd % 8 != 0 || n <= 0 || n >= (1L << 31) || (((uintptr_t)dst | (uintptr_t)src) & 15)) return -7;
   mlb_launch(kv_group_sum_k, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, (bf16*)dst, (const bf16*)src, (unsigned)n, H, Hkv, hd);

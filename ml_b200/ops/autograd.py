@@ -83,13 +83,17 @@ class SwiGLU(torch.autograd.Function):
 
 class RopeCausalAttention(torch.autograd.Function):
     """qkv[B*T, (H + 2 Hkv) hd] -> out[B*T, H hd]: rotate-half RoPE on Q and K, then causal attention (scale 1/sqrt(hd)); every key /
-    value head serves H / Hkv consecutive query heads (Hkv None: one each)."""
+    value head serves H / Hkv consecutive query heads (Hkv None: one each).  Rows behind the B*T are left alone."""
 
     @staticmethod
     def forward(ctx, qkv, cos, sin, B, T, H, hd, Hkv=None):
+        heads = H if Hkv is None else Hkv
+        width = (H + 2 * heads) * hd
+        if heads < 1 or H % heads or qkv.numel() < B * T * width or qkv.numel() % width:
+            raise ValueError(f"qkv {tuple(qkv.shape)} does not hold {B * T} rows of {H} query and 2 x {heads} key / value heads of {hd}")
         qkv = qkv.contiguous()
         q = _like(qkv, B * T, 3 * H * hd)
-        ops.rope_copy(q, qkv, cos, sin, B, T, H, hd, Hkv)
+        ops.rope_copy(q, qkv.view(-1, width)[:B * T], cos, sin, B, T, H, hd, Hkv)
         out = _like(qkv, B * T, H * hd)
         lse = _like(qkv, B, H, T, dtype=torch.float32)
         ops.attn_fwd(out, lse, q, B, T, H, hd)
@@ -109,6 +113,9 @@ class RopeCausalAttention(torch.autograd.Function):
         if ctx.Hkv not in (None, H):
             full, dqkv = dqkv, _like(q, B * T, (H + 2 * ctx.Hkv) * hd)
             ops.kv_group_sum(dqkv, full, B, T, H, hd, ctx.Hkv)
+        if ctx.shape.numel() != dqkv.numel():
+            used, dqkv = dqkv, dqkv.new_zeros(ctx.shape)
+            dqkv.view(-1, used.shape[1])[:B * T] = used
         return dqkv.view(ctx.shape), None, None, None, None, None, None, None
 
 

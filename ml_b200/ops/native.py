@@ -536,7 +536,14 @@ def rope_fwd(qkv, cos, sin, B, T, H, hd):
     _chk(lib().mlb_rope(_b(qkv), _f(cos), _f(sin), B * T, T, H, hd, 1.0, _st()), "rope_fwd")
 
 
+def _heads(name, full, grouped, B, T, H, hd, Hkv):
+    """Both tensors hold what the kernels will read and write of them."""
+    if Hkv < 1 or H % Hkv or full.numel() != B * T * 3 * H * hd or grouped.numel() != B * T * (H + 2 * Hkv) * hd:
+        raise ValueError(f"{name}: {tuple(full.shape)} and {tuple(grouped.shape)} are not {B * T} rows of {H} + 2 x {Hkv} heads of {hd}")
+
+
 def rope_copy(out, qkv, cos, sin, B, T, H, hd, Hkv=None):
+    _heads("rope_copy", out, qkv, B, T, H, hd, H if Hkv is None else Hkv)
     rc = lib().mlb_rope_copy(_b(out), _b(qkv), _f(cos), _f(sin), B * T, T, H, H if Hkv is None else Hkv, hd, _st())
     if rc == -7:      # a head size or alignment that kernel does not take: heads laid out first, then rotated in place
         N, rep = B * T, 1 if Hkv is None else H // Hkv
@@ -548,6 +555,7 @@ def rope_copy(out, qkv, cos, sin, B, T, H, hd, Hkv=None):
 
 
 def kv_group_sum(out, dqkv, B, T, H, hd, Hkv):
+    _heads("kv_group_sum", dqkv, out, B, T, H, hd, Hkv)
     rc = lib().mlb_kv_group_sum(_b(out), _b(dqkv), B * T, H, Hkv, hd, _st())
     if rc == -7:
         o, x = out.view(B * T, -1, hd), dqkv.view(B * T, 3 * H, hd)

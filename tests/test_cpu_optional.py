@@ -527,3 +527,23 @@ def test_data_parallel_replicas_of_model_parallel_groups(tmp_path):
     assert "replicas=2" in out1 and "replicas=2" in out2
     for a, b in zip(pp2dp2, one_stage):
         assert abs(a - b) < 2e-4, (pp2dp2, one_stage)
+
+
+def test_rope_causal_attention_refuses_heads_that_do_not_fit():
+    """Key / value heads that do not divide the query heads, and inputs that are not B*T rows of the heads named, are refused in
+    front of any kernel; rows behind the B*T stay out of it and get no gradient."""
+    from ml_b200.ops import autograd as F
+    from ml_b200 import ops
+    B, T, H, hd = 2, 5, 4, 8
+    cos, sin = ops.rope_tables(T, hd, 10000.0, torch.device("cpu"))
+    x = torch.randn(B * T, (H + 2 * 2) * hd)
+    for Hkv in (3, 8, 0, -2, 4, None):      # (4 and None: as many columns as they need are not there)
+        with pytest.raises(ValueError):
+            F.rope_causal_attention(x, cos, sin, B, T, H, hd, Hkv)
+    with pytest.raises(ValueError):
+        F.rope_causal_attention(x[:-1], cos, sin, B, T, H, hd, 2)
+    more = torch.cat([x, torch.randn(3, x.shape[1])]).requires_grad_(True)
+    out = F.rope_causal_attention(more, cos, sin, B, T, H, hd, 2)
+    assert torch.equal(out, F.rope_causal_attention(x, cos, sin, B, T, H, hd, 2))
+    out.sum().backward()
+    assert more.grad[:B * T].abs().sum() > 0 and not more.grad[B * T:].any()

@@ -1106,3 +1106,28 @@ def test_linear_dw_whole_waves_then_shared_tiles(M, N, K, order):
     finally:
         L.mlb_gemm_tile_order(0)
         L.mlb_gemm_streamk_whole(1)
+
+
+@pytest.mark.parametrize("B,T,H,Hkv,hd", [(2, 130, 4, 2, 64), (1, 257, 8, 2, 128), (2, 65, 6, 1, 32), (1, 40, 4, 2, 24)])
+def test_grouped_heads_through_autograd(B, T, H, Hkv, hd):
+    """Rotary embedding, repeated heads, attention and back, against 64 bits.  bf16: the rotated Q and K, P, dS and the result are rounded
+    once each (2^-9 at most, and the rotated ones enter squared scores): below 2^-6."""
+    from ml_b200.ops import autograd as F
+    torch.manual_seed(T)
+    cos, sin = ref.rope_tables(T, hd, 10000.0, dev())
+    x = rnd(B * T, (H + 2 * Hkv) * hd).requires_grad_(True)
+    dout = rnd(B * T, H * hd)
+    out = F.rope_causal_attention(x, cos, sin, B, T, H, hd, Hkv)
+    (g,) = torch.autograd.grad(out, x, dout)
+    xd = x.detach().double().requires_grad_(True)
+    q, k, v = xd.view(B, T, H + 2 * Hkv, hd).transpose(1, 2).split([H, Hkv, Hkv], 1)
+    c, s = cos.double(), sin.double()
+    rot = lambda t: torch.cat([t[..., :hd // 2] * c - t[..., hd // 2:] * s, t[..., hd // 2:] * c + t[..., :hd // 2] * s], -1)
+    k, v = (t.repeat_interleave(H // Hkv, 1) for t in (rot(k), v))
+    a = rot(q) @ k.transpose(-1, -2) / hd ** 0.5
+    a = torch.softmax(a.masked_fill(torch.ones(T, T, dtype=torch.bool, device=dev()).triu(1), float("-inf")), -1)
+    e = (a @ v).transpose(1, 2).reshape(B * T, H * hd)
+    (eg,) = torch.autograd.grad(e, xd, dout.double())
+    assert _rel(out, e) < 2 ** -6 and _rel(g, eg) < 2 ** -6
+    with pytest.raises(ValueError):
+        nat().rope_copy(torch.empty(B * T, 3 * H * hd, device=dev(), dtype=torch.bfloat16), x.detach(), cos, sin, B, T, H, hd, H + 1)
