@@ -42,10 +42,13 @@ struct ItemList {
 // Forward over pairs of query tiles (256 queries) of one (sample, head).  TMEM: S0 S1 O0 O1.  Per tile and key block
 //   S = Q K^T -> one thread per row: m, p = exp2(s c - m) -> P over S -> O += P V -> next S
 // is a chain; the two tiles run it out of phase, one on the tensor core while the other takes exponentials: they take turns.  Left
-// alone they fall into step, and a step of both tiles takes 5400 cycles instead of 3700 (8 x 2048 tokens, 16 heads: 192 -> 161 us, 853
-// TFLOP/s over the causal half).  P V starts when the first half of P is there.  160 registers leave a sub-partition with three of
-// these warps room for one 32-register warp of a communication kernel.  m is the maximum of an earlier block as long as no row of the warp has grown past it
-// by more than 2^8; only then O (in place) and l are rescaled.
+// alone they fall into step, and a step of both tiles takes 5400 cycles instead of 3700 (8 x 2048 tokens, 16 heads: 192 -> 161 us with the
+// older maximum of the next lines).  P V starts when the first half of P is there.  160 registers leave a sub-partition with three of
+// these warps room for one 32-register warp of a communication kernel.
+// m is the maximum of all blocks so far, so that a row's largest probability is 1 and costs no rounding; O (in place) and l are rescaled
+// whenever a row of the warp has a new one.  Kept from an earlier block until outgrown by 2^8 it takes 159 us instead of 180 (764 TFLOP/s
+// over the causal half), but the largest probability is rounded like the others: 2.07e-3 off the 64-bit result instead of 2.04e-3 over
+// 2048 tokens, and with scores of twice that spread 2.11e-3 instead of 1.86e-3.
 __global__ void __maxnreg__(160) attn_fwd128_k(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUtensorMap tm_out,
                                                                    const AttnArgs a) {
   mlb_pdl_sync();
@@ -215,9 +218,9 @@ __global__ void __maxnreg__(160) attn_fwd128_k(const __grid_constant__ CUtensorM
           for (int c = 0; c < 4; c++) m4[c] = max3(m4[c], __uint_as_float(r[c][i]), __uint_as_float(r[c][i + 1]));
         const float z = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * sl2;
         if (j == 0) {
-          m = z == -INFINITY ? 0.f : z;
-        } else if (__any_sync(0xffffffffu, z > m + 8.f)) {
-          const float mn = fmaxf(m, z), alpha = ex2_approx(m - mn);
+          m = z;
+        } else if (__any_sync(0xffffffffu, z > m)) {
+          const float mn = fmaxf(m, z), alpha = m == mn ? 1.f : ex2_approx(m - mn);
           m = mn;
           l *= alpha;
           wait(&bar_o[t], (gt - 1) & 1, 59);
@@ -240,7 +243,8 @@ __global__ void __maxnreg__(160) attn_fwd128_k(const __grid_constant__ CUtensorM
         const int turn = other + min(j + t, n_other);      // blocks the other tile's warp is to have taken before
         for (int spin = 0; s_turn[(t ^ 1) * 4 + lg] < turn && spin < (1 << 16) && !*s_abort; spin++) { }
         __syncwarp();
-        const uint64_t nm2 = pk2(-m, -m);
+        const float mu = m == -INFINITY ? 0.f : m;      // (nothing finite seen yet: exp2(-inf - 0) = 0)
+        const uint64_t nm2 = pk2(-mu, -mu);
         uint64_t rs2 = pk2(0.f, 0.f), rs3 = rs2;
 #pragma unroll
         for (int c = 0; c < 4; c++) {
