@@ -1960,11 +1960,11 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_q_tc_kernel(const __g
 // One block per (query row, head, sample); scores kept in shared memory.
 // `last` = index of the last key a query sees: the query's own position (causal) or T - 1 (bidirectional, the vision
 // encoder's attention).
-__global__ void attn_fwd_simt_k(bf16* __restrict__ out, float* __restrict__ lse, const bf16* __restrict__ qkv, int B, int T, int H,
-                                int hd, float scale, int causal = 1) {
-  extern __shared__ float sc[];  // T scores + 32 reduce
+// (all threads of the block; sc: T scores + 32 for the reductions)
+__device__ __forceinline__ void attn_fwd_simt_row(bf16* __restrict__ out, float* __restrict__ lse, const bf16* __restrict__ qkv, int i, int h, int b,
+                                                  int T, int H, int hd, float scale, int causal, float* sc) {
   float* red = sc + T;
-  const int i = blockIdx.x, h = blockIdx.y, b = blockIdx.z, C = H * hd;
+  const int C = H * hd;
   const int last = causal ? i : T - 1;
   const bf16* q = qkv + ((size_t)(b * T + i)) * 3 * C + h * hd;
   float mx = -INFINITY;
@@ -1988,12 +1988,16 @@ __global__ void attn_fwd_simt_k(bf16* __restrict__ out, float* __restrict__ lse,
   }
   if (threadIdx.x == 0) lse[((size_t)b * H + h) * T + i] = mx + __logf(sum);
 }
-// dQ for query i.
-__global__ void attn_bwd_q_simt_k(bf16* __restrict__ dqkv, const bf16* __restrict__ dout, const bf16* __restrict__ qkv,
-                                  const float* __restrict__ lse, const float* __restrict__ delta, int B, int T, int H, int hd,
-                                  float scale, int causal = 1) {
-  extern __shared__ float sc[];
-  const int i = blockIdx.x, h = blockIdx.y, b = blockIdx.z, C = H * hd;
+__global__ void attn_fwd_simt_k(bf16* __restrict__ out, float* __restrict__ lse, const bf16* __restrict__ qkv, int B, int T, int H,
+                                int hd, float scale, int causal = 1) {
+  extern __shared__ float simt_sc[];
+  attn_fwd_simt_row(out, lse, qkv, blockIdx.x, blockIdx.y, blockIdx.z, T, H, hd, scale, causal, simt_sc);
+}
+// dQ for query i (sc: T).
+__device__ __forceinline__ void attn_bwd_q_simt_row(bf16* __restrict__ dqkv, const bf16* __restrict__ dout, const bf16* __restrict__ qkv,
+                                                    const float* __restrict__ lse, const float* __restrict__ delta, int i, int h, int b, int T, int H,
+                                                    int hd, float scale, int causal, float* sc) {
+  const int C = H * hd;
   const int last = causal ? i : T - 1;
   const bf16* q = qkv + ((size_t)(b * T + i)) * 3 * C + h * hd;
   const bf16* dO = dout + ((size_t)(b * T + i)) * C + h * hd;
@@ -2015,14 +2019,19 @@ __global__ void attn_bwd_q_simt_k(bf16* __restrict__ dqkv, const bf16* __restric
     dqkv[((size_t)(b * T + i)) * 3 * C + h * hd + d] = __float2bfloat16(acc);
   }
 }
-// dK, dV for key j.
-__global__ void attn_bwd_kv_simt_k(bf16* __restrict__ dqkv, const bf16* __restrict__ dout, const bf16* __restrict__ qkv,
-                                   const float* __restrict__ lse, const float* __restrict__ delta, int B, int T, int H, int hd,
-                                   float scale, int causal = 1) {
-  extern __shared__ float sc[];  // p[T], ds[T]
+__global__ void attn_bwd_q_simt_k(bf16* __restrict__ dqkv, const bf16* __restrict__ dout, const bf16* __restrict__ qkv,
+                                  const float* __restrict__ lse, const float* __restrict__ delta, int B, int T, int H, int hd,
+                                  float scale, int causal = 1) {
+  extern __shared__ float simt_sc[];
+  attn_bwd_q_simt_row(dqkv, dout, qkv, lse, delta, blockIdx.x, blockIdx.y, blockIdx.z, T, H, hd, scale, causal, simt_sc);
+}
+// dK, dV for key j (sc: p[T], ds[T]).
+__device__ __forceinline__ void attn_bwd_kv_simt_row(bf16* __restrict__ dqkv, const bf16* __restrict__ dout, const bf16* __restrict__ qkv,
+                                                     const float* __restrict__ lse, const float* __restrict__ delta, int j, int h, int b, int T, int H,
+                                                     int hd, float scale, int causal, float* sc) {
   float* sp = sc;
   float* sds = sc + T;
-  const int j = blockIdx.x, h = blockIdx.y, b = blockIdx.z, C = H * hd;
+  const int C = H * hd;
   const int first = causal ? j : 0;      // first query that sees key j
   const bf16* k = qkv + ((size_t)(b * T + j)) * 3 * C + C + h * hd;
   const bf16* v = k + C;
@@ -2049,6 +2058,12 @@ __global__ void attn_bwd_kv_simt_k(bf16* __restrict__ dqkv, const bf16* __restri
     dqkv[((size_t)(b * T + j)) * 3 * C + C + h * hd + d] = __float2bfloat16(dk);
     dqkv[((size_t)(b * T + j)) * 3 * C + 2 * C + h * hd + d] = __float2bfloat16(dv);
   }
+}
+__global__ void attn_bwd_kv_simt_k(bf16* __restrict__ dqkv, const bf16* __restrict__ dout, const bf16* __restrict__ qkv,
+                                   const float* __restrict__ lse, const float* __restrict__ delta, int B, int T, int H, int hd,
+                                   float scale, int causal = 1) {
+  extern __shared__ float simt_sc[];
+  attn_bwd_kv_simt_row(dqkv, dout, qkv, lse, delta, blockIdx.x, blockIdx.y, blockIdx.z, T, H, hd, scale, causal, simt_sc);
 }
 
 int g_attn_force_simt = 0;

@@ -15,13 +15,17 @@
 // The next block's scores overwrite those columns.  MMAs are promised to run in the order of their issue only where accumulator and
 // shape are the same, so the products that read the columns are waited for first.
 // Sequences are the third dimension of the tensor maps: rows past a sample's end arrive as zeros, never as the next
-// sample's values (0 * inf would be NaN).
+// sample's values (0 * inf would be NaN).  Within a sample the products do multiply a masked key's zero with its V (or Q, K, dO), and the
+// two terms of an infinite product may cancel.  With finite values neither matters, and otherwise the row is NaN: such rows are done
+// again, at the end, by the scalar kernels' row functions, which skip masked keys.
 struct SplitArgs {
   int B, T, H, hd, causal;
   float scale;
   bf16* out;            // forward: out[B*T, C]; backward: dqkv[B*T, 3C]
   float* lse;           // [B,H,T]
   const float* delta;   // [B,H,T]
+  const bf16* qkv;
+  const bf16* dout;
 };
 
 constexpr int SPLIT_THREADS = 128;
@@ -65,14 +69,47 @@ __device__ __forceinline__ void split_load(uint8_t* dst, const CUtensorMap* tm, 
     for (int i = 0; i < boxes; i++) tc::tma_load_3d(dst + (c * boxes + i) * BOX_BYTES, tm, bar, x0 + c * 64, r0 + i * 64, z);
 }
 
+// Rows r0 + bit of the CTA's NaN rows (one word per warp), one after the other by the whole CTA; the tiles' shared memory is free.
+// Out of line: its registers must not be the kernels'.
+template <int FORM>      // 0 forward, 1 dK and dV, 2 dQ
+__device__ __noinline__ void split_redo(uint4 nan_rows, SplitArgs a, int r0, int h, int b, float* sc) {
+  for (int i = 0; i < 128; i++) {
+    const unsigned word = i < 32 ? nan_rows.x : i < 64 ? nan_rows.y : i < 96 ? nan_rows.z : nan_rows.w;
+    if (!(word >> (i & 31) & 1)) continue;
+    if (FORM == 0) attn_fwd_simt_row(a.out, a.lse, a.qkv, r0 + i, h, b, a.T, a.H, a.hd, a.scale, a.causal, sc);
+    else if (FORM == 1) attn_bwd_kv_simt_row(a.out, a.dout, a.qkv, a.lse, a.delta, r0 + i, h, b, a.T, a.H, a.hd, a.scale, a.causal, sc);
+    else attn_bwd_q_simt_row(a.out, a.dout, a.qkv, a.lse, a.delta, r0 + i, h, b, a.T, a.H, a.hd, a.scale, a.causal, sc);
+    __syncthreads();
+  }
+}
+// acc is NaN from the first value on that is NaN or infinite (times zero), two values an instruction: comparing each one is a chain of
+// predicates, 4 us of the dK / dV kernel's 43 (32 x 197 tokens, 12 heads of 64)
+__device__ __forceinline__ uint64_t note_nan(uint64_t acc, float x, float y) { return fma2(pk2(x, y), pk2(0.f, 0.f), acc); }
+__device__ __forceinline__ bool noted_nan(uint64_t a, uint64_t b) {
+  float x, y;
+  upk2(add2(a, b), x, y);
+  x += y;
+  return x != x;
+}
+
 // hd columns of the warp's 32 TMEM rows, times f, as bf16 to memory (16-byte aligned, hd a multiple of 16): dst = the lane's row,
-// rows `pitch` apart, nlive of them exist.  Whole warp.
+// rows `pitch` apart, nlive of them exist.  Whole warp.  Is the lane's row (it may not exist) NaN or infinite somewhere?
 template <int HDT>
-__device__ __forceinline__ void split_store_rows(bf16* dst, long pitch, uint32_t taddr, int hd, float f, int lane, int nlive) {
+__device__ __forceinline__ bool split_store_rows(bf16* dst, long pitch, uint32_t taddr, int hd, float f, int lane, int nlive) {
+  uint64_t n0 = pk2(0.f, 0.f), n1 = n0;
 #pragma unroll
   for (int c = 0; c < HDT; c += 32) {
     uint32_t r[32];
     tc::tmem_ld32_wait(taddr + c, r);
+#pragma unroll
+    for (int g = 0; g < 32; g += 16) {
+      if (c + g >= hd) break;
+#pragma unroll
+      for (int i = g; i < g + 16; i += 4) {
+        n0 = note_nan(n0, __uint_as_float(r[i]), __uint_as_float(r[i + 1]));
+        n1 = note_nan(n1, __uint_as_float(r[i + 2]), __uint_as_float(r[i + 3]));
+      }
+    }
     uint4 u[4];
 #pragma unroll
     for (int v = 0; v < 4; v++) {
@@ -86,6 +123,7 @@ __device__ __forceinline__ void split_store_rows(bf16* dst, long pitch, uint32_t
     for (int k = 0; k < 4; k++)
       if ((lane & ~3) + k < nlive && c + q * 8 < hd) *reinterpret_cast<uint4*>(base + k * pitch) = u[k];
   }
+  return noted_nan(n0, n1);
 }
 
 template <int HDT>
@@ -100,6 +138,7 @@ struct SplitFwdSmem {
 
 template <int HDT>
 __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_constant__ CUtensorMap tm, const SplitArgs a) {
+  __shared__ __align__(16) unsigned s_nan[4];      // rows to do again
   using S = SplitFwdSmem<HDT>;
   constexpr int CH = S::CH;
   constexpr uint32_t TMEM_COLS = HDT == 128 ? 256 : 128;
@@ -253,6 +292,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
     tc::tc_fence_before();
   }
   const float inv = 1.f / l;
+  uint64_t n0 = pk2(0.f, 0.f), n1 = n0;
   const int lane = tid & 31, nlive = *s_abort ? 0 : a.T - (qrow - lane);
   bf16* dst = a.out + ((size_t)b * a.T + qrow) * C + h * a.hd;
   __syncwarp();
@@ -262,6 +302,10 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
 #pragma unroll
     for (int v = 0; v < 4; v++) {
       const float* x = o + c + v * 8;
+      if (c + v * 8 < a.hd) {
+        n0 = note_nan(note_nan(n0, x[0], x[1]), x[2], x[3]);
+        n1 = note_nan(note_nan(n1, x[4], x[5]), x[6], x[7]);
+      }
       u[v] = make_uint4(pack_bf16(x[0] * inv, x[1] * inv), pack_bf16(x[2] * inv, x[3] * inv), pack_bf16(x[4] * inv, x[5] * inv),
                         pack_bf16(x[6] * inv, x[7] * inv));
     }
@@ -273,6 +317,9 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
       if ((lane & ~3) + k < nlive && c + q * 8 < a.hd) *reinterpret_cast<uint4*>(base + k * (long)C) = u[k];
   }
   if (lane < nlive) a.lse[((size_t)b * a.H + h) * a.T + qrow] = (m + log2f(l)) * LN2;
+  const bool nan = noted_nan(n0, n1) || !(l < INFINITY);
+  const unsigned rows = __ballot_sync(0xffffffffu, nan && lane < nlive);
+  if (lane == 0) s_nan[warp] = rows;
   tc::tc_fence_before();
   __syncthreads();
   if (*s_abort) {
@@ -288,6 +335,8 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
     __syncthreads();
   }
   if (warp == 0) tc::tmem_dealloc(t_s, TMEM_COLS);
+  const uint4 again = *reinterpret_cast<const uint4*>(s_nan);
+  if (again.x | again.y | again.z | again.w) split_redo<0>(again, a, q0, h, b, (float*)smem);
 }
 
 // Backward, KV = true: dK and dV of a 128-key tile, streaming Q / dO;  KV = false: dQ of a 128-query tile, streaming K / V.
@@ -309,6 +358,7 @@ struct SplitBwdSmem {
 template <int HDT, bool KV>
 __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUtensorMap tm_do,
                                                                   const SplitArgs a) {
+  __shared__ __align__(16) unsigned s_nan[4];      // rows to do again
   using S = SplitBwdSmem<HDT, KV>;
   constexpr int CH = S::CH;
   constexpr uint32_t TMEM_COLS = (KV && HDT == 128) ? 512 : 256;
@@ -470,12 +520,10 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
   const int lane = tid & 31, nlive = *s_abort ? 0 : a.T - (row - lane);
   bf16* dst = a.out + ((size_t)b * a.T + row) * 3 * C + xh;
   __syncwarp();
-  if (KV) {
-    split_store_rows<HDT>(dst + C, 3L * C, t_a1 + lane_addr, a.hd, a.scale, lane, nlive);
-    split_store_rows<HDT>(dst + 2 * C, 3L * C, t_a0 + lane_addr, a.hd, 1.f, lane, nlive);
-  } else {
-    split_store_rows<HDT>(dst, 3L * C, t_a0 + lane_addr, a.hd, a.scale, lane, nlive);
-  }
+  bool nan = split_store_rows<HDT>(KV ? dst + C : dst, 3L * C, (KV ? t_a1 : t_a0) + lane_addr, a.hd, a.scale, lane, nlive);
+  if (KV) nan |= split_store_rows<HDT>(dst + 2 * C, 3L * C, t_a0 + lane_addr, a.hd, 1.f, lane, nlive);
+  const unsigned rows = __ballot_sync(0xffffffffu, nan && lane < nlive);
+  if (lane == 0) s_nan[warp] = rows;
   tc::tc_fence_before();
   __syncthreads();
   if (*s_abort) {
@@ -488,6 +536,8 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
     __syncthreads();
   }
   if (warp == 0) tc::tmem_dealloc(t_s, TMEM_COLS);
+  const uint4 again = *reinterpret_cast<const uint4*>(s_nan);
+  if (again.x | again.y | again.z | again.w) split_redo<KV ? 1 : 2>(again, a, r0, h, b, (float*)smem);
 }
 
 template <int HDT>
@@ -517,7 +567,7 @@ static bool split_ok(const void* qkv, const void* a, const void* b, int T, int h
 static int split_fwd(void* out, float* lse, const void* qkv, int B, int T, int H, int hd, int causal, cudaStream_t st) {
   const CUtensorMap* tm = mlb_tmap_seq3d_cached(qkv, B, T, 3L * H * hd);
   if (!tm) return -2;
-  SplitArgs a{B, T, H, hd, causal, 1.0f / sqrtf((float)hd), (bf16*)out, lse, nullptr};
+  SplitArgs a{B, T, H, hd, causal, 1.0f / sqrtf((float)hd), (bf16*)out, lse, nullptr, (const bf16*)qkv, nullptr};
   return hd <= 32 ? split_fwd_launch<32>(tm, a, st) : hd <= 64 ? split_fwd_launch<64>(tm, a, st) : split_fwd_launch<128>(tm, a, st);
 }
 // `delta` = rowsum(dO * O) is already there
@@ -526,6 +576,6 @@ static int split_bwd(void* dqkv, const void* dout, const void* qkv, const float*
   const CUtensorMap* tm = mlb_tmap_seq3d_cached(qkv, B, T, 3L * H * hd);
   const CUtensorMap* td = mlb_tmap_seq3d_cached(dout, B, T, (long)H * hd);
   if (!tm || !td) return -2;
-  SplitArgs a{B, T, H, hd, causal, 1.0f / sqrtf((float)hd), (bf16*)dqkv, const_cast<float*>(lse), delta};
+  SplitArgs a{B, T, H, hd, causal, 1.0f / sqrtf((float)hd), (bf16*)dqkv, const_cast<float*>(lse), delta, (const bf16*)qkv, (const bf16*)dout};
   return hd <= 32 ? split_bwd_launch<32>(tm, td, a, st) : hd <= 64 ? split_bwd_launch<64>(tm, td, a, st) : split_bwd_launch<128>(tm, td, a, st);
 }

@@ -1155,3 +1155,44 @@ def test_causal_attention_128_rounds_no_row_maximum(T, spread):
     e = (torch.softmax(s, -1) @ v).transpose(0, 1).reshape(T, H * hd)
     same = (o / l).float().bfloat16().double().transpose(0, 1).reshape(T, H * hd)
     assert _rel(out, e) < 1.03 * _rel(same, e)
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("T,hd", [(64, 32), (200, 48), (197, 64), (150, 112)])
+@pytest.mark.parametrize("where,value", [("v", float("inf")), ("k", float("-inf")), ("q", float("inf")), ("dout", float("inf")), ("v", float("nan"))])
+def test_split_attention_keeps_infinities_where_they_belong(causal, T, hd, where, value):
+    """One non-finite value in one token's V, K, Q or dO: what it reaches and what it leaves alone (the rows that do not see it, under
+    the causal mask) is what the scalar kernels give, NaN, infinite or finite."""
+    if causal and hd == 64:
+        pytest.skip("that head size has its own causal kernels")
+    torch.manual_seed(T + hd)
+    B, H, at = 2, 2, T - T // 4
+    qkv, dout = rnd(B * T, 3 * H * hd), rnd(B * T, H * hd)
+    if where == "dout":
+        dout[T // 3, hd + 3] = value
+    else:
+        qkv.view(B, T, 3, H, hd)[0, at, "qkv".index(where), 1, 5] = value
+    n = nat()
+
+    def run():
+        out, lse = rnd(B * T, H * hd), torch.empty(B, H, T, device=dev())
+        dqkv = torch.zeros(B * T, 3 * H * hd, device=dev(), dtype=torch.bfloat16)
+        if causal:
+            n.attn_fwd(out, lse, qkv, B, T, H, hd)
+            n.attn_bwd(dqkv, dout, qkv, out, lse, B, T, H, hd)
+        else:
+            n.attn_bidir_fwd(out, lse, qkv, B, T, H, hd)
+            n.attn_bidir_bwd(dqkv, dout, qkv, out, lse, B, T, H, hd)
+        return out, lse, dqkv
+    got = run()
+    n.lib().mlb_attn_force_simt(1)
+    try:
+        e = run()
+    finally:
+        n.lib().mlb_attn_force_simt(0)
+    for a, b in zip(got, e):
+        assert torch.equal(a.isnan(), b.isnan())
+        assert torch.equal(a.isinf(), b.isinf()) and torch.equal(a[a.isinf()], b[b.isinf()])
+        assert _rel(a[a.isfinite()], b[b.isfinite()].double()) < 2 ** -7
+    if causal and where != "dout":
+        assert got[0][:at].isfinite().all()
