@@ -217,8 +217,10 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
     tc::tc_fence_after();
     const int k0 = j * 64;
     const int last = a.causal ? min(qrow, a.T - 1) : a.T - 1;      // last key this row sees
-    // the scores are read twice, 32 at a time (once for the maximum): a row's 64 in registers on top of its HDT output columns
-    // would cost a resident CTA
+    // The scores are read twice, 32 at a time (once for the maximum): a row's 64 in registers on top of its HDT output columns
+    // would cost a resident CTA.  At 128 output columns it is more than that: the 255 registers it takes, and the build (nvcc 12.9) then
+    // forms the operand addresses of this loop's score products wrongly from the second k-step on (the first is right, the rest come
+    // from elsewhere; the descriptors' values in the source are right, and the prologue's product is).
     auto load_scores = [&](int half, uint32_t (&r)[32]) {
       tc::tmem_ld32_wait(t_s + half * 32 + lane_addr, r);
       if (k0 + half * 32 + 31 > last) {
