@@ -2201,7 +2201,7 @@ MLB_API int mlb_attn_fwd(void* out, float* lse, const void* qkv, int B, int T, i
   const int C = H * hd;
   const float scale = 1.0f / sqrtf((float)hd);
   if (tc_ok(qkv, out, H, hd)) {
-    const CUtensorMap* tm = mlb_tmap_cached(qkv, (uint64_t)B * T, 3 * C, 3 * C, 128, 64);
+    const CUtensorMap* tm = hd == 64 ? mlb_tmap_cached(qkv, (uint64_t)B * T, 3 * C, 3 * C, 128, 64) : mlb_tmap_seq3d_cached(qkv, B, T, 3L * C);
     if (!tm) return -2;
     AttnArgs a{B, T, H, hd, scale, (bf16*)out, lse, nullptr, nullptr, nullptr, nullptr, g_fwd_rows, g_timeline};
     const long items = (long)((T + 127) / 128) * H * B;
@@ -2245,9 +2245,7 @@ MLB_API int mlb_attn_fwd(void* out, float* lse, const void* qkv, int B, int T, i
       (void)once;
       attn_fwd_tc_kernel<<<grid, ATT_THREADS, FwdSmem::TOTAL, st>>>(*tm, a);
     } else {
-      const CUtensorMap* t3 = mlb_tmap_seq3d_cached(qkv, B, T, 3L * C);
       const CUtensorMap* to = (T % 128 == 0) ? mlb_tmap_cached(out, (uint64_t)B * T, C, C, 32, 64, 2) : nullptr;
-      if (!t3) return -2;
       a.out_tma = to != nullptr;
       if (!to) to = tm;      // unused by the kernel then
       const long pairs = (long)(((T + 127) / 128 + 1) / 2) * H * B;
@@ -2257,7 +2255,7 @@ MLB_API int mlb_attn_fwd(void* out, float* lse, const void* qkv, int B, int T, i
       a.sched_stride = sched.stride;
       static int once = set_smem(attn_fwd128_k, Fwd128Smem::TOTAL);
       (void)once;
-      mlb_launch_tmem(attn_fwd128_k, grid2, dim3(FWD128_THREADS), Fwd128Smem::TOTAL, st, *t3, *to, a);
+      mlb_launch_tmem(attn_fwd128_k, grid2, dim3(FWD128_THREADS), Fwd128Smem::TOTAL, st, *tm, *to, a);
     }
     return (int)cudaGetLastError();
   }
@@ -2324,8 +2322,8 @@ static int attn_bwd_impl(void* dqkv, const void* dout, const void* qkv, const vo
   if (!have_delta) attn_delta_launch(delta, dout, out, B, T, H, hd, st);
   if (((uintptr_t)cosT | (uintptr_t)sinT) & 15) cosT = sinT = nullptr;      // the epilogues read the tables in 16-byte units; the caller rotates
   if (tc_ok(qkv, dout, H, hd) && ((uintptr_t)dqkv % 16 == 0)) {
-    const CUtensorMap* tq = mlb_tmap_cached(qkv, (uint64_t)B * T, 3 * C, 3 * C, 128, 64);
-    const CUtensorMap* td = mlb_tmap_cached(dout, (uint64_t)B * T, C, C, 128, 64);
+    const CUtensorMap* tq = hd == 64 ? mlb_tmap_cached(qkv, (uint64_t)B * T, 3 * C, 3 * C, 128, 64) : mlb_tmap_seq3d_cached(qkv, B, T, 3L * C);
+    const CUtensorMap* td = hd == 64 ? mlb_tmap_cached(dout, (uint64_t)B * T, C, C, 128, 64) : mlb_tmap_seq3d_cached(dout, B, T, C);
     if (!tq || !td) return -2;
     AttnArgs a{B, T, H, hd, scale, (bf16*)dqkv, const_cast<float*>(lse), delta, cosT, sinT, (bf16*)dq_part, 0, g_timeline};
     dim3 grid((T + 127) / 128, H, B);
@@ -2363,9 +2361,6 @@ static int attn_bwd_impl(void* dqkv, const void* dout, const void* qkv, const vo
       attn_bwd_kv_tc_kernel<<<grid, BWD_THREADS, BwdKVSmem::TOTAL, st>>>(*tq, *td, a);
       attn_bwd_q_tc_kernel<<<grid, BWD_THREADS, BwdQSmem::TOTAL, st>>>(*tq, *td, a);
     } else {
-      const CUtensorMap* t3 = mlb_tmap_seq3d_cached(qkv, B, T, 3L * C);
-      const CUtensorMap* d3 = mlb_tmap_seq3d_cached(dout, B, T, C);
-      if (!t3 || !d3) return -2;
       static int o1 = set_smem(attn_bwd_kv128_k, BwdKV128Smem::TOTAL);
       static int o2 = set_smem(attn_bwd_q128_k, BwdQ128Smem::TOTAL);
       (void)o1; (void)o2;
@@ -2379,8 +2374,8 @@ static int attn_bwd_impl(void* dqkv, const void* dout, const void* qkv, const vo
       const SchedUse sched = n_items > sms ? attn_schedule(1, B, H, T, (int)grid_p.x, st) : SchedUse{};
       a.sched = sched.table;
       a.sched_stride = sched.stride;
-      mlb_launch_tmem(attn_bwd_kv128_k, grid_p, dim3(BWD128_THREADS), BwdKV128Smem::TOTAL, st, *t3, *d3, a);
-      mlb_launch_tmem(attn_bwd_q128_k, grid_p, dim3(BWD128_THREADS), BwdQ128Smem::TOTAL, st, *t3, *d3, a);
+      mlb_launch_tmem(attn_bwd_kv128_k, grid_p, dim3(BWD128_THREADS), BwdKV128Smem::TOTAL, st, *tq, *td, a);
+      mlb_launch_tmem(attn_bwd_q128_k, grid_p, dim3(BWD128_THREADS), BwdQ128Smem::TOTAL, st, *tq, *td, a);
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return (int)e + 1000;
