@@ -76,6 +76,14 @@ __device__ __noinline__ void split_redo(uint4 nan_rows, SplitArgs a, int r0, int
   for (int i = 0; i < 128; i++) {
     const unsigned word = i < 32 ? nan_rows.x : i < 64 ? nan_rows.y : i < 96 ? nan_rows.z : nan_rows.w;
     if (!(word >> (i & 31) & 1)) continue;
+    if (FORM == 1) {      // NaN all over, rightly: nothing to do again
+      bool seen = false;
+      for (int q = (a.causal ? r0 + i : 0) + threadIdx.x; q < a.T; q += SPLIT_THREADS) {
+        const float L = a.lse[((size_t)b * a.H + h) * a.T + q];
+        seen |= L != L;
+      }
+      if (__syncthreads_or(seen)) continue;
+    }
     if (FORM == 0) attn_fwd_simt_row(a.out, a.lse, a.qkv, r0 + i, h, b, a.T, a.H, a.hd, a.scale, a.causal, sc);
     else if (FORM == 1) attn_bwd_kv_simt_row(a.out, a.dout, a.qkv, a.lse, a.delta, r0 + i, h, b, a.T, a.H, a.hd, a.scale, a.causal, sc);
     else attn_bwd_q_simt_row(a.out, a.dout, a.qkv, a.lse, a.delta, r0 + i, h, b, a.T, a.H, a.hd, a.scale, a.causal, sc);
@@ -319,7 +327,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
       if ((lane & ~3) + k < nlive && c + q * 8 < a.hd) *reinterpret_cast<uint4*>(base + k * (long)C) = u[k];
   }
   if (lane < nlive) a.lse[((size_t)b * a.H + h) * a.T + qrow] = (m + log2f(l)) * LN2;
-  const bool nan = noted_nan(n0, n1) || !(l < INFINITY);
+  const bool nan = noted_nan(n0, n1) && l == l;      // (a NaN among the scores is in all of the row, rightly)
   const unsigned rows = __ballot_sync(0xffffffffu, nan && lane < nlive);
   if (lane == 0) s_nan[warp] = rows;
   tc::tc_fence_before();
@@ -522,8 +530,10 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
   const int lane = tid & 31, nlive = *s_abort ? 0 : a.T - (row - lane);
   bf16* dst = a.out + ((size_t)b * a.T + row) * 3 * C + xh;
   __syncwarp();
+  // (a query whose lse or delta is NaN makes all of its dQ NaN, rightly, and a NaN lse all of the dK and dV that see it)
   bool nan = split_store_rows<HDT>(KV ? dst + C : dst, 3L * C, (KV ? t_a1 : t_a0) + lane_addr, a.hd, a.scale, lane, nlive);
   if (KV) nan |= split_store_rows<HDT>(dst + 2 * C, 3L * C, t_a0 + lane_addr, a.hd, 1.f, lane, nlive);
+  if (!KV) nan = nan && lse_r == lse_r && delta_r == delta_r;
   const unsigned rows = __ballot_sync(0xffffffffu, nan && lane < nlive);
   if (lane == 0) s_nan[warp] = rows;
   tc::tc_fence_before();

@@ -1159,7 +1159,8 @@ def test_causal_attention_128_rounds_no_row_maximum(T, spread):
 
 @pytest.mark.parametrize("causal", [False, True])
 @pytest.mark.parametrize("T,hd", [(64, 32), (200, 48), (197, 64), (150, 112)])
-@pytest.mark.parametrize("where,value", [("v", float("inf")), ("k", float("-inf")), ("q", float("inf")), ("dout", float("inf")), ("v", float("nan"))])
+@pytest.mark.parametrize("where,value", [("v", float("inf")), ("k", float("-inf")), ("q", float("inf")), ("dout", float("inf")), ("v", float("nan")),
+                                         ("k", float("nan"))])
 def test_split_attention_keeps_infinities_where_they_belong(causal, T, hd, where, value):
     """One non-finite value in one token's V, K, Q or dO: what it reaches and what it leaves alone (the rows that do not see it, under
     the causal mask) is what the scalar kernels give, NaN, infinite or finite."""
