@@ -1197,3 +1197,20 @@ def test_split_attention_keeps_infinities_where_they_belong(causal, T, hd, where
         assert _rel(a[a.isfinite()], b[b.isfinite()].double()) < 2 ** -7
     if causal and where != "dout":
         assert got[0][:at].isfinite().all()
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("T,hd", [(513, 16), (577, 64), (260, 80), (400, 96), (577, 128)])
+def test_split_attention_over_many_blocks(T, hd, causal):
+    """Five to ten key blocks, at every padded head size: the products of the loop and of its prologue are separate code.  Bounds as for
+    the short sequences: one rounding to bf16 (2^-9), the backward's delta another."""
+    if causal and hd in (64, 128):
+        pytest.skip("those head sizes have their own causal kernels")
+    torch.manual_seed(T + hd)
+    B, H, n = 2, 2, nat()
+    qkv, dout = rnd(B * T, 3 * H * hd), rnd(B * T, H * hd)
+    out, lse, dqkv = rnd(B * T, H * hd), torch.empty(B, H, T, device=dev()), torch.zeros(B * T, 3 * H * hd, device=dev(), dtype=torch.bfloat16)
+    (n.attn_fwd if causal else n.attn_bidir_fwd)(out, lse, qkv, B, T, H, hd)
+    (n.attn_bwd if causal else n.attn_bidir_bwd)(dqkv, dout, qkv, out, lse, B, T, H, hd)
+    eo, el, ed = _attn64(qkv, dout, B, T, H, hd, causal)
+    assert _rel(out, eo) < 2 ** -9 and _rel(lse, el) < 1e-6 and _rel(dqkv, ed) < 2 ** -8
