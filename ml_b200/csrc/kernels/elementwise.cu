@@ -9,6 +9,7 @@
 #include <cuda_fp8.h>
 #include "../no_alloc.h"
 
+#include <algorithm>
 #include <cstdio>
 
 MLB_DEFINE_ERROR_WORD(elementwise)
@@ -1172,6 +1173,31 @@ __global__ void __launch_bounds__(256) scale_dev_k(bf16* __restrict__ out, const
   for (int h = 0; h < 2; h++)
     for (long e = h ? i2 : i, end = e + 8; e < end && e < n; e++) out[e] = __float2bfloat16(__bfloat162float(x[e]) * f);
 }
+// x *= s[0], in place, rounded as above.  A factor of one (the usual gradient of a mean loss) leaves every value as it is, so the blocks
+// read the scalar and return: at 16384 x 50304 that saves the 3.3 GB pass (head and loss, forward and backward: 4213 -> 3791 us).  A grid of resident blocks
+// that walk the tensor, because the 200 K blocks of the kernel above take as long to come and go as a quarter of that.
+__global__ void __launch_bounds__(256) scale_dev_inplace_k(bf16* x, const float* __restrict__ s, long n) {
+  mlb_pdl_sync();
+  const float f = *s;
+  if (f == 1.f) return;
+  const long step = (long)gridDim.x * 4096;
+  for (long i = ((long)blockIdx.x * 512 + threadIdx.x) * 8; i < n; i += step) {
+    const long i2 = i + 256 * 8;
+    if (i2 + 7 < n) {
+      const uint4 ra = __ldcs(reinterpret_cast<const uint4*>(x + i)), rb = __ldcs(reinterpret_cast<const uint4*>(x + i2));
+      float a[8], b[8];
+      unpack8(ra, a);
+      unpack8(rb, b);
+#pragma unroll
+      for (int j = 0; j < 8; j++) { a[j] *= f; b[j] *= f; }
+      store8(x + i, a);
+      store8(x + i2, b);
+      continue;
+    }
+    for (int h = 0; h < 2; h++)
+      for (long e = h ? i2 : i, end = e + 8; e < end && e < n; e++) x[e] = __float2bfloat16(__bfloat162float(x[e]) * f);
+  }
+}
 __global__ void cast_b2f_k(float* __restrict__ out, const bf16* __restrict__ in, long n, float scale) {
   long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) out[i] = __bfloat162float(in[i]) * scale;
@@ -1482,8 +1508,22 @@ MLB_API int mlb_ce_mean(float* loss, float* losses, float* stats, void* dlogits,
   }
   LAUNCH_RET;
 }
+static long sm_count() {
+  static int n = 0;
+  if (n <= 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) { cudaGetLastError(); n = 148; }
+  }
+  return n;
+}
+// out == x: in place, and no pass at all when the factor turns out to be one
 MLB_API int mlb_scale_dev(void* out, const void* x, const float* s, long n, cudaStream_t st) {
   if (((uintptr_t)out | (uintptr_t)x) & 15) return -7;
+  if (n > 0 && out == x) {
+    mlb_launch(scale_dev_inplace_k, dim3((unsigned)std::min((n + 4095) / 4096, 8L * sm_count())), dim3(256), 0, st, (bf16*)out, s, n);
+    LAUNCH_RET;
+  }
   if (n > 0) mlb_launch(scale_dev_k, dim3((unsigned)((n + 4095) / 4096)), dim3(256), 0, st, (bf16*)out, (const bf16*)x, s, n);
   LAUNCH_RET;
 }

@@ -176,12 +176,17 @@ class CrossEntropy(torch.autograd.Function):
         ops.ce_mean(loss, losses, grad, logits, tgt)
         if grad is not None:
             ctx.save_for_backward(grad)
+            # a pack hook may have kept the tensor itself: then it is not this node's alone
+            ctx.shared = torch._C._autograd._top_saved_tensors_default_hooks(False) is not None
         return loss
 
     @staticmethod
     def backward(ctx, g):
         (dlogits,) = ctx.saved_tensors
-        out = _like(dlogits, *dlogits.shape)
+        # The last use of the saved gradient (the graph is not kept for another pass): scaled in place and handed out, and not even
+        # read when the factor is one.
+        last = not ctx.shared and not torch._C._autograd._get_current_graph_task_keep_graph()
+        out = dlogits if last else _like(dlogits, *dlogits.shape)
         ops.scale_dev(out, dlogits, g.float().contiguous())
         return out, None
 

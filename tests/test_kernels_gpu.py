@@ -1214,3 +1214,31 @@ def test_split_attention_over_many_blocks(T, hd, causal):
     (n.attn_bwd if causal else n.attn_bidir_bwd)(dqkv, dout, qkv, out, lse, B, T, H, hd)
     eo, el, ed = _attn64(qkv, dout, B, T, H, hd, causal)
     assert _rel(out, eo) < 2 ** -9 and _rel(lse, el) < 1e-6 and _rel(dqkv, ed) < 2 ** -8
+
+
+@pytest.mark.parametrize("rows,V", [(1, 8), (37, 250), (300, 4104), (1200, 512)])
+@pytest.mark.parametrize("factor", [1.0, 0.37])
+def test_cross_entropy_gradient_in_place_and_not(rows, V, factor):
+    """The saved gradient is scaled in place at its last use only: a kept graph, a pack hook that holds on to the tensor and a plain pass
+    give the same bits, and what the hook holds stays as it was."""
+    from ml_b200.ops import autograd as F
+    torch.manual_seed(rows + V)
+    x, tgt = rnd(rows, V, scale=2.0), torch.randint(0, V, (rows,), device=dev(), dtype=torch.int32)
+    leaf = x.clone().requires_grad_(True)
+    (F.cross_entropy(leaf, tgt) * factor).backward()
+    z = x.clone().requires_grad_(True)
+    loss = F.cross_entropy(z, tgt) * factor
+    first, = torch.autograd.grad(loss, z, retain_graph=True)
+    again, = torch.autograd.grad(loss, z, retain_graph=True)
+    last, = torch.autograd.grad(loss, z)
+    held = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: held.append(t) or t, lambda t: t):
+        hooked = F.cross_entropy(z, tgt) * factor
+    keep = [t.clone() for t in held]
+    through, = torch.autograd.grad(hooked, z)
+    assert held and all(torch.equal(a, b) for a, b in zip(held, keep))
+    for g in (again, last, through, leaf.grad):
+        assert torch.equal(first, g)
+    e = x.double().requires_grad_(True)
+    eg, = torch.autograd.grad(torch.nn.functional.cross_entropy(e, tgt.long()) * factor, e)
+    assert _rel(first, eg) < 2 ** -7      # (two roundings to bf16)
