@@ -1,11 +1,13 @@
-"""In-tree build of the two native libraries.
+"""In-tree build of the native libraries.
 
   ml_b200/_lib/libmlb_host.so   C++17 host runtime (RNG init, token loader, checkpoint IO, metrics writers)
   ml_b200/_lib/libmlb_cuda.so   CUDA kernels, compiled ONLY for compute_100a / sm_100a
+  ml_b200/_lib/libmlb_torch.so  the operators' host path on torch tensors (a Python extension module; ops/autograd.py)
 
 Each translation unit is compiled to an object with its own nvcc/g++ invocation (run in parallel) and
-re-used while its source hash is unchanged.  The libraries expose a plain C ABI consumed through ctypes,
-so no Python/torch headers are compiled.  `python -m ml_b200.build` builds both; importing
+re-used while its source hash is unchanged.  The first two expose a plain C ABI consumed through ctypes, without
+Python/torch headers; only the third is bound to the torch and Python it was built with (both are part of its hash).
+`python -m ml_b200.build` builds all; importing
 `ml_b200.ops.native` builds on demand when a library is missing or stale and a compiler is available.
 """
 from __future__ import annotations
@@ -23,6 +25,7 @@ CSRC = ROOT / "csrc"
 LIB = ROOT / "_lib"
 HOST_LIB = LIB / "libmlb_host.so"
 CUDA_LIB = LIB / "libmlb_cuda.so"
+TORCH_LIB = LIB / "libmlb_torch.so"
 
 NVCC_FLAGS = ["-std=c++17", "-O3", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
               "--use_fast_math", "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC", "-Xptxas", "-v",
@@ -106,6 +109,37 @@ def build_host(verbose=False):
     return HOST_LIB
 
 
+def torch_hash():
+    import torch
+    return _hash(sorted((CSRC / "torch").glob("*.cpp")), f"{torch.__version__} {sys.version_info[:2]}")
+
+
+def build_torch(verbose=False):
+    """The extension module, against the torch and the Python that run this."""
+    LIB.mkdir(exist_ok=True)
+    h = torch_hash()
+    if is_fresh(TORCH_LIB, h):
+        return TORCH_LIB
+    import sysconfig
+    import torch
+    base, nvcc = Path(torch.__file__).parent, _nvcc()
+    cuda = Path(nvcc).resolve().parent.parent if nvcc else Path("/usr/local/cuda")
+    inc = [base / "include", base / "include/torch/csrc/api/include", cuda / "include", sysconfig.get_paths()["include"]]
+    with _BuildLock("torch.lock"):
+        if is_fresh(TORCH_LIB, h):
+            return TORCH_LIB
+        tmp = TORCH_LIB.with_suffix(".so.tmp%d" % os.getpid())
+        cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+               *(f"-I{i}" for i in inc), *map(str, sorted((CSRC / "torch").glob("*.cpp"))), "-o", str(tmp), f"-L{base / 'lib'}",
+               "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10", "-lc10_cuda", "-ldl"]
+        if verbose:
+            print(" ".join(cmd))
+        subprocess.run(cmd, check=True, capture_output=not verbose)
+        os.replace(tmp, TORCH_LIB)
+        _stamp(TORCH_LIB).write_text(h)
+    return TORCH_LIB
+
+
 class _BuildLock:
     """Exclusive lock on a file in _lib/: several ranks of one job may find the library stale at the same moment; one
     builds, the others wait and then find it fresh."""
@@ -178,8 +212,9 @@ def _build_cuda_locked(h, verbose, force):
 def build_all(verbose=False, force=False):
     build_host(verbose)
     build_cuda(verbose, force)
+    build_torch(verbose)
 
 
 if __name__ == "__main__":
     build_all(verbose=True, force="--force" in sys.argv)
-    print("built", HOST_LIB, CUDA_LIB)
+    print("built", HOST_LIB, CUDA_LIB, TORCH_LIB)

@@ -208,11 +208,52 @@ class Embedding(torch.autograd.Function):
         return dw.to(ctx.dtype), None, None
 
 
-linear = Linear.apply
-rmsnorm = RMSNorm.apply
-swiglu = SwiGLU.apply
-rope_causal_attention = RopeCausalAttention.apply
-cross_entropy = CrossEntropy.apply
-bidir_attention = BidirAttention.apply
-layer_norm = LayerNorm.apply
+# What programs call.  Plain calls on CUDA tensors go through the extension module (csrc/torch/bridge.cpp), which runs the same kernels
+# on the same saved tensors without the interpreter; it declines what is not plain, and that takes the Functions above.
+def _plain(name, x, *args):
+    if not getattr(x, "is_cuda", False):
+        return NotImplemented
+    b = ops.native_module().bridge()
+    return NotImplemented if b is None else getattr(b, name)(x, *args)
+
+
+def linear(x, W, b=None):
+    y = _plain("linear", x, W, b)
+    return Linear.apply(x, W, b) if y is NotImplemented else y
+
+
+def rmsnorm(x, w, eps):
+    y = _plain("rmsnorm", x, w, eps)
+    return RMSNorm.apply(x, w, eps) if y is NotImplemented else y
+
+
+def swiglu(gu):
+    y = _plain("swiglu", gu)
+    return SwiGLU.apply(gu) if y is NotImplemented else y
+
+
+def rope_causal_attention(qkv, cos, sin, B, T, H, hd, Hkv=None):
+    if getattr(qkv, "is_cuda", False):
+        nat = ops.native_module()
+        y = _plain("rope_causal_attention", qkv, cos, sin, B, T, H, hd, Hkv, nat.FUSED_ATTN_BWD_MAX_SCRATCH if nat.FUSED_ATTN_BWD else 0)
+        if y is not NotImplemented:
+            return y
+    return RopeCausalAttention.apply(qkv, cos, sin, B, T, H, hd, Hkv)
+
+
+def cross_entropy(logits, tgt):
+    y = _plain("cross_entropy", logits, tgt)
+    return CrossEntropy.apply(logits, tgt) if y is NotImplemented else y
+
+
+def bidir_attention(qkv, B, T, H, hd):
+    y = _plain("bidir_attention", qkv, B, T, H, hd)
+    return BidirAttention.apply(qkv, B, T, H, hd) if y is NotImplemented else y
+
+
+def layer_norm(x, w, b, eps):
+    y = _plain("layer_norm", x, w, b, eps)
+    return LayerNorm.apply(x, w, b, eps) if y is NotImplemented else y
+
+
 embedding = Embedding.apply

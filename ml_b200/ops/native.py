@@ -7,8 +7,11 @@ back to PyTorch: if the library cannot be loaded the import fails.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 import os
+import subprocess
 import threading
+import warnings
 from functools import lru_cache
 
 import torch
@@ -119,6 +122,23 @@ def lib():
     if os.environ.get("ENTROPY_ATTN_DYNAMIC", "") == "1":
         L.mlb_attn_dynamic(1)
     return L
+
+
+@lru_cache(maxsize=1)
+def bridge():
+    """The operators' host path as an extension module on this library's kernels (csrc/torch/bridge.cpp), or None where it cannot be
+    built for this torch: ops/autograd.py and the functions below then call the same kernels from Python."""
+    lib()
+    try:
+        path = _build.build_torch()
+    except (OSError, subprocess.CalledProcessError) as e:
+        warnings.warn(f"libmlb_torch.so cannot be built ({e}): operators run through Python, several times slower per call")
+        return None
+    spec = importlib.util.spec_from_file_location("mlb_torch", str(path))
+    m = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(m)
+    m.bind(str(_build.external_lib("libmlb_cuda.so") or _build.CUDA_LIB))
+    return m
 
 
 def gemm_autotune(on: bool):
@@ -240,6 +260,44 @@ def _i(t, name="tensor"):
     return t.data_ptr()
 
 
+# Arguments of the entry points that the extension module has: b bf16, f fp32, i int32, u bytes (tensors, or an address as a number; 0 for
+# none), n a number, s the current stream
+_KINDS = {
+    "linear_fwd": "bbbnnnnnns", "linear_fwd_posembed": "bbbbnnnnnnns", "linear_fwd_rope": "bbbnnnnnnffnns", "linear_fwd_swiglu": "bbbbnnnnnns",
+    "linear_dx": "bbbnnnnnns", "linear_dx_delta": "bbbbfnnnnnnnns", "linear_dw": "fbbnnnnnns", "gemm": "bbbnnnnnnnnns", "gemm_dw_direct": "nnn",
+    "linear_fwd_fp8": "buunnnnnnns", "zero": "bns", "cast_f2b": "bfnns", "colsum_splits": "nn", "colsum": "bbnnfs", "rmsnorm_fwd": "bfbbnnns",
+    "add_rmsnorm_fwd": "bbfbbbnnns", "rmsnorm_fwd_fp8": "bufbbnnnns", "rmsnorm_bwd_blocks": "n", "rmsnorm_bwd": "bfbbbfbnnfis",
+    "rmsnorm_bwd_cast": "bbbbbfbnnfs", "layernorm_fwd": "bffbbbnnns", "layernorm_bwd2": "bbbnbbbffnnfs", "swiglu_fwd": "bbnns",
+    "swiglu_fwd_fp8": "bubnnns", "swiglu_bwd": "bbbnns", "rope": "bffnnnnns", "rope_copy": "bbffnnnnns", "kv_group_sum": "bbnnnns",
+    "attn_fwd": "bfbnnnns", "attn_bwd_scratch_bytes": "nnnn", "attn_bwd": "bbbbffbnnnnffs", "attn_bwd_have_delta": "bbbbffbnnnnffs",
+    "attn_bidir_fwd": "bfbnnnns", "attn_bidir_bwd": "bbbbffnnnns", "ce_mean": "fffbbinns", "ce_fwd_bwd": "fbinnnnns", "scale_dev": "bbfns",
+    "embed_fwd": "bbinnns", "embed_bwd": "fbinnnnns", "adamw": "fbfffnnnnnnnnnfs", "sum_scale": "ffnns"}
+
+
+class _Ctypes:
+    """The entry points as the extension module has them, through ctypes."""
+
+    def __getattr__(self, name):
+        fn, kinds, to = getattr(lib(), name), _KINDS[name[4:]], {"b": _b, "f": _f, "i": _i, "u": _u8}
+
+        def call(*args):
+            a = [to[k](x) if k in to and not isinstance(x, int) else x for k, x in zip(kinds, args, strict=kinds[-1] != "s")]
+            return fn(*a, _st()) if kinds[-1] == "s" else fn(*a)
+
+        setattr(self, name, call)
+        return call
+
+
+_E = None
+
+
+def _entries():
+    global _E
+    if _E is None:
+        _E = bridge() or _Ctypes()
+    return _E
+
+
 _scratch = threading.local()
 
 
@@ -269,7 +327,7 @@ def scratch(key, numel, dtype, device, zero=False):
 def linear_fwd(out, x, W):
     M, K = x.shape
     N = W.shape[0]
-    _chk(lib().mlb_linear_fwd(_b(out), _b(x), _b(W), M, N, K, out.stride(0), x.stride(0), W.stride(0), _st()), "linear_fwd")
+    _chk(_entries().mlb_linear_fwd(out, x, W, M, N, K, out.stride(0), x.stride(0), W.stride(0)), "linear_fwd")
 
 
 def linear_fwd_rope(out, x, W, cos, sin, T, rope_cols):
@@ -277,8 +335,8 @@ def linear_fwd_rope(out, x, W, cos, sin, T, rope_cols):
     columns, position = row % T).  Returns False when the shape does not take that path (nothing was launched)."""
     M, K = x.shape
     N = W.shape[0]
-    fn = lib().mlb_linear_fwd_rope
-    rc = fn(_b(out), _b(x), _b(W), M, N, K, out.stride(0), x.stride(0), W.stride(0), _f(cos), _f(sin), T, rope_cols, _st())
+    fn = _entries().mlb_linear_fwd_rope
+    rc = fn(out, x, W, M, N, K, out.stride(0), x.stride(0), W.stride(0), cos, sin, T, rope_cols)
     if rc == -7:
         return False
     _chk(rc, "linear_fwd_rope")
@@ -293,8 +351,8 @@ def linear_fwd_swiglu(gu, sw, x, W):
     I = sw.shape[1]
     if W.shape[0] != 2 * I or gu.shape[1] != 2 * I or sw.stride(0) != I:
         return False
-    fn = lib().mlb_linear_fwd_swiglu
-    rc = fn(_b(gu), _b(sw), _b(x), _b(W), M, I, K, gu.stride(0), x.stride(0), W.stride(0), _st())
+    fn = _entries().mlb_linear_fwd_swiglu
+    rc = fn(gu, sw, x, W, M, I, K, gu.stride(0), x.stride(0), W.stride(0))
     if rc == -7:
         return False
     _chk(rc, "linear_fwd_swiglu")
@@ -308,8 +366,8 @@ def linear_fwd_posembed(out, x, W, pos, period):
     N = W.shape[0]
     if pos.shape[-1] != N or not pos.is_contiguous():
         return False
-    fn = lib().mlb_linear_fwd_posembed
-    rc = fn(_b(out), _b(x), _b(W), _b(pos), period, M, N, K, out.stride(0), x.stride(0), W.stride(0), _st())
+    fn = _entries().mlb_linear_fwd_posembed
+    rc = fn(out, x, W, pos, period, M, N, K, out.stride(0), x.stride(0), W.stride(0))
     if rc == -7:
         return False
     _chk(rc, "linear_fwd_posembed")
@@ -319,13 +377,13 @@ def linear_fwd_posembed(out, x, W, pos, period):
 def linear_dx(dx, dout, W):
     M, N = dout.shape
     K = W.shape[1]
-    _chk(lib().mlb_linear_dx(_b(dx), _b(dout), _b(W), M, N, K, dx.stride(0), dout.stride(0), W.stride(0), _st()), "linear_dx")
+    _chk(_entries().mlb_linear_dx(dx, dout, W, M, N, K, dx.stride(0), dout.stride(0), W.stride(0)), "linear_dx")
 
 
 def linear_dw(dW, dout, x):
     M, N = dout.shape
     K = x.shape[1]
-    _chk(lib().mlb_linear_dw(_f(dW), _b(dout), _b(x), M, N, K, dW.stride(0), dout.stride(0), x.stride(0), _st()), "linear_dw")
+    _chk(_entries().mlb_linear_dw(dW, dout, x, M, N, K, dW.stride(0), dout.stride(0), x.stride(0)), "linear_dw")
 
 
 def linear_bias_fwd(out, x, W, b):
@@ -340,7 +398,7 @@ def linear_dw_cast(dW, dout, x):
     """dW (bf16, overwritten) = dout^T . x with fp32 accumulation and one rounding.  Either one product that stores bf16, or the
     add-reduce product into a zeroed fp32 buffer and a cast: the second cuts the reduction over the rows up to fill the machine,
     the first saves two launches and 14 bytes per element of dW.  The library's estimate of both decides."""
-    if dW.dtype == torch.bfloat16 and (lib().mlb_gemm_dw_direct(dout.shape[1], x.shape[1], dout.shape[0]) or dW.numel() == 0):
+    if dW.dtype == torch.bfloat16 and (_entries().mlb_gemm_dw_direct(dout.shape[1], x.shape[1], dout.shape[0]) or dW.numel() == 0):
         return gemm(dW, dout, x, True, True, False)
     acc = torch.empty(dW.shape, dtype=torch.float32, device=dW.device)
     zero_(acc)
@@ -353,8 +411,8 @@ def gemm(out, A, B, a_mn=False, b_mn=False, accumulate=False):
     `out` is bf16 (overwritten) or, with accumulate=True, fp32 (added to)."""
     M, K = (A.shape[1], A.shape[0]) if a_mn else A.shape
     N = B.shape[1] if b_mn else B.shape[0]
-    _chk(lib().mlb_gemm(out.data_ptr(), _b(A), _b(B), M, N, K, out.stride(0), A.stride(0), B.stride(0), int(a_mn), int(b_mn),
-                        int(accumulate), _st()), "gemm")
+    _chk(_entries().mlb_gemm(out.data_ptr(), A, B, M, N, K, out.stride(0), A.stride(0), B.stride(0), int(a_mn), int(b_mn),
+                        int(accumulate)), "gemm")
 
 
 def linear_fwd_gather(out, x, N, K, unit_dst, w_off, src_table, shard_elems, world, flags, ctr, spin_limit_s=20.0):
@@ -368,7 +426,7 @@ def linear_fwd_gather(out, x, N, K, unit_dst, w_off, src_table, shard_elems, wor
 
 # ------------------------------------------------------------------ attention
 def attn_fwd(out, lse, qkv, B, T, H, hd):
-    _chk(lib().mlb_attn_fwd(_b(out), _f(lse), _b(qkv), B, T, H, hd, _st()), "attn_fwd")
+    _chk(_entries().mlb_attn_fwd(out, lse, qkv, B, T, H, hd), "attn_fwd")
 
 
 FUSED_ATTN_BWD = True   # head size 64: single fused backward kernel (False = separate dK/dV and dQ kernels)
@@ -384,8 +442,8 @@ def linear_dx_delta(dx, dout, W, o, B, T, H):
     if Cc != H * 64 or M != B * T or dx.stride(0) != Cc or o.stride(0) != Cc:
         return False
     delta = scratch("attn_delta", B * H * T, torch.float32, dout.device)
-    fn = lib().mlb_linear_dx_delta
-    rc = fn(_b(dx), _b(dout), _b(W), _b(o), _f(delta), T, H, M, N, Cc, dx.stride(0), dout.stride(0), W.stride(0), _st())
+    fn = _entries().mlb_linear_dx_delta
+    rc = fn(dx, dout, W, o, delta, T, H, M, N, Cc, dx.stride(0), dout.stride(0), W.stride(0))
     if rc == -7:
         return False
     _chk(rc, "linear_dx_delta")
@@ -397,19 +455,18 @@ def attn_bwd(dqkv, dout, qkv, out, lse, B, T, H, hd, rope=None, have_delta=False
     have_delta: linear_dx_delta has just written this call's delta term, the pass over dO and O is left out.
     Returns True if it did (tensor-core path), False if the caller still has to call rope_bwd."""
     delta = scratch("attn_delta", B * H * T, torch.float32, qkv.device)
-    acc = part = None
+    acc = part = 0
     if hd == 64 and FUSED_ATTN_BWD:
         # per-(query tile, key tile) bf16 partials of dQ; past FUSED_ATTN_BWD_MAX_SCRATCH the two-kernel backward runs
-        nbytes = lib().mlb_attn_bwd_scratch_bytes(B, T, H, hd)
+        nbytes = _entries().mlb_attn_bwd_scratch_bytes(B, T, H, hd)
         if 0 < nbytes <= FUSED_ATTN_BWD_MAX_SCRATCH:
             part = torch.empty(nbytes // 2, dtype=torch.bfloat16, device=qkv.device)      # (too large to be kept per stream)
             acc = part.data_ptr()
-    cp = _f(rope[0]) if rope is not None else None
-    sp = _f(rope[1]) if rope is not None else None
-    fn = lib().mlb_attn_bwd
+    cp, sp = (0, 0) if rope is None else rope
+    fn = _entries().mlb_attn_bwd
     if have_delta:
-        fn = lib().mlb_attn_bwd_have_delta
-    rc = fn(_b(dqkv), _b(dout), _b(qkv), _b(out), _f(lse), _f(delta), acc, B, T, H, hd, cp, sp, _st())
+        fn = _entries().mlb_attn_bwd_have_delta
+    rc = fn(dqkv, dout, qkv, out, lse, delta, acc, B, T, H, hd, cp, sp)
     global LAUNCHES
     LAUNCHES += 2 if have_delta else 3
     if rc < 0 or rc > 1:
@@ -418,23 +475,23 @@ def attn_bwd(dqkv, dout, qkv, out, lse, B, T, H, hd, rope=None, have_delta=False
 
 
 def attn_bidir_fwd(out, lse, qkv, B, T, H, hd):
-    fn = lib().mlb_attn_bidir_fwd
-    _chk(fn(_b(out), _f(lse), _b(qkv), B, T, H, hd, _st()), "attn_bidir_fwd")
+    fn = _entries().mlb_attn_bidir_fwd
+    _chk(fn(out, lse, qkv, B, T, H, hd), "attn_bidir_fwd")
 
 
 def attn_bidir_bwd(dqkv, dout, qkv, out, lse, B, T, H, hd):
     delta = scratch("attn_delta", B * H * T, torch.float32, qkv.device)
-    fn = lib().mlb_attn_bidir_bwd
-    _chk(fn(_b(dqkv), _b(dout), _b(qkv), _b(out), _f(lse), _f(delta), B, T, H, hd, _st()), "attn_bidir_bwd")
+    fn = _entries().mlb_attn_bidir_bwd
+    _chk(fn(dqkv, dout, qkv, out, lse, delta, B, T, H, hd), "attn_bidir_bwd")
 
 
 # ------------------------------------------------------------------ embedding
 def embed_fwd(out, wte, ids):
-    _chk(lib().mlb_embed_fwd(_b(out), _b(wte), _i(ids), ids.numel(), wte.shape[1], wte.shape[0], _st()), "embed_fwd")
+    _chk(_entries().mlb_embed_fwd(out, wte, ids, ids.numel(), wte.shape[1], wte.shape[0]), "embed_fwd")
 
 
 def embed_bwd(dwte, dout, ids, T, n_pre):
-    _chk(lib().mlb_embed_bwd(_f(dwte), _b(dout), _i(ids), ids.numel(), dwte.shape[1], dwte.shape[0], T, n_pre, _st()), "embed_bwd")
+    _chk(_entries().mlb_embed_bwd(dwte, dout, ids, ids.numel(), dwte.shape[1], dwte.shape[0], T, n_pre), "embed_bwd")
 
 
 def set_prefix(x, prefix, B, T, n_pre):
@@ -448,18 +505,18 @@ def gather_prefix_grad(dprefix, dresid, B, T, n_pre):
 # ------------------------------------------------------------------ norms
 def rmsnorm_fwd(out, rstd, x, w, eps):
     rows, Cc = x.shape
-    _chk(lib().mlb_rmsnorm_fwd(_b(out), _f(rstd), _b(x), _b(w), rows, Cc, eps, _st()), "rmsnorm_fwd")
+    _chk(_entries().mlb_rmsnorm_fwd(out, rstd, x, w, rows, Cc, eps), "rmsnorm_fwd")
 
 
 def add_rmsnorm_fwd(resid, out, rstd, a, b, w, eps):
     rows, Cc = a.shape
-    _chk(lib().mlb_add_rmsnorm_fwd(_b(resid), _b(out), _f(rstd), _b(a), _b(b), _b(w), rows, Cc, eps, _st()), "add_rmsnorm_fwd")
+    _chk(_entries().mlb_add_rmsnorm_fwd(resid, out, rstd, a, b, w, rows, Cc, eps), "add_rmsnorm_fwd")
 
 
 def layernorm_fwd(out, mean, rstd, x, w, b, eps):
     rows, Cc = x.shape
-    fn = lib().mlb_layernorm_fwd
-    _chk(fn(_b(out), _f(mean), _f(rstd), _b(x), _b(w), _b(b) if b is not None else None, rows, Cc, eps, _st()), "layernorm_fwd")
+    fn = _entries().mlb_layernorm_fwd
+    _chk(fn(out, mean, rstd, x, w, 0 if b is None else b, rows, Cc, eps), "layernorm_fwd")
 
 
 def _partial(numel, device):
@@ -481,10 +538,10 @@ def layernorm_bwd(dx, dw, db, dy, x, w, mean, rstd):
 def layernorm_bwd_cast(dx, dw, db, dy, x, w, mean, rstd):
     """layernorm_bwd with dw (and db) in bf16, overwritten."""
     rows, Cc = x.shape
-    L = lib()
+    L = _entries()
     part = _partial(L.mlb_rmsnorm_bwd_blocks(rows) * 2 * Cc, x.device)
-    rc = L.mlb_layernorm_bwd2(_b(dx), _b(dw), _b(db) if db is not None else None, 1, _b(dy), _b(x), _b(w), _f(mean), _f(rstd), rows, Cc,
-                              part.data_ptr(), _st())
+    rc = L.mlb_layernorm_bwd2(dx, dw, 0 if db is None else db, 1, dy, x, w, mean, rstd, rows, Cc,
+                              part.data_ptr())
     if rc == -7:
         aw, ab = torch.zeros_like(dw, dtype=torch.float32), torch.zeros_like(dw, dtype=torch.float32)
         layernorm_bwd(dx, aw, ab, dy, x, w, mean, rstd)
@@ -498,9 +555,9 @@ def layernorm_bwd_cast(dx, dw, db, dy, x, w, mean, rstd):
 def rmsnorm_bwd_cast(dx, dw, dy, x, w, rstd, add=None):
     """rmsnorm_bwd with dw in bf16, overwritten."""
     rows, Cc = x.shape
-    L = lib()
+    L = _entries()
     part = _partial(L.mlb_rmsnorm_bwd_blocks(rows) * Cc, x.device)
-    rc = L.mlb_rmsnorm_bwd_cast(_b(dx), _b(dw), _b(dy), _b(x), _b(w), _f(rstd), _b(add) if add is not None else None, rows, Cc, part.data_ptr(), _st())
+    rc = L.mlb_rmsnorm_bwd_cast(dx, dw, dy, x, w, rstd, 0 if add is None else add, rows, Cc, part.data_ptr())
     if rc == -7:
         acc = torch.zeros_like(dw, dtype=torch.float32)
         rmsnorm_bwd(dx, acc, dy, x, w, rstd, add)
@@ -512,9 +569,9 @@ def rmsnorm_bwd_cast(dx, dw, dy, x, w, rstd, add=None):
 def colsum(out, x):
     """out[N] (bf16) = sum of x[M, N] over its rows, in fp32."""
     M, N = x.shape
-    L = lib()
+    L = _entries()
     part = _partial(L.mlb_colsum_splits(M, N) * N, x.device)
-    rc = L.mlb_colsum(_b(out), _b(x), M, N, part.data_ptr(), _st())
+    rc = L.mlb_colsum(out, x, M, N, part.data_ptr())
     if rc == -7:
         out.copy_(x.sum(0))
         return
@@ -523,17 +580,17 @@ def colsum(out, x):
 
 def rmsnorm_bwd(dx, dw, dy, x, w, rstd, add=None):
     rows, Cc = x.shape
-    L = lib()
+    L = _entries()
     blocks = L.mlb_rmsnorm_bwd_blocks(rows)
     # 32 words of tickets, zero between calls, then the partial sums
     ws = scratch("rms_bwd", 32 + (blocks + 16) * Cc, torch.float32, x.device, zero=True).data_ptr()
-    _chk(L.mlb_rmsnorm_bwd(_b(dx), _f(dw), _b(dy), _b(x), _b(w), _f(rstd), _b(add) if add is not None else None,
-                           rows, Cc, ws + 128, ws, _st()), "rmsnorm_bwd")
+    _chk(L.mlb_rmsnorm_bwd(dx, dw, dy, x, w, rstd, 0 if add is None else add,
+                           rows, Cc, ws + 128, ws), "rmsnorm_bwd")
 
 
 # ------------------------------------------------------------------ rope / swiglu / CE / AdamW
 def rope_fwd(qkv, cos, sin, B, T, H, hd):
-    _chk(lib().mlb_rope(_b(qkv), _f(cos), _f(sin), B * T, T, H, hd, 1.0, _st()), "rope_fwd")
+    _chk(_entries().mlb_rope(qkv, cos, sin, B * T, T, H, hd, 1.0), "rope_fwd")
 
 
 def _heads(name, full, grouped, B, T, H, hd, Hkv):
@@ -544,7 +601,7 @@ def _heads(name, full, grouped, B, T, H, hd, Hkv):
 
 def rope_copy(out, qkv, cos, sin, B, T, H, hd, Hkv=None):
     _heads("rope_copy", out, qkv, B, T, H, hd, H if Hkv is None else Hkv)
-    rc = lib().mlb_rope_copy(_b(out), _b(qkv), _f(cos), _f(sin), B * T, T, H, H if Hkv is None else Hkv, hd, _st())
+    rc = _entries().mlb_rope_copy(out, qkv, cos, sin, B * T, T, H, H if Hkv is None else Hkv, hd)
     if rc == -7:      # a head size or alignment that kernel does not take: heads laid out first, then rotated in place
         N, rep = B * T, 1 if Hkv is None else H // Hkv
         o, x = out.view(N, 3 * H, hd), qkv.view(N, -1, hd)
@@ -556,7 +613,7 @@ def rope_copy(out, qkv, cos, sin, B, T, H, hd, Hkv=None):
 
 def kv_group_sum(out, dqkv, B, T, H, hd, Hkv):
     _heads("kv_group_sum", dqkv, out, B, T, H, hd, Hkv)
-    rc = lib().mlb_kv_group_sum(_b(out), _b(dqkv), B * T, H, Hkv, hd, _st())
+    rc = _entries().mlb_kv_group_sum(out, dqkv, B * T, H, Hkv, hd)
     if rc == -7:
         o, x = out.view(B * T, -1, hd), dqkv.view(B * T, 3 * H, hd)
         o[:, :H] = x[:, :H]
@@ -566,23 +623,23 @@ def kv_group_sum(out, dqkv, B, T, H, hd, Hkv):
 
 
 def rope_bwd(dqkv, cos, sin, B, T, H, hd):
-    _chk(lib().mlb_rope(_b(dqkv), _f(cos), _f(sin), B * T, T, H, hd, -1.0, _st()), "rope_bwd")
+    _chk(_entries().mlb_rope(dqkv, cos, sin, B * T, T, H, hd, -1.0), "rope_bwd")
 
 
 def swiglu_fwd(out, gu):
     rows, I2 = gu.shape
-    _chk(lib().mlb_swiglu_fwd(_b(out), _b(gu), rows, I2 // 2, _st()), "swiglu_fwd")
+    _chk(_entries().mlb_swiglu_fwd(out, gu, rows, I2 // 2), "swiglu_fwd")
 
 
 def swiglu_bwd(dgu, dout, gu):
     rows, I2 = gu.shape
-    _chk(lib().mlb_swiglu_bwd(_b(dgu), _b(dout), _b(gu), rows, I2 // 2, _st()), "swiglu_bwd")
+    _chk(_entries().mlb_swiglu_bwd(dgu, dout, gu, rows, I2 // 2), "swiglu_bwd")
 
 
 def ce_fwd_bwd(losses, logits, tgt, dscale, V_valid=None, threads=512):
     rows, V = logits.shape
-    _chk(lib().mlb_ce_fwd_bwd(_f(losses), _b(logits), _i(tgt), rows, V if V_valid is None else V_valid, logits.stride(0),
-                              dscale, threads, _st()), "ce_fwd_bwd")
+    _chk(_entries().mlb_ce_fwd_bwd(losses, logits, tgt, rows, V if V_valid is None else V_valid, logits.stride(0),
+                              dscale, threads), "ce_fwd_bwd")
 
 
 def ce_mean(loss, losses, dlogits, logits, tgt):
@@ -590,16 +647,16 @@ def ce_mean(loss, losses, dlogits, logits, tgt):
     if rows == 0:
         return loss.zero_()
     stats = torch.empty(2, dtype=torch.float32, device=logits.device)
-    d = _b(dlogits) if dlogits is not None else None
-    rc = lib().mlb_ce_mean(_f(loss), _f(losses), _f(stats), d, _b(logits), _i(tgt), rows, V, _st())
+    d = 0 if dlogits is None else dlogits
+    rc = _entries().mlb_ce_mean(loss, losses, stats, d, logits, tgt, rows, V)
     if rc == -7:      # misaligned rows: through an aligned copy
         work = logits.clone() if dlogits is None else dlogits.copy_(logits)
-        rc = lib().mlb_ce_mean(_f(loss), _f(losses), _f(stats), work.data_ptr() if d else None, work.data_ptr(), _i(tgt), rows, V, _st())
+        rc = _entries().mlb_ce_mean(loss, losses, stats, work.data_ptr() if dlogits is not None else 0, work.data_ptr(), tgt, rows, V)
     _chk(rc, "ce_mean")
 
 
 def scale_dev(out, x, s):
-    _chk(lib().mlb_scale_dev(_b(out), _b(x), _f(s), out.numel(), _st()), "scale_dev")
+    _chk(_entries().mlb_scale_dev(out, x, s, out.numel()), "scale_dev")
 
 
 def ce_chunk_stats(rowmax, rowsum, tgt_logit, chunk, tgt, off):
@@ -618,9 +675,9 @@ def adamw(master, params, grads, m, v, lr, b1, b2, eps, wd, bc1, bc2, grad_scale
     """dev_hyper: optional CUDA fp32[4] = {lr, 1/bc1, 1/bc2, grad_scale} read by the kernel instead of the scalar
     arguments (lets a captured graph follow the optimizer step count)."""
     n = master.numel()
-    pp = None if (params is None or params.data_ptr() == master.data_ptr()) else _b(params)
-    hp = _f(dev_hyper) if dev_hyper is not None else None
-    _chk(lib().mlb_adamw(_f(master), pp, _f(grads), _f(m), _f(v), n, lr, b1, b2, eps, wd, bc1, bc2, grad_scale, hp, _st()), "adamw")
+    pp = 0 if (params is None or params.data_ptr() == master.data_ptr()) else params
+    hp = 0 if dev_hyper is None else dev_hyper
+    _chk(_entries().mlb_adamw(master, pp, grads, m, v, n, lr, b1, b2, eps, wd, bc1, bc2, grad_scale, hp), "adamw")
 
 
 # ------------------------------------------------------------------ vision / utilities
@@ -664,8 +721,8 @@ def linear_fwd_fp8(out, x8, W8, out_scale):
     8-bit tensor-core path (nothing was launched)."""
     M, K = x8.shape
     N = W8.shape[0]
-    fn = lib().mlb_linear_fwd_fp8
-    rc = fn(_b(out), _u8(x8), _u8(W8), M, N, K, out.stride(0), x8.stride(0), W8.stride(0), out_scale, _st())
+    fn = _entries().mlb_linear_fwd_fp8
+    rc = fn(out, x8, W8, M, N, K, out.stride(0), x8.stride(0), W8.stride(0), out_scale)
     if rc == -7:
         return False
     _chk(rc, "linear_fwd_fp8")
@@ -698,8 +755,8 @@ def linear_fwd_fp8_swiglu(gu, sw, x8, W8, out_scale):
 
 def rmsnorm_fwd_fp8(out, out8, rstd, x, w, eps, scale):
     rows, Cc = x.shape
-    fn = lib().mlb_rmsnorm_fwd_fp8
-    _chk(fn(_b(out), _u8(out8), _f(rstd), _b(x), _b(w), rows, Cc, eps, scale, _st()), "rmsnorm_fwd_fp8")
+    fn = _entries().mlb_rmsnorm_fwd_fp8
+    _chk(fn(out, out8, rstd, x, w, rows, Cc, eps, scale), "rmsnorm_fwd_fp8")
 
 
 def add_rmsnorm_fwd_fp8(resid, out, out8, rstd, a, b, w, eps, scale):
@@ -710,8 +767,8 @@ def add_rmsnorm_fwd_fp8(resid, out, out8, rstd, a, b, w, eps, scale):
 
 def swiglu_fwd_fp8(out, out8, gu, scale):
     rows, I2 = gu.shape
-    fn = lib().mlb_swiglu_fwd_fp8
-    _chk(fn(_b(out), _u8(out8), _b(gu), rows, I2 // 2, scale, _st()), "swiglu_fwd_fp8")
+    fn = _entries().mlb_swiglu_fwd_fp8
+    _chk(fn(out, out8, gu, rows, I2 // 2, scale), "swiglu_fwd_fp8")
 
 
 def cast_bf16_fp8(out8, x, scale):
@@ -733,14 +790,14 @@ def fp8_qdq(out, x, scale=1.0):
 
 def sum_scale(out, x, scale):
     """out[0] = scale * sum(x) on the device (x fp32, contiguous)."""
-    fn = lib().mlb_sum_scale
-    _chk(fn(_f(out), _f(x), x.numel(), scale, _st()), "sum_scale")
+    fn = _entries().mlb_sum_scale
+    _chk(fn(out, x, x.numel(), scale), "sum_scale")
 
 
 def zero_(x):
-    fn = lib().mlb_zero
+    fn = _entries().mlb_zero
     assert x.is_cuda and x.is_contiguous()
-    _chk(fn(x.data_ptr(), x.numel() * x.element_size(), _st()), "zero")
+    _chk(fn(x.data_ptr(), x.numel() * x.element_size()), "zero")
     global LAUNCHES
     LAUNCHES -= 1          # a memset node, not a kernel of this library: not part of the launch count
 

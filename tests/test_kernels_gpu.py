@@ -1242,3 +1242,99 @@ def test_cross_entropy_gradient_in_place_and_not(rows, V, factor):
     e = x.double().requires_grad_(True)
     eg, = torch.autograd.grad(torch.nn.functional.cross_entropy(e, tgt.long()) * factor, e)
     assert _rel(first, eg) < 2 ** -7      # (two roundings to bf16)
+
+
+def _forms(rows, C):
+    """A [rows, C] operand as programs hold it: dense, the transpose of its transpose, every other row, every other column, off a
+    16-byte boundary."""
+    yield "dense", lambda: rnd(rows, C)
+    yield "transposed", lambda: rnd(C, rows).t()
+    yield "rows", lambda: rnd(2 * rows, C)[::2]
+    yield "columns", lambda: rnd(rows, 2 * C)[:, ::2]
+    yield "offset", lambda: rnd(1, rows * C + 8).view(-1)[3:3 + rows * C].view(rows, C)
+
+
+@pytest.mark.parametrize("form", ["dense", "transposed", "rows", "columns", "offset"])
+@pytest.mark.parametrize("rows,C,N", [(1, 256, 8), (37, 256, 512), (130, 768, 384), (300, 264, 512), (200, 512, 77 * 8)])
+def test_plain_calls_are_what_the_functions_give(form, rows, C, N):
+    """The extension module and the Python Functions run the same kernels in the same order: the same bits, for every form of the operands
+    and of the incoming gradient that either takes (weight gradients with the reduction uncut, which makes their sums repeatable)."""
+    from ml_b200.ops import autograd as F
+    torch.manual_seed(rows + C + N)
+    L = nat().lib()
+
+    def both(fast, slow, leaves, shape):
+        outs = []
+        dout = dict(_forms(*shape))[form]()
+        for fn in (fast, slow):
+            ls = [t.detach().requires_grad_(True) if t is not None else None for t in leaves]
+            y = fn(*ls)
+            gs = torch.autograd.grad(y, [t for t in ls if t is not None], dout)
+            with torch.no_grad():
+                outs.append([y.detach(), fn(*ls), *gs])
+        for a, b in zip(*outs):
+            assert a.shape == b.shape and a.dtype == b.dtype and torch.equal(a, b), form
+
+    mk = dict(_forms(rows, C))[form]
+    L.mlb_gemm_set_splits(1)
+    try:
+        for b in (None, rnd(1, N).view(-1)):
+            both(lambda x, W, b: F.linear(x, W, b), lambda x, W, b: F.Linear.apply(x, W, b), [mk(), dict(_forms(N, C))[form](), b], (rows, N))
+    finally:
+        L.mlb_gemm_set_splits(0)
+    if form != "offset":      # (the norms and SwiGLU read whole vectors: such rows were never theirs)
+        w, b = rnd(1, C).view(-1), rnd(1, C).view(-1)
+        both(lambda x, w: F.rmsnorm(x, w, 1e-5), lambda x, w: F.RMSNorm.apply(x, w, 1e-5), [mk(), w], (rows, C))
+        both(lambda x, w, b: F.layer_norm(x, w, b, 1e-5), lambda x, w, b: F.LayerNorm.apply(x, w, b, 1e-5), [mk(), w, b], (rows, C))
+        both(F.swiglu, F.SwiGLU.apply, [mk()], (rows, C // 2))
+
+
+@pytest.mark.parametrize("B,T,H,Hkv,hd", [(1, 1, 1, 1, 64), (2, 130, 4, 2, 64), (1, 257, 2, 2, 128), (2, 65, 6, 1, 32), (3, 40, 4, 4, 16)])
+def test_plain_attention_calls_are_what_the_functions_give(B, T, H, Hkv, hd):
+    from ml_b200.ops import autograd as F
+    torch.manual_seed(T)
+    cos, sin = ref.rope_tables(T, hd, 10000.0, dev())
+    for width, fast, slow in (((H + 2 * Hkv) * hd, lambda x: F.rope_causal_attention(x, cos, sin, B, T, H, hd, Hkv),
+                               lambda x: F.RopeCausalAttention.apply(x, cos, sin, B, T, H, hd, Hkv)),
+                              (3 * H * hd, lambda x: F.bidir_attention(x, B, T, H, hd), lambda x: F.BidirAttention.apply(x, B, T, H, hd))):
+        x = rnd(B * T, width).requires_grad_(True)
+        for dout in (rnd(B * T, H * hd), rnd(H * hd, B * T).t()):
+            a, b = fast(x), slow(x)
+            assert torch.equal(a, b) and torch.equal(*(torch.autograd.grad(y, x, dout)[0] for y in (a, b)))
+        with torch.no_grad():
+            assert torch.equal(fast(x), slow(x))
+
+
+def test_what_the_extension_module_declines():
+    """Anything but plain tensors of the current GPU goes to the Python Functions, with their errors."""
+    from torch.utils.checkpoint import checkpoint
+    from ml_b200.ops import autograd as F
+    m, x, W = nat().bridge(), rnd(16, 256), rnd(64, 256)
+    assert isinstance(m.linear(x, W, None), torch.Tensor)
+    for a in ((x.float(), W, None), (x, W.float(), None), (x.cpu(), W, None), (x, rnd(64, 248), None), (x[:0], W, None), (x.view(-1), W, None),
+              (x, W, rnd(1, 63).view(-1)), (x, None, None), (3, W, None), (x.as_subclass(type("T", (torch.Tensor,), {})), W, None)):
+        assert m.linear(*a) is NotImplemented
+    assert m.rmsnorm(rnd(4, 264), rnd(1, 264).view(-1), 1e-5) is NotImplemented      # (its backward is another kernel)
+    with pytest.raises(AssertionError):
+        F.linear(x.float(), W)
+    with pytest.raises(AssertionError):
+        nat().linear_fwd(rnd(16, 64), x.float(), W)
+    with pytest.raises(AssertionError):
+        nat().rmsnorm_fwd(None, torch.empty(16, device=dev()), x, W[0], 1e-5)
+    with torch.autograd.forward_ad.dual_level(), pytest.raises(Exception):
+        F.linear(torch.autograd.forward_ad.make_dual(x, x), W)
+    y = checkpoint(lambda t: F.swiglu(F.linear(t, W)), x.requires_grad_(True), use_reentrant=False)
+    g, = torch.autograd.grad(y, x, torch.ones_like(y))
+    e, = torch.autograd.grad(F.SwiGLU.apply(F.Linear.apply(x, W, None)), x, torch.ones_like(y := y.detach()))
+    assert torch.equal(g, e)
+
+
+def test_entry_points_through_ctypes_and_through_the_module():
+    """The table of argument kinds is the extension module's: one call through each."""
+    n, x, W = nat(), rnd(130, 256), rnd(72, 256)
+    c, m, outs = n._Ctypes(), n.bridge(), [rnd(130, 72), rnd(130, 72)]
+    for e, o in zip((c, m), outs):
+        assert e.mlb_linear_fwd(o, x, W, 130, 72, 256, 72, 256, 256) == 0
+        with pytest.raises(AssertionError):
+            e.mlb_linear_fwd(o, x.float(), W, 130, 72, 256, 72, 256, 256)
+    assert torch.equal(*outs) and c.mlb_gemm_dw_direct(768, 768, 1003) == m.mlb_gemm_dw_direct(768, 768, 1003)
