@@ -625,6 +625,11 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         } else {
           tc::tmem_ld32_wait(taddr + c * SLAB_COLS, r);
         }
+        if (c == SLABS - 1) {      // the accumulator is in registers: its last slab is written while the next tile's products run
+          tc::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive_cluster(tc::mapa_u32(tc::smem_u32(&acc_empty[acc]), 0));
+        }
         const int col0 = n0 + c * SLAB_COLS;
         if (!rows_live || col0 >= g.N) continue;   // warp-uniform
         if (EMODE == 0) {
@@ -732,9 +737,6 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         }
         slab++;
       }
-      tc::tc_fence_before();
-      __syncwarp();
-      if (lane == 0) tc::mbar_arrive_cluster(tc::mapa_u32(tc::smem_u32(&acc_empty[acc]), 0));
     }
     if (EMODE == 0 && lane == 0) tc::tma_wait_group<0>();
   }

@@ -353,8 +353,11 @@ __device__ __forceinline__ uint32_t mapa_u32(uint32_t saddr, uint32_t rank) {
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// Arrival on a barrier of any CTA of the cluster, released at CTA scope: what it hands over are reads of tensor memory that have completed
+// (tcgen05.wait), not writes.  Released at cluster scope it waits until the L2 has taken the stores before it, which in
+// a GEMM's epilogue is ~3000 cycles of every tile (stamps, 16384 x 4096 x 768).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+  asm volatile("mbarrier.arrive.release.cta.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // Tiled loads into THIS CTA's shared memory whose completion bytes go to an mbarrier that may live in the peer CTA.
 __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorMap* map, uint32_t bar_cluster_addr, int x, int y) {

@@ -1282,7 +1282,7 @@ def test_plain_calls_are_what_the_functions_give(form, rows, C, N):
             both(lambda x, W, b: F.linear(x, W, b), lambda x, W, b: F.Linear.apply(x, W, b), [mk(), dict(_forms(N, C))[form](), b], (rows, N))
     finally:
         L.mlb_gemm_set_splits(0)
-    if form != "offset":      # (the norms and SwiGLU read whole vectors: such rows were never theirs)
+    if form != "offset" and C % 256 == 0:      # (the norms and SwiGLU read whole vectors: such rows were never theirs; other widths are not the module's)
         w, b = rnd(1, C).view(-1), rnd(1, C).view(-1)
         both(lambda x, w: F.rmsnorm(x, w, 1e-5), lambda x, w: F.RMSNorm.apply(x, w, 1e-5), [mk(), w], (rows, C))
         both(lambda x, w, b: F.layer_norm(x, w, b, 1e-5), lambda x, w, b: F.LayerNorm.apply(x, w, b, 1e-5), [mk(), w, b], (rows, C))
