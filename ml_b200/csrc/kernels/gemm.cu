@@ -14,6 +14,7 @@
 // word, frees its TMEM and returns.
 #include "../tc.cuh"
 
+#include <algorithm>
 #include <cstdio>
 #include <map>
 #include <array>
@@ -745,6 +746,143 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   if (warp == 1) tc::tmem_dealloc_pair(tmem_base, 2 * BN);
 }
 
+// ------------------------------------------------------------------ few tiles, long reductions: a cluster per tile
+// A product with a handful of 128 x 128 tiles leaves most SMs idle while a few walk the whole reduction (64 x 2048 outputs over 11008:
+// 16 CTAs, 172 k-blocks each).  Here a cluster of 2, 4 or 8 CTAs shares a tile: each multiplies its part of the k-blocks, puts the fp32 result into its
+// own shared memory (over the operand stages, which are done with), and then adds up 128 / S rows of all S parts, in the order of the ranks,
+// through distributed shared memory: no workspace, no atomics, the same bits on every run.  One tile per cluster, not persistent.
+// Bound by the latency of a k-block (~400 cycles) and by what a cluster costs at all (~9000); measured at splitk_ways.
+constexpr int SPLITK_THREADS = 192;      // producer warp, MMA warp, four epilogue warps (all of them add up)
+constexpr int SPLITK_PITCH = 132;        // floats per row of the partial tile: eight rows cover all banks with 16-byte accesses
+struct SplitKSmem {
+  static constexpr int STAGES = 6, STAGE_BYTES = 32768;
+  static constexpr int BAR = STAGES * STAGE_BYTES;
+  static constexpr int TOTAL = BAR + 256 + 1024;
+  static_assert(128 * SPLITK_PITCH * 4 <= BAR, "the partial tile lies over the stages");
+};
+struct SplitKArgs {
+  bf16* out;
+  const bf16* pos;      // added to row r: pos[r % pos_period, :] (null: nothing)
+  int M, N, ldo, tiles_m, kb_total, pos_period, a3d, b3d;
+};
+template <bool A_MN, bool B_MN>
+__global__ void __launch_bounds__(SPLITK_THREADS, 1) gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                                                                        const SplitKArgs g) {
+  using S = SplitKSmem;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint64_t* full = (uint64_t*)(smem + S::BAR);
+  uint64_t *empty = full + S::STAGES, *acc_full = empty + S::STAGES;
+  uint32_t* tmem_slot = (uint32_t*)(acc_full + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = (int)tc::cluster_ctarank(), ways = (int)tc::cluster_nctarank();
+  const int tile = (int)tc::cluster_id_x(), m0 = tile % g.tiles_m * 128, n0 = tile / g.tiles_m * 128;
+  const int kb0 = (int)((long)g.kb_total * rank / ways), kb1 = (int)((long)g.kb_total * (rank + 1) / ways);
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < S::STAGES; i++) { tc::mbar_init(&full[i], 1); tc::mbar_init(&empty[i], 1); }
+    tc::mbar_init(acc_full, 1);
+    tc::mbar_fence_init();
+    tc::tma_prefetch_desc(&tmA);
+    tc::tma_prefetch_desc(&tmB);
+  }
+  if (warp == 1) tc::tmem_alloc(tmem_slot, 128);
+  tc::tc_fence_before();
+  __syncthreads();
+  tc::tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  mlb_pdl_sync();
+  if (warp == 0) {
+    if (tc::elect_one()) {
+      bool ok = true;
+      int n = 0;      // k-blocks asked for
+      for (int kb = kb0; kb < kb1; kb++, n++) {
+        const int stage = n % S::STAGES;
+        if (n >= S::STAGES && !tc::mbar_wait(&empty[stage], (n / S::STAGES + 1) & 1, 0x31)) { ok = false; break; }
+        uint8_t *sA = smem + stage * S::STAGE_BYTES, *sB = sA + S::STAGE_BYTES / 2;
+        tc::mbar_expect_tx(&full[stage], S::STAGE_BYTES);
+        if (!A_MN) tc::tma_load_2d(sA, &tmA, &full[stage], kb * BK, m0);
+        else if (g.a3d) tc::tma_load_3d(sA, &tmA, &full[stage], 0, kb * BK, m0 / 64);
+        else
+          for (int c = 0; c < 2; c++) tc::tma_load_2d(sA + c * 8192, &tmA, &full[stage], m0 + c * 64, kb * BK);
+        if (!B_MN) tc::tma_load_2d(sB, &tmB, &full[stage], kb * BK, n0);
+        else if (g.b3d) tc::tma_load_3d(sB, &tmB, &full[stage], 0, kb * BK, n0 / 64);
+        else
+          for (int c = 0; c < 2; c++) tc::tma_load_2d(sB + c * 8192, &tmB, &full[stage], n0 + c * 64, kb * BK);
+      }
+      // (after an expired wait: what has been asked for lands before the memory is used for anything else)
+      for (int st = 0; !ok && st < S::STAGES && st < n; st++) tc::mbar_wait(&full[st], ((n - st + S::STAGES - 1) / S::STAGES - 1) & 1, 0x32);
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (tc::elect_one()) {
+      constexpr uint32_t idesc = tc::idesc_bf16(128, 128, A_MN ? 1 : 0, B_MN ? 1 : 0);
+      for (int kb = kb0, n = 0; kb < kb1; kb++, n++) {
+        const int stage = n % S::STAGES;
+        if (!tc::mbar_wait(&full[stage], (n / S::STAGES) & 1, 0x33)) break;
+        tc::tc_fence_after();
+        const uint32_t sA = tc::smem_u32(smem + stage * S::STAGE_BYTES), sB = sA + S::STAGE_BYTES / 2;
+#pragma unroll
+        for (int k = 0; k < BK / 16; k++) {
+          const uint64_t da = A_MN ? tc::smem_desc_sw128(sA + k * 2048, 8192, 1024) : tc::smem_desc_sw128(sA + k * 32, 16, 1024);
+          const uint64_t db = B_MN ? tc::smem_desc_sw128(sB + k * 2048, 8192, 1024) : tc::smem_desc_sw128(sB + k * 32, 16, 1024);
+          tc::mma_bf16_ss(tmem, da, db, idesc, (n > 0 || k > 0) ? 1u : 0u);
+        }
+        tc::mma_commit(&empty[stage]);
+      }
+      tc::mma_commit(acc_full);      // (whatever happened: what was issued is waited for)
+    }
+    __syncwarp();
+  }
+  // the last commit covers every product, and so every operand that was read
+  if (warp >= 2) tc::mbar_wait(acc_full, 0, 0x34);
+  __syncthreads();
+  tc::tc_fence_after();
+  float* part = (float*)smem;
+  if (warp >= 2) {
+    const int lg = warp & 3, row = lg * 32 + lane;
+    const uint32_t ta = tmem + ((uint32_t)(lg * 32) << 16);
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+      uint32_t r[32];
+      tc::tmem_ld32_wait(ta + c * 32, r);
+      float4* dst = reinterpret_cast<float4*>(part + row * SPLITK_PITCH + c * 32);
+#pragma unroll
+      for (int v = 0; v < 8; v++)
+        dst[v] = make_float4(__uint_as_float(r[v * 4]), __uint_as_float(r[v * 4 + 1]), __uint_as_float(r[v * 4 + 2]), __uint_as_float(r[v * 4 + 3]));
+    }
+  }
+  tc::tc_fence_before();
+  tc::cluster_sync();
+  const int rows = 128 / ways, r0 = rank * rows;
+  const uint32_t base = tc::smem_u32(part);
+  for (int i = threadIdx.x; i < rows * 16; i += SPLITK_THREADS) {
+    const int row = r0 + (i >> 4), col = (i & 15) * 8;
+    if (m0 + row >= g.M || n0 + col >= g.N) continue;
+    float x[8] = {};
+    for (int q = 0; q < ways; q++) {
+      const uint32_t a = tc::mapa_u32(base + (uint32_t)(row * SPLITK_PITCH + col) * 4, q);
+      float y[8];
+      tc::ld_cluster_f32x4(a, y);
+      tc::ld_cluster_f32x4(a + 16, y + 4);
+#pragma unroll
+      for (int e = 0; e < 8; e++) x[e] += y[e];
+    }
+    if (g.pos != nullptr) {
+      const uint4 pv = __ldg(reinterpret_cast<const uint4*>(g.pos + (size_t)((m0 + row) % g.pos_period) * g.N + n0 + col));
+      const uint32_t pw[4] = {pv.x, pv.y, pv.z, pv.w};
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        x[2 * e] += __uint_as_float(pw[e] << 16);
+        x[2 * e + 1] += __uint_as_float(pw[e] & 0xffff0000u);
+      }
+    }
+    *reinterpret_cast<uint4*>(g.out + (size_t)(m0 + row) * g.ldo + n0 + col) =
+        make_uint4(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]), pack_bf16(x[4], x[5]), pack_bf16(x[6], x[7]));
+  }
+  tc::cluster_sync();      // nobody leaves while another still reads from it
+  if (warp == 1) tc::tmem_dealloc(tmem, 128);
+}
+
 // ------------------------------------------------------------------ SIMT fallback (any shape / alignment)
 // D[m,n] = sum_k A[m*sam + k*sak] * B[n*sbn + k*sbk]; 64x64 tile, 16x16 threads, 4x4 per thread.
 template <int EPI>
@@ -1029,6 +1167,75 @@ struct RopeEpi { const float* cosT; const float* sinT; int T, cols; };
 struct SwigluEpi { bf16* out; int I; };
 struct PosEpi { const bf16* pos; int period; };
 struct DeltaEpi { const bf16* o; float* out; int T, H; };
+// Estimated cycles of a bf16-output product, launch and all (the tiles of a launch run in waves of one per SM or SM pair).
+double cost_pair(double pt, double kb, double pc) { return ceil(pt / pc) * (kb * 512.0 + 2000.0) + 7000.0; }
+double cost_c128(double ct, double kb, double sm) { return ceil(ct / sm) * (kb * 320.0 + 2000.0) + 4000.0; }
+double cost_splitk(double ct, double kb, double clusters, int ways) { return ceil(ct / clusters) * (ceil(kb / ways) * 450.0 + 5000.0) + 4000.0 + 500.0 * ways; }
+int g_splitk = -1;           // tuning hook: -1 = by cost, 1 = never, 2 / 4 / 8 = always that many CTAs per tile
+// Clusters of `ways` CTAs of gemm_splitk_kernel that are resident at once (they do not cross a GPC: 16 or so of eight, not 18)
+int splitk_clusters(int ways) {
+  static int resident[9] = {};
+  int& n = resident[ways];
+  if (n == 0) {
+    auto kern = gemm_splitk_kernel<false, false>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(num_sms() / ways * ways);
+    cfg.blockDim = dim3(SPLITK_THREADS);
+    cfg.dynamicSmemBytes = SplitKSmem::TOTAL;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = ways;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int k = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitKSmem::TOTAL) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&k, kern, &cfg) != cudaSuccess || k <= 0) {
+      cudaGetLastError();
+      k = num_sms() / (ways + ways / 4);
+    }
+    n = k;
+  }
+  return n;
+}
+// CTAs per tile (1: another kernel) and, in `best`, its cost or that of the best of the others.  Measured, us with and without: dX of 64 rows, 2048 columns
+// over 11008 24.6 (four ways) and 45.1, over 50304 67.6 and 169; 768 columns over 50304 41 (eight ways) and 164; 512 rows over 11008 34.8 (two) and 47;
+// the estimate leaves alone what a cluster makes no faster (2048 x 2048 over 64 rows 14.3 and 16.4, 768 x 2304 14.3 and 10.2).
+int splitk_ways(int M, int N, int K, double* best) {
+  const double kb = ceil_div_i(K, BK), pt = (double)ceil_div_i(M, 256) * ceil_div_i(N, 256), ct = (double)ceil_div_i(M, 128) * ceil_div_i(N, 128);
+  const double pc = pair_clusters(), sm = g_max_ctas > 0 ? g_max_ctas : num_sms();
+  double c = cost_c128(ct, kb, sm);
+  if (M > 128 && N > 128) c = std::min(c, cost_pair(pt, kb, pc));
+  int ways = 1;
+  if (g_max_ctas == 0 && g_use_pairs && g_small_tiles && g_splitk != 1 && (g_splitk > 1 || ct * 2 <= sm))
+    for (int s = 2; s <= 8 && s <= kb; s *= 2) {
+      if (g_splitk > 1 ? g_splitk != s : ct * s > sm) continue;
+      const double x = cost_splitk(ct, kb, splitk_clusters(s), s);
+      if (g_splitk == s || x < 0.9 * c) { c = x; ways = s; }
+    }
+  if (best) *best = c;
+  return ways;
+}
+template <bool A_MN, bool B_MN>
+int launch_splitk(const CUtensorMap* tmA, const CUtensorMap* tmB, const SplitKArgs& g, int tiles, int ways, cudaStream_t st) {
+  auto kern = gemm_splitk_kernel<A_MN, B_MN>;
+  static cudaError_t attr = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitKSmem::TOTAL);
+  if (attr != cudaSuccess) return (int)attr;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(tiles * ways);
+  cfg.blockDim = dim3(SPLITK_THREADS);
+  cfg.dynamicSmemBytes = SplitKSmem::TOTAL;
+  cfg.stream = st;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = ways;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = mlb_pdl_enabled() ? 2 : 1;
+  return (int)cudaLaunchKernelEx(&cfg, kern, *tmA, *tmB, g);
+}
 template <bool A_MN, bool B_MN, int EPI>
 int gemm_dispatch_impl(void* out, int ldo, const bf16* A, int lda, const bf16* B, int ldb, int M, int N, int K, cudaStream_t st,
                        const RopeEpi* rope = nullptr, const SwigluEpi* swi = nullptr, const PosEpi* pe = nullptr,
@@ -1044,9 +1251,12 @@ int gemm_dispatch_impl(void* out, int ldo, const bf16* A, int lda, const bf16* B
   if (swi && (g_force_simt || !aligned || get_encode() == nullptr || g_epi_mode != 1 || !g_use_pairs || A_MN || B_MN ||
               EPI != EPI_BF16 || N != 2 * swi->I || swi->I % 128 != 0 || M <= 128 || ((uintptr_t)swi->out & 15)))
     return -7;                                                                       // caller runs the separate kernel
-  if (pe && (g_force_simt || !aligned || get_encode() == nullptr || g_epi_mode != 1 || !g_use_pairs || EPI != EPI_BF16 || M <= 128 ||
-             N <= 128 || N % 8 != 0 || ((uintptr_t)pe->pos & 15) || pe->period < 1))
+  if (pe && (g_force_simt || !aligned || get_encode() == nullptr || g_epi_mode != 1 || !g_use_pairs || EPI != EPI_BF16 || N % 8 != 0 ||
+             ((uintptr_t)pe->pos & 15) || pe->period < 1))
     return -7;
+  const bool plain = EPI == EPI_BF16 && !rope && !swi && !dl && aligned && !g_force_simt && get_encode() != nullptr;
+  const int ways = plain ? splitk_ways(M, N, K, nullptr) : 1;
+  if (pe && ways == 1 && (M <= 128 || N <= 128)) return -7;
   if (dl && (g_force_simt || !aligned || get_encode() == nullptr || g_epi_mode != 1 || !g_use_pairs || A_MN || !B_MN || EPI != EPI_BF16 ||
              M <= 128 || N <= 128 || N != dl->H * 64 || M % dl->T != 0 || ((uintptr_t)dl->o & 15)))
     return -7;                                                                       // caller runs the separate kernels
@@ -1063,21 +1273,23 @@ int gemm_dispatch_impl(void* out, int ldo, const bf16* A, int lda, const bf16* B
   // tile pays ~25 % more per k-block for its operand traffic.
   int BN = (N > 128) ? 256 : 128;
   bool pairs = g_use_pairs && BN == 256 && M > 128;   // 256 x 256 tile shared by a CTA pair
+  const double kbs = ceil_div_i(K, BK), pt = (double)ceil_div_i(M, 256) * ceil_div_i(N, 256), ct = (double)ceil_div_i(M, 128) * ceil_div_i(N, 128);
+  const double pc = pair_clusters(), sm = g_max_ctas > 0 ? g_max_ctas : num_sms();
   if (pairs && !rope && !swi && !pe && !dl && g_small_tiles) {
-    const long kb = ceil_div_i(K, BK);
-    const long pt = (long)ceil_div_i(M, 256) * ceil_div_i(N, 256), ct = (long)ceil_div_i(M, 128) * ceil_div_i(N, 128);
-    const long pc = pair_clusters(), sm = g_max_ctas > 0 ? g_max_ctas : num_sms();
-    double cost_pair, cost_c128;
-    if (EPI == EPI_F32_ADD) {       // both forms split the reduction to fill the machine
-      cost_pair = (double)pt * kb / pc * 512.0 + 4000.0;
-      cost_c128 = (double)ct * kb / sm * 320.0 + 3000.0;
-      if (ct * kb / 8 < sm) cost_c128 = 1e30;      // too little work per CTA even at the smallest split
-    } else {
-      cost_pair = (double)((pt + pc - 1) / pc) * (kb * 512.0 + 2000.0);
-      cost_c128 = (double)((ct + sm - 1) / sm) * (kb * 320.0 + 2000.0);
+    if (EPI == EPI_F32_ADD) {
+      // Both forms split the reduction to fill the machine, and every piece of a tile costs its add-reduces.  Fitted to the times of 1003 ...
+      // 8192 rows at 768 ... 2048 columns: dW of 2304 x 768 over 1003 rows 20.5 us on pairs and 13.3 on 128-wide tiles, of 2048 x 2048 24.6 and
+      // 19.5, of 11008 x 2048 61 and 86.
+      const double units = pt * kbs / pc, pieces = ceil(units / kbs) + 1.0;
+      const double s = std::min(std::max(floor(sm / ct), 1.0), std::max(floor(kbs / 8.0), 1.0)), waves = ceil(ct * s / sm);
+      if (waves * (ceil(kbs / s) * 450.0 + 4000.0) + 4000.0 < 0.95 * (units * 768.0 + pieces * 6000.0 + 6000.0)) { pairs = false; BN = 128; }
+    } else if (cost_c128(ct, kbs, sm) < 0.9 * cost_pair(pt, kbs, pc)) {
+      pairs = false; BN = 128;
     }
-    if (cost_c128 < 0.8 * cost_pair) { pairs = false; BN = 128; }
   }
+  // Few rows: 128-wide tiles, twice as many CTAs at work, unless they come to a wave more than the wide ones save
+  if (BN == 256 && !pairs && M <= 128 && g_small_tiles && ceil(ct / sm) * (kbs * 320.0 + 2000.0) < ceil(ceil_div_i(N, 256) / sm) * (kbs * 560.0 + 2000.0)) BN = 128;
+  if (ways > 1) { pairs = false; BN = 128; }
   if (rope && !(pairs && rope->cols % 64 == 0 && N % 64 == 0)) return -7;
   GemmArgs g;
   g.cosT = rope ? rope->cosT : nullptr; g.sinT = rope ? rope->sinT : nullptr;
@@ -1126,6 +1338,12 @@ int gemm_dispatch_impl(void* out, int ldo, const bf16* A, int lda, const bf16* B
   if (!tmB) tmB = B_MN ? mlb_tmap_cached(B, K, N, ldb, 64, 64) : mlb_tmap_cached(B, N, K, ldb, b_rows, 64);
   const CUtensorMap* tmD = (EPI == EPI_BF16) ? mlb_tmap_cached(out, M, N, ldo, 32, 64, 2) : mlb_tmap_cached(out, M, N, ldo, 32, 32, 4);
   if (!tmA || !tmB || !tmD) return -2;
+  if constexpr (EPI == EPI_BF16) {
+    if (ways > 1) {
+      const SplitKArgs sk{(bf16*)out, g.pos, M, N, ldo, g.tiles_m, g.kb_total, g.pos_period, g.a3d, g.b3d};
+      return launch_splitk<A_MN, B_MN>(tmA, tmB, sk, g.tiles_m * g.tiles_n, ways, st);
+    }
+  }
   if constexpr (!A_MN && !B_MN && EPI == EPI_BF16) {
     if (pairs && pe) return launch_tc2<false, false, EPI_BF16, 1, true>(tmA, tmB, tmD, g, st);
   }
@@ -1472,12 +1690,14 @@ MLB_DEFINE_ERROR_WORD(gemm)
 // of gemm_dispatch_impl, in cycles; the two extra launches ~2.5 us each, their 14 bytes per element at 3400 bytes per cycle).
 MLB_API int mlb_gemm_dw_direct(int N, int K, int M) {
   if (N % 8 != 0 || K % 8 != 0) return 0;
-  const double kb = ceil_div_i(M, BK), pc = pair_clusters(), sm = g_max_ctas > 0 ? g_max_ctas : num_sms();
-  const double pt = (double)ceil_div_i(N, 256) * ceil_div_i(K, 256), ct = (double)ceil_div_i(N, 128) * ceil_div_i(K, 128);
-  const double direct = std::min(ceil(pt / pc) * (kb * 512.0 + 2000.0), ceil(ct / sm) * (kb * 320.0 + 2000.0));
-  const double split = std::max(pt * kb / pc, 8.0) * 512.0 + 4000.0 + 9000.0 + 14.0 * N * K / 3400.0;
+  const double kb = ceil_div_i(M, BK), pc = pair_clusters();
+  const double pt = (double)ceil_div_i(N, 256) * ceil_div_i(K, 256);
+  double direct;
+  splitk_ways(N, K, M, &direct);
+  const double split = std::max(pt * kb / pc, 8.0) * 512.0 + 8000.0 + 9000.0 + 14.0 * N * K / 3400.0;
   return direct <= split ? 1 : 0;
 }
 // The driver's code of the last tensor map it refused (a -2 of the entry points), 0 if none
 MLB_API int mlb_tmap_error(void) { return g_encode_error; }
 MLB_API void mlb_gemm_streamk_whole(int on) { g_sk_whole = on; }
+MLB_API void mlb_gemm_splitk(int ways) { g_splitk = ways; }

@@ -338,6 +338,15 @@ __device__ __forceinline__ uint32_t cluster_id_x() {
   asm volatile("mov.u32 %0, %%clusterid.x;" : "=r"(r));
   return r;
 }
+__device__ __forceinline__ uint32_t cluster_nctarank() {      // CTAs of this cluster
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+// 16 bytes of the shared memory of any CTA of the cluster
+__device__ __forceinline__ void ld_cluster_f32x4(uint32_t cluster_addr, float* x) {
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]) : "r"(cluster_addr) : "memory");
+}
 __device__ __forceinline__ uint32_t cluster_count_x() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%nclusterid.x;" : "=r"(r));

@@ -1338,3 +1338,47 @@ def test_entry_points_through_ctypes_and_through_the_module():
         with pytest.raises(AssertionError):
             e.mlb_linear_fwd(o, x.float(), W, 130, 72, 256, 72, 256, 256)
     assert torch.equal(*outs) and c.mlb_gemm_dw_direct(768, 768, 1003) == m.mlb_gemm_dw_direct(768, 768, 1003)
+
+
+@pytest.mark.parametrize("ways", [2, 4, 8])
+@pytest.mark.parametrize("M,N,K", [(1, 8, 1024), (127, 136, 520), (136, 128, 1000), (304, 264, 2056), (64, 768, 11008)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, False), (True, True)])
+def test_products_whose_reduction_a_cluster_shares(ways, M, N, K, a_mn, b_mn):
+    """Edges of the tile, reductions that the ways do not divide, fewer k-blocks per CTA than stages and more.  fp32 sums and one rounding
+    (2^-9 at most); the order of the sums is fixed, so a second run gives the same bits."""
+    if a_mn and M % 8:
+        pytest.skip("such an operand has no 16-byte rows")
+    torch.manual_seed(M + K)
+    A, B, n = rnd(*((K, M) if a_mn else (M, K))), rnd(*((K, N) if b_mn else (N, K))), nat()
+    e = (A.t() if a_mn else A).double() @ (B if b_mn else B.t()).double()
+    n.lib().mlb_gemm_splitk(ways)
+    try:
+        outs = [torch.full((M, N), float("nan"), device=dev(), dtype=torch.bfloat16) for _ in range(2)]
+        for o in outs:
+            n.gemm(o, A, B, a_mn, b_mn)
+        assert torch.equal(*outs) and _rel(outs[0], e) < 2 ** -8.5
+        if not a_mn and not b_mn:
+            pos, o = rnd(3, N), torch.empty_like(outs[0])
+            assert n.linear_fwd_posembed(o, A, B, pos, 3)
+            assert _rel(o, e + pos.double()[torch.arange(M, device=dev()) % 3]) < 2 ** -8.5
+    finally:
+        n.lib().mlb_gemm_splitk(-1)
+
+
+@pytest.mark.parametrize("rows", [1, 64, 200, 1003])
+@pytest.mark.parametrize("C,I", [(128, 384), (768, 2048), (2048, 5504)])
+def test_products_of_few_rows_by_cost(rows, C, I):
+    """Whatever form the estimate picks for a layer's products at few rows: forward, both gradients, and the add-reduce form into what was there."""
+    torch.manual_seed(rows + C)
+    n = nat()
+    for N, K in ((3 * C, C), (2 * I, C), (C, I)):
+        x, W, dout = rnd(rows, K), rnd(N, K, scale=K ** -0.5), rnd(rows, N)
+        out, dx, dW, acc = rnd(rows, N), rnd(rows, K), rnd(N, K), torch.randn(N, K, device=dev())
+        before = acc.double()
+        n.linear_fwd(out, x, W)
+        n.linear_dx(dx, dout, W)
+        n.linear_dw_cast(dW, dout, x)
+        n.linear_dw(acc, dout, x)
+        ew = dout.double().t() @ x.double()
+        assert _rel(out, x.double() @ W.double().t()) < 2 ** -8.5 and _rel(dx, dout.double() @ W.double()) < 2 ** -8.5
+        assert _rel(dW, ew) < 2 ** -8.5 and _rel(acc, before + ew) < 1e-5
