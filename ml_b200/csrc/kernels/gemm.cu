@@ -400,14 +400,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 //   acc_empty[a] leader only, 8 arrivals: the four epilogue warps of each CTA (the peer's arrive remotely)
 // Persistent: cluster c handles pair-tiles c, c + nclusters, ...; all waits are bounded as in the 1-CTA kernel, and both
 // CTAs meet at a cluster barrier before TMEM is released so neither outlives remote accesses to it.
-template <int EMODE>
 struct Gemm2Smem {
   static constexpr int A_BYTES = 128 * BK * 2;    // this CTA's rows of A
   static constexpr int B_BYTES = 128 * BK * 2;    // this CTA's half of B
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = EMODE == 0 ? 5 : 6;
-  static constexpr int BUFS = EMODE == 0 ? 2 : 1;               // staging buffers per epilogue warp
-  static constexpr int STAGING_BYTES = 8 * BUFS * 4096;
+  static constexpr int STAGES = 6;
+  static constexpr int STAGING_BYTES = 8 * 4096;                // one buffer per epilogue warp
   static constexpr int BAR_BYTES = 256;
   static constexpr int TOTAL = STAGES * STAGE_BYTES + STAGING_BYTES + BAR_BYTES + 1024;
 };
@@ -448,8 +446,12 @@ __device__ __forceinline__ void pack64(const uint32_t (&r)[32], const uint32_t (
 
 // Epilogue: eight warps per CTA; warp w reads TMEM lanes 32*(w%4).. (the lane group the hardware lets it read) and one
 // 128-column half of the accumulator.  A slab of 32 rows x 128 bytes goes through a swizzled staging buffer, then
-//   EMODE 0: TMA tiled store / fp32 add-reduce (two buffers per warp, one transfer in flight)
+//   EMODE 0: TMA tiled store / fp32 add-reduce
 //   EMODE 1: the warp itself writes it out, four full 128-byte rows per instruction (st.global.v4 / red.global.add.v4.f32)
+// bf16 outputs leave by TMA: the load/store unit is then spared a second trip of the tile through shared memory and its stores, which
+// held an epilogue warp ~1000 cycles per slab.  A tile of 16384 x 4096 over 768 takes 6100 cycles (6144 the products alone) where the warps'
+// own stores took 6900, an 8-bit one 4000 where it took 4700.  (With two buffers per warp and a stage less the loads do not keep up: 7300
+// and 4400.)  fp32 add-reduces and the SwiGLU form, whose three outputs per tile are not the accumulator's columns, keep mode 1.
 // Register budget: the ten warps land three on two of the SM's four sub-partitions (16 K registers each).  At 160
 // registers per thread those three warps leave 1 K registers, room for one 32-register warp of a small kernel from
 // another stream (the gradient-bucket kernels that run behind backward use 128-thread CTAs for that reason); at the 168
@@ -465,7 +467,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 const __grid_constant__ CUtensorMap tmD, const GemmArgs g) {
   static_assert(!F8 || (!A_MN && !B_MN && EPI == EPI_BF16), "the 8-bit form is a forward product: K-major operands, bf16 out");
   constexpr int KSTEP = F8 ? 128 : BK;     // elements of K per stage
-  using S = Gemm2Smem<EMODE>;
+  using S = Gemm2Smem;
   constexpr int STAGES = S::STAGES;
   constexpr int BN = 256, PM = 256;    // pair tile
   extern __shared__ uint8_t smem_raw[];
@@ -566,11 +568,11 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   } else {
     // ---------------------------------------------------------------- epilogue (warps 2..9 of each CTA)
     const int lg = warp & 3, half = (warp - 2) >> 2;
-    uint8_t* my_stage = staging + (warp - 2) * (S::BUFS * 4096);
+    uint8_t* my_stage = staging + (warp - 2) * 4096;
     constexpr int SLAB_COLS = (EPI == EPI_BF16) ? 64 : 32;
     constexpr int SLABS = 128 / SLAB_COLS;       // per warp and tile
     constexpr int ELEM = (EPI == EPI_BF16) ? 2 : 4;
-    int it = 0, slab = 0;
+    int it = 0;
     bool ok = true;
     WorkIter<EPI == EPI_F32_ADD> iter(g, cid, ncl);
     WorkItem w;
@@ -615,7 +617,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       }
 #pragma unroll 1
       for (int c = 0; c < SLABS; c++) {
-        uint8_t* buf = my_stage + (EMODE == 0 ? (slab & 1) * 4096 : 0);
+        uint8_t* buf = my_stage;
         uint32_t r[32], r2[32];
         if constexpr (EPI == EPI_BF16 && F8) {      // (as one statement this instance spills four times as much: 153.2 against 151.5 us, mlp_fp8)
           tc::tmem_ld32(taddr + c * SLAB_COLS, r);
@@ -634,7 +636,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         const int col0 = n0 + c * SLAB_COLS;
         if (!rows_live || col0 >= g.N) continue;   // warp-uniform
         if (EMODE == 0) {
-          if (lane == 0) tc::tma_wait_group_read<1>();   // the transfer that last used this buffer has read it
+          if (lane == 0) tc::tma_wait_group_read<0>();   // the transfer that last used the buffer has read it
           __syncwarp();
         }
         uint8_t* rowp = buf + lane * 128;
@@ -736,7 +738,6 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           }
           __syncwarp();   // the buffer is rewritten by the next slab
         }
-        slab++;
       }
     }
     if (EMODE == 0 && lane == 0) tc::tma_wait_group<0>();
@@ -1097,12 +1098,11 @@ int g_use_pairs = 1;         // tuning hook: 0 = always the 1-CTA kernel
 int g_tile_order = 0;        // tuning hook: 0 = by operand size, 1 = M first, 2 = N first
 int g_sk_groups = 1;         // tuning hook: 0 = stream-K without groups (one linear range per cluster)
 int g_streamk = 1;           // tuning hook: weight-gradient products cut into equal k-block ranges per cluster
-int g_epi_mode = 1;          // tuning hook: pair kernel's epilogue, 0 = TMA store / reduce, 1 = coalesced stores by the warps
+int g_epi_mode = -1;         // tuning hook: pair kernel's epilogue, -1 = by form, 0 = TMA store / reduce, 1 = coalesced stores by the warps
 int g_small_tiles = 1;       // tuning hook: 0 = never trade the CTA-pair tile for 128 x 128 tiles on small problems
-template <bool A_MN, bool B_MN, int EPI, int EMODE, bool POS = false, bool DELTA = false>
+template <bool A_MN, bool B_MN, int EPI, int EMODE, bool POS = false, bool DELTA = false, bool F8 = false>
 int launch_tc2(const CUtensorMap* tmA, const CUtensorMap* tmB, const CUtensorMap* tmD, GemmArgs g, cudaStream_t st) {
-  using Gemm2Smem = Gemm2Smem<EMODE>;
-  auto kern = gemm_tc2_kernel<A_MN, B_MN, EPI, EMODE, false, POS, DELTA>;
+  auto kern = gemm_tc2_kernel<A_MN, B_MN, EPI, EMODE, F8, POS, DELTA>;
   static int max_clusters = -1;
   if (max_clusters < 0) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Gemm2Smem::TOTAL);
@@ -1248,16 +1248,16 @@ int gemm_dispatch_impl(void* out, int ldo, const bf16* A, int lda, const bf16* B
   if (B_MN) aligned = aligned && (N % 8 == 0);
   if (!A_MN || !B_MN) aligned = aligned && (K % 8 == 0);
   if (rope && (g_force_simt || !aligned || get_encode() == nullptr)) return -7;   // caller rotates separately
-  if (swi && (g_force_simt || !aligned || get_encode() == nullptr || g_epi_mode != 1 || !g_use_pairs || A_MN || B_MN ||
+  if (swi && (g_force_simt || !aligned || get_encode() == nullptr || g_epi_mode == 0 || !g_use_pairs || A_MN || B_MN ||
               EPI != EPI_BF16 || N != 2 * swi->I || swi->I % 128 != 0 || M <= 128 || ((uintptr_t)swi->out & 15)))
     return -7;                                                                       // caller runs the separate kernel
-  if (pe && (g_force_simt || !aligned || get_encode() == nullptr || g_epi_mode != 1 || !g_use_pairs || EPI != EPI_BF16 || N % 8 != 0 ||
+  if (pe && (g_force_simt || !aligned || get_encode() == nullptr || g_epi_mode == 0 || !g_use_pairs || EPI != EPI_BF16 || N % 8 != 0 ||
              ((uintptr_t)pe->pos & 15) || pe->period < 1))
     return -7;
   const bool plain = EPI == EPI_BF16 && !rope && !swi && !dl && aligned && !g_force_simt && get_encode() != nullptr;
   const int ways = plain ? splitk_ways(M, N, K, nullptr) : 1;
   if (pe && ways == 1 && (M <= 128 || N <= 128)) return -7;
-  if (dl && (g_force_simt || !aligned || get_encode() == nullptr || g_epi_mode != 1 || !g_use_pairs || A_MN || !B_MN || EPI != EPI_BF16 ||
+  if (dl && (g_force_simt || !aligned || get_encode() == nullptr || g_epi_mode == 0 || !g_use_pairs || A_MN || !B_MN || EPI != EPI_BF16 ||
              M <= 128 || N <= 128 || N != dl->H * 64 || M % dl->T != 0 || ((uintptr_t)dl->o & 15)))
     return -7;                                                                       // caller runs the separate kernels
   if (g_force_simt || !aligned || get_encode() == nullptr) {
@@ -1345,12 +1345,12 @@ int gemm_dispatch_impl(void* out, int ldo, const bf16* A, int lda, const bf16* B
     }
   }
   if constexpr (!A_MN && !B_MN && EPI == EPI_BF16) {
-    if (pairs && pe) return launch_tc2<false, false, EPI_BF16, 1, true>(tmA, tmB, tmD, g, st);
+    if (pairs && pe) return launch_tc2<false, false, EPI_BF16, 0, true>(tmA, tmB, tmD, g, st);
   }
   if constexpr (!A_MN && B_MN && EPI == EPI_BF16) {
-    if (dl) return pairs ? launch_tc2<false, true, EPI_BF16, 1, false, true>(tmA, tmB, tmD, g, st) : -7;
+    if (dl) return pairs ? launch_tc2<false, true, EPI_BF16, 0, false, true>(tmA, tmB, tmD, g, st) : -7;
   }
-  if (pairs && g_epi_mode == 0) return launch_tc2<A_MN, B_MN, EPI, 0>(tmA, tmB, tmD, g, st);
+  if (pairs && (g_epi_mode == 0 || (g_epi_mode < 0 && EPI == EPI_BF16 && !swi))) return launch_tc2<A_MN, B_MN, EPI, 0>(tmA, tmB, tmD, g, st);
   if (pairs) return launch_tc2<A_MN, B_MN, EPI, 1>(tmA, tmB, tmD, g, st);
   if (BN == 256) return launch_tc<256, A_MN, B_MN, EPI>(tmA, tmB, tmD, g, st);
   return launch_tc<128, A_MN, B_MN, EPI>(tmA, tmB, tmD, g, st);
@@ -1399,7 +1399,7 @@ int gemm_dispatch(void* out, int ldo, const bf16* A, int lda, const bf16* B, int
       if (cudaMalloc(&scratch, (size_t)M * ldo * sizeof(float)) != cudaSuccess) { cudaGetLastError(); scratch = nullptr; }
       tune_out = scratch;
     }
-    plan = GemmPlan{1, 0, 1, 1, 1, 0.f};       // the static heuristics
+    plan = GemmPlan{1, 0, -1, 1, 1, 0.f};      // the static heuristics
     if (tune_out != nullptr) {
       cudaEvent_t e0, e1;
       cudaEventCreate(&e0);
@@ -1408,7 +1408,7 @@ int gemm_dispatch(void* out, int ldo, const bf16* A, int lda, const bf16* B, int
       const bool fixed_epi = rope || swi || pe;      // these epilogues exist in one form only
       for (int tile = 0; tile < (fixed_epi ? 1 : 3); tile++)
         for (int order = 1; order <= 2; order++)
-          for (int epi = fixed_epi ? 1 : 0; epi < 2; epi++)
+          for (int epi = fixed_epi ? -1 : 0; epi < (fixed_epi ? 0 : 2); epi++)
             for (int sk = (EPI == EPI_F32_ADD) ? 0 : 1; sk < 2; sk++)
               for (int skg = (EPI == EPI_F32_ADD && sk) ? 0 : 1; skg < 2; skg++) {
                 GemmPlan c{fixed_epi ? 1 : tile, order, epi, sk, skg, 0.f};
@@ -1440,7 +1440,7 @@ int gemm_fp8_dispatch(void* out, int ldo, const uint8_t* A, int lda, const uint8
                       cudaStream_t st, const SwigluEpi* swi, const RopeEpi* rope = nullptr) {
   const bool ok = ((uintptr_t)A % 16 == 0) && ((uintptr_t)B % 16 == 0) && (lda % 16 == 0) && (ldb % 16 == 0) && ((uintptr_t)out % 16 == 0) &&
                   (ldo % 8 == 0) && (N % 8 == 0) && (K % 16 == 0) && M > 128 && N > 128 && K > 0 && get_encode() != nullptr &&
-                  g_use_pairs && g_epi_mode == 1 && !g_force_simt;
+                  g_use_pairs && g_epi_mode != 0 && !g_force_simt;
   if (!ok) return -7;
   if (swi && (N != 2 * swi->I || swi->I % 128 != 0 || ((uintptr_t)swi->out & 15))) return -7;
   if (rope && !(rope->cols % 64 == 0 && N % 64 == 0)) return -7;
@@ -1460,26 +1460,8 @@ int gemm_fp8_dispatch(void* out, int ldo, const uint8_t* A, int lda, const uint8
   const CUtensorMap* tmB = mlb_tmap_cached(B, N, K, ldb, 128, 128, 1);
   const CUtensorMap* tmD = mlb_tmap_cached(out, M, N, ldo, 32, 64, 2);
   if (!tmA || !tmB || !tmD) return -2;
-  using Smem = Gemm2Smem<1>;
-  auto kern = gemm_tc2_kernel<false, false, EPI_BF16, 1, true>;
-  static int max_clusters = -1;
-  if (max_clusters < 0) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem::TOTAL);
-    if (e != cudaSuccess) return (int)e;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(num_sms() & ~1);
-    cfg.blockDim = dim3(GEMM2_THREADS);
-    cfg.dynamicSmemBytes = Smem::TOTAL;
-    int n = 0;
-    e = cudaOccupancyMaxActiveClusters(&n, kern, &cfg);
-    if (e != cudaSuccess || n <= 0) { cudaGetLastError(); n = num_sms() / 2; }
-    max_clusters = n < num_sms() / 2 ? n : num_sms() / 2;
-  }
-  int total = g.tiles_m * g.tiles_n;
-  int cap = max_clusters;
-  if (g_max_ctas > 0 && g_max_ctas / 2 < cap) cap = g_max_ctas / 2 > 0 ? g_max_ctas / 2 : 1;
-  int clusters = total < cap ? total : cap;
-  return (int)mlb_launch_tmem(kern, dim3(2 * clusters), dim3(GEMM2_THREADS), Smem::TOTAL, st, *tmA, *tmB, *tmD, g);
+  if (swi) return launch_tc2<false, false, EPI_BF16, 1, false, false, true>(tmA, tmB, tmD, g, st);
+  return launch_tc2<false, false, EPI_BF16, 0, false, false, true>(tmA, tmB, tmD, g, st);
 }
 
 }  // namespace
@@ -1675,11 +1657,12 @@ MLB_API int mlb_gemm_plan_get(int i, int* out10) {
   auto it = g_plans.begin();
   std::advance(it, i);
   out10[0] = it->first[0]; out10[1] = it->first[1]; out10[2] = it->first[2]; out10[3] = it->first[3];
-  out10[4] = it->second.tile; out10[5] = it->second.order; out10[6] = it->second.epi; out10[7] = it->second.streamk;
+  out10[4] = it->second.tile; out10[5] = it->second.order; out10[6] = it->second.epi >= 0 ? it->second.epi : (it->first[0] & 1) || (it->first[4] & 2) ? 1 : 0; out10[7] = it->second.streamk;
   out10[8] = it->second.skg; out10[9] = (int)it->second.us;
   return 0;
 }
-MLB_API void mlb_gemm_epilogue_mode(int m) { g_epi_mode = m; }
+// 1: each form's own epilogue, 0: TMA everywhere, 2: the warps' stores everywhere
+MLB_API void mlb_gemm_epilogue_mode(int m) { g_epi_mode = m == 0 ? 0 : m == 2 ? 1 : -1; }
 MLB_API void mlb_gemm_small_tiles(int on) { g_small_tiles = on; }
 MLB_API void mlb_gemm_streamk(int on) { g_streamk = on; }
 MLB_API void mlb_gemm_tile_order(int mode) { g_tile_order = mode; }
