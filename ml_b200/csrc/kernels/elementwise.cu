@@ -207,13 +207,50 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_k(bf16* __restrict__ out, flo
 
 // ------------------------------------------------------------------ LayerNorm (the prototype's norm: csrc/kernels/layer_norm_kernel.cu:12-87)
 // y = (x - mean) * rstd * w + b over the last dimension; one warp per row, statistics in fp32, mean / rstd saved for backward.
+// NV > 0: C = NV * 256, the row (and the slices of w and b) fetched once, 16 bytes a load, and kept in registers; else any C, element by element.
+template <int NV>
 __global__ void __launch_bounds__(256) layernorm_fwd_k(bf16* __restrict__ out, float* __restrict__ mean, float* __restrict__ rstd,
                                                        const bf16* __restrict__ x, const bf16* __restrict__ w, const bf16* __restrict__ b,
                                                        long rows, int C, float eps) {
+  mlb_pdl_sync();
   const int lane = threadIdx.x & 31;
   const long row = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
   const bf16* px = x + row * C;
+  if constexpr (NV > 0) {
+    uint4 rx[NV], rw[NV], rb[NV];
+#pragma unroll
+    for (int v = 0; v < NV; v++) {
+      const int i = (v * 32 + lane) * 8;
+      rx[v] = *reinterpret_cast<const uint4*>(px + i);
+      rw[v] = __ldg(reinterpret_cast<const uint4*>(w + i));
+      rb[v] = b ? __ldg(reinterpret_cast<const uint4*>(b + i)) : make_uint4(0, 0, 0, 0);
+    }
+    float f[NV][8], s = 0.f, ss = 0.f;
+#pragma unroll
+    for (int v = 0; v < NV; v++) {
+      unpack8(rx[v], f[v]);
+#pragma unroll
+      for (int j = 0; j < 8; j++) s += f[v][j];
+    }
+    const float mu = warp_sum(s) / (float)C;
+#pragma unroll
+    for (int v = 0; v < NV; v++)
+#pragma unroll
+      for (int j = 0; j < 8; j++) { const float d = f[v][j] - mu; ss += d * d; }
+    const float r = rsqrtf(warp_sum(ss) / (float)C + eps);
+    if (lane == 0) { mean[row] = mu; rstd[row] = r; }
+#pragma unroll
+    for (int v = 0; v < NV; v++) {
+      float ww[8], bb[8];
+      unpack8(rw[v], ww);
+      unpack8(rb[v], bb);
+#pragma unroll
+      for (int j = 0; j < 8; j++) f[v][j] = (f[v][j] - mu) * r * ww[j] + bb[j];
+      store8(out + row * C + (v * 32 + lane) * 8, f[v]);
+    }
+    return;
+  }
   float s = 0.f;
   for (int i = lane; i < C; i += 32) s += __bfloat162float(px[i]);
   const float mu = warp_sum(s) / (float)C;
@@ -270,7 +307,9 @@ __global__ void __launch_bounds__(256) layernorm_bwd_k(bf16* __restrict__ dx, fl
 // by whichever blocks finish last (see the end of the kernel).  Scratch: `partial` = (gridDim.x + RMS_GROUPS) * C
 // floats, `ticket` = 1 + RMS_GROUPS ints that are 0 on entry and left 0 on exit.
 constexpr int RMS_GROUPS = 16;
-template <int VPL>  // VPL = C / 256 (vectors of 8 per lane) up to 3; 0 = generic C (scalar path)
+// Up to 32 blocks (256 rows) there is one group, and its last block adds the partial rows up with all of its threads.
+// VPL = C / 256 (vectors of 8 per lane) up to 3; PART: one vector per lane of rows narrower than 256 (C % 8 == 0); 0 = generic C (scalar path).
+template <int VPL, bool PART = false>
 __global__ void __launch_bounds__(256, 2) rmsnorm_bwd_k(bf16* __restrict__ dx, float* __restrict__ dw, const bf16* __restrict__ dy,
                                                      const bf16* __restrict__ x, const bf16* __restrict__ w,
                                                      const float* __restrict__ rstd, const bf16* __restrict__ add, long rows,
@@ -287,10 +326,11 @@ __global__ void __launch_bounds__(256, 2) rmsnorm_bwd_k(bf16* __restrict__ dx, f
     constexpr bool CACHE_W = NV <= 2;  // the weight vector stays in registers (two resident blocks per SM leave 128 per thread)
     constexpr int NW = CACHE_W ? NV : 1;
     float acc[NV][8];
-    float ww[NW][8];
+    float ww[NW][8] = {};
+    const bool mine = !PART || lane * 8 < C;      // this lane has columns
 #pragma unroll
     for (int v = 0; v < NV; v++) {
-      if (CACHE_W) load8(w + (v * 32 + lane) * 8, ww[v]);
+      if (CACHE_W && mine) load8(w + (v * 32 + lane) * 8, ww[v]);
 #pragma unroll
       for (int j = 0; j < 8; j++) acc[v][j] = 0.f;
     }
@@ -305,9 +345,9 @@ __global__ void __launch_bounds__(256, 2) rmsnorm_bwd_k(bf16* __restrict__ dx, f
       for (int v = 0; v < NV; v++) {
         const long off = row * C + (v * 32 + lane) * 8;
         const int cw = CACHE_W ? v : 0;
-        xr[v] = *reinterpret_cast<const uint4*>(x + off);
-        dr[v] = *reinterpret_cast<const uint4*>(dy + off);
-        ar[v] = add ? *reinterpret_cast<const uint4*>(add + off) : make_uint4(0, 0, 0, 0);
+        xr[v] = mine ? *reinterpret_cast<const uint4*>(x + off) : make_uint4(0, 0, 0, 0);
+        dr[v] = mine ? *reinterpret_cast<const uint4*>(dy + off) : make_uint4(0, 0, 0, 0);
+        ar[v] = add && mine ? *reinterpret_cast<const uint4*>(add + off) : make_uint4(0, 0, 0, 0);
         if (!CACHE_W) load8(w + (v * 32 + lane) * 8, ww[0]);
         float xf[8], df[8];
         unpack8(xr[v], xf);
@@ -331,12 +371,12 @@ __global__ void __launch_bounds__(256, 2) rmsnorm_bwd_k(bf16* __restrict__ dx, f
           o[j] += df[j] * ww[cw][j] * r - xf[j] * k;
           acc[v][j] += df[j] * xf[j] * r;
         }
-        store8(dx + off, o);
+        if (mine) store8(dx + off, o);
       }
     }
     // fold the 8 warps' register partials in warp order (deterministic)
     for (int wv = 0; wv < nwarp; wv++) {
-      if (warp == wv) {
+      if (warp == wv && mine) {
 #pragma unroll
         for (int v = 0; v < NV; v++)
 #pragma unroll
@@ -367,7 +407,7 @@ __global__ void __launch_bounds__(256, 2) rmsnorm_bwd_k(bf16* __restrict__ dx, f
   // its group sums the group's partial rows in index order into gpartial[group]; the block that completes the last
   // group sums the group rows in order into dw.  Who does the summing depends on timing, the summation order does not.
   const int nb = (int)gridDim.x;
-  const int gsz = (nb + RMS_GROUPS - 1) / RMS_GROUPS;
+  const int gsz = nb <= 32 ? nb : (nb + RMS_GROUPS - 1) / RMS_GROUPS;
   const int grp = blockIdx.x / gsz;
   const int g_lo = grp * gsz, g_hi = min(nb, g_lo + gsz);
   const int ngroups = (nb + gsz - 1) / gsz;
@@ -378,6 +418,28 @@ __global__ void __launch_bounds__(256, 2) rmsnorm_bwd_k(bf16* __restrict__ dx, f
   __syncthreads();
   if (!is_last) return;
   __threadfence();
+  if (PART && nb <= 32) {
+    // slice q of the threads takes rows q, q + slices, ...; the slices are added in order (C < 256: at least four of them, at most 1024 floats)
+    const int vecs = C >> 2, slices = (int)blockDim.x / vecs, q = threadIdx.x / vecs, c = threadIdx.x % vecs * 4;
+    if (q < slices) {
+      float a[4] = {};
+#pragma unroll 8
+      for (int b = q; b < nb; b += slices) {
+        const float4 p = __ldcg(reinterpret_cast<const float4*>(&partial[(long)b * C + c]));
+        a[0] += p.x; a[1] += p.y; a[2] += p.z; a[3] += p.w;
+      }
+#pragma unroll
+      for (int j = 0; j < 4; j++) sh[q * C + c + j] = a[j];
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < C; i += blockDim.x) {
+      float t = 0.f;
+      for (int g = 0; g < slices; g++) t += sh[g * C + i];
+      dw[i] += t;
+    }
+    if (threadIdx.x == 0) ticket[1] = 0;
+    return;
+  }
   const bool vec4 = ((C & 3) == 0) && ((reinterpret_cast<uintptr_t>(dw) & 15) == 0) && ((reinterpret_cast<uintptr_t>(partial) & 15) == 0);
   for (int c = threadIdx.x * 4; c < C; c += blockDim.x * 4) {
     if (vec4) {
@@ -563,25 +625,27 @@ __global__ void __launch_bounds__(256) colsum_k(float* __restrict__ partial, con
   partial[(size_t)blockIdx.y * N + col] = s;
 }
 // The partial rows added up in a fixed order: columns [0, C) to dw, [C, W) to db (either may be null).  bf16: rounded and stored;
-// fp32: added to what is there.  A block takes 32 columns, 8 row slices.
+// fp32: added to what is there.  A block takes 32 columns, 32 row slices: the few hundred partial rows are ten loads or less
+// per thread, all in flight together (with 8 slices they came in five trips).
+constexpr int FOLD_THREADS = 1024;
 template <bool BF>
-__global__ void __launch_bounds__(256) fold_cols_k(void* __restrict__ dw, void* __restrict__ db, const float* __restrict__ partial, int nrows, int C, int W) {
+__global__ void __launch_bounds__(FOLD_THREADS) fold_cols_k(void* __restrict__ dw, void* __restrict__ db, const float* __restrict__ partial, int nrows, int C, int W) {
   mlb_pdl_sync();
-  __shared__ float red[8][32];
+  __shared__ float red[32][33];
   const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
   float s = 0.f;
   if (c < W) {
-#pragma unroll 8
-    for (int r = sl; r < nrows; r += 8) s += partial[(size_t)r * W + c];
+#pragma unroll 10
+    for (int r = sl; r < nrows; r += 32) s += partial[(size_t)r * W + c];
   }
   red[sl][lane] = s;
   __syncthreads();
-  if (sl != 0 || c >= W) return;
-#pragma unroll
-  for (int i = 1; i < 8; i++) s += red[i][lane];
-  void* dst = c < C ? dw : db;
+  s = warp_sum(red[lane][sl]);      // a warp per column
+  const int col = blockIdx.x * 32 + sl;
+  if (lane != 0 || col >= W) return;
+  void* dst = col < C ? dw : db;
   if (dst == nullptr) return;
-  const int i = c < C ? c : c - C;
+  const int i = col < C ? col : col - C;
   if (BF) ((bf16*)dst)[i] = __float2bfloat16(s);
   else ((float*)dst)[i] += s;
 }
@@ -1358,7 +1422,20 @@ MLB_API int mlb_adamw_fp8(float* master, void* params, void* params8, const floa
 
 MLB_API int mlb_layernorm_fwd(void* out, float* mean, float* rstd, const void* x, const void* w, const void* b, long rows, int C, float eps,
                               cudaStream_t st) {
-  layernorm_fwd_k<<<gs(rows, 8), 256, 0, st>>>((bf16*)out, mean, rstd, (const bf16*)x, (const bf16*)w, (const bf16*)b, rows, C, eps);
+  const bool vec = C % 256 == 0 && C <= 2048 && (((uintptr_t)out | (uintptr_t)x | (uintptr_t)w | (uintptr_t)b) & 15) == 0;
+#define LN(NV) \
+  mlb_launch(layernorm_fwd_k<NV>, dim3(gs(rows, 8)), dim3(256), 0, st, (bf16*)out, mean, rstd, (const bf16*)x, (const bf16*)w, (const bf16*)b, rows, C, eps)
+  switch (vec ? C / 256 : 0) {
+    case 1: LN(1); break;
+    case 2: LN(2); break;
+    case 3: LN(3); break;
+    case 4: LN(4); break;
+    case 5: LN(5); break;
+    case 6: LN(6); break;
+    case 8: LN(8); break;
+    default: LN(0); break;
+  }
+#undef LN
   LAUNCH_RET;
 }
 // dw / db (fp32, db may be NULL) are accumulated into; C * 8 bytes of shared memory must fit the default 48 KB.
@@ -1394,8 +1471,8 @@ static void norm_rows_launch(void* dx, void* dw, void* db, bool bf, const void* 
   const int blocks = mlb_rmsnorm_bwd_blocks(rows), gt = C / 8, W = LN ? 2 * C : C;
   mlb_launch(norm_bwd_rows_k<LN>, dim3(blocks), dim3(256 / gt * gt), 0, st, (bf16*)dx, (const bf16*)dy, (const bf16*)x, (const bf16*)w, mean, rstd,
              (const bf16*)add, rows, C, partial);
-  if (bf) mlb_launch(fold_cols_k<true>, dim3((W + 31) / 32), dim3(256), 0, st, dw, db, (const float*)partial, blocks, C, W);
-  else mlb_launch(fold_cols_k<false>, dim3((W + 31) / 32), dim3(256), 0, st, dw, db, (const float*)partial, blocks, C, W);
+  if (bf) mlb_launch(fold_cols_k<true>, dim3((W + 31) / 32), dim3(FOLD_THREADS), 0, st, dw, db, (const float*)partial, blocks, C, W);
+  else mlb_launch(fold_cols_k<false>, dim3((W + 31) / 32), dim3(FOLD_THREADS), 0, st, dw, db, (const float*)partial, blocks, C, W);
 }
 MLB_API int mlb_rmsnorm_bwd_cast(void* dx, void* dw, const void* dy, const void* x, const void* w, const float* rstd, const void* add, long rows, int C,
                                  float* partial, cudaStream_t st) {
@@ -1419,21 +1496,23 @@ MLB_API int mlb_colsum(void* out, const void* x, long M, int N, float* partial, 
   if (M <= 0 || N <= 0 || N % 8 != 0 || ((uintptr_t)x & 15)) return -7;
   const int S = mlb_colsum_splits(M, N);
   mlb_launch(colsum_k, dim3((N + 255) / 256, S), dim3(256), 0, st, partial, (const bf16*)x, M, N);
-  mlb_launch(fold_cols_k<true>, dim3((N + 31) / 32), dim3(256), 0, st, out, (void*)nullptr, (const float*)partial, S, N, N);
+  mlb_launch(fold_cols_k<true>, dim3((N + 31) / 32), dim3(FOLD_THREADS), 0, st, out, (void*)nullptr, (const float*)partial, S, N, N);
   LAUNCH_RET;
 }
 MLB_API int mlb_rmsnorm_bwd(void* dx, float* dw, const void* dy, const void* x, const void* w, const float* rstd, const void* add,
                             long rows, int C, float* partial, int* ticket, cudaStream_t st) {
   const int blocks = mlb_rmsnorm_bwd_blocks(rows);
-  const size_t sh = (size_t)C * sizeof(float);
-#define RB(V)                                                                                                         \
-  mlb_launch(rmsnorm_bwd_k<V>, dim3(blocks), dim3(256), sh, st, (bf16*)dx, dw, (const bf16*)dy, (const bf16*)x, (const bf16*)w, rstd,   \
+  const size_t sh = (size_t)std::max(C, 1024) * sizeof(float);
+#define RB(...)                                                                                                         \
+  mlb_launch(rmsnorm_bwd_k<__VA_ARGS__>, dim3(blocks), dim3(256), sh, st, (bf16*)dx, dw, (const bf16*)dy, (const bf16*)x, (const bf16*)w, rstd,   \
                                             (const bf16*)add, rows, C, partial, ticket)
   if (sh > 48 * 1024) return -3;
   if (C >= 1024 && norm_rows_ok(dx, dy, x, w, add, rows, C)) {      // (narrower rows fit a warp's registers, and one launch)
     norm_rows_launch<false>(dx, dw, nullptr, false, dy, x, w, nullptr, rstd, add, rows, C, partial, st);
     LAUNCH_RET;
   }
+  const bool narrow = C < 256 && C % 8 == 0 && (((uintptr_t)dx | (uintptr_t)dy | (uintptr_t)x | (uintptr_t)w | (uintptr_t)add | (uintptr_t)partial) & 15) == 0;
+  if (narrow) { RB(1, true); LAUNCH_RET; }
   switch ((C % 256 == 0) ? C / 256 : 0) {
     case 1: RB(1); break;
     case 2: RB(2); break;

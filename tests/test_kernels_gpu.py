@@ -1382,3 +1382,42 @@ def test_products_of_few_rows_by_cost(rows, C, I):
         ew = dout.double().t() @ x.double()
         assert _rel(out, x.double() @ W.double().t()) < 2 ** -8.5 and _rel(dx, dout.double() @ W.double()) < 2 ** -8.5
         assert _rel(dW, ew) < 2 ** -8.5 and _rel(acc, before + ew) < 1e-5
+
+
+@pytest.mark.parametrize("rows,C", [(1, 8), (3, 128), (256, 128), (257, 128), (300, 248), (2500, 64), (40, 256), (33, 768), (9, 264)])
+@pytest.mark.parametrize("add", [False, True])
+def test_rmsnorm_backward_of_few_or_narrow_rows(rows, C, add):
+    """One partial row per block up to 32 blocks and their sum by the last one, rows narrower than a warp's vectors, and the two-level sum beyond: dx to one
+    rounding (2^-9), dw in fp32 added to what was there, the same on a second run."""
+    torch.manual_seed(rows + C)
+    n = nat()
+    x, dy, w, a = rnd(rows, C), rnd(rows, C), 1 + rnd(1, C, scale=0.1).view(-1), rnd(rows, C) if add else None
+    out, rstd = torch.empty_like(x), torch.empty(rows, device=dev())
+    n.rmsnorm_fwd(out, rstd, x, w, 1e-5)
+    dw0 = torch.randn(C, device=dev())
+    runs = []
+    for _ in range(2):
+        dx, dw = torch.empty_like(x), dw0.clone()
+        n.rmsnorm_bwd(dx, dw, dy, x, w, rstd, a)
+        runs.append((dx, dw))
+    xd, wd = x.double().requires_grad_(True), w.double().requires_grad_(True)
+    e = xd * torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + 1e-5) * wd
+    gx, gw = torch.autograd.grad(e, [xd, wd], dy.double())
+    assert _rel(runs[0][0], gx + (a.double() if add else 0)) < 2 ** -8 and _rel(runs[0][1], dw0.double() + gw) < 1e-5
+    if C % 256 == 0 or C < 256:      # (other widths add up in shared memory as it comes)
+        assert torch.equal(runs[0][0], runs[1][0]) and torch.equal(runs[0][1], runs[1][1])
+
+
+@pytest.mark.parametrize("rows", [1, 7, 300])
+@pytest.mark.parametrize("C", [256, 512, 768, 1024, 1280, 1536, 1792, 2048, 264, 40])
+@pytest.mark.parametrize("bias", [False, True])
+def test_layernorm_forward_widths(rows, C, bias):
+    """Every width that stays in registers and two that do not, rows that do not fill a block: one rounding (2^-9), statistics in fp32."""
+    torch.manual_seed(rows + C)
+    x, w, b = rnd(rows, C) + 2, 1 + rnd(1, C, scale=0.1).view(-1), rnd(1, C).view(-1) if bias else None
+    out, mean, rstd = torch.empty_like(x), torch.empty(rows, device=dev()), torch.empty(rows, device=dev())
+    nat().layernorm_fwd(out, mean, rstd, x, w, b, 1e-5)
+    xd = x.double()
+    e = torch.nn.functional.layer_norm(xd, (C,), w.double(), b.double() if bias else None, 1e-5)
+    assert _rel(out, e) < 2 ** -8.5 and _rel(mean, xd.mean(-1)) < 1e-5
+    assert _rel(rstd, torch.rsqrt(xd.var(-1, unbiased=False) + 1e-5)) < 1e-5
