@@ -50,21 +50,25 @@ __device__ __forceinline__ void mlb_pdl_sync() {
 #ifdef __CUDACC__
 #include <cstdlib>
 #include <utility>
-// MLB_PDL: 0 (default) no kernel starts early; 1 every kernel launched through mlb_launch / mlb_launch_tmem may (measured
-// slower inside a captured step, 20.6 vs 19.8 ms: a kernel that allocates tensor memory or most of an SM's shared memory
-// cannot become resident next to its predecessor anyway, and one that does delays it); 2 only the kernels launched
-// through mlb_launch - the element-wise ones, whose CTAs fit beside a tensor-core kernel's (also measured slower in the
-// captured step: 18.1-18.5 against 17.75 ms, the early-resident CTAs take issue slots and registers from the kernel
-// they wait for).
+// Which kernels start early, without MLB_PDL: all GEMMs, attention kernels of one wave, and element-wise kernels of one wave (at most as many
+// threads as the machine holds).  A chain of small kernels is bound by launch and set-up, which then run under the kernel before: step of
+// the 4-layer / 128-wide decoder 637 -> 567 us, attention forward of a few thousand tokens 13.3 -> 10.4; GEMMs of any size gain 2 to 3 us of
+// launch gap each (step of the 12-layer decoder 17.35 -> 17.11 ms, captured 16.40 -> 16.29).
+// Larger ones stay out: their CTAs sit on the SMs while the kernel before still works there, and take registers and issue slots from
+// it (every kernel early: attention at 16 x 1024 tokens 269 -> 283 us).
+// A kernel that allocates tensor memory before its mlb_pdl_sync() may hold it while the kernel before has CTAs that are still to allocate only
+// if both fit an SM; those that allocate after it (attention at head sizes 64 and 128) have more than 200 KB of shared memory and fit beside none.
+// MLB_PDL=0: none; 1: all; 2: all element-wise ones.
+enum { MLB_PDL_NONE = 0, MLB_PDL_ALL = 1, MLB_PDL_ELEMENTWISE = 2, MLB_PDL_BY_SIZE = 3 };
 inline int mlb_pdl_mode() {
   static int mode = -1;
   if (mode < 0) {
     const char* e = getenv("MLB_PDL");
-    mode = (e != nullptr && (e[0] == '1' || e[0] == '2')) ? e[0] - '0' : 0;
+    mode = (e != nullptr && e[0] >= '0' && e[0] <= '2') ? e[0] - '0' : MLB_PDL_BY_SIZE;
   }
   return mode;
 }
-inline bool mlb_pdl_enabled() { return mlb_pdl_mode() == 1; }
+constexpr long MLB_WAVE_THREADS = 148L * 2048;
 template <typename... KArgs, typename... Args>
 inline cudaError_t mlb_launch_attr(bool early, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
@@ -81,12 +85,15 @@ inline cudaError_t mlb_launch_attr(bool early, void (*kern)(KArgs...), dim3 grid
 }
 template <typename... KArgs, typename... Args>
 inline cudaError_t mlb_launch(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
-  return mlb_launch_attr(mlb_pdl_mode() != 0, kern, grid, block, smem, st, std::forward<Args>(args)...);
+  const int mode = mlb_pdl_mode();
+  const bool early = mode == MLB_PDL_BY_SIZE ? (long)grid.x * grid.y * grid.z * block.x <= MLB_WAVE_THREADS : mode != MLB_PDL_NONE;
+  return mlb_launch_attr(early, kern, grid, block, smem, st, std::forward<Args>(args)...);
 }
-// for kernels that allocate tensor memory (GEMMs, attention): they start early only in mode 1
+// for kernels that allocate tensor memory (GEMMs, attention): `small`, of those that start early by size
+inline bool mlb_pdl_tmem(bool small) { return mlb_pdl_mode() == MLB_PDL_ALL || (mlb_pdl_mode() == MLB_PDL_BY_SIZE && small); }
 template <typename... KArgs, typename... Args>
-inline cudaError_t mlb_launch_tmem(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
-  return mlb_launch_attr(mlb_pdl_mode() == 1, kern, grid, block, smem, st, std::forward<Args>(args)...);
+inline cudaError_t mlb_launch_tmem(bool small, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+  return mlb_launch_attr(mlb_pdl_tmem(small), kern, grid, block, smem, st, std::forward<Args>(args)...);
 }
 #endif
 

@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
   uint64_t *bar_q = bars, *bar_k = bars + 1 /*[2]*/, *bar_v = bars + 3 /*[2]*/, *bar_s = bars + 5, *bar_o = bars + 6, *bar_end = bars + 7;
   uint32_t* tmem_slot = (uint32_t*)(bars + 8);
   volatile int* s_abort = (volatile int*)(bars + 9);
-  if (attn_given_up()) return;
+  if (attn_given_up()) { mlb_pdl_sync(); return; }      // (nobody behind this kernel starts before the one in front of it has ended)
 
   const int ntile = (a.T + 127) / 128;
   const int qt = ntile - 1 - (int)blockIdx.x, h = blockIdx.y, b = blockIdx.z;     // (causal: longest rows first)
@@ -379,7 +379,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
   uint32_t* tmem_slot = (uint32_t*)(bars + 6);
   volatile int* s_abort = (volatile int*)(bars + 7);
   float* stat = (float*)(smem + S::STAT);
-  if (attn_given_up()) return;
+  if (attn_given_up()) { mlb_pdl_sync(); return; }      // (nobody behind this kernel starts before the one in front of it has ended)
 
   const int tid = threadIdx.x, warp = tid >> 5;
   const int ntile = (a.T + 127) / 128;
@@ -552,11 +552,13 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
   if (again.x | again.y | again.z | again.w) split_redo<KV ? 1 : 2>(again, a, r0, h, b, (float*)smem);
 }
 
+// (small enough to start under the kernel before; two to four CTAs fit an SM)
+static bool split_wave(const SplitArgs& a) { return (long)((a.T + 127) / 128) * a.H * a.B <= 8 * 148; }
 template <int HDT>
 static int split_fwd_launch(const CUtensorMap* tm, const SplitArgs& a, cudaStream_t st) {
   static int once = (int)cudaFuncSetAttribute(attn_split_fwd_k<HDT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitFwdSmem<HDT>::TOTAL);
   if (once) return once;
-  mlb_launch_tmem(attn_split_fwd_k<HDT>, dim3((a.T + 127) / 128, a.H, a.B), dim3(SPLIT_THREADS), SplitFwdSmem<HDT>::TOTAL, st, *tm, a);
+  mlb_launch_tmem(split_wave(a), attn_split_fwd_k<HDT>, dim3((a.T + 127) / 128, a.H, a.B), dim3(SPLIT_THREADS), SplitFwdSmem<HDT>::TOTAL, st, *tm, a);
   return (int)cudaGetLastError();
 }
 template <int HDT>
@@ -565,8 +567,8 @@ static int split_bwd_launch(const CUtensorMap* tm, const CUtensorMap* td, const 
                     (int)cudaFuncSetAttribute(attn_split_bwd_k<HDT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitBwdSmem<HDT, false>::TOTAL);
   if (once) return once;
   const dim3 grid((a.T + 127) / 128, a.H, a.B);
-  mlb_launch_tmem(attn_split_bwd_k<HDT, true>, grid, dim3(SPLIT_THREADS), SplitBwdSmem<HDT, true>::TOTAL, st, *tm, *td, a);
-  mlb_launch_tmem(attn_split_bwd_k<HDT, false>, grid, dim3(SPLIT_THREADS), SplitBwdSmem<HDT, false>::TOTAL, st, *tm, *td, a);
+  mlb_launch_tmem(split_wave(a), attn_split_bwd_k<HDT, true>, grid, dim3(SPLIT_THREADS), SplitBwdSmem<HDT, true>::TOTAL, st, *tm, *td, a);
+  mlb_launch_tmem(split_wave(a), attn_split_bwd_k<HDT, false>, grid, dim3(SPLIT_THREADS), SplitBwdSmem<HDT, false>::TOTAL, st, *tm, *td, a);
   return (int)cudaGetLastError();
 }
 

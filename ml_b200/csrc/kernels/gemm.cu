@@ -1088,7 +1088,7 @@ int launch_tc(const CUtensorMap* tmA, const CUtensorMap* tmB, const CUtensorMap*
   int cap = g_max_ctas > 0 ? g_max_ctas : num_sms();
   int grid = total < cap ? total : cap;
   GatherArgs none{};
-  return (int)mlb_launch_tmem(kern, dim3(grid), dim3(GEMM_THREADS), GemmSmem<BN>::TOTAL, st, *tmA, *tmB, *tmD, g, none);
+  return (int)mlb_launch_tmem(true, kern, dim3(grid), dim3(GEMM_THREADS), GemmSmem<BN>::TOTAL, st, *tmA, *tmB, *tmD, g, none);
 }
 
 // CTA-pair kernel: one cluster of two CTAs per SM pair; the grid is sized from the number of clusters that can be
@@ -1137,7 +1137,7 @@ int launch_tc2(const CUtensorMap* tmA, const CUtensorMap* tmB, const CUtensorMap
       g.nt_fast = 0;
     }
   }
-  return (int)mlb_launch_tmem(kern, dim3(2 * clusters), dim3(GEMM2_THREADS), Gemm2Smem::TOTAL, st, *tmA, *tmB, *tmD, g);
+  return (int)mlb_launch_tmem(true, kern, dim3(2 * clusters), dim3(GEMM2_THREADS), Gemm2Smem::TOTAL, st, *tmA, *tmB, *tmD, g);
 }
 int pair_clusters() { return (g_max_ctas > 0 ? g_max_ctas : num_sms()) / 2; }
 
@@ -1233,7 +1233,7 @@ int launch_splitk(const CUtensorMap* tmA, const CUtensorMap* tmB, const SplitKAr
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = mlb_pdl_enabled() ? 2 : 1;
+  cfg.numAttrs = mlb_pdl_tmem(true) ? 2 : 1;
   return (int)cudaLaunchKernelEx(&cfg, kern, *tmA, *tmB, g);
 }
 template <bool A_MN, bool B_MN, int EPI>

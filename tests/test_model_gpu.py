@@ -391,3 +391,37 @@ def test_gradient_clipping_on_the_device(comm):
     # about mx / |g| = 1/60 as long
     assert res["eager"][1] < 0.1 * res["plain"][1] and res["graph"][1] < 0.1 * res["plain"][1], [v[1] for v in res.values()]
     assert _native().get_error() == 0
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_kernels_that_start_early_give_the_same_bits(graph):
+    """Small kernels start under the one before them (MLB_PDL unset); with MLB_PDL=0 none does.  Same kernels, same sums: same bits, through
+    a model whose every launch is small, eagerly and captured."""
+    import os
+    import subprocess
+    import sys
+    code = (
+        "import torch\n"
+        "from ml_b200 import Config\n"
+        "from ml_b200.trainer import Trainer\n"
+        "from ml_b200.ops import native\n"
+        "native.lib().mlb_gemm_set_splits(1)\n"
+        "cfg = Config(V=256, C=128, L=3, H=4, I=256, T=64)\n"
+        f"tr = Trainer(cfg, 4, 'cuda:0', lr=1e-3, wd=0.1, use_graph={graph})\n"
+        "ids, tgt = (torch.randperm(256, generator=torch.Generator().manual_seed(i)).int().cuda() for i in (1, 2))\n"      # (a token twice is added as it comes)
+        "tr.set_batch(ids, tgt)\n"
+        "for _ in range(30): tr.step()\n"
+        "torch.cuda.synchronize()\n"
+        "g = tr.model.grads.view(torch.int32).long()\n"
+        "print('SUM', tr.model.losses.view(torch.int32).long().sum().item(), (g * torch.arange(1, g.numel() + 1, device='cuda')).sum().item(), native.get_error())\n")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    out = []
+    for pdl in ("0", None):
+        env = dict(os.environ, PYTHONPATH=root)
+        env.pop("MLB_PDL", None)
+        if pdl is not None:
+            env["MLB_PDL"] = pdl
+        r = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stderr[-2000:]
+        out.append([l for l in r.stdout.splitlines() if l.startswith("SUM")][0])
+    assert out[0] == out[1] and out[0].endswith(" 0"), out
