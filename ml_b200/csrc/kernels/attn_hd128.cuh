@@ -4,7 +4,7 @@
 // exponentials take the special-function units (2048 cycles each), and in backward the products lead (2048 / 1536 cycles against
 // 1024), so the kernels are built around never letting one wait for the other; tensor memory is the constraint (a 128 x 128
 // fp32 tile is 128 of its 512 columns).  P and dS are written as bf16 pairs over the score columns they came from and are read
-// from there as the A operand of the next product: no shared memory, and no columns of their own.  MMAs are promised to run in
+// from there as the A operand of the next product: no columns of their own, and no shared memory (but for the P^T of dK / dV).  MMAs are promised to run in
 // the order of their issue only where accumulator and shape are the same, so a product that overwrites such columns is issued when
 // the one that reads them has completed (its commit is waited for).
 // All three kernels are persistent, one CTA per SM over a balanced table of items (attn_schedule); every wait is bounded and
@@ -326,25 +326,32 @@ __global__ void __maxnreg__(160) attn_fwd128_k(const __grid_constant__ CUtensorM
 }
 
 // ------------------------------------------------------------------ backward
-// dK / dV of a 128-key tile, streaming query blocks.  TMEM: S^T, dP^T, dV, dK.  The tensor core's sequence is
-//   dV(i)  S^T(i+1)  dK(i)  dP^T(i+1)  dV(i+1) ...
-// so the exponentials of block i+1 run under dK(i) and dP^T(i+1), and dS(i+1) under dV(i+1) and S^T(i+2).  512 element-wise threads: a
-// thread has one key and 32 of the block's 128 queries; its P^T / dS^T go over its own score columns.  Four warps per sub-partition
-// hide each other's TMEM and barrier latencies: with two (64 queries a thread) a block took them 3000 cycles, of which 1024 are the
-// special-function unit's.
+// dK / dV of a 128-key tile, streaming query blocks.  TMEM: S^T, dP^T, dV, dK.  Two threads issue products, as in the kernels for head
+// size 64: every tcgen05.mma and commit costs the thread that issues it 75 ... 100 cycles whatever its size, 3600 for a block's 36
+// with one thread.  One takes  S^T(i) dP^T(i) S^T(i+1) ...,  the other  dV(i) dK(i) ...
+// P^T goes to shared memory, so S^T(i+1) needs no more than that S^T(i) has been read, and the exponentials of block i+1 run under
+// dK(i) and dP^T(i+1); over its scores it would make S^T(i+1) wait for dV(i).  dS^T stays over dP^T.  512 element-wise threads: a
+// thread has one key and 32 of the block's 128 queries.  Four warps per sub-partition hide each other's TMEM and barrier
+// latencies.  The queries' statistics are one warp's work (fetched by those who use them, each block waited 800 cycles for them).
+// Shared memory is full to the last 512 bytes: nothing is left to align its base with, which is checked instead.
+// A block takes 3500 cycles (3950 with one issuing thread and P^T over its scores); what is left is the shared memory's: three of
+// the four products read both operands there, 2000 of its cycles, the tiles that arrive 500, and Q's slot is given back late (asking
+// for its lines in the L2 beforehand changed nothing).  8 x 2048 tokens, 16 heads, forward + backward: 1047 -> 1015 ... 1025 us with the same for dQ.
 struct BwdKV128Smem {
   static constexpr int K = 0;
   static constexpr int V = K + T128_BYTES;
   static constexpr int Q = V + T128_BYTES;               // 2 slots
   static constexpr int DO = Q + 2 * T128_BYTES;          // 2 slots
-  static constexpr int STAT = DO + 2 * T128_BYTES;       // 16 warps x 2 buffers x (lse * log2 e [32], delta [32])
-  static constexpr int BAR = STAT + 16 * 512;
+  static constexpr int P = DO + 2 * T128_BYTES;          // P^T of a block, two chunks of 64 queries
+  static constexpr int STAT = P + T128_BYTES;            // 2 buffers x (lse * log2 e [128], delta [128])
+  static constexpr int BAR = STAT + 2 * 1024;
   static constexpr int SCHED = BAR + 256;
-  static constexpr int TOTAL = SCHED + 256 + 1024;
+  static constexpr int TOTAL = SCHED + 256;
 };
 // dQ of a 128-query tile, streaming key blocks.  TMEM: S in two buffers, dP, dQ; dS goes over the S it came from:
-//   dP(j+1)  dQ(j)  S(j+2)  dP(j+2) ...
+//   dP(j+1)  S(j+2)  dP(j+2) ...   by one thread,   dQ(j)  dQ(j+1) ...   by another
 // keeps scores one block ahead, so the element-wise threads never wait for them.
+// A block takes 2700 cycles (3050 when one thread issued all three products, one after the other's 8 instructions).
 struct BwdQ128Smem {
   static constexpr int Q = 0;
   static constexpr int DO = Q + T128_BYTES;
@@ -355,8 +362,9 @@ struct BwdQ128Smem {
   static constexpr int TOTAL = SCHED + 256 + 1024;
 };
 constexpr int BWD128_E_WARPS = 16;      // element-wise warps: lane group w & 3, quarter of the 128 columns w >> 2
-constexpr int BWD128_MMA_WARP = BWD128_E_WARPS, BWD128_LOAD_WARP = BWD128_E_WARPS + 1;
-constexpr int BWD128_THREADS = (BWD128_E_WARPS + 2) * 32;
+constexpr int BWD128_MMA_WARP = BWD128_E_WARPS, BWD128_LOAD_WARP = BWD128_E_WARPS + 1, BWD128_GRAD_WARP = BWD128_E_WARPS + 2,
+              BWD128_STAT_WARP = BWD128_E_WARPS + 3;
+constexpr int BWD128_THREADS = (BWD128_E_WARPS + 4) * 32;      // (five warps per sub-partition, as with two of the four)
 // (split_col(ks): A-operand column of k-step ks of a bf16 tile whose 32-column quarters sit over their own fp32 columns)
 
 __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUtensorMap tm_do,
@@ -364,14 +372,19 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
   mlb_pdl_sync();
   using S = BwdKV128Smem;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint8_t* smem = smem_raw;
   uint64_t* bars = (uint64_t*)(smem + S::BAR);
   uint64_t *bar_kv = bars, *bar_kvf = bars + 1, *bar_q = bars + 2 /*[2]*/, *bar_qf = bars + 4 /*[2]*/, *bar_do = bars + 6 /*[2]*/, *bar_dof = bars + 8 /*[2]*/,
            *bar_s = bars + 10, *bar_dp = bars + 11, *bar_p = bars + 12, *bar_ds = bars + 13, *bar_done = bars + 14;
-  uint64_t* bar_end = bars + 15;      // the MMA thread's last commit
-  uint32_t* tmem_slot = (uint32_t*)(bars + 16);
-  volatile int* s_abort = (volatile int*)(bars + 17);
+  uint64_t* bar_end = bars + 15;      // [2]: the MMA threads' last commits
+  uint64_t *bar_sr = bars + 17 /* S^T read out */, *bar_st = bars + 18 /*[2] statistics there */, *bar_stf = bars + 20 /*[2] read */;
+  uint32_t* tmem_slot = (uint32_t*)(bars + 22);
+  volatile int* s_abort = (volatile int*)(bars + 23);
   if (attn_given_up()) return;
+  if ((tc::smem_u32(smem) & 1023) != 0) {
+    if (threadIdx.x == 0) mlb_set_error(MLB_ERR_BOUNDS, 0xA1);
+    return;
+  }
   const int nq = (a.T + 127) / 128, BH = a.B * a.H, C = a.H * H128;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int* srow = a.sched ? a.sched + (size_t)blockIdx.x * a.sched_stride : nullptr;
@@ -379,7 +392,7 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
   if (srow && tid < 64) s_sched[tid] = tid < a.sched_stride ? __ldg(srow + tid) : -1;
   const ItemList items{srow, s_sched, (int)blockIdx.x, (int)gridDim.x, nq * BH};
   if (tid == 0) {
-    for (int i = 0; i < 16; i++) tc::mbar_init(&bars[i], (i == 12 || i == 13) ? BWD128_E_WARPS : 1);
+    for (int i = 0; i < 22; i++) tc::mbar_init(&bars[i], (i == 12 || i == 13 || i == 17 || i >= 20) ? BWD128_E_WARPS : 1);
     *s_abort = 0;
     tc::mbar_fence_init();
     tc::tma_prefetch_desc(&tm);
@@ -401,7 +414,7 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
   // item w = key tile (heaviest, the first, first) of (sample, head)
   if (warp == BWD128_LOAD_WARP) {
     if (lane == 0) {
-      int g = 0, nkv = 0, odd = 0;      // odd: a Q without its dO
+      int g = 0, nkv = 0;
       bool ok = true;
       for (int li = 0, w; ok && (w = items.at(li)) >= 0; li++) {
         const int kt = w / BH, bh = w % BH, b = bh / a.H, xh = (bh % a.H) * H128;
@@ -412,101 +425,117 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
         split_load<2>(smem + S::V, &tm, bar_kv, 2 * C + xh, kt * 128, b, 2);
         for (int i = kt; i < nq; i++, g++) {
           const int sl = g & 1, ph = ((g >> 1) + 1) & 1;
-          if (g >= 2 && !wait(&bar_qf[sl], ph, 62)) { ok = false; break; }
+          if (g >= 2 && !wait(&bar_qf[sl], ph, 62)) { ok = false; break; }      // (dK comes after dV, and after the dP^T its dS^T was made of)
           tc::mbar_expect_tx(&bar_q[sl], T128_BYTES);
           split_load<2>(smem + S::Q + sl * T128_BYTES, &tm, &bar_q[sl], xh, i * 128, b, 2);
-          if (g >= 2 && !wait(&bar_dof[sl], ph, 63)) { ok = false; odd = 1; break; }
           tc::mbar_expect_tx(&bar_do[sl], T128_BYTES);
           split_load<2>(smem + S::DO + sl * T128_BYTES, &tm_do, &bar_do[sl], xh, i * 128, b, 2);
         }
       }
       attn_settle(bar_kv, nkv);
       for (int i = 0; i < 2; i++) {
-        attn_settle(&bar_q[i], (g + odd + 1 - i) / 2);
+        attn_settle(&bar_q[i], (g + 1 - i) / 2);
         attn_settle(&bar_do[i], (g + 1 - i) / 2);
       }
     }
   } else if (warp == BWD128_MMA_WARP) {
     if (lane == 0) {
-      constexpr uint32_t idesc_s = tc::idesc_bf16(128, 128, 0, 0), idesc_g = tc::idesc_bf16(128, H128, 0, 1);
+      constexpr uint32_t idesc_s = tc::idesc_bf16(128, 128, 0, 0);
       const uint64_t dK = desc_base_k(tc::smem_u32(smem + S::K)), dV = desc_base_k(tc::smem_u32(smem + S::V));
-      const uint64_t dQ0 = desc_base_k(tc::smem_u32(smem + S::Q)), dO0 = desc_base_k(tc::smem_u32(smem + S::DO));      // as B of the scores
-      const uint64_t gQ0 = desc_base_mn(tc::smem_u32(smem + S::Q)), gO0 = desc_base_mn(tc::smem_u32(smem + S::DO));    // as B of the gradients
+      const uint64_t dQ0 = desc_base_k(tc::smem_u32(smem + S::Q)), dO0 = desc_base_k(tc::smem_u32(smem + S::DO));
       int g = 0;
       bool ok = true;
       for (int li = 0, w; ok && (w = items.at(li)) >= 0; li++) {
         const int n = nq - w / BH;
-        auto scores = [&](int gb) {      // over P^T, which the block before's dV reads
-          if (!ok || !wait(&bar_q[gb & 1], (gb >> 1) & 1, 64) || (gb > 0 && !wait(&bar_dof[(gb - 1) & 1], ((gb - 1) >> 1) & 1, 83))) { ok = false; return; }
+        ok = wait(bar_kv, li & 1, 66);
+        for (int i = 0; i < n; i++, g++) {
+          const int sl = g & 1, ph = (g >> 1) & 1;
+          // over the scores of the block before, once those have been read
+          if (!ok || !wait(&bar_q[sl], ph, 64) || (g > 0 && !wait(bar_sr, (g - 1) & 1, 83))) { ok = false; break; }
           tc::tc_fence_after();
-          const uint64_t dQ = dQ0 + (gb & 1) * T128_UNITS;
+          const uint64_t dQ = dQ0 + sl * T128_UNITS, dO = dO0 + sl * T128_UNITS;
 #pragma unroll
           for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ss(t_s, dK + off_k(ks, TILE_BYTES), dQ + off_k(ks, TILE_BYTES), idesc_s, ks > 0);
           tc::mma_commit(bar_s);
-        };
-        auto dprobs = [&](int gb, bool last) {      // over dS^T, which the block before's dK reads
-          if (!ok || !wait(&bar_do[gb & 1], (gb >> 1) & 1, 65) || (gb > 0 && !wait(&bar_qf[(gb - 1) & 1], ((gb - 1) >> 1) & 1, 84))) { ok = false; return; }
+          // over dS^T of the block before, which its dK reads
+          if (!wait(&bar_do[sl], ph, 65) || (g > 0 && !wait(&bar_qf[sl ^ 1], ((g - 1) >> 1) & 1, 84))) { ok = false; break; }
           tc::tc_fence_after();
-          const uint64_t dO = dO0 + (gb & 1) * T128_UNITS;
 #pragma unroll
           for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ss(t_dp, dV + off_k(ks, TILE_BYTES), dO + off_k(ks, TILE_BYTES), idesc_s, ks > 0);
           tc::mma_commit(bar_dp);
-          if (last) tc::mma_commit(bar_kvf);
-        };
-        ok = wait(bar_kv, li & 1, 66);
-        scores(g);
-        dprobs(g, n == 1);
+          if (i == n - 1) tc::mma_commit(bar_kvf);
+        }
+      }
+      tc::mma_commit(&bar_end[0]);
+      attn_settle(&bar_end[0], 1);
+    }
+  } else if (warp == BWD128_GRAD_WARP) {
+    if (lane == 0) {
+      constexpr uint32_t idesc_g = tc::idesc_bf16(128, H128, 0, 1);
+      const uint64_t aP = desc_base_k(tc::smem_u32(smem + S::P));
+      const uint64_t gQ0 = desc_base_mn(tc::smem_u32(smem + S::Q)), gO0 = desc_base_mn(tc::smem_u32(smem + S::DO));
+      int g = 0;
+      bool ok = true;
+      for (int li = 0, w; ok && (w = items.at(li)) >= 0; li++) {
+        const int n = nq - w / BH;
         for (int i = 0; i < n; i++, g++) {
           const int sl = g & 1;
           const uint64_t gQ = gQ0 + sl * T128_UNITS, gO = gO0 + sl * T128_UNITS;
-          if (!ok || !wait(bar_p, g & 1, 67)) { ok = false; break; }      // (of an item's first block: also the accumulators of the previous item have been read out)
+          if (!wait(bar_p, g & 1, 67)) { ok = false; break; }      // (of an item's first block: also the accumulators of the previous item have been read out)
           tc::tc_fence_after();
 #pragma unroll
-          for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ts(t_dv, t_s + split_col(ks), gO + off_mn(ks), idesc_g, (i > 0 || ks > 0));
+          for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ss(t_dv, aP + off_k(ks, TILE_BYTES), gO + off_mn(ks), idesc_g, (i > 0 || ks > 0));
           tc::mma_commit(&bar_dof[sl]);
-          if (i + 1 < n) scores(g + 1);
-          if (!ok || !wait(bar_ds, g & 1, 68)) { ok = false; break; }
+          if (!wait(bar_ds, g & 1, 68)) { ok = false; break; }
           tc::tc_fence_after();
 #pragma unroll
           for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ts(t_dk, t_dp + split_col(ks), gQ + off_mn(ks), idesc_g, (i > 0 || ks > 0));
           tc::mma_commit(&bar_qf[sl]);
-          if (i + 1 < n) dprobs(g + 1, i + 2 == n);
-          else tc::mma_commit(bar_done);
         }
+        if (ok) tc::mma_commit(bar_done);
       }
-      tc::mma_commit(bar_end);
-      attn_settle(bar_end, 1);
+      tc::mma_commit(&bar_end[1]);
+      attn_settle(&bar_end[1], 1);
+    }
+  } else if (warp == BWD128_STAT_WARP) {
+    // statistics of a block's queries, two blocks ahead at most; a query past the end has lse = +inf: p = 0
+    int g = 0;
+    bool ok = true;
+    for (int li = 0, w; ok && (w = items.at(li)) >= 0; li++) {
+      const size_t e = (size_t)(w % BH) * a.T;
+      for (int i = w / BH; i < nq; i++, g++) {
+        float nl[4], nd[4];
+#pragma unroll
+        for (int x = 0; x < 4; x++) {
+          const int q = i * 128 + x * 32 + lane;
+          nl[x] = q < a.T ? a.lse[e + q] * LOG2E : INFINITY;
+          nd[x] = q < a.T ? a.delta[e + q] : 0.f;
+        }
+        if (g >= 2 && !wait(&bar_stf[g & 1], ((g >> 1) + 1) & 1, 63)) { ok = false; break; }
+        __syncwarp();
+        float* stat = (float*)(smem + S::STAT + (g & 1) * 1024);
+#pragma unroll
+        for (int x = 0; x < 4; x++) {
+          stat[x * 32 + lane] = nl[x];
+          stat[128 + x * 32 + lane] = nd[x];
+        }
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&bar_st[g & 1]);
+      }
     }
   } else {
     const int lg = warp & 3, qd = warp >> 2, row = lg * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(lg * 32) << 16;
     const uint32_t ts = t_s + qd * 32 + lane_addr, tdp = t_dp + qd * 32 + lane_addr;
     const float sl2 = a.scale * LOG2E;
-    float* stat = (float*)(smem + S::STAT + warp * 512);
+    uint8_t* prow = smem + S::P + (qd >> 1) * TILE_BYTES + row * 128;      // this thread's 64 bytes of P^T: units 4 (qd & 1) ... of the chunk's row
     int g = 0;
-    // statistics of the warp's 32 queries, one per lane, fetched a block ahead (an item's first ones under the epilogue before it); a
-    // query past the end has lse = +inf: p = 0
-    float nl = 0.f, nd = 0.f;
-    auto fetch = [&](int w, int i) {
-      const int q = i * 128 + qd * 32 + lane;
-      const size_t e = (size_t)(w % BH) * a.T + q;
-      nl = q < a.T ? a.lse[e] * LOG2E : INFINITY;
-      nd = q < a.T ? a.delta[e] : 0.f;
-    };
-    int w = items.at(0);
-    if (w >= 0) fetch(w, w / BH);
-    for (int li = 0; w >= 0; li++) {
+    for (int li = 0, w; (w = items.at(li)) >= 0; li++) {
       const int kt = w / BH, bh = w % BH, b = bh / a.H, h = bh % a.H;
       const int krow = kt * 128 + row;
-      auto publish = [&](int gb) {
-        stat[(gb & 1) * 64 + lane] = nl;
-        stat[(gb & 1) * 64 + 32 + lane] = nd;
-        __syncwarp();
-      };
-      publish(g);
       for (int i = kt; i < nq; i++, g++) {
-        const float* st = stat + (g & 1) * 64;
-        if (i + 1 < nq) fetch(w, i + 1);
+        const float* st = (const float*)(smem + S::STAT + (g & 1) * 1024) + qd * 32;
+        wait(&bar_st[g & 1], (g >> 1) & 1, 87);
         wait(bar_s, g & 1, 69);
         __syncwarp();
         tc::tc_fence_after();
@@ -514,6 +543,9 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
         {
           uint32_t r[32];
           tc::tmem_ld32_wait(ts, r);
+          tc::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive(bar_sr);
 #pragma unroll
           for (int e = 0; e < 32; e += 4) {
             const float4 L = *reinterpret_cast<const float4*>(st + e);
@@ -531,9 +563,11 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
         uint32_t pw[16];
 #pragma unroll
         for (int x = 0; x < 16; x++) pw[x] = pack_bf16(p[2 * x], p[2 * x + 1]);
-        tc::tmem_st16(ts, pw);
-        tc::tmem_st_wait();
-        tc::tc_fence_before();
+        if (g > 0) wait(&bar_dof[(g - 1) & 1], ((g - 1) >> 1) & 1, 86);      // dV of the block before has read its P^T
+#pragma unroll
+        for (int v = 0; v < 4; v++)
+          *reinterpret_cast<uint4*>(prow + ((((qd & 1) * 4 + v) ^ (row & 7)) << 4)) = make_uint4(pw[v * 4], pw[v * 4 + 1], pw[v * 4 + 2], pw[v * 4 + 3]);
+        tc::fence_async_smem();
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(bar_p);
         wait(bar_dp, g & 1, 70);
@@ -544,7 +578,7 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
           tc::tmem_ld32_wait(tdp, d);
 #pragma unroll
           for (int e = 0; e < 32; e += 4) {
-            const float4 D = *reinterpret_cast<const float4*>(st + 32 + e);
+            const float4 D = *reinterpret_cast<const float4*>(st + 128 + e);
             pw[e / 2] = pack_bf16(p[e] * (__uint_as_float(d[e]) - D.x), p[e + 1] * (__uint_as_float(d[e + 1]) - D.y));
             pw[e / 2 + 1] = pack_bf16(p[e + 2] * (__uint_as_float(d[e + 2]) - D.z), p[e + 3] * (__uint_as_float(d[e + 3]) - D.w));
           }
@@ -553,12 +587,12 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
         tc::tmem_st_wait();
         tc::tc_fence_before();
         __syncwarp();
-        if (lane == 0) tc::mbar_arrive(bar_ds);
-        if (i + 1 < nq) publish(g + 1);
+        if (lane == 0) {
+          tc::mbar_arrive(bar_ds);
+          tc::mbar_arrive(&bar_stf[g & 1]);
+        }
       }
       // ---- epilogue: a warp stores 64 columns of dK (quarters 0, 1; softmax scale and RoPE's backward rotation applied) or dV (2, 3)
-      w = items.at(li + 1);
-      if (w >= 0) fetch(w, w / BH);
       wait(bar_done, li & 1, 71);
       __syncwarp();
       tc::tc_fence_after();
@@ -582,10 +616,11 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = (uint64_t*)(smem + S::BAR);
   uint64_t *bar_x = bars, *bar_xf = bars + 1, *bar_k = bars + 2 /*[3]*/, *bar_kf = bars + 5 /*[3]*/, *bar_v = bars + 8 /*[2]*/, *bar_vf = bars + 10 /*[2]*/,
-           *bar_s = bars + 12 /*[2]*/, *bar_dp = bars + 14, *bar_done = bars + 15, *bar_ds = bars + 16;
-  uint64_t* bar_end = bars + 17;      // the MMA thread's last commit
-  uint32_t* tmem_slot = (uint32_t*)(bars + 18);
-  volatile int* s_abort = (volatile int*)(bars + 19);
+           *bar_s = bars + 12 /*[2]*/, *bar_dp = bars + 14, *bar_done = bars + 15,
+           *bar_ds = bars + 16 /*[2]: the thread that issues dQ may be a block behind*/;
+  uint64_t* bar_end = bars + 18;      // [2]: the MMA threads' last commits
+  uint32_t* tmem_slot = (uint32_t*)(bars + 20);
+  volatile int* s_abort = (volatile int*)(bars + 21);
   if (attn_given_up()) return;
   const int nq = (a.T + 127) / 128, BH = a.B * a.H, C = a.H * H128;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -594,7 +629,7 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
   if (srow && tid < 64) s_sched[tid] = tid < a.sched_stride ? __ldg(srow + tid) : -1;
   const ItemList items{srow, s_sched, (int)blockIdx.x, (int)gridDim.x, nq * BH};
   if (tid == 0) {
-    for (int i = 0; i < 18; i++) tc::mbar_init(&bars[i], i == 16 ? BWD128_E_WARPS : 1);
+    for (int i = 0; i < 20; i++) tc::mbar_init(&bars[i], (i == 16 || i == 17) ? BWD128_E_WARPS : 1);
     *s_abort = 0;
     tc::mbar_fence_init();
     tc::tma_prefetch_desc(&tm);
@@ -641,11 +676,10 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
     }
   } else if (warp == BWD128_MMA_WARP) {
     if (lane == 0) {
-      constexpr uint32_t idesc_s = tc::idesc_bf16(128, 128, 0, 0), idesc_g = tc::idesc_bf16(128, H128, 0, 1);
+      constexpr uint32_t idesc_s = tc::idesc_bf16(128, 128, 0, 0);
       const uint64_t dQ = desc_base_k(tc::smem_u32(smem + S::Q)), dO = desc_base_k(tc::smem_u32(smem + S::DO));
       const uint64_t dK0 = desc_base_k(tc::smem_u32(smem + S::K)), dV0 = desc_base_k(tc::smem_u32(smem + S::V));
-      const uint64_t gK0 = desc_base_mn(tc::smem_u32(smem + S::K));      // as B of dQ
-      int g = 0, kr = 0;      // kr = g % 3
+      int g = 0;
       bool ok = true;
       for (int li = 0, w; ok && (w = items.at(li)) >= 0; li++) {
         const int n = nq - w / BH;
@@ -674,23 +708,38 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
         if (n > 1) scores(g + 1);
         dprobs(g, n == 1);
         for (int j = 0; j < n; j++, g++) {
-          if (!ok || !wait(bar_ds, g & 1, 78)) { ok = false; break; }      // dP(j) read, dS(j) stored (of an item's first block: the previous dQ read out)
-          tc::tc_fence_after();
+          if (!ok || !wait(&bar_ds[g & 1], (g >> 1) & 1, 78)) { ok = false; break; }      // dP(j) read
           if (j + 1 < n) dprobs(g + 1, j + 2 == n);
+          if (j + 2 < n) scores(g + 2);
+        }
+      }
+      tc::mma_commit(&bar_end[0]);
+      attn_settle(&bar_end[0], 1);
+    }
+  } else if (warp == BWD128_GRAD_WARP) {
+    if (lane == 0) {
+      constexpr uint32_t idesc_g = tc::idesc_bf16(128, H128, 0, 1);
+      const uint64_t gK0 = desc_base_mn(tc::smem_u32(smem + S::K));
+      int g = 0, kr = 0;      // kr = g % 3
+      bool ok = true;
+      for (int li = 0, w; ok && (w = items.at(li)) >= 0; li++) {
+        const int n = nq - w / BH;
+        for (int j = 0; j < n; j++, g++) {
+          if (!wait(&bar_ds[g & 1], (g >> 1) & 1, 68)) { ok = false; break; }      // dS(j) stored (of an item's first block: the previous dQ read out)
+          tc::tc_fence_after();
           const uint64_t gK = gK0 + kr * T128_UNITS;
           const uint32_t t_ds = tmem + (g & 1) * 128;
 #pragma unroll
           for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ts(t_dq, t_ds + split_col(ks), gK + off_mn(ks), idesc_g, (j > 0 || ks > 0));
           tc::mma_commit(&bar_kf[kr]);
           kr = kr == 2 ? 0 : kr + 1;
-          if (j + 2 < n) scores(g + 2);
           if (j + 1 == n) tc::mma_commit(bar_done);
         }
       }
-      tc::mma_commit(bar_end);
-      attn_settle(bar_end, 1);
+      tc::mma_commit(&bar_end[1]);
+      attn_settle(&bar_end[1], 1);
     }
-  } else {
+  } else if (warp < BWD128_E_WARPS) {
     const int lg = warp & 3, qd = warp >> 2, row = lg * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(lg * 32) << 16;
     const float sl2 = a.scale * LOG2E;
@@ -737,7 +786,7 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
         tc::tmem_st_wait();
         tc::tc_fence_before();
         __syncwarp();
-        if (lane == 0) tc::mbar_arrive(bar_ds);
+        if (lane == 0) tc::mbar_arrive(&bar_ds[g & 1]);
       }
       // ---- epilogue: 64 columns by each warp of quarters 0 and 1
       w = items.at(li + 1);

@@ -47,10 +47,7 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t&
 
 // An earlier CTA of this library gave up on a wait: leave at once instead of queueing more waits behind it (CTA-uniform).
 __device__ __forceinline__ bool attn_given_up() {
-  __shared__ int s_skip;
-  if (threadIdx.x == 0) s_skip = *(volatile int*)&g_mlb_error;
-  __syncthreads();
-  return s_skip != 0;
+  return __syncthreads_or(threadIdx.x == 0 && *(volatile int*)&g_mlb_error != 0) != 0;
 }
 
 // A CTA one of whose waits has run out loads and multiplies nothing more.  What its threads have already issued still uses its shared
