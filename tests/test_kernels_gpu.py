@@ -1421,3 +1421,19 @@ def test_layernorm_forward_widths(rows, C, bias):
     e = torch.nn.functional.layer_norm(xd, (C,), w.double(), b.double() if bias else None, 1e-5)
     assert _rel(out, e) < 2 ** -8.5 and _rel(mean, xd.mean(-1)) < 1e-5
     assert _rel(rstd, torch.rsqrt(xd.var(-1, unbiased=False) + 1e-5)) < 1e-5
+
+
+@pytest.mark.parametrize("rows", [1, 7, 301])
+@pytest.mark.parametrize("C", [256, 512, 768, 1024, 1280, 1536, 1792, 2048])
+@pytest.mark.parametrize("bias", [False, True])
+def test_layernorm_forward_adds_in_one_order(rows, C, bias):
+    """Rows read as vectors and rows off a 16-byte boundary, read element by element, are added up in the same order: the same bits."""
+    torch.manual_seed(rows + C)
+    w, b, flat = 1 + rnd(1, C, scale=0.1).view(-1), rnd(1, C).view(-1) if bias else None, rnd(1, rows * C + 8).view(-1) + 0.3
+    outs = []
+    for x in (flat[1:1 + rows * C].clone().view(rows, C), flat[1:1 + rows * C].view(rows, C)):
+        o = torch.empty_like(x), torch.empty(rows, device=dev()), torch.empty(rows, device=dev())
+        nat().layernorm_fwd(*o, x, w, b, 1e-5)
+        outs.append(o)
+    for a, e in zip(*outs):
+        assert torch.equal(a, e)
