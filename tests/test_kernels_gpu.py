@@ -1437,3 +1437,24 @@ def test_layernorm_forward_adds_in_one_order(rows, C, bias):
         outs.append(o)
     for a, e in zip(*outs):
         assert torch.equal(a, e)
+
+
+@pytest.mark.parametrize("rows", [1, 9, 250, 1003, 2369, 9000])
+@pytest.mark.parametrize("C", [256, 768])
+def test_column_sums_fold_in_one_order(rows, C):
+    """Eight slices of every eighth partial row, added in order: exactly that, in 32 bits, from one partial row up to the most there are."""
+    torch.manual_seed(rows)
+    n = nat()
+    L, x, dy, w = n.lib(), rnd(rows, C), rnd(rows, C), rnd(1, C).view(-1)
+    o, mean, rstd, dx = torch.empty_like(x), torch.empty(rows, device=dev()), torch.empty(rows, device=dev()), torch.empty_like(x)
+    n.layernorm_fwd(o, mean, rstd, x, w, None, 1e-5)
+    part, d = torch.empty(L.mlb_rmsnorm_bwd_blocks(rows), 2 * C, device=dev()), torch.zeros(2 * C, device=dev())
+    p = lambda t: t.data_ptr()
+    assert L.mlb_layernorm_bwd2(p(dx), p(d), p(d[C:]), 0, p(dy), p(x), p(w), p(mean), p(rstd), rows, C, p(part), n._st()) == 0
+    total = None
+    for q in range(8):
+        s = torch.zeros(2 * C, device=dev())
+        for row in part[q::8]:
+            s += row
+        total = s if total is None else total + s
+    assert torch.equal(d, total)
