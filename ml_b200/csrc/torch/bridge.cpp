@@ -3,7 +3,7 @@
 // A call of a small operator costs the host more than the device: through a Python autograd.Function and ctypes a linear layer took
 // ~20 us forward and ~50 us backward for kernels of 3-10 us each.  Here are
 //   * the differentiable operators of ops/autograd.py as torch::autograd::Functions (the same kernels in the same order, the same
-//     saved tensors, so saved-tensor hooks and checkpointing see what they saw), and
+//     saved tensors, so saved-tensor hooks and checkpointing are given what they were given; what a hook gives back goes through unpacked()), and
 //   * the entry points that the training engine calls most, taking tensors (ops/native.py).
 // Every operator looks at its arguments first and returns NotImplemented for whatever is not the plain case (bf16 tensors of the current
 // device, two-dimensional, not empty, aligned, no transform or trace or dispatch mode active): ops/autograd.py then takes the Python
@@ -111,11 +111,30 @@ bool wants_grad(std::initializer_list<const Tensor*> ts) {
 }
 Maybe maybe(const Tensor& t) { return t.defined() ? Maybe(t) : Maybe(); }
 Tensor f32(const Tensor& like, at::IntArrayRef sizes) { return at::empty(sizes, like.options().dtype(at::kFloat)); }
-// A gradient as the kernels read it: rows behind each other, 16-byte aligned
+// A tensor as the kernels read it: rows behind each other, 16-byte aligned
 Tensor rows_of(const Tensor& g) {
   const Tensor c = g.contiguous();
   return aligned(c) ? c : c.clone();
 }
+
+[[noreturn]] void refuse(const std::string& why) {
+  pybind11::gil_scoped_acquire gil;
+  PyErr_SetString(PyExc_AssertionError, why.c_str());
+  python_error e;
+  e.persist();      // (nodes run on threads of the autograd engine)
+  throw e;
+}
+// A saved tensor: a hook may have handed back any other, and torch checks nothing of it.  Another device, type or size is refused
+// here, in front of the node's launches, with the error of the entry points in ops/native.py; another layout, or an address off a
+// 16-byte boundary, is copied into place.
+Tensor unpacked(const Tensor& t, const Tensor& grad, at::ScalarType type, at::IntArrayRef sizes) {
+  if (!t.defined() || t.device() != grad.device() || t.scalar_type() != type || t.layout() != at::kStrided || t.sizes() != sizes)
+    refuse("saved tensor: need " + std::string(c10::toString(type)) + " of sizes " + c10::str(sizes) + " on " + grad.device().str() + ", not " +
+           (t.defined() ? std::string(c10::toString(t.scalar_type())) + " of sizes " + c10::str(t.sizes()) + " on " + t.device().str() : "none"));
+  return rows_of(t);
+}
+Tensor unpacked_bf(const Tensor& t, const Tensor& grad, at::IntArrayRef sizes) { return unpacked(t, grad, at::kBFloat16, sizes); }
+Tensor unpacked_f32(const Tensor& t, const Tensor& grad, at::IntArrayRef sizes) { return unpacked(t, grad, at::kFloat, sizes); }
 
 // ------------------------------------------------------------------ linear
 Tensor linear_forward(const Tensor& x_, const Tensor& W_, const Tensor& b) {
@@ -134,13 +153,16 @@ Tensor linear_forward(const Tensor& x_, const Tensor& W_, const Tensor& b) {
 struct LinearFn : torch::autograd::Function<LinearFn> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& W, const Maybe& b) {
     ctx->save_for_backward({x, W});
+    ctx->saved_data["inner"] = x.size(1);
     ctx->saved_data["bias"] = b.has_value();
     return linear_forward(x, W, b.value_or(Tensor()));
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     const auto saved = ctx->get_saved_variables();
-    const Tensor x = saved[0].contiguous(), W = saved[1].contiguous(), dout = g[0].contiguous();
-    const int M = (int)x.size(0), Kd = (int)x.size(1), N = (int)W.size(0);
+    const Tensor dout = g[0].contiguous();
+    const int64_t rows = dout.size(0), cols = dout.size(1), inner = ctx->saved_data["inner"].toInt();
+    const Tensor x = unpacked_bf(saved[0], dout, {rows, inner}), W = unpacked_bf(saved[1], dout, {cols, inner});
+    const int M = (int)rows, Kd = (int)inner, N = (int)cols;
     const St st = stream();
     Tensor dx = at::empty({M, Kd}, x.options()), dW = at::empty({N, Kd}, W.options()), db;
     check(K.mlb_linear_dx(dx.data_ptr(), dout.data_ptr(), W.data_ptr(), M, N, Kd, Kd, N, Kd, st), "linear_dx");
@@ -180,8 +202,9 @@ struct RMSNormFn : torch::autograd::Function<RMSNormFn> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     const auto saved = ctx->get_saved_variables();
-    const Tensor x = saved[0].contiguous(), &w = saved[1], &rstd = saved[2], dy = rows_of(g[0]);
-    const long rows = x.size(0), C = x.size(1);
+    const Tensor dy = rows_of(g[0]);
+    const int64_t rows = dy.size(0), C = dy.size(1);
+    const Tensor x = unpacked_bf(saved[0], dy, {rows, C}), w = unpacked_bf(saved[1], dy, {C}), rstd = unpacked_f32(saved[2], dy, {rows});
     Tensor dx = at::empty_like(x), dw = at::empty_like(w);
     const Tensor part = f32(x, {K.mlb_rmsnorm_bwd_blocks(rows) * C});
     check(K.mlb_rmsnorm_bwd_cast(dx.data_ptr(), dw.data_ptr(), dy.data_ptr(), x.data_ptr(), w.data_ptr(), (const float*)rstd.data_ptr(), nullptr, rows, (int)C,
@@ -205,8 +228,10 @@ struct LayerNormFn : torch::autograd::Function<LayerNormFn> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     const auto saved = ctx->get_saved_variables();
-    const Tensor x = saved[0].contiguous(), &w = saved[1], &mean = saved[2], &rstd = saved[3], dy = rows_of(g[0]);
-    const long rows = x.size(0), C = x.size(1);
+    const Tensor dy = rows_of(g[0]);
+    const int64_t rows = dy.size(0), C = dy.size(1);
+    const Tensor x = unpacked_bf(saved[0], dy, {rows, C}), w = unpacked_bf(saved[1], dy, {C}), mean = unpacked_f32(saved[2], dy, {rows}),
+                 rstd = unpacked_f32(saved[3], dy, {rows});
     Tensor dx = at::empty_like(x), dw = at::empty_like(w), db;
     if (ctx->saved_data["bias"].toBool()) db = at::empty_like(w);
     const Tensor part = f32(x, {K.mlb_rmsnorm_bwd_blocks(rows) * 2 * C});
@@ -231,7 +256,7 @@ struct SwiGLUFn : torch::autograd::Function<SwiGLUFn> {
     return swiglu_forward(gu);
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
-    const Tensor gu = ctx->get_saved_variables()[0].contiguous(), dout = rows_of(g[0]);
+    const Tensor dout = rows_of(g[0]), gu = unpacked_bf(ctx->get_saved_variables()[0], dout, {dout.size(0), 2 * dout.size(1)});
     Tensor dgu = at::empty_like(gu);
     check(K.mlb_swiglu_bwd(dgu.data_ptr(), dout.data_ptr(), gu.data_ptr(), gu.size(0), (int)(gu.size(1) / 2), stream()), "swiglu_bwd");
     return {dgu};
@@ -255,16 +280,19 @@ struct CausalFn : torch::autograd::Function<CausalFn> {
     const Heads h{(int)B, (int)T, (int)H, (int)Hkv, (int)hd};
     const Attended r = causal_forward(qkv.contiguous(), cos, sin, h);
     ctx->save_for_backward({r.q, r.out, r.lse, cos, sin});
-    ctx->saved_data["dims"] = std::vector<int64_t>{B, T, H, Hkv, hd, max_part};
+    ctx->saved_data["dims"] = std::vector<int64_t>{B, T, H, Hkv, hd, max_part, cos.size(0), sin.size(0)};
     ctx->saved_data["shape"] = qkv.sizes().vec();
     return r.out;
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     const auto saved = ctx->get_saved_variables();
-    const Tensor &q = saved[0], &out = saved[1], &lse = saved[2], &cos = saved[3], &sin = saved[4], dout = rows_of(g[0]);
+    const Tensor dout = rows_of(g[0]);
     const auto dims = ctx->saved_data["dims"].toIntVector();
     const Heads h{(int)dims[0], (int)dims[1], (int)dims[2], (int)dims[3], (int)dims[4]};
-    const long n = (long)h.B * h.T;
+    const int64_t n = dims[0] * dims[1];
+    const Tensor q = unpacked_bf(saved[0], dout, {n, 3 * dims[2] * dims[4]}), out = unpacked_bf(saved[1], dout, {n, dims[2] * dims[4]}),
+                 lse = unpacked_f32(saved[2], dout, {dims[0], dims[2], dims[1]}), cos = unpacked_f32(saved[3], dout, {dims[6], dims[4] / 2}),
+                 sin = unpacked_f32(saved[4], dout, {dims[7], dims[4] / 2});
     const St st = stream();
     Tensor dqkv = at::empty_like(q), part;
     const Tensor delta = f32(q, {n * h.H});
@@ -299,8 +327,10 @@ struct BidirFn : torch::autograd::Function<BidirFn> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     const auto saved = ctx->get_saved_variables();
-    const Tensor q = saved[0].contiguous(), &out = saved[1], &lse = saved[2], dout = rows_of(g[0]);
+    const Tensor dout = rows_of(g[0]);
     const auto d = ctx->saved_data["dims"].toIntVector();
+    const Tensor q = unpacked_bf(saved[0], dout, {d[0] * d[1], 3 * d[2] * d[3]}), out = unpacked_bf(saved[1], dout, {d[0] * d[1], d[2] * d[3]}),
+                 lse = unpacked_f32(saved[2], dout, {d[0], d[2], d[1]});
     Tensor dqkv = at::empty_like(q);
     const Tensor delta = f32(q, {d[0] * d[1] * d[2]});
     check(K.mlb_attn_bidir_bwd(dqkv.data_ptr(), dout.data_ptr(), q.data_ptr(), out.data_ptr(), (const float*)lse.data_ptr(), (float*)delta.data_ptr(), (int)d[0],
@@ -323,11 +353,12 @@ struct CrossEntropyFn : torch::autograd::Function<CrossEntropyFn> {
   static Tensor forward(AutogradContext* ctx, const Tensor& logits, const Tensor& tgt) {
     const Crossed r = ce_forward(logits.contiguous(), tgt, true);
     ctx->save_for_backward({r.grad});
+    ctx->saved_data["shape"] = logits.sizes().vec();
     ctx->saved_data["shared"] = at::SavedTensorDefaultHooks::get_hooks().has_value();      // (see ops/autograd.py)
     return r.loss;
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
-    const Tensor d = ctx->get_saved_variables()[0];
+    const Tensor d = unpacked_bf(ctx->get_saved_variables()[0], g[0], ctx->saved_data["shape"].toIntVector());
     const bool last = !ctx->saved_data["shared"].toBool() && !torch::autograd::get_current_graph_task_keep_graph();
     Tensor out = last ? d : at::empty_like(d);
     const Tensor s = g[0].to(at::kFloat).contiguous();

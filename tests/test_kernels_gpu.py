@@ -1458,3 +1458,74 @@ def test_column_sums_fold_in_one_order(rows, C):
             s += row
         total = s if total is None else total + s
     assert torch.equal(d, total)
+
+
+def _native_nodes():
+    """name -> (operands, call through the public entry point), each a plain call of the extension module: for tests of its autograd nodes."""
+    from ml_b200.ops import autograd as F
+    B, T, H, Hkv, hd, rows, C, N = 2, 72, 4, 2, 64, 40, 256, 128
+    v = lambda n: rnd(1, n).view(-1)
+    cos, sin = ref.rope_tables(T, hd, 10000.0, dev())
+    tgt = torch.randint(0, N, (rows,), device=dev(), dtype=torch.int32)
+    return {
+        "linear": ([rnd(rows, C), rnd(N, C), v(N)], F.linear),
+        "rmsnorm": ([rnd(rows, C), v(C)], lambda x, w: F.rmsnorm(x, w, 1e-5)),
+        "layer_norm": ([rnd(rows, C), v(C), v(C)], lambda x, w, b: F.layer_norm(x, w, b, 1e-5)),
+        "swiglu": ([rnd(rows, 2 * N)], F.swiglu),
+        "rope_causal_attention": ([rnd(B * T, (H + 2 * Hkv) * hd)], lambda x: F.rope_causal_attention(x, cos, sin, B, T, H, hd, Hkv)),
+        "rope_causal_attention_128": ([rnd(B * T // 2, 3 * H * 128)],
+                                      lambda x, r=ref.rope_tables(T, 128, 10000.0, dev()): F.rope_causal_attention(x, *r, 1, T, H, 128)),
+        "bidir_attention": ([rnd(B * T, 3 * H * hd)], lambda x: F.bidir_attention(x, B, T, H, hd)),
+        "cross_entropy": ([rnd(rows, N)], lambda z: F.cross_entropy(z, tgt)),
+    }
+
+
+NATIVE_NODES = ["linear", "rmsnorm", "layer_norm", "swiglu", "rope_causal_attention", "rope_causal_attention_128", "bidir_attention", "cross_entropy"]
+
+
+def _native(y):
+    return "CppNode" in y.grad_fn.name()
+
+
+def _strided(t):      # the same values behind other strides
+    u = torch.empty(*t.shape[::-1], 2, dtype=t.dtype, device=t.device)[..., 0]
+    return u.permute(*reversed(range(t.dim()))).copy_(t)
+
+
+def _offset(t):       # ... one element off the start of a buffer
+    return torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)[1:].view(t.shape).copy_(t)
+
+
+@pytest.mark.parametrize("name", NATIVE_NODES)
+def test_saved_tensors_come_back_in_another_form(name):
+    """What a saved-tensor hook returns is not checked by torch.  The same values in another layout or off a 16-byte boundary give the same
+    gradients; another type, device or size is refused on the host, in front of the launches, as the entry points refuse it."""
+    from torch.autograd.graph import saved_tensors_hooks
+    torch.manual_seed(3)
+    ops_, call = _native_nodes()[name]
+    leaves = [t.requires_grad_(True) for t in ops_]
+    nat().lib().mlb_gemm_set_splits(1)      # (repeatable weight gradients)
+
+    def grads(change):
+        with saved_tensors_hooks(lambda t: t, change):
+            y = call(*leaves)
+        assert _native(y)
+        torch.manual_seed(4)
+        return torch.autograd.grad(y, leaves, rnd(1, *y.shape, dtype=y.dtype)[0])
+
+    try:
+        want = grads(lambda t: t)
+        for same in (_strided, _offset, lambda t: _strided(_offset(t)), lambda t: t.cpu().cuda()):
+            for a, b in zip(want, grads(same)):
+                assert torch.equal(a, b)
+        launched = nat().get_error()
+        for other in (torch.Tensor.float, torch.Tensor.double, torch.Tensor.half, torch.Tensor.cpu, lambda t: t[:-1], lambda t: t.view(-1), lambda t: t[None]):
+            changed = lambda t: other(t).dtype != t.dtype or other(t).device != t.device or other(t).shape != t.shape
+            # (a tensor that this changes nothing about is left as it is)
+            with pytest.raises(AssertionError, match="saved tensor"):
+                assert grads(lambda t: other(t) if changed(t) else t) is None
+        assert nat().get_error() == launched == 0
+        for a, b in zip(want, grads(lambda t: t)):
+            assert torch.equal(a, b)
+    finally:
+        nat().lib().mlb_gemm_set_splits(0)
