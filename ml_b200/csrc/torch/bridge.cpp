@@ -82,7 +82,7 @@ St stream() { return (St)c10::cuda::getCurrentCUDAStream().stream(); }
 void check(int rc, const char* what) { TORCH_CHECK(rc == 0, what, " failed: code ", rc); }
 
 // ------------------------------------------------------------------ which calls are plain
-// Something is watching or rewriting the operators of this thread
+// Something is watching or rewriting the operators of this thread.  Asked first: a transform's tensors have no address to look at.
 bool transformed() {
   if (torch::jit::tracer::isTracing() || c10::impl::TorchDispatchModeTLS::any_modes_set()) return true;
   const auto inc = c10::impl::tls_local_dispatch_key_set().included_;
@@ -382,17 +382,16 @@ PyObject* released(F&& f) {      // the launch without the interpreter lock
 PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   Tensor x, W, b;
-  if (n != 3 || !plain_bf(a[0], x, 2) || !plain_bf(a[1], W, 2) || x.size(1) != W.size(1)) return declined();
+  if (n != 3 || transformed() || !plain_bf(a[0], x, 2) || !plain_bf(a[1], W, 2) || x.size(1) != W.size(1)) return declined();
   if (a[2] != Py_None && (!plain_bf(a[2], b, 1) || b.size(0) != W.size(0) || !b.is_contiguous())) return declined();
-  if (transformed()) return declined();
   return released([&] { return wants_grad({&x, &W, &b}) ? LinearFn::apply(x, W, maybe(b)) : linear_forward(x, W, b); });
   END_HANDLE_TH_ERRORS
 }
 PyObject* py_rmsnorm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   Tensor x, w;
-  if (n != 3 || !plain_bf(a[0], x, 2) || !plain_bf(a[1], w, 1) || w.size(0) != x.size(1) || !w.is_contiguous() || !norm_width(x.size(1)) ||
-      !PyFloat_CheckExact(a[2]) || transformed())
+  if (n != 3 || transformed() || !plain_bf(a[0], x, 2) || !plain_bf(a[1], w, 1) || w.size(0) != x.size(1) || !w.is_contiguous() || !norm_width(x.size(1)) ||
+      !PyFloat_CheckExact(a[2]))
     return declined();
   const double eps = PyFloat_AS_DOUBLE(a[2]);
   return released([&] { return wants_grad({&x, &w}) ? RMSNormFn::apply(x, w, eps) : rmsnorm_forward(x, w, eps).out; });
@@ -401,11 +400,10 @@ PyObject* py_rmsnorm(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* py_layer_norm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   Tensor x, w, b;
-  if (n != 4 || !plain_bf(a[0], x, 2) || !plain_bf(a[1], w, 1) || w.size(0) != x.size(1) || !w.is_contiguous() || !norm_width(x.size(1)) ||
+  if (n != 4 || transformed() || !plain_bf(a[0], x, 2) || !plain_bf(a[1], w, 1) || w.size(0) != x.size(1) || !w.is_contiguous() || !norm_width(x.size(1)) ||
       !PyFloat_CheckExact(a[3]))
     return declined();
   if (a[2] != Py_None && (!plain_bf(a[2], b, 1) || b.size(0) != x.size(1) || !b.is_contiguous())) return declined();
-  if (transformed()) return declined();
   const double eps = PyFloat_AS_DOUBLE(a[3]);
   return released([&] { return wants_grad({&x, &w, &b}) ? LayerNormFn::apply(x, w, maybe(b), eps) : layernorm_forward(x.contiguous(), w, b, eps).out; });
   END_HANDLE_TH_ERRORS
@@ -413,7 +411,7 @@ PyObject* py_layer_norm(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* py_swiglu(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   Tensor gu;
-  if (n != 1 || !plain_bf(a[0], gu, 2) || gu.size(1) % 16 != 0 || transformed()) return declined();
+  if (n != 1 || transformed() || !plain_bf(a[0], gu, 2) || gu.size(1) % 16 != 0) return declined();
   return released([&] { return wants_grad({&gu}) ? SwiGLUFn::apply(gu) : swiglu_forward(gu); });
   END_HANDLE_TH_ERRORS
 }
@@ -422,7 +420,7 @@ PyObject* py_rope_causal_attention(PyObject*, PyObject* const* a, Py_ssize_t n) 
   HANDLE_TH_ERRORS
   Tensor qkv, cos, sin;
   long B, T, H, hd, Hkv;
-  if (n != 9 || !plain_bf(a[0], qkv, 2) || !plain(a[1], cos, at::kFloat, 2) || !plain(a[2], sin, at::kFloat, 2) || !int_arg(a[3], B) || !int_arg(a[4], T) ||
+  if (n != 9 || transformed() || !plain_bf(a[0], qkv, 2) || !plain(a[1], cos, at::kFloat, 2) || !plain(a[2], sin, at::kFloat, 2) || !int_arg(a[3], B) || !int_arg(a[4], T) ||
       !int_arg(a[5], H) || !int_arg(a[6], hd) || !PyLong_CheckExact(a[8]))
     return declined();
   const long part = PyLong_AsLong(a[8]);
@@ -432,7 +430,7 @@ PyObject* py_rope_causal_attention(PyObject*, PyObject* const* a, Py_ssize_t n) 
   const long rows = B * T;
   if (rows >= (1L << 31) || qkv.size(0) != rows || qkv.size(1) != (H + 2 * Hkv) * hd || rows * 3 * H * (hd / 16) >= (1L << 31) || !cos.is_contiguous() ||
       !sin.is_contiguous() || !aligned(cos) || !aligned(sin) || cos.size(0) < T || sin.size(0) < T || cos.size(1) != hd / 2 || sin.size(1) != hd / 2 ||
-      cos.requires_grad() || sin.requires_grad() || transformed())
+      cos.requires_grad() || sin.requires_grad())
     return declined();
   return released([&] {
     if (wants_grad({&qkv})) return CausalFn::apply(qkv, cos, sin, B, T, H, Hkv, hd, part);
@@ -444,15 +442,15 @@ PyObject* py_bidir_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   Tensor qkv;
   long B, T, H, hd;
-  if (n != 5 || !plain_bf(a[0], qkv, 2) || !int_arg(a[1], B) || !int_arg(a[2], T) || !int_arg(a[3], H) || !int_arg(a[4], hd)) return declined();
-  if (B < 1 || T < 1 || H < 1 || hd % 16 != 0 || hd > 128 || hd < 16 || qkv.size(0) != B * T || qkv.size(1) != 3 * H * hd || transformed()) return declined();
+  if (n != 5 || transformed() || !plain_bf(a[0], qkv, 2) || !int_arg(a[1], B) || !int_arg(a[2], T) || !int_arg(a[3], H) || !int_arg(a[4], hd)) return declined();
+  if (B < 1 || T < 1 || H < 1 || hd % 16 != 0 || hd > 128 || hd < 16 || qkv.size(0) != B * T || qkv.size(1) != 3 * H * hd) return declined();
   return released([&] { return wants_grad({&qkv}) ? BidirFn::apply(qkv, B, T, H, hd) : bidir_forward(qkv, B, T, H, hd).out; });
   END_HANDLE_TH_ERRORS
 }
 PyObject* py_cross_entropy(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   Tensor z, tgt;
-  if (n != 2 || !plain_bf(a[0], z, 2) || !plain(a[1], tgt, at::kInt, 1) || tgt.size(0) != z.size(0) || !tgt.is_contiguous() || transformed()) return declined();
+  if (n != 2 || transformed() || !plain_bf(a[0], z, 2) || !plain(a[1], tgt, at::kInt, 1) || tgt.size(0) != z.size(0) || !tgt.is_contiguous()) return declined();
   return released([&] { return wants_grad({&z}) ? CrossEntropyFn::apply(z, tgt) : ce_forward(z.contiguous(), tgt, false).loss; });
   END_HANDLE_TH_ERRORS
 }

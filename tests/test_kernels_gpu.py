@@ -1529,3 +1529,33 @@ def test_saved_tensors_come_back_in_another_form(name):
             assert torch.equal(a, b)
     finally:
         nat().lib().mlb_gemm_set_splits(0)
+
+
+@pytest.mark.parametrize("name", NATIVE_NODES)
+def test_transforms_and_modes_take_the_functions(name):
+    """Under a transform of torch.func, a trace or a dispatch mode the extension module declines (its tensors may have no memory) and the Python
+    Function runs, with its results and its errors."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+    ops_, call = _native_nodes()[name]
+    assert _native(call(*(t.requires_grad_(True) for t in ops_)))
+    ops_ = [t.detach() for t in ops_]
+    want = call(*ops_)
+    with pytest.raises(RuntimeError, match="autograd.Function with functorch"):      # (the Functions do not support them)
+        torch.func.grad(lambda x: call(x, *ops_[1:]).float().sum())(ops_[0])
+    with pytest.raises(RuntimeError, match="autograd.Function with functorch"):
+        torch.vmap(lambda x: call(x, *ops_[1:]))(torch.stack([ops_[0], ops_[0]]))
+    with pytest.raises(RuntimeError, match="autograd.Function with functorch"):      # (nor a level that is about other tensors)
+        torch.func.grad(lambda z: (call(*ops_).float() * z).sum())(torch.ones(1, device=dev()))
+
+    class Seen(TorchDispatchMode):
+        ops = []
+
+        def __torch_dispatch__(self, fn, types, args=(), kwargs=None):
+            self.ops.append(str(fn))
+            return fn(*args, **(kwargs or {}))
+
+    with Seen() as seen:
+        got = call(*ops_)
+    assert torch.equal(got, want) and any("new_empty" in o for o in seen.ops)      # (the module allocates without the dispatcher's modes looking on)
+    graph = torch.jit.trace(lambda *a: call(*a), tuple(ops_), check_trace=False).graph
+    assert any(n.kind() == "prim::PythonOp" for n in graph.nodes()), graph
