@@ -78,6 +78,8 @@ typedef std::optional<Tensor> Maybe;      // (an undefined tensor is no argument
 #define MLB_POINTER(name, ret, args) ret(*name) args = nullptr;
 struct Entries { MLB_ENTRIES(MLB_POINTER) } K;
 
+PyObject* settings = nullptr;      // the Python module whose variables FUSED_ATTN_BWD and FUSED_ATTN_BWD_MAX_SCRATCH bound attn_bwd's workspace
+
 St stream() { return (St)c10::cuda::getCurrentCUDAStream().stream(); }
 void check(int rc, const char* what) { TORCH_CHECK(rc == 0, what, " failed: code ", rc); }
 
@@ -274,13 +276,20 @@ Attended causal_forward(const Tensor& qkv, const Tensor& cos, const Tensor& sin,
   check(K.mlb_attn_fwd(r.out.data_ptr(), (float*)r.lse.data_ptr(), r.q.data_ptr(), h.B, h.T, h.H, h.hd, st), "attn_fwd");
   return r;
 }
+// May attn_bwd have a workspace of this size?  Asked in backward, as ops/native.py does: the variables may have been set since forward.
+bool scratch_allowed(long bytes) {
+  if (bytes <= 0) return false;
+  pybind11::gil_scoped_acquire gil;
+  const auto module = pybind11::reinterpret_borrow<pybind11::object>(settings);
+  return pybind11::bool_(module.attr("FUSED_ATTN_BWD")) && pybind11::int_(bytes) <= module.attr("FUSED_ATTN_BWD_MAX_SCRATCH");
+}
 struct CausalFn : torch::autograd::Function<CausalFn> {
   static Tensor forward(AutogradContext* ctx, const Tensor& qkv, const Tensor& cos, const Tensor& sin, int64_t B, int64_t T, int64_t H, int64_t Hkv,
-                        int64_t hd, int64_t max_part) {
+                        int64_t hd) {
     const Heads h{(int)B, (int)T, (int)H, (int)Hkv, (int)hd};
     const Attended r = causal_forward(qkv.contiguous(), cos, sin, h);
     ctx->save_for_backward({r.q, r.out, r.lse, cos, sin});
-    ctx->saved_data["dims"] = std::vector<int64_t>{B, T, H, Hkv, hd, max_part, cos.size(0), sin.size(0)};
+    ctx->saved_data["dims"] = std::vector<int64_t>{B, T, H, Hkv, hd, cos.size(0), sin.size(0)};
     ctx->saved_data["shape"] = qkv.sizes().vec();
     return r.out;
   }
@@ -291,13 +300,13 @@ struct CausalFn : torch::autograd::Function<CausalFn> {
     const Heads h{(int)dims[0], (int)dims[1], (int)dims[2], (int)dims[3], (int)dims[4]};
     const int64_t n = dims[0] * dims[1];
     const Tensor q = unpacked_bf(saved[0], dout, {n, 3 * dims[2] * dims[4]}), out = unpacked_bf(saved[1], dout, {n, dims[2] * dims[4]}),
-                 lse = unpacked_f32(saved[2], dout, {dims[0], dims[2], dims[1]}), cos = unpacked_f32(saved[3], dout, {dims[6], dims[4] / 2}),
-                 sin = unpacked_f32(saved[4], dout, {dims[7], dims[4] / 2});
+                 lse = unpacked_f32(saved[2], dout, {dims[0], dims[2], dims[1]}), cos = unpacked_f32(saved[3], dout, {dims[5], dims[4] / 2}),
+                 sin = unpacked_f32(saved[4], dout, {dims[6], dims[4] / 2});
     const St st = stream();
     Tensor dqkv = at::empty_like(q), part;
     const Tensor delta = f32(q, {n * h.H});
     const long bytes = h.hd == 64 ? K.mlb_attn_bwd_scratch_bytes(h.B, h.T, h.H, h.hd) : 0;
-    if (bytes > 0 && bytes <= dims[5]) part = at::empty({bytes / 2}, q.options());
+    if (scratch_allowed(bytes)) part = at::empty({bytes / 2}, q.options());
     const int rc = K.mlb_attn_bwd(dqkv.data_ptr(), dout.data_ptr(), q.data_ptr(), out.data_ptr(), (const float*)lse.data_ptr(), (float*)delta.data_ptr(),
                                   part.defined() ? part.data_ptr() : nullptr, h.B, h.T, h.H, h.hd, (const float*)cos.data_ptr(),
                                   (const float*)sin.data_ptr(), st);
@@ -308,7 +317,7 @@ struct CausalFn : torch::autograd::Function<CausalFn> {
       check(K.mlb_kv_group_sum(grouped.data_ptr(), dqkv.data_ptr(), n, h.H, h.Hkv, h.hd, st), "kv_group_sum");
       dqkv = grouped;
     }
-    return {dqkv.view(ctx->saved_data["shape"].toIntVector()), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+    return {dqkv.view(ctx->saved_data["shape"].toIntVector()), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
   }
 };
 struct Seen { Tensor q, out, lse; };
@@ -415,15 +424,14 @@ PyObject* py_swiglu(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return released([&] { return wants_grad({&gu}) ? SwiGLUFn::apply(gu) : swiglu_forward(gu); });
   END_HANDLE_TH_ERRORS
 }
-// (qkv, cos, sin, B, T, H, hd, Hkv or None, bytes of dQ partials the fused backward may use)
+// (qkv, cos, sin, B, T, H, hd, Hkv or None)
 PyObject* py_rope_causal_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   Tensor qkv, cos, sin;
   long B, T, H, hd, Hkv;
-  if (n != 9 || transformed() || !plain_bf(a[0], qkv, 2) || !plain(a[1], cos, at::kFloat, 2) || !plain(a[2], sin, at::kFloat, 2) || !int_arg(a[3], B) || !int_arg(a[4], T) ||
-      !int_arg(a[5], H) || !int_arg(a[6], hd) || !PyLong_CheckExact(a[8]))
+  if (n != 8 || transformed() || !plain_bf(a[0], qkv, 2) || !plain(a[1], cos, at::kFloat, 2) || !plain(a[2], sin, at::kFloat, 2) || !int_arg(a[3], B) || !int_arg(a[4], T) ||
+      !int_arg(a[5], H) || !int_arg(a[6], hd))
     return declined();
-  const long part = PyLong_AsLong(a[8]);
   if (a[7] == Py_None) Hkv = H;
   else if (!int_arg(a[7], Hkv)) return declined();
   if (B < 1 || T < 1 || H < 1 || Hkv < 1 || H % Hkv != 0 || hd % 16 != 0 || hd > 128 || hd < 16) return declined();
@@ -433,7 +441,7 @@ PyObject* py_rope_causal_attention(PyObject*, PyObject* const* a, Py_ssize_t n) 
       cos.requires_grad() || sin.requires_grad())
     return declined();
   return released([&] {
-    if (wants_grad({&qkv})) return CausalFn::apply(qkv, cos, sin, B, T, H, Hkv, hd, part);
+    if (wants_grad({&qkv})) return CausalFn::apply(qkv, cos, sin, B, T, H, Hkv, hd);
     return causal_forward(qkv.contiguous(), cos, sin, Heads{(int)B, (int)T, (int)H, (int)Hkv, (int)hd}).out;
   });
   END_HANDLE_TH_ERRORS
@@ -524,17 +532,21 @@ template <typename R, typename... A> struct typed_call<R(A...)> {
   }
 MLB_ENTRIES(MLB_CALL)
 
-// bind(path): the kernel library whose functions are called
-PyObject* py_bind(PyObject*, PyObject* path) {
+// bind(path, settings): the kernel library whose functions are called, the module with the variables above
+PyObject* py_bind(PyObject*, PyObject* args) {
   HANDLE_TH_ERRORS
-  const char* p = PyUnicode_AsUTF8(path);
-  if (!p) return nullptr;
+  const char* p = nullptr;
+  PyObject* module = nullptr;
+  if (!PyArg_ParseTuple(args, "sO", &p, &module)) return nullptr;
   void* h = dlopen(p, RTLD_NOW);
   TORCH_CHECK(h != nullptr, "cannot load ", p, ": ", dlerror());
 #define MLB_LOOKUP(name, ret, args)                                  \
   K.name = (ret(*) args)dlsym(h, #name);                             \
   TORCH_CHECK(K.name != nullptr, p, " has no function " #name);
   MLB_ENTRIES(MLB_LOOKUP)
+  Py_INCREF(module);
+  Py_XDECREF(settings);
+  settings = module;
   Py_RETURN_NONE;
   END_HANDLE_TH_ERRORS
 }
@@ -542,7 +554,7 @@ PyObject* py_bind(PyObject*, PyObject* path) {
 #define MLB_FAST(name) {#name, (PyCFunction)(void (*)(void))py_##name, METH_FASTCALL, nullptr}
 #define MLB_METHOD(name, ret, args) {#name, (PyCFunction)(void (*)(void))call_##name, METH_FASTCALL, nullptr},
 PyMethodDef methods[] = {MLB_FAST(linear), MLB_FAST(rmsnorm), MLB_FAST(layer_norm), MLB_FAST(swiglu), MLB_FAST(rope_causal_attention), MLB_FAST(bidir_attention),
-                         MLB_FAST(cross_entropy), MLB_ENTRIES(MLB_METHOD) {"bind", py_bind, METH_O, nullptr}, {nullptr, nullptr, 0, nullptr}};
+                         MLB_FAST(cross_entropy), MLB_ENTRIES(MLB_METHOD) {"bind", py_bind, METH_VARARGS, nullptr}, {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "mlb_torch", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

@@ -233,12 +233,8 @@ def swiglu(gu):
 
 
 def rope_causal_attention(qkv, cos, sin, B, T, H, hd, Hkv=None):
-    if getattr(qkv, "is_cuda", False):
-        nat = ops.native_module()
-        y = _plain("rope_causal_attention", qkv, cos, sin, B, T, H, hd, Hkv, nat.FUSED_ATTN_BWD_MAX_SCRATCH if nat.FUSED_ATTN_BWD else 0)
-        if y is not NotImplemented:
-            return y
-    return RopeCausalAttention.apply(qkv, cos, sin, B, T, H, hd, Hkv)
+    y = _plain("rope_causal_attention", qkv, cos, sin, B, T, H, hd, Hkv)
+    return RopeCausalAttention.apply(qkv, cos, sin, B, T, H, hd, Hkv) if y is NotImplemented else y
 
 
 def cross_entropy(logits, tgt):

@@ -10,6 +10,7 @@ import ctypes as C
 import importlib.util
 import os
 import subprocess
+import sys
 import threading
 import warnings
 from functools import lru_cache
@@ -137,7 +138,7 @@ def bridge():
     spec = importlib.util.spec_from_file_location("mlb_torch", str(path))
     m = importlib.util.module_from_spec(spec)
     spec.loader.exec_module(m)
-    m.bind(str(_build.external_lib("libmlb_cuda.so") or _build.CUDA_LIB))
+    m.bind(str(_build.external_lib("libmlb_cuda.so") or _build.CUDA_LIB), sys.modules[__name__])
     return m
 
 

@@ -1559,3 +1559,38 @@ def test_transforms_and_modes_take_the_functions(name):
     assert torch.equal(got, want) and any("new_empty" in o for o in seen.ops)      # (the module allocates without the dispatcher's modes looking on)
     graph = torch.jit.trace(lambda *a: call(*a), tuple(ops_), check_trace=False).graph
     assert any(n.kind() == "prim::PythonOp" for n in graph.nodes()), graph
+
+
+@pytest.mark.parametrize("native", [True, False])
+def test_workspace_of_the_attention_backward_is_bounded_when_it_runs(native, monkeypatch):
+    """FUSED_ATTN_BWD and FUSED_ATTN_BWD_MAX_SCRATCH hold at the time of backward, whatever they were in forward, and take any number: through the
+    extension module as through the Function."""
+    from ml_b200.ops import autograd as F
+    B, T, H, hd, n = 1, 2048, 4, 64, nat()
+    cos, sin = ref.rope_tables(T, hd, 10000.0, dev())
+    x, dout = rnd(B * T, 3 * H * hd).requires_grad_(True), rnd(B * T, H * hd)
+    need = n.lib().mlb_attn_bwd_scratch_bytes(B, T, H, hd)
+    torch.autograd.grad(F.RopeCausalAttention.apply(x, cos, sin, B, T, H, hd, None), x, dout)
+
+    def backward(**late):
+        with monkeypatch.context() as mp:
+            y = F.rope_causal_attention(x, cos, sin, B, T, H, hd) if native else F.RopeCausalAttention.apply(x, cos, sin, B, T, H, hd, None)
+            assert _native(y) == native
+            for k, v in late.items():
+                mp.setattr(n, k, v)
+            torch.cuda.synchronize()
+            torch.cuda.reset_peak_memory_stats()
+            before = torch.cuda.memory_allocated()
+            g, = torch.autograd.grad(y, x, dout)
+            return g, torch.cuda.max_memory_allocated() - before
+
+    fused, most = backward()
+    apart, least = backward(FUSED_ATTN_BWD=False)
+    assert need > 8 << 20 and least < most - need // 2      # (what else comes and goes meanwhile is smaller than that)
+    for limit, fits in ((need, True), (need - 1, False), (1 << 70, True), (float("inf"), True), (-(1 << 70), False)):
+        g, used = backward(FUSED_ATTN_BWD_MAX_SCRATCH=limit)
+        assert torch.equal(g, fused if fits else apart) and (used > most - need // 2) == fits, limit
+    with monkeypatch.context() as mp:      # (in forward it asks for nothing)
+        mp.setattr(n, "FUSED_ATTN_BWD_MAX_SCRATCH", 1 << 70)
+        y = F.rope_causal_attention(x, cos, sin, B, T, H, hd)
+    assert torch.equal(torch.autograd.grad(y, x, dout)[0], fused)
