@@ -176,17 +176,12 @@ class CrossEntropy(torch.autograd.Function):
         ops.ce_mean(loss, losses, grad, logits, tgt)
         if grad is not None:
             ctx.save_for_backward(grad)
-            # a pack hook may have kept the tensor itself: then it is not this node's alone
-            ctx.shared = torch._C._autograd._top_saved_tensors_default_hooks(False) is not None
         return loss
 
     @staticmethod
     def backward(ctx, g):
         (dlogits,) = ctx.saved_tensors
-        # The last use of the saved gradient (the graph is not kept for another pass): scaled in place and handed out, and not even
-        # read when the factor is one.
-        last = not ctx.shared and not torch._C._autograd._get_current_graph_task_keep_graph()
-        out = dlogits if last else _like(dlogits, *dlogits.shape)
+        out = _like(dlogits, *dlogits.shape)      # (not in place: a program can get at a Python node's saved tensors, or put a hook on them)
         ops.scale_dev(out, dlogits, g.float().contiguous())
         return out, None
 

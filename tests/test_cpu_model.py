@@ -469,3 +469,22 @@ def test_export_to_the_hugging_face_llama_layout(tmp_path):
     assert torch.equal(export.from_hf_state_dict(cfg, hf.state_dict()), g.master)
     with pytest.raises(ValueError, match="where the configuration needs"):
         export.from_hf_state_dict(Config(V=97, C=48, L=2, H=4, I=96, T=16), hf.state_dict())
+
+
+def test_saved_gradient_of_the_cross_entropy_stays_as_it_is():
+    """A program can read a Python node's saved tensors and put hooks on them: backward leaves both as they are."""
+    from ml_b200.ops import autograd as A
+    torch.manual_seed(0)
+    z, tgt = torch.randn(6, 8, dtype=torch.bfloat16, requires_grad=True), torch.arange(6, dtype=torch.int32)
+
+    def hooked(node):
+        held = []
+        node._raw_saved_tensors[0].register_hooks(lambda t: held.append(t) or t, lambda t: t)
+        return held[0]
+
+    for read in (lambda node: node.saved_tensors[0], hooked):
+        loss = A.cross_entropy(z, tgt)
+        seen = read(loss.grad_fn)
+        before = seen.clone()
+        g, = torch.autograd.grad(loss * 0.37, z)
+        assert torch.equal(seen, before) and torch.equal(g, (before.float() * 0.37).bfloat16())
