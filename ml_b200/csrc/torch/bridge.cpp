@@ -44,6 +44,7 @@ typedef std::optional<Tensor> Maybe;      // (an undefined tensor is no argument
   X(mlb_gemm, int, (void*, const void*, const void*, int, int, int, int, int, int, int, int, int, St))                                         \
   X(mlb_gemm_dw_direct, int, (int, int, int))                                                                                                  \
   X(mlb_linear_fwd_fp8, int, (void*, const uint8_t*, const uint8_t*, int, int, int, int, int, int, float, St))                                 \
+  X(mlb_capture_id, unsigned long long, (St))                                                                                                  \
   X(mlb_zero, int, (void*, long, St))                                                                                                          \
   X(mlb_cast_f2b, int, (void*, const float*, long, float, St))                                                                                 \
   X(mlb_colsum_splits, int, (long, int))                                                                                                       \
@@ -363,12 +364,17 @@ struct CrossEntropyFn : torch::autograd::Function<CrossEntropyFn> {
     const Crossed r = ce_forward(logits.contiguous(), tgt, true);
     ctx->save_for_backward({r.grad});
     ctx->saved_data["shape"] = logits.sizes().vec();
-    ctx->saved_data["shared"] = at::SavedTensorDefaultHooks::get_hooks().has_value();      // (see ops/autograd.py)
+    ctx->saved_data["shared"] = at::SavedTensorDefaultHooks::get_hooks().has_value();
+    ctx->saved_data["capture"] = (int64_t)K.mlb_capture_id(stream());
     return r.loss;
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     const Tensor d = unpacked_bf(ctx->get_saved_variables()[0], g[0], ctx->saved_data["shape"].toIntVector());
-    const bool last = !ctx->saved_data["shared"].toBool() && !torch::autograd::get_current_graph_task_keep_graph();
+    // The last use of the saved gradient: scaled in place and handed out, and not even read when the factor is one.  Not when the graph
+    // is kept for another pass, when a pack hook may hold the tensor itself, or when one of forward and backward is captured without the
+    // other: then a replay of the backward is another pass.
+    const bool last = !ctx->saved_data["shared"].toBool() && !torch::autograd::get_current_graph_task_keep_graph() &&
+                      ctx->saved_data["capture"].toInt() == (int64_t)K.mlb_capture_id(stream());
     Tensor out = last ? d : at::empty_like(d);
     const Tensor s = g[0].to(at::kFloat).contiguous();
     check(K.mlb_scale_dev(out.data_ptr(), d.data_ptr(), (const float*)s.data_ptr(), out.numel(), stream()), "scale_dev");

@@ -266,7 +266,7 @@ def _i(t, name="tensor"):
 _KINDS = {
     "linear_fwd": "bbbnnnnnns", "linear_fwd_posembed": "bbbbnnnnnnns", "linear_fwd_rope": "bbbnnnnnnffnns", "linear_fwd_swiglu": "bbbbnnnnnns",
     "linear_dx": "bbbnnnnnns", "linear_dx_delta": "bbbbfnnnnnnnns", "linear_dw": "fbbnnnnnns", "gemm": "bbbnnnnnnnnns", "gemm_dw_direct": "nnn",
-    "linear_fwd_fp8": "buunnnnnnns", "zero": "bns", "cast_f2b": "bfnns", "colsum_splits": "nn", "colsum": "bbnnfs", "rmsnorm_fwd": "bfbbnnns",
+    "linear_fwd_fp8": "buunnnnnnns", "capture_id": "s", "zero": "bns", "cast_f2b": "bfnns", "colsum_splits": "nn", "colsum": "bbnnfs", "rmsnorm_fwd": "bfbbnnns",
     "add_rmsnorm_fwd": "bbfbbbnnns", "rmsnorm_fwd_fp8": "bufbbnnnns", "rmsnorm_bwd_blocks": "n", "rmsnorm_bwd": "bfbbbfbnnfis",
     "rmsnorm_bwd_cast": "bbbbbfbnnfs", "layernorm_fwd": "bffbbbnnns", "layernorm_bwd2": "bbbnbbbffnnfs", "swiglu_fwd": "bbnns",
     "swiglu_fwd_fp8": "bubnnns", "swiglu_bwd": "bbbnns", "rope": "bffnnnnns", "rope_copy": "bbffnnnnns", "kv_group_sum": "bbnnnns",

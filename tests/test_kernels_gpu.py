@@ -1594,3 +1594,32 @@ def test_workspace_of_the_attention_backward_is_bounded_when_it_runs(native, mon
         mp.setattr(n, "FUSED_ATTN_BWD_MAX_SCRATCH", 1 << 70)
         y = F.rope_causal_attention(x, cos, sin, B, T, H, hd)
     assert torch.equal(torch.autograd.grad(y, x, dout)[0], fused)
+
+
+@pytest.mark.parametrize("together", [False, True])
+@pytest.mark.parametrize("factor", [1.0, 0.37])
+def test_cross_entropy_backward_replayed(together, factor):
+    """A captured backward gives the same gradient at each of its replays, behind one replay of its forward; captured with its forward it does
+    so too."""
+    from ml_b200.ops import autograd as F
+    torch.manual_seed(1)
+    z, tgt = rnd(37, 264, scale=2.0).requires_grad_(True), torch.randint(0, 264, (37,), device=dev(), dtype=torch.int32)
+    want, = torch.autograd.grad(F.cross_entropy(z, tgt) * factor, z)
+    fwd, bwd, s = torch.cuda.CUDAGraph(), torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        torch.autograd.grad(F.cross_entropy(z, tgt) * factor, z)
+        with torch.cuda.graph(fwd, stream=s):
+            loss = F.cross_entropy(z, tgt) * factor
+            if together:
+                g, = torch.autograd.grad(loss, z)
+        if not together:
+            with torch.cuda.graph(bwd, pool=fwd.pool(), stream=s):
+                g, = torch.autograd.grad(loss, z)
+    torch.cuda.current_stream().wait_stream(s)
+    for _ in range(2):
+        fwd.replay()
+        for _ in range(1 if together else 3):
+            if not together:
+                bwd.replay()
+            assert torch.equal(g, want)
