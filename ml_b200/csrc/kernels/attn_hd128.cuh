@@ -511,8 +511,8 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
           nl[x] = q < a.T ? a.lse[e + q] * LOG2E : INFINITY;
           nd[x] = q < a.T ? a.delta[e + q] : 0.f;
         }
-        if (g >= 2 && !wait(&bar_stf[g & 1], ((g >> 1) + 1) & 1, 63)) { ok = false; break; }
-        __syncwarp();
+        // (one answer for the warp: a lane whose wait has run out must not leave those behind whose wait has not)
+        if (g >= 2 && !__all_sync(0xffffffffu, wait(&bar_stf[g & 1], ((g >> 1) + 1) & 1, 63))) { ok = false; break; }
         float* stat = (float*)(smem + S::STAT + (g & 1) * 1024);
 #pragma unroll
         for (int x = 0; x < 4; x++) {
