@@ -50,8 +50,9 @@ __device__ __forceinline__ void mlb_pdl_sync() {
 #ifdef __CUDACC__
 #include <cstdlib>
 #include <utility>
-// Which kernels start early, without MLB_PDL: all GEMMs, attention kernels of one wave, and element-wise kernels of one wave (at most as many
-// threads as the machine holds).  A chain of small kernels is bound by launch and set-up, which then run under the kernel before: step of
+// Which kernels start early, without MLB_PDL: all GEMMs, the persistent attention kernels of one wave (no more items than SMs), the split attention
+// kernels up to a limit of their own (split_early), and element-wise kernels of no more threads than the machine holds (2048 an SM: one
+// wave, or two where a kernel's registers allow half as many).  A chain of small kernels is bound by launch and set-up, which then run under the kernel before: step of
 // the 4-layer / 128-wide decoder 637 -> 567 us, attention forward of a few thousand tokens 13.3 -> 10.4; GEMMs of any size gain 2 to 3 us of
 // launch gap each (step of the 12-layer decoder 17.35 -> 17.11 ms, captured 16.40 -> 16.29).
 // Larger ones stay out: their CTAs sit on the SMs while the kernel before still works there, and take registers and issue slots from
@@ -68,7 +69,14 @@ inline int mlb_pdl_mode() {
   }
   return mode;
 }
-constexpr long MLB_WAVE_THREADS = 148L * 2048;
+inline int mlb_sm_count() {
+  static const int n = [] {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) cudaGetLastError();
+    return sms > 0 ? sms : 148;
+  }();
+  return n;
+}
 template <typename... KArgs, typename... Args>
 inline cudaError_t mlb_launch_attr(bool early, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
@@ -86,7 +94,7 @@ inline cudaError_t mlb_launch_attr(bool early, void (*kern)(KArgs...), dim3 grid
 template <typename... KArgs, typename... Args>
 inline cudaError_t mlb_launch(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
   const int mode = mlb_pdl_mode();
-  const bool early = mode == MLB_PDL_BY_SIZE ? (long)grid.x * grid.y * grid.z * block.x <= MLB_WAVE_THREADS : mode != MLB_PDL_NONE;
+  const bool early = mode == MLB_PDL_BY_SIZE ? (long)grid.x * grid.y * grid.z * block.x <= 2048L * mlb_sm_count() : mode != MLB_PDL_NONE;
   return mlb_launch_attr(early, kern, grid, block, smem, st, std::forward<Args>(args)...);
 }
 // for kernels that allocate tensor memory (GEMMs, attention): `small`, of those that start early by size

@@ -549,13 +549,17 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
   if (again.x | again.y | again.z | again.w) split_redo<KV ? 1 : 2>(again, a, r0, h, b, (float*)smem);
 }
 
-// (small enough to start under the kernel before; two to four CTAs fit an SM)
-static bool split_wave(const SplitArgs& a) { return (long)((a.T + 127) / 128) * a.H * a.B <= 8 * 148; }
+// Do the kernels start under the one before them?  Four CTAs of the forward fit an SM at head sizes up to 64, two of the backward (at 128: two and
+// one), so the limit is two to eight waves.  It is where the gain has become small, not where something gets slower: forward + backward without a
+// mask, 197 tokens, 12 heads of 64, us apart and early: 0.6 CTAs per SM 43.1 and 38.3, 2.6 73.6 and 64.5, 5.2 114.6 and 107.7, 7.8 162.8 and
+// 156.7, 10 212.9 and 207.7, 21 383.9 and 377.7.  Slower where the backward's CTAs are just short of one wave, which the early ones
+// take up unevenly (1.9: 51.2 and 53.0; 577 tokens, 1.6: 96.7 and 107.0).
+static bool split_early(const SplitArgs& a) { return (long)((a.T + 127) / 128) * a.H * a.B <= 8L * mlb_sm_count(); }
 template <int HDT>
 static int split_fwd_launch(const CUtensorMap* tm, const SplitArgs& a, cudaStream_t st) {
   static int once = (int)cudaFuncSetAttribute(attn_split_fwd_k<HDT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitFwdSmem<HDT>::TOTAL);
   if (once) return once;
-  mlb_launch_tmem(split_wave(a), attn_split_fwd_k<HDT>, dim3((a.T + 127) / 128, a.H, a.B), dim3(SPLIT_THREADS), SplitFwdSmem<HDT>::TOTAL, st, *tm, a);
+  mlb_launch_tmem(split_early(a), attn_split_fwd_k<HDT>, dim3((a.T + 127) / 128, a.H, a.B), dim3(SPLIT_THREADS), SplitFwdSmem<HDT>::TOTAL, st, *tm, a);
   return (int)cudaGetLastError();
 }
 template <int HDT>
@@ -564,8 +568,8 @@ static int split_bwd_launch(const CUtensorMap* tm, const CUtensorMap* td, const 
                     (int)cudaFuncSetAttribute(attn_split_bwd_k<HDT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitBwdSmem<HDT, false>::TOTAL);
   if (once) return once;
   const dim3 grid((a.T + 127) / 128, a.H, a.B);
-  mlb_launch_tmem(split_wave(a), attn_split_bwd_k<HDT, true>, grid, dim3(SPLIT_THREADS), SplitBwdSmem<HDT, true>::TOTAL, st, *tm, *td, a);
-  mlb_launch_tmem(split_wave(a), attn_split_bwd_k<HDT, false>, grid, dim3(SPLIT_THREADS), SplitBwdSmem<HDT, false>::TOTAL, st, *tm, *td, a);
+  mlb_launch_tmem(split_early(a), attn_split_bwd_k<HDT, true>, grid, dim3(SPLIT_THREADS), SplitBwdSmem<HDT, true>::TOTAL, st, *tm, *td, a);
+  mlb_launch_tmem(split_early(a), attn_split_bwd_k<HDT, false>, grid, dim3(SPLIT_THREADS), SplitBwdSmem<HDT, false>::TOTAL, st, *tm, *td, a);
   return (int)cudaGetLastError();
 }
 

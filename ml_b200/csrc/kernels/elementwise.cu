@@ -1597,20 +1597,11 @@ MLB_API int mlb_ce_mean(float* loss, float* losses, float* stats, void* dlogits,
   }
   LAUNCH_RET;
 }
-static long sm_count() {
-  static int n = 0;
-  if (n <= 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) { cudaGetLastError(); n = 148; }
-  }
-  return n;
-}
 // out == x: in place, and no pass at all when the factor turns out to be one
 MLB_API int mlb_scale_dev(void* out, const void* x, const float* s, long n, cudaStream_t st) {
   if (((uintptr_t)out | (uintptr_t)x) & 15) return -7;
   if (n > 0 && out == x) {
-    mlb_launch(scale_dev_inplace_k, dim3((unsigned)std::min((n + 4095) / 4096, 8L * sm_count())), dim3(256), 0, st, (bf16*)out, s, n);
+    mlb_launch(scale_dev_inplace_k, dim3((unsigned)std::min((n + 4095) / 4096, 8L * mlb_sm_count())), dim3(256), 0, st, (bf16*)out, s, n);
     LAUNCH_RET;
   }
   if (n > 0) mlb_launch(scale_dev_k, dim3((unsigned)((n + 4095) / 4096)), dim3(256), 0, st, (bf16*)out, (const bf16*)x, s, n);

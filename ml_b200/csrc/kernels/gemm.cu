@@ -1060,16 +1060,7 @@ namespace {
 
 int g_sk_whole = 1;          // tuning hook: 0 = stream-K cuts up all tiles, not only those of the last, partial wave
 int g_use_3d = 1;            // tuning hook: 0 = always use 64-wide 2-D boxes for MN-major operands
-int g_num_sms = 0;
-int num_sms() {
-  if (!g_num_sms) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
-    if (g_num_sms <= 0) g_num_sms = 148;
-  }
-  return g_num_sms;
-}
+int num_sms() { return mlb_sm_count(); }
 
 int g_force_simt = 0;        // test hook: route everything through the SIMT kernel
 int g_max_ctas = 0;          // 0 = one CTA per SM; >0 caps the persistent grid (leaves SMs to a concurrent kernel)
