@@ -1442,6 +1442,7 @@ MLB_API int mlb_layernorm_fwd(void* out, float* mean, float* rstd, const void* x
     case 4: LN(4); break;
     case 5: LN(5); break;
     case 6: LN(6); break;
+    case 7: LN(7); break;
     case 8: LN(8); break;
     default: LN(0); break;
   }
