@@ -128,17 +128,16 @@ def lib():
 @lru_cache(maxsize=1)
 def bridge():
     """The operators' host path as an extension module on this library's kernels (csrc/torch/bridge.cpp), or None where it cannot be
-    built for this torch: ops/autograd.py and the functions below then call the same kernels from Python."""
+    built or loaded with this torch: ops/autograd.py and the functions below then call the same kernels from Python."""
     lib()
     try:
-        path = _build.build_torch()
-    except (OSError, subprocess.CalledProcessError) as e:
-        warnings.warn(f"libmlb_torch.so cannot be built ({e}): operators run through Python, several times slower per call")
+        spec = importlib.util.spec_from_file_location("mlb_torch", str(_build.build_torch()))
+        m = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(m)
+        m.bind(str(_build.external_lib("libmlb_cuda.so") or _build.CUDA_LIB), sys.modules[__name__])
+    except (OSError, subprocess.CalledProcessError, ImportError, RuntimeError) as e:      # (ImportError: another torch's; RuntimeError: bind)
+        warnings.warn(f"libmlb_torch.so cannot be built or loaded ({e}): operators run through Python, several times slower per call")
         return None
-    spec = importlib.util.spec_from_file_location("mlb_torch", str(path))
-    m = importlib.util.module_from_spec(spec)
-    spec.loader.exec_module(m)
-    m.bind(str(_build.external_lib("libmlb_cuda.so") or _build.CUDA_LIB), sys.modules[__name__])
     return m
 
 

@@ -581,3 +581,24 @@ def test_scratch_belongs_to_one_thread_stream_and_capture(monkeypatch):
     t.join()
     assert other[0] is not mine and get() is mine
     assert get(n=9).numel() == 9
+
+
+@pytest.mark.parametrize("failure", ["not built", "not a library", "not this kernel library"])
+def test_an_extension_module_that_cannot_be_used_is_done_without(failure, tmp_path, monkeypatch):
+    """The operators then run through Python, with a warning, whatever the reason."""
+    import subprocess
+    from ml_b200 import build
+    from ml_b200.ops import native
+    if failure == "not built":
+        def none():
+            raise subprocess.CalledProcessError(1, "g++")
+        monkeypatch.setattr(build, "build_torch", none)
+    elif failure == "not a library":
+        (tmp_path / "libmlb_torch.so").write_text("?")
+        monkeypatch.setattr(build, "build_torch", lambda: tmp_path / "libmlb_torch.so")
+    else:
+        monkeypatch.setattr(native, "lib", lambda: None)
+        monkeypatch.setattr(build, "external_lib", lambda name: build.build_host())
+    with pytest.warns(UserWarning, match="cannot be built or loaded"):
+        assert native.bridge.__wrapped__() is None
+    assert isinstance(native._Ctypes(), native._Ctypes)
