@@ -510,6 +510,14 @@ template <> struct Arg<float> {
     return (float)v;
   }
 };
+// An entry point's parameters, a letter each (see _KINDS in ops/native.py)
+template <typename T> constexpr char kind_of() {
+  using P = std::remove_cv_t<std::remove_pointer_t<T>>;
+  if constexpr (std::is_same_v<T, St>) return 's';
+  else if constexpr (std::is_pointer_v<T>) return std::is_same_v<P, void> ? 'b' : std::is_same_v<P, float> ? 'f' : std::is_same_v<P, int> ? 'i' : 'u';
+  else return std::is_same_v<T, float> ? 'd' : std::is_same_v<T, long> ? 'l' : 'n';
+}
+template <typename R, typename... A> std::string kinds_of(R (*)(A...)) { return {kind_of<A>()...}; }
 template <typename R, typename... A, size_t... I>
 PyObject* call_entry(R (*f)(A...), PyObject* const* a, Py_ssize_t n, std::index_sequence<I...>) {
   constexpr bool streamed = std::is_same_v<std::tuple_element_t<sizeof...(A) - 1, std::tuple<A...>>, St>;
@@ -557,10 +565,20 @@ PyObject* py_bind(PyObject*, PyObject* args) {
   END_HANDLE_TH_ERRORS
 }
 
+// signatures(): every entry point's parameters by name
+PyObject* py_signatures(PyObject*, PyObject*) {
+  HANDLE_TH_ERRORS
+  pybind11::dict d;
+#define MLB_KINDS(name, ret, args) d[#name] = kinds_of(K.name);
+  MLB_ENTRIES(MLB_KINDS)
+  return d.release().ptr();
+  END_HANDLE_TH_ERRORS
+}
+
 #define MLB_FAST(name) {#name, (PyCFunction)(void (*)(void))py_##name, METH_FASTCALL, nullptr}
 #define MLB_METHOD(name, ret, args) {#name, (PyCFunction)(void (*)(void))call_##name, METH_FASTCALL, nullptr},
 PyMethodDef methods[] = {MLB_FAST(linear), MLB_FAST(rmsnorm), MLB_FAST(layer_norm), MLB_FAST(swiglu), MLB_FAST(rope_causal_attention), MLB_FAST(bidir_attention),
-                         MLB_FAST(cross_entropy), MLB_ENTRIES(MLB_METHOD) {"bind", py_bind, METH_VARARGS, nullptr}, {nullptr, nullptr, 0, nullptr}};
+                         MLB_FAST(cross_entropy), MLB_ENTRIES(MLB_METHOD) {"bind", py_bind, METH_VARARGS, nullptr}, {"signatures", py_signatures, METH_NOARGS, nullptr}, {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "mlb_torch", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

@@ -22,6 +22,22 @@ from .. import build as _build
 _i32, _i64, _f32, _vp = C.c_int, C.c_long, C.c_float, C.c_void_p
 
 
+# Entry points that the extension module has, by the C type of each parameter.  b bf16, f fp32, i int32, u bytes: tensors, or an address as a
+# number (0: none); n int, l long, d float; s the current stream
+_KINDS = {
+    "linear_fwd": "bbbnnnnnns", "linear_fwd_posembed": "bbbbnnnnnnns", "linear_fwd_rope": "bbbnnnnnnffnns",
+    "linear_fwd_swiglu": "bbbbnnnnnns", "linear_dx": "bbbnnnnnns", "linear_dx_delta": "bbbbfnnnnnnnns", "linear_dw": "fbbnnnnnns",
+    "gemm": "bbbnnnnnnnnns", "gemm_dw_direct": "nnn", "linear_fwd_fp8": "buunnnnnnds", "capture_id": "s", "zero": "bls",
+    "cast_f2b": "bflds", "colsum_splits": "ln", "colsum": "bblnfs", "rmsnorm_fwd": "bfbblnds", "add_rmsnorm_fwd": "bbfbbblnds",
+    "rmsnorm_fwd_fp8": "bufbblndds", "rmsnorm_bwd_blocks": "l", "rmsnorm_bwd": "bfbbbfblnfis", "rmsnorm_bwd_cast": "bbbbbfblnfs",
+    "layernorm_fwd": "bffbbblnds", "layernorm_bwd2": "bbbnbbbfflnfs", "swiglu_fwd": "bblns", "swiglu_fwd_fp8": "bublnds",
+    "swiglu_bwd": "bbblns", "rope": "bfflnnnds", "rope_copy": "bbfflnnnns", "kv_group_sum": "bblnnns", "attn_fwd": "bfbnnnns",
+    "attn_bwd_scratch_bytes": "nnnn", "attn_bwd": "bbbbffbnnnnffs", "attn_bwd_have_delta": "bbbbffbnnnnffs",
+    "attn_bidir_fwd": "bfbnnnns", "attn_bidir_bwd": "bbbbffnnnns", "ce_mean": "fffbbilns", "ce_fwd_bwd": "fbilnldns",
+    "scale_dev": "bbfls", "embed_fwd": "bbilnns", "embed_bwd": "fbilnnnns", "adamw": "fbffflddddddddfs", "sum_scale": "fflds"}
+_CTYPES = {"n": _i32, "l": _i64, "d": _f32}      # (else a pointer)
+
+
 @lru_cache(maxsize=1)
 def lib():
     ext = _build.external_lib("libmlb_cuda.so")
@@ -32,11 +48,6 @@ def lib():
             _build.build_cuda()
     L = C.CDLL(str(ext or _build.CUDA_LIB))
     sig = {
-        "mlb_linear_fwd": [_vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _vp],
-        "mlb_linear_dx": [_vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _vp],
-        "mlb_linear_dw": [_vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _vp],
-        "mlb_gemm": [_vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _vp],
-        "mlb_gemm_dw_direct": [_i32, _i32, _i32],
         "mlb_gemm_force_simt": [_i32],
         "mlb_gemm_set_max_ctas": [_i32],
         "mlb_gemm_set_splits": [_i32],
@@ -50,68 +61,31 @@ def lib():
         "mlb_attn_fwd_mode": [_i32],
         "mlb_attn_fwd_balance": [_i32],
         "mlb_ce_mode": [_i32],
-        "mlb_attn_fwd": [_vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp],
-        "mlb_attn_bwd": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp, _vp, _vp],
-        "mlb_attn_bwd_scratch_bytes": [_i32, _i32, _i32, _i32],
-        "mlb_embed_fwd": [_vp, _vp, _vp, _i64, _i32, _i32, _vp],
-        "mlb_embed_bwd": [_vp, _vp, _vp, _i64, _i32, _i32, _i32, _i32, _vp],
         "mlb_set_prefix": [_vp, _vp, _i32, _i32, _i32, _i32, _vp],
         "mlb_gather_prefix_grad": [_vp, _vp, _i32, _i32, _i32, _i32, _vp],
-        "mlb_rmsnorm_fwd": [_vp, _vp, _vp, _vp, _i64, _i32, _f32, _vp],
-        "mlb_add_rmsnorm_fwd": [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i32, _f32, _vp],
-        "mlb_rmsnorm_bwd_blocks": [_i64],
-        "mlb_rmsnorm_bwd": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i32, _vp, _vp, _vp],
-        "mlb_rope": [_vp, _vp, _vp, _i64, _i32, _i32, _i32, _f32, _vp],
-        "mlb_rmsnorm_bwd_cast": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i32, _vp, _vp],
-        "mlb_layernorm_bwd2": [_vp, _vp, _vp, _i32, _vp, _vp, _vp, _vp, _vp, _i64, _i32, _vp, _vp],
-        "mlb_colsum_splits": [_i64, _i32],
-        "mlb_colsum": [_vp, _vp, _i64, _i32, _vp, _vp],
-        "mlb_rope_copy": [_vp, _vp, _vp, _vp, _i64, _i32, _i32, _i32, _i32, _vp],
-        "mlb_kv_group_sum": [_vp, _vp, _i64, _i32, _i32, _i32, _vp],
-        "mlb_swiglu_fwd": [_vp, _vp, _i64, _i32, _vp],
-        "mlb_swiglu_bwd": [_vp, _vp, _vp, _i64, _i32, _vp],
-        "mlb_ce_fwd_bwd": [_vp, _vp, _vp, _i64, _i32, _i64, _f32, _i32, _vp],
-        "mlb_ce_mean": [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i32, _vp],
-        "mlb_scale_dev": [_vp, _vp, _vp, _i64, _vp],
         "mlb_fp8_qdq": [_vp, _vp, _i64, _f32, _vp],
         "mlb_ce_chunk_stats": [_vp, _vp, _vp, _vp, _vp, _i64, _i32, _i64, _i32, _vp],
         "mlb_ce_chunk_grad": [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i32, _i64, _i32, _f32, _vp],
-        "mlb_adamw": [_vp, _vp, _vp, _vp, _vp, _i64, _f32, _f32, _f32, _f32, _f32, _f32, _f32, _f32, _vp, _vp],
-        "mlb_cast_f2b": [_vp, _vp, _i64, _f32, _vp],
         "mlb_cast_b2f": [_vp, _vp, _i64, _f32, _vp],
         "mlb_scale_f32": [_vp, _i64, _f32, _vp],
         "mlb_residual_add": [_vp, _vp, _vp, _i64, _vp],
         "mlb_patchify": [_vp, _vp, _i32, _i32, _i32, _i32, _i32, _vp],
         "mlb_add_posembed": [_vp, _vp, _i64, _i32, _i32, _vp],
         "mlb_posembed_grad": [_vp, _vp, _i64, _i32, _i32, _vp],
-        "mlb_linear_fwd_rope": [_vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _vp, _vp, _i32, _i32, _vp],
-        "mlb_linear_fwd_swiglu": [_vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _vp],
-        "mlb_linear_fwd_posembed": [_vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _vp],
         "mlb_linear_fwd_gather": [_vp, _vp, _i32, _i32, _i32, _i32, _i32, _vp, _i64, _vp, _i64, _i32, _vp, _vp, C.c_double, _vp],
-        "mlb_linear_dx_delta": [_vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _vp],
-        "mlb_attn_bidir_fwd": [_vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp],
-        "mlb_attn_bidir_bwd": [_vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp],
-        "mlb_layernorm_fwd": [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i32, _f32, _vp],
         "mlb_layernorm_bwd": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i32, _vp],
-        "mlb_linear_fwd_fp8": [_vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _f32, _vp],
         "mlb_linear_fwd_fp8_rope": [_vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _f32, _vp, _vp, _i32, _i32, _vp],
         "mlb_linear_fwd_fp8_swiglu": [_vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _f32, _vp],
-        "mlb_rmsnorm_fwd_fp8": [_vp, _vp, _vp, _vp, _vp, _i64, _i32, _f32, _f32, _vp],
         "mlb_add_rmsnorm_fwd_fp8": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i32, _f32, _f32, _vp],
-        "mlb_swiglu_fwd_fp8": [_vp, _vp, _vp, _i64, _i32, _f32, _vp],
         "mlb_cast_bf16_fp8": [_vp, _vp, _i64, _f32, _vp],
         "mlb_adamw_fp8": [_vp] * 6 + [_i64] + [_f32] * 9 + [_vp, _vp],
-        "mlb_sum_scale": [_vp, _vp, _i64, _f32, _vp],
-        "mlb_zero": [_vp, _i64, _vp],
     }
+    sig.update({"mlb_" + name: [_CTYPES.get(k, _vp) for k in kinds] for name, kinds in _KINDS.items()})
     for name, args in sig.items():
         fn = getattr(L, name)
         fn.argtypes = args
         fn.restype = _i32
-    L.mlb_attn_bwd_have_delta.argtypes = L.mlb_attn_bwd.argtypes
-    L.mlb_attn_bwd_have_delta.restype = _i32
     L.mlb_attn_bwd_scratch_bytes.restype = _i64
-    L.mlb_capture_id.argtypes = [_vp]
     L.mlb_capture_id.restype = C.c_ulonglong
     for tag in ("gemm", "attn", "elementwise", "comm"):
         for pre in ("mlb_get_error_", "mlb_clear_error_"):
@@ -258,20 +232,6 @@ def _f(t, name="tensor"):
 def _i(t, name="tensor"):
     assert t.is_cuda and t.dtype == torch.int32 and t.is_contiguous(), f"{name}: need contiguous CUDA int32"
     return t.data_ptr()
-
-
-# Arguments of the entry points that the extension module has: b bf16, f fp32, i int32, u bytes (tensors, or an address as a number; 0 for
-# none), n a number, s the current stream
-_KINDS = {
-    "linear_fwd": "bbbnnnnnns", "linear_fwd_posembed": "bbbbnnnnnnns", "linear_fwd_rope": "bbbnnnnnnffnns", "linear_fwd_swiglu": "bbbbnnnnnns",
-    "linear_dx": "bbbnnnnnns", "linear_dx_delta": "bbbbfnnnnnnnns", "linear_dw": "fbbnnnnnns", "gemm": "bbbnnnnnnnnns", "gemm_dw_direct": "nnn",
-    "linear_fwd_fp8": "buunnnnnnns", "capture_id": "s", "zero": "bns", "cast_f2b": "bfnns", "colsum_splits": "nn", "colsum": "bbnnfs", "rmsnorm_fwd": "bfbbnnns",
-    "add_rmsnorm_fwd": "bbfbbbnnns", "rmsnorm_fwd_fp8": "bufbbnnnns", "rmsnorm_bwd_blocks": "n", "rmsnorm_bwd": "bfbbbfbnnfis",
-    "rmsnorm_bwd_cast": "bbbbbfbnnfs", "layernorm_fwd": "bffbbbnnns", "layernorm_bwd2": "bbbnbbbffnnfs", "swiglu_fwd": "bbnns",
-    "swiglu_fwd_fp8": "bubnnns", "swiglu_bwd": "bbbnns", "rope": "bffnnnnns", "rope_copy": "bbffnnnnns", "kv_group_sum": "bbnnnns",
-    "attn_fwd": "bfbnnnns", "attn_bwd_scratch_bytes": "nnnn", "attn_bwd": "bbbbffbnnnnffs", "attn_bwd_have_delta": "bbbbffbnnnnffs",
-    "attn_bidir_fwd": "bfbnnnns", "attn_bidir_bwd": "bbbbffnnnns", "ce_mean": "fffbbinns", "ce_fwd_bwd": "fbinnnnns", "scale_dev": "bbfns",
-    "embed_fwd": "bbinnns", "embed_bwd": "fbinnnnns", "adamw": "fbfffnnnnnnnnnfs", "sum_scale": "ffnns"}
 
 
 class _Ctypes:

@@ -583,6 +583,23 @@ def test_scratch_belongs_to_one_thread_stream_and_capture(monkeypatch):
     assert get(n=9).numel() == 9
 
 
+def test_entry_points_have_one_signature():
+    """What ctypes declares, what the extension module calls and what the kernel library's sources define are the same, parameter by parameter."""
+    import re
+    from ml_b200 import build
+    from ml_b200.ops import native
+    assert native.bridge().signatures() == {"mlb_" + k: v for k, v in native._KINDS.items()}
+    letter = {"void*": "p", "bf16*": "b", "float*": "f", "int*": "i", "uint8_t*": "u", "int": "n", "long": "l", "float": "d", "cudaStream_t": "s"}
+    defined = {}
+    for src in (build.CSRC / "kernels").glob("*.cu"):
+        for name, args in re.findall(r"^MLB_API [\w ]+? (mlb_\w+)\(([^)]*)\)", src.read_text(), re.M):
+            types = [re.sub(r"\s*\w+$", "", a.replace("const ", "").strip()).replace(" *", "*") for a in args.split(",")]
+            defined[name] = "".join(letter.get(t, "?") for t in types)
+    for name, kinds in native._KINDS.items():
+        assert len(defined["mlb_" + name]) == len(kinds), name
+        assert all(d == k or (d == "p" and k in "bfiu") for d, k in zip(defined["mlb_" + name], kinds)), name      # (void*: any tensor's)
+
+
 @pytest.mark.parametrize("failure", ["not built", "not a library", "not this kernel library"])
 def test_an_extension_module_that_cannot_be_used_is_done_without(failure, tmp_path, monkeypatch):
     """The operators then run through Python, with a warning, whatever the reason."""

@@ -1329,15 +1329,93 @@ def test_what_the_extension_module_declines():
     assert torch.equal(g, e)
 
 
-def test_entry_points_through_ctypes_and_through_the_module():
-    """The table of argument kinds is the extension module's: one call through each."""
-    n, x, W = nat(), rnd(130, 256), rnd(72, 256)
-    c, m, outs = n._Ctypes(), n.bridge(), [rnd(130, 72), rnd(130, 72)]
-    for e, o in zip((c, m), outs):
-        assert e.mlb_linear_fwd(o, x, W, 130, 72, 256, 72, 256, 256) == 0
+def test_entry_points_through_ctypes_and_through_the_module(monkeypatch):
+    """Every entry point that the extension module has, called through it and through ctypes (all there is where the module cannot be built): the
+    same bits, the same refusals."""
+    n, seen = nat(), set()
+    B, T, H, hd, C, I, V = 2, 192, 4, 64, 256, 384, 512
+    M = B * T
+    cos, sin = ref.rope_tables(T, hd, 10000.0, dev())
+
+    class Spy:
+        def __init__(self, entries):
+            self.entries = entries
+
+        def __getattr__(self, name):
+            seen.add(name)
+            return getattr(self.entries, name)
+
+    def work():
+        torch.manual_seed(0)
+        made = []
+        e = lambda *sh, dtype=torch.bfloat16, fill=0: made.append(torch.full(sh, fill, device=dev(), dtype=dtype)) or made[-1]
+        f32, u8 = dict(dtype=torch.float32), dict(dtype=torch.uint8)
+        x, y, w, b = rnd(M, C), rnd(M, C), rnd(1, C).view(-1), rnd(1, C).view(-1)
+        Wq, Wgu, Wo, dq, dgu = rnd(3 * C, C), rnd(2 * I, C), rnd(C, C), rnd(M, 3 * C), rnd(M, 2 * I)
+        ids = torch.randperm(V, device=dev())[:M].int()
+        n.linear_fwd(e(M, 3 * C), x, Wq)
+        assert n.linear_fwd_posembed(e(M, 3 * C), x, Wq, rnd(7, 3 * C), 7) and n.linear_fwd_rope(e(M, 3 * C), x, Wq, cos, sin, T, 2 * C)
+        assert n.linear_fwd_swiglu(e(M, 2 * I), e(M, I), x, Wgu)
+        n.linear_dx(e(M, C), dq, Wq)
+        n.linear_dw(e(3 * C, C, **f32), dq, x)
+        n.linear_dw_cast(e(3 * C, C), dq, x)
+        n.gemm(e(M, 3 * C), x, Wq)
+        n._entries().mlb_cast_f2b(e(M, C), x.float(), x.numel(), 0.5)
+        n.zero_(e(M, C, fill=1))
+        n.colsum(e(3 * C), dq)
+        n.rmsnorm_fwd(e(M, C), rstd := e(M, **f32), x, w, 1e-5)
+        n.add_rmsnorm_fwd(e(M, C), e(M, C), e(M, **f32), x, y, w, 1e-5)
+        x8 = e(M, C, **u8)
+        n.rmsnorm_fwd_fp8(e(M, C), x8, e(M, **f32), x, w, 1e-5, 1.0)
+        W8 = e(3 * C, C, **u8)
+        n.cast_bf16_fp8(W8, Wq, 16.0)
+        assert n.linear_fwd_fp8(e(M, 3 * C), x8, W8, 1 / 16)
+        n.rmsnorm_bwd(e(M, C), e(C, **f32), y, x, w, rstd, y)
+        n.rmsnorm_bwd_cast(e(M, C), e(C), y, x, w, rstd)
+        n.layernorm_fwd(e(M, C), mean := e(M, **f32), rs := e(M, **f32), x, w, b, 1e-5)
+        n.layernorm_bwd_cast(e(M, C), e(C), e(C), y, x, w, mean, rs)
+        n.swiglu_fwd(e(M, I), dgu)
+        n.swiglu_fwd_fp8(e(M, I), e(M, I, **u8), dgu, 1.0)
+        n.swiglu_bwd(e(M, 2 * I), rnd(M, I), dgu)
+        q = rnd(M, 3 * C)
+        n.rope_fwd(made.append(q.clone()) or made[-1], cos, sin, B, T, H, hd)
+        n.rope_copy(qr := e(M, 3 * C), rnd(M, 2 * C), cos, sin, B, T, H, hd, 2)
+        n.kv_group_sum(e(M, 2 * C), q, B, T, H, hd, 2)
+        n.attn_fwd(o := e(M, C), lse := e(B, H, T, **f32), qr, B, T, H, hd)
+        assert n.linear_dx_delta(do := e(M, C), rnd(M, C), Wo, o, B, T, H)
+        assert n.attn_bwd(e(M, 3 * C), do, qr, o, lse, B, T, H, hd, (cos, sin), have_delta=True)
+        assert n.attn_bwd(e(M, 3 * C), do, qr, o, lse, B, T, H, hd, (cos, sin))
+        n.attn_bidir_fwd(o := e(M, C), lse := e(B, H, T, **f32), qr, B, T, H, hd)
+        n.attn_bidir_bwd(e(M, 3 * C), do, qr, o, lse, B, T, H, hd)
+        n.ce_mean(e(1, **f32), e(M, **f32), e(M, V), z := rnd(M, V), ids)
+        n.ce_fwd_bwd(e(M, **f32), made.append(z.clone()) or made[-1], ids, 0.5)
+        n.scale_dev(e(M, V), z, e(1, fill=0.7, **f32))
+        n.embed_fwd(e(M, C), t := rnd(V, C), ids)
+        n.embed_bwd(e(V, C, **f32), y, ids, T, 0)
+        g = torch.randn(V * C, device=dev())
+        n.adamw(e(V * C, fill=1, **f32), e(V * C), g, e(V * C, **f32), e(V * C, **f32), 1e-3, 0.9, 0.95, 1e-8, 0.1, 0.1, 0.05)
+        n.sum_scale(e(1, **f32), g, 0.25)
         with pytest.raises(AssertionError):
-            e.mlb_linear_fwd(o, x.float(), W, 130, 72, 256, 72, 256, 256)
-    assert torch.equal(*outs) and c.mlb_gemm_dw_direct(768, 768, 1003) == m.mlb_gemm_dw_direct(768, 768, 1003)
+            n.linear_fwd(e(M, 3 * C), x.float(), Wq)
+        with pytest.raises(AssertionError):
+            n.rmsnorm_fwd(e(M, C), e(M, **f32), x.t(), w, 1e-5)
+        return made
+
+    n.lib().mlb_gemm_set_splits(1)
+    outs = []
+    try:
+        for entries in (n._Ctypes(), n.bridge()):
+            seen.clear()
+            monkeypatch.setattr(n, "_E", Spy(entries))
+            outs.append(work())
+            assert seen | {"mlb_capture_id"} == {"mlb_" + k for k in n._KINDS}      # (that one is asked through ctypes)
+            assert [getattr(entries, f)(*a) for f, a in (("mlb_capture_id", ()), ("mlb_gemm_dw_direct", (768, 768, 1003)))] == [
+                0, n.lib().mlb_gemm_dw_direct(768, 768, 1003)]
+    finally:
+        n.lib().mlb_gemm_set_splits(0)
+    assert len(outs[0]) == len(outs[1])
+    for i, (p, q) in enumerate(zip(*outs)):
+        assert torch.equal(p, q), i
 
 
 @pytest.mark.parametrize("ways", [2, 4, 8])
