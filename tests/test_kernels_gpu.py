@@ -1225,6 +1225,7 @@ def test_cross_entropy_gradient_in_place_and_not(rows, V, factor):
     torch.manual_seed(rows + V)
     x, tgt = rnd(rows, V, scale=2.0), torch.randint(0, V, (rows,), device=dev(), dtype=torch.int32)
     leaf = x.clone().requires_grad_(True)
+    assert _native(F.cross_entropy(leaf, tgt))
     (F.cross_entropy(leaf, tgt) * factor).backward()
     z = x.clone().requires_grad_(True)
     loss = F.cross_entropy(z, tgt) * factor
@@ -1269,6 +1270,7 @@ def test_plain_calls_are_what_the_functions_give(form, rows, C, N):
         for fn in (fast, slow):
             ls = [t.detach().requires_grad_(True) if t is not None else None for t in leaves]
             y = fn(*ls)
+            assert _native(y) == (fn is fast and form != "offset")      # (the module takes no unaligned operand)
             gs = torch.autograd.grad(y, [t for t in ls if t is not None], dout)
             with torch.no_grad():
                 outs.append([y.detach(), fn(*ls), *gs])
@@ -1300,6 +1302,7 @@ def test_plain_attention_calls_are_what_the_functions_give(B, T, H, Hkv, hd):
         x = rnd(B * T, width).requires_grad_(True)
         for dout in (rnd(B * T, H * hd), rnd(H * hd, B * T).t()):
             a, b = fast(x), slow(x)
+            assert _native(a) and not _native(b)
             assert torch.equal(a, b) and torch.equal(*(torch.autograd.grad(y, x, dout)[0] for y in (a, b)))
         with torch.no_grad():
             assert torch.equal(fast(x), slow(x))
@@ -1324,6 +1327,7 @@ def test_what_the_extension_module_declines():
     with torch.autograd.forward_ad.dual_level(), pytest.raises(Exception):
         F.linear(torch.autograd.forward_ad.make_dual(x, x), W)
     y = checkpoint(lambda t: F.swiglu(F.linear(t, W)), x.requires_grad_(True), use_reentrant=False)
+    assert _native(y)
     g, = torch.autograd.grad(y, x, torch.ones_like(y))
     e, = torch.autograd.grad(F.SwiGLU.apply(F.Linear.apply(x, W, None)), x, torch.ones_like(y := y.detach()))
     assert torch.equal(g, e)
@@ -1701,3 +1705,52 @@ def test_cross_entropy_backward_replayed(together, factor):
             if not together:
                 bwd.replay()
             assert torch.equal(g, want)
+
+
+@pytest.mark.parametrize("name", NATIVE_NODES)
+def test_nodes_run_on_the_stream_they_are_called_on(name):
+    """Forward and backward on a side stream, behind operands that arrive late there; and from two threads at once, each on a stream of its own: the
+    bits of a call by itself."""
+    import threading
+    ops_, call = _native_nodes()[name]
+    nat().lib().mlb_gemm_set_splits(1)
+
+    def one(values, wait=0):
+        late = [torch.zeros_like(v) for v in values]
+        if wait:
+            torch.cuda._sleep(wait)
+        for t, v in zip(late, values):
+            t.copy_(v)
+        leaves = [t.requires_grad_(True) for t in late]
+        y = call(*leaves)
+        assert _native(y)
+        return [y.detach(), *torch.autograd.grad(y, leaves, torch.ones_like(y))]
+
+    try:
+        sets = [ops_, [t * 0.5 + 0.25 for t in ops_]]
+        want = [one(v) for v in sets]
+        streams = [torch.cuda.Stream() for _ in sets]
+        torch.cuda.synchronize()
+        with torch.cuda.stream(streams[0]):
+            got = one(sets[0], wait=20_000_000)      # (10 ms)
+        streams[0].synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(got, want[0]))
+        outs = [[], []]
+
+        def work(i):
+            with torch.cuda.stream(streams[i]):
+                for _ in range(10):
+                    outs[i].append(one(sets[i], wait=20_000))
+                streams[i].synchronize()
+
+        threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join(60)
+        for i in range(2):
+            assert len(outs[i]) == 10
+            for got in outs[i]:
+                assert all(torch.equal(a, b) for a, b in zip(got, want[i]))
+    finally:
+        nat().lib().mlb_gemm_set_splits(0)

@@ -393,14 +393,29 @@ def test_gradient_clipping_on_the_device(comm):
     assert _native().get_error() == 0
 
 
+def _early_and_not(code):
+    """The line that starts with SUM of a program run with MLB_PDL=0 and without it; the program prints the error word last."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    out = []
+    for pdl in ("0", None):
+        env = dict(os.environ, PYTHONPATH=root)
+        env.pop("MLB_PDL", None)
+        if pdl is not None:
+            env["MLB_PDL"] = pdl
+        r = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stderr[-2000:]
+        out.append([l for l in r.stdout.splitlines() if l.startswith("SUM")][0])
+    assert out[0] == out[1] and out[0].endswith(" 0"), out
+
+
 @pytest.mark.parametrize("graph", [False, True])
 def test_kernels_that_start_early_give_the_same_bits(graph):
     """Small kernels start under the one before them (MLB_PDL unset); with MLB_PDL=0 none does.  Same kernels, same sums: same bits, through
     a model whose every launch is small, eagerly and captured."""
-    import os
-    import subprocess
-    import sys
-    code = (
+    _early_and_not(
         "import torch\n"
         "from ml_b200 import Config\n"
         "from ml_b200.trainer import Trainer\n"
@@ -414,14 +429,30 @@ def test_kernels_that_start_early_give_the_same_bits(graph):
         "torch.cuda.synchronize()\n"
         "g = tr.model.grads.view(torch.int32).long()\n"
         "print('SUM', tr.model.losses.view(torch.int32).long().sum().item(), (g * torch.arange(1, g.numel() + 1, device='cuda')).sum().item(), native.get_error())\n")
-    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-    out = []
-    for pdl in ("0", None):
-        env = dict(os.environ, PYTHONPATH=root)
-        env.pop("MLB_PDL", None)
-        if pdl is not None:
-            env["MLB_PDL"] = pdl
-        r = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=300)
-        assert r.returncode == 0, r.stderr[-2000:]
-        out.append([l for l in r.stdout.splitlines() if l.startswith("SUM")][0])
-    assert out[0] == out[1] and out[0].endswith(" 0"), out
+
+
+def test_attention_blocks_that_start_early_give_the_same_bits():
+    """The same for norm, products, attention of every head size, with and without a mask, in one wave and in several, and a product whose long reduction a
+    cluster shares: forward and backward, each pass behind the one before."""
+    _early_and_not(
+        "import torch\n"
+        "from ml_b200.ops import autograd as F, native, ref\n"
+        "native.lib().mlb_gemm_set_splits(1)\n"
+        "def passes(hd, H, B, T, causal):\n"
+        "    C, g, total = H * hd, torch.Generator('cuda').manual_seed(1), 0\n"
+        "    r = lambda *s: torch.randn(*s, generator=g, device='cuda').bfloat16()\n"
+        "    cos, sin = ref.rope_tables(T, hd, 1e4, torch.device('cuda'))\n"
+        "    x, w, Wq, Wo, few, Wl = r(B * T, C), r(C), r(3 * C, C) / C ** 0.5, r(C, C) / C ** 0.5, r(64, 11008), r(C, 11008) / 105\n"
+        "    leaves = [t.requires_grad_(True) for t in (x, w, Wq, Wo, few, Wl)]\n"
+        "    for i in range(10):\n"
+        "        qkv = F.linear(F.layer_norm(x, w, None, 1e-5) if C % 256 == 0 else F.rmsnorm(x, w, 1e-5), Wq)\n"
+        "        y = F.linear(F.rope_causal_attention(qkv, cos, sin, B, T, H, hd) if causal else F.bidir_attention(qkv, B, T, H, hd), Wo)\n"
+        "        z = F.linear(few, Wl)\n"
+        "        gs = torch.autograd.grad([y, z], leaves, [torch.ones_like(y), torch.ones_like(z)])\n"
+        "        for t in (y, z, *gs):\n"
+        "            b = t.detach().reshape(-1).view(torch.int16).long()\n"
+        "            total = (total * 31 + (b * torch.arange(1, b.numel() + 1, device='cuda')).sum().item()) % (1 << 61)\n"
+        "    return total\n"
+        "sizes = [(16, 4, 2, 70, 1), (32, 4, 2, 300, 1), (64, 4, 2, 40, 1), (64, 12, 3, 300, 1), (64, 12, 6, 1000, 1), (128, 4, 2, 300, 1), (128, 16, 2, 600, 1),\n"
+        "         (64, 12, 4, 197, 0), (64, 12, 52, 197, 0), (128, 4, 2, 70, 0)]\n"
+        "print('SUM', *(passes(*s) for s in sizes), native.get_error())\n")
