@@ -53,7 +53,8 @@ __device__ __forceinline__ void mlb_pdl_sync() {
 // Which kernels start early, without MLB_PDL: all GEMMs, the persistent attention kernels of one wave (no more items than SMs), the split attention
 // kernels up to a limit of their own (split_early), and element-wise kernels of no more threads than the machine holds (2048 an SM: one
 // wave, or two where a kernel's registers allow half as many).  A chain of small kernels is bound by launch and set-up, which then run under the kernel before: step of
-// the 4-layer / 128-wide decoder 637 -> 567 us, attention forward of a few thousand tokens 13.3 -> 10.4; GEMMs of any size gain 2 to 3 us of
+// the 4-layer / 128-wide decoder 637 -> 567 us, rotary copy and causal attention forward, 12 heads of 64, of 500 tokens 16.5 -> 15.2, of 8 x 256
+// 14.6 -> 13.8, of 3 x 1000 31.6 -> 28.7 (in a captured graph, whose launches are closer anyway, 15.4 -> 14.8, 13.2 -> 13.6, 27.0 -> 26.8); GEMMs of any size gain 2 to 3 us of
 // launch gap each (step of the 12-layer decoder 17.35 -> 17.11 ms, captured 16.40 -> 16.29).
 // Larger ones stay out: their CTAs sit on the SMs while the kernel before still works there, and take registers and issue slots from
 // it (every kernel early: attention at 16 x 1024 tokens 269 -> 283 us).
