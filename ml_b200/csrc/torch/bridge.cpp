@@ -79,6 +79,7 @@ typedef std::optional<Tensor> Maybe;      // (an undefined tensor is no argument
 #define MLB_POINTER(name, ret, args) ret(*name) args = nullptr;
 struct Entries { MLB_ENTRIES(MLB_POINTER) } K;
 
+PyObject* address_type = nullptr;  // ops.native.Address
 PyObject* settings = nullptr;      // the Python module whose variables FUSED_ATTN_BWD and FUSED_ATTN_BWD_MAX_SCRATCH bound attn_bwd's workspace
 
 St stream() { return (St)c10::cuda::getCurrentCUDAStream().stream(); }
@@ -470,8 +471,8 @@ PyObject* py_cross_entropy(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 // ------------------------------------------------------------------ the entry points themselves
-// Arguments by the C type of the parameter: a bf16 (void*), fp32, int32 or byte tensor, which has to be contiguous and on a GPU, or its
-// address as a number (0: none); numbers.  The stream comes last and is the current one.
+// Arguments by the C type of the parameter: a bf16 (void*), fp32, int32 or byte tensor, which has to be contiguous and on a GPU, or an Address
+// of ops/native.py (a plain number, which may be anything, is refused); numbers.  The stream comes last and is the current one.
 [[noreturn]] void bad_tensor(const char* want) {
   PyErr_Format(PyExc_AssertionError, "tensor: need contiguous CUDA %s", want);
   throw python_error();
@@ -483,7 +484,7 @@ P pointer_arg(PyObject* o, at::ScalarType type, const char* want) {
     if (!t.is_cuda() || t.scalar_type() != type || !t.is_contiguous()) bad_tensor(want);
     return (P)t.data_ptr();
   }
-  if (!PyLong_Check(o)) bad_tensor(want);
+  if ((PyObject*)Py_TYPE(o) != address_type) bad_tensor(want);
   const P p = (P)PyLong_AsVoidPtr(o);
   if (!p && PyErr_Occurred()) throw python_error();
   return p;
@@ -558,6 +559,10 @@ PyObject* py_bind(PyObject*, PyObject* args) {
   K.name = (ret(*) args)dlsym(h, #name);                             \
   TORCH_CHECK(K.name != nullptr, p, " has no function " #name);
   MLB_ENTRIES(MLB_LOOKUP)
+  PyObject* address = PyObject_GetAttrString(module, "Address");
+  if (!address) return nullptr;
+  Py_XDECREF(address_type);
+  address_type = address;
   Py_INCREF(module);
   Py_XDECREF(settings);
   settings = module;

@@ -22,8 +22,14 @@ from .. import build as _build
 _i32, _i64, _f32, _vp = C.c_int, C.c_long, C.c_float, C.c_void_p
 
 
-# Entry points that the extension module has, by the C type of each parameter.  b bf16, f fp32, i int32, u bytes: tensors, or an address as a
-# number (0: none); n int, l long, d float; s the current stream
+class Address(int):
+    """Device memory by its address, where an entry point of the extension module takes no tensor: an untyped buffer, a part of a workspace."""
+
+
+NONE = Address(0)      # an optional tensor that is not there
+
+# Entry points that the extension module has, by the C type of each parameter.  b bf16, f fp32, i int32, u bytes: tensors, or an Address; n int,
+# l long, d float; s the current stream
 _KINDS = {
     "linear_fwd": "bbbnnnnnns", "linear_fwd_posembed": "bbbbnnnnnnns", "linear_fwd_rope": "bbbnnnnnnffnns",
     "linear_fwd_swiglu": "bbbbnnnnnns", "linear_dx": "bbbnnnnnns", "linear_dx_delta": "bbbbfnnnnnnnns", "linear_dw": "fbbnnnnnns",
@@ -242,7 +248,7 @@ class _Ctypes:
         fn, kinds, to = getattr(lib(), name), _KINDS[name[4:]], {"b": _b, "f": _f, "i": _i, "u": _u8}
 
         def call(*args):
-            a = [to[k](x) if k in to and not isinstance(x, int) else x for k, x in zip(kinds, args, strict=kinds[-1] != "s")]
+            a = [to[k](x) if k in to and type(x) is not Address else x for k, x in zip(kinds, args, strict=kinds[-1] != "s")]
             return fn(*a, _st()) if kinds[-1] == "s" else fn(*a)
 
         setattr(self, name, call)
@@ -372,7 +378,7 @@ def gemm(out, A, B, a_mn=False, b_mn=False, accumulate=False):
     `out` is bf16 (overwritten) or, with accumulate=True, fp32 (added to)."""
     M, K = (A.shape[1], A.shape[0]) if a_mn else A.shape
     N = B.shape[1] if b_mn else B.shape[0]
-    _chk(_entries().mlb_gemm(out.data_ptr(), A, B, M, N, K, out.stride(0), A.stride(0), B.stride(0), int(a_mn), int(b_mn),
+    _chk(_entries().mlb_gemm(Address(out.data_ptr()), A, B, M, N, K, out.stride(0), A.stride(0), B.stride(0), int(a_mn), int(b_mn),
                         int(accumulate)), "gemm")
 
 
@@ -416,18 +422,17 @@ def attn_bwd(dqkv, dout, qkv, out, lse, B, T, H, hd, rope=None, have_delta=False
     have_delta: linear_dx_delta has just written this call's delta term, the pass over dO and O is left out.
     Returns True if it did (tensor-core path), False if the caller still has to call rope_bwd."""
     delta = scratch("attn_delta", B * H * T, torch.float32, qkv.device)
-    acc = part = 0
+    part = NONE
     if hd == 64 and FUSED_ATTN_BWD:
         # per-(query tile, key tile) bf16 partials of dQ; past FUSED_ATTN_BWD_MAX_SCRATCH the two-kernel backward runs
         nbytes = _entries().mlb_attn_bwd_scratch_bytes(B, T, H, hd)
         if 0 < nbytes <= FUSED_ATTN_BWD_MAX_SCRATCH:
             part = torch.empty(nbytes // 2, dtype=torch.bfloat16, device=qkv.device)      # (too large to be kept per stream)
-            acc = part.data_ptr()
-    cp, sp = (0, 0) if rope is None else rope
+    cp, sp = (NONE, NONE) if rope is None else rope
     fn = _entries().mlb_attn_bwd
     if have_delta:
         fn = _entries().mlb_attn_bwd_have_delta
-    rc = fn(dqkv, dout, qkv, out, lse, delta, acc, B, T, H, hd, cp, sp)
+    rc = fn(dqkv, dout, qkv, out, lse, delta, part, B, T, H, hd, cp, sp)
     global LAUNCHES
     LAUNCHES += 2 if have_delta else 3
     if rc < 0 or rc > 1:
@@ -477,7 +482,7 @@ def add_rmsnorm_fwd(resid, out, rstd, a, b, w, eps):
 def layernorm_fwd(out, mean, rstd, x, w, b, eps):
     rows, Cc = x.shape
     fn = _entries().mlb_layernorm_fwd
-    _chk(fn(out, mean, rstd, x, w, 0 if b is None else b, rows, Cc, eps), "layernorm_fwd")
+    _chk(fn(out, mean, rstd, x, w, NONE if b is None else b, rows, Cc, eps), "layernorm_fwd")
 
 
 def _partial(numel, device):
@@ -501,8 +506,7 @@ def layernorm_bwd_cast(dx, dw, db, dy, x, w, mean, rstd):
     rows, Cc = x.shape
     L = _entries()
     part = _partial(L.mlb_rmsnorm_bwd_blocks(rows) * 2 * Cc, x.device)
-    rc = L.mlb_layernorm_bwd2(dx, dw, 0 if db is None else db, 1, dy, x, w, mean, rstd, rows, Cc,
-                              part.data_ptr())
+    rc = L.mlb_layernorm_bwd2(dx, dw, NONE if db is None else db, 1, dy, x, w, mean, rstd, rows, Cc, part)
     if rc == -7:
         aw, ab = torch.zeros_like(dw, dtype=torch.float32), torch.zeros_like(dw, dtype=torch.float32)
         layernorm_bwd(dx, aw, ab, dy, x, w, mean, rstd)
@@ -518,7 +522,7 @@ def rmsnorm_bwd_cast(dx, dw, dy, x, w, rstd, add=None):
     rows, Cc = x.shape
     L = _entries()
     part = _partial(L.mlb_rmsnorm_bwd_blocks(rows) * Cc, x.device)
-    rc = L.mlb_rmsnorm_bwd_cast(dx, dw, dy, x, w, rstd, 0 if add is None else add, rows, Cc, part.data_ptr())
+    rc = L.mlb_rmsnorm_bwd_cast(dx, dw, dy, x, w, rstd, NONE if add is None else add, rows, Cc, part)
     if rc == -7:
         acc = torch.zeros_like(dw, dtype=torch.float32)
         rmsnorm_bwd(dx, acc, dy, x, w, rstd, add)
@@ -532,7 +536,7 @@ def colsum(out, x):
     M, N = x.shape
     L = _entries()
     part = _partial(L.mlb_colsum_splits(M, N) * N, x.device)
-    rc = L.mlb_colsum(out, x, M, N, part.data_ptr())
+    rc = L.mlb_colsum(out, x, M, N, part)
     if rc == -7:
         out.copy_(x.sum(0))
         return
@@ -545,8 +549,8 @@ def rmsnorm_bwd(dx, dw, dy, x, w, rstd, add=None):
     blocks = L.mlb_rmsnorm_bwd_blocks(rows)
     # 32 words of tickets, zero between calls, then the partial sums
     ws = scratch("rms_bwd", 32 + (blocks + 16) * Cc, torch.float32, x.device, zero=True).data_ptr()
-    _chk(L.mlb_rmsnorm_bwd(dx, dw, dy, x, w, rstd, 0 if add is None else add,
-                           rows, Cc, ws + 128, ws), "rmsnorm_bwd")
+    _chk(L.mlb_rmsnorm_bwd(dx, dw, dy, x, w, rstd, NONE if add is None else add,
+                           rows, Cc, Address(ws + 128), Address(ws)), "rmsnorm_bwd")
 
 
 # ------------------------------------------------------------------ rope / swiglu / CE / AdamW
@@ -608,11 +612,11 @@ def ce_mean(loss, losses, dlogits, logits, tgt):
     if rows == 0:
         return loss.zero_()
     stats = torch.empty(2, dtype=torch.float32, device=logits.device)
-    d = 0 if dlogits is None else dlogits
+    d = NONE if dlogits is None else dlogits
     rc = _entries().mlb_ce_mean(loss, losses, stats, d, logits, tgt, rows, V)
     if rc == -7:      # misaligned rows: through an aligned copy
         work = logits.clone() if dlogits is None else dlogits.copy_(logits)
-        rc = _entries().mlb_ce_mean(loss, losses, stats, work.data_ptr() if dlogits is not None else 0, work.data_ptr(), tgt, rows, V)
+        rc = _entries().mlb_ce_mean(loss, losses, stats, NONE if dlogits is None else work, work, tgt, rows, V)
     _chk(rc, "ce_mean")
 
 
@@ -636,8 +640,8 @@ def adamw(master, params, grads, m, v, lr, b1, b2, eps, wd, bc1, bc2, grad_scale
     """dev_hyper: optional CUDA fp32[4] = {lr, 1/bc1, 1/bc2, grad_scale} read by the kernel instead of the scalar
     arguments (lets a captured graph follow the optimizer step count)."""
     n = master.numel()
-    pp = 0 if (params is None or params.data_ptr() == master.data_ptr()) else params
-    hp = 0 if dev_hyper is None else dev_hyper
+    pp = NONE if (params is None or params.data_ptr() == master.data_ptr()) else params
+    hp = NONE if dev_hyper is None else dev_hyper
     _chk(_entries().mlb_adamw(master, pp, grads, m, v, n, lr, b1, b2, eps, wd, bc1, bc2, grad_scale, hp), "adamw")
 
 
@@ -758,7 +762,7 @@ def sum_scale(out, x, scale):
 def zero_(x):
     fn = _entries().mlb_zero
     assert x.is_cuda and x.is_contiguous()
-    _chk(fn(x.data_ptr(), x.numel() * x.element_size()), "zero")
+    _chk(fn(Address(x.data_ptr()), x.numel() * x.element_size()), "zero")
     global LAUNCHES
     LAUNCHES -= 1          # a memset node, not a kernel of this library: not part of the launch count
 

@@ -619,3 +619,16 @@ def test_an_extension_module_that_cannot_be_used_is_done_without(failure, tmp_pa
     with pytest.warns(UserWarning, match="cannot be built or loaded"):
         assert native.bridge.__wrapped__() is None
     assert isinstance(native._Ctypes(), native._Ctypes)
+
+
+def test_entry_points_refuse_numbers_for_tensors():
+    """A number in a tensor's place, an address made up or the null of a forgotten argument, is refused before anything is launched, through the
+    extension module and through ctypes; memory without a tensor says that it is an Address."""
+    from ml_b200.ops import native
+    assert native.bridge() is not None
+    for entries in (native.bridge(), native._Ctypes()):
+        for args in ((0, 0, 16, 8), (native.NONE, 0, 16, 8), (True, native.NONE, 16, 8), (1 << 40, native.NONE, 16, 8), (None, native.NONE, 16, 8)):
+            with pytest.raises((AssertionError, AttributeError)):
+                entries.mlb_swiglu_fwd(*args)
+    with pytest.raises(AssertionError):
+        native.bridge().mlb_swiglu_fwd(torch.zeros(16, 8, dtype=torch.bfloat16), native.NONE, 16, 8)      # (of the host)
