@@ -1510,8 +1510,13 @@ MLB_API int mlb_colsum(void* out, const void* x, long M, int N, float* partial, 
   mlb_launch(fold_cols_k<true>, dim3((N + 31) / 32), dim3(FOLD_THREADS), 0, st, out, (void*)nullptr, (const float*)partial, S, N, N);
   LAUNCH_RET;
 }
+// (ticket null: the first 32 words of `partial` are the tickets)
 MLB_API int mlb_rmsnorm_bwd(void* dx, float* dw, const void* dy, const void* x, const void* w, const float* rstd, const void* add,
                             long rows, int C, float* partial, int* ticket, cudaStream_t st) {
+  if (ticket == nullptr) {
+    ticket = (int*)partial;
+    partial += 32;
+  }
   const int blocks = mlb_rmsnorm_bwd_blocks(rows);
   const size_t sh = (size_t)std::max(C, 1024) * sizeof(float);
 #define RB(...)                                                                                                         \

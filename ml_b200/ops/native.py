@@ -548,9 +548,8 @@ def rmsnorm_bwd(dx, dw, dy, x, w, rstd, add=None):
     L = _entries()
     blocks = L.mlb_rmsnorm_bwd_blocks(rows)
     # 32 words of tickets, zero between calls, then the partial sums
-    ws = scratch("rms_bwd", 32 + (blocks + 16) * Cc, torch.float32, x.device, zero=True).data_ptr()
-    _chk(L.mlb_rmsnorm_bwd(dx, dw, dy, x, w, rstd, NONE if add is None else add,
-                           rows, Cc, Address(ws + 128), Address(ws)), "rmsnorm_bwd")
+    ws = scratch("rms_bwd", 32 + (blocks + 16) * Cc, torch.float32, x.device, zero=True)
+    _chk(L.mlb_rmsnorm_bwd(dx, dw, dy, x, w, rstd, NONE if add is None else add, rows, Cc, ws, NONE), "rmsnorm_bwd")
 
 
 # ------------------------------------------------------------------ rope / swiglu / CE / AdamW
