@@ -439,10 +439,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_tc_kernel(const __gri
 // bar_o P V complete (commit) | bar_of O_blk folded (4 warps, mode 1 only).  K has 3 slots, V 4, Q 2 buffers: each is a
 // ring with a "full" barrier (TMA bytes) and a "released" barrier on which the 8 softmax warps arrive when they have
 // seen the MMAs that read the slot complete (Q K^T for K and Q, P V for V).
-// What the cycle stamps showed about the issuing threads: every tcgen05.mma and every tcgen05.commit costs its thread
-// ~75 cycles whatever the product's size, so 12 MMAs and 2 commits per key block and tile are ~1000 cycles of one
-// thread; with a single thread for both tiles that chain (3200 cycles per key block, never waiting) was the kernel's
-// pace.
+// One issuing thread per tile: with a single one for both its waits for one tile hold up the other's products.
 // The one-pass variant writes P as the upper halves of the fp32 exponentials (one byte-permute per pair instead of a
 // rounding conversion; equal speed when measured, kept for its single instruction).  Cutting off 16 mantissa bits loses
 // 2^-8 / mantissa of the value, 0.28 % on average over mantissas; the exponentials are therefore taken of
@@ -662,10 +659,9 @@ __global__ void __maxnreg__(160) attn_fwd_rows_tc_kernel(const __grid_constant__
     }
   } else if (warp == 8 || warp == 10) {
     // ---------------------------------------------------------------- MMA warps: one issuing thread per tile (warp 8: tile
-    // 0, warp 10: tile 1).  A single thread for both tiles was the kernel's pace: its serial chain of waits, descriptor
-    // arithmetic and issues took ~3200 cycles per key block, all of it busy.  Slot and phase counters are kept
+    // 0, warp 10: tile 1).  A single thread for both tiles was the kernel's pace.  Slot and phase counters are kept
     // incrementally (no division on this thread).
-    if (lane == 0) {
+    if (tc::elect_one()) {
       const int t = warp == 8 ? 0 : 1;
       constexpr uint32_t idesc_s = tc::idesc_bf16(128, 128, 0, 0);
       constexpr uint32_t idesc_o = tc::idesc_bf16(128, HD, 0, 1);     // A = P (TMEM, K-major), B = V (MN-major)
@@ -776,8 +772,8 @@ __global__ void __maxnreg__(160) attn_fwd_rows_tc_kernel(const __grid_constant__
           tc::tmem_st16(t_o + c * 32 + 16, w1);
         }
       };
-      // The slots' release barriers are arrived on from here (one lane per warp, 8 warps) rather than by tcgen05.commit:
-      // every tcgen05 instruction costs its issuing thread ~75 cycles, and that thread's chain sets the block time.
+      // The slots' release barriers are arrived on from here (one lane per warp, 8 warps) rather than by a tcgen05.commit more
+      // in the issuing thread's chain.
       auto s_seen = [&](int j) {          // Q K^T of block g has completed: its K slot, and after an item's last block Q
         if (lane == 0) {
           tc::mbar_arrive(&bar_kf[g % KN]);
@@ -1508,11 +1504,10 @@ __global__ void __maxnreg__(120) attn_bwd_fused_tc_kernel(const __grid_constant_
     }
   } else if (warp == BWDF_CTRL_WARP || warp == BWDF_SCORE_WARP) {
     // ---------------------------------------------------------------- two MMA warps: waits, tcgen05.mma, commits, nothing else
-    // Every tcgen05.mma / commit costs its issuing thread ~75 cycles whatever the product's size: 32 MMAs and two commits
-    // per query block from ONE thread were 2700 of the block's 3500 cycles, never waiting.  The 8 score MMAs have
-    // their own issuing thread, so they go out while the 24 gradient MMAs of the previous block are still being issued.
+    // The 8 score MMAs have their own issuing thread, so they go out while the other still waits for what the 24 gradient MMAs of
+    // the previous block read.
     // (Descriptors are formed by adding small constants to per-buffer bases.)
-    if (lane == 0) {
+    if (tc::elect_one()) {
       constexpr uint32_t idesc_s = tc::idesc_bf16(128, 128, 0, 0);
       constexpr uint32_t idesc_d = tc::idesc_bf16(128, HD, 0, 1);    // A K-major (P^T in TMEM / dS^T), B MN-major (dO / Q)
       constexpr uint32_t idesc_q = tc::idesc_bf16(128, HD, 1, 1);    // A MN-major (dS^T read as dS), B MN-major (K)

@@ -132,7 +132,7 @@ __global__ void __maxnreg__(160) attn_fwd128_k(const __grid_constant__ CUtensorM
       }
     }
   } else if (warp == 8 || warp == 10) {
-    if (lane == 0) {
+    if (tc::elect_one()) {
       const int t = warp == 8 ? 0 : 1;
       constexpr uint32_t idesc_s = tc::idesc_bf16(128, 128, 0, 0), idesc_o = tc::idesc_bf16(128, H128, 0, 1);
       const uint32_t t_s = tmem + t * 128, t_o = tmem + 256 + t * 128;
@@ -327,8 +327,7 @@ __global__ void __maxnreg__(160) attn_fwd128_k(const __grid_constant__ CUtensorM
 
 // ------------------------------------------------------------------ backward
 // dK / dV of a 128-key tile, streaming query blocks.  TMEM: S^T, dP^T, dV, dK.  Two threads issue products, as in the kernels for head
-// size 64: every tcgen05.mma and commit costs the thread that issues it 75 ... 100 cycles whatever its size, 3600 for a block's 36
-// with one thread.  One takes  S^T(i) dP^T(i) S^T(i+1) ...,  the other  dV(i) dK(i) ...
+// size 64, so that neither's waits hold up the other's products.  One takes  S^T(i) dP^T(i) S^T(i+1) ...,  the other  dV(i) dK(i) ...
 // P^T goes to shared memory, so S^T(i+1) needs no more than that S^T(i) has been read, and the exponentials of block i+1 run under
 // dK(i) and dP^T(i+1); over its scores it would make S^T(i+1) wait for dV(i).  dS^T stays over dP^T.  512 element-wise threads: a
 // thread has one key and 32 of the block's 128 queries.  Four warps per sub-partition hide each other's TMEM and barrier
@@ -439,7 +438,7 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
       }
     }
   } else if (warp == BWD128_MMA_WARP) {
-    if (lane == 0) {
+    if (tc::elect_one()) {
       constexpr uint32_t idesc_s = tc::idesc_bf16(128, 128, 0, 0);
       const uint64_t dK = desc_base_k(tc::smem_u32(smem + S::K)), dV = desc_base_k(tc::smem_u32(smem + S::V));
       const uint64_t dQ0 = desc_base_k(tc::smem_u32(smem + S::Q)), dO0 = desc_base_k(tc::smem_u32(smem + S::DO));
@@ -470,7 +469,7 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
       attn_settle(&bar_end[0], 1);
     }
   } else if (warp == BWD128_GRAD_WARP) {
-    if (lane == 0) {
+    if (tc::elect_one()) {
       constexpr uint32_t idesc_g = tc::idesc_bf16(128, H128, 0, 1);
       const uint64_t aP = desc_base_k(tc::smem_u32(smem + S::P));
       const uint64_t gQ0 = desc_base_mn(tc::smem_u32(smem + S::Q)), gO0 = desc_base_mn(tc::smem_u32(smem + S::DO));
@@ -675,7 +674,7 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
       for (int i = 0; i < 2; i++) attn_settle(&bar_v[i], (g + 1 - i) / 2);
     }
   } else if (warp == BWD128_MMA_WARP) {
-    if (lane == 0) {
+    if (tc::elect_one()) {
       constexpr uint32_t idesc_s = tc::idesc_bf16(128, 128, 0, 0);
       const uint64_t dQ = desc_base_k(tc::smem_u32(smem + S::Q)), dO = desc_base_k(tc::smem_u32(smem + S::DO));
       const uint64_t dK0 = desc_base_k(tc::smem_u32(smem + S::K)), dV0 = desc_base_k(tc::smem_u32(smem + S::V));
@@ -717,7 +716,7 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
       attn_settle(&bar_end[0], 1);
     }
   } else if (warp == BWD128_GRAD_WARP) {
-    if (lane == 0) {
+    if (tc::elect_one()) {
       constexpr uint32_t idesc_g = tc::idesc_bf16(128, H128, 0, 1);
       const uint64_t gK0 = desc_base_mn(tc::smem_u32(smem + S::K));
       int g = 0, kr = 0;      // kr = g % 3

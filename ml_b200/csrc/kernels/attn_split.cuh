@@ -31,8 +31,7 @@ struct SplitArgs {
 constexpr int SPLIT_THREADS = 128;
 constexpr int BOX_BYTES = 64 * 64 * 2;      // one TMA box: 64 rows x 64 columns, 128-byte swizzled rows
 
-// Offsets to a tile's first descriptor, in its address units of 16 bytes, all known at compile time: a thread that puts descriptors
-// together from scratch issues an MMA every ~200 cycles, one that adds a constant keeps up with the tensor core (64).
+// Offsets to a tile's first descriptor, in its address units of 16 bytes, all known at compile time: an issuing thread adds a constant.
 // k-step ks of 16 elements of a K-major tile whose 64-column chunks are `chunk` bytes apart; of 16 rows of an MN-major tile.
 __host__ __device__ constexpr uint64_t off_k(int ks, int chunk) { return (uint64_t)((ks >> 2) * (chunk >> 4) + (ks & 3) * 2); }
 __host__ __device__ constexpr uint64_t off_mn(int ks) { return (uint64_t)(ks * 128); }
@@ -165,6 +164,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
     tc::mbar_fence_init();
     tc::tma_prefetch_desc(&tm);
   }
+  auto leader = [&]() -> bool { return warp == 0 && tc::elect_one(); };      // the thread that loads and multiplies (whole warps ask)
   if (warp == 0) tc::tmem_alloc(tmem_slot, TMEM_COLS);
   tc::tc_fence_before();
   __syncthreads();
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
     }
     tc::mma_commit(bar_s);
   };
-  if (tid == 0) {
+  if (leader()) {
     tc::mbar_expect_tx(bar_q, 2 * CH * BOX_BYTES);
     split_load<CH>(smem + S::Q, &tm, bar_q, h * a.hd, q0, b, 2);
     load_kv(0);
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
 #pragma unroll
   for (int i = 0; i < HDT; i++) o[i] = 0.f;
   for (int j = 0; j < nkb; j++) {
-    if (tid == 0 && j + 1 < nkb && !*s_abort) load_kv(j + 1);     // (block j - 1, the buffers' last reader, is complete: bar_o of it was waited for)
+    if (leader() && j + 1 < nkb && !*s_abort) load_kv(j + 1);     // (block j - 1, the buffers' last reader, is complete: bar_o of it was waited for)
     wait(bar_s, j & 1, 42);
     __syncwarp();
     tc::tc_fence_after();
@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
     tc::tmem_st_wait();
     tc::tc_fence_before();
     __syncthreads();
-    if (tid == 0) {
+    if (leader()) {
       wait(&bar_v[j & 1], (j >> 1) & 1, 43);
       tc::tc_fence_after();
       const uint64_t dV = dV0 + (uint64_t)((j & 1) * (CH * BOX_BYTES >> 4));
@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
   tc::tc_fence_before();
   __syncthreads();
   if (*s_abort) {
-    if (tid == 0) {
+    if (leader()) {
       tc::mma_commit(bar_end);
       attn_settle(bar_end, 1);
       attn_settle(bar_q, 1);
@@ -389,6 +389,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
     tc::tma_prefetch_desc(&tm);
     tc::tma_prefetch_desc(&tm_do);
   }
+  auto leader = [&]() -> bool { return warp == 0 && tc::elect_one(); };      // the thread that loads and multiplies (whole warps ask)
   if (warp == 0) tc::tmem_alloc(tmem_slot, TMEM_COLS);
   tc::tc_fence_before();
   __syncthreads();
@@ -438,7 +439,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
     if (tid < 64) st[tid] = q < a.T ? a.lse[si + q] * LOG2E : INFINITY;
     else st[tid] = q < a.T ? a.delta[si + q] : 0.f;
   };
-  if (tid == 0) {
+  if (leader()) {
     tc::mbar_expect_tx(bar_r, 4 * CH * BOX_BYTES);
     split_load<CH>(smem + S::RX, &tm, bar_r, KV ? C + xh : xh, r0, b, 2);
     split_load<CH>(smem + S::RY, KV ? &tm : &tm_do, bar_r, KV ? 2 * C + xh : xh, r0, b, 2);
@@ -461,7 +462,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
     wait(bar_s, it & 1, 47);
     __syncwarp();
     tc::tc_fence_after();
-    if (tid == 0 && it + 1 < n && !*s_abort) load_x(it + 1);      // every MMA issued so far is complete: the other buffer is free
+    if (leader() && it + 1 < n && !*s_abort) load_x(it + 1);      // every MMA issued so far is complete: the other buffer is free
     const int c0 = (i0 + it) * 64;
     const float* st = stat + (it & 1) * 128;
     const bool both = c0 + 32 < a.T;      // (as in forward)
@@ -498,7 +499,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
     if (KV && it + 1 < n) load_stat(it + 1);
     tc::tc_fence_before();
     __syncthreads();
-    if (tid == 0) {
+    if (leader()) {
       tc::tc_fence_after();
       const uint64_t slot = (uint64_t)((it & 1) * (CH * BOX_BYTES >> 4)), sx = gsx + slot, sy = gsy + slot;
       if (!*s_abort) {
@@ -536,7 +537,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
   tc::tc_fence_before();
   __syncthreads();
   if (*s_abort) {
-    if (tid == 0) {
+    if (leader()) {
       tc::mma_commit(bar_end);
       attn_settle(bar_end, 1);
       attn_settle(bar_r, 1);

@@ -1594,7 +1594,7 @@ __global__ void __launch_bounds__(128, 1) mma_probe_kernel(long long* cycles, in
   __syncthreads();
   tc::tc_fence_after();
   const uint32_t tmem = *slot;
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32 && tc::elect_one()) {
     constexpr uint32_t idesc = tc::idesc_bf16(128, N, 0, 0);
     const uint32_t sA = tc::smem_u32(smem), sB = sA + 16384;
     const long long t0 = clock64();
