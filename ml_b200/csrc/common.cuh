@@ -48,6 +48,7 @@ __device__ __forceinline__ void mlb_pdl_sync() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 #ifdef __CUDACC__
+#include <atomic>
 #include <cstdlib>
 #include <utility>
 // Which kernels start early, without MLB_PDL: all GEMMs, the persistent attention kernels of one wave (no more items than SMs), the split attention
@@ -77,6 +78,18 @@ inline int mlb_sm_count() {
     return sms > 0 ? sms : 148;
   }();
   return n;
+}
+// More than 48 KB of dynamic shared memory for `kern`, asked for once on each device (bit of `done`; beyond 64 devices each time)
+template <typename K>
+inline cudaError_t mlb_allow_smem(K kern, size_t bytes, std::atomic<unsigned long long>& done) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const unsigned long long bit = dev < 64 ? 1ull << dev : 0;
+  if (done.load(std::memory_order_relaxed) & bit) return cudaSuccess;
+  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_relaxed);
+  return e;
 }
 template <typename... KArgs, typename... Args>
 inline cudaError_t mlb_launch_attr(bool early, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
