@@ -74,6 +74,20 @@ __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
+// An earlier CTA of this library gave up on a wait: leave at once instead of queueing more waits behind it (CTA-uniform).
+__device__ __forceinline__ bool attn_given_up() {
+  return __syncthreads_or(threadIdx.x == 0 && *(volatile int*)&g_mlb_error != 0) != 0;
+}
+
+// A CTA one of whose waits has run out loads and multiplies nothing more.  What its threads have already issued still uses its shared
+// and tensor memory, so before they are given back the issuing thread waits, 2 ms at most, for the last of it: `begun` phases of a
+// barrier that counts a load's bytes or a commit (each begun when the one before was complete).
+__device__ __forceinline__ void attn_settle(uint64_t* bar, int begun) {
+  if (begun <= 0) return;
+  const uint64_t t0 = tc::globaltimer_ns();
+  while (!tc::mbar_try(bar, (begun - 1) & 1) && tc::globaltimer_ns() - t0 < 2000000) { }
+}
+
 // packed fp32x2 arithmetic (two lanes per instruction on sm_100) and 3-input max
 __device__ __forceinline__ uint64_t pk2(float a, float b) {
   uint64_t r;
@@ -185,11 +199,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_tc_kernel(const __gri
   const uint32_t t_o = tmem + 256;   // O buffers at +256 and +256+HD
   // Bounded, sticky wait: after the first expiry in this CTA every later wait returns at once, and all threads keep
   // executing the same sequence of arrivals / named barriers, so nobody is left waiting for a thread that gave up.
-  auto wait = [&](uint64_t* bar, uint32_t phase, int where) -> bool {
-    if (*s_abort) return false;
-    if (!tc::mbar_wait(bar, phase, where)) { *s_abort = 1; return false; }
-    return true;
-  };
+  auto wait = [&](uint64_t* bar, uint32_t phase, int where) { return tc::mbar_wait_sticky(bar, phase, where, s_abort); };
 
   if (warp == ATT_SOFTMAX_WARPS) {
     // ---------------------------------------------------------------- control warp
@@ -413,6 +423,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_tc_kernel(const __gri
   }
   tc::tc_fence_before();
   __syncthreads();
+  if (tid == 0) tc::report_given_up(s_abort);
   if (warp == ATT_SOFTMAX_WARPS) tc::tmem_dealloc(tmem, TMEM_COLS);
 }
 
@@ -538,7 +549,7 @@ struct Fwd2Step {   // one key block of one item in this CTA's flattened sequenc
 // FMA pipe instead of the special-function unit - equal, 3 % and 5 % slower although the pure exponential chunks got
 // shorter; fp16 exponentials two at a time; tile 1 started half a block behind tile 0; the MMA and loader threads
 // sleeping between barrier probes.)
-template <int MODE, bool DYN = false>
+template <int MODE, bool DYN = false, bool STAMPS = false>
 __global__ void __maxnreg__(160) attn_fwd_rows_tc_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUtensorMap tm_out,
                                                                            const AttnArgs a) {
   mlb_pdl_sync();
@@ -602,12 +613,7 @@ __global__ void __maxnreg__(160) attn_fwd_rows_tc_kernel(const __grid_constant__
   __syncthreads();
   tc::tc_fence_after();
   const uint32_t tmem = *tmem_slot;     // S0 @0, S1 @128, P0 @256, P1 @320 (bf16 pairs), O0 @384, O1 @448
-  auto wait = [&](uint64_t* bar, uint32_t phase, int where) -> bool {
-    if (tc::mbar_try(bar, phase)) return true;      // the common case costs one probe
-    if (*s_abort) return false;
-    if (!tc::mbar_wait(bar, phase, where)) { *s_abort = 1; return false; }
-    return true;
-  };
+  auto wait = [&](uint64_t* bar, uint32_t phase, int where) { return tc::mbar_wait_sticky(bar, phase, where, s_abort); };
 
   if (warp == 9) {
     // ---------------------------------------------------------------- loader warp: every TMA load (and the index arithmetic)
@@ -735,7 +741,7 @@ __global__ void __maxnreg__(160) attn_fwd_rows_tc_kernel(const __grid_constant__
     const uint64_t sl2x2 = pk2(sl2, sl2);
     int g = 0;
     // first 16 blocks of CTA 0: thread 0 (tile 0) and thread 128 (tile 1), 8 stamps per block, tile 1 behind tile 0's 128
-    long long* tl = (a.timeline && blockIdx.x == 0 && (tid & 127) == 0) ? a.timeline + (tid >> 7) * 128 : nullptr;
+    long long* tl = (STAMPS && a.timeline && blockIdx.x == 0 && (tid & 127) == 0) ? a.timeline + (tid >> 7) * 128 : nullptr;
     Fwd2Step it;
     it.set_item(item_at(0), 0, total, npair, nq, BH, a.H);
     for (; it.valid; it.set_item(item_at(it.li + 1), it.li + 1, total, npair, nq, BH, a.H)) {
@@ -1063,6 +1069,7 @@ __global__ void __maxnreg__(160) attn_fwd_rows_tc_kernel(const __grid_constant__
   }
   tc::tc_fence_before();
   __syncthreads();
+  if (tid == 0) tc::report_given_up(s_abort);
   if (warp == 8) tc::tmem_dealloc(tmem, TMEM_COLS);
   if (dyn && tid == 0) attn_ctr_leave(0);
 }
@@ -1130,56 +1137,91 @@ __device__ __forceinline__ void quad_transpose(uint4 (&a)[4], int lane) {
     }
   }
 }
-// 32 bf16 columns (four 16-byte units per lane) of 32 consecutive rows to memory: `dst` = this lane's row at the first column, rows
-// `pitch` elements apart, `nlive` of the warp's rows exist (whole warp, converged).
-__device__ __forceinline__ void store_rows32(bf16* dst, long pitch, uint4 (&a)[4], int lane, int nlive) {
-  quad_transpose(a, lane);
-  const int q = lane & 3;
-  bf16* base = dst - q * pitch + q * 8;      // row of the quad's first lane, this lane's unit
-#pragma unroll
-  for (int k = 0; k < 4; k++)
-    if ((lane & ~3) + k < nlive) *reinterpret_cast<uint4*>(base + k * pitch) = a[k];
-}
-
-// Epilogue helper for the backward kernels: one warp moves 64 accumulator columns of its 32 rows from TMEM to memory as bf16:
-// columns [c0, c0+32) and [c0 + HD/2, c0 + HD/2 + 32), which are exactly RoPE's rotation pairs (i, i + HD/2).  With tables given,
-// RoPE's backward rotation (d0' = d0 c + d1 s, d1' = d1 c - d0 s) is applied.  dst_row: the lane's row, rows `pitch` apart; t its
-// position; nlive rows of the warp exist (0: nothing is stored).  Whole warp.
+// Epilogue of the backward kernels.  A warp moves accumulator columns [c0, c0 + 16) and [c0 + HD/2, c0 + HD/2 + 16) of its 32 rows, which are
+// sixteen of RoPE's rotation pairs (i, i + HD/2), from TMEM to memory as bf16, and rotates them backward (d0' = d0 c + d1 s, d1' = d1 c - d0 s).
+// Lanes 2i and 2i + 1 exchange halves first: each then has eight columns (unit lane & 1) of both their rows, so that an instruction on
+// the tables or the output touches 32 bytes in each of 16 rows instead of 16 in each of 32.  The tables are asked for ahead of the
+// accumulator: they come from the L2, and with a lane at its own row of them and the loads behind the wait an epilogue was ~10000
+// cycles of a key tile's ~39000 at head size 128 (~7500 so).
+struct RopeUnits { float c[2][8], s[2][8]; };      // [row of the lane pair][column of the unit]
 template <int HD>
-__device__ __forceinline__ void store_pairs_rope(bf16* dst_row, long pitch, uint32_t taddr, int c0, int lane, int nlive, const float* cosT,
-                                                 const float* sinT, int t, float out_scale = 1.f) {
-  uint32_t ra[32], rb[32];
-  tc::tmem_ld32x2_wait(taddr + c0, ra, taddr + c0 + HD / 2, rb);
-  float x0[32], x1[32];
+__device__ __forceinline__ void rope_units(RopeUnits& r, const float* cosT, const float* sinT, int t, int c0, int lane, int nlive) {
+  const size_t at = (size_t)(t - (lane & 1)) * (HD / 2) + c0 + (lane & 1) * 8;      // (t: the position of the lane's row)
 #pragma unroll
-  for (int i = 0; i < 32; i++) { x0[i] = __uint_as_float(ra[i]) * out_scale; x1[i] = __uint_as_float(rb[i]) * out_scale; }
-  if (cosT && lane < nlive) {   // 16-byte loads: every lane reads its own row of the tables, an instruction costs the L1 a line per lane whatever its width
-    const float4* c4 = reinterpret_cast<const float4*>(cosT + (size_t)t * (HD / 2) + c0);
-    const float4* s4 = reinterpret_cast<const float4*>(sinT + (size_t)t * (HD / 2) + c0);
+  for (int k = 0; k < 2; k++) {
+    const bool live = (lane & ~1) + k < nlive;
+    const float4* c4 = reinterpret_cast<const float4*>(cosT + at + (size_t)k * (HD / 2));
+    const float4* s4 = reinterpret_cast<const float4*>(sinT + at + (size_t)k * (HD / 2));
 #pragma unroll
-    for (int q = 0; q < 8; q++) {
-      const float4 cv = __ldg(c4 + q), sv = __ldg(s4 + q);
-      const float cc[4] = {cv.x, cv.y, cv.z, cv.w}, ss[4] = {sv.x, sv.y, sv.z, sv.w};
-#pragma unroll
-      for (int e = 0; e < 4; e++) {
-        const float d0 = x0[q * 4 + e], d1 = x1[q * 4 + e];
-        x0[q * 4 + e] = d0 * cc[e] + d1 * ss[e];
-        x1[q * 4 + e] = d1 * cc[e] - d0 * ss[e];
-      }
+    for (int v = 0; v < 2; v++) {
+      *reinterpret_cast<float4*>(&r.c[k][v * 4]) = live ? __ldg(c4 + v) : make_float4(0.f, 0.f, 0.f, 0.f);
+      *reinterpret_cast<float4*>(&r.s[k][v * 4]) = live ? __ldg(s4 + v) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
   }
+}
+__device__ __forceinline__ void pair_exchange(float (&x)[16], int lane) {
+  const bool up = lane & 1;
+#pragma unroll
+  for (int e = 0; e < 8; e++) {
+    const float v = __shfl_xor_sync(0xffffffffu, up ? x[e] : x[8 + e], 1);
+    if (up) x[e] = v; else x[8 + e] = v;
+  }
+}
+__device__ __forceinline__ uint4 pack8(const float* x) {
+  return make_uint4(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]), pack_bf16(x[4], x[5]), pack_bf16(x[6], x[7]));
+}
+// ra, rb: the lane's sixteen fp32 values of either half in; lo[k], hi[k] out: unit lane & 1 of either half of row (lane & ~1) + k.  Whole warp.
+__device__ __forceinline__ void rotate_pairs16(const uint32_t* ra, const uint32_t* rb, int lane, float out_scale, bool rotate, const RopeUnits& r,
+                                               uint4 (&lo)[2], uint4 (&hi)[2]) {
+  float x0[16], x1[16];
+#pragma unroll
+  for (int i = 0; i < 16; i++) { x0[i] = __uint_as_float(ra[i]) * out_scale; x1[i] = __uint_as_float(rb[i]) * out_scale; }
   __syncwarp();
-  uint4 u[4];
+  pair_exchange(x0, lane);
+  pair_exchange(x1, lane);
+  if (rotate) {
 #pragma unroll
-  for (int v = 0; v < 4; v++)
-    u[v] = make_uint4(pack_bf16(x0[v * 8], x0[v * 8 + 1]), pack_bf16(x0[v * 8 + 2], x0[v * 8 + 3]), pack_bf16(x0[v * 8 + 4], x0[v * 8 + 5]),
-                      pack_bf16(x0[v * 8 + 6], x0[v * 8 + 7]));
-  store_rows32(dst_row + c0, pitch, u, lane, nlive);
+    for (int i = 0; i < 16; i++) {
+      const float d0 = x0[i], d1 = x1[i], c = r.c[i >> 3][i & 7], s = r.s[i >> 3][i & 7];
+      x0[i] = d0 * c + d1 * s;
+      x1[i] = d1 * c - d0 * s;
+    }
+  }
 #pragma unroll
-  for (int v = 0; v < 4; v++)
-    u[v] = make_uint4(pack_bf16(x1[v * 8], x1[v * 8 + 1]), pack_bf16(x1[v * 8 + 2], x1[v * 8 + 3]), pack_bf16(x1[v * 8 + 4], x1[v * 8 + 5]),
-                      pack_bf16(x1[v * 8 + 6], x1[v * 8 + 7]));
-  store_rows32(dst_row + c0 + HD / 2, pitch, u, lane, nlive);
+  for (int k = 0; k < 2; k++) { lo[k] = pack8(x0 + k * 8); hi[k] = pack8(x1 + k * 8); }
+}
+// dst_row: the lane's row, rows `pitch` elements apart; nlive rows of the warp exist (0: nothing is stored).  Whole warp.
+template <int HD>
+__device__ __forceinline__ void store_pairs16_regs(bf16* dst_row, long pitch, const uint32_t* ra, const uint32_t* rb, int c0, int lane, int nlive,
+                                                   float out_scale, bool rotate, const RopeUnits& r) {
+  uint4 lo[2], hi[2];
+  rotate_pairs16(ra, rb, lane, out_scale, rotate, r, lo, hi);
+  bf16* base = dst_row - (lane & 1) * pitch + c0 + (lane & 1) * 8;
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    if ((lane & ~1) + k < nlive) {
+      *reinterpret_cast<uint4*>(base + k * pitch) = lo[k];
+      *reinterpret_cast<uint4*>(base + k * pitch + HD / 2) = hi[k];
+    }
+  }
+}
+template <int HD>
+__device__ __forceinline__ void store_pairs16(bf16* dst_row, long pitch, uint32_t taddr, int c0, int lane, int nlive, float out_scale, bool rotate,
+                                              const RopeUnits& r) {
+  uint32_t ra[16], rb[16];
+  tc::tmem_ld16x2_wait(taddr + c0, ra, taddr + c0 + HD / 2, rb);
+  store_pairs16_regs<HD>(dst_row, pitch, ra, rb, c0, lane, nlive, out_scale, rotate, r);
+}
+// all HD columns, by one warp
+template <int HD>
+__device__ __forceinline__ void store_row_pairs(bf16* dst_row, long pitch, uint32_t taddr, int lane, int nlive, const float* cosT, const float* sinT,
+                                                int t, float out_scale = 1.f) {
+#pragma unroll
+  for (int c0 = 0; c0 < HD / 2; c0 += 16) {
+    RopeUnits r;
+    if (cosT) rope_units<HD>(r, cosT, sinT, t, c0, lane, nlive);
+    store_pairs16<HD>(dst_row, pitch, taddr, c0, lane, nlive, out_scale, cosT != nullptr, r);
+  }
 }
 
 constexpr int BWD_THREADS = 512;
@@ -1330,8 +1372,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kv_tc_kernel(const __
     if (cq < 2) {
       const bool is_k = cq == 0;
       bf16* dst = a.out + ((size_t)(row0 + krow)) * 3 * C + (is_k ? C : 2 * C) + h * HD;
-      store_pairs_rope<HD>(dst, 3L * C, (is_k ? t_dk : t_dv) + lane_addr, 0, lane, a.T - (krow - lane), is_k ? a.cosT : nullptr,
-                           is_k ? a.sinT : nullptr, krow);
+      store_row_pairs<HD>(dst, 3L * C, (is_k ? t_dk : t_dv) + lane_addr, lane, a.T - (krow - lane), is_k ? a.cosT : nullptr,
+                          is_k ? a.sinT : nullptr, krow);
     }
   }
   tc::tc_fence_before();
@@ -1346,83 +1388,93 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kv_tc_kernel(const __
 //     P^T = exp2(S^T*c - lse), dS^T = P^T (dP^T - delta)    (512 threads, packed f32x2 math)
 //     dV += P^T dO   (P^T stays in TMEM as the bf16 A operand),   dK += dS^T Q,   dQ_i = dS K   (dS^T in shared memory)
 // The pipeline keeps the tensor core and the element-wise warps busy at the same time:
-//   * as soon as the element-wise warps have S^T / dP^T of block j in registers they release the TMEM columns and the
-//     control thread issues the score MMAs of block j+1 (Q / dO tiles are triple buffered so they are already there);
-//   * the exponentials of block j+1 are computed while dV / dK / dQ of block j run; only the stores of P^T / dS^T wait
-//     for those MMAs (one TMEM region, one shared-memory tile);
+//   * as soon as the element-wise warps have S^T (dP^T) of block j in registers they hand its TMEM columns back and the score thread
+//     issues S^T (dP^T) of block j+1 (Q / dO tiles are triple buffered so they are already there);
+//   * dV, dK and dQ of block j run under the element-wise work on block j+1;
+//   * nothing stops at the end of a key tile: K has two slots, V is asked for when the last dP^T is there, Q and dO are rings over all
+//     of the CTA's blocks, and dV / dK leave TMEM for the drain warps before they are rotated and sent;
+//   * the element-wise warps read scores as fragments (two adjacent queries of each eight, for several keys): a query's statistics then cost
+//     a quarter of the shared-memory reads, which the MMAs' operands compete for, and stores of 8 x 8 matrices need no shuffles;
+//   * code is kept small (two passes over 32 columns instead of one over 64, waits of few instructions, work items taken apart once, no
+//     time stamps): six roles share the SM's instruction cache, and its misses were the bound: 935 k of 6.1 M requests a launch of
+//     16 x 1024 tokens, 316 k now.
+// 16 x 1024 tokens, 12 heads: 136 -> 100 us (32 x 256: 53 -> 40 with the finishing kernel).  Taking out the exponentials, the MMAs, the dQ
+// stores or the dK / dV epilogue one at a time changes that by 5 to 11 us each: none of them alone is the bound any more.
 //   * dQ_j is a partial sum over key tiles.  fp32 add-reduces into one accumulator (TMA or vector red) ran into the
 //     L2's atomic throughput (32 KB per block and SM); instead every (query tile, key tile) pair owns a bf16 tile of a
-//     partial buffer, written with plain stores right after block j+1's operands are handed over, and a second
+//     partial buffer, and a second
 //     kernel adds the partials of a query row in fp32 in key-tile order (deterministic), applies the scale and RoPE's
 //     backward rotation and writes bf16 dQ.
-// Warps: 8 element-wise (TMEM lane group x 64-query half), 4 drain (dQ partial tiles, dK / dV epilogue), 2 MMA issuers (scores / gradients), 1 loader.
-// mbarriers: bar_s scores complete (commit) | bar_free S^T/dP^T read out (8 warps) | bar_p P^T/dS^T stored (8 warps) |
-// bar_dv dV MMAs complete (commit: P^T may be overwritten) | bar_d[2] dV/dK/dQ MMAs complete (commit, alternating so
-// that a waiter two blocks behind cannot mistake a phase) | bar_dqf dQ read out (4 warps) | bar_epi dK/dV of a key tile read out (4 warps).
-struct BwdFusedSmem {
-  static constexpr int K = 0;
-  static constexpr int V = K + TILE_BYTES;
-  static constexpr int Q = V + TILE_BYTES;               // 3 buffers
-  static constexpr int DO = Q + 3 * TILE_BYTES;          // 3 buffers
+// Warps: 8 element-wise (TMEM lane group x 64-query half), 4 drain (dQ partial tiles, dK / dV epilogue), 2 MMA issuers (scores / gradients), 1 loader,
+// 1 for the queries' statistics.
+// mbarriers: bar_k[2] bar_v bar_q[3] tiles there (TMA) | bar_kf[2] bar_vf bar_qf[3] their last readers complete (commit) | bar_s, bar_dp S^T, dP^T
+// complete (commit; bar_s: statistics there too) | bar_sf, bar_dpf read out (8 warps) | bar_p P^T / dS^T stored (8 warps) | bar_stf[2] statistics
+// read (8 warps) | bar_dv dV complete (commit: P^T may be overwritten) | bar_d[2] dV / dK / dQ complete (commit, alternating so that a waiter two blocks behind cannot mistake a phase) |
+// bar_dqf dQ read out (4 warps) | bar_ev, bar_ek dV, dK of a key tile read out (4 warps).
+struct BwdFusedSmem {      // (full: the base is checked to be aligned instead of being aligned here)
+  static constexpr int K = 0;                            // 2 slots: an item's dQ reads K to its end
+  static constexpr int V = K + 2 * TILE_BYTES;
+  static constexpr int Q = V + TILE_BYTES;               // 3 slots
+  static constexpr int DO = Q + 3 * TILE_BYTES;          // 3 slots
   static constexpr int DST = DO + 3 * TILE_BYTES;        // 2 buffers x [128 keys x 128 queries] bf16
   static constexpr int DQS = DST + 4 * TILE_BYTES;       // dQ staging: 4 drain warps x [32 rows x 128 B] bf16, swizzled
-  static constexpr int STAT = DQS + TILE_BYTES;          // 8 warps x (-lse*log2e [64], -delta [64])
-  static constexpr int BAR = STAT + 4096;
-  static constexpr int SCHED = BAR + 256;                // this CTA's first 64 work items
-  static constexpr int TOTAL = SCHED + 768 + 1024;             // SCHED: 64 items, or a ring of 64 (value, sequence number) + end marker
+  static constexpr int STAT = DQS + TILE_BYTES;          // 2 buffers x (-lse * log2 e [128], -delta [128])
+  static constexpr int BAR = STAT + 2048;
+  static constexpr int SCHED = BAR + 256;
+  static constexpr int TOTAL = SCHED + 768;              // SCHED: this CTA's first 48 items, or a ring of 64 (value, sequence number) + end marker
 };
+static_assert(BwdFusedSmem::TOTAL <= 227 * 1024, "shared memory of an SM");
 
 constexpr int BWDF_E_WARPS = 8;       // element-wise warps: TMEM lane group (w & 3) x 64-query column half (w >> 2)
 constexpr int BWDF_D_WARPS = 4;       // drain warps: dQ partial tiles and the dK / dV epilogue, one TMEM lane group each
-// Warp w runs on scheduler w % 4.  Warp 12 stays idle so that the two MMA warps (13, 14) and the loader warp (15) land on
-// schedulers 1, 2 and 3: every scheduler then carries two element-wise warps, one drain warp and at most one light warp.
+// Warp w runs on scheduler w % 4: every scheduler carries two element-wise warps, one drain warp and one light warp.
+constexpr int BWDF_STAT_WARP = BWDF_E_WARPS + BWDF_D_WARPS;       // fetches the queries' statistics (scheduler 0)
 constexpr int BWDF_SCORE_WARP = BWDF_E_WARPS + BWDF_D_WARPS + 1;  // issues S^T / dP^T (scheduler 1)
 constexpr int BWDF_CTRL_WARP = BWDF_E_WARPS + BWDF_D_WARPS + 2;   // issues dV / dK / dQ (scheduler 2)
 constexpr int BWDF_LOAD_WARP = BWDF_CTRL_WARP + 1;                // issues every TMA load
 constexpr int BWDF_THREADS = (BWDF_LOAD_WARP + 1) * 32;
 
-template <bool DYN>
+template <bool DYN, bool STAMPS = false>      // (STAMPS: with the timeline; without, its instructions are not in anybody's way)
 __global__ void __maxnreg__(120) attn_bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tm_qkv,
                                                                             const __grid_constant__ CUtensorMap tm_do,
-                                                                            const __grid_constant__ CUtensorMap tm_dq, const AttnArgs a) {
+                                                                            const __grid_constant__ CUtensorMap tm_dq,
+                                                                            const __grid_constant__ CUtensorMap tm_out, const AttnArgs a) {
   mlb_pdl_sync();
   using S = BwdFusedSmem;
   constexpr int HD = 64;
   constexpr uint32_t TMEM_COLS = 512;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint8_t* smem = smem_raw;
   uint64_t* bars = (uint64_t*)(smem + S::BAR);
-  uint64_t *bar_kv = bars, *bar_q = bars + 1 /*[3]*/, *bar_s = bars + 4, *bar_free = bars + 5, *bar_p = bars + 6, *bar_dv = bars + 7,
-           *bar_dqf = bars + 8, *bar_epi = bars + 9, *bar_d = bars + 12 /*[2]: block blk completes bar_d[blk & 1]*/;
-  uint32_t* tmem_slot = (uint32_t*)(bars + 10);
-  volatile int* s_abort = (volatile int*)(bars + 11);
-  float* s_stat = (float*)(smem + S::STAT);   // [8 warps][-lse*log2e x64 | -delta x64]
-  {
-    __shared__ int s_skip;
-    if (threadIdx.x == 0) s_skip = *(volatile int*)&g_mlb_error;
-    __syncthreads();
-    if (s_skip != 0) return;
+  uint64_t *bar_k = bars /*[2]*/, *bar_kf = bars + 2 /*[2]*/, *bar_v = bars + 4, *bar_vf = bars + 5, *bar_q = bars + 6 /*[3]*/, *bar_qf = bars + 9 /*[3]*/,
+           *bar_s = bars + 12, *bar_sf = bars + 13, *bar_dp = bars + 14, *bar_dpf = bars + 15, *bar_p = bars + 16, *bar_dv = bars + 18,
+           *bar_d = bars + 19 /*[2]: block blk completes bar_d[blk & 1]*/, *bar_dqf = bars + 21, *bar_ev = bars + 22, *bar_ek = bars + 23;
+  uint64_t* bar_end = bars + 24;      // [2]: the MMA threads' last commits
+  uint64_t* bar_stf = bars + 26;      // [2]: statistics read
+  uint32_t* tmem_slot = (uint32_t*)(bars + 28);
+  volatile int* s_abort = (volatile int*)(bars + 29);
+  if (attn_given_up()) return;
+  if ((tc::smem_u32(smem) & 1023) != 0) {
+    if (threadIdx.x == 0) mlb_set_error(MLB_ERR_BOUNDS, 0xA2);
+    return;
   }
   const int nq = (a.T + 127) / 128;
   const int C = a.H * HD;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // Persistent CTAs: work item w = key tile kt = w / (B*H) of (sample, head) w % (B*H), so the items are in descending
   // cost order (a key tile meets the nq - kt query tiles at or after it).  A CTA's items come from the host's balanced
-  // schedule (rows end with -1 entries; the first 64 are copied to shared memory), else round robin over the grid.
+  // schedule (rows end with -1 entries), else round robin over the grid.
   const int BH = a.B * a.H, total = nq * BH;
   const int* srow = a.sched ? a.sched + (size_t)blockIdx.x * a.sched_stride : nullptr;
   int* s_sched = (int*)(smem + S::SCHED);
-  if (srow && tid < 64) s_sched[tid] = tid < a.sched_stride ? __ldg(srow + tid) : -1;
   struct Item { int kt, b, h, row0; bool valid; };
   constexpr bool dyn = DYN;
-  ItemRing ring{(volatile int*)s_sched, (volatile int*)s_sched + 64, 0};
-  if (dyn && tid <= 64) s_sched[64 + tid] = tid < 64 ? 0 : 0x7fffffff;
-  const bool publisher = warp == BWDF_LOAD_WARP && lane == 0;
-  auto item_at = [&](int li) -> Item {
-    int w;
-    if (dyn) w = publisher ? ring.draw(li, 1, total) : ring.read(li, s_abort);
-    else if (srow) w = li < 64 ? s_sched[li] : __ldg(srow + li);
-    else { w = blockIdx.x + li * gridDim.x; if (w >= total) w = -1; }
+  auto item_no = [&](int li) -> int {      // number of this CTA's li-th item, or -1
+    if (srow) return li < a.sched_stride ? __ldg(srow + li) : -1;
+    const int w = blockIdx.x + li * gridDim.x;
+    return w < total ? w : -1;
+  };
+  auto item_of = [&](int w) -> Item {
     Item r;
     r.valid = w >= 0;
     if (!r.valid) w = 0;
@@ -1433,18 +1485,33 @@ __global__ void __maxnreg__(120) attn_bwd_fused_tc_kernel(const __grid_constant_
     r.row0 = r.b * a.T;
     return r;
   };
+  // Six roles look every item up: the first 48 are taken apart once, here (dynamic: a ring of 64 numbers instead)
+  int4* s_item = (int4*)s_sched;
+  if (!dyn && tid < 48) {
+    const Item r = item_of(item_no(tid));
+    s_item[tid] = make_int4(r.valid ? r.kt : -1, r.b, r.h, r.row0);
+  }
+  ItemRing ring{(volatile int*)s_sched, (volatile int*)s_sched + 64, 0};
+  if (dyn && tid <= 64) s_sched[64 + tid] = tid < 64 ? 0 : 0x7fffffff;
+  const bool publisher = warp == BWDF_LOAD_WARP && lane == 0;
+  auto item_at = [&](int li) -> Item {
+    if (dyn) return item_of(publisher ? ring.draw(li, 1, total) : ring.read(li, s_abort));
+    if (li >= 48) return item_of(item_no(li));
+    const int4 v = s_item[li];
+    return Item{v.x, v.y, v.z, v.w, v.x >= 0};
+  };
 
   if (tid == 0) {
-    tc::mbar_init(bar_kv, 1);
-    for (int i = 0; i < 3; i++) tc::mbar_init(&bar_q[i], 1);
-    tc::mbar_init(bar_s, 1); tc::mbar_init(bar_dv, 1); tc::mbar_init(&bar_d[0], 1); tc::mbar_init(&bar_d[1], 1);
-    tc::mbar_init(bar_free, BWDF_E_WARPS); tc::mbar_init(bar_p, BWDF_E_WARPS);
-    tc::mbar_init(bar_dqf, BWDF_D_WARPS); tc::mbar_init(bar_epi, BWDF_D_WARPS);
+    for (int i = 0; i < 28; i++) {
+      const bool e = i == 13 || (i >= 15 && i <= 17) || i >= 26, d = i >= 21 && i <= 23;      // element-wise / drain warps arrive, else a thread or a commit
+      tc::mbar_init(&bars[i], e ? BWDF_E_WARPS : d ? BWDF_D_WARPS : i == 12 ? 2 : 1);         // (bar_s: the commit and the statistics warp)
+    }
     *s_abort = 0;
     tc::mbar_fence_init();
     tc::tma_prefetch_desc(&tm_qkv);
     tc::tma_prefetch_desc(&tm_do);
     tc::tma_prefetch_desc(&tm_dq);
+    tc::tma_prefetch_desc(&tm_out);
   }
   if (warp == BWDF_CTRL_WARP) tc::tmem_alloc(tmem_slot, TMEM_COLS);
   tc::tc_fence_before();
@@ -1453,59 +1520,49 @@ __global__ void __maxnreg__(120) attn_bwd_fused_tc_kernel(const __grid_constant_
   const uint32_t tmem = *tmem_slot;
   // S^T 128 | dP^T 128 | P^T (bf16 pairs) 64 | dV 64 | dK 64 | dQ 64
   const uint32_t t_st = tmem, t_dpt = tmem + 128, t_pt = tmem + 256, t_dv = tmem + 320, t_dk = tmem + 384, t_dq = tmem + 448;
-  auto wait = [&](uint64_t* bar, uint32_t phase, int where) -> bool {
-    if (tc::mbar_try(bar, phase)) return true;
-    if (*s_abort) return false;
-    if (!tc::mbar_wait(bar, phase, where)) { *s_abort = 1; return false; }
-    return true;
-  };
-  long long* tl = (a.timeline && blockIdx.x == 0 && lane == 0) ? a.timeline : nullptr;
+  auto wait = [&](uint64_t* bar, uint32_t phase, int where) { return tc::mbar_wait_sticky(bar, phase, where, s_abort); };
+  long long* tl = (STAMPS && a.timeline && blockIdx.x == 0 && lane == 0) ? a.timeline : nullptr;
 
   if (warp == BWDF_LOAD_WARP) {
     // ---------------------------------------------------------------- loader warp: every TMA load
+    // Running block blk of this CTA goes into Q / dO slot blk % 3, whatever item it is of; an item's K into slot item & 1, its V once the
+    // item before has its last dP^T.
     if (lane == 0) {
-      auto load_kv = [&](const Item& w) {
-        tc::mbar_expect_tx(bar_kv, 2 * TILE_BYTES);
-        tc::tma_load_2d(smem + S::K, &tm_qkv, bar_kv, C + w.h * HD, w.row0 + w.kt * 128);
-        tc::tma_load_2d(smem + S::V, &tm_qkv, bar_kv, 2 * C + w.h * HD, w.row0 + w.kt * 128);
-      };
-      auto load_q_do = [&](const Item& w, int i, int g) {          // g: running block number, buffer g % 3
-        const int buf = g % 3;
-        tc::mbar_expect_tx(&bar_q[buf], 2 * TILE_BYTES);
-        tc::tma_load_2d(smem + S::Q + buf * TILE_BYTES, &tm_qkv, &bar_q[buf], w.h * HD, w.row0 + i * 128);
-        tc::tma_load_2d(smem + S::DO + buf * TILE_BYTES, &tm_do, &bar_q[buf], w.h * HD, w.row0 + i * 128);
-      };
-      int blk = 0;
-      Item cur = item_at(0);
-      if (cur.valid) {
-        load_kv(cur);
-        load_q_do(cur, cur.kt, 0);
-        if (nq - cur.kt > 1) load_q_do(cur, cur.kt + 1, 1);
+      int blk = 0, nk = 0, nv = 0, odd = 0;      // odd: a block that is not counted
+      bool ok = true;
+      for (int li = 0; ok; li++) {
+        const Item w = item_at(li);
+        if (!w.valid) break;
+        for (int i = w.kt; i < nq; i++, blk++) {
+          if (i == w.kt) {
+            if (li >= 2 && !wait(&bar_kf[li & 1], ((li >> 1) + 1) & 1, 43)) { ok = false; break; }
+            nk++;
+            tc::mbar_expect_tx(&bar_k[li & 1], TILE_BYTES);
+            tc::tma_load_2d(smem + S::K + (li & 1) * TILE_BYTES, &tm_qkv, &bar_k[li & 1], C + w.h * HD, w.row0 + w.kt * 128);
+          }
+          const int buf = blk % 3;
+          if (blk >= 3 && !wait(&bar_qf[buf], (blk / 3 + 1) & 1, 44)) { ok = false; break; }
+          tc::mbar_expect_tx(&bar_q[buf], 2 * TILE_BYTES);
+          tc::tma_load_2d(smem + S::Q + buf * TILE_BYTES, &tm_qkv, &bar_q[buf], w.h * HD, w.row0 + i * 128);
+          tc::tma_load_2d(smem + S::DO + buf * TILE_BYTES, &tm_do, &bar_q[buf], w.h * HD, w.row0 + i * 128);
+          if (i == w.kt) {
+            if (li > 0 && !wait(bar_vf, (li - 1) & 1, 52)) { ok = false; odd = 1; break; }
+            nv++;
+            tc::mbar_expect_tx(bar_v, TILE_BYTES);
+            tc::tma_load_2d(smem + S::V, &tm_qkv, bar_v, 2 * C + w.h * HD, w.row0 + w.kt * 128);
+          }
+        }
       }
-      for (int li = 0; cur.valid; li++) {
-        const int kt = cur.kt;
-        const int n_it = nq - kt;
-        for (int it = 0; it < n_it; it++, blk++) {
-          // the tiles of block it+2 go where block it-1's were: its dV / dK MMAs must have finished reading them
-          // (every completion of bar_d is observed, so this thread's parity never falls a whole period behind)
-          if (blk > 0) wait(&bar_d[(blk - 1) & 1], ((blk - 1) >> 1) & 1, 43);
-          if (it + 2 < n_it) load_q_do(cur, kt + it + 2, blk + 2);
-        }
-        const Item nx = item_at(li + 1);
-        if (nx.valid) {
-          // every MMA of this key tile is complete: K, V and all Q / dO buffers are free for the next item
-          wait(&bar_d[(blk - 1) & 1], ((blk - 1) >> 1) & 1, 44);
-          load_kv(nx);
-          load_q_do(nx, nx.kt, blk);
-          if (nq - nx.kt > 1) load_q_do(nx, nx.kt + 1, blk + 1);
-        }
-        cur = nx;
+      if (*s_abort) {
+        for (int i = 0; i < 2; i++) attn_settle(&bar_k[i], (nk + 1 - i) / 2);
+        attn_settle(bar_v, nv);
+        for (int i = 0; i < 3; i++) attn_settle(&bar_q[i], (blk + odd + 2 - i) / 3);
       }
     }
   } else if (warp == BWDF_CTRL_WARP || warp == BWDF_SCORE_WARP) {
     // ---------------------------------------------------------------- two MMA warps: waits, tcgen05.mma, commits, nothing else
     // The 8 score MMAs have their own issuing thread, so they go out while the other still waits for what the 24 gradient MMAs of
-    // the previous block read.
+    // the previous block read.  Neither stops at the end of an item.
     // (Descriptors are formed by adding small constants to per-buffer bases.)
     if (tc::elect_one()) {
       constexpr uint32_t idesc_s = tc::idesc_bf16(128, 128, 0, 0);
@@ -1517,241 +1574,338 @@ __global__ void __maxnreg__(120) attn_bwd_fused_tc_kernel(const __grid_constant_
       const uint64_t dQmn = desc_base_mn(tc::smem_u32(smem + S::Q)), dDOmn = desc_base_mn(tc::smem_u32(smem + S::DO));
       const uint64_t dKmn = desc_base_mn(tc::smem_u32(smem + S::K));
       const uint64_t dSTk = desc_base_k(tc::smem_u32(smem + S::DST)), dSTmn = desc_base_mn(tc::smem_u32(smem + S::DST));
-      auto issue_scores = [&](int buf, uint32_t q_phase) {
-        if (!wait(&bar_q[buf], q_phase, 41)) return;
-        tc::tc_fence_after();
-        const uint64_t o = (uint64_t)buf * TILE_D;
-#pragma unroll
-        for (int ks = 0; ks < HD / 16; ks++) tc::mma_bf16_ss(t_st, dKk + ks * 2, dQk + o + ks * 2, idesc_s, ks > 0);
-#pragma unroll
-        for (int ks = 0; ks < HD / 16; ks++) tc::mma_bf16_ss(t_dpt, dVk + ks * 2, dDOk + o + ks * 2, idesc_s, ks > 0);
-      };
       int blk = 0, buf = 0, q_use = 0;     // buffer blk % 3 and how many times it has been filled before (blk / 3)
+      bool ok = true;
       if (warp == BWDF_SCORE_WARP) {
-        // the score products: S^T / dP^T of block j+1 as soon as block j's have been read out of TMEM
-        for (int item = 0;; item++) {
+        for (int item = 0; ok; item++) {
           const Item cur = item_at(item);
           if (!cur.valid) break;
           const int n_it = nq - cur.kt;
-          if (wait(bar_kv, item & 1, 40)) issue_scores(buf, q_use & 1);
-          tc::mma_commit(bar_s);
+          const uint64_t k = dKk + (uint64_t)(item & 1) * TILE_D;
+          ok = wait(&bar_k[item & 1], (item >> 1) & 1, 40);
           for (int it = 0; it < n_it; it++, blk++) {
-            int nbuf = buf + 1, nq_use = q_use;
-            if (nbuf == 3) { nbuf = 0; nq_use++; }
-            // S^T / dP^T of this block are in registers: the score MMAs of the next block may overwrite them
-            wait(bar_free, blk & 1, 42);
-            if (it + 1 < n_it) {
-              tc::tc_fence_after();
-              issue_scores(nbuf, nq_use & 1);
-              tc::mma_commit(bar_s);
-            }
-            buf = nbuf; q_use = nq_use;
+            // over the scores of the block before, once those have been read
+            if (!ok || !wait(&bar_q[buf], q_use & 1, 41) || (blk > 0 && !wait(bar_sf, (blk - 1) & 1, 42))) { ok = false; break; }
+            tc::tc_fence_after();
+            const uint64_t o = (uint64_t)buf * TILE_D;
+#pragma unroll
+            for (int ks = 0; ks < HD / 16; ks++) tc::mma_bf16_ss(t_st, k + ks * 2, dQk + o + ks * 2, idesc_s, ks > 0);
+            tc::mma_commit(bar_s);
+            if ((it == 0 && !wait(bar_v, item & 1, 53)) || (blk > 0 && !wait(bar_dpf, (blk - 1) & 1, 54))) { ok = false; break; }
+            tc::tc_fence_after();
+#pragma unroll
+            for (int ks = 0; ks < HD / 16; ks++) tc::mma_bf16_ss(t_dpt, dVk + ks * 2, dDOk + o + ks * 2, idesc_s, ks > 0);
+            tc::mma_commit(bar_dp);
+            if (it + 1 == n_it) tc::mma_commit(bar_vf);
+            if (++buf == 3) { buf = 0; q_use++; }
           }
         }
+        tc::mma_commit(&bar_end[0]);
+        attn_settle(&bar_end[0], 1);
       } else {
         // the gradient products of block j once P^T / dS^T are stored
-        for (int item = 0;; item++) {
+        for (int item = 0; ok; item++) {
           const Item cur = item_at(item);
           if (!cur.valid) break;
           const int n_it = nq - cur.kt;
+          const uint64_t k = dKmn + (uint64_t)(item & 1) * TILE_D;
           for (int it = 0; it < n_it; it++, blk++) {
-            bool go = wait(bar_p, blk & 1, 45);     // P^T in TMEM, dS^T in shared memory
+            const uint64_t o = (uint64_t)buf * TILE_D, od = (uint64_t)(blk & 1) * 2 * TILE_D;     // od: dS^T buffer of this block
+            const uint32_t acc = it > 0;
+            // P^T and dS^T stored, dO there; of an item's first block: the item before has its dV read out
+            if (!wait(bar_p, blk & 1, 45) || !wait(&bar_q[buf], q_use & 1, 41) || (it == 0 && item > 0 && !wait(bar_ev, (item - 1) & 1, 46))) { ok = false; break; }
             if (tl) tl[blk * 8 + 5] = clock64();
-            if (it == 0) go = wait(bar_kv, item & 1, 40) && go;       // (seen by the score thread long ago; this thread reads K too)
-            go = wait(&bar_q[buf], q_use & 1, 41) && go;
-            if (it == 0 && item > 0) go = wait(bar_epi, (item - 1) & 1, 46) && go;   // previous tile's dK / dV have been read out
-            const bool dv_go = go;
-            if (go) {
-              tc::tc_fence_after();
-              const uint64_t o = (uint64_t)buf * TILE_D;
-              const uint64_t od = (uint64_t)(blk & 1) * 2 * TILE_D;     // dS^T buffer of this block
-              const uint32_t acc = it > 0;
-#pragma unroll
-              for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ts(t_dv, t_pt + ks * 8, dDOmn + o + ks * 128, idesc_d, acc | (ks > 0));
-              tc::mma_commit(bar_dv);       // P^T's columns are free for the next block while dK and dQ are still going
-#pragma unroll
-              for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ss(t_dk, dSTk + od + (ks >> 2) * TILE_D + (ks & 3) * 2, dQmn + o + ks * 128, idesc_d, acc | (ks > 0));
-              if (blk > 0) go = wait(bar_dqf, (blk - 1) & 1, 47);   // the previous dQ tile has left TMEM
-              if (go) {
-                tc::tc_fence_after();
-#pragma unroll
-                for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ss(t_dq, dSTmn + od + ks * 128, dKmn + ks * 128, idesc_q, ks > 0);
-              }
-            }
-            if (!dv_go) tc::mma_commit(bar_dv);     // (aborting: keep the barrier's phases in step)
+            tc::tc_fence_after();
+#pragma unroll 2
+            for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ts(t_dv, t_pt + ks * 8, dDOmn + o + ks * 128, idesc_d, acc | (ks > 0));
+            tc::mma_commit(bar_dv);       // P^T's columns are free for the next block while dK and dQ are still going
+            if (it == 0 && item > 0 && !wait(bar_ek, (item - 1) & 1, 56)) { ok = false; break; }
+            tc::tc_fence_after();
+#pragma unroll 2
+            for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ss(t_dk, dSTk + od + (ks >> 2) * TILE_D + (ks & 3) * 2, dQmn + o + ks * 128, idesc_d, acc | (ks > 0));
+            // the previous dQ tile has left TMEM; K is there (the scores have seen it; this thread reads it too)
+            if ((blk > 0 && !wait(bar_dqf, (blk - 1) & 1, 47)) || (it == 0 && !wait(&bar_k[item & 1], (item >> 1) & 1, 40))) { ok = false; break; }
+            tc::tc_fence_after();
+#pragma unroll 2
+            for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ss(t_dq, dSTmn + od + ks * 128, k + ks * 128, idesc_q, ks > 0);
             tc::mma_commit(&bar_d[blk & 1]);
+            tc::mma_commit(&bar_qf[buf]);
+            if (it + 1 == n_it) tc::mma_commit(&bar_kf[item & 1]);
             if (tl) tl[blk * 8 + 6] = clock64();
             if (++buf == 3) { buf = 0; q_use++; }
           }
         }
+        tc::mma_commit(&bar_end[1]);
+        attn_settle(&bar_end[1], 1);
+      }
+    }
+  } else if (warp == BWDF_STAT_WARP) {
+    // ---------------------------------------------------------------- statistics of a block's queries, two blocks ahead at most; a query past the end
+    // has lse = +inf: p = 0.  Its arrival is one half of bar_s, so nobody waits for it apart.
+    int blk = 0;
+    bool ok = true;
+    for (int item = 0; ok; item++) {
+      const Item cur = item_at(item);
+      if (!cur.valid) break;
+      const size_t e = ((size_t)cur.b * a.H + cur.h) * a.T;
+      for (int i = cur.kt; i < nq; i++, blk++) {
+        float nl[4], nd[4];
+#pragma unroll
+        for (int x = 0; x < 4; x++) {
+          const int q = i * 128 + x * 32 + lane;
+          nl[x] = q < a.T ? -a.lse[e + q] * LOG2E : -INFINITY;
+          nd[x] = q < a.T ? -a.delta[e + q] : 0.f;
+        }
+        // (one answer for the warp: a lane whose wait has run out must not leave those behind whose wait has not)
+        if (blk >= 2 && !__all_sync(0xffffffffu, wait(&bar_stf[blk & 1], ((blk >> 1) + 1) & 1, 59))) { ok = false; break; }
+        float* stat = (float*)(smem + S::STAT) + (blk & 1) * 256;
+#pragma unroll
+        for (int x = 0; x < 4; x++) {
+          stat[x * 32 + lane] = nl[x];
+          stat[128 + x * 32 + lane] = nd[x];
+        }
+        // (of this block's phase and not of the one before)
+        if (blk > 0 && !__all_sync(0xffffffffu, wait(bar_s, (blk - 1) & 1, 51))) { ok = false; break; }
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(bar_s);
       }
     }
   } else if (warp < BWDF_E_WARPS) {
     // ---------------------------------------------------------------- 8 element-wise warps
-    const int lg = warp & 3, ch = warp >> 2, row = lg * 32 + lane;
+    const int lg = warp & 3, ch = warp >> 2;
     const uint32_t lane_addr = (uint32_t)(lg * 32) << 16;
     const float sl2 = a.scale * LOG2E;
     const uint64_t sl2x2 = pk2(sl2, sl2);
-    // per-query statistics: each warp keeps the 64 queries of its column half in a private shared-memory slot
-    // (-lse*log2e, -delta; queries past the end give P = 0).  Lane l fetches queries l and l+32 of the NEXT block while
-    // this block is processed, so neither the load latency nor a CTA-wide barrier sits between two blocks.
-    float* my_stat = s_stat + warp * 128;
-    auto fetch_stat = [&](const Item& w, int i, float (&l)[2], float (&d)[2]) {
-#pragma unroll
-      for (int u = 0; u < 2; u++) {
-        const int q = i * 128 + ch * 64 + u * 32 + lane;
-        const size_t si = ((size_t)w.b * a.H + w.h) * a.T + q;
-        l[u] = (q < a.T) ? a.lse[si] : INFINITY;
-        d[u] = (q < a.T) ? a.delta[si] : 0.f;
-      }
-    };
+    const int c0 = ch * 64;      // first query column of this warp
+    const int fr = lane >> 2, fc = 2 * (lane & 3);      // this thread's row and column in a fragment's 8 x 8 matrices
+    const uint32_t ds_base = tc::smem_u32(smem + S::DST);
     int blk = 0;
     for (int item = 0;; item++) {
       const Item cur = item_at(item);
       if (!cur.valid) break;
-      const int kt = cur.kt;
-      const int k0 = kt * 128, krow = k0 + row;
-      const int n_it = nq - kt;
-      float st_l[2], st_d[2];
-      fetch_stat(cur, kt, st_l, st_d);
+      const int kt = cur.kt, n_it = nq - kt;
       for (int it = 0; it < n_it; it++, blk++) {
-        const int i = kt + it, q0 = i * 128;
-        __syncwarp();
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-          my_stat[u * 32 + lane] = -st_l[u] * LOG2E;
-          my_stat[64 + u * 32 + lane] = -st_d[u];
-        }
-        __syncwarp();
-        if (it + 1 < n_it) fetch_stat(cur, i + 1, st_l, st_d);
+        const float* stat = (const float*)(smem + S::STAT) + (blk & 1) * 256 + c0 + fc;
         if (tl && warp == 0) tl[blk * 8 + 0] = clock64();
-        wait(bar_s, blk & 1, 48);          // S^T, dP^T of this block are complete
+        wait(bar_s, blk & 1, 48);          // S^T of this block is complete, its statistics are there
         tc::tc_fence_after();
         if (tl && warp == 0) tl[blk * 8 + 1] = clock64();
-        // dS^T of this block goes into the shared-memory tile that block blk-2's dK / dQ MMAs read
-        if (blk >= 2) wait(&bar_d[blk & 1], ((blk >> 1) + 1) & 1, 51);
-        uint32_t pw[2][16];
-        const bool diag = (it == 0);
-#pragma unroll
-        for (int hf = 0; hf < 2; hf++) {
-          uint32_t rs[32], rd[32];
-          const int c0 = ch * 64 + hf * 32;      // first query column of this pass
-          tc::tmem_ld32x2_wait(t_st + lane_addr + c0, rs, t_dpt + lane_addr + c0, rd);
-          if (hf == 1) {
+        // 32 columns at a time, and not unrolled: the instructions of all roles have to stay in the SM's cache
+#pragma unroll 1
+        for (int jh = 0; jh < 2; jh++) {
+          float p[2][16];      // [16 rows][fragment]
+          uint32_t r[2][16], w[2][8];
+          const float* st = stat + jh * 32;
+          tc::tmem_ld_frag_wait(t_st + lane_addr + c0 + jh * 32, r);
+          if (jh == 1) {
             tc::tc_fence_before();
             __syncwarp();
-            if (lane == 0) tc::mbar_arrive(bar_free);
+            if (lane == 0) tc::mbar_arrive(bar_sf);
           }
 #pragma unroll
-          for (int v8 = 0; v8 < 4; v8++) {
-            const int qc = c0 + v8 * 8;
-            const float* sn = my_stat + hf * 32 + v8 * 8;
-            float nl[8], nd[8];
-            uint32_t dw[4];
-            *reinterpret_cast<float4*>(nl) = *reinterpret_cast<const float4*>(sn);
-            *reinterpret_cast<float4*>(nl + 4) = *reinterpret_cast<const float4*>(sn + 4);
-            *reinterpret_cast<float4*>(nd) = *reinterpret_cast<const float4*>(sn + 64);
-            *reinterpret_cast<float4*>(nd + 4) = *reinterpret_cast<const float4*>(sn + 68);
+          for (int j = 0; j < 4; j++) {
+            const float2 nl = *reinterpret_cast<const float2*>(st + j * 8);
 #pragma unroll
-            for (int x = 0; x < 4; x++) {
-              const int e = v8 * 8 + 2 * x;
-              float z0, z1;
-              upk2(fma2(pk2(__uint_as_float(rs[e]), __uint_as_float(rs[e + 1])), sl2x2, pk2(nl[2 * x], nl[2 * x + 1])), z0, z1);
-              float p0 = ex2_approx(z0), p1 = ex2_approx(z1);
-              if (diag) {
-                if (q0 + qc + 2 * x < krow) p0 = 0.f;
-                if (q0 + qc + 2 * x + 1 < krow) p1 = 0.f;
+            for (int h = 0; h < 2; h++)
+#pragma unroll
+              for (int v = 0; v < 2; v++) {
+                const int e = 4 * j + 2 * v;
+                float z0, z1;
+                upk2(fma2(pk2(__uint_as_float(r[h][e]), __uint_as_float(r[h][e + 1])), sl2x2, pk2(nl.x, nl.y)), z0, z1);
+                p[h][e] = ex2_approx(z0);
+                p[h][e + 1] = ex2_approx(z1);
               }
-              const uint64_t t2 = add2(pk2(__uint_as_float(rd[e]), __uint_as_float(rd[e + 1])), pk2(nd[2 * x], nd[2 * x + 1]));
-              float d0, d1;
-              upk2(mul2(pk2(p0, p1), t2), d0, d1);
-              pw[hf][v8 * 4 + x] = pack_bf16(p0, p1);
-              dw[x] = pack_bf16(d0, d1);
-            }
-            // dS^T goes straight into the buffer that block blk-2 used: only the two TMEM stores of P^T are left to do
-            // once the previous block's dV MMAs are out of the way
-            *reinterpret_cast<uint4*>(smem + S::DST + (blk & 1) * 2 * TILE_BYTES + sw_off(row, qc)) = make_uint4(dw[0], dw[1], dw[2], dw[3]);
           }
+          if (it == 0 && c0 + jh * 32 <= lg * 32) {      // the diagonal block: no query before the key (8 x 8 matrices under, on and over the diagonal)
+            const bool under = c0 + jh * 32 < lg * 32;
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+#pragma unroll
+              for (int e = 0; e < 16; e++) {
+                const int j = e >> 2, row8 = 2 * h + ((e >> 1) & 1);
+                if (under || j < row8 || (j == row8 && fc + (e & 1) < fr)) p[h][e] = 0.f;
+              }
+          }
+#pragma unroll
+          for (int h = 0; h < 2; h++)
+#pragma unroll
+            for (int x = 0; x < 8; x++) w[h][x] = pack_bf16(p[h][2 * x], p[h][2 * x + 1]);
+          if (jh == 0) {
+            // P^T's TMEM columns belong to the previous block's dV MMAs until they complete.  (dS^T goes into the tile that block blk-2's dK / dQ
+            // MMAs read: complete then too, they were committed before that dV.)
+            if (blk > 0) wait(bar_dv, (blk - 1) & 1, 49);
+            wait(bar_dp, blk & 1, 57);
+            __syncwarp();
+            tc::tc_fence_after();
+          }
+          tc::tmem_st_frag(t_pt + lane_addr + ch * 32 + jh * 16, w);
+          tc::tmem_ld_frag_wait(t_dpt + lane_addr + c0 + jh * 32, r);
+          if (jh == 1) {
+            tc::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(bar_dpf);
+          }
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            const float2 nd = *reinterpret_cast<const float2*>(st + 128 + j * 8);
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+#pragma unroll
+              for (int v = 0; v < 2; v++) {
+                const int e = 4 * j + 2 * v;
+                float d0, d1;
+                upk2(mul2(pk2(p[h][e], p[h][e + 1]), add2(pk2(__uint_as_float(r[h][e]), __uint_as_float(r[h][e + 1])), pk2(nd.x, nd.y))), d0, d1);
+                w[h][2 * j + v] = pack_bf16(d0, d1);
+              }
+          }
+          // lane l has the address of row l % 8 of matrix l / 8: rows + 8 (l / 8 % 2), columns + 8 (l / 16)
+#pragma unroll
+          for (int h = 0; h < 2; h++)
+#pragma unroll
+            for (int j = 0; j < 4; j += 2)
+              tc::stmatrix_x4(ds_base + (blk & 1) * 2 * TILE_BYTES + sw_off(lg * 32 + h * 16 + (lane & 15), c0 + jh * 32 + j * 8 + (lane >> 4) * 8),
+                              w[h][2 * j], w[h][2 * j + 1], w[h][2 * j + 2], w[h][2 * j + 3]);
         }
-        tc::fence_async_smem();
         if (tl && warp == 0) tl[blk * 8 + 2] = clock64();
-        // P^T's TMEM columns belong to the previous block's dV MMAs until they complete
-        if (blk > 0) { wait(bar_dv, (blk - 1) & 1, 49); tc::tc_fence_after(); }
-        if (tl && warp == 0) tl[blk * 8 + 3] = clock64();
-        tc::tmem_st16(t_pt + lane_addr + ch * 32, pw[0]);
-        tc::tmem_st16(t_pt + lane_addr + ch * 32 + 16, pw[1]);
         tc::tmem_st_wait();
-
         tc::tc_fence_before();
+        tc::fence_async_smem();
         __syncwarp();
-        if (lane == 0) tc::mbar_arrive(bar_p);
-        if (tl && warp == 0) tl[blk * 8 + 4] = clock64();
+        if (lane == 0) {
+          tc::mbar_arrive(bar_p);
+          tc::mbar_arrive(&bar_stf[blk & 1]);
+        }
+        if (tl && warp == 0) tl[blk * 8 + 3] = tl[blk * 8 + 4] = clock64();
       }
     }
   } else if (warp < BWDF_E_WARPS + BWDF_D_WARPS) {
     // ---------------------------------------------------------------- 4 drain warps
-    // dQ partial of (query block i, this key tile): TMEM -> bf16 -> its own tile of the partial buffer (a full 128-byte
-    // row per thread; no atomics, the finishing kernel adds the key tiles' partials in a fixed order); after the last
-    // block of a key tile also dK (scaled, RoPE backward) and dV.
-    const int lg = warp & 3, row = lg * 32 + lane;
+    // dQ partial of (query block i, this key tile): TMEM -> bf16 -> its own tile of the partial buffer (no atomics, the finishing kernel adds
+    // the key tiles' partials in a fixed order); after the last block of a key tile also dV and dK (scaled, RoPE backward).  The accumulators are handed back as soon as they are in registers: the
+    // next item's products wait for no more than that.
+    const int lg = warp & 3, fr = lane >> 2, fc = 2 * (lane & 3);
     const uint32_t lane_addr = (uint32_t)(lg * 32) << 16;
     const int npairs = nq * (nq + 1) / 2;
     uint8_t* stage = smem + S::DQS + lg * 4096;
+    const uint32_t stage_u32 = tc::smem_u32(stage);
     if (warp != BWDF_E_WARPS) tl = nullptr;
     int blk = 0;
     for (int item = 0;; item++) {
       const Item cur = item_at(item);
       if (!cur.valid) break;
       const int kt = cur.kt, b = cur.b, h = cur.h, row0 = cur.row0;
-      const int krow = kt * 128 + row;
       const int n_it = nq - kt;
-      for (int it = 0; it < n_it; it++, blk++) {
-        const int i = kt + it;
-        wait(&bar_d[blk & 1], (blk >> 1) & 1, 50);          // dV, dK, dQ MMAs of this block are complete
-        tc::tc_fence_after();
-        uint32_t r0[32], r1[32];
-        tc::tmem_ld32x2_wait(t_dq + lane_addr, r0, t_dq + lane_addr + 32, r1);
+      // RoPE's tables for 16 rows of the warp's 32, laid out as a fragment: columns 8 j + fc, + 1 of rows 8 v + fr
+      float2 tc2[8], ts2[8];
+      auto tables = [&](int h) {
+#pragma unroll
+        for (int v = 0; v < 2; v++) {
+          const size_t at = (size_t)min(kt * 128 + lg * 32 + h * 16 + v * 8 + fr, a.T - 1) * (HD / 2) + fc;
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            tc2[2 * j + v] = __ldg(reinterpret_cast<const float2*>(a.cosT + at + j * 8));
+            ts2[2 * j + v] = __ldg(reinterpret_cast<const float2*>(a.sinT + at + j * 8));
+          }
+        }
+      };
+      auto handed_back = [&](uint64_t* free_bar) {      // the accumulator is in registers, its columns are the MMA thread's again
         tc::tc_fence_before();
         __syncwarp();
-        if (lane == 0) tc::mbar_arrive(bar_dqf);
-        // bf16 rows go through a swizzled staging tile and leave with ONE TMA store per warp: per-lane stores to 32
-        // different lines would occupy the load/store unit that the element-wise warps need at the same moment
-        if (lane == 0) tc::tma_wait_group_read<0>();      // the previous tile has been read out of the staging buffer
+        if (lane == 0) tc::mbar_arrive(free_bar);
+      };
+      // 32 bf16 rows go through a swizzled staging tile and leave with ONE TMA store per warp: stores to 16 or 32 lines an instruction would
+      // occupy the load/store unit that the element-wise warps need at the same moment
+      auto stage_free = [&]() {      // the tile before has been read out of the staging buffer
+        if (lane == 0) tc::tma_wait_group_read<0>();
         __syncwarp();
-        uint8_t* rowp = stage + lane * 128;
+      };
+      auto stage_tile = [&](uint32_t taddr, uint64_t* free_bar) {
+        stage_free();
 #pragma unroll
-        for (int v = 0; v < 8; v++) {
-          const uint32_t* src = (v < 4) ? &r0[v * 8] : &r1[(v - 4) * 8];
-          uint4 pk;
-          pk.x = pack_bf16(__uint_as_float(src[0]), __uint_as_float(src[1]));
-          pk.y = pack_bf16(__uint_as_float(src[2]), __uint_as_float(src[3]));
-          pk.z = pack_bf16(__uint_as_float(src[4]), __uint_as_float(src[5]));
-          pk.w = pack_bf16(__uint_as_float(src[6]), __uint_as_float(src[7]));
-          *reinterpret_cast<uint4*>(rowp + ((v ^ (lane & 7)) << 4)) = pk;
+        for (int hf = 0; hf < 2; hf++) {
+          uint32_t r[32];
+          tc::tmem_ld32_wait(taddr + lane_addr + hf * 32, r);
+          if (hf == 1) handed_back(free_bar);
+#pragma unroll
+          for (int v = 0; v < 4; v++)
+            *reinterpret_cast<uint4*>(stage + lane * 128 + (((hf * 4 + v) ^ (lane & 7)) << 4)) = pack8(reinterpret_cast<const float*>(&r[v * 8]));
         }
+      };
+      auto stage_send = [&](const CUtensorMap* m, int x, int y) {
         tc::fence_async_smem();
         __syncwarp();
         if (lane == 0) {
-          tc::tma_store_2d(&tm_dq, stage, h * HD, (int)((((long)b * npairs + (i * (i + 1) / 2 + kt)) * 128) + lg * 32));
+          if (!*s_abort) tc::tma_store_2d(m, stage, x, y);
           tc::tma_commit_group();
         }
+      };
+      const int krow0 = row0 + kt * 128 + lg * 32, nlive = a.T - (kt * 128 + lg * 32);
+      // dK (x = C) or dV (2 C).  Rows past the sample's end are the next sample's: a part of a tile is stored by row.
+      auto send_grad = [&](int x) {
+        x += h * HD;
+        if (nlive >= 32) { stage_send(&tm_out, x, krow0); return; }
+        __syncwarp();
+#pragma unroll 1
+        for (int r = lane >> 3; r < nlive && !*s_abort; r += 4)
+          *reinterpret_cast<uint4*>(a.out + (size_t)(krow0 + r) * 3 * C + x + (lane & 7) * 8) =
+              *reinterpret_cast<const uint4*>(stage + r * 128 + (((lane & 7) ^ (r & 7)) << 4));
+        __syncwarp();
+      };
+      for (int it = 0; it < n_it; it++, blk++) {
+        const int i = kt + it;
+        if (it + 1 == n_it) {      // dV is complete before dK and dQ
+          if (a.cosT) tables(0);
+          wait(bar_dv, blk & 1, 58);
+          __syncwarp();
+          tc::tc_fence_after();
+          stage_tile(t_dv, bar_ev);
+          send_grad(2 * C);
+        }
+        wait(&bar_d[blk & 1], (blk >> 1) & 1, 50);          // dV, dK, dQ MMAs of this block are complete
+        __syncwarp();
+        tc::tc_fence_after();
+        stage_tile(t_dq, bar_dqf);
+        stage_send(&tm_dq, h * HD, (int)((((long)b * npairs + (i * (i + 1) / 2 + kt)) * 128) + lg * 32));
         if (tl && warp == BWDF_E_WARPS) tl[blk * 8 + 7] = clock64();
       }
-      // the wait above covered the last block: dV and dK of this key tile are final
-      {
-        bf16* dk = a.out + ((size_t)(row0 + krow)) * 3 * C + C + h * HD;
-        const int nlive = *s_abort ? 0 : a.T - (krow - lane);
-        store_pairs_rope<HD>(dk, 3L * C, t_dk + lane_addr, 0, lane, nlive, a.cosT, a.sinT, krow, a.scale);
-        store_pairs_rope<HD>(dk + C, 3L * C, t_dv + lane_addr, 0, lane, nlive, nullptr, nullptr, krow, 1.f);
+      // the wait above covered the last block: dK of this key tile is final
+      stage_free();
+#pragma unroll 1
+      for (int half = 0; half < 2; half++) {      // 16 rows
+        uint32_t x0[16], x1[16];
+        tc::tmem_ld_frag16x2_wait(t_dk + lane_addr + ((uint32_t)(half * 16) << 16), x0, x1);
+        if (half == 1) handed_back(bar_ek);
+        uint32_t w0[8], w1[8];
+#pragma unroll
+        for (int m = 0; m < 8; m++) {
+          float a0 = __uint_as_float(x0[2 * m]) * a.scale, a1 = __uint_as_float(x1[2 * m]) * a.scale;
+          float b0 = __uint_as_float(x0[2 * m + 1]) * a.scale, b1 = __uint_as_float(x1[2 * m + 1]) * a.scale;
+          if (a.cosT) {      // d0' = d0 c + d1 s, d1' = d1 c - d0 s
+            const float d0 = a0, e0 = b0;
+            a0 = d0 * tc2[m].x + a1 * ts2[m].x;
+            a1 = a1 * tc2[m].x - d0 * ts2[m].x;
+            b0 = e0 * tc2[m].y + b1 * ts2[m].y;
+            b1 = b1 * tc2[m].y - e0 * ts2[m].y;
+          }
+          w0[m] = pack_bf16(a0, b0);
+          w1[m] = pack_bf16(a1, b1);
+        }
+        if (half == 0 && a.cosT) tables(1);
+        const int r = half * 16 + (lane & 15);
+#pragma unroll
+        for (int j = 0; j < 4; j += 2) {
+          const int u = j + (lane >> 4);
+          tc::stmatrix_x4(stage_u32 + r * 128 + ((u ^ (r & 7)) << 4), w0[2 * j], w0[2 * j + 1], w0[2 * j + 2], w0[2 * j + 3]);
+          tc::stmatrix_x4(stage_u32 + r * 128 + (((u + 4) ^ (r & 7)) << 4), w1[2 * j], w1[2 * j + 1], w1[2 * j + 2], w1[2 * j + 3]);
+        }
       }
-      tc::tc_fence_before();
-      __syncwarp();
-      if (lane == 0) tc::mbar_arrive(bar_epi);
+      send_grad(C);
     }
     if (lane == 0) tc::tma_wait_group<0>();     // every partial tile of this warp has been written
   }
   tc::tc_fence_before();
   __syncthreads();
+  if (tid == 0) tc::report_given_up(s_abort);
   if (warp == BWDF_CTRL_WARP) tc::tmem_dealloc(tmem, TMEM_COLS);
   if (dyn && tid == 0) attn_ctr_leave(1);
 }
@@ -1944,7 +2098,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_q_tc_kernel(const __g
   tc::tc_fence_after();
   if (__all_sync(0xffffffffu, ok) && cq == 0) {
     bf16* dst = a.out + ((size_t)(row0 + qrow)) * 3 * C + h * HD;
-    store_pairs_rope<HD>(dst, 3L * C, t_dq + lane_addr, 0, lane, a.T - (qrow - lane), a.cosT, a.sinT, qrow);
+    store_row_pairs<HD>(dst, 3L * C, t_dq + lane_addr, lane, a.T - (qrow - lane), a.cosT, a.sinT, qrow);
   }
   tc::tc_fence_before();
   __syncthreads();
@@ -2217,21 +2371,22 @@ MLB_API int mlb_attn_fwd(void* out, float* lse, const void* qkv, int B, int T, i
       const CUtensorMap* to = (T % 128 == 0 && g_fwd_rows >= 2) ? mlb_tmap_cached(out, (uint64_t)B * T, C, C, 32, 64, 2) : nullptr;
       a.out_tma = to != nullptr;
       if (!to) to = tm;      // unused by the kernel then
-#define MLB_FWD2(MODE)                                                                                                             \
+#define MLB_FWD2(...)                                                                                                              \
   {                                                                                                                            \
-    static int once = set_smem(attn_fwd_rows_tc_kernel<MODE>, Fwd2Smem::TOTAL);                                          \
+    static int once = set_smem(attn_fwd_rows_tc_kernel<__VA_ARGS__>, Fwd2Smem::TOTAL);                                          \
     (void)once;                                                                                                                \
-    mlb_launch_tmem(pairs <= sms, attn_fwd_rows_tc_kernel<MODE>, grid2, dim3(FWD2_THREADS), Fwd2Smem::TOTAL, st, *tm, *to, a);              \
+    mlb_launch_tmem(pairs <= sms, attn_fwd_rows_tc_kernel<__VA_ARGS__>, grid2, dim3(FWD2_THREADS), Fwd2Smem::TOTAL, st, *tm, *to, a);       \
   }
-      if (a.dynamic && g_fwd_rows != 1 && g_fwd_rows != 2) {
-        static int once = set_smem(attn_fwd_rows_tc_kernel<3, true>, Fwd2Smem::TOTAL);
-        (void)once;
-        mlb_launch_tmem(pairs <= sms, attn_fwd_rows_tc_kernel<3, true>, grid2, dim3(FWD2_THREADS), Fwd2Smem::TOTAL, st, *tm, *to, a);
+      if (a.dynamic) {
+        MLB_FWD2(3, true)
       } else {
         switch (g_fwd_rows) {
           case 1: MLB_FWD2(1) break;
           case 2: MLB_FWD2(2) break;
-          default: MLB_FWD2(3) break;
+          default:
+            if (a.timeline) MLB_FWD2(3, false, true)
+            else MLB_FWD2(3)
+            break;
         }
       }
 #undef MLB_FWD2
@@ -2326,10 +2481,8 @@ static int attn_bwd_impl(void* dqkv, const void* dout, const void* qkv, const vo
       // single fused kernel + dQ finish; the partial buffer is [B * nq(nq+1)/2 * 128 rows, C] bf16
       const long nqh = (T + 127) / 128;
       const CUtensorMap* tpart = mlb_tmap_cached(dq_part, (uint64_t)B * (nqh * (nqh + 1) / 2) * 128, C, C, 32, 64, 2);
-      if (!tpart) return -2;
-      static int o0 = set_smem(attn_bwd_fused_tc_kernel<false>, BwdFusedSmem::TOTAL);
-      static int o1 = set_smem(attn_bwd_fused_tc_kernel<true>, BwdFusedSmem::TOTAL);
-      (void)o0; (void)o1;
+      const CUtensorMap* tout = mlb_tmap_cached(dqkv, (uint64_t)B * T, 3 * C, 3 * C, 32, 64, 2);      // dK and dV leave through it
+      if (!tpart || !tout) return -2;
       // persistent CTAs, one per SM, over the (key tile, sample, head) items
       int sms = 0, devid = 0;
       cudaGetDevice(&devid);
@@ -2341,8 +2494,16 @@ static int attn_bwd_impl(void* dqkv, const void* dout, const void* qkv, const vo
       const SchedUse sched = (n_items > sms && !a.dynamic) ? attn_schedule(1, B, H, T, (int)grid_f.x, st) : SchedUse{};
       a.sched = sched.table;
       a.sched_stride = sched.stride;
-      if (a.dynamic) mlb_launch_tmem(n_items <= sms, attn_bwd_fused_tc_kernel<true>, grid_f, dim3(BWDF_THREADS), BwdFusedSmem::TOTAL, st, *tq, *td, *tpart, a);
-      else mlb_launch_tmem(n_items <= sms, attn_bwd_fused_tc_kernel<false>, grid_f, dim3(BWDF_THREADS), BwdFusedSmem::TOTAL, st, *tq, *td, *tpart, a);
+#define MLB_BWDF(...)                                                                                                                        \
+  {                                                                                                                                          \
+    static int once = set_smem(attn_bwd_fused_tc_kernel<__VA_ARGS__>, BwdFusedSmem::TOTAL);                                                  \
+    (void)once;                                                                                                                              \
+    mlb_launch_tmem(n_items <= sms, attn_bwd_fused_tc_kernel<__VA_ARGS__>, grid_f, dim3(BWDF_THREADS), BwdFusedSmem::TOTAL, st, *tq, *td, *tpart, *tout, a); \
+  }
+      if (a.dynamic) MLB_BWDF(true)
+      else if (a.timeline) MLB_BWDF(false, true)
+      else MLB_BWDF(false)
+#undef MLB_BWDF
       const long groups = (long)B * T * H * (hd / 32);
       mlb_launch(attn_dq_finish_k, dim3((unsigned)((groups + 255) / 256)), dim3(256), 0, st, (bf16*)dqkv, (const bf16*)dq_part, (long)B * T, T, H, hd, scale, cosT, sinT);
       cudaError_t e = cudaGetLastError();

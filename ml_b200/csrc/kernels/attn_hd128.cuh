@@ -86,13 +86,7 @@ __global__ void __maxnreg__(160) attn_fwd128_k(const __grid_constant__ CUtensorM
   __syncthreads();
   tc::tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  auto wait = [&](uint64_t* bar, uint32_t phase, int where) -> bool {
-    if (tc::mbar_try(bar, phase)) return true;
-    if (*s_abort) return false;
-    if (tc::mbar_wait(bar, phase, where)) return true;
-    *s_abort = 1;
-    return false;
-  };
+  auto wait = [&](uint64_t* bar, uint32_t phase, int where) { return tc::mbar_wait_sticky(bar, phase, where, s_abort); };
   // item w = pair (heaviest first) of (sample, head); tile t of it has n(t) key blocks (none when the pair has no second tile)
   struct Item { int pair, b, h, nkb; };
   auto item_of = [&](int w) {
@@ -322,6 +316,7 @@ __global__ void __maxnreg__(160) attn_fwd128_k(const __grid_constant__ CUtensorM
   }
   tc::tc_fence_before();
   __syncthreads();
+  if (tid == 0) tc::report_given_up(s_abort);
   if (warp == 8) tc::tmem_dealloc(tmem, 512);
 }
 
@@ -373,12 +368,13 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw;
   uint64_t* bars = (uint64_t*)(smem + S::BAR);
-  uint64_t *bar_kv = bars, *bar_kvf = bars + 1, *bar_q = bars + 2 /*[2]*/, *bar_qf = bars + 4 /*[2]*/, *bar_do = bars + 6 /*[2]*/, *bar_dof = bars + 8 /*[2]*/,
+  uint64_t *bar_k = bars, *bar_kf = bars + 1, *bar_q = bars + 2 /*[2]*/, *bar_qf = bars + 4 /*[2]*/, *bar_do = bars + 6 /*[2]*/, *bar_dof = bars + 8 /*[2]*/,
            *bar_s = bars + 10, *bar_dp = bars + 11, *bar_p = bars + 12, *bar_ds = bars + 13, *bar_done = bars + 14;
   uint64_t* bar_end = bars + 15;      // [2]: the MMA threads' last commits
   uint64_t *bar_sr = bars + 17 /* S^T read out */, *bar_st = bars + 18 /*[2] statistics there */, *bar_stf = bars + 20 /*[2] read */;
-  uint32_t* tmem_slot = (uint32_t*)(bars + 22);
-  volatile int* s_abort = (volatile int*)(bars + 23);
+  uint64_t *bar_v = bars + 22, *bar_vf = bars + 23;
+  uint32_t* tmem_slot = (uint32_t*)(bars + 24);
+  volatile int* s_abort = (volatile int*)(bars + 25);
   if (attn_given_up()) return;
   if ((tc::smem_u32(smem) & 1023) != 0) {
     if (threadIdx.x == 0) mlb_set_error(MLB_ERR_BOUNDS, 0xA1);
@@ -391,7 +387,7 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
   if (srow && tid < 64) s_sched[tid] = tid < a.sched_stride ? __ldg(srow + tid) : -1;
   const ItemList items{srow, s_sched, (int)blockIdx.x, (int)gridDim.x, nq * BH};
   if (tid == 0) {
-    for (int i = 0; i < 22; i++) tc::mbar_init(&bars[i], (i == 12 || i == 13 || i == 17 || i >= 20) ? BWD128_E_WARPS : 1);
+    for (int i = 0; i < 24; i++) tc::mbar_init(&bars[i], (i == 12 || i == 13 || i == 17 || i == 20 || i == 21) ? BWD128_E_WARPS : 1);
     *s_abort = 0;
     tc::mbar_fence_init();
     tc::tma_prefetch_desc(&tm);
@@ -403,38 +399,42 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
   tc::tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const uint32_t t_s = tmem, t_dp = tmem + 128, t_dv = tmem + 256, t_dk = tmem + 384;
-  auto wait = [&](uint64_t* bar, uint32_t phase, int where) -> bool {
-    if (tc::mbar_try(bar, phase)) return true;
-    if (*s_abort) return false;
-    if (tc::mbar_wait(bar, phase, where)) return true;
-    *s_abort = 1;
-    return false;
-  };
+  auto wait = [&](uint64_t* bar, uint32_t phase, int where) { return tc::mbar_wait_sticky(bar, phase, where, s_abort); };
   // item w = key tile (heaviest, the first, first) of (sample, head)
   if (warp == BWD128_LOAD_WARP) {
     if (lane == 0) {
-      int g = 0, nkv = 0;
+      // The next key tile's K is asked for when the last S^T of this one is there, its V when the last dP^T is: they arrive under the
+      // rest of this tile's products and its epilogue
+      int g = 0, nk = 0, nv = 0, odd = 0;      // odd: a block that is not counted
       bool ok = true;
       for (int li = 0, w; ok && (w = items.at(li)) >= 0; li++) {
         const int kt = w / BH, bh = w % BH, b = bh / a.H, xh = (bh % a.H) * H128;
-        if (li > 0 && !wait(bar_kvf, (li - 1) & 1, 61)) break;
-        nkv++;
-        tc::mbar_expect_tx(bar_kv, 2 * T128_BYTES);
-        split_load<2>(smem + S::K, &tm, bar_kv, C + xh, kt * 128, b, 2);
-        split_load<2>(smem + S::V, &tm, bar_kv, 2 * C + xh, kt * 128, b, 2);
         for (int i = kt; i < nq; i++, g++) {
           const int sl = g & 1, ph = ((g >> 1) + 1) & 1;
+          if (i == kt) {
+            if (li > 0 && !wait(bar_kf, (li - 1) & 1, 61)) { ok = false; break; }
+            nk++;
+            tc::mbar_expect_tx(bar_k, T128_BYTES);
+            split_load<2>(smem + S::K, &tm, bar_k, C + xh, kt * 128, b, 2);
+          }
           if (g >= 2 && !wait(&bar_qf[sl], ph, 62)) { ok = false; break; }      // (dK comes after dV, and after the dP^T its dS^T was made of)
           tc::mbar_expect_tx(&bar_q[sl], T128_BYTES);
           split_load<2>(smem + S::Q + sl * T128_BYTES, &tm, &bar_q[sl], xh, i * 128, b, 2);
           tc::mbar_expect_tx(&bar_do[sl], T128_BYTES);
           split_load<2>(smem + S::DO + sl * T128_BYTES, &tm_do, &bar_do[sl], xh, i * 128, b, 2);
+          if (i == kt) {
+            if (li > 0 && !wait(bar_vf, (li - 1) & 1, 88)) { ok = false; odd = 1; break; }
+            nv++;
+            tc::mbar_expect_tx(bar_v, T128_BYTES);
+            split_load<2>(smem + S::V, &tm, bar_v, 2 * C + xh, kt * 128, b, 2);
+          }
         }
       }
-      attn_settle(bar_kv, nkv);
+      attn_settle(bar_k, nk);
+      attn_settle(bar_v, nv);
       for (int i = 0; i < 2; i++) {
-        attn_settle(&bar_q[i], (g + 1 - i) / 2);
-        attn_settle(&bar_do[i], (g + 1 - i) / 2);
+        attn_settle(&bar_q[i], (g + odd + 1 - i) / 2);
+        attn_settle(&bar_do[i], (g + odd + 1 - i) / 2);
       }
     }
   } else if (warp == BWD128_MMA_WARP) {
@@ -446,7 +446,7 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
       bool ok = true;
       for (int li = 0, w; ok && (w = items.at(li)) >= 0; li++) {
         const int n = nq - w / BH;
-        ok = wait(bar_kv, li & 1, 66);
+        ok = wait(bar_k, li & 1, 66);
         for (int i = 0; i < n; i++, g++) {
           const int sl = g & 1, ph = (g >> 1) & 1;
           // over the scores of the block before, once those have been read
@@ -456,13 +456,15 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
 #pragma unroll
           for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ss(t_s, dK + off_k(ks, TILE_BYTES), dQ + off_k(ks, TILE_BYTES), idesc_s, ks > 0);
           tc::mma_commit(bar_s);
+          if (i == n - 1) tc::mma_commit(bar_kf);
+          if (i == 0) ok = wait(bar_v, li & 1, 89);
           // over dS^T of the block before, which its dK reads
-          if (!wait(&bar_do[sl], ph, 65) || (g > 0 && !wait(&bar_qf[sl ^ 1], ((g - 1) >> 1) & 1, 84))) { ok = false; break; }
+          if (!ok || !wait(&bar_do[sl], ph, 65) || (g > 0 && !wait(&bar_qf[sl ^ 1], ((g - 1) >> 1) & 1, 84))) { ok = false; break; }
           tc::tc_fence_after();
 #pragma unroll
           for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ss(t_dp, dV + off_k(ks, TILE_BYTES), dO + off_k(ks, TILE_BYTES), idesc_s, ks > 0);
           tc::mma_commit(bar_dp);
-          if (i == n - 1) tc::mma_commit(bar_kvf);
+          if (i == n - 1) tc::mma_commit(bar_vf);
         }
       }
       tc::mma_commit(&bar_end[0]);
@@ -480,7 +482,9 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
         for (int i = 0; i < n; i++, g++) {
           const int sl = g & 1;
           const uint64_t gQ = gQ0 + sl * T128_UNITS, gO = gO0 + sl * T128_UNITS;
-          if (!wait(bar_p, g & 1, 67)) { ok = false; break; }      // (of an item's first block: also the accumulators of the previous item have been read out)
+          // (of an item's first block bar_p says too that the accumulators of the previous item have been read out; P^T is there without dP^T,
+          // so that dO is has to be asked for)
+          if (!wait(bar_p, g & 1, 67) || !wait(&bar_do[sl], (g >> 1) & 1, 93)) { ok = false; break; }
           tc::tc_fence_after();
 #pragma unroll
           for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ss(t_dv, aP + off_k(ks, TILE_BYTES), gO + off_mn(ks), idesc_g, (i > 0 || ks > 0));
@@ -591,19 +595,25 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
           tc::mbar_arrive(&bar_stf[g & 1]);
         }
       }
-      // ---- epilogue: a warp stores 64 columns of dK (quarters 0, 1; softmax scale and RoPE's backward rotation applied) or dV (2, 3)
+      // ---- epilogue: of dV, which is complete before dK, and then of dK (softmax scale and RoPE's backward rotation applied) every warp
+      // stores 32 columns; the rotation tables are on their way from the start
+      RopeUnits rp;
+      if (a.cosT) rope_units<H128>(rp, a.cosT, a.sinT, krow, qd * 16, lane, a.T - (krow - lane));
+      wait(&bar_dof[(g - 1) & 1], ((g - 1) >> 1) & 1, 90);
+      __syncwarp();
+      tc::tc_fence_after();
+      bf16* dst = a.out + ((size_t)(b * a.T + krow)) * 3 * C + C + h * H128;
+      store_pairs16<H128>(dst + C, 3L * C, t_dv + lane_addr, qd * 16, lane, *s_abort ? 0 : a.T - (krow - lane), 1.f, false, rp);
       wait(bar_done, li & 1, 71);
       __syncwarp();
       tc::tc_fence_after();
-      const bool is_k = qd < 2;
-      bf16* dst = a.out + ((size_t)(b * a.T + krow)) * 3 * C + (is_k ? C : 2 * C) + h * H128;
-      store_pairs_rope<H128>(dst, 3L * C, (is_k ? t_dk : t_dv) + lane_addr, (qd & 1) * 32, lane, *s_abort ? 0 : a.T - (krow - lane),
-                             is_k ? a.cosT : nullptr, is_k ? a.sinT : nullptr, krow, is_k ? a.scale : 1.f);
+      store_pairs16<H128>(dst, 3L * C, t_dk + lane_addr, qd * 16, lane, *s_abort ? 0 : a.T - (krow - lane), a.scale, a.cosT != nullptr, rp);
       tc::tc_fence_before();
     }
   }
   tc::tc_fence_before();
   __syncthreads();
+  if (tid == 0) tc::report_given_up(s_abort);
   if (warp == BWD128_MMA_WARP) tc::tmem_dealloc(tmem, 512);
 }
 
@@ -614,12 +624,13 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = (uint64_t*)(smem + S::BAR);
-  uint64_t *bar_x = bars, *bar_xf = bars + 1, *bar_k = bars + 2 /*[3]*/, *bar_kf = bars + 5 /*[3]*/, *bar_v = bars + 8 /*[2]*/, *bar_vf = bars + 10 /*[2]*/,
+  uint64_t *bar_q = bars, *bar_qf = bars + 1, *bar_k = bars + 2 /*[3]*/, *bar_kf = bars + 5 /*[3]*/, *bar_v = bars + 8 /*[2]*/, *bar_vf = bars + 10 /*[2]*/,
            *bar_s = bars + 12 /*[2]*/, *bar_dp = bars + 14, *bar_done = bars + 15,
            *bar_ds = bars + 16 /*[2]: the thread that issues dQ may be a block behind*/;
   uint64_t* bar_end = bars + 18;      // [2]: the MMA threads' last commits
-  uint32_t* tmem_slot = (uint32_t*)(bars + 20);
-  volatile int* s_abort = (volatile int*)(bars + 21);
+  uint64_t *bar_o = bars + 20 /* dO */, *bar_of = bars + 21;
+  uint32_t* tmem_slot = (uint32_t*)(bars + 22);
+  volatile int* s_abort = (volatile int*)(bars + 23);
   if (attn_given_up()) return;
   const int nq = (a.T + 127) / 128, BH = a.B * a.H, C = a.H * H128;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -628,7 +639,7 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
   if (srow && tid < 64) s_sched[tid] = tid < a.sched_stride ? __ldg(srow + tid) : -1;
   const ItemList items{srow, s_sched, (int)blockIdx.x, (int)gridDim.x, nq * BH};
   if (tid == 0) {
-    for (int i = 0; i < 20; i++) tc::mbar_init(&bars[i], (i == 16 || i == 17) ? BWD128_E_WARPS : 1);
+    for (int i = 0; i < 22; i++) tc::mbar_init(&bars[i], (i == 16 || i == 17) ? BWD128_E_WARPS : 1);
     *s_abort = 0;
     tc::mbar_fence_init();
     tc::tma_prefetch_desc(&tm);
@@ -640,36 +651,39 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
   tc::tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const uint32_t t_dp = tmem + 256, t_dq = tmem + 384;      // S buffers at +0 and +128
-  auto wait = [&](uint64_t* bar, uint32_t phase, int where) -> bool {
-    if (tc::mbar_try(bar, phase)) return true;
-    if (*s_abort) return false;
-    if (tc::mbar_wait(bar, phase, where)) return true;
-    *s_abort = 1;
-    return false;
-  };
+  auto wait = [&](uint64_t* bar, uint32_t phase, int where) { return tc::mbar_wait_sticky(bar, phase, where, s_abort); };
   // item w = query tile (heaviest, the last, first) of (sample, head), with qt + 1 key blocks
   if (warp == BWD128_LOAD_WARP) {
     if (lane == 0) {
-      int g = 0, nx = 0, odd = 0;      // odd: a K without its V
+      // The next query tile's Q is asked for when the last scores of this one are there, its dO when the last dP is
+      int g = 0, nx = 0, no = 0, odd = 0;      // odd: a K without its V
       bool ok = true;
       for (int li = 0, w; ok && (w = items.at(li)) >= 0; li++) {
         const int qt = nq - 1 - w / BH, bh = w % BH, b = bh / a.H, xh = (bh % a.H) * H128;
-        if (li > 0 && !wait(bar_xf, (li - 1) & 1, 72)) break;
-        nx++;
-        tc::mbar_expect_tx(bar_x, 2 * T128_BYTES);
-        split_load<2>(smem + S::Q, &tm, bar_x, xh, qt * 128, b, 2);
-        split_load<2>(smem + S::DO, &tm_do, bar_x, xh, qt * 128, b, 2);
         for (int j = 0; j <= qt; j++, g++) {
           const int ks = g % 3, vs = g & 1;
+          if (j == 0) {
+            if (li > 0 && !wait(bar_qf, (li - 1) & 1, 72)) { ok = false; break; }
+            nx++;
+            tc::mbar_expect_tx(bar_q, T128_BYTES);
+            split_load<2>(smem + S::Q, &tm, bar_q, xh, qt * 128, b, 2);
+          }
           if (g >= 3 && !wait(&bar_kf[ks], (g / 3 + 1) & 1, 73)) { ok = false; break; }
           tc::mbar_expect_tx(&bar_k[ks], T128_BYTES);
           split_load<2>(smem + S::K + ks * T128_BYTES, &tm, &bar_k[ks], C + xh, j * 128, b, 2);
+          if (j == 0) {
+            if (li > 0 && !wait(bar_of, (li - 1) & 1, 91)) { ok = false; odd = 1; break; }
+            no++;
+            tc::mbar_expect_tx(bar_o, T128_BYTES);
+            split_load<2>(smem + S::DO, &tm_do, bar_o, xh, qt * 128, b, 2);
+          }
           if (g >= 2 && !wait(&bar_vf[vs], ((g >> 1) + 1) & 1, 74)) { ok = false; odd = 1; break; }
           tc::mbar_expect_tx(&bar_v[vs], T128_BYTES);
           split_load<2>(smem + S::V + vs * T128_BYTES, &tm, &bar_v[vs], 2 * C + xh, j * 128, b, 2);
         }
       }
-      attn_settle(bar_x, nx);
+      attn_settle(bar_q, nx);
+      attn_settle(bar_o, no);
       for (int i = 0; i < 3; i++) attn_settle(&bar_k[i], (g + odd + 2 - i) / 3);
       for (int i = 0; i < 2; i++) attn_settle(&bar_v[i], (g + 1 - i) / 2);
     }
@@ -678,39 +692,45 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
       constexpr uint32_t idesc_s = tc::idesc_bf16(128, 128, 0, 0);
       const uint64_t dQ = desc_base_k(tc::smem_u32(smem + S::Q)), dO = desc_base_k(tc::smem_u32(smem + S::DO));
       const uint64_t dK0 = desc_base_k(tc::smem_u32(smem + S::K)), dV0 = desc_base_k(tc::smem_u32(smem + S::V));
-      int g = 0;
+      // a block of this CTA's sequence of items, which the products run through without a break: block j of n of item li
+      struct Cursor { int li, j, n; };
+      auto blocks = [&](int li) { const int w = items.at(li); return w < 0 ? 0 : nq - w / BH; };      // 0: past the last item
+      auto next = [&](Cursor c) {
+        if (c.n > 0 && ++c.j == c.n) { c.li++; c.j = 0; c.n = blocks(c.li); }
+        return c;
+      };
       bool ok = true;
-      for (int li = 0, w; ok && (w = items.at(li)) >= 0; li++) {
-        const int n = nq - w / BH;
-        auto scores = [&](int gb) {      // over dS of block gb - 2, which its dQ reads
-          const int sl = gb % 3;
-          if (!ok || !wait(&bar_k[sl], (gb / 3) & 1, 75) || (gb > 1 && !wait(&bar_kf[(gb - 2) % 3], ((gb - 2) / 3) & 1, 85))) { ok = false; return; }
-          tc::tc_fence_after();
-          const uint64_t dK = dK0 + sl * T128_UNITS;
-          const uint32_t t_s = tmem + (gb & 1) * 128;
+      auto scores = [&](int gb, const Cursor& c) {      // over dS of block gb - 2, which its dQ reads
+        const int sl = gb % 3;
+        if (!ok || (c.j == 0 && !wait(bar_q, c.li & 1, 77)) || !wait(&bar_k[sl], (gb / 3) & 1, 75) ||
+            (gb > 1 && !wait(&bar_kf[(gb - 2) % 3], ((gb - 2) / 3) & 1, 85))) { ok = false; return; }
+        tc::tc_fence_after();
+        const uint64_t dK = dK0 + sl * T128_UNITS;
+        const uint32_t t_s = tmem + (gb & 1) * 128;
 #pragma unroll
-          for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ss(t_s, dQ + off_k(ks, TILE_BYTES), dK + off_k(ks, TILE_BYTES), idesc_s, ks > 0);
-          tc::mma_commit(&bar_s[gb & 1]);
-        };
-        auto dprobs = [&](int gb, bool last) {
-          if (!ok || !wait(&bar_v[gb & 1], (gb >> 1) & 1, 76)) { ok = false; return; }
-          tc::tc_fence_after();
-          const uint64_t dV = dV0 + (gb & 1) * T128_UNITS;
+        for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ss(t_s, dQ + off_k(ks, TILE_BYTES), dK + off_k(ks, TILE_BYTES), idesc_s, ks > 0);
+        tc::mma_commit(&bar_s[gb & 1]);
+        if (c.j + 1 == c.n) tc::mma_commit(bar_qf);
+      };
+      auto dprobs = [&](int gb, const Cursor& c) {
+        if (!ok || (c.j == 0 && !wait(bar_o, c.li & 1, 92)) || !wait(&bar_v[gb & 1], (gb >> 1) & 1, 76)) { ok = false; return; }
+        tc::tc_fence_after();
+        const uint64_t dV = dV0 + (gb & 1) * T128_UNITS;
 #pragma unroll
-          for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ss(t_dp, dO + off_k(ks, TILE_BYTES), dV + off_k(ks, TILE_BYTES), idesc_s, ks > 0);
-          tc::mma_commit(bar_dp);
-          tc::mma_commit(&bar_vf[gb & 1]);
-          if (last) tc::mma_commit(bar_xf);      // (the last scores were issued before)
-        };
-        ok = wait(bar_x, li & 1, 77);
-        scores(g);
-        if (n > 1) scores(g + 1);
-        dprobs(g, n == 1);
-        for (int j = 0; j < n; j++, g++) {
-          if (!ok || !wait(&bar_ds[g & 1], (g >> 1) & 1, 78)) { ok = false; break; }      // dP(j) read
-          if (j + 1 < n) dprobs(g + 1, j + 2 == n);
-          if (j + 2 < n) scores(g + 2);
-        }
+        for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ss(t_dp, dO + off_k(ks, TILE_BYTES), dV + off_k(ks, TILE_BYTES), idesc_s, ks > 0);
+        tc::mma_commit(bar_dp);
+        tc::mma_commit(&bar_vf[gb & 1]);
+        if (c.j + 1 == c.n) tc::mma_commit(bar_of);
+      };
+      Cursor c0{0, 0, blocks(0)}, c1 = next(c0), c2 = next(c1);
+      if (c0.n > 0) scores(0, c0);
+      if (c1.n > 0) scores(1, c1);
+      if (c0.n > 0) dprobs(0, c0);
+      for (int g = 0; ok && c0.n > 0; g++) {
+        if (!wait(&bar_ds[g & 1], (g >> 1) & 1, 78)) break;      // dP of this block read
+        if (c1.n > 0) dprobs(g + 1, c1);
+        if (c2.n > 0) scores(g + 2, c2);
+        c0 = c1; c1 = c2; c2 = next(c2);
       }
       tc::mma_commit(&bar_end[0]);
       attn_settle(&bar_end[0], 1);
@@ -787,20 +807,21 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&bar_ds[g & 1]);
       }
-      // ---- epilogue: 64 columns by each warp of quarters 0 and 1
+      // ---- epilogue: 32 columns by each warp, the rotation tables ahead of the last product
       w = items.at(li + 1);
       if (w >= 0) fetch(w);
+      RopeUnits rp;
+      if (a.cosT) rope_units<H128>(rp, a.cosT, a.sinT, qrow, qd * 16, lane, a.T - (qrow - lane));
       wait(bar_done, li & 1, 81);
       __syncwarp();
       tc::tc_fence_after();
-      if (qd < 2) {
-        bf16* dst = a.out + ((size_t)(b * a.T + qrow)) * 3 * C + h * H128;
-        store_pairs_rope<H128>(dst, 3L * C, t_dq + lane_addr, qd * 32, lane, *s_abort ? 0 : a.T - (qrow - lane), a.cosT, a.sinT, qrow, a.scale);
-      }
+      store_pairs16<H128>(a.out + ((size_t)(b * a.T + qrow)) * 3 * C + h * H128, 3L * C, t_dq + lane_addr, qd * 16, lane, *s_abort ? 0 : a.T - (qrow - lane),
+                          a.scale, a.cosT != nullptr, rp);
       tc::tc_fence_before();
     }
   }
   tc::tc_fence_before();
   __syncthreads();
+  if (tid == 0) tc::report_given_up(s_abort);
   if (warp == BWD128_MMA_WARP) tc::tmem_dealloc(tmem, 512);
 }

@@ -44,20 +44,6 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t&
   lo = pack_bf16(a - __uint_as_float(hi << 16), b - __uint_as_float(hi & 0xffff0000u));
 }
 
-// An earlier CTA of this library gave up on a wait: leave at once instead of queueing more waits behind it (CTA-uniform).
-__device__ __forceinline__ bool attn_given_up() {
-  return __syncthreads_or(threadIdx.x == 0 && *(volatile int*)&g_mlb_error != 0) != 0;
-}
-
-// A CTA one of whose waits has run out loads and multiplies nothing more.  What its threads have already issued still uses its shared
-// and tensor memory, so before they are given back the issuing thread waits, 2 ms at most, for the last of it: `begun` phases of a
-// barrier that counts a load's bytes or a commit (each begun when the one before was complete).
-__device__ __forceinline__ void attn_settle(uint64_t* bar, int begun) {
-  if (begun <= 0) return;
-  const uint64_t t0 = tc::globaltimer_ns();
-  while (!tc::mbar_try(bar, (begun - 1) & 1) && tc::globaltimer_ns() - t0 < 2000000) { }
-}
-
 // rows [r0, r0 + 64 * boxes) of `CH` 64-column chunks starting at column x0 of sample z
 template <int CH>
 __device__ __forceinline__ void split_load(uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, int x0, int r0, int z, int boxes) {
@@ -172,10 +158,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
   mlb_pdl_sync();
   const uint32_t t_s = *tmem_slot, t_o = t_s + 64, lane_addr = (uint32_t)(warp * 32) << 16;
   // Bounded, sticky: after one expiry every later wait of the CTA returns at once and all threads keep the same sequence of barriers
-  auto wait = [&](uint64_t* bar, uint32_t phase, int where) {
-    if (*s_abort) return;
-    if (!tc::mbar_wait(bar, phase, where)) *s_abort = 1;
-  };
+  auto wait = [&](uint64_t* bar, uint32_t phase, int where) { return tc::mbar_wait_sticky(bar, phase, where, s_abort); };
   const int nblk = (a.T + 63) / 64;
   const int nkb = a.causal ? min(nblk, q0 / 64 + 2) : nblk;
   const uint32_t idesc_s = tc::idesc_bf16(128, 64, 0, 0), idesc_o = tc::idesc_bf16(128, a.hd, 0, 1);
@@ -331,6 +314,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
   __syncthreads();
   if (*s_abort) {
     if (leader()) {
+      tc::report_given_up(s_abort);
       tc::mma_commit(bar_end);
       attn_settle(bar_end, 1);
       attn_settle(bar_q, 1);
@@ -397,10 +381,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
   mlb_pdl_sync();
   const uint32_t t_s = *tmem_slot, t_d = t_s + 64, t_a0 = t_s + 128, t_a1 = t_a0 + HDT;      // a0: dV or dQ, a1: dK
   const uint32_t lane_addr = (uint32_t)(warp * 32) << 16;
-  auto wait = [&](uint64_t* bar, uint32_t phase, int where) {
-    if (*s_abort) return;
-    if (!tc::mbar_wait(bar, phase, where)) *s_abort = 1;
-  };
+  auto wait = [&](uint64_t* bar, uint32_t phase, int where) { return tc::mbar_wait_sticky(bar, phase, where, s_abort); };
   const int nblk = (a.T + 63) / 64;
   const int i0 = (KV && a.causal) ? r0 / 64 : 0;
   const int n = (!KV && a.causal) ? min(nblk, r0 / 64 + 2) : nblk - i0;
@@ -538,6 +519,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
   __syncthreads();
   if (*s_abort) {
     if (leader()) {
+      tc::report_given_up(s_abort);
       tc::mma_commit(bar_end);
       attn_settle(bar_end, 1);
       attn_settle(bar_r, 1);

@@ -45,18 +45,35 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
 #ifndef MLB_MBAR_TIMEOUT_NS
 #define MLB_MBAR_TIMEOUT_NS 4000000000ull
 #endif
+// (As few instructions as it can be, here and below: a kernel has dozens of waits, and what they hold besides the first probe pushes its
+// loops out of the SM's instruction cache.  A probe sleeps in hardware for a while, so reading the clock after each costs nothing.)
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int where = 0) {
   if (mbar_try(bar, parity)) return true;
-  uint64_t t0 = globaltimer_ns();
-  for (;;) {
+  const uint64_t t0 = globaltimer_ns();
 #pragma unroll 1
-    for (int i = 0; i < 2048; i++)
-      if (mbar_try(bar, parity)) return true;
+  while (!mbar_try(bar, parity)) {
     if (globaltimer_ns() - t0 > MLB_MBAR_TIMEOUT_NS) {
       mlb_set_error(MLB_ERR_MBAR_TIMEOUT, where);
       return false;
     }
   }
+  return true;
+}
+// The same for a CTA that gives up as one: the first wait to run out leaves its number in *given_up (shared memory), and every other one returns
+// at once.  The CTA reports it at its end (report_given_up, one thread, behind a barrier of all).
+__device__ __forceinline__ bool mbar_wait_sticky(uint64_t* bar, uint32_t parity, int where, volatile int* given_up) {
+  if (mbar_try(bar, parity)) return true;
+  const uint64_t t0 = globaltimer_ns();
+#pragma unroll 1
+  do {
+    if (*given_up) return false;
+    if (mbar_try(bar, parity)) return true;
+  } while (globaltimer_ns() - t0 <= MLB_MBAR_TIMEOUT_NS);
+  *given_up = where;
+  return false;
+}
+__device__ __forceinline__ void report_given_up(volatile int* given_up) {
+  if (*given_up) mlb_set_error(MLB_ERR_MBAR_TIMEOUT, *given_up);
 }
 
 // Same bound, but the polling thread sleeps between probes so that it does not compete for issue slots with warps that
@@ -208,6 +225,67 @@ __device__ __forceinline__ void tmem_ld32x2_wait(uint32_t taddr_a, uint32_t (&a)
         "=&r"(b[23]), "=&r"(b[24]), "=&r"(b[25]), "=&r"(b[26]), "=&r"(b[27]), "=&r"(b[28]), "=&r"(b[29]), "=&r"(b[30]), "=&r"(b[31])
       : "r"(taddr_a), "r"(taddr_b)
       : "memory");
+}
+__device__ __forceinline__ void tmem_ld16x2_wait(uint32_t taddr_a, uint32_t (&a)[16], uint32_t taddr_b, uint32_t (&b)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%32];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%33];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=&r"(a[0]), "=&r"(a[1]), "=&r"(a[2]), "=&r"(a[3]), "=&r"(a[4]), "=&r"(a[5]), "=&r"(a[6]), "=&r"(a[7]), "=&r"(a[8]), "=&r"(a[9]),
+        "=&r"(a[10]), "=&r"(a[11]), "=&r"(a[12]), "=&r"(a[13]), "=&r"(a[14]), "=&r"(a[15]), "=&r"(b[0]), "=&r"(b[1]), "=&r"(b[2]),
+        "=&r"(b[3]), "=&r"(b[4]), "=&r"(b[5]), "=&r"(b[6]), "=&r"(b[7]), "=&r"(b[8]), "=&r"(b[9]), "=&r"(b[10]), "=&r"(b[11]),
+        "=&r"(b[12]), "=&r"(b[13]), "=&r"(b[14]), "=&r"(b[15])
+      : "r"(taddr_a), "r"(taddr_b)
+      : "memory");
+}
+// Fragments: 32 columns of the warp's 32 rows, spread as a matrix instruction's accumulator is.  r[h][4 j + 2 v + x] is row 16 h + 8 v + lane / 4,
+// column 8 j + 2 (lane % 4) + x: a thread has two adjacent columns of each eight, for four rows, so that what belongs to a column is
+// read from shared memory once for four rows and by a quarter of the lanes.
+__device__ __forceinline__ void tmem_ld_frag_wait(uint32_t taddr, uint32_t (&r)[2][16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%32];\n\t"
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+      "{%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%33];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=&r"(r[0][0]), "=&r"(r[0][1]), "=&r"(r[0][2]), "=&r"(r[0][3]), "=&r"(r[0][4]), "=&r"(r[0][5]), "=&r"(r[0][6]), "=&r"(r[0][7]),
+        "=&r"(r[0][8]), "=&r"(r[0][9]), "=&r"(r[0][10]), "=&r"(r[0][11]), "=&r"(r[0][12]), "=&r"(r[0][13]), "=&r"(r[0][14]),
+        "=&r"(r[0][15]), "=&r"(r[1][0]), "=&r"(r[1][1]), "=&r"(r[1][2]), "=&r"(r[1][3]), "=&r"(r[1][4]), "=&r"(r[1][5]), "=&r"(r[1][6]),
+        "=&r"(r[1][7]), "=&r"(r[1][8]), "=&r"(r[1][9]), "=&r"(r[1][10]), "=&r"(r[1][11]), "=&r"(r[1][12]), "=&r"(r[1][13]),
+        "=&r"(r[1][14]), "=&r"(r[1][15])
+      : "r"(taddr), "r"(taddr + (16u << 16))
+      : "memory");
+}
+// The same 32 columns packed in pairs (bf16 of columns 2 c, 2 c + 1 in 32-bit column c): w[h][2 j + v] is row 16 h + 8 v + lane / 4, column
+// 4 j + lane % 4 of the sixteen.
+__device__ __forceinline__ void tmem_st_frag(uint32_t taddr, const uint32_t (&w)[2][8]) {
+  asm volatile("tcgen05.st.sync.aligned.16x128b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(w[0][0]), "r"(w[0][1]),
+               "r"(w[0][2]), "r"(w[0][3]), "r"(w[0][4]), "r"(w[0][5]), "r"(w[0][6]), "r"(w[0][7])
+               : "memory");
+  asm volatile("tcgen05.st.sync.aligned.16x128b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr + (16u << 16)), "r"(w[1][0]),
+               "r"(w[1][1]), "r"(w[1][2]), "r"(w[1][3]), "r"(w[1][4]), "r"(w[1][5]), "r"(w[1][6]), "r"(w[1][7])
+               : "memory");
+}
+// 64 columns of 16 rows (the address's lane: the first), the first 32 in a, the others in b: fragments as above of one h.
+__device__ __forceinline__ void tmem_ld_frag16x2_wait(uint32_t taddr, uint32_t (&a)[16], uint32_t (&b)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%32];\n\t"
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+      "{%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%33];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=&r"(a[0]), "=&r"(a[1]), "=&r"(a[2]), "=&r"(a[3]), "=&r"(a[4]), "=&r"(a[5]), "=&r"(a[6]), "=&r"(a[7]), "=&r"(a[8]), "=&r"(a[9]),
+        "=&r"(a[10]), "=&r"(a[11]), "=&r"(a[12]), "=&r"(a[13]), "=&r"(a[14]), "=&r"(a[15]), "=&r"(b[0]), "=&r"(b[1]), "=&r"(b[2]),
+        "=&r"(b[3]), "=&r"(b[4]), "=&r"(b[5]), "=&r"(b[6]), "=&r"(b[7]), "=&r"(b[8]), "=&r"(b[9]), "=&r"(b[10]), "=&r"(b[11]),
+        "=&r"(b[12]), "=&r"(b[13]), "=&r"(b[14]), "=&r"(b[15])
+      : "r"(taddr), "r"(taddr + 32)
+      : "memory");
+}
+// Four 8 x 8 bf16 matrices of such a fragment to shared memory: lane l gives the 16 bytes of row l % 8 of matrix l / 8.
+__device__ __forceinline__ void stmatrix_x4(uint32_t saddr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(saddr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 // 128 consecutive columns
 __device__ __forceinline__ void tmem_ld32x4_wait(uint32_t taddr, uint32_t (&r)[4][32]) {
