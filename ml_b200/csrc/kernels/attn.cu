@@ -1137,91 +1137,60 @@ __device__ __forceinline__ void quad_transpose(uint4 (&a)[4], int lane) {
     }
   }
 }
-// Epilogue of the backward kernels.  A warp moves accumulator columns [c0, c0 + 16) and [c0 + HD/2, c0 + HD/2 + 16) of its 32 rows, which are
-// sixteen of RoPE's rotation pairs (i, i + HD/2), from TMEM to memory as bf16, and rotates them backward (d0' = d0 c + d1 s, d1' = d1 c - d0 s).
-// Lanes 2i and 2i + 1 exchange halves first: each then has eight columns (unit lane & 1) of both their rows, so that an instruction on
-// the tables or the output touches 32 bytes in each of 16 rows instead of 16 in each of 32.  The tables are asked for ahead of the
-// accumulator: they come from the L2, and with a lane at its own row of them and the loads behind the wait an epilogue was ~10000
-// cycles of a key tile's ~39000 at head size 128 (~7500 so).
-struct RopeUnits { float c[2][8], s[2][8]; };      // [row of the lane pair][column of the unit]
+// 32 bf16 columns (four 16-byte units per lane) of 32 consecutive rows to memory: `dst` = this lane's row at the first column, rows
+// `pitch` elements apart, `nlive` of the warp's rows exist (whole warp, converged).
+__device__ __forceinline__ void store_rows32(bf16* dst, long pitch, uint4 (&a)[4], int lane, int nlive) {
+  quad_transpose(a, lane);
+  const int q = lane & 3;
+  bf16* base = dst - q * pitch + q * 8;      // row of the quad's first lane, this lane's unit
+#pragma unroll
+  for (int k = 0; k < 4; k++)
+    if ((lane & ~3) + k < nlive) *reinterpret_cast<uint4*>(base + k * pitch) = a[k];
+}
+
+// Epilogue helper for the backward kernels of two launches: one warp moves 64 accumulator columns of its 32 rows from TMEM to memory as bf16:
+// columns [c0, c0+32) and [c0 + HD/2, c0 + HD/2 + 32), which are exactly RoPE's rotation pairs (i, i + HD/2).  With tables given,
+// RoPE's backward rotation (d0' = d0 c + d1 s, d1' = d1 c - d0 s) is applied.  dst_row: the lane's row, rows `pitch` apart; t its
+// position; nlive rows of the warp exist (0: nothing is stored).  Whole warp.
 template <int HD>
-__device__ __forceinline__ void rope_units(RopeUnits& r, const float* cosT, const float* sinT, int t, int c0, int lane, int nlive) {
-  const size_t at = (size_t)(t - (lane & 1)) * (HD / 2) + c0 + (lane & 1) * 8;      // (t: the position of the lane's row)
+__device__ __forceinline__ void store_pairs_rope(bf16* dst_row, long pitch, uint32_t taddr, int c0, int lane, int nlive, const float* cosT,
+                                                 const float* sinT, int t, float out_scale = 1.f) {
+  uint32_t ra[32], rb[32];
+  tc::tmem_ld32x2_wait(taddr + c0, ra, taddr + c0 + HD / 2, rb);
+  float x0[32], x1[32];
 #pragma unroll
-  for (int k = 0; k < 2; k++) {
-    const bool live = (lane & ~1) + k < nlive;
-    const float4* c4 = reinterpret_cast<const float4*>(cosT + at + (size_t)k * (HD / 2));
-    const float4* s4 = reinterpret_cast<const float4*>(sinT + at + (size_t)k * (HD / 2));
+  for (int i = 0; i < 32; i++) { x0[i] = __uint_as_float(ra[i]) * out_scale; x1[i] = __uint_as_float(rb[i]) * out_scale; }
+  if (cosT && lane < nlive) {   // 16-byte loads: every lane reads its own row of the tables, an instruction costs the L1 a line per lane whatever its width
+    const float4* c4 = reinterpret_cast<const float4*>(cosT + (size_t)t * (HD / 2) + c0);
+    const float4* s4 = reinterpret_cast<const float4*>(sinT + (size_t)t * (HD / 2) + c0);
 #pragma unroll
-    for (int v = 0; v < 2; v++) {
-      *reinterpret_cast<float4*>(&r.c[k][v * 4]) = live ? __ldg(c4 + v) : make_float4(0.f, 0.f, 0.f, 0.f);
-      *reinterpret_cast<float4*>(&r.s[k][v * 4]) = live ? __ldg(s4 + v) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int q = 0; q < 8; q++) {
+      const float4 cv = __ldg(c4 + q), sv = __ldg(s4 + q);
+      const float cc[4] = {cv.x, cv.y, cv.z, cv.w}, ss[4] = {sv.x, sv.y, sv.z, sv.w};
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        const float d0 = x0[q * 4 + e], d1 = x1[q * 4 + e];
+        x0[q * 4 + e] = d0 * cc[e] + d1 * ss[e];
+        x1[q * 4 + e] = d1 * cc[e] - d0 * ss[e];
+      }
     }
   }
-}
-__device__ __forceinline__ void pair_exchange(float (&x)[16], int lane) {
-  const bool up = lane & 1;
+  __syncwarp();
+  uint4 u[4];
 #pragma unroll
-  for (int e = 0; e < 8; e++) {
-    const float v = __shfl_xor_sync(0xffffffffu, up ? x[e] : x[8 + e], 1);
-    if (up) x[e] = v; else x[8 + e] = v;
-  }
+  for (int v = 0; v < 4; v++)
+    u[v] = make_uint4(pack_bf16(x0[v * 8], x0[v * 8 + 1]), pack_bf16(x0[v * 8 + 2], x0[v * 8 + 3]), pack_bf16(x0[v * 8 + 4], x0[v * 8 + 5]),
+                      pack_bf16(x0[v * 8 + 6], x0[v * 8 + 7]));
+  store_rows32(dst_row + c0, pitch, u, lane, nlive);
+#pragma unroll
+  for (int v = 0; v < 4; v++)
+    u[v] = make_uint4(pack_bf16(x1[v * 8], x1[v * 8 + 1]), pack_bf16(x1[v * 8 + 2], x1[v * 8 + 3]), pack_bf16(x1[v * 8 + 4], x1[v * 8 + 5]),
+                      pack_bf16(x1[v * 8 + 6], x1[v * 8 + 7]));
+  store_rows32(dst_row + c0 + HD / 2, pitch, u, lane, nlive);
 }
+
 __device__ __forceinline__ uint4 pack8(const float* x) {
   return make_uint4(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]), pack_bf16(x[4], x[5]), pack_bf16(x[6], x[7]));
-}
-// ra, rb: the lane's sixteen fp32 values of either half in; lo[k], hi[k] out: unit lane & 1 of either half of row (lane & ~1) + k.  Whole warp.
-__device__ __forceinline__ void rotate_pairs16(const uint32_t* ra, const uint32_t* rb, int lane, float out_scale, bool rotate, const RopeUnits& r,
-                                               uint4 (&lo)[2], uint4 (&hi)[2]) {
-  float x0[16], x1[16];
-#pragma unroll
-  for (int i = 0; i < 16; i++) { x0[i] = __uint_as_float(ra[i]) * out_scale; x1[i] = __uint_as_float(rb[i]) * out_scale; }
-  __syncwarp();
-  pair_exchange(x0, lane);
-  pair_exchange(x1, lane);
-  if (rotate) {
-#pragma unroll
-    for (int i = 0; i < 16; i++) {
-      const float d0 = x0[i], d1 = x1[i], c = r.c[i >> 3][i & 7], s = r.s[i >> 3][i & 7];
-      x0[i] = d0 * c + d1 * s;
-      x1[i] = d1 * c - d0 * s;
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < 2; k++) { lo[k] = pack8(x0 + k * 8); hi[k] = pack8(x1 + k * 8); }
-}
-// dst_row: the lane's row, rows `pitch` elements apart; nlive rows of the warp exist (0: nothing is stored).  Whole warp.
-template <int HD>
-__device__ __forceinline__ void store_pairs16_regs(bf16* dst_row, long pitch, const uint32_t* ra, const uint32_t* rb, int c0, int lane, int nlive,
-                                                   float out_scale, bool rotate, const RopeUnits& r) {
-  uint4 lo[2], hi[2];
-  rotate_pairs16(ra, rb, lane, out_scale, rotate, r, lo, hi);
-  bf16* base = dst_row - (lane & 1) * pitch + c0 + (lane & 1) * 8;
-#pragma unroll
-  for (int k = 0; k < 2; k++) {
-    if ((lane & ~1) + k < nlive) {
-      *reinterpret_cast<uint4*>(base + k * pitch) = lo[k];
-      *reinterpret_cast<uint4*>(base + k * pitch + HD / 2) = hi[k];
-    }
-  }
-}
-template <int HD>
-__device__ __forceinline__ void store_pairs16(bf16* dst_row, long pitch, uint32_t taddr, int c0, int lane, int nlive, float out_scale, bool rotate,
-                                              const RopeUnits& r) {
-  uint32_t ra[16], rb[16];
-  tc::tmem_ld16x2_wait(taddr + c0, ra, taddr + c0 + HD / 2, rb);
-  store_pairs16_regs<HD>(dst_row, pitch, ra, rb, c0, lane, nlive, out_scale, rotate, r);
-}
-// all HD columns, by one warp
-template <int HD>
-__device__ __forceinline__ void store_row_pairs(bf16* dst_row, long pitch, uint32_t taddr, int lane, int nlive, const float* cosT, const float* sinT,
-                                                int t, float out_scale = 1.f) {
-#pragma unroll
-  for (int c0 = 0; c0 < HD / 2; c0 += 16) {
-    RopeUnits r;
-    if (cosT) rope_units<HD>(r, cosT, sinT, t, c0, lane, nlive);
-    store_pairs16<HD>(dst_row, pitch, taddr, c0, lane, nlive, out_scale, cosT != nullptr, r);
-  }
 }
 
 constexpr int BWD_THREADS = 512;
@@ -1372,8 +1341,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kv_tc_kernel(const __
     if (cq < 2) {
       const bool is_k = cq == 0;
       bf16* dst = a.out + ((size_t)(row0 + krow)) * 3 * C + (is_k ? C : 2 * C) + h * HD;
-      store_row_pairs<HD>(dst, 3L * C, (is_k ? t_dk : t_dv) + lane_addr, lane, a.T - (krow - lane), is_k ? a.cosT : nullptr,
-                          is_k ? a.sinT : nullptr, krow);
+      store_pairs_rope<HD>(dst, 3L * C, (is_k ? t_dk : t_dv) + lane_addr, 0, lane, a.T - (krow - lane), is_k ? a.cosT : nullptr,
+                           is_k ? a.sinT : nullptr, krow);
     }
   }
   tc::tc_fence_before();
@@ -2098,7 +2067,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_q_tc_kernel(const __g
   tc::tc_fence_after();
   if (__all_sync(0xffffffffu, ok) && cq == 0) {
     bf16* dst = a.out + ((size_t)(row0 + qrow)) * 3 * C + h * HD;
-    store_row_pairs<HD>(dst, 3L * C, t_dq + lane_addr, lane, a.T - (qrow - lane), a.cosT, a.sinT, qrow);
+    store_pairs_rope<HD>(dst, 3L * C, t_dq + lane_addr, 0, lane, a.T - (qrow - lane), a.cosT, a.sinT, qrow);
   }
   tc::tc_fence_before();
   __syncthreads();
@@ -2530,8 +2499,10 @@ static int attn_bwd_impl(void* dqkv, const void* dout, const void* qkv, const vo
       const SchedUse sched = n_items > sms ? attn_schedule(1, B, H, T, (int)grid_p.x, st) : SchedUse{};
       a.sched = sched.table;
       a.sched_stride = sched.stride;
-      mlb_launch_tmem(n_items <= sms, attn_bwd_kv128_k, grid_p, dim3(BWD128_THREADS), BwdKV128Smem::TOTAL, st, *tq, *td, a);
-      mlb_launch_tmem(n_items <= sms, attn_bwd_q128_k, grid_p, dim3(BWD128_THREADS), BwdQ128Smem::TOTAL, st, *tq, *td, a);
+      const CUtensorMap* tout = mlb_tmap_cached(dqkv, (uint64_t)B * T, 3 * C, 3 * C, 32, 64, 2);      // the gradients leave through it
+      if (!tout) return -2;
+      mlb_launch_tmem(n_items <= sms, attn_bwd_kv128_k, grid_p, dim3(BWD128_THREADS), BwdKV128Smem::TOTAL, st, *tq, *td, *tout, a);
+      mlb_launch_tmem(n_items <= sms, attn_bwd_q128_k, grid_p, dim3(BWD128_THREADS), BwdQ128Smem::TOTAL, st, *tq, *td, *tout, a);
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return (int)e + 1000;

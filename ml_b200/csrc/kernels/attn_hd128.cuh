@@ -324,13 +324,15 @@ __global__ void __maxnreg__(160) attn_fwd128_k(const __grid_constant__ CUtensorM
 // dK / dV of a 128-key tile, streaming query blocks.  TMEM: S^T, dP^T, dV, dK.  Two threads issue products, as in the kernels for head
 // size 64, so that neither's waits hold up the other's products.  One takes  S^T(i) dP^T(i) S^T(i+1) ...,  the other  dV(i) dK(i) ...
 // P^T goes to shared memory, so S^T(i+1) needs no more than that S^T(i) has been read, and the exponentials of block i+1 run under
-// dK(i) and dP^T(i+1); over its scores it would make S^T(i+1) wait for dV(i).  dS^T stays over dP^T.  512 element-wise threads: a
-// thread has one key and 32 of the block's 128 queries.  Four warps per sub-partition hide each other's TMEM and barrier
-// latencies.  The queries' statistics are one warp's work (fetched by those who use them, each block waited 800 cycles for them).
-// Shared memory is full to the last 512 bytes: nothing is left to align its base with, which is checked instead.
-// A block takes 3500 cycles (3950 with one issuing thread and P^T over its scores); what is left is the shared memory's: three of
-// the four products read both operands there, 2000 of its cycles, the tiles that arrive 500, and Q's slot is given back late (asking
-// for its lines in the L2 beforehand changed nothing).  8 x 2048 tokens, 16 heads, forward + backward: 1047 -> 1015 ... 1025 us with the same for dQ.
+// dK(i) and dP^T(i+1); over its scores it would make S^T(i+1) wait for dV(i) (tried: the same time).  dS^T stays over dP^T.  Sixteen element-wise
+// warps, 32 keys by 32 of the block's 128 queries each, hide each other's TMEM and barrier latencies.  They read scores as fragments (two
+// adjacent queries of each eight, for four keys), which reads a query's statistics a quarter as often from the shared memory that the
+// products' operands come from.  The statistics are one warp's work (fetched by those who use them, each block waited 800 cycles for
+// them).  Shared memory is full to the last 512 bytes: nothing is left to align its base with, which is checked instead.
+// K, V and the first Q, dO of the next key tile are asked for as soon as their places are free, and its scores do not wait for this tile's
+// epilogue, which sends dV and dK by TMA out of P's place: with loads behind the end of a tile and stores of 32 lines an instruction a change of
+// tile was 12600 of 39500 cycles, now 7800.  A block takes 3500 cycles: its products 2048, its shared-memory traffic ~2900 (operands 1800,
+// arriving tiles 512, P^T, statistics).  8 x 2048 tokens, 16 heads, both kernels: 655 -> 622 us.
 struct BwdKV128Smem {
   static constexpr int K = 0;
   static constexpr int V = K + T128_BYTES;
@@ -345,7 +347,8 @@ struct BwdKV128Smem {
 // dQ of a 128-query tile, streaming key blocks.  TMEM: S in two buffers, dP, dQ; dS goes over the S it came from:
 //   dP(j+1)  S(j+2)  dP(j+2) ...   by one thread,   dQ(j)  dQ(j+1) ...   by another
 // keeps scores one block ahead, so the element-wise threads never wait for them.
-// A block takes 2700 cycles (3050 when one thread issued all three products, one after the other's 8 instructions).
+// The products run through the CTA's query tiles without a break; dQ leaves by TMA out of dO's place, which is loaded for the next tile behind
+// that.  A block takes ~2350 cycles, a change of tile 5700 (13000 with loads and stores at its end).
 struct BwdQ128Smem {
   static constexpr int Q = 0;
   static constexpr int DO = Q + T128_BYTES;
@@ -361,8 +364,58 @@ constexpr int BWD128_MMA_WARP = BWD128_E_WARPS, BWD128_LOAD_WARP = BWD128_E_WARP
 constexpr int BWD128_THREADS = (BWD128_E_WARPS + 4) * 32;      // (five warps per sub-partition, as with two of the four)
 // (split_col(ks): A-operand column of k-step ks of a bf16 tile whose 32-column quarters sit over their own fp32 columns)
 
+// Epilogue of both: of an accumulator a warp takes columns [16 qd, + 16) and [64 + 16 qd, + 16) of its 32 rows, sixteen of RoPE's rotation pairs, as
+// fragments, rotates them backward, and puts them as bf16 into a [128 x 128] tile in shared memory that leaves by TMA: no shuffles, and
+// stores that touch 16 lines an instruction keep the load / store unit for thousands of cycles.
+struct Rope128 { float2 c[2][4], s[2][4]; };      // [16 rows][2 j + v]: columns 8 j + fc, + 1 of row 8 v + fr
+__device__ __forceinline__ void rope128(Rope128& r, const float* cosT, const float* sinT, int row0, int c0, int lane, int T) {
+#pragma unroll
+  for (int h = 0; h < 2; h++)
+#pragma unroll
+    for (int v = 0; v < 2; v++) {
+      const size_t at = (size_t)min(row0 + h * 16 + v * 8 + (lane >> 2), T - 1) * (H128 / 2) + c0 + 2 * (lane & 3);
+#pragma unroll
+      for (int j = 0; j < 2; j++) {
+        r.c[h][2 * j + v] = __ldg(reinterpret_cast<const float2*>(cosT + at + j * 8));
+        r.s[h][2 * j + v] = __ldg(reinterpret_cast<const float2*>(sinT + at + j * 8));
+      }
+    }
+}
+__device__ __forceinline__ void tile128_out(uint32_t tile, const uint32_t (&a)[2][8], const uint32_t (&b)[2][8], int lg, int c0, int lane, float f, bool rotate,
+                                            const Rope128& r) {
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    uint32_t wa[4], wb[4];
+#pragma unroll
+    for (int m = 0; m < 4; m++) {
+      float a0 = __uint_as_float(a[h][2 * m]) * f, a1 = __uint_as_float(b[h][2 * m]) * f;
+      float b0 = __uint_as_float(a[h][2 * m + 1]) * f, b1 = __uint_as_float(b[h][2 * m + 1]) * f;
+      if (rotate) {      // d0' = d0 c + d1 s, d1' = d1 c - d0 s
+        const float2 c = r.c[h][m], s = r.s[h][m];
+        const float d0 = a0, e0 = b0;
+        a0 = d0 * c.x + a1 * s.x;
+        a1 = a1 * c.x - d0 * s.x;
+        b0 = e0 * c.y + b1 * s.y;
+        b1 = b1 * c.y - e0 * s.y;
+      }
+      wa[m] = pack_bf16(a0, b0);
+      wb[m] = pack_bf16(a1, b1);
+    }
+    // lane l has the address of row l % 8 of matrix l / 8: rows + 8 (l / 8 % 2), columns + 8 (l / 16)
+    const int row = lg * 32 + h * 16 + (lane & 15), col = c0 + (lane >> 4) * 8;
+    tc::stmatrix_x4(tile + sw_off(row, col), wa[0], wa[1], wa[2], wa[3]);
+    tc::stmatrix_x4(tile + sw_off(row, col + 64), wb[0], wb[1], wb[2], wb[3]);
+  }
+}
+// rows [32 lg, 32 lg + nlive) of such a tile to memory by the four warps that wrote them (thread 0 ... 127), for a part of a tile
+__device__ __forceinline__ void tile128_rows(bf16* dst, long pitch, const uint8_t* tile, int lg, int nlive, int thread) {
+#pragma unroll 1
+  for (int r = thread >> 4; r < nlive; r += 8)
+    *reinterpret_cast<uint4*>(dst + r * pitch + (thread & 15) * 8) = *reinterpret_cast<const uint4*>(tile + sw_off(lg * 32 + r, (thread & 15) * 8));
+}
+
 __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUtensorMap tm_do,
-                                                                      const AttnArgs a) {
+                                                                      const __grid_constant__ CUtensorMap tm_out, const AttnArgs a) {
   mlb_pdl_sync();
   using S = BwdKV128Smem;
   extern __shared__ uint8_t smem_raw[];
@@ -392,6 +445,7 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
     tc::mbar_fence_init();
     tc::tma_prefetch_desc(&tm);
     tc::tma_prefetch_desc(&tm_do);
+    tc::tma_prefetch_desc(&tm_out);
   }
   if (warp == BWD128_MMA_WARP) tc::tmem_alloc(tmem_slot, 512);
   tc::tc_fence_before();
@@ -511,8 +565,8 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
 #pragma unroll
         for (int x = 0; x < 4; x++) {
           const int q = i * 128 + x * 32 + lane;
-          nl[x] = q < a.T ? a.lse[e + q] * LOG2E : INFINITY;
-          nd[x] = q < a.T ? a.delta[e + q] : 0.f;
+          nl[x] = q < a.T ? -a.lse[e + q] * LOG2E : -INFINITY;
+          nd[x] = q < a.T ? -a.delta[e + q] : 0.f;
         }
         // (one answer for the warp: a lane whose wait has run out must not leave those behind whose wait has not)
         if (g >= 2 && !__all_sync(0xffffffffu, wait(&bar_stf[g & 1], ((g >> 1) + 1) & 1, 63))) { ok = false; break; }
@@ -527,49 +581,73 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
       }
     }
   } else {
-    const int lg = warp & 3, qd = warp >> 2, row = lg * 32 + lane;
+    const int lg = warp & 3, qd = warp >> 2;
+    const int fr = lane >> 2, fc = 2 * (lane & 3);      // this thread's row and column in a fragment's 8 x 8 matrices
     const uint32_t lane_addr = (uint32_t)(lg * 32) << 16;
     const uint32_t ts = t_s + qd * 32 + lane_addr, tdp = t_dp + qd * 32 + lane_addr;
     const float sl2 = a.scale * LOG2E;
-    uint8_t* prow = smem + S::P + (qd >> 1) * TILE_BYTES + row * 128;      // this thread's 64 bytes of P^T: units 4 (qd & 1) ... of the chunk's row
+    const uint64_t sl2x2 = pk2(sl2, sl2);
+    const uint32_t p_tile = tc::smem_u32(smem + S::P);
+    const uint32_t p_at = p_tile + sw_off(lg * 32 + (lane & 15), qd * 32 + (lane >> 4) * 8);      // stmatrix address of rows 0 ... 15, columns 0 ... 15
+    const uint32_t p_at16 = p_tile + sw_off(lg * 32 + (lane & 15), qd * 32 + 16 + (lane >> 4) * 8);      // of columns 16 ... 31
+    const bool sender = qd == 0 && lane == 0;      // of the 32 rows of four warps
+    auto rows_read = [&]() {      // the rows that the sender's last store takes out of P's tile have been read: the four warps may write there again
+      if (sender) tc::tma_wait_group_read<0>();
+      named_bar_sync(1 + lg, 128);
+    };
     int g = 0;
     for (int li = 0, w; (w = items.at(li)) >= 0; li++) {
       const int kt = w / BH, bh = w % BH, b = bh / a.H, h = bh % a.H;
-      const int krow = kt * 128 + row;
       for (int i = kt; i < nq; i++, g++) {
-        const float* st = (const float*)(smem + S::STAT + (g & 1) * 1024) + qd * 32;
+        const float* st = (const float*)(smem + S::STAT + (g & 1) * 1024) + qd * 32 + fc;
         wait(&bar_st[g & 1], (g >> 1) & 1, 87);
         wait(bar_s, g & 1, 69);
         __syncwarp();
         tc::tc_fence_after();
-        float p[32];
+        float p[2][16];
+        uint32_t wp[2][8];
         {
-          uint32_t r[32];
-          tc::tmem_ld32_wait(ts, r);
+          uint32_t r[2][16];
+          tc::tmem_ld_frag_wait(ts, r);
           tc::tc_fence_before();
           __syncwarp();
           if (lane == 0) tc::mbar_arrive(bar_sr);
 #pragma unroll
-          for (int e = 0; e < 32; e += 4) {
-            const float4 L = *reinterpret_cast<const float4*>(st + e);
-            p[e] = ex2_approx(fmaf(__uint_as_float(r[e]), sl2, -L.x));
-            p[e + 1] = ex2_approx(fmaf(__uint_as_float(r[e + 1]), sl2, -L.y));
-            p[e + 2] = ex2_approx(fmaf(__uint_as_float(r[e + 2]), sl2, -L.z));
-            p[e + 3] = ex2_approx(fmaf(__uint_as_float(r[e + 3]), sl2, -L.w));
+          for (int j = 0; j < 4; j++) {
+            const float2 nl = *reinterpret_cast<const float2*>(st + j * 8);
+#pragma unroll
+            for (int x = 0; x < 2; x++)
+#pragma unroll
+              for (int v = 0; v < 2; v++) {
+                const int e = 4 * j + 2 * v;
+                float z0, z1;
+                upk2(fma2(pk2(__uint_as_float(r[x][e]), __uint_as_float(r[x][e + 1])), sl2x2, pk2(nl.x, nl.y)), z0, z1);
+                p[x][e] = ex2_approx(z0);
+                p[x][e + 1] = ex2_approx(z1);
+              }
           }
         }
-        if (i == kt) {      // the diagonal block: query before key
+        if (i == kt && qd <= lg) {      // the diagonal block: no query before the key (8 x 8 matrices under, on and over the diagonal)
 #pragma unroll
-          for (int e = 0; e < 32; e++)
-            if (qd * 32 + e < row) p[e] = 0.f;
+          for (int x = 0; x < 2; x++)
+#pragma unroll
+            for (int e = 0; e < 16; e++) {
+              const int j = e >> 2, row8 = 2 * x + ((e >> 1) & 1);
+              if (qd < lg || j < row8 || (j == row8 && fc + (e & 1) < fr)) p[x][e] = 0.f;
+            }
         }
-        uint32_t pw[16];
 #pragma unroll
-        for (int x = 0; x < 16; x++) pw[x] = pack_bf16(p[2 * x], p[2 * x + 1]);
+        for (int x = 0; x < 2; x++)
+#pragma unroll
+          for (int m = 0; m < 8; m++) wp[x][m] = pack_bf16(p[x][2 * m], p[x][2 * m + 1]);
         if (g > 0) wait(&bar_dof[(g - 1) & 1], ((g - 1) >> 1) & 1, 86);      // dV of the block before has read its P^T
+        if (i == kt && li > 0) rows_read();
+        __syncwarp();
 #pragma unroll
-        for (int v = 0; v < 4; v++)
-          *reinterpret_cast<uint4*>(prow + ((((qd & 1) * 4 + v) ^ (row & 7)) << 4)) = make_uint4(pw[v * 4], pw[v * 4 + 1], pw[v * 4 + 2], pw[v * 4 + 3]);
+        for (int x = 0; x < 2; x++) {
+          tc::stmatrix_x4(p_at + x * 2048, wp[x][0], wp[x][1], wp[x][2], wp[x][3]);
+          tc::stmatrix_x4(p_at16 + x * 2048, wp[x][4], wp[x][5], wp[x][6], wp[x][7]);
+        }
         tc::fence_async_smem();
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(bar_p);
@@ -577,16 +655,23 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
         __syncwarp();
         tc::tc_fence_after();
         {
-          uint32_t d[32];
-          tc::tmem_ld32_wait(tdp, d);
+          uint32_t d[2][16];
+          tc::tmem_ld_frag_wait(tdp, d);
 #pragma unroll
-          for (int e = 0; e < 32; e += 4) {
-            const float4 D = *reinterpret_cast<const float4*>(st + 128 + e);
-            pw[e / 2] = pack_bf16(p[e] * (__uint_as_float(d[e]) - D.x), p[e + 1] * (__uint_as_float(d[e + 1]) - D.y));
-            pw[e / 2 + 1] = pack_bf16(p[e + 2] * (__uint_as_float(d[e + 2]) - D.z), p[e + 3] * (__uint_as_float(d[e + 3]) - D.w));
+          for (int j = 0; j < 4; j++) {
+            const float2 nd = *reinterpret_cast<const float2*>(st + 128 + j * 8);
+#pragma unroll
+            for (int x = 0; x < 2; x++)
+#pragma unroll
+              for (int v = 0; v < 2; v++) {
+                const int e = 4 * j + 2 * v;
+                float d0, d1;
+                upk2(mul2(pk2(p[x][e], p[x][e + 1]), add2(pk2(__uint_as_float(d[x][e]), __uint_as_float(d[x][e + 1])), pk2(nd.x, nd.y))), d0, d1);
+                wp[x][2 * j + v] = pack_bf16(d0, d1);
+              }
           }
         }
-        tc::tmem_st16(tdp, pw);
+        tc::tmem_st_frag(tdp, wp);
         tc::tmem_st_wait();
         tc::tc_fence_before();
         __syncwarp();
@@ -595,21 +680,39 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
           tc::mbar_arrive(&bar_stf[g & 1]);
         }
       }
-      // ---- epilogue: of dV, which is complete before dK, and then of dK (softmax scale and RoPE's backward rotation applied) every warp
-      // stores 32 columns; the rotation tables are on their way from the start
-      RopeUnits rp;
-      if (a.cosT) rope_units<H128>(rp, a.cosT, a.sinT, krow, qd * 16, lane, a.T - (krow - lane));
+      // ---- epilogue: dV, which is complete before dK, and then dK (softmax scale and RoPE's backward rotation applied), both through P's tile
+      Rope128 rp;
+      const int row0 = kt * 128 + lg * 32, nlive = a.T - row0;
+      auto send = [&](int x) {
+        x += h * H128;
+        tc::fence_async_smem();
+        named_bar_sync(1 + lg, 128);
+        if (nlive < 32) {
+          if (!*s_abort) tile128_rows(a.out + ((size_t)b * a.T + row0) * 3 * C + x, 3L * C, smem + S::P, lg, nlive, qd * 32 + lane);
+        } else if (sender) {
+          if (!*s_abort)
+            for (int c = 0; c < 2; c++) tc::tma_store_2d(&tm_out, smem + S::P + c * TILE_BYTES + lg * 4096, x + c * 64, b * a.T + row0);
+          tc::tma_commit_group();
+        }
+      };
+      uint32_t ra[2][8], rb[2][8];
       wait(&bar_dof[(g - 1) & 1], ((g - 1) >> 1) & 1, 90);
       __syncwarp();
       tc::tc_fence_after();
-      bf16* dst = a.out + ((size_t)(b * a.T + krow)) * 3 * C + C + h * H128;
-      store_pairs16<H128>(dst + C, 3L * C, t_dv + lane_addr, qd * 16, lane, *s_abort ? 0 : a.T - (krow - lane), 1.f, false, rp);
+      tc::tmem_ld_pairs_wait(t_dv + lane_addr + qd * 16, ra, t_dv + lane_addr + 64 + qd * 16, rb);
+      tile128_out(p_tile, ra, rb, lg, qd * 16, lane, 1.f, false, rp);
+      if (a.cosT) rope128(rp, a.cosT, a.sinT, row0, qd * 16, lane, a.T);      // (sooner there are no registers for them)
+      send(2 * C);
       wait(bar_done, li & 1, 71);
       __syncwarp();
       tc::tc_fence_after();
-      store_pairs16<H128>(dst, 3L * C, t_dk + lane_addr, qd * 16, lane, *s_abort ? 0 : a.T - (krow - lane), a.scale, a.cosT != nullptr, rp);
+      tc::tmem_ld_pairs_wait(t_dk + lane_addr + qd * 16, ra, t_dk + lane_addr + 64 + qd * 16, rb);
       tc::tc_fence_before();
+      rows_read();
+      tile128_out(p_tile, ra, rb, lg, qd * 16, lane, a.scale, a.cosT != nullptr, rp);
+      send(C);
     }
+    if (sender) tc::tma_wait_group<0>();
   }
   tc::tc_fence_before();
   __syncthreads();
@@ -618,7 +721,7 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
 }
 
 __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUtensorMap tm_do,
-                                                                     const AttnArgs a) {
+                                                                     const __grid_constant__ CUtensorMap tm_out, const AttnArgs a) {
   mlb_pdl_sync();
   using S = BwdQ128Smem;
   extern __shared__ uint8_t smem_raw[];
@@ -628,9 +731,9 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
            *bar_s = bars + 12 /*[2]*/, *bar_dp = bars + 14, *bar_done = bars + 15,
            *bar_ds = bars + 16 /*[2]: the thread that issues dQ may be a block behind*/;
   uint64_t* bar_end = bars + 18;      // [2]: the MMA threads' last commits
-  uint64_t *bar_o = bars + 20 /* dO */, *bar_of = bars + 21;
-  uint32_t* tmem_slot = (uint32_t*)(bars + 22);
-  volatile int* s_abort = (volatile int*)(bars + 23);
+  uint64_t *bar_o = bars + 20 /* dO */, *bar_of = bars + 21 /* dQ has left dO's place */, *bar_out = bars + 22 /* dQ is there */;
+  uint32_t* tmem_slot = (uint32_t*)(bars + 23);
+  volatile int* s_abort = (volatile int*)(bars + 24);
   if (attn_given_up()) return;
   const int nq = (a.T + 127) / 128, BH = a.B * a.H, C = a.H * H128;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -639,11 +742,12 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
   if (srow && tid < 64) s_sched[tid] = tid < a.sched_stride ? __ldg(srow + tid) : -1;
   const ItemList items{srow, s_sched, (int)blockIdx.x, (int)gridDim.x, nq * BH};
   if (tid == 0) {
-    for (int i = 0; i < 22; i++) tc::mbar_init(&bars[i], (i == 16 || i == 17) ? BWD128_E_WARPS : 1);
+    for (int i = 0; i < 23; i++) tc::mbar_init(&bars[i], (i == 16 || i == 17 || i == 22) ? BWD128_E_WARPS : 1);
     *s_abort = 0;
     tc::mbar_fence_init();
     tc::tma_prefetch_desc(&tm);
     tc::tma_prefetch_desc(&tm_do);
+    tc::tma_prefetch_desc(&tm_out);
   }
   if (warp == BWD128_MMA_WARP) tc::tmem_alloc(tmem_slot, 512);
   tc::tc_fence_before();
@@ -655,13 +759,14 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
   // item w = query tile (heaviest, the last, first) of (sample, head), with qt + 1 key blocks
   if (warp == BWD128_LOAD_WARP) {
     if (lane == 0) {
-      // The next query tile's Q is asked for when the last scores of this one are there, its dO when the last dP is
-      int g = 0, nx = 0, no = 0, odd = 0;      // odd: a K without its V
+      // The next query tile's Q is asked for when the last scores of this one are there, its dO when dQ has left by its place
+      // (behind the first two K: it comes last, and nothing waits for it alone)
+      int g = 0, gv = 0, nx = 0, no = 0;
       bool ok = true;
       for (int li = 0, w; ok && (w = items.at(li)) >= 0; li++) {
         const int qt = nq - 1 - w / BH, bh = w % BH, b = bh / a.H, xh = (bh % a.H) * H128;
-        for (int j = 0; j <= qt; j++, g++) {
-          const int ks = g % 3, vs = g & 1;
+        for (int j = 0; j <= qt; j++) {
+          const int ks = g % 3, vs = gv & 1;
           if (j == 0) {
             if (li > 0 && !wait(bar_qf, (li - 1) & 1, 72)) { ok = false; break; }
             nx++;
@@ -669,23 +774,25 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
             split_load<2>(smem + S::Q, &tm, bar_q, xh, qt * 128, b, 2);
           }
           if (g >= 3 && !wait(&bar_kf[ks], (g / 3 + 1) & 1, 73)) { ok = false; break; }
+          g++;
           tc::mbar_expect_tx(&bar_k[ks], T128_BYTES);
           split_load<2>(smem + S::K + ks * T128_BYTES, &tm, &bar_k[ks], C + xh, j * 128, b, 2);
-          if (j == 0) {
-            if (li > 0 && !wait(bar_of, (li - 1) & 1, 91)) { ok = false; odd = 1; break; }
+          if (j == min(1, qt)) {
+            if (li > 0 && !wait(bar_of, (li - 1) & 1, 91)) { ok = false; break; }
             no++;
             tc::mbar_expect_tx(bar_o, T128_BYTES);
             split_load<2>(smem + S::DO, &tm_do, bar_o, xh, qt * 128, b, 2);
           }
-          if (g >= 2 && !wait(&bar_vf[vs], ((g >> 1) + 1) & 1, 74)) { ok = false; odd = 1; break; }
+          if (gv >= 2 && !wait(&bar_vf[vs], ((gv >> 1) + 1) & 1, 74)) { ok = false; break; }
+          gv++;
           tc::mbar_expect_tx(&bar_v[vs], T128_BYTES);
           split_load<2>(smem + S::V + vs * T128_BYTES, &tm, &bar_v[vs], 2 * C + xh, j * 128, b, 2);
         }
       }
       attn_settle(bar_q, nx);
       attn_settle(bar_o, no);
-      for (int i = 0; i < 3; i++) attn_settle(&bar_k[i], (g + odd + 2 - i) / 3);
-      for (int i = 0; i < 2; i++) attn_settle(&bar_v[i], (g + 1 - i) / 2);
+      for (int i = 0; i < 3; i++) attn_settle(&bar_k[i], (g + 2 - i) / 3);
+      for (int i = 0; i < 2; i++) attn_settle(&bar_v[i], (gv + 1 - i) / 2);
     }
   } else if (warp == BWD128_MMA_WARP) {
     if (tc::elect_one()) {
@@ -720,7 +827,6 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
         for (int ks = 0; ks < 8; ks++) tc::mma_bf16_ss(t_dp, dO + off_k(ks, TILE_BYTES), dV + off_k(ks, TILE_BYTES), idesc_s, ks > 0);
         tc::mma_commit(bar_dp);
         tc::mma_commit(&bar_vf[gb & 1]);
-        if (c.j + 1 == c.n) tc::mma_commit(bar_of);
       };
       Cursor c0{0, 0, blocks(0)}, c1 = next(c0), c2 = next(c1);
       if (c0.n > 0) scores(0, c0);
@@ -758,12 +864,29 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
       tc::mma_commit(&bar_end[1]);
       attn_settle(&bar_end[1], 1);
     }
+  } else if (warp == BWD128_STAT_WARP) {
+    // dQ tiles on their way out
+    if (lane == 0) {
+      bool ok = true;
+      for (int li = 0, w; ok && (w = items.at(li)) >= 0; li++) {
+        const int qt = nq - 1 - w / BH, bh = w % BH, b = bh / a.H, x = (bh % a.H) * H128;
+        ok = wait(bar_out, li & 1, 94);
+        if (!ok) break;
+        for (int lg = 0; lg < 4; lg++)
+          if (a.T - (qt * 128 + lg * 32) >= 32)
+            for (int c = 0; c < 2; c++) tc::tma_store_2d(&tm_out, smem + S::DO + c * TILE_BYTES + lg * 4096, x + c * 64, b * a.T + qt * 128 + lg * 32);
+        tc::tma_commit_group();
+        tc::tma_wait_group_read<0>();
+        tc::mbar_arrive(bar_of);
+      }
+      tc::tma_wait_group<0>();
+    }
   } else if (warp < BWD128_E_WARPS) {
     const int lg = warp & 3, qd = warp >> 2, row = lg * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(lg * 32) << 16;
     const float sl2 = a.scale * LOG2E;
     int g = 0;
-    float next_nl = 0.f, next_delta = 0.f;      // this thread's query of the next item (fetched under the epilogue before it)
+    float next_nl = 0.f, next_delta = 0.f;      // this thread's query of the next item (fetched at the start of the one before it)
     auto fetch = [&](int w) {
       const int q = (nq - 1 - w / BH) * 128 + row;
       const size_t e = (size_t)(w % BH) * a.T + q;
@@ -774,8 +897,9 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
     if (w >= 0) fetch(w);
     for (int li = 0; w >= 0; li++) {
       const int qt = nq - 1 - w / BH, bh = w % BH, b = bh / a.H, h = bh % a.H;
-      const int qrow = qt * 128 + row;
       const float nl = next_nl, delta = next_delta;
+      w = items.at(li + 1);
+      if (w >= 0) fetch(w);
       for (int j = 0; j <= qt; j++, g++) {
         const uint32_t ts = tmem + (g & 1) * 128 + qd * 32 + lane_addr, tdp = t_dp + qd * 32 + lane_addr;
         wait(&bar_s[g & 1], (g >> 1) & 1, 79);
@@ -807,17 +931,24 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&bar_ds[g & 1]);
       }
-      // ---- epilogue: 32 columns by each warp, the rotation tables ahead of the last product
-      w = items.at(li + 1);
-      if (w >= 0) fetch(w);
-      RopeUnits rp;
-      if (a.cosT) rope_units<H128>(rp, a.cosT, a.sinT, qrow, qd * 16, lane, a.T - (qrow - lane));
+      // ---- epilogue, through dO's tile, which every dP has read
+      Rope128 rp;
+      const int row0 = qt * 128 + lg * 32, nlive = a.T - row0;
+      if (a.cosT) rope128(rp, a.cosT, a.sinT, row0, qd * 16, lane, a.T);
+      uint32_t ra[2][8], rb[2][8];
       wait(bar_done, li & 1, 81);
       __syncwarp();
       tc::tc_fence_after();
-      store_pairs16<H128>(a.out + ((size_t)(b * a.T + qrow)) * 3 * C + h * H128, 3L * C, t_dq + lane_addr, qd * 16, lane, *s_abort ? 0 : a.T - (qrow - lane),
-                          a.scale, a.cosT != nullptr, rp);
+      tc::tmem_ld_pairs_wait(t_dq + lane_addr + qd * 16, ra, t_dq + lane_addr + 64 + qd * 16, rb);
       tc::tc_fence_before();
+      tile128_out(tc::smem_u32(smem + S::DO), ra, rb, lg, qd * 16, lane, a.scale, a.cosT != nullptr, rp);
+      if (nlive < 32) {
+        named_bar_sync(1 + lg, 128);
+        if (!*s_abort) tile128_rows(a.out + ((size_t)b * a.T + row0) * 3 * C + h * H128, 3L * C, smem + S::DO, lg, nlive, qd * 32 + lane);
+      }
+      tc::fence_async_smem();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(bar_out);
     }
   }
   tc::tc_fence_before();

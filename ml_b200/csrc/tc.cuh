@@ -226,20 +226,6 @@ __device__ __forceinline__ void tmem_ld32x2_wait(uint32_t taddr_a, uint32_t (&a)
       : "r"(taddr_a), "r"(taddr_b)
       : "memory");
 }
-__device__ __forceinline__ void tmem_ld16x2_wait(uint32_t taddr_a, uint32_t (&a)[16], uint32_t taddr_b, uint32_t (&b)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%32];\n\t"
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%33];\n\t"
-      "tcgen05.wait::ld.sync.aligned;"
-      : "=&r"(a[0]), "=&r"(a[1]), "=&r"(a[2]), "=&r"(a[3]), "=&r"(a[4]), "=&r"(a[5]), "=&r"(a[6]), "=&r"(a[7]), "=&r"(a[8]), "=&r"(a[9]),
-        "=&r"(a[10]), "=&r"(a[11]), "=&r"(a[12]), "=&r"(a[13]), "=&r"(a[14]), "=&r"(a[15]), "=&r"(b[0]), "=&r"(b[1]), "=&r"(b[2]),
-        "=&r"(b[3]), "=&r"(b[4]), "=&r"(b[5]), "=&r"(b[6]), "=&r"(b[7]), "=&r"(b[8]), "=&r"(b[9]), "=&r"(b[10]), "=&r"(b[11]),
-        "=&r"(b[12]), "=&r"(b[13]), "=&r"(b[14]), "=&r"(b[15])
-      : "r"(taddr_a), "r"(taddr_b)
-      : "memory");
-}
 // Fragments: 32 columns of the warp's 32 rows, spread as a matrix instruction's accumulator is.  r[h][4 j + 2 v + x] is row 16 h + 8 v + lane / 4,
 // column 8 j + 2 (lane % 4) + x: a thread has two adjacent columns of each eight, for four rows, so that what belongs to a column is
 // read from shared memory once for four rows and by a quarter of the lanes.
@@ -281,6 +267,21 @@ __device__ __forceinline__ void tmem_ld_frag16x2_wait(uint32_t taddr, uint32_t (
         "=&r"(b[3]), "=&r"(b[4]), "=&r"(b[5]), "=&r"(b[6]), "=&r"(b[7]), "=&r"(b[8]), "=&r"(b[9]), "=&r"(b[10]), "=&r"(b[11]),
         "=&r"(b[12]), "=&r"(b[13]), "=&r"(b[14]), "=&r"(b[15])
       : "r"(taddr), "r"(taddr + 32)
+      : "memory");
+}
+// Twice 16 columns of the warp's 32 rows: a[h][4 j + 2 v + x] is row 16 h + 8 v + lane / 4, column 8 j + 2 (lane % 4) + x.
+__device__ __forceinline__ void tmem_ld_pairs_wait(uint32_t taddr_a, uint32_t (&a)[2][8], uint32_t taddr_b, uint32_t (&b)[2][8]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%32];\n\t"
+      "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%8, %9, %10, %11, %12, %13, %14, %15}, [%33];\n\t"
+      "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%16, %17, %18, %19, %20, %21, %22, %23}, [%34];\n\t"
+      "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%24, %25, %26, %27, %28, %29, %30, %31}, [%35];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=&r"(a[0][0]), "=&r"(a[0][1]), "=&r"(a[0][2]), "=&r"(a[0][3]), "=&r"(a[0][4]), "=&r"(a[0][5]), "=&r"(a[0][6]), "=&r"(a[0][7]),
+        "=&r"(a[1][0]), "=&r"(a[1][1]), "=&r"(a[1][2]), "=&r"(a[1][3]), "=&r"(a[1][4]), "=&r"(a[1][5]), "=&r"(a[1][6]), "=&r"(a[1][7]),
+        "=&r"(b[0][0]), "=&r"(b[0][1]), "=&r"(b[0][2]), "=&r"(b[0][3]), "=&r"(b[0][4]), "=&r"(b[0][5]), "=&r"(b[0][6]), "=&r"(b[0][7]),
+        "=&r"(b[1][0]), "=&r"(b[1][1]), "=&r"(b[1][2]), "=&r"(b[1][3]), "=&r"(b[1][4]), "=&r"(b[1][5]), "=&r"(b[1][6]), "=&r"(b[1][7])
+      : "r"(taddr_a), "r"(taddr_a + (16u << 16)), "r"(taddr_b), "r"(taddr_b + (16u << 16))
       : "memory");
 }
 // Four 8 x 8 bf16 matrices of such a fragment to shared memory: lane l gives the 16 bytes of row l % 8 of matrix l / 8.

@@ -1754,3 +1754,25 @@ def test_nodes_run_on_the_stream_they_are_called_on(name):
                 assert all(torch.equal(a, b) for a, b in zip(got, want[i]))
     finally:
         nat().lib().mlb_gemm_set_splits(0)
+
+
+@pytest.mark.parametrize("T", [1, 31, 33, 96, 127, 129, 161, 255, 300, 385])
+@pytest.mark.parametrize("B,H,hd", [(1, 2, 64), (40, 6, 64), (1, 2, 128), (24, 8, 128)])
+def test_causal_backward_at_tile_edges_with_rope(B, T, H, hd):
+    """Gradients through RoPE where a tile's last 32 rows are whole (they leave by TMA), cut (by row) or not there, with one item per CTA and with
+    several.  Against 64 bits; the bound is that of the test without RoPE: P, dS and the result in bf16, the rounding of O in delta."""
+    torch.manual_seed(T + hd + B)
+    qkv, dout = rnd(B * T, 3 * H * hd), rnd(B * T, H * hd)
+    cos, sin = ref.rope_tables(T, hd, 10000.0, dev())
+    n = nat()
+    rot = qkv.clone()
+    n.rope_fwd(rot, cos, sin, B, T, H, hd)
+    out, lse, dqkv = rnd(B * T, H * hd), torch.empty(B, H, T, device=dev()), torch.full_like(qkv, float("nan"))
+    n.attn_fwd(out, lse, rot, B, T, H, hd)
+    assert n.attn_bwd(dqkv, dout, rot, out, lse, B, T, H, hd, rope=(cos, sin))
+    _, _, ed = _attn64(rot, dout, B, T, H, hd, True)
+    e = ed.view(B, T, 3, H, 2, hd // 2).clone()
+    c, s = cos.double().view(1, T, 1, 1, hd // 2), sin.double().view(1, T, 1, 1, hd // 2)
+    d0, d1 = e[:, :, :2, :, 0].clone(), e[:, :, :2, :, 1].clone()
+    e[:, :, :2, :, 0], e[:, :, :2, :, 1] = d0 * c + d1 * s, d1 * c - d0 * s
+    assert _rel(dqkv, e.view_as(dqkv)) < 2 ** -7
