@@ -39,9 +39,12 @@ __device__ __forceinline__ uint64_t desc64_base_mn(uint32_t base) { return tc::s
 // TMEM column of the hi term of k-step ks (16 rows of the 64-row block); the lo term is 16 columns further
 __device__ __forceinline__ uint32_t split_col(int ks) { return (uint32_t)((ks >> 1) * 32 + (ks & 1) * 8); }
 
-__device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo) {
+__device__ __forceinline__ void split2(uint64_t ab, uint32_t& hi, uint32_t& lo) {      // (two values an instruction, here and in the kernels)
+  float a, b;
+  upk2(ab, a, b);
   hi = pack_bf16(a, b);
-  lo = pack_bf16(a - __uint_as_float(hi << 16), b - __uint_as_float(hi & 0xffff0000u));
+  upk2(add2(ab, pk2(-__uint_as_float(hi << 16), -__uint_as_float(hi & 0xffff0000u))), a, b);
+  lo = pack_bf16(a, b);
 }
 
 // rows [r0, r0 + 64 * boxes) of `CH` 64-column chunks starting at column x0 of sample z
@@ -150,7 +153,9 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
     tc::mbar_fence_init();
     tc::tma_prefetch_desc(&tm);
   }
-  auto leader = [&]() -> bool { return warp == 0 && tc::elect_one(); };      // the thread that loads and multiplies (whole warps ask)
+  // The threads that multiply and that load (whole warps ask): of two warps, each has its own rows to work on besides
+  auto leader = [&]() -> bool { return warp == 0 && tc::elect_one(); };
+  auto loader = [&]() -> bool { return warp == 3 && tc::elect_one(); };
   if (warp == 0) tc::tmem_alloc(tmem_slot, TMEM_COLS);
   tc::tc_fence_before();
   __syncthreads();
@@ -165,7 +170,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
   const int nks = a.hd >> 4;
   const uint64_t dQ = desc_base_k(tc::smem_u32(smem + S::Q)), dK0 = desc_base_k(tc::smem_u32(smem + S::K)),
                  dV0 = desc64_base_mn(tc::smem_u32(smem + S::V));
-  int loads = 0;      // blocks of K and V asked for (thread 0)
+  int loads = 0;      // blocks of K and V asked for (loader)
   auto load_kv = [&](int j) {
     const int sl = j & 1;
     loads = j + 1;
@@ -185,10 +190,12 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
     }
     tc::mma_commit(bar_s);
   };
-  if (leader()) {
+  if (loader()) {
     tc::mbar_expect_tx(bar_q, 2 * CH * BOX_BYTES);
     split_load<CH>(smem + S::Q, &tm, bar_q, h * a.hd, q0, b, 2);
     load_kv(0);
+  }
+  if (leader()) {
     wait(bar_q, 0, 40);
     issue_s(0);
   }
@@ -199,7 +206,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
 #pragma unroll
   for (int i = 0; i < HDT; i++) o[i] = 0.f;
   for (int j = 0; j < nkb; j++) {
-    if (leader() && j + 1 < nkb && !*s_abort) load_kv(j + 1);     // (block j - 1, the buffers' last reader, is complete: bar_o of it was waited for)
+    if (loader() && j + 1 < nkb && !*s_abort) load_kv(j + 1);     // (block j - 1, the buffers' last reader, is complete: bar_o of it was waited for)
     wait(bar_s, j & 1, 42);
     __syncwarp();
     tc::tc_fence_after();
@@ -219,17 +226,19 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
     };
     // (an encoder's sequence is a square and the class token: its last block has few keys, and the second half of it none)
     const bool both = k0 + 32 < a.T;
-    float mx = m;
+    float top = -INFINITY;
 #pragma unroll
     for (int half = 0; half < 2; half++) {
       if (half && !both) break;
       uint32_t r[32];
       load_scores(half, r);
 #pragma unroll
-      for (int i = 0; i < 32; i += 2) mx = max3(mx, __uint_as_float(r[i]) * sl2, __uint_as_float(r[i + 1]) * sl2);
+      for (int i = 0; i < 32; i += 2) top = max3(top, __uint_as_float(r[i]), __uint_as_float(r[i + 1]));
     }
+    const float mx = fmaxf(m, top * sl2);      // (the largest product is that of the largest score)
     const float mu = mx == -INFINITY ? 0.f : mx;      // nothing finite seen yet: exp2(-inf - 0) = 0
     const float alpha = ex2_approx(m - mu);
+    const uint64_t sl2x2 = pk2(sl2, sl2), nmu2 = pk2(-mu, -mu), alpha2 = pk2(alpha, alpha);
     m = mx;
     float rs = 0.f;
 #pragma unroll
@@ -239,10 +248,12 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
       load_scores(half, r);
 #pragma unroll
       for (int i = 0; i < 16; i++) {
-        const float p0 = ex2_approx(fmaf(__uint_as_float(r[2 * i]), sl2, -mu));
-        const float p1 = ex2_approx(fmaf(__uint_as_float(r[2 * i + 1]), sl2, -mu));
+        float p0, p1;
+        upk2(fma2(pk2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), sl2x2, nmu2), p0, p1);
+        p0 = ex2_approx(p0);
+        p1 = ex2_approx(p1);
         rs += p0 + p1;
-        split2(p0, p1, hi[i], lo[i]);
+        split2(pk2(p0, p1), hi[i], lo[i]);
       }
       tc::tmem_st16(t_s + half * 32 + lane_addr, hi);
       tc::tmem_st16(t_s + half * 32 + 16 + lane_addr, lo);
@@ -277,7 +288,8 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
       uint32_t ro[32];
       tc::tmem_ld32_wait(t_o + c + lane_addr, ro);
 #pragma unroll
-      for (int i = 0; i < 32; i++) o[c + i] = fmaf(o[c + i], alpha, __uint_as_float(ro[i]));
+      for (int i = 0; i < 32; i += 2)
+        upk2(fma2(pk2(o[c + i], o[c + i + 1]), alpha2, pk2(__uint_as_float(ro[i]), __uint_as_float(ro[i + 1]))), o[c + i], o[c + i + 1]);
     }
     tc::tc_fence_before();
   }
@@ -317,6 +329,8 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_fwd_k(const __grid_c
       tc::report_given_up(s_abort);
       tc::mma_commit(bar_end);
       attn_settle(bar_end, 1);
+    }
+    if (loader()) {
       attn_settle(bar_q, 1);
       for (int sl = 0; sl < 2; sl++) {
         attn_settle(&bar_k[sl], (loads + 1 - sl) / 2);
@@ -373,7 +387,9 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
     tc::tma_prefetch_desc(&tm);
     tc::tma_prefetch_desc(&tm_do);
   }
-  auto leader = [&]() -> bool { return warp == 0 && tc::elect_one(); };      // the thread that loads and multiplies (whole warps ask)
+  // The threads that multiply and that load (whole warps ask): of two warps, each has its own rows to work on besides
+  auto leader = [&]() -> bool { return warp == 0 && tc::elect_one(); };
+  auto loader = [&]() -> bool { return warp == 3 && tc::elect_one(); };
   if (warp == 0) tc::tmem_alloc(tmem_slot, TMEM_COLS);
   tc::tc_fence_before();
   __syncthreads();
@@ -391,7 +407,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
   const uint64_t drx = desc_base_k(tc::smem_u32(smem + S::RX)), dry = desc_base_k(tc::smem_u32(smem + S::RY));
   const uint64_t dsx = desc_base_k(tc::smem_u32(smem + S::SX)), dsy = desc_base_k(tc::smem_u32(smem + S::SY));      // as B of the scores
   const uint64_t gsx = desc64_base_mn(tc::smem_u32(smem + S::SX)), gsy = desc64_base_mn(tc::smem_u32(smem + S::SY));   // as B of the gradients
-  int loads = 0;      // streamed blocks asked for (thread 0)
+  int loads = 0;      // streamed blocks asked for (loader)
   auto load_x = [&](int it) {
     const int sl = it & 1, y = (i0 + it) * 64;
     loads = it + 1;
@@ -413,61 +429,77 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
         if (ks < nks) tc::mma_bf16_ss(t_d, dry + off_k(ks, TILE_BYTES), sy + off_k(ks, BOX_BYTES), idesc_s, ks > 0);
     }
   };
-  // statistics of the 64 streamed queries (KV form); a query past the end has lse = +inf: p = 0
+  // statistics of the 64 streamed queries (KV form), -lse log2 e and -delta; a query past the end has lse = +inf: p = 0
   auto load_stat = [&](int it) {
     const int q = (i0 + it) * 64 + (tid & 63);
     float* st = stat + (it & 1) * 128;
-    if (tid < 64) st[tid] = q < a.T ? a.lse[si + q] * LOG2E : INFINITY;
-    else st[tid] = q < a.T ? a.delta[si + q] : 0.f;
+    if (tid < 64) st[tid] = q < a.T ? -a.lse[si + q] * LOG2E : -INFINITY;
+    else st[tid] = q < a.T ? -a.delta[si + q] : 0.f;
   };
-  if (leader()) {
+  if (loader()) {
     tc::mbar_expect_tx(bar_r, 4 * CH * BOX_BYTES);
     split_load<CH>(smem + S::RX, &tm, bar_r, KV ? C + xh : xh, r0, b, 2);
     split_load<CH>(smem + S::RY, KV ? &tm : &tm_do, bar_r, KV ? 2 * C + xh : xh, r0, b, 2);
     load_x(0);
+  }
+  if (leader()) {
     wait(bar_r, 0, 45);
     issue_scores(0);
     tc::mma_commit(bar_s);
   }
   const float sl2 = a.scale * LOG2E;
   const int row = r0 + tid;
-  float lse_r = INFINITY, delta_r = 0.f;      // dQ form: this thread's query
+  const uint64_t sl2x2 = pk2(sl2, sl2);
+  float nlse_r = -INFINITY, ndelta_r = 0.f;      // dQ form: this thread's query, -lse log2 e and -delta
   if (KV) {
     load_stat(0);
   } else if (row < a.T) {
-    lse_r = a.lse[si + row] * LOG2E;
-    delta_r = a.delta[si + row];
+    nlse_r = -a.lse[si + row] * LOG2E;
+    ndelta_r = -a.delta[si + row];
   }
   __syncthreads();
   for (int it = 0; it < n; it++) {
     wait(bar_s, it & 1, 47);
     __syncwarp();
     tc::tc_fence_after();
-    if (leader() && it + 1 < n && !*s_abort) load_x(it + 1);      // every MMA issued so far is complete: the other buffer is free
+    if (loader() && it + 1 < n && !*s_abort) load_x(it + 1);      // every MMA issued so far is complete: the other buffer is free
     const int c0 = (i0 + it) * 64;
     const float* st = stat + (it & 1) * 128;
     const bool both = c0 + 32 < a.T;      // (as in forward)
+    const bool cut = KV ? a.causal && c0 < r0 + 128 : (a.causal && c0 + 63 > r0) || c0 + 64 > a.T;      // is any of the tile's pairs masked?
 #pragma unroll
     for (int half = 0; half < 2; half++) {
       if (half && !both) break;
       uint32_t rs[32], rd[32];
       tc::tmem_ld32x2_wait(t_s + half * 32 + lane_addr, rs, t_d + half * 32 + lane_addr, rd);
+      float p[32];
+#pragma unroll
+      for (int e = 0; e < 32; e += 4) {
+        const float4 nl = KV ? *reinterpret_cast<const float4*>(st + half * 32 + e) : make_float4(nlse_r, nlse_r, nlse_r, nlse_r);
+        float z[4];
+        upk2(fma2(pk2(__uint_as_float(rs[e]), __uint_as_float(rs[e + 1])), sl2x2, pk2(nl.x, nl.y)), z[0], z[1]);
+        upk2(fma2(pk2(__uint_as_float(rs[e + 2]), __uint_as_float(rs[e + 3])), sl2x2, pk2(nl.z, nl.w)), z[2], z[3]);
+#pragma unroll
+        for (int x = 0; x < 4; x++) p[e + x] = ex2_approx(z[x]);
+      }
+      if (cut) {      // causal: the key may not lie behind the query; dQ form: keys past the end are not there (KV form: lse = +inf)
+#pragma unroll
+        for (int e = 0; e < 32; e++) {
+          const int col = c0 + half * 32 + e;
+          if (KV ? col < row : ((a.causal && col > row) || col >= a.T)) p[e] = 0.f;
+        }
+      }
       uint32_t hi[16], lo[16], gh[16], gl[16];
 #pragma unroll
-      for (int i = 0; i < 16; i++) {
-        float p[2], g[2];
-#pragma unroll
-        for (int x = 0; x < 2; x++) {
-          const int e = 2 * i + x, col = half * 32 + e;
-          const float L = KV ? st[col] : lse_r, D = KV ? st[64 + col] : delta_r;
-          float pv = ex2_approx(fmaf(__uint_as_float(rs[e]), sl2, -L));
-          // causal: the key may not lie behind the query; dQ form: keys past the end are not there (KV form: lse = +inf)
-          if (KV ? (a.causal && c0 + col < row) : ((a.causal && c0 + col > row) || c0 + col >= a.T)) pv = 0.f;
-          p[x] = pv;
-          g[x] = pv * (__uint_as_float(rd[e]) - D);
+      for (int e = 0; e < 32; e += 4) {
+        const float4 nd = KV ? *reinterpret_cast<const float4*>(st + 64 + half * 32 + e) : make_float4(ndelta_r, ndelta_r, ndelta_r, ndelta_r);
+        const uint64_t p01 = pk2(p[e], p[e + 1]), p23 = pk2(p[e + 2], p[e + 3]);
+        if (KV) {
+          split2(p01, hi[e / 2], lo[e / 2]);
+          split2(p23, hi[e / 2 + 1], lo[e / 2 + 1]);
         }
-        if (KV) split2(p[0], p[1], hi[i], lo[i]);
-        split2(g[0], g[1], gh[i], gl[i]);
+        split2(mul2(p01, add2(pk2(__uint_as_float(rd[e]), __uint_as_float(rd[e + 1])), pk2(nd.x, nd.y))), gh[e / 2], gl[e / 2]);
+        split2(mul2(p23, add2(pk2(__uint_as_float(rd[e + 2]), __uint_as_float(rd[e + 3])), pk2(nd.z, nd.w))), gh[e / 2 + 1], gl[e / 2 + 1]);
       }
       if (KV) {
         tc::tmem_st16(t_s + half * 32 + lane_addr, hi);
@@ -512,7 +544,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
   // (a query whose lse or delta is NaN makes all of its dQ NaN, rightly, and a NaN lse all of the dK and dV that see it)
   bool nan = split_store_rows<HDT>(KV ? dst + C : dst, 3L * C, (KV ? t_a1 : t_a0) + lane_addr, a.hd, a.scale, lane, nlive);
   if (KV) nan |= split_store_rows<HDT>(dst + 2 * C, 3L * C, t_a0 + lane_addr, a.hd, 1.f, lane, nlive);
-  if (!KV) nan = nan && lse_r == lse_r && delta_r == delta_r;
+  if (!KV) nan = nan && nlse_r == nlse_r && ndelta_r == ndelta_r;
   const unsigned rows = __ballot_sync(0xffffffffu, nan && lane < nlive);
   if (lane == 0) s_nan[warp] = rows;
   tc::tc_fence_before();
@@ -522,6 +554,8 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
       tc::report_given_up(s_abort);
       tc::mma_commit(bar_end);
       attn_settle(bar_end, 1);
+    }
+    if (loader()) {
       attn_settle(bar_r, 1);
       for (int sl = 0; sl < 2; sl++) attn_settle(&bar_x[sl], (loads + 1 - sl) / 2);
     }
