@@ -312,8 +312,8 @@ __global__ void __launch_bounds__(256) layernorm_bwd_k(bf16* __restrict__ dx, fl
 // floats, `ticket` = 1 + RMS_GROUPS ints that are 0 on entry and left 0 on exit.
 constexpr int RMS_GROUPS = 16;
 // Up to 32 blocks (256 rows) there is one group, and its last block adds the partial rows up with all of its threads.
-// VPL = C / 256 (vectors of 8 per lane) up to 3; PART: one vector per lane of rows narrower than 256 (C % 8 == 0); 0 = generic C (scalar path).
-template <int VPL, bool PART = false>
+// NARROW: one vector of eight per lane, rows narrower than 256 (C % 8 == 0); otherwise any C, alignment and width, by scalars.
+template <bool NARROW>
 __global__ void __launch_bounds__(256, 2) rmsnorm_bwd_k(bf16* __restrict__ dx, float* __restrict__ dw, const bf16* __restrict__ dy,
                                                      const bf16* __restrict__ x, const bf16* __restrict__ w,
                                                      const float* __restrict__ rstd, const bf16* __restrict__ add, long rows,
@@ -325,66 +325,41 @@ __global__ void __launch_bounds__(256, 2) rmsnorm_bwd_k(bf16* __restrict__ dx, f
   for (int i = threadIdx.x; i < C; i += blockDim.x) sh[i] = 0.f;
   __syncthreads();
   const float invC = 1.f / (float)C;
-  if (VPL > 0) {
-    constexpr int NV = VPL > 0 ? VPL : 1;
-    constexpr bool CACHE_W = NV <= 2;  // the weight vector stays in registers (two resident blocks per SM leave 128 per thread)
-    constexpr int NW = CACHE_W ? NV : 1;
-    float acc[NV][8];
-    float ww[NW][8] = {};
-    const bool mine = !PART || lane * 8 < C;      // this lane has columns
+  if (NARROW) {
+    float acc[8], ww[8] = {};
+    const bool mine = lane * 8 < C;      // this lane has columns
+    if (mine) load8(w + lane * 8, ww);
 #pragma unroll
-    for (int v = 0; v < NV; v++) {
-      if (CACHE_W && mine) load8(w + (v * 32 + lane) * 8, ww[v]);
-#pragma unroll
-      for (int j = 0; j < 8; j++) acc[v][j] = 0.f;
-    }
+    for (int j = 0; j < 8; j++) acc[j] = 0.f;
     for (long row = (long)blockIdx.x * nwarp + warp; row < rows; row += (long)gridDim.x * nwarp) {
       const float r = rstd[row];
-      // The row's x, dy and residual-stream gradient stay in registers PACKED (four registers per eight values) between
-      // the two passes, and every load of the row is issued before the row's reduction: `add` does not depend on it, and
-      // fetching it only afterwards cost a second DRAM round trip per row.
-      uint4 xr[NV], dr[NV], ar[NV];
-      float dot = 0.f;
+      // every load of the row is issued before its reduction: `add` does not depend on it, and fetching it only
+      // afterwards cost a second DRAM round trip per row
+      const long off = row * C + lane * 8;
+      const uint4 zero = make_uint4(0, 0, 0, 0);
+      const uint4 xr = mine ? *reinterpret_cast<const uint4*>(x + off) : zero;
+      const uint4 dr = mine ? *reinterpret_cast<const uint4*>(dy + off) : zero;
+      const uint4 ar = add && mine ? *reinterpret_cast<const uint4*>(add + off) : zero;
+      float xf[8], df[8], o[8], dot = 0.f;
+      unpack8(xr, xf);
+      unpack8(dr, df);
+      unpack8(ar, o);
 #pragma unroll
-      for (int v = 0; v < NV; v++) {
-        const long off = row * C + (v * 32 + lane) * 8;
-        const int cw = CACHE_W ? v : 0;
-        xr[v] = mine ? *reinterpret_cast<const uint4*>(x + off) : make_uint4(0, 0, 0, 0);
-        dr[v] = mine ? *reinterpret_cast<const uint4*>(dy + off) : make_uint4(0, 0, 0, 0);
-        ar[v] = add && mine ? *reinterpret_cast<const uint4*>(add + off) : make_uint4(0, 0, 0, 0);
-        if (!CACHE_W) load8(w + (v * 32 + lane) * 8, ww[0]);
-        float xf[8], df[8];
-        unpack8(xr[v], xf);
-        unpack8(dr[v], df);
-#pragma unroll
-        for (int j = 0; j < 8; j++) dot += df[j] * ww[cw][j] * xf[j];
-      }
+      for (int j = 0; j < 8; j++) dot += df[j] * ww[j] * xf[j];
       dot = warp_sum(dot);
       const float k = r * r * r * invC * dot;
 #pragma unroll
-      for (int v = 0; v < NV; v++) {
-        const long off = row * C + (v * 32 + lane) * 8;
-        const int cw = CACHE_W ? v : 0;
-        if (!CACHE_W) load8(w + (v * 32 + lane) * 8, ww[0]);
-        float xf[8], df[8], o[8];
-        unpack8(xr[v], xf);
-        unpack8(dr[v], df);
-        unpack8(ar[v], o);
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-          o[j] += df[j] * ww[cw][j] * r - xf[j] * k;
-          acc[v][j] += df[j] * xf[j] * r;
-        }
-        if (mine) store8(dx + off, o);
+      for (int j = 0; j < 8; j++) {
+        o[j] += df[j] * ww[j] * r - xf[j] * k;
+        acc[j] += df[j] * xf[j] * r;
       }
+      if (mine) store8(dx + off, o);
     }
     // fold the 8 warps' register partials in warp order (deterministic)
     for (int wv = 0; wv < nwarp; wv++) {
       if (warp == wv && mine) {
 #pragma unroll
-        for (int v = 0; v < NV; v++)
-#pragma unroll
-          for (int j = 0; j < 8; j++) sh[(v * 32 + lane) * 8 + j] += acc[v][j];
+        for (int j = 0; j < 8; j++) sh[lane * 8 + j] += acc[j];
       }
       __syncthreads();
     }
@@ -422,7 +397,7 @@ __global__ void __launch_bounds__(256, 2) rmsnorm_bwd_k(bf16* __restrict__ dx, f
   __syncthreads();
   if (!is_last) return;
   __threadfence();
-  if (PART && nb <= 32) {
+  if (NARROW && nb <= 32) {
     // slice q of the threads takes rows q, q + slices, ...; the slices are added in order (C < 256: at least four of them, at most 1024 floats)
     const int vecs = C >> 2, slices = (int)blockDim.x / vecs, q = threadIdx.x / vecs, c = threadIdx.x % vecs * 4;
     if (q < slices) {
@@ -507,8 +482,7 @@ static constexpr int norm_ring_bytes(int vecs) { return 2 * 256 * 16 * vecs; }
 // Norm backward over whole rows per thread group: C / 8 threads share a row, each owning 8 columns for all of the group's rows, so the
 // column sums (dw, and db of LayerNorm) stay in 8 (16) registers and need no folding over a warp's rows.  Three rows at a time:
 // their 6-9 16-byte loads are in flight together and their dots cost one barrier.  One warp per row (rmsnorm_bwd_k)
-// needs C / 4 accumulators per lane, which at C = 2048 spill: 72 us for 16384 rows against 44 here and 4 for the fold.  (Below 1024 columns
-// the same ring gained that kernel nothing: 16384 x 768 with a residual 25.2 and 25.3 us.)
+// needs C / 4 accumulators per lane, which at C = 2048 spill: 72 us for 16384 rows against 44 here and 4 for the fold.
 // Partial sums: partial[block][C (RMS) | 2 C (LN: dw, db)], added up by fold_cols_k.
 // Shapes: C % 256 == 0 and C <= 2048 (whole warps, at most 256 threads a row).
 constexpr int NB_ROWS = 3;
@@ -666,7 +640,8 @@ __global__ void __launch_bounds__(256) colsum_k(float* __restrict__ partial, con
   partial[(size_t)blockIdx.y * N + col] = s;
 }
 // The partial rows added up in a fixed order: columns [0, C) to dw, [C, W) to db (either may be null).  bf16: rounded and stored;
-// fp32: added to what is there.  A block takes 32 columns, 8 row slices: slice q adds rows q, q + 8, ... and the slices are added in order.
+// fp32: added to what is there.  A block takes 32 columns, 8 row slices: slice q adds rows q, q + 8, ..., a trip's loads and the slices as trees (a chain of
+// sums errs more: 16384 x 768 normal numbers, dw to 2.2e-5 rms as chains, 1.7e-5 so).
 // Bound by latency: FOLD_ROWS loads are in flight per thread, up to 296 rows come in four trips (all 40 at once 0.6 us more; norm backward and fold of
 // 3152 x 768 9.7 us with 10, 10.1 with 40, 11.0 in a plain loop).
 constexpr int FOLD_THREADS = 256, FOLD_ROWS = 10;
@@ -682,14 +657,16 @@ __global__ void __launch_bounds__(FOLD_THREADS) fold_cols_k(void* __restrict__ d
 #pragma unroll
       for (int k = 0; k < FOLD_ROWS; k++) v[k] = r + 8 * k < nrows ? partial[(size_t)(r + 8 * k) * W + c] : 0.f;
 #pragma unroll
-      for (int k = 0; k < FOLD_ROWS; k++) s += v[k];
+      for (int w = 1; w < FOLD_ROWS; w *= 2)
+#pragma unroll
+        for (int k = 0; k + w < FOLD_ROWS; k += 2 * w) v[k] += v[k + w];
+      s += v[0];
     }
   }
   red[sl][lane] = s;
   __syncthreads();
   if (sl != 0 || c >= W) return;
-#pragma unroll
-  for (int i = 1; i < 8; i++) s += red[i][lane];
+  s = ((red[0][lane] + red[1][lane]) + (red[2][lane] + red[3][lane])) + ((red[4][lane] + red[5][lane]) + (red[6][lane] + red[7][lane]));
   void* dst = c < C ? dw : db;
   if (dst == nullptr) return;
   const int i = c < C ? c : c - C;
@@ -1563,18 +1540,17 @@ MLB_API int mlb_rmsnorm_bwd(void* dx, float* dw, const void* dy, const void* x, 
   mlb_launch(rmsnorm_bwd_k<__VA_ARGS__>, dim3(blocks), dim3(256), sh, st, (bf16*)dx, dw, (const bf16*)dy, (const bf16*)x, (const bf16*)w, rstd,   \
                                             (const bf16*)add, rows, C, partial, ticket)
   if (sh > 48 * 1024) return -3;
-  if (C >= 1024 && norm_rows_ok(dx, dy, x, w, add, rows, C)) {      // (narrower rows fit a warp's registers, and one launch)
+  // Whole multiples of 256 columns: a block's threads share a row instead of a warp having one, and the partial rows are folded by a
+  // kernel of their own, which overlaps this one's end.  One warp a row, with the fold by the blocks that finish last, against this, inputs
+  // not in L2: 16384 x 768 31.7 -> 29.7 us, 4096 x 768 21 -> 17.4, 64 x 768 13.3 -> 11.3, 65536 x 256 46 -> 35.8, 4096 x 512 17.4 = 17.4,
+  // 16384 x 512 25.6 = 25.6 (in L2 14.1 -> 16.1, the one size that is slower).
+  if (norm_rows_ok(dx, dy, x, w, add, rows, C)) {
     norm_rows_launch<false>(dx, dw, nullptr, false, dy, x, w, nullptr, rstd, add, rows, C, partial, st);
     LAUNCH_RET;
   }
   const bool narrow = C < 256 && C % 8 == 0 && (((uintptr_t)dx | (uintptr_t)dy | (uintptr_t)x | (uintptr_t)w | (uintptr_t)add | (uintptr_t)partial) & 15) == 0;
-  if (narrow) { RB(1, true); LAUNCH_RET; }
-  switch ((C % 256 == 0) ? C / 256 : 0) {
-    case 1: RB(1); break;
-    case 2: RB(2); break;
-    case 3: RB(3); break;
-    default: RB(0); break;
-  }
+  if (narrow) RB(true);
+  else RB(false);
 #undef RB
   LAUNCH_RET;
 }

@@ -1490,6 +1490,20 @@ def test_rmsnorm_backward_of_few_or_narrow_rows(rows, C, add):
         assert torch.equal(runs[0][0], runs[1][0]) and torch.equal(runs[0][1], runs[1][1])
 
 
+@pytest.mark.parametrize("rows,C,shift", [(1, 256, 0), (25, 512, 0), (2369, 256, 0), (7200, 768, 0), (25, 512, 1), (9, 768, 8), (3, 256, 4)])
+def test_rmsnorm_backward_of_whole_vectors_of_columns(rows, C, shift):
+    """Rows that share a block's threads, past one round of its groups, and the same widths from a place where vectors may not be loaded."""
+    torch.manual_seed(rows + C)
+    big = rnd(rows * C + 8)
+    x, dy, w, a = big[shift:shift + rows * C].view(rows, C), rnd(rows, C), 1 + rnd(1, C, scale=0.1).view(-1), rnd(rows, C)
+    rstd = torch.rand(rows, device=dev()) + 0.5
+    dx, dw = torch.empty_like(a), torch.ones(C, device=dev())
+    nat().rmsnorm_bwd(dx, dw, dy, x, w, rstd, a)
+    xd, dd, wd, r = x.double(), dy.double(), w.double(), rstd.double()[:, None]
+    ex = a.double() + r * wd * dd - xd * r ** 3 / C * (dd * wd * xd).sum(1, keepdim=True)
+    assert _rel(dx, ex) < 2 ** -8 and _rel(dw, 1 + (dd * xd * r).sum(0)) < 1e-5
+
+
 @pytest.mark.parametrize("rows", [1, 7, 300])
 @pytest.mark.parametrize("C", [256, 512, 768, 1024, 1280, 1536, 1792, 2048, 264, 40])
 @pytest.mark.parametrize("bias", [False, True])
