@@ -640,12 +640,13 @@ __global__ void __launch_bounds__(256) colsum_k(float* __restrict__ partial, con
   partial[(size_t)blockIdx.y * N + col] = s;
 }
 // The partial rows added up in a fixed order: columns [0, C) to dw, [C, W) to db (either may be null).  bf16: rounded and stored;
-// fp32: added to what is there.  A block takes 32 columns, 8 row slices: slice q adds rows q, q + 8, ..., a trip's loads and the slices as trees (a chain of
-// sums errs more: 16384 x 768 normal numbers, dw to 2.2e-5 rms as chains, 1.7e-5 so).
+// fp32: added to what is there.  A block takes 32 columns, 8 row slices: slice q adds rows q, q + 8, ... and the slices are added in order.
+// TREE: a trip's loads and the slices are added as trees instead, for RMSNorm's fp32 dw (16384 x 768 normal numbers: off by 1.7e-5 rms,
+// 2.2e-5 in order).
 // Bound by latency: FOLD_ROWS loads are in flight per thread, up to 296 rows come in four trips (all 40 at once 0.6 us more; norm backward and fold of
 // 3152 x 768 9.7 us with 10, 10.1 with 40, 11.0 in a plain loop).
 constexpr int FOLD_THREADS = 256, FOLD_ROWS = 10;
-template <bool BF>
+template <bool BF, bool TREE = false>
 __global__ void __launch_bounds__(FOLD_THREADS) fold_cols_k(void* __restrict__ dw, void* __restrict__ db, const float* __restrict__ partial, int nrows, int C, int W) {
   mlb_pdl_sync();
   __shared__ float red[8][32];
@@ -656,17 +657,27 @@ __global__ void __launch_bounds__(FOLD_THREADS) fold_cols_k(void* __restrict__ d
       float v[FOLD_ROWS];
 #pragma unroll
       for (int k = 0; k < FOLD_ROWS; k++) v[k] = r + 8 * k < nrows ? partial[(size_t)(r + 8 * k) * W + c] : 0.f;
+      if (TREE) {
 #pragma unroll
-      for (int w = 1; w < FOLD_ROWS; w *= 2)
+        for (int w = 1; w < FOLD_ROWS; w *= 2)
 #pragma unroll
-        for (int k = 0; k + w < FOLD_ROWS; k += 2 * w) v[k] += v[k + w];
-      s += v[0];
+          for (int k = 0; k + w < FOLD_ROWS; k += 2 * w) v[k] += v[k + w];
+        s += v[0];
+      } else {
+#pragma unroll
+        for (int k = 0; k < FOLD_ROWS; k++) s += v[k];
+      }
     }
   }
   red[sl][lane] = s;
   __syncthreads();
   if (sl != 0 || c >= W) return;
-  s = ((red[0][lane] + red[1][lane]) + (red[2][lane] + red[3][lane])) + ((red[4][lane] + red[5][lane]) + (red[6][lane] + red[7][lane]));
+  if (TREE) {
+    s = ((s + red[1][lane]) + (red[2][lane] + red[3][lane])) + ((red[4][lane] + red[5][lane]) + (red[6][lane] + red[7][lane]));
+  } else {
+#pragma unroll
+    for (int i = 1; i < 8; i++) s += red[i][lane];
+  }
   void* dst = c < C ? dw : db;
   if (dst == nullptr) return;
   const int i = c < C ? c : c - C;
@@ -1500,7 +1511,7 @@ static void norm_rows_launch(void* dx, void* dw, void* db, bool bf, const void* 
   mlb_launch(norm_bwd_rows_k<LN>, dim3(blocks), dim3(256 / gt * gt), ring, st, (bf16*)dx, (const bf16*)dy, (const bf16*)x, (const bf16*)w, mean, rstd,
              (const bf16*)add, rows, C, partial);
   if (bf) mlb_launch(fold_cols_k<true>, dim3((W + 31) / 32), dim3(FOLD_THREADS), 0, st, dw, db, (const float*)partial, blocks, C, W);
-  else mlb_launch(fold_cols_k<false>, dim3((W + 31) / 32), dim3(FOLD_THREADS), 0, st, dw, db, (const float*)partial, blocks, C, W);
+  else mlb_launch(fold_cols_k<false, !LN>, dim3((W + 31) / 32), dim3(FOLD_THREADS), 0, st, dw, db, (const float*)partial, blocks, C, W);
 }
 MLB_API int mlb_rmsnorm_bwd_cast(void* dx, void* dw, const void* dy, const void* x, const void* w, const float* rstd, const void* add, long rows, int C,
                                  float* partial, cudaStream_t st) {
