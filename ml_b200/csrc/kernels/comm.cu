@@ -10,7 +10,7 @@
 //      new bf16 parameters into every rank's parameter buffer (peer stores);
 //   3. exit barrier: the last CTA to finish signals every peer and waits for their signals, so when the kernel ends all
 //      peers have stopped reading this rank's gradients and this rank's parameters are complete.
-// The same kernel with world = 1 is a fused mean-scale + AdamW.  Reduce-scatter + sharded AdamW for ZeRO-style
+// With world = 1 this is a fused mean-scale + AdamW (fp32 gradients: ddp_single_kernel, without the barriers).  Reduce-scatter + sharded AdamW for ZeRO-style
 // sharding is the same kernel with `bcast` = 0 (parameters stay sharded).
 // Every wait on a peer flag is bounded (the caller passes the limit; the engine's default is 20 s, tests pass a fraction
 // of a second): on expiry the kernel records MLB_ERR_FLAG_TIMEOUT and returns.
@@ -151,6 +151,13 @@ __device__ __forceinline__ uint2 adamw4(const BucketArgs& a, long e, const float
   o.y = pack_bf16(p.z, p.w);
   return o;
 }
+__device__ __forceinline__ bf16 adamw1(const BucketArgs& a, long e, float g, float lr, float inv_bc1, float inv_bc2, float scale) {
+  g *= scale;
+  float mj = a.b1 * a.m[e] + (1.f - a.b1) * g, vj = a.b2 * a.v[e] + (1.f - a.b2) * g * g, pj = a.master[e];
+  pj -= lr * (mj * inv_bc1 / (sqrtf(vj * inv_bc2) + a.eps) + a.wd * pj);
+  a.m[e] = mj; a.v[e] = vj; a.master[e] = pj;
+  return __float2bfloat16(pj);
+}
 __device__ __forceinline__ void store_params4(const BucketArgs& a, long e, uint2 o, int W) {
   if (a.bcast && a.params_mc) {
     asm volatile("multimem.st.relaxed.sys.global.v2.bf16x2 [%0], {%1, %2};" ::"l"(a.params_mc + e), "r"(o.x), "r"(o.y) : "memory");
@@ -235,12 +242,9 @@ __device__ __forceinline__ void ddp_bucket_body(const BucketArgs& a) {
       for (long e = lo + nvec * 4; e < hi; e++) {
         float g = 0.f;
         for (int w = 0; w < W; w++) g += *((volatile float*)(a.grads[w] + e));
-        g *= scale;
-        float mj = a.b1 * a.m[e] + (1.f - a.b1) * g, vj = a.b2 * a.v[e] + (1.f - a.b2) * g * g, pj = a.master[e];
-        pj -= lr * (mj * inv_bc1 / (sqrtf(vj * inv_bc2) + a.eps) + a.wd * pj);
-        a.m[e] = mj; a.v[e] = vj; a.master[e] = pj;
+        const bf16 p = adamw1(a, e, g, lr, inv_bc1, inv_bc2, scale);
         for (int w = 0; w < W; w++)
-          if (a.bcast || w == a.rank) a.params[w][e] = __float2bfloat16(pj);
+          if (a.bcast || w == a.rank) a.params[w][e] = p;
       }
     }
   }
@@ -264,6 +268,24 @@ template <int GM>
 __global__ void __maxnreg__(32) ddp_bucket_lean_kernel(const BucketArgs a) { ddp_bucket_body<GM>(a); }
 template <int GM>
 __global__ void __launch_bounds__(256, 4) ddp_bucket_kernel(const BucketArgs a) { ddp_bucket_body<GM>(a); }
+
+// One rank, fp32 gradients: nobody to wait for or to tell, so a thread takes one vector and the grid is as long as the bucket.  Bound by
+// memory, 30 bytes a parameter: threads that start in the order of their addresses keep the four reads and four writes within few
+// DRAM pages, which a resident grid that strides over the bucket loses, its CTAs drifting apart.  163 M parameters:
+// 918 us with a resident grid, 714 so (6.8 TB/s); 7 M: 56.5 and 36.4, 1 M: 19.8 and 15.3.
+__global__ void __launch_bounds__(256) ddp_single_kernel(const BucketArgs a) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) a.epoch_ctr[a.bucket]++;
+  float lr = a.lr, inv_bc1 = a.inv_bc1, inv_bc2 = a.inv_bc2, scale = a.scale;
+  if (a.dev_hyper) { lr = a.dev_hyper[0]; inv_bc1 = a.dev_hyper[1]; inv_bc2 = a.dev_hyper[2]; scale = a.dev_hyper[3]; }
+  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < a.n / 4) {
+    const long e = a.off + i * 4;
+    const float4 g = *reinterpret_cast<const float4*>(a.grads[0] + e);
+    *reinterpret_cast<uint2*>(a.params[0] + e) = adamw4(a, e, &g.x, lr, inv_bc1, inv_bc2, scale);
+  } else if (i == a.n / 4) {
+    for (long e = a.off + i * 4; e < a.off + a.n; e++) a.params[0][e] = adamw1(a, e, a.grads[0][e], lr, inv_bc1, inv_bc2, scale);
+  }
+}
 
 // All-gather by peer loads: dst[w*chunk_bytes ...] = shard of rank w, for every w; 16-byte vectors, system-scope loads.
 // No barrier is needed here: the producer of the shards (the reduce-scatter + AdamW kernel of the previous step) ends
@@ -340,7 +362,7 @@ MLB_API int mlb_ddp_bucket_max_ctas(int gmode, int lean) {
 // One bucket of the fused data-parallel gradient step.  Pointer arrays live in device memory (world entries each).
 //   gmode        GM_* above.  The multicast modes need the matching multicast address; the bf16 modes need the staging
 //                pointer table (and `done_counter` 2 * max_buckets ints long), off and n multiples of 8.
-//   ctas         grid size (256 threads each; at most mlb_ddp_bucket_max_ctas); lean != 0 selects the 32-register form, of 128 threads
+//   ctas         grid size (256 threads each; at most mlb_ddp_bucket_max_ctas; one rank with fp32 gradients has a grid of the bucket's length); lean != 0 selects the 32-register form, of 128 threads
 MLB_API int mlb_ddp_bucket2(const void* grads_ptrs, const void* params_ptrs, const void* flags_ptrs, float* master, float* m, float* v,
                             int* done_counter, int* epoch_ctr, long off, long n, int rank, int world, int bucket, int max_buckets,
                             int bcast, float lr, float b1, float b2, float eps, float wd, float bc1, float bc2, float scale,
@@ -366,6 +388,10 @@ MLB_API int mlb_ddp_bucket2(const void* grads_ptrs, const void* params_ptrs, con
   const int most = mlb_ddp_bucket_max_ctas(gmode, lean);
   if (most > 0 && ctas > most) ctas = most;
   const int grid = (int)(want < ctas ? want : ctas);
+  if (world == 1 && gmode == GM_F32_PEER && !lean) {
+    ddp_single_kernel<<<n > 0 ? (unsigned)(n / 1024 + 1) : 1u, 256, 0, st>>>(a);      // (the last block: the 0 ... 3 elements of no vector)
+    return (int)cudaGetLastError();
+  }
   // An SM's split between L1 and shared memory is fixed while CTAs are resident on it.  The tensor-core kernels need the
   // largest shared-memory split; a bucket CTA that got onto an idle SM first with the default (L1-heavy) split would keep
   // their CTAs (and with them whole clusters of a persistent grid) waiting until it leaves.  So these kernels ask for

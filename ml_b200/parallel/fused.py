@@ -49,9 +49,9 @@ class FusedGradEngine:
     def __init__(self, model, world: int, rank: int, group=None, ctas: int = 0, bcast: bool = True, spin_limit_s: float = 20.0,
                  overlap=None, buckets=None, bf16_reduce: bool = False):
         """ctas: CTAs (128 threads) of an overlapped bucket kernel (0 = ENTROPY_FUSED_CTAS or 148); a launch that has the
-        machine to itself uses four per SM, of 256 threads (with two, 32 KB in flight per SM do not cover the memory's latency: one
-        rank, 163 M parameters, 1120 us; with four 950 us, 5.2 TB/s; with eight 1040 us); in the bf16 modes, whose whole grid has to
-        be resident, the library allows two.  overlap: bucket kernels behind backward on a side stream (default: with more than
+        machine to itself uses four per SM, of 256 threads (with two, 32 KB in flight per SM do not cover the memory's latency: 163 M
+        parameters on one rank 1120 us; with four 950 us; with eight 1040 us; one rank alone has a kernel without a resident grid, 714 us);
+        in the bf16 modes, whose whole grid has to be resident, the library allows two.  overlap: bucket kernels behind backward on a side stream (default: with more than
         two ranks; ENTROPY_FUSED_OVERLAP=0 / 1 decides otherwise).  bf16_reduce: reduce bf16 staging copies instead of the fp32 gradients."""
         self.model, self.world, self.rank, self.group = model, world, rank, group
         self.bcast, self.spin_limit_s = bcast, spin_limit_s

@@ -549,3 +549,34 @@ def test_bf16_bucket_grid_is_resident(lean):
     e -= 1e-3 * (gb / (gb.abs() + 1e-8) + 0.1 * e)
     assert (master - e).abs().max() < 1e-5      # (fp32 arithmetic on values of order 1 and a step of 1e-3)
     assert torch.equal(p, master.bfloat16())
+
+
+@pytest.mark.parametrize("off,n", [(0, 1), (0, 3), (4, 4), (8, 1023), (0, 1024), (4, 1025), (12, 4102), (0, 300007)])
+@pytest.mark.parametrize("dev_hyper", [False, True])
+def test_one_rank_update_is_the_bucket_kernels(off, n, dev_hyper):
+    """One rank's update, a thread per vector, against the bucket kernel (its form for shared SMs): the same bits, nothing outside the bucket, the epoch counted."""
+    from ml_b200.ops import native
+    L, dev, N = native.lib(), torch.device("cuda:0"), 300032
+    torch.manual_seed(n)
+    g, master, m, v = torch.randn(N, device=dev), torch.randn(N, device=dev), 0.1 * torch.randn(N, device=dev), torch.rand(N, device=dev)
+    hyper = torch.tensor([2e-3, 1.5, 1.25, 0.5], device=dev) if dev_hyper else None
+    fn = L.mlb_ddp_bucket2
+    fn.argtypes = [C.c_void_p] * 8 + [C.c_long, C.c_long] + [C.c_int] * 5 + [C.c_float] * 8 + [C.c_void_p, C.c_int, C.c_double] + \
+        [C.c_void_p] * 4 + [C.c_int, C.c_int, C.c_void_p]
+    runs = []
+    for lean in (1, 0):
+        a, b, c, p = master.clone(), m.clone(), v.clone(), master.bfloat16()
+        flags, done, epoch = (torch.zeros(k, dtype=torch.int32, device=dev) for k in (2 * L.mlb_comm_max_world(), 2, 1))
+        tab = torch.tensor([t.data_ptr() for t in (g, p, flags)], dtype=torch.int64, device=dev)
+        for _ in range(2):
+            rc = fn(tab.data_ptr(), tab.data_ptr() + 8, tab.data_ptr() + 16, a.data_ptr(), b.data_ptr(), c.data_ptr(), done.data_ptr(), epoch.data_ptr(),
+                    off, n, 0, 1, 0, 1, 1, 1e-3, 0.9, 0.95, 1e-8, 0.1, 0.1, 0.05, 1.0, None if hyper is None else hyper.data_ptr(), 592, 1.0,
+                    None, None, None, None, 0, lean, torch.cuda.current_stream().cuda_stream)
+            assert rc == 0
+        torch.cuda.synchronize()
+        assert native.get_error() == 0 and int(epoch) == 2
+        runs.append((a, b, c, p))
+    for x, y, before in zip(runs[0], runs[1], (master, m, v, master.bfloat16())):
+        assert torch.equal(x, y)
+        assert torch.equal(y[:off], before[:off]) and torch.equal(y[off + n:], before[off + n:])
+    assert not torch.equal(runs[1][1][off:off + n], m[off:off + n])      # (the step of one parameter can be less than its last bit in bf16)
