@@ -1880,45 +1880,46 @@ __global__ void __maxnreg__(120) attn_bwd_fused_tc_kernel(const __grid_constant_
 }
 
 // dQ partial tiles -> bf16 Q slice of dqkv[rows, 3C]: sum over the key tiles kt <= i of query tile i (fp32, fixed
-// order), times `scale`, optional RoPE backward.  One thread per (row, head, group of 16 rotation pairs); the partial
-// layout is [B][i(i+1)/2 + kt][128][C] bf16.
+// order), times `scale`, optional RoPE backward.  One thread per (row, head, group of 8 rotation pairs); the partial
+// layout is [B][i(i+1)/2 + kt][128][C] bf16.  Bound by the loads of the partial tiles (113 MB for 16 x 1024 x 12 heads, most of it still in
+// L2): 16-byte loads of neighbouring lanes follow one another (32 bytes a lane took half of each line at a time), two tiles in flight
+// (one, four, eight: 24.6, 25.0, 26.5 us), read once so that they leave L2 first (30.3 without), the tiles written last before the older ones.
+// 16 x 1024 x 12 heads 27.4 -> 22.8 us, 4 x 2048 x 12 39 -> 18.4, 32 x 256 x 12 13.8 -> 7.2.
 __global__ void __launch_bounds__(256) attn_dq_finish_k(bf16* __restrict__ dqkv, const bf16* __restrict__ part, long rows, int T, int H,
                                                         int hd, float scale, const float* __restrict__ cosT,
                                                         const float* __restrict__ sinT) {
   mlb_pdl_sync();
-  const int h2 = hd >> 1, gph = h2 >> 4, gpr = H * gph;   // groups of 16 pairs per head / per row
+  const int h2 = hd >> 1, gph = h2 >> 3, gpr = H * gph;   // groups of 8 pairs per head / per row
   // rows * gpr fits 31 bits (checked by the host): 32-bit index arithmetic
-  const unsigned idx = blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned idx = (gridDim.x - 1 - blockIdx.x) * blockDim.x + threadIdx.x;      // (the last rows first)
   if (idx >= (unsigned)rows * gpr) return;
   const unsigned r = idx / (unsigned)gpr;
   const int g = idx % (unsigned)gpr, h = g / gph, v = g % gph;
   const int t = r % (unsigned)T, C = H * hd;
   const long b = r / (unsigned)T;
   const int nq = (T + 127) / 128, npairs = nq * (nq + 1) / 2, i = t >> 7;
-  const bf16* base = part + ((b * npairs + (long)i * (i + 1) / 2) * 128 + (t & 127)) * C + h * hd + v * 16;
-  float x0[16], x1[16];
+  const bf16* base = part + ((b * npairs + (long)i * (i + 1) / 2) * 128 + (t & 127)) * C + h * hd + v * 8;
+  float x0[8], x1[8];
 #pragma unroll
-  for (int k = 0; k < 16; k++) { x0[k] = 0.f; x1[k] = 0.f; }
+  for (int k = 0; k < 8; k++) { x0[k] = 0.f; x1[k] = 0.f; }
 #pragma unroll 2
   for (int kt = 0; kt <= i; kt++) {
-    const uint4* p0 = reinterpret_cast<const uint4*>(base + (long)kt * 128 * C);
-    const uint4* p1 = reinterpret_cast<const uint4*>(base + (long)kt * 128 * C + h2);
-    const uint4 a0 = __ldcs(p0), a1 = __ldcs(p0 + 1), b0 = __ldcs(p1), b1 = __ldcs(p1 + 1);
-    const uint32_t wa[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-    const uint32_t wb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+    const uint4 a = __ldcs(reinterpret_cast<const uint4*>(base + (long)kt * 128 * C));
+    const uint4 c = __ldcs(reinterpret_cast<const uint4*>(base + (long)kt * 128 * C + h2));
+    const uint32_t wa[4] = {a.x, a.y, a.z, a.w}, wc[4] = {c.x, c.y, c.z, c.w};
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
+    for (int k = 0; k < 4; k++) {
       x0[2 * k] += __uint_as_float(wa[k] << 16); x0[2 * k + 1] += __uint_as_float(wa[k] & 0xffff0000u);
-      x1[2 * k] += __uint_as_float(wb[k] << 16); x1[2 * k + 1] += __uint_as_float(wb[k] & 0xffff0000u);
+      x1[2 * k] += __uint_as_float(wc[k] << 16); x1[2 * k + 1] += __uint_as_float(wc[k] & 0xffff0000u);
     }
   }
 #pragma unroll
-  for (int k = 0; k < 16; k++) { x0[k] *= scale; x1[k] *= scale; }
+  for (int k = 0; k < 8; k++) { x0[k] *= scale; x1[k] *= scale; }
   if (cosT) {
-    const float4* c4 = reinterpret_cast<const float4*>(cosT + (long)t * h2 + v * 16);
-    const float4* s4 = reinterpret_cast<const float4*>(sinT + (long)t * h2 + v * 16);
+    const float4* c4 = reinterpret_cast<const float4*>(cosT + (long)t * h2 + v * 8);
+    const float4* s4 = reinterpret_cast<const float4*>(sinT + (long)t * h2 + v * 8);
 #pragma unroll
-    for (int i4 = 0; i4 < 4; i4++) {
+    for (int i4 = 0; i4 < 2; i4++) {
       const float4 c = c4[i4], sn = s4[i4];
       const float cc[4] = {c.x, c.y, c.z, c.w}, ss[4] = {sn.x, sn.y, sn.z, sn.w};
 #pragma unroll
@@ -1929,17 +1930,9 @@ __global__ void __launch_bounds__(256) attn_dq_finish_k(bf16* __restrict__ dqkv,
       }
     }
   }
-  bf16* o0 = dqkv + (long)r * 3L * C + h * hd + v * 16;
-#pragma unroll
-  for (int i2 = 0; i2 < 2; i2++) {
-    uint4 w0, w1;
-    w0.x = pack_bf16(x0[8 * i2], x0[8 * i2 + 1]); w0.y = pack_bf16(x0[8 * i2 + 2], x0[8 * i2 + 3]);
-    w0.z = pack_bf16(x0[8 * i2 + 4], x0[8 * i2 + 5]); w0.w = pack_bf16(x0[8 * i2 + 6], x0[8 * i2 + 7]);
-    w1.x = pack_bf16(x1[8 * i2], x1[8 * i2 + 1]); w1.y = pack_bf16(x1[8 * i2 + 2], x1[8 * i2 + 3]);
-    w1.z = pack_bf16(x1[8 * i2 + 4], x1[8 * i2 + 5]); w1.w = pack_bf16(x1[8 * i2 + 6], x1[8 * i2 + 7]);
-    *reinterpret_cast<uint4*>(o0 + 8 * i2) = w0;
-    *reinterpret_cast<uint4*>(o0 + h2 + 8 * i2) = w1;
-  }
+  bf16* o0 = dqkv + (long)r * 3L * C + h * hd + v * 8;
+  *reinterpret_cast<uint4*>(o0) = make_uint4(pack_bf16(x0[0], x0[1]), pack_bf16(x0[2], x0[3]), pack_bf16(x0[4], x0[5]), pack_bf16(x0[6], x0[7]));
+  *reinterpret_cast<uint4*>(o0 + h2) = make_uint4(pack_bf16(x1[0], x1[1]), pack_bf16(x1[2], x1[3]), pack_bf16(x1[4], x1[5]), pack_bf16(x1[6], x1[7]));
 }
 
 // ================================================================== backward: dQ (one CTA per 128-query tile)
@@ -2446,7 +2439,7 @@ static int attn_bwd_impl(void* dqkv, const void* dout, const void* qkv, const vo
     if (!tq || !td) return -2;
     AttnArgs a{B, T, H, hd, scale, (bf16*)dqkv, const_cast<float*>(lse), delta, cosT, sinT, (bf16*)dq_part, 0, g_timeline};
     dim3 grid((T + 127) / 128, H, B);
-    if (hd == 64 && dq_part != nullptr && ((uintptr_t)dq_part % 16 == 0) && (long)B * T * H * (hd / 32) < (1L << 31)) {
+    if (hd == 64 && dq_part != nullptr && ((uintptr_t)dq_part % 16 == 0) && (long)B * T * H * (hd / 16) < (1L << 31)) {
       // single fused kernel + dQ finish; the partial buffer is [B * nq(nq+1)/2 * 128 rows, C] bf16
       const long nqh = (T + 127) / 128;
       const CUtensorMap* tpart = mlb_tmap_cached(dq_part, (uint64_t)B * (nqh * (nqh + 1) / 2) * 128, C, C, 32, 64, 2);
@@ -2473,7 +2466,7 @@ static int attn_bwd_impl(void* dqkv, const void* dout, const void* qkv, const vo
       else if (a.timeline) MLB_BWDF(false, true)
       else MLB_BWDF(false)
 #undef MLB_BWDF
-      const long groups = (long)B * T * H * (hd / 32);
+      const long groups = (long)B * T * H * (hd / 16);
       mlb_launch(attn_dq_finish_k, dim3((unsigned)((groups + 255) / 256)), dim3(256), 0, st, (bf16*)dqkv, (const bf16*)dq_part, (long)B * T, T, H, hd, scale, cosT, sinT);
       cudaError_t e = cudaGetLastError();
       if (e != cudaSuccess) return (int)e + 1000;
