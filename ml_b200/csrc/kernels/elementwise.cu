@@ -641,22 +641,24 @@ __global__ void __launch_bounds__(256) colsum_k(float* __restrict__ partial, con
 }
 // The partial rows added up in a fixed order: columns [0, C) to dw, [C, W) to db (either may be null).  bf16: rounded and stored;
 // fp32: added to what is there.  A block takes 32 columns, 8 row slices: slice q adds rows q, q + 8, ... and the slices are added in order.
-// TREE: a trip's loads and the slices are added as trees instead, for RMSNorm's fp32 dw (16384 x 768 normal numbers: off by 1.7e-5 rms,
-// 2.2e-5 in order).
+// TREE: for RMSNorm's fp32 dw, where no order is promised: 32 slices, so that 296 rows come in one trip (norm backward and fold of 16384 x 768
+// in L2 20.8 -> 19.2 us, 4096 x 768 10.7 -> 9.7), a trip's loads and the slices added as trees (normal numbers: off by 1.7e-5 rms, 2.2e-5 in
+// the order above).
 // Bound by latency: FOLD_ROWS loads are in flight per thread, up to 296 rows come in four trips (all 40 at once 0.6 us more; norm backward and fold of
 // 3152 x 768 9.7 us with 10, 10.1 with 40, 11.0 in a plain loop).
-constexpr int FOLD_THREADS = 256, FOLD_ROWS = 10;
+constexpr int FOLD_THREADS = 256, FOLD_TREE_THREADS = 1024, FOLD_ROWS = 10;
 template <bool BF, bool TREE = false>
-__global__ void __launch_bounds__(FOLD_THREADS) fold_cols_k(void* __restrict__ dw, void* __restrict__ db, const float* __restrict__ partial, int nrows, int C, int W) {
+__global__ void __launch_bounds__(TREE ? FOLD_TREE_THREADS : FOLD_THREADS) fold_cols_k(void* __restrict__ dw, void* __restrict__ db, const float* __restrict__ partial, int nrows, int C, int W) {
   mlb_pdl_sync();
-  __shared__ float red[8][32];
+  constexpr int SL = (TREE ? FOLD_TREE_THREADS : FOLD_THREADS) / 32;
+  __shared__ float red[SL][32];
   const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
   float s = 0.f;
   if (c < W) {
-    for (int r = sl; r < nrows; r += 8 * FOLD_ROWS) {
+    for (int r = sl; r < nrows; r += SL * FOLD_ROWS) {
       float v[FOLD_ROWS];
 #pragma unroll
-      for (int k = 0; k < FOLD_ROWS; k++) v[k] = r + 8 * k < nrows ? partial[(size_t)(r + 8 * k) * W + c] : 0.f;
+      for (int k = 0; k < FOLD_ROWS; k++) v[k] = r + SL * k < nrows ? partial[(size_t)(r + SL * k) * W + c] : 0.f;
       if (TREE) {
 #pragma unroll
         for (int w = 1; w < FOLD_ROWS; w *= 2)
@@ -673,10 +675,17 @@ __global__ void __launch_bounds__(FOLD_THREADS) fold_cols_k(void* __restrict__ d
   __syncthreads();
   if (sl != 0 || c >= W) return;
   if (TREE) {
-    s = ((s + red[1][lane]) + (red[2][lane] + red[3][lane])) + ((red[4][lane] + red[5][lane]) + (red[6][lane] + red[7][lane]));
+    float v[SL];
+#pragma unroll
+    for (int k = 0; k < SL; k++) v[k] = red[k][lane];
+#pragma unroll
+    for (int w = 1; w < SL; w *= 2)
+#pragma unroll
+      for (int k = 0; k + w < SL; k += 2 * w) v[k] += v[k + w];
+    s = v[0];
   } else {
 #pragma unroll
-    for (int i = 1; i < 8; i++) s += red[i][lane];
+    for (int i = 1; i < SL; i++) s += red[i][lane];
   }
   void* dst = c < C ? dw : db;
   if (dst == nullptr) return;
@@ -1511,7 +1520,7 @@ static void norm_rows_launch(void* dx, void* dw, void* db, bool bf, const void* 
   mlb_launch(norm_bwd_rows_k<LN>, dim3(blocks), dim3(256 / gt * gt), ring, st, (bf16*)dx, (const bf16*)dy, (const bf16*)x, (const bf16*)w, mean, rstd,
              (const bf16*)add, rows, C, partial);
   if (bf) mlb_launch(fold_cols_k<true>, dim3((W + 31) / 32), dim3(FOLD_THREADS), 0, st, dw, db, (const float*)partial, blocks, C, W);
-  else mlb_launch(fold_cols_k<false, !LN>, dim3((W + 31) / 32), dim3(FOLD_THREADS), 0, st, dw, db, (const float*)partial, blocks, C, W);
+  else mlb_launch(fold_cols_k<false, !LN>, dim3((W + 31) / 32), dim3(LN ? FOLD_THREADS : FOLD_TREE_THREADS), 0, st, dw, db, (const float*)partial, blocks, C, W);
 }
 MLB_API int mlb_rmsnorm_bwd_cast(void* dx, void* dw, const void* dy, const void* x, const void* w, const float* rstd, const void* add, long rows, int C,
                                  float* partial, cudaStream_t st) {
@@ -1553,8 +1562,8 @@ MLB_API int mlb_rmsnorm_bwd(void* dx, float* dw, const void* dy, const void* x, 
   if (sh > 48 * 1024) return -3;
   // Whole multiples of 256 columns: a block's threads share a row instead of a warp having one, and the partial rows are folded by a
   // kernel of their own, which overlaps this one's end.  One warp a row, with the fold by the blocks that finish last, against this, inputs
-  // not in L2: 16384 x 768 31.7 -> 29.7 us, 4096 x 768 21 -> 17.4, 64 x 768 13.3 -> 11.3, 65536 x 256 46 -> 35.8, 4096 x 512 17.4 = 17.4,
-  // 16384 x 512 25.6 = 25.6 (in L2 14.1 -> 16.1, the one size that is slower).
+  // not in L2: 16384 x 768 31.7 -> 27.6 us, 4096 x 768 21 -> 15.4, 64 x 768 13.3 -> 11.3, 65536 x 256 46 -> 33.8, 4096 x 512 17.4 -> 15.4,
+  // 16384 x 512 25.6 -> 23.6 (in L2 14.1 -> 14.8, the one size that is slower).
   if (norm_rows_ok(dx, dy, x, w, add, rows, C)) {
     norm_rows_launch<false>(dx, dw, nullptr, false, dy, x, w, nullptr, rstd, add, rows, C, partial, st);
     LAUNCH_RET;
