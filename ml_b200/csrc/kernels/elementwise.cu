@@ -47,37 +47,54 @@ __device__ __forceinline__ void store8_e4m3(uint8_t* p, const float (&f)[8], flo
 // A token id outside [0, V) (a token file made with a larger vocabulary, a damaged file) would index past the table:
 // such a row gets zeros / no gradient, and the error word says so (MLB_ERR_BOUNDS, detail 0xE1 forward, 0xE2 backward,
 // 0xCE for a cross-entropy target), so the step that read it fails on the host instead of corrupting memory.
-__global__ void embed_fwd_k(bf16* __restrict__ out, const bf16* __restrict__ wte, const int* __restrict__ ids, int C, int V) {
+// A warp per row, four to a block: with a block per row the rate at which blocks start was the bound (16384 of them take 20 us, whatever
+// they do), then the two dependent trips of a row, its id and the table.  16384 x 768, 50304 rows in the table: 22.6 -> 16.4 us
+// (in L2 20.5 -> 8.2), 2048 x 128 2.9 -> 1.6.
+__global__ void __launch_bounds__(128) embed_fwd_k(bf16* __restrict__ out, const bf16* __restrict__ wte, const int* __restrict__ ids, long rows, int C, int V) {
   mlb_pdl_sync();
-  const long row = blockIdx.x;
+  const int lane = threadIdx.x & 31;
+  const long row = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (row >= rows) return;
   const int id = ids[row];
   bf16* dst = out + row * C;
   if ((unsigned)id >= (unsigned)V) {
-    if (threadIdx.x == 0) mlb_set_error(MLB_ERR_BOUNDS, 0xE1);
-    for (int i = threadIdx.x; i < C; i += blockDim.x) dst[i] = __float2bfloat16(0.f);
+    if (lane == 0) mlb_set_error(MLB_ERR_BOUNDS, 0xE1);
+    for (int i = lane; i < C; i += 32) dst[i] = __float2bfloat16(0.f);
     return;
   }
   const bf16* src = wte + (long)id * C;
   if ((C & 7) == 0) {
-    for (int i = threadIdx.x * 8; i < C; i += blockDim.x * 8)
-      *reinterpret_cast<uint4*>(dst + i) = *reinterpret_cast<const uint4*>(src + i);
+#pragma unroll 4
+    for (int i = lane * 8; i < C; i += 256) *reinterpret_cast<uint4*>(dst + i) = *reinterpret_cast<const uint4*>(src + i);
   } else {
-    for (int i = threadIdx.x; i < C; i += blockDim.x) dst[i] = src[i];
+    for (int i = lane; i < C; i += 32) dst[i] = src[i];
   }
 }
-__global__ void embed_bwd_k(float* __restrict__ dwte, const bf16* __restrict__ dout, const int* __restrict__ ids, int C,
-                            int V, int T, int n_pre) {
+// The same; four neighbouring elements an atomic addition where the rows allow it.  16384 x 768, 50304 rows: 41 -> 26.7 us (in L2 20.6 -> 12.3),
+// 1003 rows 2.6 -> 2.8.
+__global__ void __launch_bounds__(128) embed_bwd_k(float* __restrict__ dwte, const bf16* __restrict__ dout, const int* __restrict__ ids, long rows, int C,
+                                                   int V, int T, int n_pre) {
   mlb_pdl_sync();
-  const long row = blockIdx.x;
-  if ((int)(row % T) < n_pre) return;
+  const int lane = threadIdx.x & 31;
+  const long row = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (row >= rows || (int)(row % T) < n_pre) return;
   const int id = ids[row];
   if ((unsigned)id >= (unsigned)V) {
-    if (threadIdx.x == 0) mlb_set_error(MLB_ERR_BOUNDS, 0xE2);
+    if (lane == 0) mlb_set_error(MLB_ERR_BOUNDS, 0xE2);
     return;
   }
   float* dst = dwte + (long)id * C;
   const bf16* src = dout + row * C;
-  for (int i = threadIdx.x; i < C; i += blockDim.x) atomicAdd(dst + i, __bfloat162float(src[i]));
+  if ((C & 3) == 0 && ((reinterpret_cast<uintptr_t>(dwte) & 15) | (reinterpret_cast<uintptr_t>(dout) & 7)) == 0) {
+#pragma unroll 4
+    for (int i = lane * 4; i < C; i += 128) {
+      const uint2 u = *reinterpret_cast<const uint2*>(src + i);
+      asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + i), "f"(__uint_as_float(u.x << 16)),
+                   "f"(__uint_as_float(u.x & 0xffff0000u)), "f"(__uint_as_float(u.y << 16)), "f"(__uint_as_float(u.y & 0xffff0000u)) : "memory");
+    }
+  } else {
+    for (int i = lane; i < C; i += 32) atomicAdd(dst + i, __bfloat162float(src[i]));
+  }
 }
 __global__ void set_prefix_k(bf16* __restrict__ x, const bf16* __restrict__ prefix, int B, int T, int n_pre, int C) {
   mlb_pdl_sync();
@@ -1385,11 +1402,11 @@ static int g_ce_smem = 0;     // tuning hook: 0 = always the two-pass cross-entr
 MLB_API void mlb_ce_mode(int smem_row) { g_ce_smem = smem_row; }
 
 MLB_API int mlb_embed_fwd(void* out, const void* wte, const int* ids, long BT, int C, int V, cudaStream_t st) {
-  mlb_launch(embed_fwd_k, dim3((unsigned)BT), dim3(96), 0, st, (bf16*)out, (const bf16*)wte, ids, C, V);
+  mlb_launch(embed_fwd_k, dim3((unsigned)((BT + 3) / 4)), dim3(128), 0, st, (bf16*)out, (const bf16*)wte, ids, (long)BT, C, V);
   LAUNCH_RET;
 }
 MLB_API int mlb_embed_bwd(float* dwte, const void* dout, const int* ids, long BT, int C, int V, int T, int n_pre, cudaStream_t st) {
-  mlb_launch(embed_bwd_k, dim3((unsigned)BT), dim3(256), 0, st, dwte, (const bf16*)dout, ids, C, V, T, n_pre);
+  mlb_launch(embed_bwd_k, dim3((unsigned)((BT + 3) / 4)), dim3(128), 0, st, dwte, (const bf16*)dout, ids, (long)BT, C, V, T, n_pre);
   LAUNCH_RET;
 }
 MLB_API int mlb_set_prefix(void* x, const void* prefix, int B, int T, int n_pre, int C, cudaStream_t st) {

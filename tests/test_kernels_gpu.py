@@ -564,6 +564,24 @@ def test_embedding_and_prefix():
     assert torch.equal(g.view(B, n_pre, C), d.view(B, T, C)[:, :n_pre])
 
 
+@pytest.mark.parametrize("BT,C,shift", [(1, 8, 0), (5, 768, 0), (4098, 132, 0), (301, 102, 0), (9, 20, 0), (66, 128, 2), (7, 1, 0)])
+def test_embedding_rows_and_widths(BT, C, shift):
+    """Rows past the last whole block, widths of whole vectors or not, gradients from a place where vectors may not be loaded, prefix positions left out."""
+    torch.manual_seed(BT + C)
+    V, T, n_pre = 37, BT if BT % 3 else BT // 3, 0 if BT < 5 else 2
+    wte, ids = rnd(V, C), torch.randint(0, V, (BT,), device=dev(), dtype=torch.int32)
+    out = torch.full((BT + 1, C), 7.0, device=dev(), dtype=torch.bfloat16)
+    nat().embed_fwd(out[:BT], wte, ids)
+    assert torch.equal(out[:BT], wte[ids.long()]) and (out[BT] == 7).all()
+    d, dw = rnd(BT * C + shift).view(-1)[shift:].view(BT, C), torch.ones(V, C, device=dev())
+    nat().embed_bwd(dw, d, ids, T, n_pre)
+    live = torch.arange(BT, device=dev()) % T >= n_pre
+    e = torch.ones(V, C, device=dev(), dtype=torch.float64).index_add_(0, ids[live].long(), d[live].double())
+    # at most BT additions in any order, each rounding a partial sum of at most 1 + sum |d|
+    bound = BT * 2.0 ** -24 * torch.ones(V, C, device=dev(), dtype=torch.float64).index_add_(0, ids[live].long(), d[live].double().abs())
+    assert ((dw - e).abs() <= bound).all()
+
+
 def test_vision_helpers_and_casts():
     torch.manual_seed(14)
     B, g = 2, 3
