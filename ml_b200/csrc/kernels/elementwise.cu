@@ -657,40 +657,51 @@ __global__ void __launch_bounds__(256) colsum_k(float* __restrict__ partial, con
   partial[(size_t)blockIdx.y * N + col] = s;
 }
 // The partial rows added up in a fixed order: columns [0, C) to dw, [C, W) to db (either may be null).  bf16: rounded and stored;
-// fp32: added to what is there.  A block takes 32 columns, 8 row slices: slice q adds rows q, q + 8, ... and the slices are added in order.
-// TREE: for RMSNorm's fp32 dw, where no order is promised: 32 slices, so that 296 rows come in one trip (norm backward and fold of 16384 x 768
-// in L2 20.8 -> 19.2 us, 4096 x 768 10.7 -> 9.7), a trip's loads and the slices added as trees (normal numbers: off by 1.7e-5 rms, 2.2e-5 in
-// the order above).
-// Bound by latency: FOLD_ROWS loads are in flight per thread, up to 296 rows come in four trips (all 40 at once 0.6 us more; norm backward and fold of
-// 3152 x 768 9.7 us with 10, 10.1 with 40, 11.0 in a plain loop).
-constexpr int FOLD_THREADS = 256, FOLD_TREE_THREADS = 1024, FOLD_ROWS = 10;
-template <bool BF, bool TREE = false>
-__global__ void __launch_bounds__(TREE ? FOLD_TREE_THREADS : FOLD_THREADS) fold_cols_k(void* __restrict__ dw, void* __restrict__ db, const float* __restrict__ partial, int nrows, int C, int W) {
+// fp32: added to what is there.  A block takes 32 columns; slice q of eight adds rows q, q + 8, ... and the slices are added in order.
+// Bound by latency, so the rows come in one trip of FOLD_ROWS loads a thread: up to 80 rows to eight warps, each of which adds what it loads
+// (with 32: column sums of 1003 x 4096 4.5 -> 4.9 us); more rows, 296 at most here, to 32 warps, from which they wait in shared memory for the
+// eight that add them (with 8, four trips; norm backward and fold of 3152 x 768 9.3 -> 8.5 us, LayerNorm 10.4 -> 9.3, 16384 x 768 20.2 -> 19.0).
+// TREE: for RMSNorm's fp32 dw, where no order is promised: as many slices as warps, a trip's loads and the slices added as trees
+// (16384 x 768 normal numbers: off by 1.7e-5 rms, 2.2e-5 in the order above).
+constexpr int FOLD_ROWS = 10;
+template <bool BF, bool TREE, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) fold_cols_k(void* __restrict__ dw, void* __restrict__ db, const float* __restrict__ partial, int nrows, int C, int W) {
   mlb_pdl_sync();
-  constexpr int SL = (TREE ? FOLD_TREE_THREADS : FOLD_THREADS) / 32;
-  __shared__ float red[SL][32];
-  const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
+  constexpr int TRIP = WARPS * FOLD_ROWS, SL = TREE ? WARPS : 8;
+  __shared__ float rowbuf[SL == WARPS ? 1 : TRIP][32], red[SL][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
   float s = 0.f;
-  if (c < W) {
-    for (int r = sl; r < nrows; r += SL * FOLD_ROWS) {
-      float v[FOLD_ROWS];
+  for (int r0 = 0; r0 < nrows; r0 += TRIP) {
+    float v[FOLD_ROWS];
 #pragma unroll
-      for (int k = 0; k < FOLD_ROWS; k++) v[k] = r + SL * k < nrows ? partial[(size_t)(r + SL * k) * W + c] : 0.f;
-      if (TREE) {
+    for (int k = 0; k < FOLD_ROWS; k++) {
+      const int r = r0 + warp + WARPS * k;
+      v[k] = r < nrows && c < W ? partial[(size_t)r * W + c] : 0.f;
+    }
+    if (TREE) {
 #pragma unroll
-        for (int w = 1; w < FOLD_ROWS; w *= 2)
+      for (int w = 1; w < FOLD_ROWS; w *= 2)
 #pragma unroll
-          for (int k = 0; k + w < FOLD_ROWS; k += 2 * w) v[k] += v[k + w];
-        s += v[0];
-      } else {
+        for (int k = 0; k + w < FOLD_ROWS; k += 2 * w) v[k] += v[k + w];
+      s += v[0];
+    } else if (SL == WARPS) {
 #pragma unroll
-        for (int k = 0; k < FOLD_ROWS; k++) s += v[k];
+      for (int k = 0; k < FOLD_ROWS; k++) s += v[k];
+    } else {
+      if (r0 > 0) __syncthreads();
+#pragma unroll
+      for (int k = 0; k < FOLD_ROWS; k++) rowbuf[warp + WARPS * k][lane] = v[k];
+      __syncthreads();
+      if (warp < SL) {
+        const int n = min(TRIP, nrows - r0);
+#pragma unroll 8
+        for (int r = warp; r < n; r += SL) s += rowbuf[r][lane];
       }
     }
   }
-  red[sl][lane] = s;
+  if (warp < SL) red[warp][lane] = s;
   __syncthreads();
-  if (sl != 0 || c >= W) return;
+  if (warp != 0 || c >= W) return;
   if (TREE) {
     float v[SL];
 #pragma unroll
@@ -709,6 +720,11 @@ __global__ void __launch_bounds__(TREE ? FOLD_TREE_THREADS : FOLD_THREADS) fold_
   const int i = c < C ? c : c - C;
   if (BF) ((bf16*)dst)[i] = __float2bfloat16(s);
   else ((float*)dst)[i] += s;
+}
+template <bool BF, bool TREE = false>
+static void fold_launch(void* dw, void* db, const float* partial, int nrows, int C, int W, cudaStream_t st) {
+  if (nrows > 8 * FOLD_ROWS) mlb_launch(fold_cols_k<BF, TREE, 32>, dim3((W + 31) / 32), dim3(1024), 0, st, dw, db, partial, nrows, C, W);
+  else mlb_launch(fold_cols_k<BF, TREE, 8>, dim3((W + 31) / 32), dim3(256), 0, st, dw, db, partial, nrows, C, W);
 }
 
 // ------------------------------------------------------------------ RoPE (in place on the Q and K slices of qkv[B*T, 3C])
@@ -1536,8 +1552,8 @@ static void norm_rows_launch(void* dx, void* dw, void* db, bool bf, const void* 
   if (mlb_allow_smem(norm_bwd_rows_k<LN>, ring, allowed) != cudaSuccess) return;      // (the caller asks for the error)
   mlb_launch(norm_bwd_rows_k<LN>, dim3(blocks), dim3(256 / gt * gt), ring, st, (bf16*)dx, (const bf16*)dy, (const bf16*)x, (const bf16*)w, mean, rstd,
              (const bf16*)add, rows, C, partial);
-  if (bf) mlb_launch(fold_cols_k<true>, dim3((W + 31) / 32), dim3(FOLD_THREADS), 0, st, dw, db, (const float*)partial, blocks, C, W);
-  else mlb_launch(fold_cols_k<false, !LN>, dim3((W + 31) / 32), dim3(LN ? FOLD_THREADS : FOLD_TREE_THREADS), 0, st, dw, db, (const float*)partial, blocks, C, W);
+  if (bf) fold_launch<true>(dw, db, partial, blocks, C, W, st);
+  else fold_launch<false, !LN>(dw, db, partial, blocks, C, W, st);
 }
 MLB_API int mlb_rmsnorm_bwd_cast(void* dx, void* dw, const void* dy, const void* x, const void* w, const float* rstd, const void* add, long rows, int C,
                                  float* partial, cudaStream_t st) {
@@ -1561,7 +1577,7 @@ MLB_API int mlb_colsum(void* out, const void* x, long M, int N, float* partial, 
   if (M <= 0 || N <= 0 || N % 8 != 0 || ((uintptr_t)x & 15)) return -7;
   const int S = mlb_colsum_splits(M, N);
   mlb_launch(colsum_k, dim3((N + 255) / 256, S), dim3(256), 0, st, partial, (const bf16*)x, M, N);
-  mlb_launch(fold_cols_k<true>, dim3((N + 31) / 32), dim3(FOLD_THREADS), 0, st, out, (void*)nullptr, (const float*)partial, S, N, N);
+  fold_launch<true>(out, nullptr, partial, S, N, N, st);
   LAUNCH_RET;
 }
 // (ticket null: the first 32 words of `partial` are the tickets)
@@ -1580,7 +1596,7 @@ MLB_API int mlb_rmsnorm_bwd(void* dx, float* dw, const void* dy, const void* x, 
   // Whole multiples of 256 columns: a block's threads share a row instead of a warp having one, and the partial rows are folded by a
   // kernel of their own, which overlaps this one's end.  One warp a row, with the fold by the blocks that finish last, against this, inputs
   // not in L2: 16384 x 768 31.7 -> 27.6 us, 4096 x 768 21 -> 15.4, 64 x 768 13.3 -> 11.3, 65536 x 256 46 -> 33.8, 4096 x 512 17.4 -> 15.4,
-  // 16384 x 512 25.6 -> 23.6 (in L2 14.1 -> 14.8, the one size that is slower).
+  // 16384 x 512 25.6 -> 23.6 (in L2 14.1 = 14.1).
   if (norm_rows_ok(dx, dy, x, w, add, rows, C)) {
     norm_rows_launch<false>(dx, dw, nullptr, false, dy, x, w, nullptr, rstd, add, rows, C, partial, st);
     LAUNCH_RET;

@@ -1574,6 +1574,12 @@ def test_column_sums_fold_in_one_order(rows, C):
     assert torch.equal(d, total)
 
 
+@pytest.mark.parametrize("rows", [640, 641, 648, 2367])
+def test_column_sums_fold_at_a_trips_end(rows):
+    """80 partial rows are the most that eight warps take in one trip; one more, and 32 warps load them."""
+    test_column_sums_fold_in_one_order(rows, 256)
+
+
 def _native_nodes():
     """name -> (operands, call through the public entry point), each a plain call of the extension module: for tests of its autograd nodes."""
     from ml_b200.ops import autograd as F
