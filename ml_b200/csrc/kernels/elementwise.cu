@@ -329,8 +329,8 @@ __global__ void __launch_bounds__(256) layernorm_bwd_k(bf16* __restrict__ dx, fl
 // floats, `ticket` = 1 + RMS_GROUPS ints that are 0 on entry and left 0 on exit.
 constexpr int RMS_GROUPS = 16;
 // Up to 32 blocks (256 rows) there is one group, and its last block adds the partial rows up with all of its threads.
-// NARROW: one vector of eight per lane, rows narrower than 256 (C % 8 == 0); otherwise any C, alignment and width, by scalars.
-template <bool NARROW>
+// VPL = C / 256 (vectors of 8 per lane) up to 3; PART: one vector per lane of rows narrower than 256 (C % 8 == 0); 0 = generic C (scalar path).
+template <int VPL, bool PART = false>
 __global__ void __launch_bounds__(256, 2) rmsnorm_bwd_k(bf16* __restrict__ dx, float* __restrict__ dw, const bf16* __restrict__ dy,
                                                      const bf16* __restrict__ x, const bf16* __restrict__ w,
                                                      const float* __restrict__ rstd, const bf16* __restrict__ add, long rows,
@@ -342,41 +342,66 @@ __global__ void __launch_bounds__(256, 2) rmsnorm_bwd_k(bf16* __restrict__ dx, f
   for (int i = threadIdx.x; i < C; i += blockDim.x) sh[i] = 0.f;
   __syncthreads();
   const float invC = 1.f / (float)C;
-  if (NARROW) {
-    float acc[8], ww[8] = {};
-    const bool mine = lane * 8 < C;      // this lane has columns
-    if (mine) load8(w + lane * 8, ww);
+  if (VPL > 0) {
+    constexpr int NV = VPL > 0 ? VPL : 1;
+    constexpr bool CACHE_W = NV <= 2;  // the weight vector stays in registers (two resident blocks per SM leave 128 per thread)
+    constexpr int NW = CACHE_W ? NV : 1;
+    float acc[NV][8];
+    float ww[NW][8] = {};
+    const bool mine = !PART || lane * 8 < C;      // this lane has columns
 #pragma unroll
-    for (int j = 0; j < 8; j++) acc[j] = 0.f;
+    for (int v = 0; v < NV; v++) {
+      if (CACHE_W && mine) load8(w + (v * 32 + lane) * 8, ww[v]);
+#pragma unroll
+      for (int j = 0; j < 8; j++) acc[v][j] = 0.f;
+    }
     for (long row = (long)blockIdx.x * nwarp + warp; row < rows; row += (long)gridDim.x * nwarp) {
       const float r = rstd[row];
-      // every load of the row is issued before its reduction: `add` does not depend on it, and fetching it only
-      // afterwards cost a second DRAM round trip per row
-      const long off = row * C + lane * 8;
-      const uint4 zero = make_uint4(0, 0, 0, 0);
-      const uint4 xr = mine ? *reinterpret_cast<const uint4*>(x + off) : zero;
-      const uint4 dr = mine ? *reinterpret_cast<const uint4*>(dy + off) : zero;
-      const uint4 ar = add && mine ? *reinterpret_cast<const uint4*>(add + off) : zero;
-      float xf[8], df[8], o[8], dot = 0.f;
-      unpack8(xr, xf);
-      unpack8(dr, df);
-      unpack8(ar, o);
+      // The row's x, dy and residual-stream gradient stay in registers PACKED (four registers per eight values) between
+      // the two passes, and every load of the row is issued before the row's reduction: `add` does not depend on it, and
+      // fetching it only afterwards cost a second DRAM round trip per row.
+      uint4 xr[NV], dr[NV], ar[NV];
+      float dot = 0.f;
 #pragma unroll
-      for (int j = 0; j < 8; j++) dot += df[j] * ww[j] * xf[j];
+      for (int v = 0; v < NV; v++) {
+        const long off = row * C + (v * 32 + lane) * 8;
+        const int cw = CACHE_W ? v : 0;
+        xr[v] = mine ? *reinterpret_cast<const uint4*>(x + off) : make_uint4(0, 0, 0, 0);
+        dr[v] = mine ? *reinterpret_cast<const uint4*>(dy + off) : make_uint4(0, 0, 0, 0);
+        ar[v] = add && mine ? *reinterpret_cast<const uint4*>(add + off) : make_uint4(0, 0, 0, 0);
+        if (!CACHE_W) load8(w + (v * 32 + lane) * 8, ww[0]);
+        float xf[8], df[8];
+        unpack8(xr[v], xf);
+        unpack8(dr[v], df);
+#pragma unroll
+        for (int j = 0; j < 8; j++) dot += df[j] * ww[cw][j] * xf[j];
+      }
       dot = warp_sum(dot);
       const float k = r * r * r * invC * dot;
 #pragma unroll
-      for (int j = 0; j < 8; j++) {
-        o[j] += df[j] * ww[j] * r - xf[j] * k;
-        acc[j] += df[j] * xf[j] * r;
+      for (int v = 0; v < NV; v++) {
+        const long off = row * C + (v * 32 + lane) * 8;
+        const int cw = CACHE_W ? v : 0;
+        if (!CACHE_W) load8(w + (v * 32 + lane) * 8, ww[0]);
+        float xf[8], df[8], o[8];
+        unpack8(xr[v], xf);
+        unpack8(dr[v], df);
+        unpack8(ar[v], o);
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          o[j] += df[j] * ww[cw][j] * r - xf[j] * k;
+          acc[v][j] += df[j] * xf[j] * r;
+        }
+        if (mine) store8(dx + off, o);
       }
-      if (mine) store8(dx + off, o);
     }
     // fold the 8 warps' register partials in warp order (deterministic)
     for (int wv = 0; wv < nwarp; wv++) {
       if (warp == wv && mine) {
 #pragma unroll
-        for (int j = 0; j < 8; j++) sh[lane * 8 + j] += acc[j];
+        for (int v = 0; v < NV; v++)
+#pragma unroll
+          for (int j = 0; j < 8; j++) sh[(v * 32 + lane) * 8 + j] += acc[v][j];
       }
       __syncthreads();
     }
@@ -414,7 +439,7 @@ __global__ void __launch_bounds__(256, 2) rmsnorm_bwd_k(bf16* __restrict__ dx, f
   __syncthreads();
   if (!is_last) return;
   __threadfence();
-  if (NARROW && nb <= 32) {
+  if (PART && nb <= 32) {
     // slice q of the threads takes rows q, q + slices, ...; the slices are added in order (C < 256: at least four of them, at most 1024 floats)
     const int vecs = C >> 2, slices = (int)blockDim.x / vecs, q = threadIdx.x / vecs, c = threadIdx.x % vecs * 4;
     if (q < slices) {
@@ -1595,15 +1620,24 @@ MLB_API int mlb_rmsnorm_bwd(void* dx, float* dw, const void* dy, const void* x, 
   if (sh > 48 * 1024) return -3;
   // Whole multiples of 256 columns: a block's threads share a row instead of a warp having one, and the partial rows are folded by a
   // kernel of their own, which overlaps this one's end.  One warp a row, with the fold by the blocks that finish last, against this, inputs
-  // not in L2: 16384 x 768 31.7 -> 27.6 us, 4096 x 768 21 -> 15.4, 64 x 768 13.3 -> 11.3, 65536 x 256 46 -> 33.8, 4096 x 512 17.4 -> 15.4,
-  // 16384 x 512 25.6 -> 23.6 (in L2 14.1 = 14.1).
-  if (norm_rows_ok(dx, dy, x, w, add, rows, C)) {
+  // not in L2: 16384 x 768 31.7 -> 27.6 us, 4096 x 768 21 -> 15.4, 65536 x 256 46 -> 33.8, 4096 x 512 17.4 -> 15.4, 16384 x 512 25.6 -> 23.6
+  // (in L2 14.1 = 14.1).  In a small model's step, though, the host's launches are the bound and one less is worth more than the 2 us by which
+  // this is shorter there too; the step's products grow as rows C^2, and so does the line.  Steps of two layers, us, one launch and two: 256 wide,
+  // 512 rows 358 and 368, 4096 rows 363 and 374, 8192 rows 444 and 443; 512 wide, 1024 rows 361 and 370, 2048 rows 411 and 399; 768 wide,
+  // 128 rows 392 and 401, 512 rows 459 and 443.
+  const bool rows_ok = norm_rows_ok(dx, dy, x, w, add, rows, C);
+  if (rows_ok && (C >= 1024 || rows * C * C > 1L << 28)) {
     norm_rows_launch<false>(dx, dw, nullptr, false, dy, x, w, nullptr, rstd, add, rows, C, partial, st);
     LAUNCH_RET;
   }
   const bool narrow = C < 256 && C % 8 == 0 && (((uintptr_t)dx | (uintptr_t)dy | (uintptr_t)x | (uintptr_t)w | (uintptr_t)add | (uintptr_t)partial) & 15) == 0;
-  if (narrow) RB(true);
-  else RB(false);
+  if (narrow) { RB(1, true); LAUNCH_RET; }
+  switch (rows_ok ? C / 256 : 0) {
+    case 1: RB(1); break;
+    case 2: RB(2); break;
+    case 3: RB(3); break;
+    default: RB(0); break;
+  }
 #undef RB
   LAUNCH_RET;
 }

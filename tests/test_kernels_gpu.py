@@ -1508,9 +1508,11 @@ def test_rmsnorm_backward_of_few_or_narrow_rows(rows, C, add):
         assert torch.equal(runs[0][0], runs[1][0]) and torch.equal(runs[0][1], runs[1][1])
 
 
-@pytest.mark.parametrize("rows,C,shift", [(1, 256, 0), (25, 512, 0), (2369, 256, 0), (7200, 768, 0), (25, 512, 1), (9, 768, 8), (3, 256, 4)])
+@pytest.mark.parametrize("rows,C,shift", [(1, 256, 0), (25, 512, 0), (2369, 256, 0), (7200, 768, 0), (25, 512, 1), (9, 768, 8), (3, 256, 4),
+                                          (4096, 256, 0), (4097, 256, 0), (1024, 512, 0), (1025, 512, 0), (455, 768, 0), (456, 768, 0)])
 def test_rmsnorm_backward_of_whole_vectors_of_columns(rows, C, shift):
-    """Rows that share a block's threads, past one round of its groups, and the same widths from a place where vectors may not be loaded."""
+    """A row per warp and rows that share a block's threads, either side of the line, past one round of the groups, and the same widths from a place where
+    vectors may not be loaded."""
     torch.manual_seed(rows + C)
     big = rnd(rows * C + 8)
     x, dy, w, a = big[shift:shift + rows * C].view(rows, C), rnd(rows, C), 1 + rnd(1, C, scale=0.1).view(-1), rnd(rows, C)
