@@ -1365,9 +1365,9 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kv_tc_kernel(const __
 //   * the element-wise warps read scores as fragments (two adjacent queries of each eight, for several keys): a query's statistics then cost
 //     a quarter of the shared-memory reads, which the MMAs' operands compete for, and stores of 8 x 8 matrices need no shuffles;
 //   * code is kept small (two passes over 32 columns instead of one over 64, waits of few instructions, work items taken apart once, no
-//     time stamps): six roles share the SM's instruction cache, and its misses were the bound: 935 k of 6.1 M requests a launch of
-//     16 x 1024 tokens, 316 k now.
-// 16 x 1024 tokens, 12 heads: 136 -> 100 us (32 x 256: 53 -> 40 with the finishing kernel).  Taking out the exponentials, the MMAs, the dQ
+//     time stamps): six roles share the SM's instruction cache, and its misses were the bound: 694 k of 5.46 M requests a launch of
+//     16 x 1024 tokens before this form (935 k of 6.1 M with everything unrolled), 316 k of 4.64 M now.
+// 16 x 1024 tokens, 12 heads: 136 -> 100 us (32 x 256: 53 -> 40 with the finishing kernel as it was then).  Taking out the exponentials, the MMAs, the dQ
 // stores or the dK / dV epilogue one at a time changes that by 5 to 11 us each: none of them alone is the bound any more.
 //   * dQ_j is a partial sum over key tiles.  fp32 add-reduces into one accumulator (TMA or vector red) ran into the
 //     L2's atomic throughput (32 KB per block and SM); instead every (query tile, key tile) pair owns a bf16 tile of a
@@ -2201,10 +2201,10 @@ MLB_API void mlb_attn_force_simt(int on) { g_attn_force_simt = on; }
 MLB_API void mlb_attn_fwd_mode(int rows) { g_fwd_rows = rows; }
 // 1: the persistent attention kernels draw their work items from a device counter (see ItemRing); 0: host-built table
 MLB_API void mlb_attn_dynamic(int on) { g_attn_dynamic = on; }
-// Diagnostic: device buffer of at least 8 * (query blocks per CTA) int64 that CTA (0,0,0) of the fused backward fills
-// with SM cycle stamps, eight per block: element-wise warp 0 before / after the score wait, after its exponentials,
-// after the previous block's MMAs completed, after P^T / dS^T are stored; control thread when it saw P^T and when the
-// block's MMAs were issued; first drain warp when the dQ partial was stored.  nullptr switches it off.
+// Diagnostic: device buffer of at least 8 * (query blocks per CTA) int64 that CTA (0,0,0) of the fused backward (an instantiation of
+// its own: the stamps cost the other one instruction-cache misses) fills with SM cycle stamps, eight per block: element-wise warp 0
+// before / after the score wait, after both halves of its exponentials, twice when it has handed P^T / dS^T over; gradient thread when it
+// saw P^T and when the block's MMAs were issued; first drain warp when the dQ partial was stored.  nullptr switches it off.
 MLB_API void mlb_attn_set_timeline(void* buf) { g_timeline = (long long*)buf; }
 
 // Balanced static schedules for the persistent attention kernels.  Work items (forward: pair p of a (sample, head);

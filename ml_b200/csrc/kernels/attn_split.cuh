@@ -568,7 +568,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) attn_split_bwd_k(const __grid_c
 
 // Do the kernels start under the one before them?  Four CTAs of the forward fit an SM at head sizes up to 64, two of the backward (at 128: two and
 // one), so the limit is two to eight waves.  It is where the gain has become small, not where something gets slower: forward + backward without a
-// mask, 197 tokens, 12 heads of 64, us apart and early: 0.6 CTAs per SM 43.1 and 38.3, 2.6 73.6 and 64.5, 5.2 114.6 and 107.7, 7.8 162.8 and
+// mask, 197 tokens, 12 heads of 64, us apart and early (kernels a tenth slower than these): 0.6 CTAs per SM 43.1 and 38.3, 2.6 73.6 and 64.5, 5.2 114.6 and 107.7, 7.8 162.8 and
 // 156.7, 10 212.9 and 207.7, 21 383.9 and 377.7.  Slower where the backward's CTAs are just short of one wave, which the early ones
 // take up unevenly (1.9: 51.2 and 53.0; 577 tokens, 1.6: 96.7 and 107.0).
 static bool split_early(const SplitArgs& a) { return (long)((a.T + 127) / 128) * a.H * a.B <= 8L * mlb_sm_count(); }
