@@ -1582,6 +1582,21 @@ def test_column_sums_fold_at_a_trips_end(rows):
     test_column_sums_fold_in_one_order(rows, 256)
 
 
+@pytest.mark.parametrize("B,T,H,hd", [(11, 1000, 12, 64), (33, 125, 16, 128)])
+def test_attention_backward_of_many_rows_is_that_of_each_sample(B, T, H, hd):
+    """From 2^20 vectors on a thread sums two of them for rowsum(dO * O), the last block not full: the gradients are those of one sample at a time, bit for bit."""
+    torch.manual_seed(B)
+    n = nat()
+    qkv, dout = rnd(B * T, 3 * H * hd), rnd(B * T, H * hd)
+    out, lse, d = torch.empty_like(dout), torch.empty(B, H, T, device=dev()), torch.empty_like(qkv)
+    n.attn_fwd(out, lse, qkv, B, T, H, hd)
+    n.attn_bwd(d, dout, qkv, out, lse, B, T, H, hd)
+    for b in (0, B // 2, B - 1):
+        r, e = slice(b * T, (b + 1) * T), torch.empty(T, 3 * H * hd, device=dev(), dtype=torch.bfloat16)
+        n.attn_bwd(e, dout[r], qkv[r], out[r], lse[b:b + 1], 1, T, H, hd)
+        assert torch.equal(d[r], e)
+
+
 def _native_nodes():
     """name -> (operands, call through the public entry point), each a plain call of the extension module: for tests of its autograd nodes."""
     from ml_b200.ops import autograd as F
