@@ -1597,6 +1597,26 @@ def test_attention_backward_of_many_rows_is_that_of_each_sample(B, T, H, hd):
         assert torch.equal(d[r], e)
 
 
+@pytest.mark.parametrize("rows,V", [(3, 8), (700, 512), (40, 1016), (7, 1024), (7, 1032), (40, 2056)])
+def test_cross_entropy_either_side_of_its_block_sizes(rows, V):
+    torch.manual_seed(V)
+    n, z = nat(), rnd(rows, V, scale=3.0)
+    tgt = torch.randint(0, V, (rows,), device=dev(), dtype=torch.int32)
+    tgt[rows // 2] = -1
+    zd, live = z.double(), (tgt >= 0).double()
+    lse, zt = torch.logsumexp(zd, -1), zd.gather(1, tgt.clamp(min=0).long()[:, None])[:, 0]
+    loss, losses, dz = torch.empty((), device=dev()), torch.empty(rows, device=dev()), torch.empty_like(z)
+    n.ce_mean(loss, losses, dz, z, tgt)
+    # fp32 sums of at most 16 terms a thread and nine levels over the threads, the exponentials off by 2 ulp: below 2^-17 of the sum
+    assert ((losses - (lse - zt) * live).abs() < 2 ** -17 + 2 ** -22 * lse.abs()).all()
+    g = (zd - lse[:, None]).exp()
+    g[torch.arange(rows, device=dev()), tgt.clamp(min=0).long()] -= 1
+    assert _rel(dz, g * (live / live.sum())[:, None]) < 2 ** -8
+    in_place, ls = z.clone(), torch.empty(rows, device=dev())
+    n.ce_fwd_bwd(ls, in_place, tgt, 1.0 / float(live.sum()))
+    assert torch.equal(ls, losses) and torch.equal(in_place, dz)
+
+
 def _native_nodes():
     """name -> (operands, call through the public entry point), each a plain call of the extension module: for tests of its autograd nodes."""
     from ml_b200.ops import autograd as F
