@@ -872,8 +872,8 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_q128_k(const __gri
         const int qt = nq - 1 - w / BH, bh = w % BH, b = bh / a.H, x = (bh % a.H) * H128;
         ok = wait(bar_out, li & 1, 94);
         if (!ok) break;
-        for (int lg = 0; lg < 4; lg++)
-          if (a.T - (qt * 128 + lg * 32) >= 32)
+        for (int lg = 0; lg < 4; lg++)      // (the tile comes here after a wait that ran out, too)
+          if (!*s_abort && a.T - (qt * 128 + lg * 32) >= 32)
             for (int c = 0; c < 2; c++) tc::tma_store_2d(&tm_out, smem + S::DO + c * TILE_BYTES + lg * 4096, x + c * 64, b * a.T + qt * 128 + lg * 32);
         tc::tma_commit_group();
         tc::tma_wait_group_read<0>();

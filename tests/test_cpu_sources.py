@@ -1,0 +1,56 @@
+"""What the kernel sources have to keep to and no run can show: what happens after a wait has run out, and what needs a whole warp."""
+import re
+from pathlib import Path
+
+KERNELS = Path(__file__).resolve().parent.parent / "ml_b200" / "csrc" / "kernels"
+
+
+def _kernels():
+    """(file, name, body without comments, line breaks kept) of every __global__ function."""
+    for path in sorted(list(KERNELS.glob("*.cu")) + list(KERNELS.glob("*.cuh"))):
+        text = re.sub(r"/\*.*?\*/", lambda m: re.sub(r"[^\n]", " ", m.group(0)), path.read_text(), flags=re.S)
+        text = re.sub(r"//[^\n]*", "", text)
+        for m in re.finditer(r"__global__\s+void[^;{]*?\b(\w+)\s*\((?:[^()]|\([^()]*\))*\)\s*\{", text):
+            depth, i = 1, m.end()
+            while depth:
+                depth += {"{": 1, "}": -1}.get(text[i], 0)
+                i += 1
+            yield path.name, m.group(1), text[m.start():i], text.count("\n", 0, m.start()) + 1
+
+
+def _heads(body, at):
+    """The statement that position `at` is in up to there, and the heads of the blocks around it, innermost first."""
+    i = at
+    while i > 0:
+        end, parens = i, 0
+        while i > 0:
+            c = body[i - 1]
+            parens += {")": 1, "(": -1}.get(c, 0)
+            if parens <= 0 and c in "{};":
+                break
+            i -= 1
+        yield body[i:end]
+        depth = 0      # to the brace that opens the block around
+        while i > 0:
+            i -= 1
+            depth += {"}": 1, "{": -1}.get(body[i], 0)
+            if depth < 0:
+                break
+
+
+def test_the_kernels_are_found():
+    names = {name for _, name, _, _ in _kernels()}
+    assert {"attn_bwd_q128_k", "attn_bwd_kv128_k", "attn_bwd_fused_tc_kernel", "attn_fwd_rows_tc_kernel", "attn_split_bwd_k", "gemm_tc_kernel"} <= names
+
+
+def test_a_block_that_has_given_up_stores_no_tile():
+    """After a wait has run out, what stands in tensor and shared memory is nobody's result: each tile that leaves asks for the block's word first."""
+    found, unasked = 0, []
+    for file, name, body, line in _kernels():
+        if "s_abort" not in body:
+            continue
+        for m in re.finditer(r"\btc::tma_store_2d\(|\btile128_rows\(", body):
+            found += 1
+            if not any("*s_abort" in head for head in _heads(body, m.start())):
+                unasked.append(f"{file}:{line + body.count(chr(10), 0, m.start())} {name}")
+    assert found >= 7 and not unasked, unasked
