@@ -334,6 +334,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_tc_kernel(const __gri
         const int kc0 = j * 128 + cq * 32;
         if (!have_scores) {   // first block of this CTA: nothing was prefetched
           wait(&bar_s[sl], (g >> 1) & 1, 17);
+          __syncwarp();
           tc::tc_fence_after();
           tc::tmem_ld32_wait(tmem + sl * 128 + lane_addr + cq * 32, r);
           have_scores = true;
@@ -382,6 +383,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_tc_kernel(const __gri
         const bool more = (j + 1 < it.nkb) || (it.w + stride < total);
         if (more) {
           wait(&bar_s[(g + 1) & 1], ((g + 1) >> 1) & 1, 17);
+          __syncwarp();
           tc::tc_fence_after();
           tc::tmem_ld32(tmem + ((g + 1) & 1) * 128 + lane_addr + cq * 32, r);
         } else {
@@ -389,6 +391,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_tc_kernel(const __gri
         }
         if (j > 0) {   // fold in the previous block, whose P V product had a whole softmax to complete
           wait(&bar_o[(g - 1) & 1], ((g - 1) >> 1) & 1, 18);
+          __syncwarp();
           tc::tc_fence_after();
           fold(g - 1, alpha_prev);     // its tcgen05.wait::ld also covers the score prefetch
           tc::tmem_ld_tie(r);
@@ -398,6 +401,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_tc_kernel(const __gri
         alpha_prev = alpha;
       }
       wait(&bar_o[(g - 1) & 1], ((g - 1) >> 1) & 1, 19);
+      __syncwarp();
       tc::tc_fence_after();
       fold(g - 1, alpha_prev);
       // combine the four partial row sums (third exchange buffer: the max buffers may already be in use by a fast warp
@@ -794,6 +798,7 @@ __global__ void __maxnreg__(160) attn_fwd_rows_tc_kernel(const __grid_constant__
           // The first block of an item always takes the exact way.  j, qt and the votes are uniform over the warp.
           if (tl && g < 16) tl[g * 8 + 0] = clock64();
           wait(&bar_s[t], g & 1, 67);
+          __syncwarp();
           tc::tc_fence_after();
           s_seen(j);
           if (tl && g < 16) tl[g * 8 + 1] = clock64();
@@ -803,6 +808,7 @@ __global__ void __maxnreg__(160) attn_fwd_rows_tc_kernel(const __grid_constant__
           auto free_p = [&]() {
             if (!p_free) {
               wait(&bar_o[t], (g - 1) & 1, 68);
+              __syncwarp();
               tc::tc_fence_after();
               if (lane == 0) tc::mbar_arrive(&bar_vf[(g - 1) % VN]);     // P V of block g-1 is done with its V slot
               p_free = true;
@@ -914,6 +920,7 @@ __global__ void __maxnreg__(160) attn_fwd_rows_tc_kernel(const __grid_constant__
         }
         if (tl && g < 16) tl[g * 8 + 0] = clock64();
         wait(&bar_s[t], g & 1, 67);
+        __syncwarp();
         tc::tc_fence_after();
         s_seen(j);
         if (tl && g < 16) tl[g * 8 + 1] = clock64();
@@ -959,6 +966,7 @@ __global__ void __maxnreg__(160) attn_fwd_rows_tc_kernel(const __grid_constant__
         if (tl && g < 16) tl[g * 8 + 2] = clock64();
         if (j > 0) {   // the previous block's P V has had the whole row-maximum pass to complete; P's columns are free after it
           wait(&bar_o[t], (g - 1) & 1, 68);
+          __syncwarp();
           tc::tc_fence_after();
           if (lane == 0) tc::mbar_arrive(&bar_vf[(g - 1) % VN]);
           if (tl && g < 16) tl[g * 8 + 5] = clock64();
@@ -1011,6 +1019,7 @@ __global__ void __maxnreg__(160) attn_fwd_rows_tc_kernel(const __grid_constant__
         alpha_prev = alpha;
       }
       wait(&bar_o[t], (g - 1) & 1, 69);
+      __syncwarp();
       tc::tc_fence_after();
       if (lane == 0) tc::mbar_arrive(&bar_vf[(g - 1) % VN]);
       fold(alpha_prev);
@@ -1300,7 +1309,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kv_tc_kernel(const __
       else s_delta[tid - 128] = (q < a.T) ? a.delta[si] : 0.f;
     }
     __syncthreads();
-    if (!tc::mbar_wait(bar_s, it & 1, 22)) { ok = false; break; }
+    if (!__all_sync(0xffffffffu, tc::mbar_wait(bar_s, it & 1, 22))) { ok = false; break; }
     tc::tc_fence_after();
     // every MMA issued so far has completed: the other Q/dO buffer (read by the previous dV/dK) can be refilled
     if (tid == 0 && it + 1 < n_it) load_q_do(i + 1, buf ^ 1);
@@ -1669,6 +1678,7 @@ __global__ void __maxnreg__(120) attn_bwd_fused_tc_kernel(const __grid_constant_
         const float* stat = (const float*)(smem + S::STAT) + (blk & 1) * 256 + c0 + fc;
         if (tl && warp == 0) tl[blk * 8 + 0] = clock64();
         wait(bar_s, blk & 1, 48);          // S^T of this block is complete, its statistics are there
+        __syncwarp();
         tc::tc_fence_after();
         if (tl && warp == 0) tl[blk * 8 + 1] = clock64();
         // 32 columns at a time, and not unrolled: the instructions of all roles have to stay in the SM's cache
@@ -2029,7 +2039,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_q_tc_kernel(const __g
   for (int j = 0; j < nkb; j++) {
     const int buf = j & 1;
     const int k0 = j * 128;
-    if (!tc::mbar_wait(bar_s, j & 1, 32)) { ok = false; break; }
+    if (!__all_sync(0xffffffffu, tc::mbar_wait(bar_s, j & 1, 32))) { ok = false; break; }
     tc::tc_fence_after();
     if (tid == 0 && j + 1 < nkb) load_kv(j + 1, buf ^ 1);
     const bool diag = (j == qt);

@@ -641,8 +641,8 @@ __global__ void __launch_bounds__(BWD128_THREADS, 1) attn_bwd_kv128_k(const __gr
 #pragma unroll
           for (int m = 0; m < 8; m++) wp[x][m] = pack_bf16(p[x][2 * m], p[x][2 * m + 1]);
         if (g > 0) wait(&bar_dof[(g - 1) & 1], ((g - 1) >> 1) & 1, 86);      // dV of the block before has read its P^T
-        if (i == kt && li > 0) rows_read();
         __syncwarp();
+        if (i == kt && li > 0) rows_read();
 #pragma unroll
         for (int x = 0; x < 2; x++) {
           tc::stmatrix_x4(p_at + x * 2048, wp[x][0], wp[x][1], wp[x][2], wp[x][3]);

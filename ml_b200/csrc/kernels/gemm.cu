@@ -312,7 +312,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       const int mt = t % g.tiles_m, nt = (t / g.tiles_m) % g.tiles_n;
       const int m0 = mt * BM, n0 = nt * BN;
       const int acc = it & 1, acc_phase = (it >> 1) & 1;
-      if (!tc::mbar_wait(&acc_full[acc], acc_phase, 4)) { ok = false; break; }
+      if (!__all_sync(0xffffffffu, tc::mbar_wait(&acc_full[acc], acc_phase, 4))) { ok = false; break; }
       tc::tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(lg * 32) << 16) + acc * BN;
       const bool rows_live = (m0 + lg * 32) < g.M;
@@ -579,7 +579,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     for (; ok && iter.next(w); it++) {
       const int m0 = w.mt * PM + (int)rank * 128 + lg * 32, n0 = w.nt * BN + half * 128;
       const int acc = it & 1, acc_phase = (it >> 1) & 1;
-      if (!tc::mbar_wait(&acc_full[acc], acc_phase, 0x24)) { ok = false; break; }
+      if (!__all_sync(0xffffffffu, tc::mbar_wait(&acc_full[acc], acc_phase, 0x24))) { ok = false; break; }
       tc::tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(lg * 32) << 16) + acc * BN + half * 128;
       const bool rows_live = m0 < g.M;

@@ -47,6 +47,8 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
 #endif
 // (As few instructions as it can be, here and below: a kernel has dozens of waits, and what they hold besides the first probe pushes its
 // loops out of the SM's instruction cache.  A probe sleeps in hardware for a while, so reading the clock after each costs nothing.)
+// Lanes may leave in different rounds: a whole warp that waits is brought together (__syncwarp, or a vote where the answer decides) before
+// it touches tensor memory, stores matrices or meets at a named barrier.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int where = 0) {
   if (mbar_try(bar, parity)) return true;
   const uint64_t t0 = globaltimer_ns();

@@ -54,3 +54,40 @@ def test_a_block_that_has_given_up_stores_no_tile():
             if not any("*s_abort" in head for head in _heads(body, m.start())):
                 unasked.append(f"{file}:{line + body.count(chr(10), 0, m.start())} {name}")
     assert found >= 7 and not unasked, unasked
+
+
+ONE_THREAD = re.compile(r"lane == 0|tid == 0|threadIdx\.x == 0|elect_one\(\)|\bleader\(\)|\bloader\(\)|auto issue_\w+ = \[&\]")
+WAIT = re.compile(r"(?<!\w)(?:tc::)?(?:wait|mbar_wait)\(")
+
+
+def _close(body, at):
+    """Position behind the parenthesis that closes the one before `at`."""
+    depth = 1
+    while depth:
+        depth += {"(": 1, ")": -1}.get(body[at], 0)
+        at += 1
+    return at
+
+
+def test_a_warp_is_together_again_behind_its_waits():
+    """A wait is a loop that lanes can leave in different rounds, and tensor-memory accesses, matrix stores and named barriers take a whole warp: behind the
+    last wait of a row the warp is brought together before anything else.  Where the answer decides, the lanes have one answer."""
+    found, apart = 0, []
+    for file, name, body, line in _kernels():
+        if "mbar_wait" not in body:
+            continue
+        for m in WAIT.finditer(body):
+            heads = list(_heads(body, m.start()))
+            if "auto wait" in heads[0] or any(ONE_THREAD.search(h) for h in heads):
+                continue
+            found += 1
+            end = _close(body, m.end())
+            where = f"{file}:{line + body.count(chr(10), 0, m.start())} {name}"
+            if body[end] != ";":      # its answer is asked for
+                if not heads[0].rstrip().endswith("__all_sync(0xffffffffu,"):
+                    apart.append(where)
+                continue
+            rest = body[end + 1:].lstrip()
+            if not re.match(r"__syncwarp\(\)|__syncthreads\(\)|(?:if \([^;{}]*\) )?wait\(|(?:tc::tc_fence_after\(\);\s*)?if \(__all_sync\(", rest):
+                apart.append(where)
+    assert found > 20 and not apart, "\n".join(apart)
