@@ -195,7 +195,8 @@ _ERR_CODES = {1: "an mbarrier wait inside a kernel's pipeline ran out", 2: "a wa
               3: "an index was out of range"}
 _ERR_BOUNDS = {0xE1: "token id outside the vocabulary (embedding forward)", 0xE2: "token id outside the vocabulary (embedding backward)",
                0xCE: "target outside the vocabulary (cross-entropy)",
-               0xA1: "shared memory of the attention backward does not start on a 1024-byte boundary"}
+               0xA1: "shared memory of the attention backward (head size 128) does not start on a 1024-byte boundary",
+               0xA2: "shared memory of the attention backward (head size 64) does not start on a 1024-byte boundary"}
 
 
 def describe_error(err: int) -> str:

@@ -91,3 +91,10 @@ def test_a_warp_is_together_again_behind_its_waits():
             if not re.match(r"__syncwarp\(\)|__syncthreads\(\)|(?:if \([^;{}]*\) )?wait\(|(?:tc::tc_fence_after\(\);\s*)?if \(__all_sync\(", rest):
                 apart.append(where)
     assert found > 20 and not apart, "\n".join(apart)
+
+
+def test_every_refused_index_has_its_words():
+    from ml_b200.ops.native import describe_error
+    details = {int(d, 16) for path in KERNELS.glob("*.cu*") for d in re.findall(r"MLB_ERR_BOUNDS, (0x[0-9A-Fa-f]+)\)", path.read_text())}
+    assert 0xE1 in details
+    assert not [hex(d) for d in details if describe_error(3 << 24 | d).endswith(f"detail {d:#x}")]
