@@ -502,8 +502,7 @@ struct ItemRing {
       if (li >= seq[64]) return -1;
       if (*abort_flag) return -1;
     }
-    mlb_set_error(MLB_ERR_MBAR_TIMEOUT, 0x7f);
-    *abort_flag = 1;
+    *abort_flag = 0x7f;      // (reported at the block's end)
     return -1;
   }
 };
@@ -2216,6 +2215,38 @@ bool tc_ok(const void* qkv, const void* other, int H, int hd) {
   return !g_attn_force_simt && (hd == 64 || hd == 128) && ((uintptr_t)qkv % 16 == 0) && ((uintptr_t)other % 16 == 0) && (C % 8 == 0);
 }
 
+// Waits that run out (diagnostic): every warp of a block waits, 2 ms at most, on a barrier that nobody arrives on, warp w under the number w + 1, then
+// once more on it, then on one that is complete.  Nothing is in flight that the block would have to wait for.  Of each thread, four ints: did the waits
+// return true (bits 0, 1, 2), the block's word after the first wait and at the end, microseconds of the second.
+constexpr int WAIT_PROBE_THREADS = 256;
+__global__ void __launch_bounds__(WAIT_PROBE_THREADS) wait_probe_k(int4* out) {
+  __shared__ uint64_t bars[2];
+  __shared__ int s_word;
+  volatile int* s_abort = &s_word;
+  const int tid = threadIdx.x;
+  if (tid == 0) {
+    tc::mbar_init(&bars[0], 1);
+    tc::mbar_init(&bars[1], 1);
+    *s_abort = 0;
+    tc::mbar_fence_init();
+    tc::mbar_arrive(&bars[1]);
+  }
+  __syncthreads();
+  auto wait = [&](uint64_t* bar, int where) { return tc::mbar_wait_sticky<2000000>(bar, 0, where, s_abort); };
+  const int where = (tid >> 5) + 1;
+  const bool first = wait(&bars[0], where);
+  __syncwarp();
+  const int word = *s_abort;
+  const uint64_t t0 = tc::globaltimer_ns();
+  const bool again = wait(&bars[0], 100 + where);
+  __syncwarp();
+  const uint64_t t1 = tc::globaltimer_ns();
+  const bool done = wait(&bars[1], 200 + where);
+  __syncthreads();
+  out[blockIdx.x * WAIT_PROBE_THREADS + tid] = make_int4(first | again << 1 | done << 2, word, *s_abort, (int)((t1 - t0) / 1000));
+  if (tid == 0) tc::report_given_up(s_abort);
+}
+
 }  // namespace
 
 static long long* g_timeline = nullptr;
@@ -2227,6 +2258,12 @@ MLB_API void mlb_attn_dynamic(int on) { g_attn_dynamic = on; }
 // its own: the stamps cost the other one instruction-cache misses) fills with SM cycle stamps, eight per block: element-wise warp 0
 // before / after the score wait, after both halves of its exponentials, twice when it has handed P^T / dS^T over; gradient thread when it
 // saw P^T and when the block's MMAs were issued; first drain warp when the dQ partial was stored.  nullptr switches it off.
+// `out`: blocks x 256 x 4 ints, see wait_probe_k.  Leaves the error word set.
+MLB_API int mlb_attn_wait_probe(void* out, int blocks, cudaStream_t st) {
+  if (blocks < 1 || blocks > 4096 || ((uintptr_t)out & 15)) return -7;
+  wait_probe_k<<<blocks, WAIT_PROBE_THREADS, 0, st>>>((int4*)out);
+  return (int)cudaGetLastError();
+}
 MLB_API void mlb_attn_set_timeline(void* buf) { g_timeline = (long long*)buf; }
 
 // Balanced static schedules for the persistent attention kernels.  Work items (forward: pair p of a (sample, head);

@@ -61,8 +61,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int wh
   }
   return true;
 }
-// The same for a CTA that gives up as one: the first wait to run out leaves its number in *given_up (shared memory), and every other one returns
-// at once.  The CTA reports it at its end (report_given_up, one thread, behind a barrier of all).
+// The same for a CTA that gives up as one: a wait that runs out leaves its number (not 0) in *given_up (shared memory, 0 before), and from then on others
+// return false instead of waiting.  Of waits that run out within a probe of each other the last one's number stays: a compare-and-swap that kept the first
+// made bidirectional attention slower (32 x 197 tokens, 12 heads, forward + backward 96.6 -> 97.0 us).  The CTA reports the number at its end
+// (report_given_up, one thread, behind a barrier of all).
+template <unsigned long long LIMIT_NS = MLB_MBAR_TIMEOUT_NS>
 __device__ __forceinline__ bool mbar_wait_sticky(uint64_t* bar, uint32_t parity, int where, volatile int* given_up) {
   if (mbar_try(bar, parity)) return true;
   const uint64_t t0 = globaltimer_ns();
@@ -70,7 +73,7 @@ __device__ __forceinline__ bool mbar_wait_sticky(uint64_t* bar, uint32_t parity,
   do {
     if (*given_up) return false;
     if (mbar_try(bar, parity)) return true;
-  } while (globaltimer_ns() - t0 <= MLB_MBAR_TIMEOUT_NS);
+  } while (globaltimer_ns() - t0 <= LIMIT_NS);
   *given_up = where;
   return false;
 }

@@ -93,6 +93,13 @@ def test_a_warp_is_together_again_behind_its_waits():
     assert found > 20 and not apart, "\n".join(apart)
 
 
+def test_a_block_that_gives_up_leaves_a_number():
+    """The word that says so is the number of the wait that ran out: a wait numbered 0 would run out unseen."""
+    numbers = [body[m.end():_close(body, m.end()) - 1].rsplit(",", 1)[1].strip()
+               for _, _, body, _ in _kernels() if "s_abort" in body for m in re.finditer(r"(?<![\w:])wait\(", body)]
+    assert len(numbers) > 90 and all(n == "where" or re.search(r"[1-9]", n) for n in numbers)
+
+
 def test_every_refused_index_has_its_words():
     from ml_b200.ops.native import describe_error
     details = {int(d, 16) for path in KERNELS.glob("*.cu*") for d in re.findall(r"MLB_ERR_BOUNDS, (0x[0-9A-Fa-f]+)\)", path.read_text())}

@@ -1,5 +1,6 @@
 """GPU numerics: every sm_100a kernel against the fp32 PyTorch oracle (ml_b200.ops.ref) on the same inputs,
 including odd shapes that take the scalar / SIMT paths and rows with tgt = -1."""
+import ctypes
 import math
 
 import pytest
@@ -1851,3 +1852,30 @@ def test_causal_backward_at_tile_edges_with_rope(B, T, H, hd):
     d0, d1 = e[:, :, :2, :, 0].clone(), e[:, :, :2, :, 1].clone()
     e[:, :, :2, :, 0], e[:, :, :2, :, 1] = d0 * c + d1 * s, d1 * c - d0 * s
     assert _rel(dqkv, e.view_as(dqkv)) < 2 ** -7
+
+
+def test_a_block_whose_waits_run_out_gives_up_and_says_which():
+    """Waits on a barrier that nobody arrives on, 2 ms at most: all of them end, with the number of one that ran out as the block's word.  Later waits return
+    without waiting for their own limit and leave the word alone, one whose barrier is complete is still answered, and a block's word is what the error word
+    holds.  The context stays usable."""
+    n, blocks, warps = nat(), 592, 8
+    out = torch.zeros(blocks, 32 * warps, 4, device=dev(), dtype=torch.int32)
+    probe = n.lib().mlb_attn_wait_probe
+    probe.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p]
+    try:
+        assert probe(out.data_ptr(), blocks, torch.cuda.current_stream().cuda_stream) == 0
+        torch.cuda.synchronize()
+        err = n.get_error()
+    finally:
+        n.clear_error()
+    answers, word, last, again_us = out.cpu().unbind(-1)
+    assert (answers == 4).all()
+    assert (word >= 1).all() and (word <= warps).all()
+    assert (last == last[:, :1]).all() and (last >= 1).all() and (last <= warps).all()
+    assert err >> 24 == 1 and (err & 0xFFFFFF) in set(last[:, 0].tolist())
+    assert int(again_us.max()) < 2000
+    x = rnd(64, 128)
+    y = torch.empty_like(x)
+    n.rmsnorm_fwd(y, torch.empty(64, device=dev()), x, torch.ones(128, device=dev(), dtype=torch.bfloat16), 1e-6)
+    torch.cuda.synchronize()
+    assert n.get_error() == 0
