@@ -47,37 +47,55 @@ __device__ __forceinline__ void store8_e4m3(uint8_t* p, const float (&f)[8], flo
 // A token id outside [0, V) (a token file made with a larger vocabulary, a damaged file) would index past the table:
 // such a row gets zeros / no gradient, and the error word says so (MLB_ERR_BOUNDS, detail 0xE1 forward, 0xE2 backward,
 // 0xCE for a cross-entropy target), so the step that read it fails on the host instead of corrupting memory.
-// A warp per row, four to a block: with a block per row the rate at which blocks start was the bound (16384 of them take 20 us, whatever
-// they do), then the two dependent trips of a row, its id and the table.  16384 x 768, 50304 rows in the table: 22.6 -> 16.4 us
-// (in L2 20.5 -> 8.2), 2048 x 128 2.9 -> 1.6.
+// PER threads a row: a warp, four rows to a block, because with a block per row the rate at which blocks start is the bound (16384 of them take 17 us,
+// whatever they do); a block of 128 where few rows leave that rate to spare and a warp would have to go round (the rules stand at the entry points).
+// Then the dependent trips of a row are what is left, its id, the table, so four items of each thread are in flight at a time; an unrolled loop is not
+// enough, its remainder goes one by one (768 columns are three vectors a lane).  us with the rows in L2: a block per row (96 and 256 threads, single
+// additions), a warp in an unrolled loop, this.  Forward 64 x 768 1.11, 1.68, 1.17; 64 x 2048 1.65, 1.69, 1.20; 1003 x 768 1.43, 1.70, 1.54; 16384 x 768
+// 17.6, 5.7, 5.6.  Backward, four neighbouring elements an atomic addition where the rows allow it: 64 x 768 1.67, 2.31, 1.27; 64 x 2048 2.54, 4.18, 1.39;
+// 1003 x 768 2.34, 2.52, 1.81; 1003 x 1001 2.70, 9.54, 2.40; 16384 x 768 19.1, 10.7, 10.5.  Slower than the block per row: up to 0.1 us forward at 768 columns
+// and less than 1184 rows, up to 0.4 backward at some 513 odd columns.
+template <int PER, typename T, typename Load, typename Store>
+__device__ __forceinline__ void by_fours(int lane, int items, Load load, Store store) {
+  for (int i = lane; i < items; i += 4 * PER) {
+    T v[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (i + k * PER < items) v[k] = load(i + k * PER);
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (i + k * PER < items) store(i + k * PER, v[k]);
+  }
+}
+template <int PER>
 __global__ void __launch_bounds__(128) embed_fwd_k(bf16* __restrict__ out, const bf16* __restrict__ wte, const int* __restrict__ ids, long rows, int C, int V) {
   mlb_pdl_sync();
-  const int lane = threadIdx.x & 31;
-  const long row = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x % PER;
+  const long row = (long)blockIdx.x * (128 / PER) + threadIdx.x / PER;
   if (row >= rows) return;
   const int id = ids[row];
   bf16* dst = out + row * C;
   if ((unsigned)id >= (unsigned)V) {
     if (lane == 0) mlb_set_error(MLB_ERR_BOUNDS, 0xE1);
-    for (int i = lane; i < C; i += 32) dst[i] = __float2bfloat16(0.f);
+    for (int i = lane; i < C; i += PER) dst[i] = __float2bfloat16(0.f);
     return;
   }
   const bf16* src = wte + (long)id * C;
   if ((C & 7) == 0) {
-#pragma unroll 4
-    for (int i = lane * 8; i < C; i += 256) *reinterpret_cast<uint4*>(dst + i) = *reinterpret_cast<const uint4*>(src + i);
-  } else {
-    for (int i = lane; i < C; i += 32) dst[i] = src[i];
+    by_fours<PER, uint4>(lane, C >> 3, [&](int i) { return reinterpret_cast<const uint4*>(src)[i]; }, [&](int i, uint4 v) { reinterpret_cast<uint4*>(dst)[i] = v; });
+  } else if (C <= 4 * PER) {
+    by_fours<PER, bf16>(lane, C, [&](int i) { return src[i]; }, [&](int i, bf16 v) { dst[i] = v; });
+  } else {      // (several trips by fours: 16384 x 513 9.1 us, so 6.2)
+    for (int i = lane; i < C; i += PER) dst[i] = src[i];
   }
 }
-// The same; four neighbouring elements an atomic addition where the rows allow it.  16384 x 768, 50304 rows: 41 -> 26.7 us (in L2 20.6 -> 12.3),
-// 1003 rows 2.6 -> 2.8.
+template <int PER>
 __global__ void __launch_bounds__(128) embed_bwd_k(float* __restrict__ dwte, const bf16* __restrict__ dout, const int* __restrict__ ids, long rows, int C,
-                                                   int V, int T, int n_pre) {
+                                                   int V, int T, int n_pre, bool vec) {
   mlb_pdl_sync();
-  const int lane = threadIdx.x & 31;
-  const long row = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (row >= rows || (int)(row % T) < n_pre) return;
+  const int lane = threadIdx.x % PER;
+  const long row = (long)blockIdx.x * (128 / PER) + threadIdx.x / PER;
+  if (row >= rows || (n_pre > 0 && (int)(row % T) < n_pre)) return;
   const int id = ids[row];
   if ((unsigned)id >= (unsigned)V) {
     if (lane == 0) mlb_set_error(MLB_ERR_BOUNDS, 0xE2);
@@ -85,16 +103,13 @@ __global__ void __launch_bounds__(128) embed_bwd_k(float* __restrict__ dwte, con
   }
   float* dst = dwte + (long)id * C;
   const bf16* src = dout + row * C;
-  if ((C & 3) == 0 && ((reinterpret_cast<uintptr_t>(dwte) & 15) | (reinterpret_cast<uintptr_t>(dout) & 7)) == 0) {
-#pragma unroll 4
-    for (int i = lane * 4; i < C; i += 128) {
-      const uint2 u = *reinterpret_cast<const uint2*>(src + i);
-      asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + i), "f"(__uint_as_float(u.x << 16)),
+  if (vec)
+    by_fours<PER, uint2>(lane, C >> 2, [&](int i) { return reinterpret_cast<const uint2*>(src)[i]; }, [&](int i, uint2 u) {
+      asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + i * 4), "f"(__uint_as_float(u.x << 16)),
                    "f"(__uint_as_float(u.x & 0xffff0000u)), "f"(__uint_as_float(u.y << 16)), "f"(__uint_as_float(u.y & 0xffff0000u)) : "memory");
-    }
-  } else {
-    for (int i = lane; i < C; i += 32) atomicAdd(dst + i, __bfloat162float(src[i]));
-  }
+    });
+  else
+    by_fours<PER, bf16>(lane, C, [&](int i) { return src[i]; }, [&](int i, bf16 v) { atomicAdd(dst + i, __bfloat162float(v)); });
 }
 __global__ void set_prefix_k(bf16* __restrict__ x, const bf16* __restrict__ prefix, int B, int T, int n_pre, int C) {
   mlb_pdl_sync();
@@ -1442,12 +1457,25 @@ inline int gs(long n, int per_block) { return (int)((n + per_block - 1) / per_bl
 static int g_ce_smem = 0;     // tuning hook: 0 = always the two-pass cross-entropy kernel
 MLB_API void mlb_ce_mode(int smem_row) { g_ce_smem = smem_row; }
 
+// Does a row get a block?  Where its items (vectors, or elements where it has none) are more than the 128 that a warp has in flight, and up to as many
+// rows as leave the start of blocks to spare.  With a block and with a warp, us: forward 1184 x 1024 1.57 and 1.93, 1536 x 1024 1.87 and 2.07, 2048 x 1024
+// 2.40 and 1.81; long rows are bound by memory sooner (768 x 4096 2.4 ... 3.1 and 2.7).  Backward 768 x 1024 1.93 and 2.01, 1184 x 1024 2.39 and 2.13;
+// single additions, 2048 x 1001 3.6 and 4.7, 4096 x 1001 5.7 and 5.8, 16384 x 513 17.7 and 10.8.
+static bool embed_fwd_wide(long rows, int C) { return (C % 8 == 0 ? C / 8 : C) >= 128 && rows <= 1184 && rows * C <= 1L << 21; }
+static bool embed_bwd_wide(long rows, int C, bool vec) { return vec ? C >= 512 && rows <= 1024 : C >= 128 && rows <= (C >= 512 ? 2048 : 1024); }
 MLB_API int mlb_embed_fwd(void* out, const void* wte, const int* ids, long BT, int C, int V, cudaStream_t st) {
-  mlb_launch(embed_fwd_k, dim3((unsigned)((BT + 3) / 4)), dim3(128), 0, st, (bf16*)out, (const bf16*)wte, ids, (long)BT, C, V);
+  if (embed_fwd_wide(BT, C))
+    mlb_launch(embed_fwd_k<128>, dim3((unsigned)BT), dim3(128), 0, st, (bf16*)out, (const bf16*)wte, ids, (long)BT, C, V);
+  else
+    mlb_launch(embed_fwd_k<32>, dim3((unsigned)((BT + 3) / 4)), dim3(128), 0, st, (bf16*)out, (const bf16*)wte, ids, (long)BT, C, V);
   LAUNCH_RET;
 }
 MLB_API int mlb_embed_bwd(float* dwte, const void* dout, const int* ids, long BT, int C, int V, int T, int n_pre, cudaStream_t st) {
-  mlb_launch(embed_bwd_k, dim3((unsigned)((BT + 3) / 4)), dim3(128), 0, st, dwte, (const bf16*)dout, ids, (long)BT, C, V, T, n_pre);
+  const bool vec = C % 4 == 0 && (((uintptr_t)dwte & 15) | ((uintptr_t)dout & 7)) == 0;
+  if (embed_bwd_wide(BT, C, vec))
+    mlb_launch(embed_bwd_k<128>, dim3((unsigned)BT), dim3(128), 0, st, dwte, (const bf16*)dout, ids, (long)BT, C, V, T, n_pre, vec);
+  else
+    mlb_launch(embed_bwd_k<32>, dim3((unsigned)((BT + 3) / 4)), dim3(128), 0, st, dwte, (const bf16*)dout, ids, (long)BT, C, V, T, n_pre, vec);
   LAUNCH_RET;
 }
 MLB_API int mlb_set_prefix(void* x, const void* prefix, int B, int T, int n_pre, int C, cudaStream_t st) {

@@ -583,6 +583,14 @@ def test_embedding_rows_and_widths(BT, C, shift):
     assert ((dw - e).abs() <= bound).all()
 
 
+# (forward a block per row: items >= 128 in up to 1184 rows and 2^21 elements; backward: 128 items in up to 1024 rows, 2048 of single additions)
+@pytest.mark.parametrize("BT,C,shift", [(1, 768, 0), (1024, 512, 0), (1025, 512, 0), (1184, 1024, 0), (1185, 1024, 0), (1025, 2048, 0), (3, 4104, 0), (2048, 513, 0),
+                                        (2049, 513, 0), (1024, 129, 0), (1025, 127, 0), (40, 1024, 1), (40, 1020, 2)])
+def test_embedding_either_side_of_its_lines(BT, C, shift):
+    """A warp and a block per row, whole and partial trips of four items a thread."""
+    test_embedding_rows_and_widths(BT, C, shift)
+
+
 def test_vision_helpers_and_casts():
     torch.manual_seed(14)
     B, g = 2, 3
