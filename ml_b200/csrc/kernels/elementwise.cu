@@ -711,31 +711,40 @@ __global__ void __launch_bounds__(WARPS * 32) fold_cols_k(void* __restrict__ dw,
   __shared__ float rowbuf[SL == WARPS ? 1 : TRIP][32], red[SL][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
   float s = 0.f;
-  for (int r0 = 0; r0 < nrows; r0 += TRIP) {
-    float v[FOLD_ROWS];
+  if (!TREE && SL == WARPS) {      // (the columns asked about once and not in each load: 40 registers, 32 in the other form; column sums of 3152 x 2304 4.60 -> 4.39 us)
+    if (c < W) {
+      for (int r = warp; r < nrows; r += TRIP) {
+        float v[FOLD_ROWS];
 #pragma unroll
-    for (int k = 0; k < FOLD_ROWS; k++) {
-      const int r = r0 + warp + WARPS * k;
-      v[k] = r < nrows && c < W ? partial[(size_t)r * W + c] : 0.f;
+        for (int k = 0; k < FOLD_ROWS; k++) v[k] = r + WARPS * k < nrows ? partial[(size_t)(r + WARPS * k) * W + c] : 0.f;
+#pragma unroll
+        for (int k = 0; k < FOLD_ROWS; k++) s += v[k];
+      }
     }
-    if (TREE) {
+  } else {
+    for (int r0 = 0; r0 < nrows; r0 += TRIP) {
+      float v[FOLD_ROWS];
 #pragma unroll
-      for (int w = 1; w < FOLD_ROWS; w *= 2)
+      for (int k = 0; k < FOLD_ROWS; k++) {
+        const int r = r0 + warp + WARPS * k;
+        v[k] = r < nrows && c < W ? partial[(size_t)r * W + c] : 0.f;
+      }
+      if (TREE) {
 #pragma unroll
-        for (int k = 0; k + w < FOLD_ROWS; k += 2 * w) v[k] += v[k + w];
-      s += v[0];
-    } else if (SL == WARPS) {
+        for (int w = 1; w < FOLD_ROWS; w *= 2)
 #pragma unroll
-      for (int k = 0; k < FOLD_ROWS; k++) s += v[k];
-    } else {
-      if (r0 > 0) __syncthreads();
+          for (int k = 0; k + w < FOLD_ROWS; k += 2 * w) v[k] += v[k + w];
+        s += v[0];
+      } else {
+        if (r0 > 0) __syncthreads();
 #pragma unroll
-      for (int k = 0; k < FOLD_ROWS; k++) rowbuf[warp + WARPS * k][lane] = v[k];
-      __syncthreads();
-      if (warp < SL) {
-        const int n = min(TRIP, nrows - r0);
+        for (int k = 0; k < FOLD_ROWS; k++) rowbuf[warp + WARPS * k][lane] = v[k];
+        __syncthreads();
+        if (warp < SL) {
+          const int n = min(TRIP, nrows - r0);
 #pragma unroll 8
-        for (int r = warp; r < n; r += SL) s += rowbuf[r][lane];
+          for (int r = warp; r < n; r += SL) s += rowbuf[r][lane];
+        }
       }
     }
   }
