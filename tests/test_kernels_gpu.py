@@ -858,6 +858,24 @@ def _attn64(qkv, dout, B, T, H, hd, causal):
     return out.detach(), torch.logsumexp(s, -1).detach(), g.permute(1, 3, 0, 2, 4).reshape(B * T, 3 * H * hd)
 
 
+def _attn_bwd_bound64(qkv, dout, B, T, H, hd):
+    """How far each element of causal attention's dqkv may be from 64 bits before its last rounding.  Rounding to bf16 costs 2^-9 of a value, twice that is
+    allowed for what is not written out (exponentials, sums in 32 bits).  P is rounded for dV, dS for dQ and dK, dQ's partial sums once more; the forward's P
+    is cut off (2^-7), and what that and its rounding do to O reaches dS through delta = rowsum(dO O)."""
+    q, k, v = qkv.double().view(B, T, 3, H, hd).permute(2, 0, 3, 1, 4)
+    g = dout.double().view(B, T, H, hd).transpose(1, 2)
+    sc = hd ** -0.5
+    P = torch.softmax((q @ k.transpose(-1, -2) * sc).masked_fill(torch.ones(T, T, dtype=torch.bool, device=q.device).triu(1), float("-inf")), -1)
+    O = P @ v
+    dS = P * (g @ v.transpose(-1, -2) - (g * O).sum(-1, keepdim=True))
+    d_delta = (g.abs() * (2 ** -7 * (P @ v.abs()) + 2 ** -8 * O.abs())).sum(-1, keepdim=True)
+    E = 2 ** -8 * dS.abs() + P * d_delta
+    bq = sc * (E + 2 ** -8 * dS.abs()) @ k.abs()
+    bk = sc * E.transpose(-1, -2) @ q.abs()
+    bv = 2 ** -8 * P.transpose(-1, -2) @ g.abs()
+    return torch.stack((bq, bk, bv)).permute(1, 3, 0, 2, 4).reshape(B * T, 3 * H * hd).contiguous()
+
+
 def _rel(a, e):
     return ((a.double() - e).norm() / e.norm()).item()
 
@@ -1860,6 +1878,44 @@ def test_causal_backward_at_tile_edges_with_rope(B, T, H, hd):
     d0, d1 = e[:, :, :2, :, 0].clone(), e[:, :, :2, :, 1].clone()
     e[:, :, :2, :, 0], e[:, :, :2, :, 1] = d0 * c + d1 * s, d1 * c - d0 * s
     assert _rel(dqkv, e.view_as(dqkv)) < 2 ** -7
+    # and each element, so that no row of one head can be another's: the norm above would let one pass
+    b = _attn_bwd_bound64(rot, dout, B, T, H, hd).view(B, T, 3, H, 2, hd // 2)
+    b0, b1 = b[:, :, :2, :, 0].clone(), b[:, :, :2, :, 1].clone()
+    b[:, :, :2, :, 0], b[:, :, :2, :, 1] = b0 * c.abs() + b1 * s.abs(), b1 * c.abs() + b0 * s.abs()
+    b += 2 ** -8 * e.abs()
+    far = ((dqkv.double().view_as(e) - e).abs() / (b + 1e-30)).amax((0, 1, 3, 4, 5))
+    assert (far <= 1).all(), far.tolist()
+
+
+@pytest.mark.parametrize("hd,B,T,H", [(64, 640, 16, 16), (64, 320, 130, 16), (128, 640, 16, 16), (128, 320, 130, 16)])
+def test_attention_with_more_items_than_a_block_keeps_at_hand(hd, B, T, H):
+    """A block takes its first 48 (64) work items from shared memory and later ones from the schedule: with 69 and more to a block on 148 SMs each sample is
+    still what it is alone, one item to a block, bit for bit.  Head size 64: from the device's counter too, through a ring of 64."""
+    assert B * H * ((T + 127) // 128) > 64 * torch.cuda.get_device_properties(0).multi_processor_count
+    torch.manual_seed(T + hd)
+    n = nat()
+    qkv, dout = rnd(B * T, 3 * H * hd), rnd(B * T, H * hd)
+    rope = ref.rope_tables(T, hd, 10000.0, dev())
+
+    def run(r, samples):
+        q, g = qkv[r], dout[r]
+        out, lse, d = torch.empty_like(g), torch.empty(samples, H, T, device=dev()), torch.full_like(q, float("nan"))
+        n.attn_fwd(out, lse, q, samples, T, H, hd)
+        assert n.attn_bwd(d, g, q, out, lse, samples, T, H, hd, rope=rope)
+        return out.view(samples, T, -1), lse, d.view(samples, T, -1)
+
+    alone = [run(slice(b * T, (b + 1) * T), 1) for b in range(0, B, 7)]
+    want = [torch.cat(x) for x in zip(*alone)]
+    for dynamic in (False, True) if hd == 64 else (False,):
+        n.attn_dynamic(dynamic)
+        try:
+            got = run(slice(None), B)
+            torch.cuda.synchronize()
+        finally:
+            n.attn_dynamic(False)
+        assert n.get_error() == 0
+        assert all(torch.equal(x[::7], w) for x, w in zip(got, want))
+        assert not got[2].isnan().any()
 
 
 def test_a_block_whose_waits_run_out_gives_up_and_says_which():
