@@ -1374,7 +1374,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kv_tc_kernel(const __
 // Persistent CTAs, one per SM; a work item is one 128-key tile of a (sample, head) and loops over the query tiles
 // i >= its own; the items of a CTA come from a balanced schedule built on the host (attn_schedule).  Per query block:
 //     S^T = K Q^T, dP^T = V dO^T                            (two MMAs into TMEM)
-//     P^T = exp2(S^T*c - lse), dS^T = P^T (dP^T - delta)    (512 threads, packed f32x2 math)
+//     P^T = exp2(S^T*c - lse), dS^T = P^T (dP^T - delta)    (8 warps, packed f32x2 math)
 //     dV += P^T dO   (P^T stays in TMEM as the bf16 A operand),   dK += dS^T Q,   dQ_i = dS K   (dS^T in shared memory)
 // The pipeline keeps the tensor core and the element-wise warps busy at the same time:
 //   * as soon as the element-wise warps have S^T (dP^T) of block j in registers they hand its TMEM columns back and the score thread

@@ -1658,10 +1658,11 @@ MLB_API int mlb_rmsnorm_bwd(void* dx, float* dw, const void* dy, const void* x, 
   // Whole multiples of 256 columns: a block's threads share a row instead of a warp having one, and the partial rows are folded by a
   // kernel of their own, which overlaps this one's end.  One warp a row, with the fold by the blocks that finish last, against this, inputs
   // not in L2: 16384 x 768 31.7 -> 27.6 us, 4096 x 768 21 -> 15.4, 65536 x 256 46 -> 33.8, 4096 x 512 17.4 -> 15.4, 16384 x 512 25.6 -> 23.6
-  // (in L2 14.1 = 14.1).  In a small model's step, though, the host's launches are the bound and one less is worth more than the 2 us by which
+  // (in L2 14.1 = 14.1; without a residual gradient 18.0 -> 14.7 and 22.3 -> 19.4 at 16384 x 512 and 768, but in L2 13.1 -> 13.6 and 17.2 -> 18.0).
+  // In a small model's step, though, the host's launches are the bound and one less is worth more than the 2 us by which
   // this is shorter there too; the step's products grow as rows C^2, and so does the line.  Steps of two layers, us, one launch and two: 256 wide,
   // 512 rows 358 and 368, 4096 rows 363 and 374, 8192 rows 444 and 443; 512 wide, 1024 rows 361 and 370, 2048 rows 411 and 399; 768 wide,
-  // 128 rows 392 and 401, 512 rows 459 and 443.
+  // 128 rows 392 and 401, 512 rows 459 and 443.  (All of that uncaptured: a captured step, which has no launches to save, pays the 2 us a norm below the line.)
   const bool rows_ok = norm_rows_ok(dx, dy, x, w, add, rows, C);
   if (rows_ok && (C >= 1024 || rows * C * C > 1L << 28)) {
     norm_rows_launch<false>(dx, dw, nullptr, false, dy, x, w, nullptr, rstd, add, rows, C, partial, st);
